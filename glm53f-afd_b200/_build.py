@@ -1,4 +1,4 @@
-"""Compiles the CUDA sources under csrc/ into libglm53f_kda.so beside this file (nvcc, sm_100a only)."""
+"""Compiles the CUDA sources under csrc/ into libglm53f_kda.so beside this file (nvcc, sm_100a only), and the host module."""
 from __future__ import annotations
 
 import os
@@ -8,6 +8,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 LIB = os.path.join(HERE, "libglm53f_kda.so")
+HOST = os.path.join(HERE, "_host.so")  # a Python module: the native host path of the per-layer launches
 
 # The IEEE flags are the reference's (crates/glm53f-kda/build.rs:63-68): the chain, the replays and the prologue
 # must not contract a multiply and an add, or a replayed prefix stops matching serial steps bit for bit.
@@ -55,7 +56,25 @@ def build(force: bool = False, verbose: bool = False) -> str:
         objs.append(obj)
     if force or _stale(LIB, objs):
         subprocess.check_call([nvcc(), "-gencode", "arch=compute_100a,code=sm_100a", "-shared", "-o", LIB, *objs])
+    build_host(force)
     return LIB
+
+
+def build_host(force: bool = False) -> str:
+    """csrc/host_calls.cpp against Python's and torch's headers, linked to the library beside it."""
+    src = os.path.join(CSRC, "host_calls.cpp")
+    if force or _stale(HOST, [src, os.path.join(INCLUDE, "glm53f_kda.h")]):
+        import sysconfig
+
+        import torch
+
+        t = os.path.dirname(torch.__file__)
+        cuda = os.path.dirname(os.path.dirname(nvcc()))
+        subprocess.check_call(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-I" + INCLUDE,
+                               "-I" + sysconfig.get_paths()["include"], "-isystem", os.path.join(t, "include"), "-isystem", os.path.join(cuda, "include"), src,
+                               "-o", HOST, "-L" + HERE, "-l:" + os.path.basename(LIB), "-L" + os.path.join(t, "lib"), "-lc10", "-lc10_cuda", "-ltorch_python",
+                               "-ltorch_cpu", "-Wl,-rpath,$ORIGIN"])
+    return HOST
 
 
 if __name__ == "__main__":

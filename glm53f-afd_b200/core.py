@@ -83,6 +83,11 @@ def decode_batch(heads, rows, cu_rows, q, k, v, g, beta, state, state_off, *, st
     """glm53f_kda_core_decode_batch / _verify_batch.  `rows` = total rows (host), `cu_rows` int32 [batch+1] and
     `state_off` int64 [batch] on the device.  state_out: "in_place", None (verify: not written) or a tensor.
     saves = (k f32, v bf16, g f32, beta f32) makes it the verify entry point."""
+    code = ffi.host().core_decode(heads, rows, cu_rows, q, k, v, g, beta, state, state_off, state_out, flags, gate, norm_w, eps, out, saves,
+                                  max_state_off)
+    if code >= 0:
+        return _launched(code, "glm53f_kda_core_decode_batch" if saves is None else "glm53f_kda_core_verify_batch")
+    # Not the plain accepted call: the same checks here, with their errors.
     batch = cu_rows.numel() - 1
     _need(cu_rows, "cu_rows", (torch.int32,), 2)
     _need(state_off, "state_off", (torch.int64,), batch)

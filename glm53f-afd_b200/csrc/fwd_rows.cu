@@ -5,11 +5,14 @@
 // walks the row 2 KiB at a time; a mark's rows are pool pages of 394,944 bytes, so a launch there is 181-376 blocks
 // with one 16-byte load in flight per thread.  Here the (row, 32 KiB tile) pairs of a launch are spread over the
 // whole grid and a thread keeps eight independent 16-byte loads in flight before its first store (32 KiB per block
-// of 256 threads and iteration, up to eight blocks per SM), with streaming cache hints in both directions: the data
-// is not read again soon.  Rows of at most 4 KiB (the token rows other callers of the same entry points move) go one
+// of 256 threads and iteration, up to eight blocks per SM).  Loads carry the streaming hint; stores keep the normal
+// policy, so that a mark that is read back soon (a fork or rewind follows its snapshot) still finds part of its 73 MiB in
+// the 126 MB L2: snapshot + fork of four slots 215 -> 190 us against streaming stores.  Rows of at most 4 KiB (the token rows other callers of the same entry points move) go one
 // warp per row.
 //
 // Results are the bytes of the reference's kernel: dst[i] = src[idx[i]] (gather) or dst[idx[i]] = src[i] (scatter).
+
+#include <cstring>
 
 #include "common.cuh"
 #include "glm53f_fwd_rows.h"
@@ -33,9 +36,11 @@ constexpr int kCopyThreads = ROWS_THREADS;
 constexpr int kVecs = ROWS_VECS;                       // 16-byte loads in flight per thread
 constexpr int kTileChunks = kCopyThreads * kVecs;      // 16-byte chunks per tile: 32 KiB
 constexpr int kSmallChunks = 32 * kVecs;               // rows up to 4 KiB: one warp per row
+constexpr int kInlinePages = 900;                      // page lists up to this length travel in the kernel's parameters
+constexpr int kInlineWords = 1000;                     // words one store_words launch carries
 
 __device__ __forceinline__ uint4 load_stream(const uint4* p) { return __ldcs(p); }
-__device__ __forceinline__ void store_stream(uint4* p, const uint4& v) { __stcs(p, v); }
+__device__ __forceinline__ void store_cached(uint4* p, const uint4& v) { *p = v; }
 
 // Copies chunks [first, first + n * stride) of a row, at most kVecs per caller thread: all loads, then all stores.
 __device__ __forceinline__ void copy_vecs(const uint4* __restrict__ s, uint4* __restrict__ d, long long first, int stride, long long chunks) {
@@ -48,7 +53,7 @@ __device__ __forceinline__ void copy_vecs(const uint4* __restrict__ s, uint4* __
 #pragma unroll
     for (int j = 0; j < kVecs; ++j) {
         const long long c = first + (long long)j * stride;
-        if (c < chunks) store_stream(d + c, v[j]);
+        if (c < chunks) store_cached(d + c, v[j]);
     }
 }
 
@@ -88,8 +93,21 @@ struct MarkParts {
     long long units;          // all marks' units
 };
 
+// A mark's page list: a device array, or carried in the kernel's parameters.  The second form spares the host the
+// copy of the list to the device (a blocking copy from pageable memory before every mark: 20 of the 80 us that a mark and
+// a fork took on the host); kInlinePages entries keep the parameters under the 4 KiB every launch can carry.
+struct DevicePages {
+    const int32_t* idx;
+    __device__ __forceinline__ long long operator()(long long i) const { return idx[i]; }
+};
+struct InlinePages {
+    int32_t idx[kInlinePages];
+    __device__ __forceinline__ long long operator()(long long i) const { return idx[i]; }
+};
+
+template <typename Pages>
 __global__ void __launch_bounds__(kCopyThreads, ROWS_MIN_BLOCKS) mark_copy_kernel(uint8_t* __restrict__ pages, long long page_chunks, int tiles_per_page,
-                                                                 const int32_t* __restrict__ page_idx, const MarkParts m, int save) {
+                                                                 const __grid_constant__ Pages page_idx, const __grid_constant__ MarkParts m, int save) {
     for (long long u0 = blockIdx.x; u0 < m.units; u0 += gridDim.x) {
         const long long mark = u0 / m.first_unit[3], u = u0 - mark * m.first_unit[3];
         const int p = u >= m.first_unit[2] ? 2 : u >= m.first_unit[1] ? 1 : 0;
@@ -99,12 +117,21 @@ __global__ void __launch_bounds__(kCopyThreads, ROWS_MIN_BLOCKS) mark_copy_kerne
         // What this page holds of the part: a whole page, or the part's remainder.
         const long long left = m.chunks[p] - page * page_chunks;
         const long long n = left < page_chunks ? left : page_chunks;
-        uint4* in_pool = reinterpret_cast<uint4*>(pages) + (long long)page_idx[mark * m.mark_pages + m.first_page[p] + page] * page_chunks;
+        uint4* in_pool = reinterpret_cast<uint4*>(pages) + page_idx(mark * m.mark_pages + m.first_page[p] + page) * page_chunks;
         uint4* in_arena = reinterpret_cast<uint4*>(m.part[p]) + (m.slots ? (long long)m.slots[mark] * m.slot_chunks[p] : 0) + page * page_chunks;
         const long long c0 = (long long)tile * kTileChunks + threadIdx.x;
         if (save) copy_vecs(in_arena, in_pool, c0, kCopyThreads, n);
         else copy_vecs(in_pool, in_arena, c0, kCopyThreads, n);
     }
+}
+
+// A few words of host data into device memory, in stream order, without a staging buffer or a wait: they travel in the
+// kernel's parameters.  Batch metadata (a few hundred bytes per round) goes this way.
+struct Words {
+    uint32_t w[kInlineWords];
+};
+__global__ void __launch_bounds__(256) store_words_kernel(uint32_t* __restrict__ dst, int n, const __grid_constant__ Words words) {
+    for (int i = threadIdx.x; i < n; i += 256) dst[i] = words.w[i];
 }
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
@@ -151,7 +178,8 @@ extern "C" int32_t glm53f_fwd_scatter_rows(const uint8_t* src, int64_t src_strid
 namespace kda {
 namespace {
 int32_t mark_copy_launch(uint8_t* pages, int64_t page_bytes, const int32_t* page_idx, uint8_t* const part[3], const int64_t part_bytes[3],
-                         const int64_t* slot_stride, const int32_t* slots, int32_t marks, int32_t save, cudaStream_t stream) {
+                         const int64_t* slot_stride, const int32_t* slots, int32_t marks, int32_t save, cudaStream_t stream,
+                         const int32_t* host_idx = nullptr, int32_t host_pages = 0) {
     if (!part || !part_bytes || page_bytes <= 0 || page_bytes % 16 || marks < 0) return cudaErrorInvalidValue;
     MarkParts m{};
     const long long page_chunks = page_bytes / 16;
@@ -177,8 +205,15 @@ int32_t mark_copy_launch(uint8_t* pages, int64_t page_bytes, const int32_t* page
     m.slots = slots;
     m.units = unit * marks;
     if (m.units == 0) return cudaSuccess;
-    if (!pages || !aligned16(pages) || !page_idx) return cudaErrorInvalidValue;
-    mark_copy_kernel<<<grid_for(m.units), kCopyThreads, 0, stream>>>(pages, page_chunks, (int)tiles, page_idx, m, save != 0);
+    if (!pages || !aligned16(pages) || (!page_idx && !host_idx)) return cudaErrorInvalidValue;
+    if (host_idx) {
+        if (host_pages != m.mark_pages || host_pages > kInlinePages) return cudaErrorInvalidValue;
+        InlinePages list;
+        memcpy(list.idx, host_idx, (size_t)host_pages * sizeof(int32_t));
+        mark_copy_kernel<<<grid_for(m.units), kCopyThreads, 0, stream>>>(pages, page_chunks, (int)tiles, list, m, save != 0);
+    } else {
+        mark_copy_kernel<<<grid_for(m.units), kCopyThreads, 0, stream>>>(pages, page_chunks, (int)tiles, DevicePages{page_idx}, m, save != 0);
+    }
     return cudaGetLastError();
 }
 }  // namespace
@@ -194,4 +229,23 @@ extern "C" int32_t glm53f_kda_mark_copy_slots(uint8_t* pages, int64_t page_bytes
                                               int32_t save, glm53f_stream_t stream) {
     if (!slot_stride || (marks > 0 && !slots)) return cudaErrorInvalidValue;
     return kda::mark_copy_launch(pages, page_bytes, page_idx, arena, part_bytes, slot_stride, slots, marks, save, stream);
+}
+
+extern "C" int32_t glm53f_kda_mark_copy_list(uint8_t* pages, int64_t page_bytes, const int32_t* page_list, int32_t n_pages, uint8_t* const part[3],
+                                             const int64_t part_bytes[3], int32_t save, glm53f_stream_t stream) {
+    if (!page_list || n_pages < 0 || n_pages > kda::kInlinePages) return cudaErrorInvalidValue;
+    return kda::mark_copy_launch(pages, page_bytes, nullptr, part, part_bytes, nullptr, nullptr, 1, save, stream, page_list, n_pages);
+}
+
+extern "C" int32_t glm53f_kda_store_words(uint32_t* dst, const uint32_t* host, int32_t words, glm53f_stream_t stream) {
+    if (words < 0 || (words > 0 && (!dst || !host || (reinterpret_cast<uintptr_t>(dst) & 3)))) return cudaErrorInvalidValue;
+    kda::Words buf;
+    for (int32_t at = 0; at < words; at += kda::kInlineWords) {
+        const int n = words - at < kda::kInlineWords ? words - at : kda::kInlineWords;
+        memcpy(buf.w, host + at, (size_t)n * sizeof(uint32_t));
+        kda::store_words_kernel<<<1, 256, 0, stream>>>(dst + at, n, buf);
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }

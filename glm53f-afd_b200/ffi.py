@@ -54,12 +54,14 @@ SIGNATURES = {
     "glm53f_fwd_scatter_rows": (I32, [P, I64, P, P, I64, I32, I64, P]),
     "glm53f_kda_mark_copy": (I32, [P, I64, P, P, P, I32, P]),
     "glm53f_kda_mark_copy_slots": (I32, [P, I64, P, P, P, P, P, I32, I32, P]),
+    "glm53f_kda_mark_copy_list": (I32, [P, I64, P, I32, P, P, I32, P]),
+    "glm53f_kda_store_words": (I32, [P, P, I32, P]),
     # include/glm53f_proj.h: the projections' GEMM (the arguments of glm53f_fwd_gemv_bf16 without its split-K scratch)
     "glm53f_kda_proj_bf16": (I32, [P, I64, I64, P, I64, I64, I32, I32, I32, I32, P, I32, I64, I64, P]),
 }
 
 # The reference's thirteen (crates/glm53f-kda/tests/provenance.rs:41-69 asserts exactly these).
-REFERENCE_SYMBOLS = [n for n in SIGNATURES if n.startswith("glm53f_kda_") and "_core_" not in n and "_gather_" not in n and n not in ("glm53f_kda_device_status", "glm53f_kda_debug_wait_test", "glm53f_kda_prefill_mode", "glm53f_kda_verify_mode", "glm53f_kda_commit_mode", "glm53f_kda_mark_copy", "glm53f_kda_mark_copy_slots", "glm53f_kda_proj_bf16", "glm53f_kda_chain_commit_batch")]
+REFERENCE_SYMBOLS = [n for n in SIGNATURES if n.startswith("glm53f_kda_") and "_core_" not in n and "_gather_" not in n and n not in ("glm53f_kda_device_status", "glm53f_kda_debug_wait_test", "glm53f_kda_prefill_mode", "glm53f_kda_verify_mode", "glm53f_kda_commit_mode", "glm53f_kda_mark_copy", "glm53f_kda_mark_copy_slots", "glm53f_kda_mark_copy_list", "glm53f_kda_store_words", "glm53f_kda_proj_bf16", "glm53f_kda_chain_commit_batch")]
 
 
 def library_path() -> str:
@@ -84,6 +86,24 @@ def load(path: str | None = None):
     if path == _build.LIB:
         _lib = lib
     return lib
+
+
+_native = None
+
+
+def host():
+    """The native host path of the per-layer launches (csrc/host_calls.cpp).  Raises if it has not been built."""
+    global _native
+    if _native is None:
+        if not os.path.exists(_build.HOST):
+            raise RuntimeError(f"{_build.HOST} is missing: build it with `python -c 'import __graft_entry__ as g; g.build()'`")
+        import torch  # noqa: F401  its libraries are what the module links
+
+        from . import _host as module, kernel as K
+
+        module.bind(K.DeviceBuffer, K.RowView, K.Weights, K.Saves, K.ChainBatch, K.BatchMeta, K.Stream)
+        _native = module
+    return _native
 
 
 def __getattr__(name: str):

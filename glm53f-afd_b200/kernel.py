@@ -122,6 +122,12 @@ class Stream:
         (self.stream if self.stream is not None else torch.cuda.current_stream()).synchronize()
 
 
+def raw_stream(stream: Stream) -> int:
+    """The stream's address (0: the legacy default stream)."""
+    raw = ffi.host().raw_stream(stream)
+    return (stream.raw().value or 0) if raw is None else raw
+
+
 def _launched(code: int, what: str) -> None:
     if code == 0:
         return
@@ -418,10 +424,18 @@ class BatchMeta:
     def __init__(self, capacity: int):
         self.capacity = capacity
         self._requests: list[Request] = []
-        self.cu_rows = DeviceBuffer.zeroed((capacity + 1) * 4)
-        self.keep_d = DeviceBuffer.zeroed(capacity * 4)
-        self.conv_off = DeviceBuffer.zeroed(capacity * 8)
-        self.state_off = DeviceBuffer.zeroed(capacity * 8)
+        # One allocation, so that one copy brings everything up to date: cu_rows, keep (int32), conv and state offsets
+        # (int64), each part from a multiple of 16 bytes.
+        self._at = [0]
+        for n in ((capacity + 1) * 4, capacity * 4, capacity * 8, capacity * 8):
+            self._at.append((self._at[-1] + n + 15) // 16 * 16)
+        self._all = DeviceBuffer.zeroed(self._at[-1])
+        part = lambda i, n: DeviceBuffer(self._all.t[self._at[i]:self._at[i] + n])
+        self.cu_rows = part(0, (capacity + 1) * 4)
+        self.keep_d = part(1, capacity * 4)
+        self.conv_off = part(2, capacity * 8)
+        self.state_off = part(3, capacity * 8)
+        self._extent = None  # what a launch's checks need of the requests: see _set
 
     @classmethod
     def new(cls, capacity: int) -> "BatchMeta":
@@ -430,6 +444,21 @@ class BatchMeta:
     def set(self, requests: Sequence[Request], keep: Optional[Sequence[int]] = None) -> None:
         """Set the requests and, for replays and conv shifts, the rows each keeps (None: all).  Copies to the device
         synchronously."""
+        image = self._set(requests, keep)
+        torch = _torch()
+        self._all.t.copy_(torch.from_numpy(image.view(np.uint8)))
+        if self._all.t.is_cuda:
+            torch.cuda.synchronize()
+
+    def set_on(self, requests: Sequence[Request], keep: Optional[Sequence[int]], stream: Stream) -> None:
+        """`set` in the order of `stream`, without waiting for it: for launches on that stream."""
+        if not self._all.t.is_cuda:
+            return self.set(requests, keep)
+        image = self._set(requests, keep)
+        _launched(ffi.glm53f_kda_store_words(self._all.ptr(), image.ctypes.data, image.size, stream.raw()), "glm53f_kda_store_words")
+
+    def _set(self, requests: Sequence[Request], keep: Optional[Sequence[int]]) -> np.ndarray:
+        """Check the requests, take them over and return the device image (32-bit words)."""
         if len(requests) == 0 or len(requests) > self.capacity:
             raise Invalid(f"{len(requests)} requests for a capacity of {self.capacity}")
         if keep is None:
@@ -446,11 +475,18 @@ class BatchMeta:
                 raise Invalid("total rows do not fit in 32 bits")
             cu.append(nxt)
         keep32 = [_to_i32(k, "keep") for k in keep]
-        self.cu_rows.upload(np.asarray(cu, np.int32))
-        self.keep_d.upload(np.asarray(keep32, np.int32))
-        self.conv_off.upload(np.asarray([r.conv_offset for r in requests], np.int64))
-        self.state_off.upload(np.asarray([r.state_offset for r in requests], np.int64))
+        conv, state = [r.conv_offset for r in requests], [r.state_offset for r in requests]
+        image = np.zeros(self._at[-1] // 4, np.int32)
+        n, at = len(requests), [a // 4 for a in self._at]
+        image[:n + 1] = cu
+        image[at[1]:at[1] + n] = keep32
+        image[at[2]:at[2] + 2 * n].view(np.int64)[:] = conv
+        image[at[3]:at[3] + 2 * n].view(np.int64)[:] = state
+        # requests, rows, then of the conv and the state offsets: least, greatest, least distance between two
+        spread = lambda v: (v[0], v[-1], min((b - a for a, b in zip(v, v[1:])), default=1 << 62))
+        self._extent = (n, cu[-1], *spread(sorted(conv)), *spread(sorted(state)))
         self._requests = list(requests)
+        return image
 
     def requests(self) -> list[Request]:
         return self._requests
@@ -518,6 +554,10 @@ class ChainBatch:
         self._launch_as(meta, stream, StateType.Bf16)
 
     def _launch_as(self, meta: BatchMeta, stream: Stream, st: StateType) -> None:
+        code = ffi.host().chain_batch(self, meta, stream, st is StateType.Bf16)
+        if code >= 0:
+            return _launched(code, "glm53f_kda_chain_batch")
+        # Not the plain accepted call: the same checks here, with their errors.
         es, h = st.bytes(), self.weights.heads
         batch, total = meta.batch(), meta.total_rows()
         _check_rows(h, total, self.p, self.b_off, self.a, self.g, self.out)

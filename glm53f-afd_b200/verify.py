@@ -84,6 +84,8 @@ class KdaVerify:
         self.meta = K.BatchMeta.new(max_requests)
         self.pending: Optional[list[_Req]] = None
         self._st = K.StateType.Bf16 if l.kda_state_bf16 else K.StateType.F32
+        self._meta_on = None  # the stream the rounds' metadata and launches are ordered on (-1: several)
+        self._views = [None] * l.kda_layers  # per layer, made on first use: (arenas seen, state and conv buffers, p rows, saves)
 
     # ---- verify -----------------------------------------------------------------------------------------------
     def verify(self, windows: Sequence[tuple[marks.GlmKv, int]]) -> None:
@@ -97,27 +99,44 @@ class KdaVerify:
             raise Invalid(f"{sum(rows)} verify rows exceed the scratch of {self.v.rows}")
         if any(kv.pool is not self.pool for kv, _ in windows):
             raise Invalid("a slot of another pool")
-        self.meta.set([K.Request(r, kv.conv_elem_offset(), kv.state_elem_offset()) for kv, r in windows])
+        self._set_meta([K.Request(r, kv.conv_elem_offset(), kv.state_elem_offset()) for kv, r in windows], None, self.pool.stream)
         self.pending = [_Req(kv.slot, kv.tokens(), r) for kv, r in windows]
         for kv, r in windows:
             kv.pending = r
 
+    def _set_meta(self, requests, keep, stream: K.Stream) -> None:
+        """The batch metadata in the order of `stream`: the host runs on while earlier launches are still queued."""
+        self._order(stream)
+        self.meta.set_on(requests, keep, stream)
+        self._meta_on = K.raw_stream(stream) if self.pool.state.t.is_cuda else None
+
+    def _order(self, stream: K.Stream) -> None:
+        """Before work on `stream`: when the round so far is on another stream, wait for it (from then on before every call
+        of the round, since its launches are on several streams)."""
+        if self._meta_on is not None and K.raw_stream(stream) != self._meta_on:
+            K._torch().cuda.synchronize()
+            self._meta_on = -1
+
     def _layer_views(self, j: int):
-        l = self.pool.cfg.layout
-        sn, cn = l.state_elems_per_layer() * l.kda_state_elem_bytes(), l.conv_elems_per_layer() * 2
-        return K.DeviceBuffer(self.pool.state.t[j * sn:]), K.DeviceBuffer(self.pool.conv.t[j * cn:])
+        seen, v = (self.pool.state.t, self.pool.conv.t), self._views[j]
+        if v is None or v[0][0] is not seen[0] or v[0][1] is not seen[1]:
+            l = self.pool.cfg.layout
+            sn, cn = l.state_elems_per_layer() * l.kda_state_elem_bytes(), l.conv_elems_per_layer() * 2
+            v = self._views[j] = (seen, K.DeviceBuffer(seen[0][j * sn:]), K.DeviceBuffer(seen[1][j * cn:]), self.v.p_rows(j),
+                                  None if self.v.recompute else self.v.layer_saves(j))
+        return v[1:]
 
     def layer(self, j: int, a: K.RowView, g: K.RowView, out: K.RowView, stream: Optional[K.Stream] = None) -> None:
         """KDA layer j of the open round: the chain over the windows' rows in `scratch.p_rows(j)`, states read but not
         written, replay inputs saved (forward.rs:3484-3560 in Mode::Verify)."""
         if self.pending is None:
             raise Invalid("no verify is open")
-        state, conv = self._layer_views(j)
+        state, conv, p_rows, saves = self._layer_views(j)
         if self.v.recompute and not (a.buf is self.v.a and a.offset == self.v.a_rows(j).offset):
             raise Invalid("recompute mode: layer j's decay-gate rows live in scratch.a_rows(j)")
-        cb = K.ChainBatch(self.weights[j], self.v.p_rows(j), KDA_QKV, a, g, conv, state, K.StateOut.Skip, out,
-                          None if self.v.recompute else self.v.layer_saves(j))
+        cb = K.ChainBatch(self.weights[j], p_rows, KDA_QKV, a, g, conv, state, K.StateOut.Skip, out, saves)
         stream = stream or self.pool.stream
+        self._order(stream)
         if self._st is K.StateType.Bf16:
             cb.launch_bf16_state(self.meta, stream)
         else:
@@ -138,7 +157,7 @@ class KdaVerify:
                 raise Invalid(f"commit of {k} rows does not match the pending verify of slot {kv.slot}")
         l = self.pool.cfg.layout
         stream = stream or self.pool.stream
-        self.meta.set(self.meta.requests(), list(keep))
+        self._set_meta(self.meta.requests(), list(keep), stream)
         # The arenas are slot-major ([slot][layer]...): layer strides of one layer's elements, request offsets of whole
         # slots.  The checked wrappers of kernel.py assume layer-major arenas, so, like the reference's forward, this goes
         # to the entry points directly (forward.rs:1972-2031).
@@ -148,8 +167,8 @@ class KdaVerify:
             # No saves: every layer's chain again over the kept rows, in place, from the rows the round kept.  The decay
             # rows stand in for the output-gate rows: the outputs go to a sink.
             for j, w in enumerate(self.weights):
-                state, conv = self._layer_views(j)
-                pr, ar = self.v.p_rows(j), self.v.a_rows(j)
+                state, conv, pr, _ = self._layer_views(j)
+                ar = self.v.a_rows(j)
                 K._launched(ffi.glm53f_kda_chain_commit_batch(
                     KDA_HEADS, m.batch(), m.cu_rows.ptr(), m.keep_d.ptr(), pr.ptr(), pr.stride, KDA_QKV, ar.ptr(), ar.stride, ar.ptr(), ar.stride,
                     conv.ptr(), m.conv_off.ptr(), w.conv_w.ptr(), state.ptr(), m.state_off.ptr(), 1 if self._st is K.StateType.Bf16 else 0,

@@ -69,6 +69,17 @@ int32_t glm53f_kda_mark_copy_slots(uint8_t* pages, int64_t page_bytes, const int
                                    const int64_t part_bytes[3], const int64_t slot_stride[3], const int32_t* slots,
                                    int32_t marks, int32_t save, glm53f_stream_t stream);
 
+/* glm53f_kda_mark_copy with the page list on the host (an addition): `page_list` holds the mark's n_pages entries (at most
+ * 900; they travel in the kernel's parameters) and is read during the call, so no list has to be copied to the device
+ * first.  n_pages is the sum over p of ceil(part_bytes[p] / page_bytes); another count or a longer list is rejected
+ * with 1. */
+int32_t glm53f_kda_mark_copy_list(uint8_t* pages, int64_t page_bytes, const int32_t* page_list, int32_t n_pages,
+                                  uint8_t* const part[3], const int64_t part_bytes[3], int32_t save, glm53f_stream_t stream);
+
+/* `words` 32-bit words of host memory, read during the call, stored at dst in stream order (an addition; batch
+ * metadata): no staging buffer, no wait, capturable in a graph.  dst is 4-byte aligned. */
+int32_t glm53f_kda_store_words(uint32_t* dst, const uint32_t* host, int32_t words, glm53f_stream_t stream);
+
 #ifdef __cplusplus
 }
 #endif
