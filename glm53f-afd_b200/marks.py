@@ -37,6 +37,7 @@ TAIL = 1_552               # one DSA layer's tail record: 16 + 3 x 512 (cache.rs
 KDA_HEADS, KDA_DIM = 64, 128
 KDA_QKV = 3 * KDA_HEADS * KDA_DIM  # 24,576 (crates/glm53f-forward/src/shape.rs:23-32)
 KDA_WINDOW = 3
+INLINE_PAGES = 900  # a page list up to this length travels in the copy kernel's parameters (include/glm53f_fwd_rows.h)
 
 
 class OutOfMemory(RuntimeError):
@@ -109,28 +110,35 @@ class KvLayout:
 
 
 class PageAlloc:
-    """Reference counts and the free list of a pool of physical pages (kvplan.rs:150-204)."""
+    """Reference counts and the free list of a pool of physical pages (kvplan.rs:150-204).  Both are arrays: a mark takes
+    and gives back hundreds of pages at a time, which page by page was a third of the host time of a mark."""
 
     def __init__(self, pages: int):
-        self._free = list(range(pages - 1, -1, -1))  # popped from the end: the lowest page first
-        self._refs = [0] * pages
+        self._stack = np.arange(pages - 1, -1, -1, dtype=np.int32)  # free pages, taken from the end: the lowest page first
+        self._free = pages
+        self._refs = np.zeros(pages, np.int32)
 
     def total(self) -> int:
         return len(self._refs)
 
     def free(self) -> int:
-        return len(self._free)
+        return self._free
 
     def refs(self, page: int) -> int:
-        return self._refs[page]
+        return int(self._refs[page])
 
     def alloc(self) -> Optional[int]:
         if not self._free:
             return None
-        p = self._free.pop()
-        assert self._refs[p] == 0
-        self._refs[p] = 1
-        return p
+        return int(self.alloc_many(1)[0])
+
+    def alloc_many(self, n: int) -> np.ndarray:
+        """`n` calls of `alloc`, the caller having checked `free()`: the pages, lowest first."""
+        self._free -= n
+        pages = np.sort(self._stack[self._free:self._free + n])
+        assert not self._refs[pages].any()
+        self._refs[pages] = 1
+        return pages
 
     def share(self, page: int) -> None:
         assert self._refs[page] > 0, "sharing a free page"
@@ -140,9 +148,19 @@ class PageAlloc:
         assert self._refs[page] > 0, "releasing a free page"
         self._refs[page] -= 1
         if self._refs[page] == 0:
-            self._free.append(page)
+            self._stack[self._free] = page
+            self._free += 1
             return True
         return False
+
+    def release_many(self, pages: np.ndarray) -> None:
+        """`release` of each of several distinct pages in turn."""
+        left = self._refs[pages] - 1
+        assert (left >= 0).all(), "releasing a free page"
+        self._refs[pages] = left
+        gone = pages[left == 0]
+        self._stack[self._free:self._free + len(gone)] = gone
+        self._free += len(gone)
 
 
 @dataclass(frozen=True)
@@ -177,6 +195,8 @@ class KvPool:
         self.conv = DeviceBuffer.zeroed(cfg.max_slots * l.conv_bytes())
         self.tails = DeviceBuffer.zeroed(cfg.max_slots * max(l.tails_bytes(), 16))
         self.mark_index = DeviceBuffer.alloc(max(l.mark_pages(), 1) * 4)
+        self.mark_pages = l.mark_pages()
+        self.mark_sizes = (C.c_int64 * 3)(*[n for _, n, _ in l.mark_regions()])
         self.alloc = PageAlloc(cfg.pages)
         self._free_slots = list(range(cfg.max_slots - 1, -1, -1))
 
@@ -201,7 +221,7 @@ class KvPool:
         if len({kv.slot for kv in kvs}) != len(kvs):
             raise Invalid("the same slot twice in one batch")
         n = len(kvs)
-        lists = torch.tensor([m._pages for m in marks_], dtype=torch.int32).reshape(-1).to(self.pages.t.device)
+        lists = torch.from_numpy(np.concatenate([m._pages for m in marks_])).to(self.pages.t.device)
         slots = torch.tensor([kv.slot for kv in kvs], dtype=torch.int32).to(self.pages.t.device)
         arenas = (C.c_void_p * 3)(self.state.as_ptr(), self.conv.as_ptr(), self.tails.as_ptr())
         sizes = (C.c_int64 * 3)(*[r[1] for r in l.mark_regions()])
@@ -218,7 +238,7 @@ class KvPool:
         need = self.cfg.layout.mark_pages()
         if self.alloc.free() < need * len(kvs):
             raise OutOfMemory(f"{len(kvs)} snapshot marks take {need * len(kvs)} pages of the KV pool, {self.alloc.free()} are free")
-        out = [KvMark(kv.tokens(), sorted(self.alloc.alloc() for _ in range(need)), self) for kv in kvs]
+        out = [KvMark(kv.tokens(), self.alloc.alloc_many(need), self) for kv in kvs]
         if kvs:
             self._copy_marks(kvs, out, True)
         return out
@@ -249,7 +269,7 @@ class KvMark:
     """A slot's positional state at `tokens`, held in pages of the pool (kv.rs:207-236).  `drop()` (or garbage
     collection) gives the pages back."""
 
-    def __init__(self, tokens: int, pages: list[int], pool: KvPool):
+    def __init__(self, tokens: int, pages: np.ndarray, pool: KvPool):
         self.tokens = tokens
         self._pages = pages
         self._pool = pool
@@ -261,12 +281,12 @@ class KvMark:
         return len(self._pages)
 
     def page_list(self) -> list[int]:
-        return list(self._pages)
+        return self._pages.tolist()
 
     def drop(self) -> None:
-        for p in self._pages:
-            self._pool.alloc.release(p)
-        self._pages = []
+        pages, self._pages = self._pages, self._pages[:0]
+        if len(pages):
+            self._pool.alloc.release_many(pages)
 
     def __del__(self):
         try:
@@ -283,6 +303,7 @@ class GlmKv:
         self.slot = slot
         self._tokens = 0
         self.pending = 0  # rows of an uncommitted verify window
+        self._at = (self._state_at(), self._conv_at(), self._tails_at())
 
     def layout(self) -> KvLayout:
         return self.pool.cfg.layout
@@ -341,7 +362,7 @@ class GlmKv:
 
     def _arenas(self):
         p = self.pool
-        return [(p.state, self._state_at()), (p.conv, self._conv_at()), (p.tails, self._tails_at())]
+        return [(p.state, self._at[0]), (p.conv, self._at[1]), (p.tails, self._at[2])]
 
     # ---- the copy ---------------------------------------------------------------------------------------------
     def _copy_mark(self, mark: KvMark, save: bool) -> None:
@@ -352,8 +373,12 @@ class GlmKv:
         l, p = self.layout(), self.pool
         pb = l.page_bytes
         n_idx = len(mark._pages)
+        if p.fused and n_idx <= INLINE_PAGES and p.pages.t.is_cuda:
+            parts = (C.c_void_p * 3)(*[a.as_ptr() + at for a, at in self._arenas()])
+            return _launched(ffi.load().glm53f_kda_mark_copy_list(p.pages.as_ptr(), pb, mark._pages.ctypes.data, n_idx, parts, p.mark_sizes, 1 if save else 0, p.stream.raw()),
+                             "mark pages")
         # The list buffer is reused in stream order.
-        p.mark_index.t[:n_idx * 4].view(torch.int32).copy_(torch.tensor(mark._pages, dtype=torch.int32))
+        p.mark_index.t[:n_idx * 4].view(torch.int32).copy_(torch.from_numpy(mark._pages))
         lib = ffi.load()
         s = p.stream.raw()
         if p.fused:
@@ -372,7 +397,7 @@ class GlmKv:
                     rc = lib.glm53f_fwd_gather_rows(p.pages.as_ptr(), pb, idx, arena.as_ptr() + at, pb, full, pb, s)
                 _launched(rc, "mark pages")
             if rem > 0:
-                page = mark._pages[first + full] * pb
+                page = int(mark._pages[first + full]) * pb
                 if save:
                     p.pages.t[page:page + rem].copy_(arena.t[at + full * pb:at + full * pb + rem])
                 else:
@@ -385,12 +410,11 @@ class GlmKv:
         few free pages (nothing is allocated then), kv.rs:482-509."""
         if self.pending != 0:
             raise Invalid("mark inside an uncommitted verify window")
-        need = self.layout().mark_pages()
+        need = self.pool.mark_pages
         a = self.pool.alloc
         if a.free() < need:
             raise OutOfMemory(f"a snapshot mark takes {need} pages of the KV pool, {a.free()} are free")
-        pages = sorted(a.alloc() for _ in range(need))
-        mark = KvMark(self._tokens, pages, self.pool)
+        mark = KvMark(self._tokens, a.alloc_many(need), self.pool)
         self._copy_mark(mark, True)
         return mark
 
@@ -408,7 +432,12 @@ class GlmKv:
             raise Invalid("fork across pools")
         if mark.tokens != to or to > src._tokens:
             raise Invalid(f"fork of {to} tokens with a mark at {mark.tokens} from a slot of {src._tokens}")
-        self.reset()
+        if mark._pool is not self.pool:
+            self.reset()
+            raise Invalid("a mark of another pool")
+        # The slot's state is not cleared first: the copy covers every byte of it.
+        self._tokens = 0
+        self.pending = 0
         self._copy_mark(mark, False)
         self._tokens = to
 
@@ -430,7 +459,7 @@ class GlmKv:
                 while k + run < pages and mark._pages[first + k + run] == mark._pages[first + k] + run:
                     run += 1
                 nbytes = min(n - k * pb, run * pb)
-                at = mark._pages[first + k] * pb
+                at = int(mark._pages[first + k]) * pb
                 dst[off + k * pb:off + k * pb + nbytes] = p.pages.t[at:at + nbytes].cpu().numpy()
                 k += run
             first += pages

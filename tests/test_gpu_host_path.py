@@ -1,0 +1,63 @@
+"""The native host path and what it uploads by: words carried in kernel parameters at the edges of a launch's capacity,
+page lists in parameters against page lists on the device, and the launches it must leave to the Python checks."""
+import ctypes as C
+import importlib
+
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [0, 1, 255, 257, 999, 1000, 1001, 2500])
+def test_store_words(pkg, n):
+    lib = pkg.ffi.load()
+    host = np.random.default_rng(n).integers(0, 1 << 32, max(n, 1), dtype=np.uint32)
+    dst = torch.zeros(n + 4, dtype=torch.int32, device="cuda")
+    assert lib.glm53f_kda_store_words(dst.data_ptr(), host.ctypes.data, n, torch.cuda.current_stream().cuda_stream) == 0
+    got = dst.cpu().numpy().view(np.uint32)
+    assert (got[:n] == host[:n]).all() and not got[n:].any()
+
+
+@pytest.mark.parametrize("n_pages", [1, 899, 900])
+@pytest.mark.parametrize("save", [1, 0])
+def test_mark_copy_with_the_page_list_in_the_parameters(pkg, n_pages, save):
+    lib = pkg.ffi.load()
+    pb, rng = 1024, np.random.default_rng(n_pages)
+    pages = np.sort(rng.permutation(n_pages + 5)[:n_pages]).astype(np.int32)
+    size = n_pages * pb - 16 * (n_pages > 1)  # a last page that is not full
+    stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    sizes = (C.c_int64 * 3)(size, 0, 0)
+    both = []
+    for inline in (False, True):
+        g = torch.Generator(device="cuda").manual_seed(3)
+        pool = torch.randint(0, 256, ((n_pages + 5) * pb,), dtype=torch.uint8, device="cuda", generator=g)
+        part = torch.randint(0, 256, (size,), dtype=torch.uint8, device="cuda", generator=g)
+        parts = (C.c_void_p * 3)(part.data_ptr(), None, None)
+        if inline:
+            assert lib.glm53f_kda_mark_copy_list(pool.data_ptr(), pb, pages.ctypes.data, n_pages, parts, sizes, save, stream) == 0
+        else:
+            d = torch.from_numpy(pages).cuda()
+            assert lib.glm53f_kda_mark_copy(pool.data_ptr(), pb, d.data_ptr(), parts, sizes, save, stream) == 0
+        both.append((pool.cpu(), part.cpu()))
+    assert torch.equal(both[0][0], both[1][0]) and torch.equal(both[0][1], both[1][1])
+    # a list of another length, or one too long for the parameters, is rejected before anything runs
+    assert lib.glm53f_kda_mark_copy_list(pool.data_ptr(), pb, pages.ctypes.data, n_pages - 1, parts, sizes, save, stream) == 1
+    assert lib.glm53f_kda_mark_copy_list(pool.data_ptr(), pb, pages.ctypes.data, 901, parts, sizes, save, stream) == 1
+
+
+def test_calls_with_an_error_keep_their_errors(pkg):
+    core, h = importlib.import_module("glm53f-afd_b200.core"), 2
+    z = lambda n, d: torch.zeros(n, dtype=d, device="cuda")
+    cu, off = torch.tensor([0, 1], dtype=torch.int32, device="cuda"), z(1, torch.int64)
+    ok = dict(heads=h, rows=1, cu_rows=cu, q=z(h * 128, torch.bfloat16), k=z(h * 128, torch.bfloat16), v=z(h * 128, torch.bfloat16),
+              g=z(h * 128, torch.float32), beta=z(h, torch.float32), state=z(h * 128 * 128, torch.float32), state_off=off,
+              out=z(h * 128, torch.bfloat16))
+    core.decode_batch(**ok)
+    for bad, text in ((dict(q=z(h * 128 - 1, torch.bfloat16)), "q holds"), (dict(g=z(h * 128, torch.float64)), "g has dtype"), (dict(out=None), "rejected"),
+                      (dict(v=z(h * 128, torch.bfloat16).cpu()), "v must be"), (dict(flags=64), "rejected"), (dict(max_state_off=1), "exceeds")):
+        with pytest.raises(core.Invalid, match=text):
+            core.decode_batch(**{**ok, **bad})
+    torch.cuda.synchronize()
+    assert core.device_status() == 0
