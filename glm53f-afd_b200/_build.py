@@ -15,6 +15,7 @@ HOST = os.path.join(HERE, "_host.so")  # a Python module: the native host path o
 IEEE = ["--fmad=false", "--ftz=false", "--prec-div=true", "--prec-sqrt=true"]
 SOURCES = {
     "kda_chain.cu": IEEE,
+    "kda_rows.cu": IEEE,
     "kda_conv.cu": IEEE,
     "kda_prefill.cu": IEEE,
     "kda_verify_tc.cu": IEEE,  # the chunked verify: its replay saves must carry the exact path's bits (the same expf)

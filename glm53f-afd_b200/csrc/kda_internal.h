@@ -23,6 +23,34 @@ int core_chain_launch(int32_t heads, int32_t batch, const int32_t* cu_rows, cons
                       const int64_t* state_off, bool bf16_state, int32_t flags, const glm53f_bf16* gate,
                       const glm53f_bf16* norm_w, float eps, glm53f_bf16* out, cudaStream_t stream);
 
+// The exact recurrence over a pass of cooked rows (kda_rows.cu): rows row_shift .. row_shift + pass_rows - 1 of every request,
+// request b's at rows b * pass_rows of q, k, g (the decay multiplier), v and beta.  rows_launch leaves bf16(y) in `out`
+// (rows of the whole call, out_stride apart); rows_norm_launch normalises every row of `out` (max_rows >= the longest
+// request's).  cu == nullptr: one request of rows1 rows.  out, gate and norm_w are 8-byte aligned, strides multiples of 4.
+struct RowsParams {
+    int H, rows1, pass_rows, row_shift, max_rows;
+    const int32_t* cu;
+    const float *q, *k, *g, *beta;
+    const uint16_t* v;
+    const void* state_in;
+    void* state_out;
+    const long long* state_off;
+    uint16_t* out;
+    long long out_stride;
+    const uint16_t* gate;
+    long long gate_stride;
+    const uint16_t* norm_w;
+    float eps;
+    unsigned long long neg_zero2;  // set by rows_launch
+};
+int rows_launch(RowsParams p, int batch, bool bf16_state, cudaStream_t stream);
+int rows_norm_launch(const RowsParams& p, int batch, cudaStream_t stream);
+// Its prologue (kda_prologue.cu): the chain's q, k, decay multiplier, v and beta, bit for bit.
+int exact_prologue_launch(int32_t heads, int32_t batch, const int32_t* cu_rows, int32_t rows1, int32_t pass_rows, int32_t row_shift,
+                          const glm53f_bf16* p, int64_t p_stride, int64_t b_off, const glm53f_bf16* a, int64_t a_stride,
+                          const glm53f_bf16* conv, const int64_t* conv_off, const glm53f_bf16* conv_w, const float* a_log,
+                          const float* dt_bias, float lower, float* q, float* k, float* g, glm53f_bf16* v, float* beta, cudaStream_t stream);
+
 // Window past `keep` rows for every (layer, request): keep from keep[b], else keep1 if >= 0, else the request's
 // whole row count (the prefill's advance).
 int conv_shift_launch(int32_t channels, int32_t layers, int32_t batch, const int32_t* cu_rows, const int32_t* keep,

@@ -6,7 +6,9 @@
 //
 // The layer entry points have two forms, chosen by glm53f_kda_prefill_mode (the reference gates its own chunked kernel
 // the same way, crates/glm53f-forward/src/forward.rs:210,3580):
-//   exact (default)   the row-by-row recurrence of kda_chain.cu: the chain's results bit for bit;
+//   exact (default)   the row-by-row recurrence, the chain's results bit for bit: passes of (layer prologue -> recurrence of
+//                     kda_rows.cu) over the caller's workspace and one launch of the output norm; short or unaligned calls
+//                     run the chain of kda_chain.cu itself;
 //   chunked           passes of (layer prologue -> chunk-64 tcgen05 kernel of kda_prefill_tc.cu with the gated norm
 //                     fused) over the caller's workspace, which holds one pass's core inputs; agrees with the chain
 //                     to the rounding of bf16 operands, like every chunked form.  The kernels cover the whole gate
@@ -91,6 +93,52 @@ int chunked_layer_prefill(int32_t heads, int32_t batch, const int32_t* cu_rows, 
     return 0;
 }
 
+// The exact form for prompt segments: passes of (prologue, recurrence) over the caller's workspace, then the output norm
+// over all rows (kda_rows.cu).  kNotEligible when rows are not aligned for vector access, when the workspace holds fewer than
+// 16 rows a pass (the reference's formula gives 16 x 2,176 bytes per head for 16 rows; a row and head takes 1,796), or for a
+// handful of rows, where one launch of the chain (1.5 us a row) ends before three launches have.
+constexpr int64_t kExactBytesPerRowHead = 3 * DK * 4 + DK * 2 + 4;
+constexpr int kExactMinRows = 8;
+int exact_layer_prefill(int32_t heads, int32_t batch, const int32_t* cu_rows, int32_t max_rows, const glm53f_bf16* p,
+                        int64_t p_stride, int64_t b_off, const glm53f_bf16* a, int64_t a_stride, const glm53f_bf16* g,
+                        int64_t g_stride, const glm53f_bf16* conv, const int64_t* conv_off, const glm53f_bf16* conv_w,
+                        const void* state_in, void* state_out, const int64_t* state_off, bool bf16_state, const float* a_log,
+                        const float* dt_bias, const glm53f_bf16* norm_w, float eps, float lower, glm53f_bf16* out,
+                        int64_t out_stride, float* workspace, int64_t workspace_bytes, cudaStream_t st) {
+    auto al = [](const void* x, int n) { return (reinterpret_cast<uintptr_t>(x) & (uintptr_t)(n - 1)) == 0; };
+    if (max_rows < kExactMinRows || !al(out, 8) || !al(g, 8) || !al(norm_w, 8) || !al(workspace, 16) || !al(p, 8) || !al(a, 8) || !al(conv, 8) ||
+        !al(conv_w, 16) || !al(dt_bias, 16) || p_stride % 4 || a_stride % 4 || g_stride % 4 || out_stride % 4)
+        return kNotEligible;
+    int64_t pass = workspace_bytes / ((int64_t)batch * heads * kExactBytesPerRowHead) / 16 * 16;
+    const int64_t need = ((int64_t)max_rows + 15) / 16 * 16;
+    if (pass > need) pass = need;
+    if (pass < 16 || (int64_t)batch * pass > 0x7fffffffll || (int64_t)batch * heads * (need / 4) > 0x7fffffffll) return kNotEligible;
+    const int64_t passes = (need + pass - 1) / pass;
+    pass = (need + 16 * passes - 1) / (16 * passes) * 16;  // of equal length
+    const int64_t cap = (int64_t)batch * pass * heads * DK;
+    float* q = workspace;
+    float *k = q + cap, *dec = k + cap;
+    glm53f_bf16* v = reinterpret_cast<glm53f_bf16*>(dec + cap);
+    float* beta = reinterpret_cast<float*>(v + cap);
+    RowsParams x{};
+    x.H = heads; x.rows1 = max_rows; x.pass_rows = (int)pass; x.max_rows = max_rows;
+    x.cu = cu_rows;
+    x.q = q; x.k = k; x.g = dec; x.v = v; x.beta = beta;
+    x.state_out = state_out; x.state_off = reinterpret_cast<const long long*>(state_off);
+    x.out = out; x.out_stride = out_stride;
+    x.gate = g; x.gate_stride = g_stride; x.norm_w = norm_w; x.eps = eps;
+    for (int64_t shift = 0; shift < max_rows; shift += pass) {
+        int rc = exact_prologue_launch(heads, batch, cu_rows, max_rows, (int)pass, (int)shift, p, p_stride, b_off, a, a_stride, conv, conv_off, conv_w,
+                                       a_log, dt_bias, lower, q, k, dec, v, beta, st);
+        if (rc != 0) return rc;
+        x.row_shift = (int)shift;
+        x.state_in = shift == 0 ? state_in : state_out;
+        rc = rows_launch(x, batch, bf16_state, st);
+        if (rc != 0) return rc;
+    }
+    return rows_norm_launch(x, batch, st);
+}
+
 // Reference kda_prefill.cu:638-657.
 int prefill_entry(int32_t heads, int32_t batch, bool batched, const int32_t* cu_rows, int32_t rows, int32_t max_rows,
                   const glm53f_bf16* p, int64_t p_stride, int64_t b_off, const glm53f_bf16* a, int64_t a_stride,
@@ -116,7 +164,11 @@ int prefill_entry(int32_t heads, int32_t batch, bool batched, const int32_t* cu_
             return conv_shift_launch(3 * heads * DK, 1, batch, cu_rows, nullptr, -1, rows, conv, 0, conv_off, p, 0, p_stride, st);
         }
     }
-    int rc = layer_chain_launch(heads, batch, cu_rows, rows, p, p_stride, b_off, a, a_stride, g, g_stride, conv, conv_off, conv_w,
+    int rc = exact_layer_prefill(heads, batch, cu_rows, batched ? max_rows : rows, p, p_stride, b_off, a, a_stride, g, g_stride, conv, conv_off, conv_w,
+                                 state_in, state_out, state_off, bf16_state, a_log, dt_bias, norm_w, eps, lower, out, out_stride, workspace,
+                                 workspace_bytes, st);
+    if (rc == kNotEligible)
+        rc = layer_chain_launch(heads, batch, cu_rows, rows, p, p_stride, b_off, a, a_stride, g, g_stride, conv, conv_off, conv_w,
                                 state_in, state_out, state_off, bf16_state, a_log, dt_bias, norm_w, eps, lower, out, out_stride, st);
     if (rc != 0) return rc;
     // The window past the segment (reference kda_prefill.cu:687-690); stream order puts it after the chain's reads.

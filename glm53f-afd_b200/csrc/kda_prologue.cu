@@ -1,4 +1,4 @@
-// The layer prologue of the chunked forms: projection rows to the core's inputs.
+// The layer prologue of the chunked forms and of the exact prefill: projection rows to the core's inputs.
 //
 // The layer entry points take the engine's rows (q | k | v projections, beta logits, the forget-gate row); the chunked
 // tensor-core kernels take what the recurrence is defined on: q and k after the short convolution, SiLU and the L2
@@ -16,7 +16,7 @@
 // allow 24 resident warps per SM.  (A warp that walks 16 rows with the three earlier rows sliding in registers needs
 // 143 registers and was half as fast.)
 //
-// Two sinks:
+// Three sinks:
 //  * a prefill pass: dense core inputs for one pass of rows in the caller's workspace.  q and k are rounded to fp16
 //    (they lie in [-1, 1]; eleven mantissa bits), the one place where the chunked prefill departs from the chain's
 //    FP32 q and k before the tensor-core products: with bf16's eight bits the rounding of k alone, which reaches the
@@ -26,6 +26,8 @@
 //    multiplier exp(log decay) and beta go to the replay saves, which a verify call must write anyway and which hold
 //    exactly these values (the bits the exact form saves), and q goes, as fp16, to the 256 bytes of `out` that the
 //    same (row, head) output will overwrite.  Windows of up to 16 rows.
+//  * a pass of the exact prefill (kda_rows.cu): as the verify sink, q in f32 with the chain's arithmetic too, all of it in
+//    the caller's workspace.
 
 #include <cuda_fp16.h>
 
@@ -59,7 +61,10 @@ struct ProParams {
     long long out_stride;
     float *k_save, *g_save, *b_save;
     uint16_t* v_save;
+    float* qf;  // exact sink: q in f32 (k, decay multiplier, v and beta through the saves' pointers)
+    int rows1;  // cu == nullptr: one request of rows1 rows
 };
+enum Sink : int { kFast = 0, kVerify = 1, kExact = 2 };
 
 // The verify sink keeps the chain's IEEE arithmetic (its results are the replay saves, bit for bit); the prefill sink
 // feeds tensor-core products that round every operand to bf16 anyway, so there the divisions, exponentials and
@@ -99,8 +104,13 @@ __device__ __forceinline__ uint2 pack4(const float (&x)[4]) {
                       (uint32_t)f32_to_bf16_bits(x[2]) | ((uint32_t)f32_to_bf16_bits(x[3]) << 16));
 }
 
-template <bool VERIFY>
+template <int SINK>
 __global__ void __launch_bounds__(128, 6) layer_prologue_kernel(const ProParams p) {
+    constexpr bool VERIFY = SINK == kVerify, EXACT = SINK == kExact, FAST = SINK == kFast;
+    if constexpr (EXACT) {
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+    }
     const int lane = threadIdx.x & 31, H = p.H;
     // a block = four consecutive rows of one (request, head): neighbours share their predecessors in L1
     const int quads = p.pass_rows / 4;
@@ -110,11 +120,11 @@ __global__ void __launch_bounds__(128, 6) layer_prologue_kernel(const ProParams 
     // A prefill pass covers pass_rows rows of every request.  A verify window is meant to have at most 16 rows; should one be
     // longer (the chunk kernel then reports status 122 and leaves the rows past 16 without outputs), its replay saves are
     // still written for EVERY row, so that a commit of any prefix replays real values: the warp goes on in steps of 16.
-    const int r0 = p.cu[b], n_all = max(p.cu[b + 1] - r0 - p.row_shift, 0), n = VERIFY ? n_all : min(n_all, p.pass_rows);
+    const int r0 = p.cu ? p.cu[b] : 0, n_all = max((p.cu ? p.cu[b + 1] - r0 : p.rows1) - p.row_shift, 0), n = VERIFY ? n_all : min(n_all, p.pass_rows);
     for (int j = j_first; j < n; j += p.pass_rows) {
     const int c0 = lane * 4, jj = p.row_shift + j;  // row of the request
     const long long C = 3LL * H * DK, gr = (long long)r0 + jj;
-    const uint16_t* window = p.conv + p.conv_off[b];
+    const uint16_t* window = p.conv + (p.conv_off ? p.conv_off[b] : 0);
     uint2 x[TAPS][3];  // [tap: rows jj-3 .. jj][part]; rows before the request's first come from the conv window
 #pragma unroll
     for (int d = 0; d < TAPS; ++d) {
@@ -149,8 +159,8 @@ __global__ void __launch_bounds__(128, 6) layer_prologue_kernel(const ProParams 
             acc = acc + __uint_as_float(ww[2 * c] & 0xffff0000u) * xv[1][c];
             acc = acc + __uint_as_float(ww[2 * c + 1] << 16) * xv[2][c];
             acc = acc + __uint_as_float(ww[2 * c + 1] & 0xffff0000u) * xv[3][c];
-            // q reaches only the outputs, which carry bf16-operand rounding in both chunked forms: always the fast form
-            act[part][c] = bf16_round(part == 0 ? silu_<true>(acc) : silu_<!VERIFY>(acc));
+            // q reaches only the outputs, which carry bf16-operand rounding in both chunked forms: the fast form there
+            act[part][c] = bf16_round(part == 0 ? silu_<!EXACT>(acc) : silu_<FAST>(acc));
         }
     }
     // L2 norms of q and k (eps 1e-6 inside the root), q also times 128^-0.5.
@@ -164,7 +174,7 @@ __global__ void __launch_bounds__(128, 6) layer_prologue_kernel(const ProParams 
         }
         sq = butterfly(sq);
         sk = butterfly(sk);
-        const float iq = inv_norm_<true>(sq), ik = inv_norm_<!VERIFY>(sk);
+        const float iq = inv_norm_<!EXACT>(sq), ik = inv_norm_<FAST>(sk);
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
             qn[c] = (act[0][c] * iq) * (1.0f / sqrtf((float)DK));
@@ -175,8 +185,8 @@ __global__ void __launch_bounds__(128, 6) layer_prologue_kernel(const ProParams 
     unpack4(a_bits, a4);
     const float dtb[4] = {dtb4.x, dtb4.y, dtb4.z, dtb4.w};
 #pragma unroll
-    for (int c = 0; c < 4; ++c) lg[c] = p.lower * sigmoid_<!VERIFY>(decay_rate * (a4[c] + dtb[c]));
-    const float bt = bf16_round(sigmoid_<!VERIFY>(blogit));
+    for (int c = 0; c < 4; ++c) lg[c] = p.lower * sigmoid_<FAST>(decay_rate * (a4[c] + dtb[c]));
+    const float bt = bf16_round(sigmoid_<FAST>(blogit));
     if constexpr (VERIFY) {
         const long long sv = (gr * H + h) * DK + c0;
         if (j < p.pass_rows) *reinterpret_cast<uint2*>(p.q + gr * p.out_stride + (long long)h * DK + c0) = pack4_fp16(qn);  // rows past 16 get no output: leave theirs alone
@@ -184,6 +194,13 @@ __global__ void __launch_bounds__(128, 6) layer_prologue_kernel(const ProParams 
         *reinterpret_cast<uint2*>(p.v_save + sv) = pack4(act[2]);
         *reinterpret_cast<float4*>(p.g_save + sv) = make_float4(expf(lg[0]), expf(lg[1]), expf(lg[2]), expf(lg[3]));
         if (lane == 0) p.b_save[gr * H + h] = bt;
+    } else if constexpr (EXACT) {
+        const long long orow = (long long)b * p.pass_rows + j, at = (orow * H + h) * DK + c0;
+        *reinterpret_cast<float4*>(p.qf + at) = make_float4(qn[0], qn[1], qn[2], qn[3]);
+        *reinterpret_cast<float4*>(p.k_save + at) = make_float4(kn[0], kn[1], kn[2], kn[3]);
+        *reinterpret_cast<float4*>(p.g_save + at) = make_float4(expf(lg[0]), expf(lg[1]), expf(lg[2]), expf(lg[3]));
+        *reinterpret_cast<uint2*>(p.v_save + at) = pack4(act[2]);
+        if (lane == 0) p.b_save[orow * H + h] = bt;
     } else {
         const long long orow = (long long)b * p.pass_rows + j, at = (orow * H + h) * DK + c0;
         *reinterpret_cast<uint2*>(p.q + at) = pack4_fp16(qn);
@@ -195,12 +212,20 @@ __global__ void __launch_bounds__(128, 6) layer_prologue_kernel(const ProParams 
     }
 }
 
-template <bool VERIFY>
+template <int SINK>
 int launch(const ProParams& pp, cudaStream_t stream) {
     const long long blocks = (long long)pp.batch * pp.H * (pp.pass_rows / 4);
     if (blocks > 0x7fffffffLL) return kInvalid;
-    layer_prologue_kernel<VERIFY><<<(unsigned)blocks, 128, 0, stream>>>(pp);
-    return (int)cudaGetLastError();
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.blockDim = dim3(128);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = SINK == kExact ? 1 : 0;  // the exact sink's kernel waits for its predecessors itself
+    return (int)cudaLaunchKernelEx(&cfg, layer_prologue_kernel<SINK>, pp);
 }
 
 }  // namespace
@@ -219,7 +244,23 @@ int layer_prologue_launch(int32_t heads, int32_t batch, const int32_t* cu_rows, 
     pp.conv = conv; pp.conv_off = reinterpret_cast<const long long*>(conv_off); pp.cw = conv_w;
     pp.a_log = a_log; pp.dt_bias = dt_bias; pp.lower = lower;
     pp.q = q; pp.k = k; pp.v = v; pp.g = g; pp.beta = beta;
-    return launch<false>(pp, stream);
+    return launch<kFast>(pp, stream);
+}
+
+int exact_prologue_launch(int32_t heads, int32_t batch, const int32_t* cu_rows, int32_t rows1, int32_t pass_rows, int32_t row_shift,
+                          const glm53f_bf16* p, int64_t p_stride, int64_t b_off, const glm53f_bf16* a, int64_t a_stride,
+                          const glm53f_bf16* conv, const int64_t* conv_off, const glm53f_bf16* conv_w, const float* a_log,
+                          const float* dt_bias, float lower, float* q, float* k, float* g, glm53f_bf16* v, float* beta, cudaStream_t stream) {
+    if (pass_rows < 16 || pass_rows % 16 != 0) return kInvalid;
+    ProParams pp{};
+    pp.H = heads; pp.batch = batch; pp.pass_rows = pass_rows; pp.row_shift = row_shift;
+    pp.cu = cu_rows; pp.rows1 = rows1;
+    pp.P = p; pp.p_stride = p_stride; pp.b_off = b_off;
+    pp.A = a; pp.a_stride = a_stride;
+    pp.conv = conv; pp.conv_off = reinterpret_cast<const long long*>(conv_off); pp.cw = conv_w;
+    pp.a_log = a_log; pp.dt_bias = dt_bias; pp.lower = lower;
+    pp.qf = q; pp.k_save = k; pp.g_save = g; pp.v_save = v; pp.b_save = beta;
+    return launch<kExact>(pp, stream);
 }
 
 // The prologue of the chunked verify: windows of up to 16 rows per request; see the head of the file for where the
@@ -237,7 +278,7 @@ int verify_prologue_launch(int32_t heads, int32_t batch, const int32_t* cu_rows,
     pp.a_log = a_log; pp.dt_bias = dt_bias; pp.lower = lower;
     pp.q = out; pp.out_stride = out_stride;
     pp.k_save = k_save; pp.v_save = v_save; pp.g_save = g_save; pp.b_save = b_save;
-    return launch<true>(pp, stream);
+    return launch<kVerify>(pp, stream);
 }
 
 }  // namespace kda

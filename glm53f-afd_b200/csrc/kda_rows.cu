@@ -1,0 +1,193 @@
+// The exact recurrence over many rows of few requests (prompt segments of the layer prefill's exact form): the rows' inputs
+// are cooked beforehand, for a pass of rows at once, and the outputs are normalised afterwards, so that what is left serial
+// is the delta rule alone.
+//
+//   layer_prologue_kernel (kda_prologue.cu)   every row of a pass in parallel: q, k, the decay multiplier (f32), v (bf16), beta
+//   rows_kernel                               the state through the pass's rows; each row's read-out, rounded to bf16, in `out`
+//   rows_norm_kernel                          the gated RMSNorm over every row, in place in `out`
+//
+// The persistent pipeline (kda_chain.cu) cooks, steps and normalises row after row on one SM per (request, head): 1.55 us a
+// row, 64 of 148 SMs busy for one prompt.  Here, as in the commit replay, a WARP is the unit of work -- eight of a unit's
+// value rows never interact with the others --, reads what its lanes need of a cooked row straight into registers, rows
+// ahead, and meets no barrier; a unit's sixteen warps are four blocks, so a prompt of 64 heads puts work on every SM.
+//
+// What bounds it: a row is a chain of dependent steps (decayed state, k-product, five shuffles, update) with two warps a
+// scheduler for one prompt, the FP32 pipe (112 two-wide operations a row and warp) for four.  One prompt of 701 rows, f32
+// states: 1,087 -> 402 us (0.5 us a row); four prompts: 1,222 us.  Measured against it at 701 rows: three rows in flight 406,
+// five blocks an SM (96 registers, spills) 515, four value rows a warp 451, rows through shared memory by asynchronous copies 457.
+//
+// Same arithmetic in the same order with the same rounding points (a bf16 state is rounded after every row, the read-out
+// before the norm): the chain's bits.
+
+#include "common.cuh"
+#include "glm53f_kda.h"
+#include "kda_internal.h"
+#include "recurrence.cuh"
+
+namespace kda {
+namespace {
+
+constexpr int kRowsWarps = 4, kRowsThreads = kRowsWarps * 32, kParts = kRecWarps / kRowsWarps;
+constexpr int kPerSm = 4;    // blocks an SM holds: 128 registers a thread
+constexpr int kAhead = 2;    // rows in flight in registers, 14 each
+
+struct CookedRow {
+    float4 k, g, q;
+    uint16_t v;  // bf16 bits, widened when the row's turn comes: a conversion at the load would wait for it there and then
+    float beta;
+};
+
+template <typename S>
+__global__ void __launch_bounds__(kRowsThreads, kPerSm) rows_kernel(const __grid_constant__ RowsParams p) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const unsigned unit = blockIdx.x / kParts;
+    const int uw = (int)(blockIdx.x % kParts) * kRowsWarps + warp;  // this warp's place among the unit's 16
+    const int h = (int)(unit % (unsigned)p.H), b = (int)(unit / (unsigned)p.H);
+    const int r0 = p.cu ? p.cu[b] : 0, all = p.cu ? p.cu[b + 1] - r0 : p.rows1;
+    const int n = min(max(all - p.row_shift, 0), p.pass_rows);
+    if (n == 0 && p.state_in == p.state_out) return;
+    const long long s_elem = (p.state_off ? p.state_off[b] : 0) + (long long)h * DV * DK;
+    f32x2 s[kPairs][4];
+    load_rows_global<S>(reinterpret_cast<const S*>(p.state_in) + s_elem, uw, lane, s);
+    const long long first = (long long)b * p.pass_rows * p.H + h;      // (row, head) index of the pass's row 0
+    const int mine = uw * kRowsPerLane + ((lane >> 1) & 7);            // the value row whose sums this lane receives
+    auto fetch = [&](int r) {
+        const long long rh = first + (long long)r * p.H, at = rh * DK;
+        CookedRow x;
+        x.k = *reinterpret_cast<const float4*>(p.k + at + lane * 4);
+        x.g = *reinterpret_cast<const float4*>(p.g + at + lane * 4);
+        x.q = *reinterpret_cast<const float4*>(p.q + at + lane * 4);
+        x.v = p.v[at + mine];
+        x.beta = p.beta[rh];
+        return x;
+    };
+    // A row's read-out is reduced together with the next row's k-product: one chain of shuffles a row.  sums[0..7] are the
+    // k-product's partial sums, sums[8..15] the read-out's; lanes 0-15 then hold the k-products, lanes 16-31 the previous
+    // row's read-outs, two lanes to a value row.
+    float sums[2 * kRowsPerLane] = {};
+    uint16_t* out = p.out + ((long long)r0 + p.row_shift) * p.out_stride + (long long)h * DV + mine;
+    auto step = [&](const CookedRow& x, bool first_row) {
+        const f32x2 kk[4] = {pack2(x.k.x, x.k.x), pack2(x.k.y, x.k.y), pack2(x.k.z, x.k.z), pack2(x.k.w, x.k.w)};
+        const f32x2 gg[4] = {pack2(x.g.x, x.g.x), pack2(x.g.y, x.g.y), pack2(x.g.z, x.g.z), pack2(x.g.w, x.g.w)};
+        if constexpr (sizeof(S) == 2) {
+            if (!first_row) round_rows(s);  // after a row's read-out; the last row's rounding is the store's
+        }
+#pragma unroll
+        for (int jp = 0; jp < kPairs; ++jp)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) s[jp][i] = mul2(s[jp][i], gg[i], p.neg_zero2);
+        rows_partial(s, kk, sums, p.neg_zero2);
+        const float sum = butterfly_of<2 * kRowsPerLane>(sums, lane);
+        if (!first_row) {
+            if ((lane & 17) == 16) *out = f32_to_bf16_bits(sum);
+            out += p.out_stride;
+        }
+        const float d = (bf16_bits_to_f32(x.v) - sum) * x.beta;
+#pragma unroll
+        for (int jp = 0; jp < kPairs; ++jp) {
+            const f32x2 delta = pack2(__shfl_sync(FULL, d, 4 * jp), __shfl_sync(FULL, d, 4 * jp + 2));
+#pragma unroll
+            for (int i = 0; i < 4; ++i) s[jp][i] = add2(s[jp][i], mul2(kk[i], delta, p.neg_zero2));
+        }
+        const f32x2 qq[4] = {pack2(x.q.x, x.q.x), pack2(x.q.y, x.q.y), pack2(x.q.z, x.q.z), pack2(x.q.w, x.q.w)};
+        rows_partial(s, qq, sums + kRowsPerLane, p.neg_zero2);
+    };
+    if (n > 0) {
+        CookedRow ring[kAhead];  // row r waits in ring[r % kAhead]
+#pragma unroll
+        for (int j = 0; j < kAhead; ++j) ring[j] = fetch(min(j, n - 1));
+        int r = 0;
+        for (; r + kAhead <= n; r += kAhead)
+#pragma unroll
+            for (int j = 0; j < kAhead; ++j) {
+                const CookedRow x = ring[j];
+                ring[j] = fetch(min(r + j + kAhead, n - 1));
+                step(x, r + j == 0);
+            }
+#pragma unroll
+        for (int j = 0; j < kAhead; ++j)
+            if (r + j < n) step(ring[j], r + j == 0);
+        const float o = butterfly_of<2 * kRowsPerLane>(sums, lane);
+        if ((lane & 17) == 16) *out = f32_to_bf16_bits(o);
+    }
+    store_rows_global<S>(reinterpret_cast<S*>(p.state_out) + s_elem, uw, lane, s);
+}
+
+// The gated RMSNorm of every row (kda.cu:188-201), one warp per (row, head): `out` holds bf16(y) and receives the output.
+__global__ void __launch_bounds__(128) rows_norm_kernel(const __grid_constant__ RowsParams p) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int lane = threadIdx.x & 31;
+    const unsigned quads = (unsigned)(p.max_rows + 3) / 4, unit = blockIdx.x / quads;
+    const int j = (int)(blockIdx.x % quads) * 4 + (threadIdx.x >> 5);
+    const int h = (int)(unit % (unsigned)p.H), b = (int)(unit / (unsigned)p.H);
+    const int r0 = p.cu ? p.cu[b] : 0, n = p.cu ? p.cu[b + 1] - r0 : p.rows1;
+    if (j >= n) return;
+    const long long gr = (long long)r0 + j, col = (long long)h * DV + lane * 4;
+    uint16_t* dst = p.out + gr * p.out_stride + col;
+    const uint2 yb = *reinterpret_cast<const uint2*>(dst), gb = *reinterpret_cast<const uint2*>(p.gate + gr * p.gate_stride + col);
+    const uint2 wb = *reinterpret_cast<const uint2*>(p.norm_w + lane * 4);
+    const uint32_t yw4[4] = {yb.x << 16, yb.x & 0xffff0000u, yb.y << 16, yb.y & 0xffff0000u};
+    const uint32_t gw4[4] = {gb.x << 16, gb.x & 0xffff0000u, gb.y << 16, gb.y & 0xffff0000u};
+    const uint32_t nw4[4] = {wb.x << 16, wb.x & 0xffff0000u, wb.y << 16, wb.y & 0xffff0000u};
+    float ss = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) ss = ss + __uint_as_float(yw4[i]) * __uint_as_float(yw4[i]);
+    ss = butterfly1(ss);
+    const float rinv = 1.0f / sqrtf(ss / (float)DV + p.eps);
+    uint16_t o[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float yn = __uint_as_float(yw4[i]) * rinv;
+        const float yw = __uint_as_float(nw4[i]) * yn;
+        o[i] = f32_to_bf16_bits(yw * sigmoidf_(__uint_as_float(gw4[i])));
+    }
+    *reinterpret_cast<uint2*>(dst) = make_uint2((uint32_t)o[0] | ((uint32_t)o[1] << 16), (uint32_t)o[2] | ((uint32_t)o[3] << 16));
+}
+
+int launch(void (*kernel)(RowsParams), unsigned grid, const RowsParams& p, cudaStream_t stream, size_t smem = 0) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.dynamicSmemBytes = smem;
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(kRowsThreads);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // the kernels wait for their predecessors themselves
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return (int)cudaLaunchKernelEx(&cfg, kernel, p);
+}
+
+}  // namespace
+
+int rows_launch(RowsParams p, int batch, bool bf16_state, cudaStream_t stream) {
+    p.neg_zero2 = 0x8000000080000000ull;
+    const long long blocks = (long long)p.H * batch * kParts;
+    if (blocks > 0x7fffffffLL) return kInvalid;
+    auto* kernel = bf16_state ? rows_kernel<__nv_bfloat16> : rows_kernel<float>;
+    // Blocks that start while the prologue before them still fills most SMs would crowd onto the SMs that free up first, and
+    // a row takes as long as the fullest SM needs: shared memory nobody uses keeps a launch to its fair share of blocks per SM.
+    constexpr size_t kSmemPerSm = 227 * 1024;
+    const long long share = (blocks + sm_count() - 1) / sm_count();
+    const size_t pad = share < kPerSm ? kSmemPerSm / (size_t)(share + 1) + 1024 : 0;
+    static int configured[2] = {-1, -1};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (configured[bf16_state] != dev) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemPerSm);
+        if (e != cudaSuccess) return (int)e;
+        configured[bf16_state] = dev;
+    }
+    return launch(kernel, (unsigned)blocks, p, stream, pad);
+}
+
+int rows_norm_launch(const RowsParams& p, int batch, cudaStream_t stream) {
+    const long long blocks = (long long)p.H * batch * ((p.max_rows + 3) / 4);
+    if (blocks > 0x7fffffffLL) return kInvalid;
+    return blocks == 0 ? 0 : launch(rows_norm_kernel, (unsigned)blocks, p, stream);
+}
+
+}  // namespace kda
