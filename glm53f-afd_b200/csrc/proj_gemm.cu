@@ -16,7 +16,7 @@
 //           tile's accumulator to the epilogue when its last stage is in; owns the TMEM allocation;
 //   warps 2-5  epilogue: tcgen05.ld of the finished accumulator (lane = feature, column = row), convert, store.
 // Two accumulators alternate, so the epilogue of a tile overlaps the MMAs of the next; blocks walk the tile list with
-// the row tile fastest (blocks that run together share a weight tile in L2).  With NR <= 128 a block stays under
+// the row tile fastest (blocks that run together share a weight tile in L2).  A block stays under
 // 113 KiB of shared memory so that two fit an SM and every tile of a decode-size launch is in flight at once
 // (measured for the fused projection at 16 rows, 193 tiles: 38 us so, 48 us with one deeper-ringed block per SM).
 //
@@ -24,8 +24,8 @@
 // stage loop -- never on how many rows the launch has or which NR it picked (tests hold this bitwise).
 //
 // Few tiles (o_proj at decode: 32 feature tiles of k = 8192) would leave most SMs idle: there the k range of a tile is
-// split over the blocks of a thread-block cluster, each with its own accumulator, and rank 0 adds the partial tiles
-// in rank order through distributed shared memory (no scratch in global memory, the same bits every run).
+// split over the blocks of a thread-block cluster, each with its own accumulator, and the blocks add the partial tiles,
+// each for some of the rows, in rank order through distributed shared memory (no scratch in global memory, the same bits every run).
 //
 // Every wait is bounded (codes 130-135 in the device status word); TMEM is freed on every path; every block of a
 // cluster reaches the closing cluster barrier on every path.
@@ -37,14 +37,10 @@
 #include "common.cuh"
 #include "glm53f_proj.h"
 #include "kda_internal.h"
+#include "proj_gemm.cuh"
 #include "tc.cuh"
 
 namespace kda {
-
-// proj_gemm_pair.cu: 256 x 256 tiles on SM pairs, for launches with many rows.
-int proj_gemm_pair_launch(const CUtensorMap& tm_w, int w_swapped, const CUtensorMap& tm_x, int x_swapped, void* out, long long ldo, long long o_gstride,
-                          int groups, int rows, int n, int k, int out_f32, int* status, cudaStream_t stream);
-
 namespace {
 
 constexpr int kBM = 128;            // output features per tile (UMMA M)
@@ -59,14 +55,14 @@ template <int NR, bool SPLIT>
 struct Cfg {
     static constexpr int kBBytes = NR * 128;
     static constexpr int kStageBytes = kABytes + kBBytes;
-    static constexpr int kStages = SPLIT ? (NR == 16 ? 5 : NR == 32 ? 4 : NR == 64 ? 3 : 4) : (NR == 16 ? 6 : NR == 32 ? 5 : NR == 64 ? 4 : NR == 128 ? 3 : 4);
+    static constexpr int kStages = SPLIT ? (NR == 16 ? 5 : NR == 32 ? 4 : 3) : (NR == 16 ? 6 : NR == 32 ? 5 : 4);
     static constexpr int kTmemCols = 2 * NR < 32 ? 32 : 2 * NR;
-    static constexpr int kRedBytes = SPLIT ? kBM * NR * 4 : 0;  // this block's partial tile, f32 [128][NR]
+    static constexpr int kRedBytes = SPLIT ? kBM * NR * 4 : 0;  // this block's partial tile, f32 [NR][128]
     static constexpr int oRed = kStages * kStageBytes;
     static constexpr int oBars = oRed + kRedBytes;  // full[S], empty[S], acc_full[2], acc_empty[2], red_full, red_empty
     static constexpr int oCtl = oBars + (2 * kStages + 6) * 8;
     static constexpr int kBytes = oCtl + 16 + 1024;      // + slack to align the stages to 1024 bytes
-    static constexpr int kBlocksPerSm = (NR <= 64 || (NR == 128 && !SPLIT)) ? 2 : 1;
+    static constexpr int kBlocksPerSm = 2;
 };
 
 struct GemmParams {
@@ -77,6 +73,7 @@ struct GemmParams {
     int n_tiles, r_tiles;
     int w_swapped, x_swapped;  // the map's coordinates are (k, group, row) instead of (k, row, group)
     long long tiles;
+    int overlap;  // 0: alone; 1: the first of two independent launches; 2: the second (see glm53f_kda_proj_bf16_many)
     int* status;
 };
 
@@ -107,9 +104,9 @@ __device__ __forceinline__ void peer_mbar_arrive(uint32_t remote_bar) {
 }
 __device__ __forceinline__ void fence_cluster() { asm volatile("fence.acq_rel.cluster;" ::: "memory"); }
 
-__device__ __forceinline__ float4 peer_load4(uint32_t remote_addr) {
-    float4 v;
-    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(remote_addr) : "memory");
+__device__ __forceinline__ float peer_load(uint32_t remote_addr) {
+    float v;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(remote_addr) : "memory");
     return v;
 }
 
@@ -124,8 +121,8 @@ __global__ void __launch_bounds__(kGemmThreads, Cfg<NR, (KS > 1)>::kBlocksPerSm)
     uint64_t* empty = full + C::kStages;
     uint64_t* acc_full = empty + C::kStages;
     uint64_t* acc_empty = acc_full + 2;
-    uint64_t* red_full = acc_empty + 2;   // rank 0: every peer's partial is in its buffer
-    uint64_t* red_empty = red_full + 1;   // peers: rank 0 has read the partial
+    uint64_t* red_full = acc_empty + 2;   // every block's partial of this tile is in its buffer
+    uint64_t* red_empty = red_full + 1;   // every block has read this block's partial
     constexpr uint32_t ks = KS;
     const uint32_t kr = SPLIT ? cluster_rank() : 0u;
     const long long tile0 = blockIdx.x / ks, tile_step = gridDim.x / ks;
@@ -142,8 +139,8 @@ __global__ void __launch_bounds__(kGemmThreads, Cfg<NR, (KS > 1)>::kBlocksPerSm)
             mbar_init(&acc_full[i], 1);
             mbar_init(&acc_empty[i], kEpiThreads / 32);
         }
-        mbar_init(red_full, ks > 1 ? (ks - 1) * (kEpiThreads / 32) : 1);
-        mbar_init(red_empty, kEpiThreads / 32);
+        mbar_init(red_full, ks * (kEpiThreads / 32));
+        mbar_init(red_empty, ks * (kEpiThreads / 32));
         ctl[0] = 0u;
         ctl[1] = 0u;
         mbar_init_fence();
@@ -161,9 +158,13 @@ __global__ void __launch_bounds__(kGemmThreads, Cfg<NR, (KS > 1)>::kBlocksPerSm)
     tc::fence_after_sync();
     const uint32_t tm = *tmem_slot;
     const WaitCtx ctx{ctl, ctl + 1, p.status};
-    launch_dependents();
     bool opened = !SPLIT;  // whether this thread has completed the opening cluster barrier
-    grid_dependency_wait();  // before the first global access: an earlier kernel may be writing the weight or the rows
+    // Before the first global access: an earlier kernel may be writing the weight or the rows.  Of two independent launches the
+    // first lets the second in only once the kernels before both have finished, and the second does not wait for the first
+    // until its own end, where whatever follows it expects both to be done.
+    if (p.overlap == 0) launch_dependents();
+    if (p.overlap != 2) grid_dependency_wait();
+    if (p.overlap != 0) launch_dependents();
 
     if (warp == 0) {
         if (lane == 0) {
@@ -189,32 +190,32 @@ __global__ void __launch_bounds__(kGemmThreads, Cfg<NR, (KS > 1)>::kBlocksPerSm)
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            constexpr uint32_t idesc = tc::idesc_bf16(kBM, NR, 0, 0, 0);
-            int s = 0, buf = 0;
-            uint32_t ph = 0, acc_ph[2] = {0, 0};
-            for (long long t = tile0; t < p.tiles; t += tile_step) {
-                if (!mbar_wait(&acc_empty[buf], acc_ph[buf] ^ 1u, ctx, kStatusGemmAccEmpty)) goto done;
+        // The whole warp runs this loop and one lane issues (tc::mma_bf16_if): operands stay in uniform registers.
+        constexpr uint32_t idesc = tc::idesc_bf16(kBM, NR, 0, 0, 0);
+        const uint32_t leader = tc::elect_one();
+        int s = 0, buf = 0;
+        uint32_t ph = 0, acc_ph[2] = {0, 0};
+        for (long long t = tile0; t < p.tiles; t += tile_step) {
+            if (!tc::warp_all(mbar_wait(&acc_empty[buf], acc_ph[buf] ^ 1u, ctx, kStatusGemmAccEmpty))) goto done;
+            tc::fence_after_sync();
+            const uint32_t d = tm + (uint32_t)(buf * NR);
+            for (int kb = 0; kb < kb_n; ++kb) {
+                if (!tc::warp_all(mbar_wait(&full[s], ph, ctx, kStatusGemmFull))) goto done;
                 tc::fence_after_sync();
-                const uint32_t d = tm + (uint32_t)(buf * NR);
-                for (int kb = 0; kb < kb_n; ++kb) {
-                    if (!mbar_wait(&full[s], ph, ctx, kStatusGemmFull)) goto done;
-                    tc::fence_after_sync();
-                    const unsigned char* st = smem + s * C::kStageBytes;
+                const unsigned char* st = smem + s * C::kStageBytes;
 #pragma unroll
-                    for (int i = 0; i < kBK / 16; ++i)
-                        tc::mma_bf16(d, tc::desc_sw128_kmajor(st, kBM, 16 * i), tc::desc_sw128_kmajor(st + kABytes, NR, 16 * i), idesc, kb > 0 || i > 0);
-                    tc::mma_commit(&empty[s]);
-                    if (++s == C::kStages) {
-                        s = 0;
-                        ph ^= 1u;
-                    }
+                for (int i = 0; i < kBK / 16; ++i)
+                    tc::mma_bf16_if(leader, d, tc::desc_sw128_kmajor(st, kBM, 16 * i), tc::desc_sw128_kmajor(st + kABytes, NR, 16 * i), idesc, kb > 0 || i > 0);
+                tc::mma_commit_if(leader, &empty[s]);
+                if (++s == C::kStages) {
+                    s = 0;
+                    ph ^= 1u;
                 }
-                tc::mma_commit(&acc_full[buf]);
-                acc_ph[buf] ^= 1u;
-                buf ^= 1;
-                ctl[0] = ctl[0] + 1u;
             }
+            tc::mma_commit_if(leader, &acc_full[buf]);
+            acc_ph[buf] ^= 1u;
+            buf ^= 1;
+            if (leader) ctl[0] = ctl[0] + 1u;
         }
     } else {
         const int q = warp & 3;  // the TMEM lane quarter this warp may read
@@ -251,62 +252,50 @@ __global__ void __launch_bounds__(kGemmThreads, Cfg<NR, (KS > 1)>::kBlocksPerSm)
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&acc_empty[buf]);
             } else {
-                // The tile's K splits live in the blocks of this cluster.  Peers park their partial tile in their own
-                // shared memory; rank 0 adds them to its own in rank order (a fixed order: the same bits every time)
-                // through distributed shared memory, and stores.  32 columns at a time.
-                constexpr int CW = NR < 32 ? NR : 32;
-                float* red = reinterpret_cast<float*>(smem + C::oRed) + fl * NR;
+                // The tile's K splits live in the blocks of this cluster.  Every block parks its partial tile in its own shared
+                // memory and then finishes NR / KS of the tile's rows: it adds the blocks' partials in rank order (a fixed order:
+                // the same bits every time) through distributed shared memory, and stores.  (With rank 0 alone adding everything
+                // a launch of 64 rows of the 4096 -> 256 factor took 25 us.)
+                constexpr int CW = NR / KS;
+                float* red = reinterpret_cast<float*>(smem + C::oRed) + fl;  // [NR rows][128 features]
                 if (!opened) {  // the opening cluster barrier: every peer's barriers and buffers exist
                     cluster_wait();
                     opened = true;
                 }
-                if (kr != 0) {
-                    if (!mbar_wait(red_empty, red_ph ^ 1u, ctx, kStatusGemmRedEmpty)) goto done;  // rank 0 is done with the last one
-                    fence_cluster();
-                } else {
-                    if (!mbar_wait(red_full, red_ph, ctx, kStatusGemmRedFull)) goto done;
-                    fence_cluster();
-                }
+                if (!mbar_wait(red_empty, red_ph ^ 1u, ctx, kStatusGemmRedEmpty)) goto done;  // the last tile's partial has been read
+                fence_cluster();
 #pragma unroll 1
-                for (int c0 = 0; c0 < NR; c0 += CW) {
-                    float v[CW];
+                for (int c0 = 0; c0 < NR; c0 += 16) {
+                    uint32_t r[16];
+                    tc::tmem_ld16(tc::tmem_addr(tm, q, buf * NR + c0), r);
+                    tc::tmem_ld_wait();
 #pragma unroll
-                    for (int c1 = 0; c1 < CW; c1 += 16) {
-                        uint32_t r[16];
-                        tc::tmem_ld16(tc::tmem_addr(tm, q, buf * NR + c0 + c1), r);
-                        tc::tmem_ld_wait();
-#pragma unroll
-                        for (int j = 0; j < 16; ++j) v[c1 + j] = __uint_as_float(r[j]);
-                    }
-                    if (kr != 0) {
-#pragma unroll
-                        for (int j = 0; j < CW; j += 4) *reinterpret_cast<float4*>(red + c0 + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-                    } else {
-#pragma unroll
-                        for (uint32_t r = 1; r < ks; ++r) {
-                            const uint32_t remote = peer_smem(red + c0, r);
-#pragma unroll
-                            for (int j = 0; j < CW; j += 4) {
-                                const float4 t4 = peer_load4(remote + (uint32_t)j * 4);
-                                v[j] = v[j] + t4.x;
-                                v[j + 1] = v[j + 1] + t4.y;
-                                v[j + 2] = v[j + 2] + t4.z;
-                                v[j + 3] = v[j + 3] + t4.w;
-                            }
-                        }
-#pragma unroll
-                        for (int j = 0; j < CW; ++j) store(c0 + j, v[j]);
-                    }
+                    for (int j = 0; j < 16; ++j) red[(c0 + j) * kBM] = __uint_as_float(r[j]);
                 }
                 tc::fence_before_sync();
                 fence_cluster();
                 __syncwarp();
-                if (lane == 0) {
-                    mbar_arrive(&acc_empty[buf]);
-                    if (kr != 0) peer_mbar_arrive(peer_smem(red_full, 0));
-                    else
-                        for (uint32_t r = 1; r < ks; ++r) peer_mbar_arrive(peer_smem(red_empty, r));
+                if (lane == 0) mbar_arrive(&acc_empty[buf]);
+                if (lane < KS) peer_mbar_arrive(peer_smem(red_full, lane));
+                if (!mbar_wait(red_full, red_ph, ctx, kStatusGemmRedFull)) goto done;
+                fence_cluster();
+                float v[CW][KS];
+#pragma unroll
+                for (uint32_t r = 0; r < ks; ++r) {
+                    const uint32_t remote = peer_smem(red + kr * CW * kBM, r);
+#pragma unroll
+                    for (int c = 0; c < CW; ++c) v[c][r] = peer_load(remote + (uint32_t)(c * kBM * 4));
                 }
+#pragma unroll
+                for (int c = 0; c < CW; ++c) {
+                    float sum = v[c][0];
+#pragma unroll
+                    for (uint32_t r = 1; r < ks; ++r) sum = sum + v[c][r];
+                    store((int)kr * CW + c, sum);
+                }
+                fence_cluster();
+                __syncwarp();
+                if (lane < KS) peer_mbar_arrive(peer_smem(red_empty, lane));
                 red_ph ^= 1u;
             }
             buf ^= 1;
@@ -319,6 +308,7 @@ done:
         while (global_timer_ns() - t0 < 2000000ull) {
         }
     }
+    if (p.overlap == 2) grid_dependency_wait();
     tc::fence_before_sync();
     __syncthreads();
     if (warp == 1) tc::tmem_dealloc(tm, C::kTmemCols);
@@ -341,11 +331,17 @@ EncodeTiled encode_tiled() {
     return fn;
 }
 
+constexpr int kFewRows = 64;        // launches of up to this many rows run here, larger ones on SM pairs
+// ... and a K-split shape by itself up to here: its splits run side by side on a cluster, on a pair one after another (o_proj at
+// 128 rows: 36 us on pairs, 24 so)
+constexpr int kFewRowsSplit = 128;
+constexpr int kSplitRowsMax = 512;  // ... and up to this many keep the K split's summation order
+
 // A [groups][rows][k] bf16 matrix (row stride ld, group stride gstride, in elements) as a 3-D map with boxes of
 // 64 k x box_rows rows in the 128-byte swizzle; rows past the extent read as zero.  The dimensions are ordered by
 // stride -- (k, rows, groups), or (k, groups, rows) when the groups interleave inside a row (`swapped`).
 bool matrix_map(CUtensorMap* tm, int* swapped, const void* base, long long k, long long rows, long long groups, long long ld, long long gstride,
-                int box_rows) {
+                int box_rows, int box_k = kBK) {
     EncodeTiled enc = encode_tiled();
     if (enc == nullptr) return false;
     const long long gs = groups > 1 ? gstride : rows * ld;
@@ -353,7 +349,7 @@ bool matrix_map(CUtensorMap* tm, int* swapped, const void* base, long long k, lo
     if (groups > 1 && !*swapped && gs < rows * ld) return false;  // neither nesting: not a layout the callers have
     const cuuint64_t dims[3] = {(cuuint64_t)k, (cuuint64_t)(*swapped ? groups : rows), (cuuint64_t)(*swapped ? rows : groups)};
     const cuuint64_t strides[2] = {(cuuint64_t)(*swapped ? gs : ld) * 2, (cuuint64_t)(*swapped ? ld : gs) * 2};
-    const cuuint32_t box[3] = {(cuuint32_t)kBK, *swapped ? 1u : (cuuint32_t)box_rows, *swapped ? (cuuint32_t)box_rows : 1u};
+    const cuuint32_t box[3] = {(cuuint32_t)box_k, *swapped ? 1u : (cuuint32_t)box_rows, *swapped ? (cuuint32_t)box_rows : 1u};
     const cuuint32_t estr[3] = {1u, 1u, 1u};
     return enc(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
@@ -361,8 +357,8 @@ bool matrix_map(CUtensorMap* tm, int* swapped, const void* base, long long k, lo
 
 // K splits for a launch of few tiles (little n, deep k: o_proj at decode): the largest of 8, 4, 2 that divides the
 // k blocks into runs of at least four and still leaves every block of a one-row-tile launch resident at once.  It is
-// a function of (n, k, groups) alone for every launch on row tiles of up to 128 rows (all launches of up to 512 rows), so
-// a row's bits do not depend on `rows` there.  Measured for
+// a function of (n, k, groups) alone in all launches of up to 512 rows (beyond 64 rows the same parts of k are summed in the
+// same order on SM pairs), so a row's bits do not depend on `rows` there.  Measured for
 // o_proj at 16 rows (32 tiles): no split 40.7 us, 2 splits 27.1, 4 splits 20.9, 8 splits (two waves of clusters) 24.7.
 int pick_ksplit(long long tiles, int kblocks, long long resident) {
     for (int s = 8; s >= 2; s >>= 1)
@@ -417,61 +413,128 @@ int launch_gemm(GemmParams& p, const void* x, long long ldx, long long x_gstride
     p.r_tiles = (p.rows + NR - 1) / NR;
     p.tiles = (long long)groups * p.n_tiles * p.r_tiles;
     const long long cap = (long long)sm_count() * Cfg<NR, false>::kBlocksPerSm;
-    if constexpr (NR <= 128) {
-        // The split is chosen for ONE row tile, whatever the launch's row count: a row's bits then depend on
-        // (groups, n, k) only.  More row tiles than fit at once are walked by the same clusters.
-        const int ks = pick_ksplit((long long)groups * p.n_tiles, p.kblocks, sm_count());  // clusters were measured at one block per SM
-        const long long fit = cap / ks;
-        const long long clusters = p.tiles < fit ? p.tiles : fit;
-        if (ks == 8) return launch_one<NR, 8>(p, clusters, stream);
-        if (ks == 4) return launch_one<NR, 4>(p, clusters, stream);
-        if (ks == 2) return launch_one<NR, 2>(p, clusters, stream);
-    }
+    // The split is chosen for ONE row tile, whatever the launch's row count: a row's bits then depend on (groups, n, k) only.
+    const int ks = pick_ksplit((long long)groups * p.n_tiles, p.kblocks, sm_count());  // clusters were measured at one block per SM
+    const long long fit = cap / ks;
+    const long long clusters = p.tiles < fit ? p.tiles : fit;
+    if (ks == 8) return launch_one<NR, 8>(p, clusters, stream);
+    if (ks == 4) return launch_one<NR, 4>(p, clusters, stream);
+    if (ks == 2) return launch_one<NR, 2>(p, clusters, stream);
     return launch_one<NR, 1>(p, p.tiles < cap ? p.tiles : cap, stream);
 }
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
+// Rows per tile of a launch on SM pairs: the multiple of 16 with the least time by the counts of the machine.  A stage of 64 k
+// takes a pair 2 NR cycles of tensor pipe and 16 KiB + 64 NR bytes per block through a port of about 60 bytes a cycle; a tile
+// costs about 1,500 cycles beside its stages, or its epilogue (500 cycles for 64 rows) where that is longer; pairs take
+// tiles in rounds.  (At 333 rows of the fused projection: two tiles of 176 rows, 194 of them in three rounds.)
+int pick_row_tile(long long feature_tiles, int rows, int kblocks, int most) {
+    const long long pairs = sm_count() / 2;
+    int best = most;
+    double least = 1e30;
+    for (int nr = 16; nr <= most; nr += 16) {
+        const long long r_tiles = (rows + nr - 1) / nr, rounds = (feature_tiles * r_tiles + pairs - 1) / pairs;
+        const double load = (16384.0 + 64.0 * nr) / 60.0, mma = 2.0 * nr, stages = kblocks * (load > mma ? load : mma), out = (nr + 63) / 64 * 500.0;
+        const double time = (double)rounds * ((stages > out ? stages : out) + 1500.0);
+        if (time < least * 0.999) {
+            least = time;
+            best = nr;
+        }
+        if (r_tiles == 1) break;
+    }
+    return best;
+}
+
+int k_segments(const glm53f_proj_job& j) {
+    return j.rows <= kSplitRowsMax ? pick_ksplit((long long)j.groups * ((j.n + kBM - 1) / kBM), j.k / kBK, sm_count()) : 1;
+}
+
+bool pair_problem(PairProblem& q, const glm53f_proj_job& j) {
+    q = PairProblem{};
+    q.out = j.out;
+    q.ldo = j.ldo;
+    q.o_gstride = j.groups > 1 ? j.o_gstride : 0;
+    q.rows = j.rows;
+    q.n = j.n;
+    q.kblocks = j.k / kBK;
+    q.out_f32 = j.out_f32 != 0;
+    q.segments = k_segments(j);
+    q.n_tiles = (j.n + 2 * kBM - 1) / (2 * kBM);
+    q.row_tile = pick_row_tile((long long)j.groups * q.n_tiles, j.rows, q.kblocks, q.segments > 1 ? 128 : 256);
+    q.r_tiles = (j.rows + q.row_tile - 1) / q.row_tile;
+    q.tiles = (long long)j.groups * q.n_tiles * q.r_tiles;
+    if (q.tiles > 0x3fffffff) return false;
+    if (!matrix_map(&q.tm_w, &q.w_swapped, j.w, j.k, j.n, j.groups, j.ldw, j.w_gstride, kBM) ||
+        !matrix_map(&q.tm_x, &q.x_swapped, j.x, j.k, j.rows, j.groups, j.ldx, j.x_gstride, q.row_tile / 2))
+        return false;
+    // bf16 rows that start on 16 bytes leave as tensor stores (boxes of 64 features x 16 rows).
+    q.tensor_out = !q.out_f32 && aligned16(j.out) && j.ldo % 8 == 0 && (j.groups == 1 || (j.o_gstride % 8 == 0 && j.o_gstride > 0)) &&
+                   matrix_map(&q.tm_out, &q.out_swapped, j.out, j.n, j.rows, j.groups, j.ldo, j.o_gstride, 16, 64);
+    return true;
+}
+
+// Whether the arguments are those of a GEMM the kernels take (kInvalid otherwise); rows == 0 needs no pointers.
+int check_job(const glm53f_proj_job& j) {
+    if (j.groups < 1 || j.rows < 0 || j.n < 1 || j.k < kBK || j.k % kBK || j.n % 8 || j.ldx % 8 || j.ldw % 8 || j.ldx < j.k || j.ldw < j.k || j.ldo < j.n)
+        return kInvalid;
+    if (j.groups > 1 && (j.x_gstride % 8 || j.w_gstride % 8 || j.x_gstride < 0 || j.w_gstride < 0 || j.o_gstride < 0)) return kInvalid;
+    if (j.rows == 0) return 0;
+    if (!j.x || !j.w || !j.out || !aligned16(j.x) || !aligned16(j.w) || (reinterpret_cast<uintptr_t>(j.out) & (j.out_f32 ? 3 : 1))) return kInvalid;
+    return 0;
+}
+
+int few_rows(const glm53f_proj_job& j, int overlap, int* status, cudaStream_t stream) {
+    GemmParams p{};
+    p.out = j.out;
+    p.ldo = j.ldo;
+    p.o_gstride = j.groups > 1 ? j.o_gstride : 0;
+    p.rows = j.rows;
+    p.n = j.n;
+    p.kblocks = j.k / kBK;
+    p.out_f32 = j.out_f32 != 0;
+    p.n_tiles = (j.n + kBM - 1) / kBM;
+    p.overlap = overlap;
+    p.status = status;
+    if (!matrix_map(&p.tm_w, &p.w_swapped, j.w, j.k, j.n, j.groups, j.ldw, j.w_gstride, kBM)) return (int)cudaErrorNotSupported;
+    if (j.rows <= 16) return launch_gemm<16>(p, j.x, j.ldx, j.x_gstride, j.groups, j.k, stream);
+    if (j.rows <= 32) return launch_gemm<32>(p, j.x, j.ldx, j.x_gstride, j.groups, j.k, stream);
+    return launch_gemm<64>(p, j.x, j.ldx, j.x_gstride, j.groups, j.k, stream);
+}
+
 }  // namespace
 }  // namespace kda
+
+extern "C" int32_t glm53f_kda_proj_bf16_many(const glm53f_proj_job* jobs, int32_t count, glm53f_stream_t stream) {
+    using namespace kda;
+    if (!jobs || count < 0) return kInvalid;
+    for (int i = 0; i < count; ++i)
+        if (check_job(jobs[i]) != 0) return kInvalid;
+    int* status = status_word();
+    if (status == nullptr) return (int)cudaErrorUnknown;
+    for (int i = 0; i < count; ++i) {
+        const glm53f_proj_job& j = jobs[i];
+        if (j.rows == 0) continue;
+        const bool two = i + 1 < count && jobs[i + 1].rows > 0 && (jobs[i + 1].rows <= kFewRows) == (j.rows <= kFewRows);
+        int rc = 0;
+        if (j.rows <= kFewRows || (!two && j.rows <= kFewRowsSplit && k_segments(j) > 1)) {
+            rc = few_rows(j, two ? 1 : 0, status, stream);
+            if (rc == 0 && two) rc = few_rows(jobs[++i], 2, status, stream);
+        } else {
+            PairProblem q[kPairProblems];
+            if (!pair_problem(q[0], j) || (two && !pair_problem(q[1], jobs[i + 1]))) return (int)cudaErrorNotSupported;
+            rc = proj_gemm_pair_launch(q, two ? 2 : 1, status, stream);
+            i += two ? 1 : 0;
+        }
+        if (rc != 0) return rc;
+    }
+    return 0;
+}
 
 extern "C" int32_t glm53f_kda_proj_bf16(const uint16_t* x, int64_t ldx, int64_t x_gstride, const uint16_t* w, int64_t ldw, int64_t w_gstride,
                                         int32_t groups, int32_t rows, int32_t n, int32_t k, void* out, int32_t out_f32, int64_t ldo,
                                         int64_t o_gstride, glm53f_stream_t stream) {
-    using namespace kda;
-    if (groups < 1 || rows < 0 || n < 1 || k < kBK || k % kBK || n % 8 || ldx % 8 || ldw % 8 || ldx < k || ldw < k || ldo < n) return kInvalid;
-    if (groups > 1 && (x_gstride % 8 || w_gstride % 8 || x_gstride < 0 || w_gstride < 0 || o_gstride < 0)) return kInvalid;
-    if (rows == 0) return 0;
-    if (!x || !w || !out || !aligned16(x) || !aligned16(w) || (reinterpret_cast<uintptr_t>(out) & (out_f32 ? 3 : 1))) return kInvalid;
-    GemmParams p{};
-    p.out = out;
-    p.ldo = ldo;
-    p.o_gstride = groups > 1 ? o_gstride : 0;
-    p.rows = rows;
-    p.n = n;
-    p.kblocks = k / kBK;
-    p.out_f32 = out_f32 != 0;
-    p.n_tiles = (n + kBM - 1) / kBM;
-    p.status = status_word();
-    if (p.status == nullptr) return (int)cudaErrorUnknown;
-    if (!matrix_map(&p.tm_w, &p.w_swapped, w, k, n, groups, ldw, w_gstride, kBM)) return (int)cudaErrorNotSupported;
-    if (rows <= 16) return launch_gemm<16>(p, x, ldx, x_gstride, groups, k, stream);
-    if (rows <= 32) return launch_gemm<32>(p, x, ldx, x_gstride, groups, k, stream);
-    if (rows <= 64) return launch_gemm<64>(p, x, ldx, x_gstride, groups, k, stream);
-    if (rows <= 128) return launch_gemm<128>(p, x, ldx, x_gstride, groups, k, stream);
-    // Wide row tiles once there are rows enough to fill the GPU with them; otherwise narrower ones, two blocks per SM,
-    // which quantise better (measured for n = 24,640: 384 rows 81 us against 96 us, 768 rows 144 us against 141 us).
-    if (rows > 512 && (long long)groups * p.n_tiles * ((rows + 255) / 256) >= sm_count()) {
-        // Enough 256 x 256 tiles for every SM pair: the two-block kernel (GLM53F_KDA_PROJ_PAIR=0 keeps one block per tile).
-        static const bool pair = [] {
-            const char* e = getenv("GLM53F_KDA_PROJ_PAIR");
-            return e == nullptr || e[0] != '0';
-        }();
-        if (pair) {
-            if (!matrix_map(&p.tm_x, &p.x_swapped, x, k, rows, groups, ldx, x_gstride, 128)) return (int)cudaErrorNotSupported;
-            return proj_gemm_pair_launch(p.tm_w, p.w_swapped, p.tm_x, p.x_swapped, out, ldo, o_gstride, groups, rows, n, k, out_f32 != 0, p.status, stream);
-        }
-        return launch_gemm<256>(p, x, ldx, x_gstride, groups, k, stream);
-    }
-    return launch_gemm<128>(p, x, ldx, x_gstride, groups, k, stream);
+    const glm53f_proj_job job{x, ldx, x_gstride, w, ldw, w_gstride, groups, rows, n, k, out, out_f32, ldo, o_gstride};
+    const int rc = kda::check_job(job);
+    return rc != 0 || rows == 0 ? rc : glm53f_kda_proj_bf16_many(&job, 1, stream);
 }

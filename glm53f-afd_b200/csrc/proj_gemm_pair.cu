@@ -1,5 +1,5 @@
-// The projection GEMM for many rows on SM pairs: out[g][r][o] = sum_k x[g][r][k] * w[g][o][k] with 256 x 256 tiles
-// computed by tcgen05.mma.cta_group::2.
+// The projection GEMM for many rows on SM pairs: out[g][r][o] = sum_k x[g][r][k] * w[g][o][k] with tiles of 256 features x NR
+// rows computed by tcgen05.mma.cta_group::2, NR a multiple of 16 up to 256 chosen per launch.
 //
 // Why a pair.  With one block per tile (proj_gemm.cu) a 128 x 256 tile reads 48 KiB of operands from L2 per 4.2 MFLOP;
 // the tensor pipe then waits on the copies a quarter of the time.  Two blocks of a cluster that share a 256 x 256 tile
@@ -9,10 +9,23 @@
 // Protocol (block 0 of the pair leads):
 //   producer (warp 0, both blocks)  tensor copies of the block's weight tile and its half of the rows into its own
 //                                   ring; the copies of BOTH blocks complete the LEADER's stage barrier;
-//   MMA (warp 1 of the leader)      one thread issues the pair's MMAs (M = 256, N = 256, K = 16) and commits each stage
-//                                   to both blocks' `empty` barriers, each finished tile to both `acc_full` barriers;
-//   epilogue (warps 2-5, both)      each block drains its own 128 features x 256 rows from its tensor memory and
-//                                   arrives on the leader's `acc_empty`.
+//   MMA (warp 1 of the leader)      one thread issues the pair's MMAs (M = 256, N = NR, K = 16) and commits each stage
+//                                   to both blocks' `empty` barriers, each finished accumulator to both `acc_full` barriers;
+//   epilogue (warps 2-9, both)      each block drains its own 128 features x NR rows from its tensor memory, through
+//                                   shared memory (a thread holds ONE feature of sixteen rows; rows of 64 features leave as
+//                                   tiled tensor stores), and arrives on the leader's `acc_empty`.
+// The epilogue's way out was what bounded wide launches: with two-byte stores straight from the registers a 256 x 256 tile
+// took 17 us to leave, as long as a k of 4,096 takes to compute, and the k = 128 gate factor (67 MB of results at 2,048 rows)
+// ran at 0.5 TB/s.
+//
+// A launch carries up to two independent problems (their tiles in one list): the 4096 -> 256 first gate factor has one feature
+// tile and is all latency by itself (114 us at 2,048 rows as its own K-split launch); beside the fused [q|k|v|b] projection
+// of the same rows it is one tile column more.
+//
+// K segments.  A shape whose small launches split k over a cluster (proj_gemm.cu) adds its partial sums in f32 in split order;
+// a row's bits must not depend on the launch's row count, so here such a shape's tile runs its k in the same segments, each
+// into a fresh accumulator, and the epilogue adds them in the same order (kept in registers: NR <= 128 then).
+//
 // Tensor memory is allocated by both blocks together (512 columns: two accumulators).  Every wait is bounded (codes
 // 140-143); both blocks reach the collective TMEM release and the closing cluster barrier on every path.
 
@@ -21,22 +34,29 @@
 #include "common.cuh"
 #include "glm53f_proj.h"
 #include "kda_internal.h"
+#include "proj_gemm.cuh"
 #include "tc.cuh"
 
 namespace kda {
 namespace {
 
 constexpr int kPM = 128;           // features per block (256 per pair)
-constexpr int kPN = 256;           // rows per tile (128 loaded by each block)
+constexpr int kPN = 256;           // rows per tile at most (half of them loaded by each block)
 constexpr int kPK = 64;
-constexpr int kPairThreads = 192;
+constexpr int kPairThreads = 320;  // producer, MMA, eight epilogue warps
 constexpr int kPairStages = 6;
 constexpr int kPairABytes = kPM * 128, kPairBBytes = (kPN / 2) * 128;
 constexpr int kPairStageBytes = kPairABytes + kPairBBytes;  // 32 KiB
 constexpr int kPairTmemCols = 512;
-constexpr int oPairBars = kPairStages * kPairStageBytes;
+constexpr int kSplitRows = 128;    // rows per tile at most when k runs in segments
+// Output staging: two buffers per pair of epilogue warps, each two boxes of 16 rows x 64 features in the 128-byte swizzle.
+// (NR is a multiple of 16, not of 32; a fence and two barriers per sixteen rows were most of the epilogue's time.)
+constexpr int kBoxRows = 16, kChunk = 2 * kBoxRows, kOutBuf = kChunk * 128;
+constexpr int oPairOut = kPairStages * kPairStageBytes;
+constexpr int oPairBars = oPairOut + 8 * kOutBuf;
 constexpr int oPairCtl = oPairBars + (2 * kPairStages + 4) * 8;
 constexpr int kPairSmem = oPairCtl + 16 + 1024;
+static_assert(kPairSmem <= 232448, "shared memory budget");
 
 enum : int { kStatusPairEmpty = 140, kStatusPairFull = 141, kStatusPairAccFull = 142, kStatusPairAccEmpty = 143 };
 
@@ -71,28 +91,43 @@ __device__ __forceinline__ void pair_tmem_alloc(uint32_t* smem_result, uint32_t 
 __device__ __forceinline__ void pair_tmem_dealloc(uint32_t taddr, uint32_t cols) {
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
 }
-__device__ __forceinline__ void pair_mma(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, bool accumulate) {
+// Issued by the whole warp with `leader` set in one lane: the operands then stay in uniform registers.  (Inside an `if` of one
+// lane the compiler moves every operand of every MMA over from the lane's registers: about 90 cycles an instruction, 360 of
+// the 590 cycles a stage took.)
+__device__ __forceinline__ void pair_mma(uint32_t leader, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, bool accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"((uint32_t)accumulate)
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"((uint32_t)accumulate), "r"(leader)
         : "memory");
 }
-// `bar_addr` (a shared::cluster address, this block's or the pair's) completes once the pair's MMAs issued so far have.
-__device__ __forceinline__ void pair_commit(uint32_t bar_addr) {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_addr) : "memory");
+// The barrier at this shared-memory offset in BOTH blocks completes once the pair's MMAs issued so far by this thread have
+// (one commit with a block mask instead of one per block).
+__device__ __forceinline__ void pair_commit(uint32_t leader, uint64_t* bar) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t"
+        "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}" ::"r"(smem_u32(bar)),
+        "h"((uint16_t)3), "r"(leader)
+        : "memory");
 }
 
 struct PairParams {
-    CUtensorMap tm_w, tm_x;
-    void* out;
-    long long ldo, o_gstride;
-    int rows, n, kblocks, out_f32;
-    int n_tiles, r_tiles;
-    int w_swapped, x_swapped;
-    long long tiles;
+    PairProblem problem[kPairProblems];
+    long long tiles0, tiles;  // the first problem's tiles, all tiles
     int* status;
 };
+
+// Tile t of the launch: its problem and its place there (row tiles fastest: pairs that run together share a weight tile in L2).
+struct PairTile {
+    const PairProblem& q;
+    int rt, nt, g;
+};
+__device__ __forceinline__ PairTile pair_tile(const PairParams& p, long long t) {
+    const bool second = t >= p.tiles0;
+    const PairProblem& q = p.problem[second ? 1 : 0];
+    const int i = (int)(second ? t - p.tiles0 : t), u = i / q.r_tiles;
+    return {q, i - u * q.r_tiles, u % q.n_tiles, u / q.n_tiles};
+}
 
 __global__ void __launch_bounds__(kPairThreads, 1) proj_gemm_pair_kernel(const __grid_constant__ PairParams p) {
     extern __shared__ unsigned char smem_raw[];
@@ -113,7 +148,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) proj_gemm_pair_kernel(const _
         }
         for (int i = 0; i < 2; ++i) {
             mbar_init(&acc_full[i], 1);
-            mbar_init(&acc_empty[i], 8);  // four epilogue warps of each block
+            mbar_init(&acc_empty[i], 16);  // eight epilogue warps of each block
         }
         ctl[0] = 0u;
         ctl[1] = 0u;
@@ -127,25 +162,27 @@ __global__ void __launch_bounds__(kPairThreads, 1) proj_gemm_pair_kernel(const _
     tc::fence_after_sync();
     const uint32_t tm = *tmem_slot;
     const WaitCtx ctx{ctl, ctl + 1, p.status};
+    // Programmatic dependent launch: nothing global is touched before the kernels ahead have finished.
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
 
     if (warp == 0) {
         if (lane == 0) {
             int s = 0;
             uint32_t ph = 0;
             for (long long t = tile0; t < p.tiles; t += tile_step) {
-                const int rt = (int)(t % p.r_tiles);
-                const long long u = t / p.r_tiles;
-                const int nt = (int)(u % p.n_tiles), g = (int)(u / p.n_tiles);
-                const int f0 = nt * 2 * kPM + (int)rank * kPM, r0 = rt * kPN + (int)rank * (kPN / 2);
-                for (int kb = 0; kb < p.kblocks; ++kb) {
+                const PairTile x = pair_tile(p, t);
+                const int half = x.q.row_tile / 2;
+                const int f0 = x.nt * 2 * kPM + (int)rank * kPM, r0 = x.rt * x.q.row_tile + (int)rank * half;
+                const void *mw = &x.q.tm_w, *mx = &x.q.tm_x; const int nkb = x.q.kblocks; const uint32_t tx = 2u * (uint32_t)(kPairABytes + half * 128);
+                const int wy = x.q.w_swapped ? x.g : f0, wz = x.q.w_swapped ? f0 : x.g, xy = x.q.x_swapped ? x.g : r0, xz = x.q.x_swapped ? r0 : x.g;
+                const uint32_t bar0 = pair_addr(&full[0], 0);
+                for (int kb = 0; kb < nkb; ++kb) {
                     if (!mbar_wait(&empty[s], ph ^ 1u, ctx, kStatusPairEmpty)) goto done;
                     unsigned char* st = smem + s * kPairStageBytes;
-                    if (rank == 0) mbar_arrive_expect_tx(&full[s], 2 * kPairStageBytes);
-                    const uint32_t bar = pair_addr(&full[s], 0);
-                    if (p.w_swapped) pair_tensor_load(st, &p.tm_w, kb * kPK, g, f0, bar);
-                    else pair_tensor_load(st, &p.tm_w, kb * kPK, f0, g, bar);
-                    if (p.x_swapped) pair_tensor_load(st + kPairABytes, &p.tm_x, kb * kPK, g, r0, bar);
-                    else pair_tensor_load(st + kPairABytes, &p.tm_x, kb * kPK, r0, g, bar);
+                    if (rank == 0) mbar_arrive_expect_tx(&full[s], tx);
+                    pair_tensor_load(st, mw, kb * kPK, wy, wz, bar0 + 8 * s);
+                    pair_tensor_load(st + kPairABytes, mx, kb * kPK, xy, xz, bar0 + 8 * s);
                     if (++s == kPairStages) {
                         s = 0;
                         ph ^= 1u;
@@ -154,66 +191,89 @@ __global__ void __launch_bounds__(kPairThreads, 1) proj_gemm_pair_kernel(const _
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
-            constexpr uint32_t idesc = tc::idesc_bf16(2 * kPM, kPN, 0, 0, 0);
+        if (rank == 0) {
+            const uint32_t leader = tc::elect_one();
             int s = 0, buf = 0;
             uint32_t ph = 0, acc_ph[2] = {0, 0};
             for (long long t = tile0; t < p.tiles; t += tile_step) {
-                if (!mbar_wait(&acc_empty[buf], acc_ph[buf] ^ 1u, ctx, kStatusPairAccEmpty)) goto done;
-                tc::fence_after_sync();
-                const uint32_t d = tm + (uint32_t)(buf * kPN);
-                for (int kb = 0; kb < p.kblocks; ++kb) {
-                    if (!mbar_wait(&full[s], ph, ctx, kStatusPairFull)) goto done;
+                const PairTile x = pair_tile(p, t);
+                const uint32_t idesc = tc::idesc_bf16(2 * kPM, 0, 0, 0, 0) | ((uint32_t)(x.q.row_tile >> 3) << 17);
+                const int segments = x.q.segments, seg_kb = x.q.kblocks / segments;
+                for (int seg = 0; seg < segments; ++seg) {
+                    if (!tc::warp_all(mbar_wait(&acc_empty[buf], acc_ph[buf] ^ 1u, ctx, kStatusPairAccEmpty))) goto done;
                     tc::fence_after_sync();
-                    const unsigned char* st = smem + s * kPairStageBytes;
+                    const uint32_t d = tm + (uint32_t)(buf * kPN);
+                    for (int kb = 0; kb < seg_kb; ++kb) {
+                        if (!tc::warp_all(mbar_wait(&full[s], ph, ctx, kStatusPairFull))) goto done;
+                        tc::fence_after_sync();
+                        const unsigned char* st = smem + s * kPairStageBytes;
 #pragma unroll
-                    for (int i = 0; i < kPK / 16; ++i)
-                        pair_mma(d, tc::desc_sw128_kmajor(st, kPM, 16 * i), tc::desc_sw128_kmajor(st + kPairABytes, kPN / 2, 16 * i), idesc, kb > 0 || i > 0);
-                    pair_commit(smem_u32(&empty[s]));
-                    pair_commit(pair_addr(&empty[s], 1));
-                    if (++s == kPairStages) {
-                        s = 0;
-                        ph ^= 1u;
+                        for (int i = 0; i < kPK / 16; ++i)
+                            pair_mma(leader, d, tc::desc_sw128_kmajor(st, kPM, 16 * i), tc::desc_sw128_kmajor(st + kPairABytes, kPN / 2, 16 * i), idesc, kb > 0 || i > 0);
+                        pair_commit(leader, &empty[s]);
+                        if (++s == kPairStages) {
+                            s = 0;
+                            ph ^= 1u;
+                        }
                     }
+                    pair_commit(leader, &acc_full[buf]);
+                    acc_ph[buf] ^= 1u;
+                    buf ^= 1;
+                    if (leader) ctl[0] = ctl[0] + 1u;
                 }
-                pair_commit(smem_u32(&acc_full[buf]));
-                pair_commit(pair_addr(&acc_full[buf], 1));
-                acc_ph[buf] ^= 1u;
-                buf ^= 1;
-                ctl[0] = ctl[0] + 1u;
             }
         }
     } else {
-        const int q = warp & 3;
-        int buf = 0;
+        const int q = warp & 3;                             // the TMEM lane quarter this warp may read
+        const int set = (warp - 2) >> 2;                    // two sets of four warps share a tile's rows, 32 at a time in turn
+        const int side = q >> 1, fl = (q & 1) * 32 + lane;  // feature fl of the block's 64-feature box `side`
+        const int bar = 1 + set * 2 + side;                 // the two warps that fill a box together
+        unsigned char* boxes = smem + oPairOut + (set * 2 + side) * 2 * kOutBuf;
+        const bool issuer = (q & 1) == 0 && lane == 0;      // issues the boxes' tensor stores
+        int buf = 0, out_buf = 0;
         uint32_t acc_ph[2] = {0, 0};
-        for (long long t = tile0; t < p.tiles; t += tile_step) {
-            const int rt = (int)(t % p.r_tiles);
-            const long long u = t / p.r_tiles;
-            const int nt = (int)(u % p.n_tiles), g = (int)(u / p.n_tiles);
-            if (!mbar_wait(&acc_full[buf], acc_ph[buf], ctx, kStatusPairAccFull)) goto done;
-            acc_ph[buf] ^= 1u;
-            tc::fence_after_sync();
-            const int f = nt * 2 * kPM + (int)rank * kPM + q * 32 + lane;
-            const bool f_ok = f < p.n;
-            const long long row0 = (long long)rt * kPN;
-            unsigned char* base = reinterpret_cast<unsigned char*>(p.out) + ((long long)g * p.o_gstride + f) * (p.out_f32 ? 4 : 2);
-#pragma unroll 1
-            for (int c0 = 0; c0 < kPN; c0 += 16) {
-                uint32_t r[16];
-                tc::tmem_ld16(tc::tmem_addr(tm, q, buf * kPN + c0), r);
-                tc::tmem_ld_wait();
-                if (f_ok) {
+        // The tile's rows c0 .. c0 + 31 (those below row_tile) out: lane = feature, v[j] = row c0 + j.
+        auto emit = [&](const PairTile& x, int c0, const float (&v)[kChunk]) {
+            const long long row0 = (long long)x.rt * x.q.row_tile + c0;
+            const int f0 = x.nt * 2 * kPM + (int)rank * kPM + side * 64;
+            if (row0 >= x.q.rows) return;  // the whole chunk is past the last row (the same for every thread)
+            if (x.q.tensor_out) {
+                unsigned char* box = boxes + out_buf * kOutBuf;
+                out_buf ^= 1;
+                if (issuer) bulk_wait_read<1>();  // this buffer's last stores have been read
+                named_bar_sync(bar, 64);
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) {
-                        const long long row = row0 + c0 + j;
-                        if (row < p.rows) {
-                            if (p.out_f32) *reinterpret_cast<float*>(base + row * p.ldo * 4) = __uint_as_float(r[j]);
-                            else *reinterpret_cast<uint16_t*>(base + row * p.ldo * 2) = f32_to_bf16_bits(__uint_as_float(r[j]));
+                for (int j = 0; j < kChunk; j += 2) {
+                    const uint32_t two = tc::bf16x2(v[j], v[j + 1]);
+                    *reinterpret_cast<uint16_t*>(box + j * 128 + (((fl >> 3) ^ (j & 7)) << 4) + (fl & 7) * 2) = (uint16_t)two;
+                    *reinterpret_cast<uint16_t*>(box + (j + 1) * 128 + (((fl >> 3) ^ ((j + 1) & 7)) << 4) + (fl & 7) * 2) = (uint16_t)(two >> 16);
+                }
+                fence_proxy_async_smem();
+                named_bar_sync(bar, 64);
+                if (issuer) {
+                    if (f0 < x.q.n)  // features and rows past the extents are clipped by the copy
+#pragma unroll
+                        for (int half = 0; half < 2; ++half) {
+                            if (c0 + half * kBoxRows >= x.q.row_tile || row0 + half * kBoxRows >= x.q.rows) break;
+                            const void* src = box + half * kBoxRows * 128;
+                            if (x.q.out_swapped) tensor_store_3d(&x.q.tm_out, f0, x.g, (int)row0 + half * kBoxRows, src);
+                            else tensor_store_3d(&x.q.tm_out, f0, (int)row0 + half * kBoxRows, x.g, src);
                         }
+                    bulk_commit();
+                }
+            } else if (f0 + fl < x.q.n) {
+                unsigned char* base = reinterpret_cast<unsigned char*>(x.q.out) + ((long long)x.g * x.q.o_gstride + f0 + fl) * (x.q.out_f32 ? 4 : 2);
+#pragma unroll
+                for (int j = 0; j < kChunk; ++j) {
+                    const long long row = row0 + j;
+                    if (row < x.q.rows && c0 + j < x.q.row_tile) {
+                        if (x.q.out_f32) *reinterpret_cast<float*>(base + row * x.q.ldo * 4) = v[j];
+                        else *reinterpret_cast<uint16_t*>(base + row * x.q.ldo * 2) = f32_to_bf16_bits(v[j]);
                     }
                 }
             }
+        };
+        auto release = [&] {
             tc::fence_before_sync();
             __syncwarp();
             if (lane == 0) {
@@ -222,7 +282,57 @@ __global__ void __launch_bounds__(kPairThreads, 1) proj_gemm_pair_kernel(const _
                 ctl[0] = ctl[0] + 1u;
             }
             buf ^= 1;
+        };
+        for (long long t = tile0; t < p.tiles; t += tile_step) {
+            const PairTile x = pair_tile(p, t);
+            // The warps of a box meet at its barrier: they decide together whether an accumulator came.
+            auto arrived = [&] {
+                const bool ok = mbar_wait(&acc_full[buf], acc_ph[buf], ctx, kStatusPairAccFull);
+                acc_ph[buf] ^= 1u;
+                const bool all = named_bar_all(bar, 64, ok);
+                tc::fence_after_sync();
+                return all;
+            };
+            if (x.q.segments == 1) {
+                if (!arrived()) goto done;
+                for (int c0 = set * kChunk; c0 < x.q.row_tile; c0 += 2 * kChunk) {
+                    uint32_t r[kChunk];
+                    tc::tmem_ld32(tc::tmem_addr(tm, q, buf * kPN + c0), r);
+                    tc::tmem_ld_wait();
+                    float v[kChunk];
+#pragma unroll
+                    for (int j = 0; j < kChunk; ++j) v[j] = __uint_as_float(r[j]);
+                    emit(x, c0, v);
+                }
+                release();
+            } else {
+                float sum[kSplitRows / kChunk / 2][kChunk];
+                for (int seg = 0; seg < x.q.segments; ++seg) {
+                    if (!arrived()) goto done;
+#pragma unroll
+                    for (int c = 0; c < kSplitRows / kChunk / 2; ++c) {
+                        const int c0 = (2 * c + set) * kChunk;
+                        if (c0 >= x.q.row_tile) break;
+#pragma unroll
+                        for (int j0 = 0; j0 < kChunk; j0 += 16) {
+                            uint32_t r[16];
+                            tc::tmem_ld16(tc::tmem_addr(tm, q, buf * kPN + c0 + j0), r);
+                            tc::tmem_ld_wait();
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) sum[c][j0 + j] = seg == 0 ? __uint_as_float(r[j]) : sum[c][j0 + j] + __uint_as_float(r[j]);
+                        }
+                    }
+                    release();
+                }
+#pragma unroll
+                for (int c = 0; c < kSplitRows / kChunk / 2; ++c) {
+                    const int c0 = (2 * c + set) * kChunk;
+                    if (c0 >= x.q.row_tile) break;
+                    emit(x, c0, sum[c]);
+                }
+            }
         }
+        if (issuer) bulk_wait_all<0>();
     }
 done:
     // After an abort, copies into this block's shared memory may still be in flight: give them a bounded time.
@@ -240,9 +350,7 @@ done:
 
 }  // namespace
 
-// Declared in kda_internal.h: the tensor maps are built by the caller (proj_gemm.cu), boxes of 128 rows each.
-int proj_gemm_pair_launch(const CUtensorMap& tm_w, int w_swapped, const CUtensorMap& tm_x, int x_swapped, void* out, long long ldo, long long o_gstride,
-                          int groups, int rows, int n, int k, int out_f32, int* status, cudaStream_t stream) {
+int proj_gemm_pair_launch(const PairProblem* problems, int n, int* status, cudaStream_t stream) {
     static int configured_dev = -1;
     int dev = 0;
     cudaGetDevice(&dev);
@@ -252,20 +360,9 @@ int proj_gemm_pair_launch(const CUtensorMap& tm_w, int w_swapped, const CUtensor
         configured_dev = dev;
     }
     PairParams p{};
-    p.tm_w = tm_w;
-    p.tm_x = tm_x;
-    p.w_swapped = w_swapped;
-    p.x_swapped = x_swapped;
-    p.out = out;
-    p.ldo = ldo;
-    p.o_gstride = groups > 1 ? o_gstride : 0;
-    p.rows = rows;
-    p.n = n;
-    p.kblocks = k / kPK;
-    p.out_f32 = out_f32;
-    p.n_tiles = (n + 2 * kPM - 1) / (2 * kPM);
-    p.r_tiles = (rows + kPN - 1) / kPN;
-    p.tiles = (long long)groups * p.n_tiles * p.r_tiles;
+    for (int i = 0; i < n; ++i) p.problem[i] = problems[i];
+    p.tiles0 = problems[0].tiles;
+    p.tiles = p.tiles0 + (n > 1 ? problems[1].tiles : 0);
     p.status = status;
     const long long pairs_cap = sm_count() / 2;
     const long long pairs = p.tiles < pairs_cap ? p.tiles : pairs_cap;
@@ -274,13 +371,15 @@ int proj_gemm_pair_launch(const CUtensorMap& tm_w, int w_swapped, const CUtensor
     cfg.blockDim = dim3(kPairThreads);
     cfg.dynamicSmemBytes = kPairSmem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     return (int)cudaLaunchKernelEx(&cfg, proj_gemm_pair_kernel, p);
 }
 

@@ -65,6 +65,16 @@ __device__ __forceinline__ constexpr uint32_t idesc_bf16(int M, int N, int a_mn_
            ((uint32_t)b_mn_major << 16) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
+// One lane of a converged warp (always the same one): 1 there, 0 in the others.
+__device__ __forceinline__ uint32_t elect_one() {
+    uint32_t is;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(is));
+    return is;
+}
+// Whether `ok` holds in every lane, as a value the compiler knows to be the same in all of them: code behind a branch on it
+// stays converged, so what it computes from uniform inputs stays in uniform registers.
+__device__ __forceinline__ bool warp_all(bool ok) { return __all_sync(0xffffffffu, ok); }
+
 // D[tmem] (+)= A[smem] * B[smem], issued by one thread.
 __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, bool accumulate) {
     asm volatile(
@@ -76,6 +86,24 @@ __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a_desc, uint6
 // Makes `bar` complete once every MMA issued so far by this thread has finished (implies fence::before_thread_sync).
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
+// The same two issued by a converged warp with `leader` set in one lane (elect_one).  Inside an `if` of one lane the compiler
+// moves every operand of every MMA over from that lane's registers, about 90 cycles an instruction; issued so, descriptors
+// computed from uniform values are uniform registers already.
+__device__ __forceinline__ void mma_bf16_if(uint32_t leader, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, bool accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"((uint32_t)accumulate), "r"(leader)
+        : "memory");
+}
+__device__ __forceinline__ void mma_commit_if(uint32_t leader, uint64_t* bar) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar)),
+        "r"(leader)
+        : "memory");
 }
 
 // ---- TMEM <-> registers: 32 lanes x 32 columns of 32 bits per warp; thread l of warp w touches lane 32*(w%4)+l -------

@@ -58,10 +58,20 @@ SIGNATURES = {
     "glm53f_kda_store_words": (I32, [P, P, I32, P]),
     # include/glm53f_proj.h: the projections' GEMM (the arguments of glm53f_fwd_gemv_bf16 without its split-K scratch)
     "glm53f_kda_proj_bf16": (I32, [P, I64, I64, P, I64, I64, I32, I32, I32, I32, P, I32, I64, I64, P]),
+    "glm53f_kda_proj_bf16_many": (I32, [P, I32, P]),
 }
 
+
+class ProjJob(C.Structure):
+    """glm53f_proj_job (include/glm53f_proj.h)."""
+
+    _fields_ = [("x", P), ("ldx", I64), ("x_gstride", I64), ("w", P), ("ldw", I64), ("w_gstride", I64), ("groups", I32), ("rows", I32), ("n", I32),
+                ("k", I32), ("out", P), ("out_f32", I32), ("ldo", I64), ("o_gstride", I64)]
+
+
+
 # The reference's thirteen (crates/glm53f-kda/tests/provenance.rs:41-69 asserts exactly these).
-REFERENCE_SYMBOLS = [n for n in SIGNATURES if n.startswith("glm53f_kda_") and "_core_" not in n and "_gather_" not in n and n not in ("glm53f_kda_device_status", "glm53f_kda_debug_wait_test", "glm53f_kda_prefill_mode", "glm53f_kda_verify_mode", "glm53f_kda_commit_mode", "glm53f_kda_mark_copy", "glm53f_kda_mark_copy_slots", "glm53f_kda_mark_copy_list", "glm53f_kda_store_words", "glm53f_kda_proj_bf16", "glm53f_kda_chain_commit_batch")]
+REFERENCE_SYMBOLS = [n for n in SIGNATURES if n.startswith("glm53f_kda_") and "_core_" not in n and "_gather_" not in n and n not in ("glm53f_kda_device_status", "glm53f_kda_debug_wait_test", "glm53f_kda_prefill_mode", "glm53f_kda_verify_mode", "glm53f_kda_commit_mode", "glm53f_kda_mark_copy", "glm53f_kda_mark_copy_slots", "glm53f_kda_mark_copy_list", "glm53f_kda_store_words", "glm53f_kda_proj_bf16", "glm53f_kda_proj_bf16_many", "glm53f_kda_chain_commit_batch")]
 
 
 def library_path() -> str:

@@ -55,6 +55,14 @@ def bf16(x: torch.Tensor, ldx: int, x_gstride: int, w: Bf16Mat, rows: int, out: 
     """out[g][m][o] = sum_k x[g][m][k] w[g][o][k] (Gemm::bf16, gemm.rs:212-235); offsets in elements of x / out."""
     if rows == 0:
         return
+    j = _job(x, ldx, x_gstride, w, rows, out, ldo, o_gstride, out_f32, x_offset, out_offset)
+    stream = torch.cuda.current_stream().cuda_stream
+    code = ffi.glm53f_kda_proj_bf16(*(getattr(j, f) for f, _ in j._fields_), stream)
+    _launched(code, "glm53f_kda_proj_bf16")
+
+
+def _job(x, ldx, x_gstride, w: Bf16Mat, rows, out, ldo, o_gstride, out_f32=False, x_offset=0, out_offset=0) -> ffi.ProjJob:
+    """The checked arguments of one GEMM."""
     if x.dtype not in (torch.bfloat16, torch.int16, torch.uint16) or w.t.dtype not in (torch.bfloat16, torch.int16, torch.uint16):
         raise Invalid("x and the weight are bf16")
     if out.dtype != (torch.float32 if out_f32 else x.dtype) and not (not out_f32 and out.element_size() == 2):
@@ -63,10 +71,8 @@ def bf16(x: torch.Tensor, ldx: int, x_gstride: int, w: Bf16Mat, rows: int, out: 
     need_o = out_offset + (w.groups - 1) * o_gstride + (rows - 1) * ldo + w.n
     if x.numel() < need_x or out.numel() < need_o or w.t.numel() < (w.groups - 1) * w.gstride + (w.n - 1) * w.ld + w.k:
         raise Invalid("a buffer is smaller than the shapes named")
-    stream = torch.cuda.current_stream().cuda_stream
-    code = ffi.glm53f_kda_proj_bf16(x.data_ptr() + 2 * x_offset, ldx, x_gstride, w.t.data_ptr(), w.ld, w.gstride, w.groups, rows, w.n, w.k,
-                                    out.data_ptr() + out_offset * out.element_size(), 1 if out_f32 else 0, ldo, o_gstride, stream)
-    _launched(code, "glm53f_kda_proj_bf16")
+    return ffi.ProjJob(x.data_ptr() + 2 * x_offset, ldx, x_gstride, w.t.data_ptr(), w.ld, w.gstride, w.groups, rows, w.n, w.k,
+                       out.data_ptr() + out_offset * out.element_size(), 1 if out_f32 else 0, ldo, o_gstride)
 
 
 @dataclass
@@ -83,6 +89,19 @@ class KdaProjW:
 def kda_input_projections(normed: torch.Tensor, rows: int, w: KdaProjW, p: torch.Tensor, fga: torch.Tensor, ag: torch.Tensor) -> None:
     """The three GEMMs of a KDA layer's input (forward.rs:3494-3542): p [rows][24,640] = normed . qkvb^T; fga
     [rows][256] = normed . fga^T; ag [rows][2 x 8192] = per group g, fga[:, 128 g : 128 g + 128] . fgb[g]^T."""
-    bf16(normed, HIDDEN, 0, w.qkvb, rows, p, KDA_P_COLS, 0)
-    bf16(normed, HIDDEN, 0, w.fga, rows, fga, 2 * KDA_DIM, 0)
+    if rows == 0:
+        return
+    both = (_job(normed, HIDDEN, 0, w.fga, rows, fga, 2 * KDA_DIM, 0), _job(normed, HIDDEN, 0, w.qkvb, rows, p, KDA_P_COLS, 0))
+    apart = _disjoint(p, fga) and _disjoint(p, normed) and _disjoint(fga, normed)
+    stream = torch.cuda.current_stream().cuda_stream
+    if apart:  # the first gate factor beside the fused projection of the same rows
+        _launched(ffi.glm53f_kda_proj_bf16_many((ffi.ProjJob * 2)(*both), 2, stream), "glm53f_kda_proj_bf16_many")
+    else:
+        bf16(normed, HIDDEN, 0, w.qkvb, rows, p, KDA_P_COLS, 0)
+        bf16(normed, HIDDEN, 0, w.fga, rows, fga, 2 * KDA_DIM, 0)
     bf16(fga, 2 * KDA_DIM, KDA_DIM, w.fgb, rows, ag, 2 * KDA_WIDTH, KDA_WIDTH)
+
+
+def _disjoint(a: torch.Tensor, b: torch.Tensor) -> bool:
+    lo, hi = sorted(((t.data_ptr(), t.data_ptr() + t.numel() * t.element_size()) for t in (a, b)))
+    return lo[1] <= hi[0]

@@ -39,6 +39,22 @@ int32_t glm53f_kda_proj_bf16(const uint16_t* x, int64_t ldx, int64_t x_gstride, 
                              int64_t w_gstride, int32_t groups, int32_t rows, int32_t n, int32_t k, void* out,
                              int32_t out_f32, int64_t ldo, int64_t o_gstride, glm53f_stream_t stream);
 
+/* Several GEMMs that do not depend on one another (none reads or writes what another writes), each as
+ * glm53f_kda_proj_bf16 with the job's fields as its arguments: neighbours share a launch or run beside one another (the fused
+ * [q|k|v|b] projection and the first gate factor of the same rows).  `jobs` is read during the call.  Every job is checked
+ * before anything is launched. */
+typedef struct glm53f_proj_job {
+    const uint16_t* x;
+    int64_t ldx, x_gstride;
+    const uint16_t* w;
+    int64_t ldw, w_gstride;
+    int32_t groups, rows, n, k;
+    void* out;
+    int32_t out_f32;
+    int64_t ldo, o_gstride;
+} glm53f_proj_job;
+int32_t glm53f_kda_proj_bf16_many(const glm53f_proj_job* jobs, int32_t count, glm53f_stream_t stream);
+
 #ifdef __cplusplus
 }
 #endif
