@@ -165,11 +165,13 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
         group_sync();
         tc::fence_after_sync();
     };
-    auto mma_issue = [&](uint64_t* bar, auto&& issue) {
-        if (gt == 0) {
-            issue();
-            tc::mma_commit(bar);
-            atomicAdd(const_cast<uint32_t*>(ctx.progress), 1u);
+    auto mma_issue = [&](uint64_t* bar, auto&& issue) {  // by one lane of the group's first warp, the warp converged
+        if (gw == 0) {
+            const uint32_t leader = tc::elect_one();
+            issue(leader);
+            tc::mma_commit_if(leader, bar);
+            if (leader) atomicAdd(const_cast<uint32_t*>(ctx.progress), 1u);
+            __syncwarp();
         }
     };
     uint32_t raw_phase = 0, mma_phase = 0, lm_phase = 0;
@@ -333,24 +335,26 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
         }
         }
         publish();
-        // ---- 3a. L^T, one block column of 16 rows i a warp: [64 j x 16 i] = column side (tile I) x row side (block I)^T.  Eight
-        // threads (lane 0 of every warp) issue the eight small products of L^T and M^T, so none of them issues for long; each
+        // ---- 3a. L^T, one block column of 16 rows i a warp: [64 j x 16 i] = column side (tile I) x row side (block I)^T.  The
+        // eight warps issue the eight small products of L^T and M^T (one lane each), so none of them issues for long; each
         // commits to the same barrier, which completes when all eight have.
-        if (lane == 0 && gw < 4) {
+        if (gw < 4) {
+            const uint32_t leader = tc::elect_one();
             if (narrow) {  // one product, all 64 rows i at once, row side Kg (a commit with nothing pending arrives at once)
                 constexpr uint32_t id64 = tc::idesc_bf16(64, 64, 0, 0, 0);
                 if (gw == 0)
                     for (int k0 = 0; k0 < DK; k0 += 16)
-                        tc::mma_bf16(tm + gcL, tc::desc_sw128_kmajor(gs + gKc + kc_tile(3), CH, k0), tc::desc_sw128_kmajor(gs + gK, CH, k0), id64, k0 > 0);
+                        tc::mma_bf16_if(leader, tm + gcL, tc::desc_sw128_kmajor(gs + gKc + kc_tile(3), CH, k0), tc::desc_sw128_kmajor(gs + gK, CH, k0), id64, k0 > 0);
             } else {
             constexpr uint32_t id = tc::idesc_bf16(64, 16, 0, 0, 0);
             const int I = gw;
             const unsigned char* kct = gs + gKc + kc_tile(I);
             for (int k0 = 0; k0 < DK; k0 += 16)
-                tc::mma_bf16(tm + gcL + 16 * I, tc::desc_sw128_kmajor(kct, 16 * (I + 1), k0), tc::desc_sw128_kmajor(gs + gKb + I * 2048, CH, k0), id, k0 > 0);
+                tc::mma_bf16_if(leader, tm + gcL + 16 * I, tc::desc_sw128_kmajor(kct, 16 * (I + 1), k0), tc::desc_sw128_kmajor(gs + gKb + I * 2048, CH, k0), id, k0 > 0);
             }
-            tc::mma_commit(bar_lm);
-            atomicAdd(const_cast<uint32_t*>(ctx.progress), 1u);
+            tc::mma_commit_if(leader, bar_lm);
+            if (leader) atomicAdd(const_cast<uint32_t*>(ctx.progress), 1u);
+            __syncwarp();
         }
         // ---- 3b. the tiles made from q, while L^T runs: row side Qgb = Q a (over Q); Qg = Q exp(G) out to the workspace -------
 #pragma unroll
@@ -374,21 +378,23 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
         }
         publish();
         // ---- 3c. M^T the same way, by the other four warps ------------------------------------------------------------------------
-        if (lane == 0 && gw >= 4) {
+        if (gw >= 4) {
+            const uint32_t leader = tc::elect_one();
             if (narrow) {
                 constexpr uint32_t id64 = tc::idesc_bf16(64, 64, 0, 0, 0);
                 if (gw == 4)
                     for (int k0 = 0; k0 < DK; k0 += 16)
-                        tc::mma_bf16(tm + gcM, tc::desc_sw128_kmajor(gs + gKc + kc_tile(3), CH, k0), tc::desc_sw128_kmajor(gs + gQ, CH, k0), id64, k0 > 0);
+                        tc::mma_bf16_if(leader, tm + gcM, tc::desc_sw128_kmajor(gs + gKc + kc_tile(3), CH, k0), tc::desc_sw128_kmajor(gs + gQ, CH, k0), id64, k0 > 0);
             } else {
             constexpr uint32_t id = tc::idesc_bf16(64, 16, 0, 0, 0);
             const int I = gw - 4;
             const unsigned char* kct = gs + gKc + kc_tile(I);
             for (int k0 = 0; k0 < DK; k0 += 16)
-                tc::mma_bf16(tm + gcM + 16 * I, tc::desc_sw128_kmajor(kct, 16 * (I + 1), k0), tc::desc_sw128_kmajor(gs + gQ + I * 2048, CH, k0), id, k0 > 0);
+                tc::mma_bf16_if(leader, tm + gcM + 16 * I, tc::desc_sw128_kmajor(kct, 16 * (I + 1), k0), tc::desc_sw128_kmajor(gs + gQ + I * 2048, CH, k0), id, k0 > 0);
             }
-            tc::mma_commit(bar_lm);
-            atomicAdd(const_cast<uint32_t*>(ctx.progress), 1u);
+            tc::mma_commit_if(leader, bar_lm);
+            if (leader) atomicAdd(const_cast<uint32_t*>(ctx.progress), 1u);
+            __syncwarp();
         }
         if (!mma_wait(bar_lm, lm_phase)) break;
 
@@ -452,16 +458,16 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
         publish();
 
         // ---- 6. W = T' Kg (bf16 T'), U = T' V (T' hi + lo) -------------------------------------------------------------------
-        mma_issue(bar_mma, [&] {
+        mma_issue(bar_mma, [&](uint32_t leader) {
             constexpr uint32_t id = tc::idesc_bf16(64, 128, 0, 1, 0);
             const unsigned char* tph = gs + gTp;
             const unsigned char* tpl = gs + gTp + kBox;
             for (int k0 = 0; k0 < CH; k0 += 16)
-                tc::mma_bf16(tm + gcW, tc::desc_sw128_kmajor(tph, CH, k0), tc::desc_sw128_mnmajor(gs + gK, CH, k0), id, k0 > 0);
+                tc::mma_bf16_if(leader, tm + gcW, tc::desc_sw128_kmajor(tph, CH, k0), tc::desc_sw128_mnmajor(gs + gK, CH, k0), id, k0 > 0);
             for (int k0 = 0; k0 < CH; k0 += 16)
-                tc::mma_bf16(tm + gcU, tc::desc_sw128_kmajor(tph, CH, k0), tc::desc_sw128_mnmajor(gs + gV, CH, k0), id, k0 > 0);
+                tc::mma_bf16_if(leader, tm + gcU, tc::desc_sw128_kmajor(tph, CH, k0), tc::desc_sw128_mnmajor(gs + gV, CH, k0), id, k0 > 0);
             for (int k0 = 0; k0 < CH; k0 += 16)
-                tc::mma_bf16(tm + gcU, tc::desc_sw128_kmajor(tpl, CH, k0), tc::desc_sw128_mnmajor(gs + gV, CH, k0), id, true);
+                tc::mma_bf16_if(leader, tm + gcU, tc::desc_sw128_kmajor(tpl, CH, k0), tc::desc_sw128_mnmajor(gs + gV, CH, k0), id, true);
         });
         if (!mma_wait(bar_mma, mma_phase)) break;
         // Nothing of this item is left in the group's shared memory: the loader may bring the next item in.
@@ -709,11 +715,13 @@ __device__ void state_role(const SpParams& p, unsigned char* smem, const uint32_
 
     uint32_t mma_phase = 0;
     bool alive = true;
-    auto mma_issue = [&](auto&& issue) {
-        if (tid == 0) {
-            issue();
-            tc::mma_commit(bar_mma);
-            atomicAdd(const_cast<uint32_t*>(ctl), 1u);
+    auto mma_issue = [&](auto&& issue) {  // by one lane of warp 0, the warp converged (tc::mma_bf16_if)
+        if (warp == 0) {
+            const uint32_t leader = tc::elect_one();
+            issue(leader);
+            tc::mma_commit_if(leader, bar_mma);
+            if (leader) atomicAdd(const_cast<uint32_t*>(ctl), 1u);
+            __syncwarp();
         }
     };
     auto mma_wait = [&]() -> bool {
@@ -751,13 +759,13 @@ __device__ void state_role(const SpParams& p, unsigned char* smem, const uint32_
         }
         publish_operands();
         const uint32_t tO = (c & 1) ? tQS1 : tQS;
-        mma_issue([&] {
+        mma_issue([&](uint32_t leader) {
             constexpr uint32_t id = tc::idesc_bf16(64, NV, 0, 1, 0), idn = tc::idesc_bf16(64, NV, 0, 1, 1);
             if (wk.emit)
                 for (int k0 = 0; k0 < DK; k0 += 16)
-                    tc::mma_bf16(tm + tO, tc::desc_kmajor_bf16(smem + sSlot + wQg, CH, 0, k0), tc::desc_mnmajor_bf16(smem + sS16, 128, 0, k0), id, k0 > 0);
+                    tc::mma_bf16_if(leader, tm + tO, tc::desc_kmajor_bf16(smem + sSlot + wQg, CH, 0, k0), tc::desc_mnmajor_bf16(smem + sS16, 128, 0, k0), id, k0 > 0);
             for (int k0 = 0; k0 < DK; k0 += 16)
-                tc::mma_bf16(tm + tD, tc::desc_kmajor_bf16(smem + sSlot + wW, CH, 0, k0), tc::desc_mnmajor_bf16(smem + sS16, 128, 0, k0), idn, k0 > 0);
+                tc::mma_bf16_if(leader, tm + tD, tc::desc_kmajor_bf16(smem + sSlot + wW, CH, 0, k0), tc::desc_mnmajor_bf16(smem + sS16, 128, 0, k0), idn, k0 > 0);
         });
         return true;
     };
@@ -824,19 +832,19 @@ __device__ void state_role(const SpParams& p, unsigned char* smem, const uint32_
 
         // ---- O = QS + M D;  S += Kdec^T D (hi hi + hi lo + lo hi) ------------------------------------------------------------
         if (!mbar_wait(&full[2], par, ctx, kStatusWaitPrefill)) { alive = false; break; }
-        mma_issue([&] {
+        mma_issue([&](uint32_t leader) {
             constexpr uint32_t idm = tc::idesc_bf16(64, NV, 1, 1, 0), ids = tc::idesc_bf16(128, NV, 1, 1, 0);  // M arrives with its rows contiguous
             const unsigned char* kdhi = smem + sSlot + wKdHi;
             const unsigned char* kdlo = smem + sSlot + wKdLo;
             if (wk.emit)
                 for (int k0 = 0; k0 < CH; k0 += 16)
-                    tc::mma_bf16(tm + tO, tc::desc_mnmajor_bf16(smem + sSlot + wMm, CH, 0, k0), tc::desc_mnmajor_bf16(smem + sDhi, CH, 0, k0), idm, true);
+                    tc::mma_bf16_if(leader, tm + tO, tc::desc_mnmajor_bf16(smem + sSlot + wMm, CH, 0, k0), tc::desc_mnmajor_bf16(smem + sDhi, CH, 0, k0), idm, true);
             for (int k0 = 0; k0 < CH; k0 += 16)
-                tc::mma_bf16(tm + tS, tc::desc_mnmajor_bf16(kdhi, CH, 0, k0), tc::desc_mnmajor_bf16(smem + sDhi, CH, 0, k0), ids, true);
+                tc::mma_bf16_if(leader, tm + tS, tc::desc_mnmajor_bf16(kdhi, CH, 0, k0), tc::desc_mnmajor_bf16(smem + sDhi, CH, 0, k0), ids, true);
             for (int k0 = 0; k0 < CH; k0 += 16)
-                tc::mma_bf16(tm + tS, tc::desc_mnmajor_bf16(kdhi, CH, 0, k0), tc::desc_mnmajor_bf16(smem + sDlo, CH, 0, k0), ids, true);
+                tc::mma_bf16_if(leader, tm + tS, tc::desc_mnmajor_bf16(kdhi, CH, 0, k0), tc::desc_mnmajor_bf16(smem + sDlo, CH, 0, k0), ids, true);
             for (int k0 = 0; k0 < CH; k0 += 16)
-                tc::mma_bf16(tm + tS, tc::desc_mnmajor_bf16(kdlo, CH, 0, k0), tc::desc_mnmajor_bf16(smem + sDhi, CH, 0, k0), ids, true);
+                tc::mma_bf16_if(leader, tm + tS, tc::desc_mnmajor_bf16(kdlo, CH, 0, k0), tc::desc_mnmajor_bf16(smem + sDhi, CH, 0, k0), ids, true);
         });
         if (!mma_wait()) { alive = false; break; }
         if (tid == 0) mbar_arrive(&empty[2]);

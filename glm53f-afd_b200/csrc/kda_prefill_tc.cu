@@ -165,12 +165,15 @@ __global__ void __launch_bounds__(kThreadsTc, 1) prefill_tc_kernel(const __grid_
         return;
     }
 
-    // One round of MMAs: thread 0 issues and commits, everybody waits for the tensor core.
+    // One round of MMAs: warp 0 issues (one lane, the warp converged: see tc::mma_bf16_if) and commits, everybody waits for the
+    // tensor core.
     auto mma_round = [&](auto&& issue) -> bool {
-        if (tid == 0) {
-            issue();
-            tc::mma_commit(bar_mma);
-            atomicAdd(const_cast<uint32_t*>(ctl), 1u);
+        if (warp == 0) {
+            const uint32_t leader = tc::elect_one();
+            issue(leader);
+            tc::mma_commit_if(leader, bar_mma);
+            if (leader) atomicAdd(const_cast<uint32_t*>(ctl), 1u);
+            __syncwarp();
         }
         if (!mbar_wait(bar_mma, mma_phase, ctx, kStatusWaitPrefill)) return false;
         mma_phase ^= 1u;
@@ -298,13 +301,13 @@ __global__ void __launch_bounds__(kThreadsTc, 1) prefill_tc_kernel(const __grid_
             }
             publish_operands();
             if (tid == 0 && s + CH < T) mbar_arrive(bar_free);  // the staging area is free for the next chunk's rows
-            if (!mma_round([&] {
+            if (!mma_round([&](uint32_t leader) {
                     constexpr uint32_t id = tc::idesc_bf16(64, 64, 0, 0, 0);
                     const unsigned char* kit = smem + oKc + kc_tile(3);
                     for (int k0 = 0; k0 < DK; k0 += 16)
-                        tc::mma_bf16(tm + cL, tc::desc_kmajor_bf16(kit, CH, 0, k0), tc::desc_kmajor_bf16(smem + oKg, CH, 0, k0), id, k0 > 0);
+                        tc::mma_bf16_if(leader, tm + cL, tc::desc_kmajor_bf16(kit, CH, 0, k0), tc::desc_kmajor_bf16(smem + oKg, CH, 0, k0), id, k0 > 0);
                     for (int k0 = 0; k0 < DK; k0 += 16)
-                        tc::mma_bf16(tm + cMm, tc::desc_kmajor_bf16(kit, CH, 0, k0), tc::desc_kmajor_bf16(smem + oQg, CH, 0, k0), id, k0 > 0);
+                        tc::mma_bf16_if(leader, tm + cMm, tc::desc_kmajor_bf16(kit, CH, 0, k0), tc::desc_kmajor_bf16(smem + oQg, CH, 0, k0), id, k0 > 0);
                 })) { alive = false; break; }
         } else {
         // ---- 2. operand tiles: lane <-> row, one 16-byte cell (8 channels) at a time.  Row sides Kgb = K a -> oKg, Qgb = Q a ->
@@ -362,15 +365,15 @@ __global__ void __launch_bounds__(kThreadsTc, 1) prefill_tc_kernel(const __grid_
         publish_operands();
 
         // ---- 3. L^T and M^T, one block column of 16 rows i at a time: [64 j x 16 i] = column side (tile I) x row side (block I)^T
-        if (!mma_round([&] {
+        if (!mma_round([&](uint32_t leader) {
                 constexpr uint32_t id = tc::idesc_bf16(64, 16, 0, 0, 0);
                 for (int I = 0; I < 4; ++I) {
                     const unsigned char* kct = smem + oKc + kc_tile(I);
                     const int R = 16 * (I + 1);
                     for (int k0 = 0; k0 < DK; k0 += 16)
-                        tc::mma_bf16(tm + cL + 16 * I, tc::desc_kmajor_bf16(kct, R, 0, k0), tc::desc_kmajor_bf16(smem + oKg, CH, 16 * I, k0), id, k0 > 0);
+                        tc::mma_bf16_if(leader, tm + cL + 16 * I, tc::desc_kmajor_bf16(kct, R, 0, k0), tc::desc_kmajor_bf16(smem + oKg, CH, 16 * I, k0), id, k0 > 0);
                     for (int k0 = 0; k0 < DK; k0 += 16)
-                        tc::mma_bf16(tm + cMm + 16 * I, tc::desc_kmajor_bf16(kct, R, 0, k0), tc::desc_kmajor_bf16(smem + oQg, CH, 16 * I, k0), id, k0 > 0);
+                        tc::mma_bf16_if(leader, tm + cMm + 16 * I, tc::desc_kmajor_bf16(kct, R, 0, k0), tc::desc_kmajor_bf16(smem + oQg, CH, 16 * I, k0), id, k0 > 0);
                 }
             })) { alive = false; break; }
 
@@ -471,14 +474,14 @@ __global__ void __launch_bounds__(kThreadsTc, 1) prefill_tc_kernel(const __grid_
         publish_operands();
 
         // ---- 6. W = T' Kg (bf16 T'), U = T' V (T' hi + lo) -------------------------------------------------------------------
-        if (!mma_round([&] {
+        if (!mma_round([&](uint32_t leader) {
                 constexpr uint32_t id = tc::idesc_bf16(64, 128, 0, 1, 0);
                 for (int k0 = 0; k0 < CH; k0 += 16)
-                    tc::mma_bf16(tm + cW, tc::desc_kmajor_bf16(smem + oTpHi, CH, 0, k0), tc::desc_mnmajor_bf16(smem + oKg, CH, 0, k0), id, k0 > 0);
+                    tc::mma_bf16_if(leader, tm + cW, tc::desc_kmajor_bf16(smem + oTpHi, CH, 0, k0), tc::desc_mnmajor_bf16(smem + oKg, CH, 0, k0), id, k0 > 0);
                 for (int k0 = 0; k0 < CH; k0 += 16)
-                    tc::mma_bf16(tm + cU, tc::desc_kmajor_bf16(smem + oTpHi, CH, 0, k0), tc::desc_mnmajor_bf16(smem + oV, CH, 0, k0), id, k0 > 0);
+                    tc::mma_bf16_if(leader, tm + cU, tc::desc_kmajor_bf16(smem + oTpHi, CH, 0, k0), tc::desc_mnmajor_bf16(smem + oV, CH, 0, k0), id, k0 > 0);
                 for (int k0 = 0; k0 < CH; k0 += 16)
-                    tc::mma_bf16(tm + cU, tc::desc_kmajor_bf16(smem + oTpLo, CH, 0, k0), tc::desc_mnmajor_bf16(smem + oV, CH, 0, k0), id, true);
+                    tc::mma_bf16_if(leader, tm + cU, tc::desc_kmajor_bf16(smem + oTpLo, CH, 0, k0), tc::desc_mnmajor_bf16(smem + oV, CH, 0, k0), id, true);
             })) { alive = false; break; }
 
         // ---- 7. W to bf16 cells; 8. S to bf16 cells (over Kg | Kinv, both dead), the decayed S back to tensor memory ------------
@@ -507,12 +510,12 @@ __global__ void __launch_bounds__(kThreadsTc, 1) prefill_tc_kernel(const __grid_
         publish_operands();
 
         // ---- 9. QS = Qg S;  D = U - W S (negated A, accumulated onto U) ----------------------------------------------------------
-        if (!mma_round([&] {
+        if (!mma_round([&](uint32_t leader) {
                 constexpr uint32_t id = tc::idesc_bf16(64, 128, 0, 1, 0), idn = tc::idesc_bf16(64, 128, 0, 1, 1);
                 for (int k0 = 0; k0 < DK; k0 += 16)
-                    tc::mma_bf16(tm + cQS, tc::desc_kmajor_bf16(smem + oQg, CH, 0, k0), tc::desc_mnmajor_bf16(smem + oS16, 128, 0, k0), id, k0 > 0);
+                    tc::mma_bf16_if(leader, tm + cQS, tc::desc_kmajor_bf16(smem + oQg, CH, 0, k0), tc::desc_mnmajor_bf16(smem + oS16, 128, 0, k0), id, k0 > 0);
                 for (int k0 = 0; k0 < DK; k0 += 16)
-                    tc::mma_bf16(tm + cU, tc::desc_kmajor_bf16(smem + oW, CH, 0, k0), tc::desc_mnmajor_bf16(smem + oS16, 128, 0, k0), idn, true);
+                    tc::mma_bf16_if(leader, tm + cU, tc::desc_kmajor_bf16(smem + oW, CH, 0, k0), tc::desc_mnmajor_bf16(smem + oS16, 128, 0, k0), idn, true);
             })) { alive = false; break; }
 
         // ---- 10. D as bf16 hi + lo cells (over T' | V, both dead) -------------------------------------------------------------------
@@ -540,16 +543,16 @@ __global__ void __launch_bounds__(kThreadsTc, 1) prefill_tc_kernel(const __grid_
         publish_operands();
 
         // ---- 11. O = QS + M D;  S += Kdec^T D (hi hi + hi lo + lo hi) ------------------------------------------------------------------
-        if (!mma_round([&] {
+        if (!mma_round([&](uint32_t leader) {
                 constexpr uint32_t idm = tc::idesc_bf16(64, 128, 1, 1, 0), ids = tc::idesc_bf16(128, 128, 1, 1, 0);  // M has its rows contiguous
                 for (int k0 = 0; k0 < CH; k0 += 16)
-                    tc::mma_bf16(tm + cQS, tc::desc_mnmajor_bf16(smem + oMm, CH, 0, k0), tc::desc_mnmajor_bf16(smem + oDhi, CH, 0, k0), idm, true);
+                    tc::mma_bf16_if(leader, tm + cQS, tc::desc_mnmajor_bf16(smem + oMm, CH, 0, k0), tc::desc_mnmajor_bf16(smem + oDhi, CH, 0, k0), idm, true);
                 for (int k0 = 0; k0 < CH; k0 += 16)
-                    tc::mma_bf16(tm + cS, tc::desc_mnmajor_bf16(smem + oKdHi, CH, 0, k0), tc::desc_mnmajor_bf16(smem + oDhi, CH, 0, k0), ids, true);
+                    tc::mma_bf16_if(leader, tm + cS, tc::desc_mnmajor_bf16(smem + oKdHi, CH, 0, k0), tc::desc_mnmajor_bf16(smem + oDhi, CH, 0, k0), ids, true);
                 for (int k0 = 0; k0 < CH; k0 += 16)
-                    tc::mma_bf16(tm + cS, tc::desc_mnmajor_bf16(smem + oKdHi, CH, 0, k0), tc::desc_mnmajor_bf16(smem + oDlo, CH, 0, k0), ids, true);
+                    tc::mma_bf16_if(leader, tm + cS, tc::desc_mnmajor_bf16(smem + oKdHi, CH, 0, k0), tc::desc_mnmajor_bf16(smem + oDlo, CH, 0, k0), ids, true);
                 for (int k0 = 0; k0 < CH; k0 += 16)
-                    tc::mma_bf16(tm + cS, tc::desc_mnmajor_bf16(smem + oKdLo, CH, 0, k0), tc::desc_mnmajor_bf16(smem + oDhi, CH, 0, k0), ids, true);
+                    tc::mma_bf16_if(leader, tm + cS, tc::desc_mnmajor_bf16(smem + oKdLo, CH, 0, k0), tc::desc_mnmajor_bf16(smem + oDhi, CH, 0, k0), ids, true);
             })) { alive = false; break; }
 
         // ---- 12. outputs: bf16(y), or the gated RMSNorm of bf16(y); a thread holds 32 columns of its row -------------------------------

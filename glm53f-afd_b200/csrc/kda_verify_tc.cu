@@ -285,14 +285,16 @@ __global__ void __launch_bounds__(kVThreads, 3) verify_tc_kernel(const __grid_co
         else cp_async_commit();
 
         // ---- B. L^T and M^T -------------------------------------------------------------------------------------------------
-        if (t == 0) {
+        if (warp == 0) {
+            const uint32_t leader = tc::elect_one();
             constexpr uint32_t id = tc::idesc_bf16(128, WIN, 0, 0, 0);
             for (int k0 = 0; k0 < DK; k0 += 16)
-                tc::mma_bf16(tm, tc::desc_sw128_kmajor(smem + vKc, WIN, k0), tc::desc_sw128_kmajor(smem + vKgb, WIN, k0), id, k0 > 0);
+                tc::mma_bf16_if(leader, tm, tc::desc_sw128_kmajor(smem + vKc, WIN, k0), tc::desc_sw128_kmajor(smem + vKgb, WIN, k0), id, k0 > 0);
             for (int k0 = 0; k0 < DK; k0 += 16)
-                tc::mma_bf16(tm + 16, tc::desc_sw128_kmajor(smem + vKc, WIN, k0), tc::desc_sw128_kmajor(smem + vQgb, WIN, k0), id, k0 > 0);
-            tc::mma_commit(bar);
-            atomicAdd(const_cast<uint32_t*>(ctl), 1u);
+                tc::mma_bf16_if(leader, tm + 16, tc::desc_sw128_kmajor(smem + vKc, WIN, k0), tc::desc_sw128_kmajor(smem + vQgb, WIN, k0), id, k0 > 0);
+            tc::mma_commit_if(leader, bar);
+            if (leader) atomicAdd(const_cast<uint32_t*>(ctl), 1u);
+            __syncwarp();
         }
 #pragma unroll
         for (int r = 0; r < WIN; ++r) *reinterpret_cast<uint16_t*>(smem + vQg + sw_elem(WIN, r, t)) = f32_to_bf16_bits(qe[r]);
@@ -351,14 +353,16 @@ __global__ void __launch_bounds__(kVThreads, 3) verify_tc_kernel(const __grid_co
         tc::fence_after_sync();
 
         // ---- D. (W S)^T and (Qg S)^T: the state tile as it lies in memory is the M operand ---------------------------------------
-        if (t == 0) {
+        if (warp == 0) {
+            const uint32_t leader = tc::elect_one();
             constexpr uint32_t id = tc::idesc_bf16(128, WIN, 0, 0, 0);
             for (int k0 = 0; k0 < DK; k0 += 16)
-                tc::mma_bf16(tm, tc::desc_sw128_kmajor(smem + vS, DV, k0), tc::desc_sw128_kmajor(smem + vW, WIN, k0), id, k0 > 0);
+                tc::mma_bf16_if(leader, tm, tc::desc_sw128_kmajor(smem + vS, DV, k0), tc::desc_sw128_kmajor(smem + vW, WIN, k0), id, k0 > 0);
             for (int k0 = 0; k0 < DK; k0 += 16)
-                tc::mma_bf16(tm + 16, tc::desc_sw128_kmajor(smem + vS, DV, k0), tc::desc_sw128_kmajor(smem + vQg, WIN, k0), id, k0 > 0);
-            tc::mma_commit(bar);
-            atomicAdd(const_cast<uint32_t*>(ctl), 1u);
+                tc::mma_bf16_if(leader, tm + 16, tc::desc_sw128_kmajor(smem + vS, DV, k0), tc::desc_sw128_kmajor(smem + vQg, WIN, k0), id, k0 > 0);
+            tc::mma_commit_if(leader, bar);
+            if (leader) atomicAdd(const_cast<uint32_t*>(ctl), 1u);
+            __syncwarp();
         }
         ok = mbar_wait(bar, phase, ctx, kStatusWaitPrefill);
         phase ^= 1u;
@@ -559,12 +563,14 @@ __global__ void __launch_bounds__(kVThreads, kCBlocks) commit_tc_kernel(const __
             tc::fence_after_sync();
 
             // ---- B. L^T ---------------------------------------------------------------------------------------------------
-            if (t == 0) {
+            if (warp == 0) {
+                const uint32_t leader = tc::elect_one();
                 constexpr uint32_t id = tc::idesc_bf16(128, WIN, 0, 0, 0);
                 for (int k0 = 0; k0 < DK; k0 += 16)
-                    tc::mma_bf16(tm, tc::desc_sw128_kmajor(smem + cKc, WIN, k0), tc::desc_sw128_kmajor(smem + cKgb, WIN, k0), id, k0 > 0);
-                tc::mma_commit(bar);
-                atomicAdd(const_cast<uint32_t*>(ctl), 1u);
+                    tc::mma_bf16_if(leader, tm, tc::desc_sw128_kmajor(smem + cKc, WIN, k0), tc::desc_sw128_kmajor(smem + cKgb, WIN, k0), id, k0 > 0);
+                tc::mma_commit_if(leader, bar);
+                if (leader) atomicAdd(const_cast<uint32_t*>(ctl), 1u);
+                __syncwarp();
             }
             ok = mbar_wait(bar, phase, ctx, kStatusWaitPrefill);
             phase ^= 1u;
@@ -615,12 +621,14 @@ __global__ void __launch_bounds__(kVThreads, kCBlocks) commit_tc_kernel(const __
             tc::fence_after_sync();
 
             // ---- D. (W S)^T = S W^T --------------------------------------------------------------------------------------------
-            if (t == 0) {
+            if (warp == 0) {
+                const uint32_t leader = tc::elect_one();
                 constexpr uint32_t id = tc::idesc_bf16(128, WIN, 0, 0, 0);
                 for (int k0 = 0; k0 < DK; k0 += 16)
-                    tc::mma_bf16(tm, tc::desc_sw128_kmajor(smem + cS, DV, k0), tc::desc_sw128_kmajor(smem + cW, WIN, k0), id, k0 > 0);
-                tc::mma_commit(bar);
-                atomicAdd(const_cast<uint32_t*>(ctl), 1u);
+                    tc::mma_bf16_if(leader, tm, tc::desc_sw128_kmajor(smem + cS, DV, k0), tc::desc_sw128_kmajor(smem + cW, WIN, k0), id, k0 > 0);
+                tc::mma_commit_if(leader, bar);
+                if (leader) atomicAdd(const_cast<uint32_t*>(ctl), 1u);
+                __syncwarp();
             }
             ok = mbar_wait(bar, phase, ctx, kStatusWaitPrefill);
             phase ^= 1u;
@@ -653,13 +661,15 @@ __global__ void __launch_bounds__(kVThreads, kCBlocks) commit_tc_kernel(const __
             tc::fence_after_sync();
 
             // ---- F. the update D^T x Kdec: [value row][key channel], three products of halves ------------------------------------
-            if (t == 0) {
+            if (warp == 0) {
+                const uint32_t leader = tc::elect_one();
                 constexpr uint32_t id = tc::idesc_bf16(128, 128, 0, 0, 0);
-                tc::mma_bf16(tm, tc::desc_kmajor_bf16(smem + cDT, DV, 0, 0), tc::desc_kmajor_bf16(smem + cKdT, DK, 0, 0), id, false);
-                tc::mma_bf16(tm, tc::desc_kmajor_bf16(smem + cDT, DV, 0, 0), tc::desc_kmajor_bf16(smem + cKdT + 4096, DK, 0, 0), id, true);
-                tc::mma_bf16(tm, tc::desc_kmajor_bf16(smem + cDT + 4096, DV, 0, 0), tc::desc_kmajor_bf16(smem + cKdT, DK, 0, 0), id, true);
-                tc::mma_commit(bar);
-                atomicAdd(const_cast<uint32_t*>(ctl), 1u);
+                tc::mma_bf16_if(leader, tm, tc::desc_kmajor_bf16(smem + cDT, DV, 0, 0), tc::desc_kmajor_bf16(smem + cKdT, DK, 0, 0), id, false);
+                tc::mma_bf16_if(leader, tm, tc::desc_kmajor_bf16(smem + cDT, DV, 0, 0), tc::desc_kmajor_bf16(smem + cKdT + 4096, DK, 0, 0), id, true);
+                tc::mma_bf16_if(leader, tm, tc::desc_kmajor_bf16(smem + cDT + 4096, DV, 0, 0), tc::desc_kmajor_bf16(smem + cKdT, DK, 0, 0), id, true);
+                tc::mma_commit_if(leader, bar);
+                if (leader) atomicAdd(const_cast<uint32_t*>(ctl), 1u);
+                __syncwarp();
             }
             ok = mbar_wait(bar, phase, ctx, kStatusWaitPrefill);
             phase ^= 1u;
