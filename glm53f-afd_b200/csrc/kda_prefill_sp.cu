@@ -139,7 +139,7 @@ static_assert(gTp % 1024 == 0 && gKc % 1024 == 0, "swizzled tiles are 1024-byte 
 // exp(Gm_I - Gm_J) for I > J.  The scan's totals use the first two rows before the tables are written.
 constexpr int gTab = gKc + kKcBytes, gBeta = gTab + kTabs * 512, gBars = gBeta + CH * 4, gItem = gBars + 32, gGl = gItem + 16;  // gGl: exp(G_last) [128]
 constexpr int kGroupBytes = 114688;
-static_assert(4 * kBox <= kKcBytes && gP + 32 * 32 * 4 <= gKc + kKcBytes && gTp + kTile <= gP && gGl + 512 <= kGroupBytes && kGroupBytes % 1024 == 0, "group map");
+static_assert(4 * kBox <= kKcBytes && gP + 32 * PS * 4 <= gTab && gTp + kTile <= gP && gGl + 512 <= kGroupBytes && kGroupBytes % 1024 == 0, "group map");
 static_assert(kGroups * kGroupBytes <= oCtl, "two groups must fit below the block's control words");
 constexpr uint32_t gcL = 0, gcM = 64, gcW = 0, gcU = 128, kGroupCols = 256;
 
@@ -435,9 +435,7 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
             const float* Lm = reinterpret_cast<const float*>(gs + gL);
             float* Tm = reinterpret_cast<float*>(gs + gT);
             float* Pm = reinterpret_cast<float*>(gs + gP);
-            invert_diag16<kGroupThreads>(Lm, Tm, gt, BAR);
-            invert_level<4, kGroupThreads>(Lm, Tm, Pm, gt, BAR);
-            invert_level<5, kGroupThreads>(Lm, Tm, Pm, gt, BAR);
+            invert<kGroupThreads>(Lm, Tm, Pm, gt, BAR);
             const int i = gt & 63, cq = gt >> 6;
 #pragma unroll
             for (int cc = 0; cc < 2; ++cc) {

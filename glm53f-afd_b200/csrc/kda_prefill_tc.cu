@@ -8,8 +8,8 @@
 //   G_i   = g_0 + ... + g_i per key channel (FP32 scan, thread = channel), E = exp(G), E_last = exp(G_63)
 //   Kg = k*E, Qg = q*E, Kinv = k/E, Kdec = k * E_last/E                       (operand tiles, written by hand)
 //   L = Kg Kinv^T, M = Qg Kinv^T      64x64x128 MMAs; L strictly lower * beta_i, M lower incl. diagonal
-//   T  = (I + L)^-1                   FP32 on the CUDA cores by recursive doubling: the lower-left block of every
-//                                     2sz x 2sz diagonal block is -T22 (L21 T11), sz = 1 .. 32;  T' = T diag(beta)
+//   T  = (I + L)^-1                   16 x 16 diagonal blocks by substitution, then the lower-left block of every
+//                                     2sz x 2sz diagonal block is -T22 (L21 T11), sz = 16, 32;  T' = T diag(beta)
 //   W  = T' Kg,  U = T' V             64x128x64 MMAs; T' as bf16 hi + lo for U
 //   D  = U - W S,  QS = Qg S          64x128x128 MMAs on a bf16 copy of S; D accumulates in place (negated A)
 //   O  = QS + M D                     64x128x64 MMA
@@ -445,11 +445,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1) prefill_tc_kernel(const __grid_
             const float* Lm = reinterpret_cast<const float*>(smem + oL);
             float* Tm = reinterpret_cast<float*>(smem + oT);
             float* Pm = reinterpret_cast<float*>(smem + oP);
-            // Recursive doubling.  T starts as the identity; at block size sz the lower-left sz x sz block of every
-            // 2sz x 2sz diagonal block is -T22 (L21 T11), all blocks and elements in parallel.
-            invert_diag16(Lm, Tm, tid);
-            invert_level<4>(Lm, Tm, Pm, tid);
-            invert_level<5>(Lm, Tm, Pm, tid);
+            invert(Lm, Tm, Pm, tid);
             // 5c. T' = T diag(beta) as bf16 hi + lo cells.  T' lands on the scratch itself, so every thread first reads
             // its eight values of T, then the block synchronises, then the cells are written.
             {
