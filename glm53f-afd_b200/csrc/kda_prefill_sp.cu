@@ -15,7 +15,7 @@
 // are handed out through a counter in the workspace), on two halves of the workspace that swap from launch to
 // launch.  Stream order between launches is the only synchronisation: no block ever waits on another block.
 //
-// Workspace slot of one (chain, chunk) item, bytes: Qg 0 | W 16,384 | M 32,768 | Kdec hi 40,960 | Kdec lo 57,344 |
+// Workspace slot of one (chain, chunk) item, bytes: Qg over W 0 (cells of 128 rows) | M 32,768 | Kdec hi 40,960 | Kdec lo 57,344 |
 // U 73,728 (FP32, 32 cells of four value channels x 64 rows) | E_last 106,496 (128 floats); 107,008 per slot = 1,672 per row and head, inside
 // the 2,176 the reference's prefill workspace formula provides (kernels/kda_prefill.cu:40-43, 695-698).  The last
 // 256 bytes of the workspace hold the two item counters.
@@ -37,7 +37,7 @@ using namespace pf;
 
 // U is kept in FP32 as 16-byte cells of four value channels, [32 cells][64 rows], so that both its writer (a thread
 // holds a row's channels) and its reader store and load consecutive cells.
-constexpr int wQg = 0, wW = kTile, wMm = 2 * kTile, wKdHi = wMm + kTile / 2, wKdLo = wKdHi + kTile, wU = wKdLo + kTile;
+constexpr int wQW = 0, wMm = 2 * kTile /* after Qg | W stacked as one operand of 128 rows */, wKdHi = wMm + kTile / 2, wKdLo = wKdHi + kTile, wU = wKdLo + kTile;
 constexpr int kUBytes = CH * DV * 4, wEgl = wU + kUBytes, kSlotBytes = wEgl + 512;
 static_assert(kSlotBytes == 107008 && wU == 73728, "workspace slot layout");
 
@@ -100,9 +100,10 @@ __device__ __forceinline__ unsigned char* slot_of(unsigned char* ws, int seg_chu
 // The state role's barriers sit behind every tile (set up once at kernel entry, never repurposed).  The intra role's
 // live inside its two groups' areas, which the state role -- it runs first in a block -- uses as tile space, so they are
 // set up when the intra role starts.
-constexpr int oBarsState = kSmemTc, kSmemSp = kSmemTc + 128;
-// 16 compute warps, the loader warp, and (state role only) a warp that moves finished output rows to global memory.
-constexpr int kThreadsSp = kCompute + 64, kLoaderWarp = kCompute / 32, kOutWarp = kCompute / 32 + 1;
+constexpr int oBarsState = kSmemTc, kSmemSp = kSmemTc + 192;
+// 16 compute warps, the loader warp, and (state role only) a warp that moves finished output rows to global memory and one that
+// issues the tensor-core products.
+constexpr int kThreadsSp = kCompute + 96, kLoaderWarp = kCompute / 32, kOutWarp = kCompute / 32 + 1, kMmaWarp = kCompute / 32 + 2;
 static_assert(kSmemSp <= 232448, "shared memory budget");
 
 // =====================================================================================================================
@@ -374,7 +375,7 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
             }
             // narrow: Qg itself is M's row side
             *reinterpret_cast<uint4*>(gs + gQ + box_piece(r, c)) = narrow ? make_uint4(qg[0], qg[1], qg[2], qg[3]) : make_uint4(qgb[0], qgb[1], qgb[2], qgb[3]);
-            *reinterpret_cast<uint4*>(cell(slot + wQg, CH, c, r)) = make_uint4(qg[0], qg[1], qg[2], qg[3]);
+            *reinterpret_cast<uint4*>(cell(slot + wQW, 2 * CH, c, r)) = make_uint4(qg[0], qg[1], qg[2], qg[3]);
         }
         publish();
         // ---- 3c. M^T the same way, by the other four warps ------------------------------------------------------------------------
@@ -482,7 +483,7 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
                 tc::tmem_ld_wait();
                 if (lane < 16) {
 #pragma unroll
-                    for (int cc = 0; cc < 4; ++cc) *reinterpret_cast<uint4*>(cell(slot + wW, CH, col / 8 + cc, i)) = pack8(r + cc * 8);
+                    for (int cc = 0; cc < 4; ++cc) *reinterpret_cast<uint4*>(cell(slot + wQW, 2 * CH, col / 8 + cc, CH + i)) = pack8(r + cc * 8);
                 }
                 tc::tmem_ld32(tc::tmem_addr(tm, quad, gcU + col), r);
                 tc::tmem_ld_wait();
@@ -592,22 +593,43 @@ __device__ void intra_role(const SpParams& p, unsigned char* smem, const uint32_
     }
     __syncthreads();
     if (warp == kLoaderWarp || warp == kOutWarp) intra_loader(p, smem, ctx, warp == kLoaderWarp ? 0 : 1);
-    else intra_group(p, smem, tm, ctx, warp < kGroupThreads / 32 ? 0 : 1);
+    else if (warp != kMmaWarp) intra_group(p, smem, tm, ctx, warp < kGroupThreads / 32 ? 0 : 1);
     tc::fence_before_sync();
     __syncthreads();
 }
 
 // =====================================================================================================================
 // Pass 2: the state recurrence of one chain over the segment's chunks, from the workspace.
+//
+// The walk is a chain of dependent steps per chunk, so nothing that can wait sits on it and no two roles meet at a block
+// barrier (mbarriers only):
+//   all 16 warps     S (tensor memory) to bf16 cells; then, behind the first product, the decayed S back
+//   MMA warp         [QS; WS] = [Qg; W] S as ONE product of 128 rows (lanes 0-63 and 64-127 of the accumulator; as two products
+//                    of 64 rows it takes twice the tensor time)
+//   warps of lanes 64-127   D = U - WS as bf16 hi + lo cells
+//   MMA warp         S += Kdec^T D (hi hi + hi lo + lo hi), which the next chunk waits for; then O = QS + M D, which it does not
+//   warps of lanes 0-63     the outputs, beside the next chunk's first product and D
+// Measured per chunk at 64 chains: 5,800 cycles with block barriers around every step, MEASURE_ME so.
 // =====================================================================================================================
 // Shared memory mirrors a workspace slot (three groups, each with its own full/empty barrier pair, refilled by the
 // loader warp as soon as the tensor core has consumed them), then S as bf16 cells and D hi/lo.
 constexpr int sSlot = 0, sS16 = (kSlotBytes + 1023) / 1024 * 1024, sDhi = sS16 + 2 * kTile, sDlo = sDhi + kTile, sRed = sDlo + kTile;
 // Finished output rows (bf16) wait in one of two tiles for the output warp: two boxes of 64 rows x 128 bytes each (value
 // channels 0-63, 64-127) in the 128-byte swizzle of box_piece(), which is what the tiled tensor stores read.
-constexpr int sOut = sRed + 4 * CH * 4, kOutTile = 2 * kBox;
+constexpr int sOut = sRed + 2 * 4 * CH * 4, kOutTile = 2 * kBox;
 static_assert(sOut % 1024 == 0 && sOut + 2 * kOutTile <= oBars, "state role shared memory");
-constexpr uint32_t tS = 0, tQS = 128, tD = 256, tQS1 = 384;  // QS/O accumulators alternate between chunks
+constexpr uint32_t tS = 0, tA = 128;  // the state; two accumulators of 128 columns that alternate between chunks
+
+// The state role's barriers and their arrival counts.
+// bO and bOFree come in pairs, one per accumulator, so that no barrier can complete a phase while somebody still has to see the
+// one before.
+enum : int { bFull = 0, bEmpty = 3, bQSWS = 6, bSNew = 7, bS16 = 8, bSDec = 9, bD = 10, bO = 11, bOFree = 13, bOutFull = 15, bOutEmpty = 17, kStateBars = 19 };
+__device__ __forceinline__ int state_bar_count(int i) {
+    if (i == bS16 || i == bSDec) return kCompute / 32;                                          // every compute warp
+    if (i == bD || i == bEmpty + 1 || i == bOFree || i == bOFree + 1 || i == bOutFull || i == bOutFull + 1) return kCompute / 64;  // half of them
+    return 1;
+}
+static_assert(kStateBars * 8 <= 192, "state role barriers");
 
 // NV = the value channels this block owns (all 128, or 64: a chain's value columns never interact, so two blocks can
 // share a chain when chains are few and the serial walk over the chunks is what takes the time); value channels
@@ -627,15 +649,12 @@ template <int NV>
 __device__ void state_role(const SpParams& p, unsigned char* smem, const uint32_t tm, const int chain, const int vpart, const Walk wk) {
     constexpr int C = NV / 4, CELLS = C / 8;
     const int v0 = vpart * NV;
-    uint64_t* full = reinterpret_cast<uint64_t*>(smem + oBarsState);  // [3]
-    uint64_t* empty = full + 3;                                       // [3]
-    uint64_t* bar_mma = full + 6;
-    uint64_t* out_full = full + 7;   // [2]
-    uint64_t* out_empty = full + 9;  // [2]
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + oBarsState);
+    uint64_t *full = bars + bFull, *empty = bars + bEmpty, *out_full = bars + bOutFull, *out_empty = bars + bOutEmpty;
     volatile uint32_t* ctl = reinterpret_cast<volatile uint32_t*>(smem + oCtl);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int quad = warp & 3, cg = warp >> 2;
-    const int lane_row128 = quad * 32 + lane, lane_row64 = quad * 16 + lane;
+    const int lane_row128 = quad * 32 + lane;
     const int H = p.H, b = chain / H, h = chain % H;
     const long long row0 = p.cu[b];
     const int T = p.cu[b + 1] - p.cu[b];
@@ -695,7 +714,7 @@ __device__ void state_role(const SpParams& p, unsigned char* smem, const uint32_
                 const unsigned char* slot = slot_of(p.ws_state, p.seg_chunks, chain, j - p.state_chunk0);
                 if (!mbar_wait(&empty[0], ph, ctx, kStatusWaitPrefill)) break;
                 mbar_arrive_expect_tx(&full[0], 2 * kTile + 512);
-                bulk_load(smem + sSlot + wQg, slot + wQg, 2 * kTile, &full[0]);
+                bulk_load(smem + sSlot + wQW, slot + wQW, 2 * kTile, &full[0]);
                 bulk_load(smem + sSlot + wEgl, slot + wEgl, 512, &full[0]);
                 if (!mbar_wait(&empty[1], ph, ctx, kStatusWaitPrefill)) break;
                 mbar_arrive_expect_tx(&full[1], NV * CH * 4);
@@ -711,60 +730,75 @@ __device__ void state_role(const SpParams& p, unsigned char* smem, const uint32_
         return;
     }
 
-    uint32_t mma_phase = 0;
-    bool alive = true;
-    auto mma_issue = [&](auto&& issue) {  // by one lane of warp 0, the warp converged (tc::mma_bf16_if)
-        if (warp == 0) {
-            const uint32_t leader = tc::elect_one();
-            issue(leader);
-            tc::mma_commit_if(leader, bar_mma);
+    if (warp == kMmaWarp) {
+        const uint32_t leader = tc::elect_one();
+        auto wait = [&](int i, int c) { return tc::warp_all(mbar_wait(&bars[i], (uint32_t)(c & 1), ctx, kStatusWaitPrefill)); };
+        constexpr uint32_t id = tc::idesc_bf16(128, NV, 0, 1, 0), idt = tc::idesc_bf16(128, NV, 1, 1, 0);
+        for (int c = 0; c < j1 - j0; ++c) {
+            const uint32_t acc = tm + tA + (uint32_t)(c & 1) * 128;
+            if (!wait(bFull, c) || !wait(bS16, c)) break;
+            if (wk.emit && c >= 2 && !wait(bOFree + (c & 1), (c >> 1) - 1)) break;  // chunk c - 2's outputs have left this accumulator
+            tc::fence_after_sync();
+#pragma unroll
+            for (int k0 = 0; k0 < DK; k0 += 16)
+                tc::mma_bf16_if(leader, acc, tc::desc_kmajor_bf16(smem + sSlot + wQW, 2 * CH, 0, k0), tc::desc_mnmajor_bf16(smem + sS16, 128, 0, k0), id, k0 > 0);
+            tc::mma_commit_if(leader, &bars[bQSWS]);
+            tc::mma_commit_if(leader, &empty[0]);  // Qg, W are consumed (and E_last, read before bS16)
+            if (!wait(bFull + 2, c) || !wait(bD, c) || !wait(bSDec, c)) break;
+            tc::fence_after_sync();
+            const unsigned char *kdhi = smem + sSlot + wKdHi, *kdlo = smem + sSlot + wKdLo, *dhi = smem + sDhi, *dlo = smem + sDlo;
+#pragma unroll
+            for (int k0 = 0; k0 < CH; k0 += 16) tc::mma_bf16_if(leader, tm + tS, tc::desc_mnmajor_bf16(kdhi, CH, 0, k0), tc::desc_mnmajor_bf16(dhi, CH, 0, k0), idt, true);
+#pragma unroll
+            for (int k0 = 0; k0 < CH; k0 += 16) tc::mma_bf16_if(leader, tm + tS, tc::desc_mnmajor_bf16(kdhi, CH, 0, k0), tc::desc_mnmajor_bf16(dlo, CH, 0, k0), idt, true);
+#pragma unroll
+            for (int k0 = 0; k0 < CH; k0 += 16) tc::mma_bf16_if(leader, tm + tS, tc::desc_mnmajor_bf16(kdlo, CH, 0, k0), tc::desc_mnmajor_bf16(dhi, CH, 0, k0), idt, true);
+            tc::mma_commit_if(leader, &bars[bSNew]);
+            if (wk.emit) {
+                // M has 64 rows; the operand's other 64 are whatever lies behind it (Kdec) and reach lanes 64-127 only, whose WS
+                // has been read.
+#pragma unroll
+                for (int k0 = 0; k0 < CH; k0 += 16)
+                    tc::mma_bf16_if(leader, acc, tc::desc_mnmajor_bf16(smem + sSlot + wMm, CH, 0, k0), tc::desc_mnmajor_bf16(dhi, CH, 0, k0), idt, true);
+                tc::mma_commit_if(leader, &bars[bO + (c & 1)]);
+            }
+            tc::mma_commit_if(leader, &empty[2]);
             if (leader) atomicAdd(const_cast<uint32_t*>(ctl), 1u);
             __syncwarp();
         }
-    };
-    auto mma_wait = [&]() -> bool {
-        if (!mbar_wait(bar_mma, mma_phase, ctx, kStatusWaitPrefill)) return false;
-        mma_phase ^= 1u;
-        tc::fence_after_sync();
-        return true;
-    };
-    auto publish_operands = [&]() {
-        fence_proxy_async_smem();
         tc::fence_before_sync();
-        compute_sync();
-        tc::fence_after_sync();
+        __syncthreads();
+        return;
+    }
+
+    bool alive = true;
+    auto wait = [&](int i, int c) { return mbar_wait(&bars[i], (uint32_t)(c & 1), ctx, kStatusWaitPrefill); };
+    // What this warp wrote for the tensor core, or left in (or took out of) tensor memory, is there: one arrival a warp.
+    auto arrive = [&](int i) {
+        tc::fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars[i]);
     };
-    // S as bf16 cells for chunk c's products, the decayed S back to tensor memory, then QS = Qg S and -W S are started
-    // (not waited for) into the chunk's accumulators.
+    // S as bf16 cells for chunk c's products, then the decayed S back to tensor memory.
     auto begin_chunk = [&](int c) -> bool {
-        if (!mbar_wait(&full[0], (uint32_t)(c & 1), ctx, kStatusWaitPrefill)) return false;
-        const float* egl = reinterpret_cast<const float*>(smem + sSlot + wEgl);
-        {
-            uint32_t r[C];
-            tc::tmem_ld<C>(tc::tmem_addr(tm, quad, tS + cg * C), r);
-            tc::tmem_ld_wait();
-            if (p.state_bf16) {
+        if (!wait(bFull, c)) return false;
+        uint32_t r[C];
+        tc::tmem_ld<C>(tc::tmem_addr(tm, quad, tS + cg * C), r);
+        const float el = reinterpret_cast<const float*>(smem + sSlot + wEgl)[lane_row128];
+        tc::tmem_ld_wait();
+        if (p.state_bf16) {
 #pragma unroll
-                for (int jj = 0; jj < C; ++jj) r[jj] = __float_as_uint(bf16_round(__uint_as_float(r[jj])));
-            }
-#pragma unroll
-            for (int cc = 0; cc < CELLS; ++cc) *reinterpret_cast<uint4*>(cell(smem + sS16, 128, cg * CELLS + cc, lane_row128)) = pack8(r + cc * 8);
-            const float el = egl[lane_row128];
-#pragma unroll
-            for (int jj = 0; jj < C; ++jj) r[jj] = __float_as_uint(__uint_as_float(r[jj]) * el);
-            tc::tmem_st<C>(tc::tmem_addr(tm, quad, tS + cg * C), r);
-            tc::tmem_st_wait();
+            for (int jj = 0; jj < C; ++jj) r[jj] = __float_as_uint(bf16_round(__uint_as_float(r[jj])));
         }
-        publish_operands();
-        const uint32_t tO = (c & 1) ? tQS1 : tQS;
-        mma_issue([&](uint32_t leader) {
-            constexpr uint32_t id = tc::idesc_bf16(64, NV, 0, 1, 0), idn = tc::idesc_bf16(64, NV, 0, 1, 1);
-            if (wk.emit)
-                for (int k0 = 0; k0 < DK; k0 += 16)
-                    tc::mma_bf16_if(leader, tm + tO, tc::desc_kmajor_bf16(smem + sSlot + wQg, CH, 0, k0), tc::desc_mnmajor_bf16(smem + sS16, 128, 0, k0), id, k0 > 0);
-            for (int k0 = 0; k0 < DK; k0 += 16)
-                tc::mma_bf16_if(leader, tm + tD, tc::desc_kmajor_bf16(smem + sSlot + wW, CH, 0, k0), tc::desc_mnmajor_bf16(smem + sS16, 128, 0, k0), idn, k0 > 0);
-        });
+#pragma unroll
+        for (int cc = 0; cc < CELLS; ++cc) *reinterpret_cast<uint4*>(cell(smem + sS16, 128, cg * CELLS + cc, lane_row128)) = pack8(r + cc * 8);
+        fence_proxy_async_smem();
+        arrive(bS16);
+#pragma unroll
+        for (int jj = 0; jj < C; ++jj) r[jj] = __float_as_uint(__uint_as_float(r[jj]) * el);
+        tc::tmem_st<C>(tc::tmem_addr(tm, quad, tS + cg * C), r);
+        tc::tmem_st_wait();
+        arrive(bSDec);
         return true;
     };
 
@@ -786,89 +820,73 @@ __device__ void state_role(const SpParams& p, unsigned char* smem, const uint32_
         tc::tmem_st<C>(tc::tmem_addr(tm, quad, tS + cg * C), r);
         tc::tmem_st_wait();
     }
-    tc::fence_before_sync();
-    compute_sync();
-    tc::fence_after_sync();
-    if (j0 < j1 && !begin_chunk(0)) alive = false;
+    // The warps that share output rows vote at a barrier in every chunk when the norm is fused; one that gives up before it
+    // still takes part.
+    const bool votes = NV == DV && wk.emit && p.gate != nullptr && quad < 2;
+    auto leave = [&] {
+        if (votes) named_bar_all(4 + quad, 128, false);
+        alive = false;
+    };
+    if (j0 < j1 && !begin_chunk(0)) leave();
 
     for (int j = j0; alive && j < j1; ++j) {
         const int c = j - j0, n = min(CH, T - j * CH);
-        const uint32_t par = (uint32_t)(c & 1), tO = (c & 1) ? tQS1 : tQS;
+        const uint32_t acc = tA + (uint32_t)(c & 1) * 128 + cg * C;
         const long long gr0 = row0 + (long long)j * CH;
-        if (!mma_wait()) { alive = false; break; }
-        if (tid == 0) mbar_arrive(&empty[0]);  // Qg, W and exp(G_last) are consumed (begin_chunk read E_last before the products)
-
-        // ---- D = U - W S as bf16 hi + lo cells ---------------------------------------------------------------------------
-        if (!mbar_wait(&full[1], par, ctx, kStatusWaitPrefill)) { alive = false; break; }
-        {
+        // ---- D = U - W S as bf16 hi + lo cells, by the warps whose lanes hold W S -----------------------------------------
+        if (quad >= 2) {
+            if (!wait(bFull + 1, c) || !wait(bQSWS, c)) { alive = false; break; }
+            tc::fence_after_sync();
+            const int i = lane_row128 - CH;
             uint32_t r[C];
-            tc::tmem_ld<C>(tc::tmem_addr(tm, quad, tD + cg * C), r);
+            tc::tmem_ld<C>(tc::tmem_addr(tm, quad, acc), r);
+            unsigned char* Ut = smem + sSlot + wU;  // this block's slice of U: NV / 4 cells of four value channels
             tc::tmem_ld_wait();
-            if (lane < 16) {
-                unsigned char* Ut = smem + sSlot + wU;  // this block's slice of U: NV / 4 cells of four value channels
 #pragma unroll
-                for (int cc = 0; cc < CELLS; ++cc) {
-                    const float4 u0 = *reinterpret_cast<const float4*>(cell(Ut, CH, cg * (C / 4) + cc * 2, lane_row64));
-                    const float4 u1 = *reinterpret_cast<const float4*>(cell(Ut, CH, cg * (C / 4) + cc * 2 + 1, lane_row64));
-                    const float uu[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
-                    uint32_t wh[4], wl[4];
+            for (int cc = 0; cc < CELLS; ++cc) {
+                const float4 u0 = *reinterpret_cast<const float4*>(cell(Ut, CH, cg * (C / 4) + cc * 2, i));
+                const float4 u1 = *reinterpret_cast<const float4*>(cell(Ut, CH, cg * (C / 4) + cc * 2 + 1, i));
+                const float uu[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
+                uint32_t wh[4], wl[4];
 #pragma unroll
-                    for (int jj = 0; jj < 4; ++jj) {
-                        float h0, l0, h1, l1;
-                        tc::split_bf16((wk.use_u ? uu[2 * jj] : 0.0f) + __uint_as_float(r[cc * 8 + 2 * jj]), h0, l0);
-                        tc::split_bf16((wk.use_u ? uu[2 * jj + 1] : 0.0f) + __uint_as_float(r[cc * 8 + 2 * jj + 1]), h1, l1);
-                        wh[jj] = tc::bf16x2(h0, h1);
-                        wl[jj] = tc::bf16x2(l0, l1);
-                    }
-                    *reinterpret_cast<uint4*>(cell(smem + sDhi, CH, cg * CELLS + cc, lane_row64)) = make_uint4(wh[0], wh[1], wh[2], wh[3]);
-                    *reinterpret_cast<uint4*>(cell(smem + sDlo, CH, cg * CELLS + cc, lane_row64)) = make_uint4(wl[0], wl[1], wl[2], wl[3]);
-                }
+                for (int jj = 0; jj < 4; ++jj)
+                    tc::split_bf16x2((wk.use_u ? uu[2 * jj] : 0.0f) - __uint_as_float(r[cc * 8 + 2 * jj]),
+                                     (wk.use_u ? uu[2 * jj + 1] : 0.0f) - __uint_as_float(r[cc * 8 + 2 * jj + 1]), wh[jj], wl[jj]);
+                *reinterpret_cast<uint4*>(cell(smem + sDhi, CH, cg * CELLS + cc, i)) = make_uint4(wh[0], wh[1], wh[2], wh[3]);
+                *reinterpret_cast<uint4*>(cell(smem + sDlo, CH, cg * CELLS + cc, i)) = make_uint4(wl[0], wl[1], wl[2], wl[3]);
             }
+            fence_proxy_async_smem();
+            arrive(bD);
+            if (lane == 0) mbar_arrive(&empty[1]);  // U is consumed
         }
-        publish_operands();
-        if (tid == 0) mbar_arrive(&empty[1]);
+        if (!wait(bSNew, c)) { leave(); break; }
+        tc::fence_after_sync();
+        if (j + 1 < j1 && !begin_chunk(c + 1)) { leave(); break; }
 
-        // ---- O = QS + M D;  S += Kdec^T D (hi hi + hi lo + lo hi) ------------------------------------------------------------
-        if (!mbar_wait(&full[2], par, ctx, kStatusWaitPrefill)) { alive = false; break; }
-        mma_issue([&](uint32_t leader) {
-            constexpr uint32_t idm = tc::idesc_bf16(64, NV, 1, 1, 0), ids = tc::idesc_bf16(128, NV, 1, 1, 0);  // M arrives with its rows contiguous
-            const unsigned char* kdhi = smem + sSlot + wKdHi;
-            const unsigned char* kdlo = smem + sSlot + wKdLo;
-            if (wk.emit)
-                for (int k0 = 0; k0 < CH; k0 += 16)
-                    tc::mma_bf16_if(leader, tm + tO, tc::desc_mnmajor_bf16(smem + sSlot + wMm, CH, 0, k0), tc::desc_mnmajor_bf16(smem + sDhi, CH, 0, k0), idm, true);
-            for (int k0 = 0; k0 < CH; k0 += 16)
-                tc::mma_bf16_if(leader, tm + tS, tc::desc_mnmajor_bf16(kdhi, CH, 0, k0), tc::desc_mnmajor_bf16(smem + sDhi, CH, 0, k0), ids, true);
-            for (int k0 = 0; k0 < CH; k0 += 16)
-                tc::mma_bf16_if(leader, tm + tS, tc::desc_mnmajor_bf16(kdhi, CH, 0, k0), tc::desc_mnmajor_bf16(smem + sDlo, CH, 0, k0), ids, true);
-            for (int k0 = 0; k0 < CH; k0 += 16)
-                tc::mma_bf16_if(leader, tm + tS, tc::desc_mnmajor_bf16(kdlo, CH, 0, k0), tc::desc_mnmajor_bf16(smem + sDhi, CH, 0, k0), ids, true);
-        });
-        if (!mma_wait()) { alive = false; break; }
-        if (tid == 0) mbar_arrive(&empty[2]);
-
-        // The next chunk's first products run on the tensor core while this chunk's outputs leave.
-        if (j + 1 < j1 && !begin_chunk(c + 1)) { alive = false; break; }
-
-        // ---- outputs: bf16(y), or the gated RMSNorm of bf16(y) ------------------------------------------------------------------
-        if (wk.emit) {
+        // ---- outputs: bf16(y), or the gated RMSNorm of bf16(y), by the warps whose lanes hold O --------------------------------
+        if (wk.emit && quad < 2) {
+            bool ok = wait(bO + (c & 1), c >> 1);
+            tc::fence_after_sync();
             uint32_t r[C];
-            tc::tmem_ld<C>(tc::tmem_addr(tm, quad, tO + cg * C), r);
+            tc::tmem_ld<C>(tc::tmem_addr(tm, quad, acc), r);
             tc::tmem_ld_wait();
-            const int i = lane_row64;
-            const bool live = lane < 16 && i < n;
+            arrive(bOFree + (c & 1));
+            const int i = lane_row128;
+            const bool live = i < n;
             const long long at = ((gr0 + i) * H + h) * DV + v0 + cg * C;
             float y[C];
 #pragma unroll
             for (int jj = 0; jj < C; ++jj) y[jj] = bf16_round(__uint_as_float(r[jj]));
-            if (NV == DV && p.gate != nullptr) {  // the norm needs a row's every value channel: whole-head blocks only
-                float* red = reinterpret_cast<float*>(smem + sRed);
+            ok = ok && mbar_wait(&out_empty[c & 1], (uint32_t)(((c >> 1) & 1) ^ 1), ctx, kStatusWaitPrefill);
+            if (votes) {  // the norm needs a row's every value channel: whole-head blocks only
+                float* red = reinterpret_cast<float*>(smem + sRed) + (c & 1) * 4 * CH;
                 float ss = 0.0f;
 #pragma unroll
                 for (int jj = 0; jj < C; ++jj) ss = fmaf(y[jj], y[jj], ss);
-                if (lane < 16) red[cg * CH + i] = ss;
-                compute_sync();
-                if (live) {
+                red[cg * CH + i] = ss;
+                // The four warps that share these rows meet here, and decide together whether they go on.
+                ok = named_bar_all(4 + quad, 128, ok);
+                if (live && ok) {
                     const float tot = (red[i] + red[CH + i]) + (red[2 * CH + i] + red[3 * CH + i]);
                     const float rinv = 1.0f / sqrtf(tot / (float)DV + p.eps);
 #pragma unroll
@@ -877,17 +895,14 @@ __device__ void state_role(const SpParams& p, unsigned char* smem, const uint32_
                         y[jj] = w * (y[jj] * rinv) * (1.0f / (1.0f + __expf(-gt)));
                     }
                 }
-                compute_sync();  // the partial sums are read before the next chunk's are written
             }
             // Into the output tile (the output warp takes it from there).
-            if (!mbar_wait(&out_empty[c & 1], (uint32_t)(((c >> 1) & 1) ^ 1), ctx, kStatusWaitPrefill)) { alive = false; break; }
-            if (lane < 16) {
-                unsigned char* dst = smem + sOut + (c & 1) * kOutTile;
+            if (!ok) { alive = false; break; }
+            unsigned char* dst = smem + sOut + (c & 1) * kOutTile;
 #pragma unroll
-                for (int c4 = 0; c4 < CELLS; ++c4)
-                    *reinterpret_cast<uint4*>(dst + box_piece(i, cg * CELLS + c4)) = make_uint4(tc::bf16x2(y[c4 * 8], y[c4 * 8 + 1]), tc::bf16x2(y[c4 * 8 + 2], y[c4 * 8 + 3]),
-                                                                          tc::bf16x2(y[c4 * 8 + 4], y[c4 * 8 + 5]), tc::bf16x2(y[c4 * 8 + 6], y[c4 * 8 + 7]));
-            }
+            for (int c4 = 0; c4 < CELLS; ++c4)
+                *reinterpret_cast<uint4*>(dst + box_piece(i, cg * CELLS + c4)) = make_uint4(tc::bf16x2(y[c4 * 8], y[c4 * 8 + 1]), tc::bf16x2(y[c4 * 8 + 2], y[c4 * 8 + 3]),
+                                                                      tc::bf16x2(y[c4 * 8 + 4], y[c4 * 8 + 5]), tc::bf16x2(y[c4 * 8 + 6], y[c4 * 8 + 7]));
             fence_proxy_async_smem();  // the tensor stores read the tile through the async proxy
             __syncwarp();
             if (lane == 0) mbar_arrive(&out_full[c & 1]);
@@ -920,9 +935,7 @@ __global__ void __launch_bounds__(kThreadsSp, 1) prefill_sp_kernel(const __grid_
     const int tid = threadIdx.x, warp = tid >> 5;
     if (tid == 0) {
         uint64_t* bs = reinterpret_cast<uint64_t*>(smem + oBarsState);
-        for (int i = 0; i < 7; ++i) mbar_init(bs + i, 1);  // state role: full[3], empty[3], mma
-        for (int i = 0; i < 2; ++i) mbar_init(bs + 7 + i, kCompute / 32);  // output tile full: one arrival per compute warp
-        for (int i = 0; i < 2; ++i) mbar_init(bs + 9 + i, 1);               // output tile empty
+        for (int i = 0; i < kStateBars; ++i) mbar_init(bs + i, state_bar_count(i));
         ctl[0] = 0u;
         ctl[1] = 0u;
         mbar_init_fence();

@@ -172,5 +172,11 @@ __device__ __forceinline__ void split_bf16(float x, float& hi, float& lo) {
     lo = x - hi;
 }
 
+// The same for a pair, packed: hi and lo halves of (x0, x1).
+__device__ __forceinline__ void split_bf16x2(float x0, float x1, uint32_t& hi, uint32_t& lo) {
+    hi = bf16x2(x0, x1);
+    lo = bf16x2(x0 - __uint_as_float(hi << 16), x1 - __uint_as_float(hi & 0xffff0000u));
+}
+
 }  // namespace tc
 }  // namespace kda
