@@ -15,8 +15,8 @@
 // are handed out through a counter in the workspace), on two halves of the workspace that swap from launch to
 // launch.  Stream order between launches is the only synchronisation: no block ever waits on another block.
 //
-// Workspace slot of one (chain, chunk) item, bytes: Qg over W 0 (cells of 128 rows) | M 32,768 | Kdec hi 40,960 | Kdec lo 57,344 |
-// U 73,728 (FP32, 32 cells of four value channels x 64 rows) | E_last 106,496 (128 floats); 107,008 per slot = 1,672 per row and head, inside
+// Workspace slot of one (chain, chunk) item, bytes: Qg 0 | W 16,384 (cells of eight rows, [8][128 key channels]) | M 32,768 | Kdec hi 40,960 | Kdec lo 57,344 |
+// U 73,728 (FP32, cells of four rows, [2][16][64 value channels]) | E_last 106,496 (128 floats); 107,008 per slot = 1,672 per row and head, inside
 // the 2,176 the reference's prefill workspace formula provides (kernels/kda_prefill.cu:40-43, 695-698).  The last
 // 256 bytes of the workspace hold the two item counters.
 
@@ -35,9 +35,10 @@ namespace {
 
 using namespace pf;
 
-// U is kept in FP32 as 16-byte cells of four value channels, [32 cells][64 rows], so that both its writer (a thread
-// holds a row's channels) and its reader store and load consecutive cells.
-constexpr int wQW = 0, wMm = 2 * kTile /* after Qg | W stacked as one operand of 128 rows */, wKdHi = wMm + kTile / 2, wKdLo = wKdHi + kTile, wU = wKdLo + kTile;
+// U is kept in FP32 as 16-byte cells of four rows of a value channel, the channels in two halves, so that both its writer (a
+// thread holds a channel's rows) and its reader store and load consecutive cells and half of the channels is one piece.
+__device__ __forceinline__ int u_cell(int row4, int v) { return (((v >> 6) * 16 + row4) * 64 + (v & 63)) * 16; }
+constexpr int wQg = 0, wW = kTile, wMm = 2 * kTile, wKdHi = wMm + kTile / 2, wKdLo = wKdHi + kTile, wU = wKdLo + kTile;
 constexpr int kUBytes = CH * DV * 4, wEgl = wU + kUBytes, kSlotBytes = wEgl + 512;
 static_assert(kSlotBytes == 107008 && wU == 73728, "workspace slot layout");
 
@@ -72,7 +73,6 @@ struct SpParams {
     int state_chunk0, has_state;
     uint16_t* full[8];       // head-sharded launches: every rank's full [rows][heads_total][128] output buffer, or none
     int ranks, heads_total, head0;
-    int parts;               // state-role blocks per chain: 1, or 2 (each owns half of the value channels)
     unsigned int* counters;  // [2] item counters: this launch hands items out of counters[ctr], and zeroes the other
     int ctr;
     int* status;
@@ -90,7 +90,7 @@ struct SpParams {
     const float* scan_carry_in;  // super-blocks: the FP32 state before this launch's range, [chain][128 x 128] (NULL: state_in)
     float* scan_carry_out;       // super-blocks: the FP32 state after this launch's range (scan_p1 == K)
     float* scan_ab;     // [chain][K - 1][2][128 x 128]: B_s, A_s in the state's layout
-    float* scan_start;  // [chain][K][128 x 128]: the state before each segment (segment 0: unused, the caller's state)
+    float* scan_start;  // [chain][K][128 x 128]: the state before each segment
 };
 
 __device__ __forceinline__ unsigned char* slot_of(unsigned char* ws, int seg_chunks, int chain, int jj) {
@@ -142,7 +142,7 @@ constexpr int gTab = gKc + kKcBytes, gBeta = gTab + kTabs * 512, gBars = gBeta +
 constexpr int kGroupBytes = 114688;
 static_assert(4 * kBox <= kKcBytes && gP + 32 * PS * 4 <= gTab && gTp + kTile <= gP && gGl + 512 <= kGroupBytes && kGroupBytes % 1024 == 0, "group map");
 static_assert(kGroups * kGroupBytes <= oCtl, "two groups must fit below the block's control words");
-constexpr uint32_t gcL = 0, gcM = 64, gcW = 0, gcU = 128, kGroupCols = 256;
+constexpr uint32_t gcL = 0, gcM = 64, gcW = 0, gcU = 64, kGroupCols = 128;
 
 // G = 0 or 1, a runtime value: both groups run the same instructions (one copy of this code in the instruction cache).
 __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* smem, const uint32_t tm_block, const WaitCtx& ctx, const int G) {
@@ -375,7 +375,7 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
             }
             // narrow: Qg itself is M's row side
             *reinterpret_cast<uint4*>(gs + gQ + box_piece(r, c)) = narrow ? make_uint4(qg[0], qg[1], qg[2], qg[3]) : make_uint4(qgb[0], qgb[1], qgb[2], qgb[3]);
-            *reinterpret_cast<uint4*>(cell(slot + wQW, 2 * CH, c, r)) = make_uint4(qg[0], qg[1], qg[2], qg[3]);
+            *reinterpret_cast<uint4*>(cell(slot + wQg, CH, c, r)) = make_uint4(qg[0], qg[1], qg[2], qg[3]);
         }
         publish();
         // ---- 3c. M^T the same way, by the other four warps ------------------------------------------------------------------------
@@ -456,43 +456,39 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
         }
         publish();
 
-        // ---- 6. W = T' Kg (bf16 T'), U = T' V (T' hi + lo) -------------------------------------------------------------------
+        // ---- 6. W^T = Kg^T T'^T (bf16 T'), U^T = V^T T'^T (T' hi + lo): 128 channels x 64 rows (as 64 rows x 128 channels the
+        // products take the same instructions at half the rate) ------------------------------------------------------------
         mma_issue(bar_mma, [&](uint32_t leader) {
-            constexpr uint32_t id = tc::idesc_bf16(64, 128, 0, 1, 0);
+            constexpr uint32_t id = tc::idesc_bf16(128, 64, 1, 0, 0);
             const unsigned char* tph = gs + gTp;
             const unsigned char* tpl = gs + gTp + kBox;
+#pragma unroll
             for (int k0 = 0; k0 < CH; k0 += 16)
-                tc::mma_bf16_if(leader, tm + gcW, tc::desc_sw128_kmajor(tph, CH, k0), tc::desc_sw128_mnmajor(gs + gK, CH, k0), id, k0 > 0);
+                tc::mma_bf16_if(leader, tm + gcW, tc::desc_sw128_mnmajor(gs + gK, CH, k0), tc::desc_sw128_kmajor(tph, CH, k0), id, k0 > 0);
+#pragma unroll
             for (int k0 = 0; k0 < CH; k0 += 16)
-                tc::mma_bf16_if(leader, tm + gcU, tc::desc_sw128_kmajor(tph, CH, k0), tc::desc_sw128_mnmajor(gs + gV, CH, k0), id, k0 > 0);
+                tc::mma_bf16_if(leader, tm + gcU, tc::desc_sw128_mnmajor(gs + gV, CH, k0), tc::desc_sw128_kmajor(tph, CH, k0), id, k0 > 0);
+#pragma unroll
             for (int k0 = 0; k0 < CH; k0 += 16)
-                tc::mma_bf16_if(leader, tm + gcU, tc::desc_sw128_kmajor(tpl, CH, k0), tc::desc_sw128_mnmajor(gs + gV, CH, k0), id, true);
+                tc::mma_bf16_if(leader, tm + gcU, tc::desc_sw128_mnmajor(gs + gV, CH, k0), tc::desc_sw128_kmajor(tpl, CH, k0), id, true);
         });
         if (!mma_wait(bar_mma, mma_phase)) break;
         // Nothing of this item is left in the group's shared memory: the loader may bring the next item in.
         if (gt == 0) mbar_arrive(bar_free);
 
-        // ---- 7. W as bf16 cells and U as FP32 rows, from tensor memory to the workspace ---------------------------------------
+        // ---- 7. W as bf16 cells and U as FP32 cells, from tensor memory (lane = channel, column = row) to the workspace ----------
         {
-            const int i = lane_row64;
+            const int ch = quad * 32 + lane;
+            uint32_t r[32];
+            tc::tmem_ld32(tc::tmem_addr(tm, quad, gcW + cg * 32), r);
+            tc::tmem_ld_wait();
 #pragma unroll
-            for (int half = 0; half < 2; ++half) {
-                uint32_t r[32];
-                const int col = cg * 64 + half * 32;
-                tc::tmem_ld32(tc::tmem_addr(tm, quad, gcW + col), r);
-                tc::tmem_ld_wait();
-                if (lane < 16) {
+            for (int cc = 0; cc < 4; ++cc) *reinterpret_cast<uint4*>(cell(slot + wW, DK, cg * 4 + cc, ch)) = pack8(r + cc * 8);
+            tc::tmem_ld32(tc::tmem_addr(tm, quad, gcU + cg * 32), r);
+            tc::tmem_ld_wait();
 #pragma unroll
-                    for (int cc = 0; cc < 4; ++cc) *reinterpret_cast<uint4*>(cell(slot + wQW, 2 * CH, col / 8 + cc, CH + i)) = pack8(r + cc * 8);
-                }
-                tc::tmem_ld32(tc::tmem_addr(tm, quad, gcU + col), r);
-                tc::tmem_ld_wait();
-                if (lane < 16) {
-#pragma unroll
-                    for (int j2 = 0; j2 < 8; ++j2)
-                        *reinterpret_cast<uint4*>(cell(slot + wU, CH, col / 4 + j2, i)) = make_uint4(r[j2 * 4], r[j2 * 4 + 1], r[j2 * 4 + 2], r[j2 * 4 + 3]);
-                }
-            }
+            for (int j2 = 0; j2 < 8; ++j2)
+                *reinterpret_cast<uint4*>(slot + wU + u_cell(cg * 8 + j2, ch)) = make_uint4(r[j2 * 4], r[j2 * 4 + 1], r[j2 * 4 + 2], r[j2 * 4 + 3]);
         }
         tc::fence_before_sync();
         group_sync();
@@ -601,39 +597,39 @@ __device__ void intra_role(const SpParams& p, unsigned char* smem, const uint32_
 // =====================================================================================================================
 // Pass 2: the state recurrence of one chain over the segment's chunks, from the workspace.
 //
-// The walk is a chain of dependent steps per chunk, so nothing that can wait sits on it and no two roles meet at a block
-// barrier (mbarriers only):
-//   all 16 warps     S (tensor memory) to bf16 cells; then, behind the first product, the decayed S back
-//   MMA warp         [QS; WS] = [Qg; W] S as ONE product of 128 rows (lanes 0-63 and 64-127 of the accumulator; as two products
-//                    of 64 rows it takes twice the tensor time)
-//   warps of lanes 64-127   D = U - WS as bf16 hi + lo cells
-//   MMA warp         S += Kdec^T D (hi hi + hi lo + lo hi), which the next chunk waits for; then O = QS + M D, which it does not
-//   warps of lanes 0-63     the outputs, beside the next chunk's first product and D
-// Measured per chunk at 64 chains: 5,800 cycles with block barriers around every step, MEASURE_ME so.
+// The state lives transposed in tensor memory: lane = value channel, columns = key channels (FP32).  The walk is a chain of
+// dependent steps per chunk, so nothing that can wait sits on it and no two roles meet at a block barrier (mbarriers only):
+//   all 16 warps     S^T to bf16 pairs, in tensor memory; then, behind the first product, the decayed S^T back
+//   MMA warp         (W S)^T = S^T W^T, 128 value channels x 64 rows, which D waits for; then (Qg S)^T, which it does not
+//   all 16 warps     D^T = U^T - (W S)^T as bf16 hi + lo pairs, in tensor memory
+//   MMA warp         S^T += D^T Kdec (hi hi + lo hi + hi lo), which the next chunk waits for; then O^T = (Qg S)^T + D^T M^T
+//   all 16 warps     the outputs of the chunk before, while the state's product runs
+// Transposed, every product uses the tensor core's full height, every lane holds results, and the operands that change (S, D)
+// are A operands that never leave tensor memory; what comes from the workspace is the B side, so shared memory has room for
+// two chunks of it and a load has a whole chunk's time to arrive.
+// Measured per chunk at 64 chains: 5,800 cycles with products of 64 rows, S and D through shared memory and block barriers
+// around every step; MEASURE_ME so.
 // =====================================================================================================================
-// Shared memory mirrors a workspace slot (three groups, each with its own full/empty barrier pair, refilled by the
-// loader warp as soon as the tensor core has consumed them), then S as bf16 cells and D hi/lo.
-constexpr int sSlot = 0, sS16 = (kSlotBytes + 1023) / 1024 * 1024, sDhi = sS16 + 2 * kTile, sDlo = sDhi + kTile, sRed = sDlo + kTile;
+// Shared memory: two buffers of [Qg | W], two of [M | Kdec hi | Kdec lo] and exp(G_last), one of U, each with a full / empty pair.
 // Finished output rows (bf16) wait in one of two tiles for the output warp: two boxes of 64 rows x 128 bytes each (value
 // channels 0-63, 64-127) in the 128-byte swizzle of box_piece(), which is what the tiled tensor stores read.
-constexpr int sOut = sRed + 2 * 4 * CH * 4, kOutTile = 2 * kBox;
-static_assert(sOut % 1024 == 0 && sOut + 2 * kOutTile <= oBars, "state role shared memory");
-constexpr uint32_t tS = 0, tA = 128;  // the state; two accumulators of 128 columns that alternate between chunks
+constexpr int kQW = 2 * kTile, kMKd = kTile / 2 + 2 * kTile, kOutTile = 2 * kBox;
+constexpr int sQW = 0, sMKd = sQW + 2 * kQW, sU = sMKd + 2 * kMKd, sOut = sU + kUBytes, sRed = sOut + 2 * kOutTile, sE = sRed + 2 * 4 * CH * 4;
+static_assert(sOut % 1024 == 0 && sE + 2 * 512 <= oBars, "state role shared memory");
+// Tensor memory columns: S^T; its bf16 pairs; (W S)^T; (Qg S)^T and O^T, two accumulators that alternate between chunks; D^T hi, lo.
+constexpr uint32_t tS = 0, tS16 = 128, tWS = 192, tO = 256, tDhi = 384, tDlo = 416;
 
-// The state role's barriers and their arrival counts.
-// bO and bOFree come in pairs, one per accumulator, so that no barrier can complete a phase while somebody still has to see the
-// one before.
-enum : int { bFull = 0, bEmpty = 3, bQSWS = 6, bSNew = 7, bS16 = 8, bSDec = 9, bD = 10, bO = 11, bOFree = 13, bOutFull = 15, bOutEmpty = 17, kStateBars = 19 };
+// The state role's barriers and their arrival counts.  Those of a buffer that alternates between chunks come in pairs, so that
+// no barrier can complete a phase while somebody still has to see the one before.
+enum : int { bFullQW = 0, bFullMKd = 2, bFullU = 4, bEmptyQW = 5, bEmptyMKd = 7, bEmptyU = 9, bWS = 10, bSNew = 11, bS16 = 12, bSDec = 13, bD = 14, bO = 15, bOFree = 17,
+             bOutFull = 19, bOutEmpty = 21, kStateBars = 23 };
 __device__ __forceinline__ int state_bar_count(int i) {
-    if (i == bS16 || i == bSDec) return kCompute / 32;                                          // every compute warp
-    if (i == bD || i == bEmpty + 1 || i == bOFree || i == bOFree + 1 || i == bOutFull || i == bOutFull + 1) return kCompute / 64;  // half of them
-    return 1;
+    // one arrival per compute warp, or one in all
+    const bool warps = i == bEmptyU || i == bS16 || i == bSDec || i == bD || i == bOFree || i == bOFree + 1 || i == bOutFull || i == bOutFull + 1;
+    return warps ? kCompute / 32 : 1;
 }
 static_assert(kStateBars * 8 <= 192, "state role barriers");
 
-// NV = the value channels this block owns (all 128, or 64: a chain's value columns never interact, so two blocks can
-// share a chain when chains are few and the serial walk over the chunks is what takes the time); value channels
-// [vpart * NV, vpart * NV + NV).  A warp then covers C = NV / 4 accumulator columns.
 // What one walk of the state role covers: chunks [ja, jb) of its chain, where the state comes from and goes to, whether
 // U takes part (not in the walk that yields a segment's transition) and whether outputs are produced.
 struct Walk {
@@ -645,62 +641,53 @@ struct Walk {
     bool use_u, emit;
 };
 
-template <int NV>
-__device__ void state_role(const SpParams& p, unsigned char* smem, const uint32_t tm, const int chain, const int vpart, const Walk wk) {
-    constexpr int C = NV / 4, CELLS = C / 8;
-    const int v0 = vpart * NV;
+__device__ void state_role(const SpParams& p, unsigned char* smem, const uint32_t tm, const int chain, const Walk wk) {
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + oBarsState);
-    uint64_t *full = bars + bFull, *empty = bars + bEmpty, *out_full = bars + bOutFull, *out_empty = bars + bOutEmpty;
     volatile uint32_t* ctl = reinterpret_cast<volatile uint32_t*>(smem + oCtl);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int quad = warp & 3, cg = warp >> 2;
-    const int lane_row128 = quad * 32 + lane;
     const int H = p.H, b = chain / H, h = chain % H;
     const long long row0 = p.cu[b];
     const int T = p.cu[b + 1] - p.cu[b];
     const int nch = (T + CH - 1) / CH;
-    const int j0 = min(wk.ja, nch), j1 = min(nch, wk.jb);
+    const int j0 = min(wk.ja, nch), j1 = min(nch, wk.jb), count = j1 - j0;
     const long long s_elem = p.state_off[b] + (long long)h * DV * DK;
     // A chain with no chunk in this range: only the first segment has anything to do (an empty sequence copies its state);
     // a scan walk always delivers its end state.
     if (p.scan_pass == 0 && j0 >= j1 && !(j0 == 0 && p.state_out != p.state_in)) return;
     const WaitCtx ctx{ctl, ctl + 1, p.status};
+    auto wait = [&](int i, int phase) { return mbar_wait(&bars[i], (uint32_t)(phase & 1), ctx, kStatusWaitPrefill); };
 
-    if (warp == kOutWarp && !wk.emit) {
-        tc::fence_before_sync();
-        __syncthreads();
-        return;
-    }
     if (warp == kOutWarp) {
         // The output warp: each finished tile of rows goes to the shard-local `out` and, for a head-sharded launch, into
         // every rank's full buffer -- the all-gather, done here: a peer's buffer is reached over NVLink.  A full chunk
         // leaves by tiled tensor stores (two per destination), off the compute warps' path; a sequence's last, partial
         // chunk by the warp's own stores, so that no row beyond the sequence is touched.
-        for (int j = j0; j < j1; ++j) {
-            const int c = j - j0, n = min(CH, T - j * CH);
-            const long long gr0 = row0 + (long long)j * CH;
-            if (!mbar_wait(&out_full[c & 1], (uint32_t)((c >> 1) & 1), ctx, kStatusWaitPrefill)) break;
+        for (int c = 0; wk.emit && c < count; ++c) {
+            const int n = min(CH, T - (j0 + c) * CH);
+            const long long gr0 = row0 + (long long)(j0 + c) * CH;
+            if (!wait(bOutFull + (c & 1), c >> 1)) break;
             const unsigned char* tile = smem + sOut + (c & 1) * kOutTile;
             if (n == CH) {
                 if (lane == 0) {
-                    for (int x = 0; x < NV / 64; ++x) {
-                        if (p.out != nullptr) tensor_store_3d(&p.tm_out, v0 + x * 64, h, (int)gr0, tile + x * kBox);
-                        for (int pe = 0; pe < p.ranks; ++pe) tensor_store_3d(&p.tm_full[pe], v0 + x * 64, p.head0 + h, (int)gr0, tile + x * kBox);
+                    for (int x = 0; x < 2; ++x) {
+                        if (p.out != nullptr) tensor_store_3d(&p.tm_out, x * 64, h, (int)gr0, tile + x * kBox);
+                        for (int pe = 0; pe < p.ranks; ++pe) tensor_store_3d(&p.tm_full[pe], x * 64, p.head0 + h, (int)gr0, tile + x * kBox);
                     }
                     bulk_commit();
                     bulk_wait_read<0>();  // the tile has been read: the compute warps may refill it
                 }
             } else {
-                for (int e = lane; e < n * (NV / 8); e += 32) {
-                    const int r = e / (NV / 8), piece = e % (NV / 8);
+                for (int e = lane; e < n * 16; e += 32) {
+                    const int r = e >> 4, piece = e & 15;
                     const uint4 v4 = *reinterpret_cast<const uint4*>(tile + box_piece(r, piece));
-                    if (p.out != nullptr) *reinterpret_cast<uint4*>(p.out + ((gr0 + r) * H + h) * DV + v0 + piece * 8) = v4;
-                    const long long at_full = ((gr0 + r) * p.heads_total + p.head0 + h) * DV + v0 + piece * 8;
+                    if (p.out != nullptr) *reinterpret_cast<uint4*>(p.out + ((gr0 + r) * H + h) * DV + piece * 8) = v4;
+                    const long long at_full = ((gr0 + r) * p.heads_total + p.head0 + h) * DV + piece * 8;
                     for (int pe = 0; pe < p.ranks; ++pe) *reinterpret_cast<uint4*>(p.full[pe] + at_full) = v4;
                 }
             }
             __syncwarp();
-            if (lane == 0) mbar_arrive(&out_empty[c & 1]);
+            if (lane == 0) mbar_arrive(&bars[bOutEmpty + (c & 1)]);
         }
         if (lane == 0) bulk_wait_all<0>();
         tc::fence_before_sync();
@@ -709,60 +696,62 @@ __device__ void state_role(const SpParams& p, unsigned char* smem, const uint32_
     }
     if (warp == kLoaderWarp) {
         if (lane == 0) {
-            uint32_t ph = 1;  // the empty barriers start released
-            for (int j = j0; j < j1; ++j) {
-                const unsigned char* slot = slot_of(p.ws_state, p.seg_chunks, chain, j - p.state_chunk0);
-                if (!mbar_wait(&empty[0], ph, ctx, kStatusWaitPrefill)) break;
-                mbar_arrive_expect_tx(&full[0], 2 * kTile + 512);
-                bulk_load(smem + sSlot + wQW, slot + wQW, 2 * kTile, &full[0]);
-                bulk_load(smem + sSlot + wEgl, slot + wEgl, 512, &full[0]);
-                if (!mbar_wait(&empty[1], ph, ctx, kStatusWaitPrefill)) break;
-                mbar_arrive_expect_tx(&full[1], NV * CH * 4);
-                bulk_load(smem + sSlot + wU, slot + wU + (size_t)(v0 / 4) * CH * 16, NV * CH * 4, &full[1]);
-                if (!mbar_wait(&empty[2], ph, ctx, kStatusWaitPrefill)) break;
-                mbar_arrive_expect_tx(&full[2], kTile / 2 + 2 * kTile);
-                bulk_load(smem + sSlot + wMm, slot + wMm, kTile / 2 + 2 * kTile, &full[2]);
-                ph ^= 1u;
+            for (int c = 0; c < count; ++c) {
+                const unsigned char* slot = slot_of(p.ws_state, p.seg_chunks, chain, j0 + c - p.state_chunk0);
+                const int x = c & 1;
+                if (!wait(bEmptyQW + x, (c >> 1) ^ 1)) break;  // an empty barrier starts released
+                mbar_arrive_expect_tx(&bars[bFullQW + x], kQW);
+                bulk_load(smem + sQW + x * kQW, slot + wQg, kQW, &bars[bFullQW + x]);
+                if (!wait(bEmptyMKd + x, (c >> 1) ^ 1)) break;
+                mbar_arrive_expect_tx(&bars[bFullMKd + x], kMKd + 512);
+                bulk_load(smem + sE + x * 512, slot + wEgl, 512, &bars[bFullMKd + x]);
+                bulk_load(smem + sMKd + x * kMKd, slot + wMm, kMKd, &bars[bFullMKd + x]);
+                if (!wait(bEmptyU, c ^ 1)) break;
+                mbar_arrive_expect_tx(&bars[bFullU], kUBytes);
+                bulk_load(smem + sU, slot + wU, kUBytes, &bars[bFullU]);
             }
         }
         tc::fence_before_sync();
         __syncthreads();
         return;
     }
-
     if (warp == kMmaWarp) {
         const uint32_t leader = tc::elect_one();
-        auto wait = [&](int i, int c) { return tc::warp_all(mbar_wait(&bars[i], (uint32_t)(c & 1), ctx, kStatusWaitPrefill)); };
-        constexpr uint32_t id = tc::idesc_bf16(128, NV, 0, 1, 0), idt = tc::idesc_bf16(128, NV, 1, 1, 0);
-        for (int c = 0; c < j1 - j0; ++c) {
-            const uint32_t acc = tm + tA + (uint32_t)(c & 1) * 128;
-            if (!wait(bFull, c) || !wait(bS16, c)) break;
-            if (wk.emit && c >= 2 && !wait(bOFree + (c & 1), (c >> 1) - 1)) break;  // chunk c - 2's outputs have left this accumulator
+        auto ready = [&](int i, int phase) { return tc::warp_all(wait(i, phase)); };
+        constexpr uint32_t idw = tc::idesc_bf16(DV, CH, 0, 1, 0), idq = tc::idesc_bf16(DV, CH, 0, 0, 0), ids = tc::idesc_bf16(DV, DK, 0, 1, 0);
+        for (int c = 0; c < count; ++c) {
+            const int x = c & 1;
+            const uint32_t acc = tm + tO + (uint32_t)x * 64;
+            const unsigned char *qw = smem + sQW + x * kQW, *mm = smem + sMKd + x * kMKd, *kdhi = mm + kTile / 2, *kdlo = kdhi + kTile;
+            if (!ready(bFullQW + x, c >> 1) || !ready(bS16, c)) break;
             tc::fence_after_sync();
 #pragma unroll
             for (int k0 = 0; k0 < DK; k0 += 16)
-                tc::mma_bf16_if(leader, acc, tc::desc_kmajor_bf16(smem + sSlot + wQW, 2 * CH, 0, k0), tc::desc_mnmajor_bf16(smem + sS16, 128, 0, k0), id, k0 > 0);
-            tc::mma_commit_if(leader, &bars[bQSWS]);
-            tc::mma_commit_if(leader, &empty[0]);  // Qg, W are consumed (and E_last, read before bS16)
-            if (!wait(bFull + 2, c) || !wait(bD, c) || !wait(bSDec, c)) break;
+                tc::mma_bf16_ts_if(leader, tm + tWS, tm + tS16 + k0 / 2, tc::desc_mnmajor_bf16(qw + kTile, DK, 0, k0), idw, k0 > 0);
+            tc::mma_commit_if(leader, &bars[bWS]);
+            if (wk.emit) {
+                if (c >= 2 && !ready(bOFree + x, (c >> 1) - 1)) break;  // chunk c - 2's outputs have left this accumulator
+                tc::fence_after_sync();
+#pragma unroll
+                for (int k0 = 0; k0 < DK; k0 += 16)
+                    tc::mma_bf16_ts_if(leader, acc, tm + tS16 + k0 / 2, tc::desc_kmajor_bf16(qw, CH, 0, k0), idq, k0 > 0);
+            }
+            tc::mma_commit_if(leader, &bars[bEmptyQW + x]);
+            if (!ready(bFullMKd + x, c >> 1) || !ready(bSDec, c) || !ready(bD, c)) break;
             tc::fence_after_sync();
-            const unsigned char *kdhi = smem + sSlot + wKdHi, *kdlo = smem + sSlot + wKdLo, *dhi = smem + sDhi, *dlo = smem + sDlo;
 #pragma unroll
-            for (int k0 = 0; k0 < CH; k0 += 16) tc::mma_bf16_if(leader, tm + tS, tc::desc_mnmajor_bf16(kdhi, CH, 0, k0), tc::desc_mnmajor_bf16(dhi, CH, 0, k0), idt, true);
+            for (int k0 = 0; k0 < CH; k0 += 16) tc::mma_bf16_ts_if(leader, tm + tS, tm + tDhi + k0 / 2, tc::desc_mnmajor_bf16(kdhi, CH, 0, k0), ids, true);
 #pragma unroll
-            for (int k0 = 0; k0 < CH; k0 += 16) tc::mma_bf16_if(leader, tm + tS, tc::desc_mnmajor_bf16(kdhi, CH, 0, k0), tc::desc_mnmajor_bf16(dlo, CH, 0, k0), idt, true);
+            for (int k0 = 0; k0 < CH; k0 += 16) tc::mma_bf16_ts_if(leader, tm + tS, tm + tDlo + k0 / 2, tc::desc_mnmajor_bf16(kdhi, CH, 0, k0), ids, true);
 #pragma unroll
-            for (int k0 = 0; k0 < CH; k0 += 16) tc::mma_bf16_if(leader, tm + tS, tc::desc_mnmajor_bf16(kdlo, CH, 0, k0), tc::desc_mnmajor_bf16(dhi, CH, 0, k0), idt, true);
+            for (int k0 = 0; k0 < CH; k0 += 16) tc::mma_bf16_ts_if(leader, tm + tS, tm + tDhi + k0 / 2, tc::desc_mnmajor_bf16(kdlo, CH, 0, k0), ids, true);
             tc::mma_commit_if(leader, &bars[bSNew]);
             if (wk.emit) {
-                // M has 64 rows; the operand's other 64 are whatever lies behind it (Kdec) and reach lanes 64-127 only, whose WS
-                // has been read.
 #pragma unroll
-                for (int k0 = 0; k0 < CH; k0 += 16)
-                    tc::mma_bf16_if(leader, acc, tc::desc_mnmajor_bf16(smem + sSlot + wMm, CH, 0, k0), tc::desc_mnmajor_bf16(dhi, CH, 0, k0), idt, true);
-                tc::mma_commit_if(leader, &bars[bO + (c & 1)]);
+                for (int k0 = 0; k0 < CH; k0 += 16) tc::mma_bf16_ts_if(leader, acc, tm + tDhi + k0 / 2, tc::desc_mnmajor_bf16(mm, CH, 0, k0), idw, true);
+                tc::mma_commit_if(leader, &bars[bO + x]);
             }
-            tc::mma_commit_if(leader, &empty[2]);
+            tc::mma_commit_if(leader, &bars[bEmptyMKd + x]);
             if (leader) atomicAdd(const_cast<uint32_t*>(ctl), 1u);
             __syncwarp();
         }
@@ -772,155 +761,215 @@ __device__ void state_role(const SpParams& p, unsigned char* smem, const uint32_
     }
 
     bool alive = true;
-    auto wait = [&](int i, int c) { return mbar_wait(&bars[i], (uint32_t)(c & 1), ctx, kStatusWaitPrefill); };
     // What this warp wrote for the tensor core, or left in (or took out of) tensor memory, is there: one arrival a warp.
     auto arrive = [&](int i) {
         tc::fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive(&bars[i]);
     };
-    // S as bf16 cells for chunk c's products, then the decayed S back to tensor memory.
+    // This thread's value channel (tensor-memory lane), 32 key channels of the state and 16 rows of the other accumulators.
+    const int v = quad * 32 + lane, k_first = cg * 32, i0 = cg * 16;
+    // S^T as bf16 pairs for chunk c's products, then the decayed S^T back.
     auto begin_chunk = [&](int c) -> bool {
-        if (!wait(bFull, c)) return false;
-        uint32_t r[C];
-        tc::tmem_ld<C>(tc::tmem_addr(tm, quad, tS + cg * C), r);
-        const float el = reinterpret_cast<const float*>(smem + sSlot + wEgl)[lane_row128];
+        uint32_t r[32], pr[16];
+        tc::tmem_ld32(tc::tmem_addr(tm, quad, tS + k_first), r);
         tc::tmem_ld_wait();
-        if (p.state_bf16) {
 #pragma unroll
-            for (int jj = 0; jj < C; ++jj) r[jj] = __float_as_uint(bf16_round(__uint_as_float(r[jj])));
-        }
-#pragma unroll
-        for (int cc = 0; cc < CELLS; ++cc) *reinterpret_cast<uint4*>(cell(smem + sS16, 128, cg * CELLS + cc, lane_row128)) = pack8(r + cc * 8);
-        fence_proxy_async_smem();
+        for (int x = 0; x < 16; ++x) pr[x] = tc::bf16x2(__uint_as_float(r[2 * x]), __uint_as_float(r[2 * x + 1]));
+        tc::tmem_st16(tc::tmem_addr(tm, quad, tS16 + k_first / 2), pr);
+        tc::tmem_st_wait();
         arrive(bS16);
+        if (p.state_bf16) {  // a bf16 state is rounded once per chunk
 #pragma unroll
-        for (int jj = 0; jj < C; ++jj) r[jj] = __float_as_uint(__uint_as_float(r[jj]) * el);
-        tc::tmem_st<C>(tc::tmem_addr(tm, quad, tS + cg * C), r);
+            for (int x = 0; x < 16; ++x) {
+                r[2 * x] = pr[x] << 16;
+                r[2 * x + 1] = pr[x] & 0xffff0000u;
+            }
+        }
+        if (!wait(bFullMKd + (c & 1), c >> 1)) return false;
+        const float4* el = reinterpret_cast<const float4*>(smem + sE + (c & 1) * 512 + k_first * 4);
+#pragma unroll
+        for (int x = 0; x < 8; ++x) {
+            const float4 e = el[x];
+            r[4 * x] = __float_as_uint(__uint_as_float(r[4 * x]) * e.x);
+            r[4 * x + 1] = __float_as_uint(__uint_as_float(r[4 * x + 1]) * e.y);
+            r[4 * x + 2] = __float_as_uint(__uint_as_float(r[4 * x + 2]) * e.z);
+            r[4 * x + 3] = __float_as_uint(__uint_as_float(r[4 * x + 3]) * e.w);
+        }
+        tc::tmem_st32(tc::tmem_addr(tm, quad, tS + k_first), r);
         tc::tmem_st_wait();
         arrive(bSDec);
         return true;
     };
 
-    // ---- the incoming state into tensor memory: lane = key channel, columns = value channel -----------------------
+    // ---- the incoming state into tensor memory; a thread's 32 key channels are consecutive in every state buffer ------------
+    const long long s_at = s_elem + (long long)v * DK + k_first;
+    const int b_at = v * DK + k_first;
     {
         const void* src = j0 == 0 ? p.state_in : p.state_out;
-        uint32_t r[C];
+        uint32_t r[32];
+        if (wk.init == 1 || wk.init == 2) {
 #pragma unroll
-        for (int j = 0; j < C; ++j) {
-            const int vch = v0 + cg * C + j;
-            const long long at = s_elem + (long long)vch * DK + lane_row128;
-            float x;
-            if (wk.init == 1) x = 0.0f;
-            else if (wk.init == 2) x = vch == lane_row128 ? 1.0f : 0.0f;
-            else if (wk.init == 3) x = wk.from[vch * DK + lane_row128];
-            else x = p.state_bf16 ? bf16_bits_to_f32(reinterpret_cast<const uint16_t*>(src)[at]) : reinterpret_cast<const float*>(src)[at];
-            r[j] = __float_as_uint(x);
-        }
-        tc::tmem_st<C>(tc::tmem_addr(tm, quad, tS + cg * C), r);
-        tc::tmem_st_wait();
-    }
-    // The warps that share output rows vote at a barrier in every chunk when the norm is fused; one that gives up before it
-    // still takes part.
-    const bool votes = NV == DV && wk.emit && p.gate != nullptr && quad < 2;
-    auto leave = [&] {
-        if (votes) named_bar_all(4 + quad, 128, false);
-        alive = false;
-    };
-    if (j0 < j1 && !begin_chunk(0)) leave();
-
-    for (int j = j0; alive && j < j1; ++j) {
-        const int c = j - j0, n = min(CH, T - j * CH);
-        const uint32_t acc = tA + (uint32_t)(c & 1) * 128 + cg * C;
-        const long long gr0 = row0 + (long long)j * CH;
-        // ---- D = U - W S as bf16 hi + lo cells, by the warps whose lanes hold W S -----------------------------------------
-        if (quad >= 2) {
-            if (!wait(bFull + 1, c) || !wait(bQSWS, c)) { alive = false; break; }
-            tc::fence_after_sync();
-            const int i = lane_row128 - CH;
-            uint32_t r[C];
-            tc::tmem_ld<C>(tc::tmem_addr(tm, quad, acc), r);
-            unsigned char* Ut = smem + sSlot + wU;  // this block's slice of U: NV / 4 cells of four value channels
-            tc::tmem_ld_wait();
+            for (int x = 0; x < 32; ++x) r[x] = wk.init == 2 && k_first + x == v ? __float_as_uint(1.0f) : 0u;
+        } else if (wk.init == 0 && p.state_bf16) {
+            const uint16_t* at = reinterpret_cast<const uint16_t*>(src) + s_at;
+            if ((reinterpret_cast<uintptr_t>(at) & 15) == 0) {
 #pragma unroll
-            for (int cc = 0; cc < CELLS; ++cc) {
-                const float4 u0 = *reinterpret_cast<const float4*>(cell(Ut, CH, cg * (C / 4) + cc * 2, i));
-                const float4 u1 = *reinterpret_cast<const float4*>(cell(Ut, CH, cg * (C / 4) + cc * 2 + 1, i));
-                const float uu[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
-                uint32_t wh[4], wl[4];
+                for (int x = 0; x < 4; ++x) {
+                    const uint4 w = reinterpret_cast<const uint4*>(at)[x];
+                    const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
-                for (int jj = 0; jj < 4; ++jj)
-                    tc::split_bf16x2((wk.use_u ? uu[2 * jj] : 0.0f) - __uint_as_float(r[cc * 8 + 2 * jj]),
-                                     (wk.use_u ? uu[2 * jj + 1] : 0.0f) - __uint_as_float(r[cc * 8 + 2 * jj + 1]), wh[jj], wl[jj]);
-                *reinterpret_cast<uint4*>(cell(smem + sDhi, CH, cg * CELLS + cc, i)) = make_uint4(wh[0], wh[1], wh[2], wh[3]);
-                *reinterpret_cast<uint4*>(cell(smem + sDlo, CH, cg * CELLS + cc, i)) = make_uint4(wl[0], wl[1], wl[2], wl[3]);
-            }
-            fence_proxy_async_smem();
-            arrive(bD);
-            if (lane == 0) mbar_arrive(&empty[1]);  // U is consumed
-        }
-        if (!wait(bSNew, c)) { leave(); break; }
-        tc::fence_after_sync();
-        if (j + 1 < j1 && !begin_chunk(c + 1)) { leave(); break; }
-
-        // ---- outputs: bf16(y), or the gated RMSNorm of bf16(y), by the warps whose lanes hold O --------------------------------
-        if (wk.emit && quad < 2) {
-            bool ok = wait(bO + (c & 1), c >> 1);
-            tc::fence_after_sync();
-            uint32_t r[C];
-            tc::tmem_ld<C>(tc::tmem_addr(tm, quad, acc), r);
-            tc::tmem_ld_wait();
-            arrive(bOFree + (c & 1));
-            const int i = lane_row128;
-            const bool live = i < n;
-            const long long at = ((gr0 + i) * H + h) * DV + v0 + cg * C;
-            float y[C];
-#pragma unroll
-            for (int jj = 0; jj < C; ++jj) y[jj] = bf16_round(__uint_as_float(r[jj]));
-            ok = ok && mbar_wait(&out_empty[c & 1], (uint32_t)(((c >> 1) & 1) ^ 1), ctx, kStatusWaitPrefill);
-            if (votes) {  // the norm needs a row's every value channel: whole-head blocks only
-                float* red = reinterpret_cast<float*>(smem + sRed) + (c & 1) * 4 * CH;
-                float ss = 0.0f;
-#pragma unroll
-                for (int jj = 0; jj < C; ++jj) ss = fmaf(y[jj], y[jj], ss);
-                red[cg * CH + i] = ss;
-                // The four warps that share these rows meet here, and decide together whether they go on.
-                ok = named_bar_all(4 + quad, 128, ok);
-                if (live && ok) {
-                    const float tot = (red[i] + red[CH + i]) + (red[2 * CH + i] + red[3 * CH + i]);
-                    const float rinv = 1.0f / sqrtf(tot / (float)DV + p.eps);
-#pragma unroll
-                    for (int jj = 0; jj < C; ++jj) {
-                        const float gt = bf16_bits_to_f32(p.gate[at + jj]), w = bf16_bits_to_f32(p.norm_w[cg * C + jj]);
-                        y[jj] = w * (y[jj] * rinv) * (1.0f / (1.0f + __expf(-gt)));
+                    for (int y = 0; y < 4; ++y) {
+                        r[8 * x + 2 * y] = ww[y] << 16;
+                        r[8 * x + 2 * y + 1] = ww[y] & 0xffff0000u;
                     }
                 }
-            }
-            // Into the output tile (the output warp takes it from there).
-            if (!ok) { alive = false; break; }
-            unsigned char* dst = smem + sOut + (c & 1) * kOutTile;
+            } else {
 #pragma unroll
-            for (int c4 = 0; c4 < CELLS; ++c4)
-                *reinterpret_cast<uint4*>(dst + box_piece(i, cg * CELLS + c4)) = make_uint4(tc::bf16x2(y[c4 * 8], y[c4 * 8 + 1]), tc::bf16x2(y[c4 * 8 + 2], y[c4 * 8 + 3]),
-                                                                      tc::bf16x2(y[c4 * 8 + 4], y[c4 * 8 + 5]), tc::bf16x2(y[c4 * 8 + 6], y[c4 * 8 + 7]));
-            fence_proxy_async_smem();  // the tensor stores read the tile through the async proxy
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&out_full[c & 1]);
+                for (int x = 0; x < 32; ++x) r[x] = (uint32_t)at[x] << 16;
+            }
+        } else {
+            const float* at = wk.init == 3 ? wk.from + b_at : reinterpret_cast<const float*>(src) + s_at;
+            if ((reinterpret_cast<uintptr_t>(at) & 15) == 0) {
+#pragma unroll
+                for (int x = 0; x < 8; ++x) {
+                    const uint4 w = reinterpret_cast<const uint4*>(at)[x];
+                    r[4 * x] = w.x; r[4 * x + 1] = w.y; r[4 * x + 2] = w.z; r[4 * x + 3] = w.w;
+                }
+            } else {
+#pragma unroll
+                for (int x = 0; x < 32; ++x) r[x] = __float_as_uint(at[x]);
+            }
         }
+        tc::tmem_st32(tc::tmem_addr(tm, quad, tS + k_first), r);
+        tc::tmem_st_wait();
     }
+    // The four warps that share output rows vote at a barrier in every chunk when the norm is fused; one that gives up before
+    // it still takes part.
+    const bool votes = wk.emit && p.gate != nullptr;
+    auto leave = [&] {
+        if (votes) named_bar_all(4 + cg, 128, false);
+        alive = false;
+    };
+    if (count > 0 && !begin_chunk(0)) leave();
+
+    const float nw = votes ? bf16_bits_to_f32(p.norm_w[v]) : 0.0f;
+    // ---- a chunk's outputs: bf16(y), or the gated RMSNorm of bf16(y) ---------------------------------------------------
+    auto emit = [&](int c) -> bool {
+        const int i_first = (j0 + c) * CH, n = min(CH, T - i_first);
+        const long long gr0 = row0 + i_first;
+        bool ok = wait(bO + (c & 1), c >> 1);
+        tc::fence_after_sync();
+        uint32_t r[16];
+        tc::tmem_ld16(tc::tmem_addr(tm, quad, tO + (uint32_t)(c & 1) * 64 + i0), r);
+        tc::tmem_ld_wait();
+        arrive(bOFree + (c & 1));
+        ok = ok && wait(bOutEmpty + (c & 1), (c >> 1) ^ 1);
+        if (votes) {  // the norm needs a row's every value channel: whole-head blocks only
+            float y[16], gt[16], sq[16];
+#pragma unroll
+            for (int x = 0; x < 16; ++x) {
+                y[x] = bf16_round(__uint_as_float(r[x]));
+                sq[x] = y[x] * y[x];
+                gt[x] = i0 + x < n ? bf16_bits_to_f32(p.gate[((gr0 + i0 + x) * H + h) * DV + v]) : 0.0f;
+            }
+            // The sixteen rows' sums over the warp's 32 channels: lane l ends with row l / 2's.
+#pragma unroll
+            for (int half = 8; half >= 1; half >>= 1) {
+                const bool up = (lane & (2 * half)) != 0;
+#pragma unroll
+                for (int x = 0; x < half; ++x) sq[x] = (up ? sq[half + x] : sq[x]) + __shfl_xor_sync(0xffffffffu, up ? sq[x] : sq[half + x], 2 * half);
+            }
+            sq[0] += __shfl_xor_sync(0xffffffffu, sq[0], 1);
+            float* red = reinterpret_cast<float*>(smem + sRed) + (c & 1) * 4 * CH;
+            if ((lane & 1) == 0) red[quad * CH + i0 + (lane >> 1)] = sq[0];
+            ok = named_bar_all(4 + cg, 128, ok);
+            float rinv = 0.0f;
+            if (lane < 16) {
+                const float tot = (red[i0 + lane] + red[CH + i0 + lane]) + (red[2 * CH + i0 + lane] + red[3 * CH + i0 + lane]);
+                rinv = 1.0f / sqrtf(tot / (float)DV + p.eps);
+            }
+#pragma unroll
+            for (int x = 0; x < 16; ++x)
+                r[x] = __float_as_uint(nw * (y[x] * __shfl_sync(0xffffffffu, rinv, x)) * __fdividef(1.0f, 1.0f + __expf(-gt[x])));
+        }
+        // Into the output tile (the output warp takes it from there).
+        if (!ok) return false;
+        unsigned char* dst = smem + sOut + (c & 1) * kOutTile;
+        {
+#pragma unroll
+            for (int x = 0; x < 16; x += 2) {
+                const uint32_t two = tc::bf16x2(__uint_as_float(r[x]), __uint_as_float(r[x + 1]));
+                *reinterpret_cast<uint16_t*>(dst + box_piece(i0 + x, v >> 3) + (v & 7) * 2) = (uint16_t)two;
+                *reinterpret_cast<uint16_t*>(dst + box_piece(i0 + x + 1, v >> 3) + (v & 7) * 2) = (uint16_t)(two >> 16);
+            }
+        }
+        fence_proxy_async_smem();  // the tensor stores read the tile through the async proxy
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars[bOutFull + (c & 1)]);
+        return true;
+    };
+    for (int c = 0; alive && c < count; ++c) {
+        // ---- D^T = U^T - (W S)^T as bf16 hi + lo pairs of rows ------------------------------------------------------------
+        float uu[16];
+        if (!wait(bFullU, c)) { leave(); break; }
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+            const float4 u4 = *reinterpret_cast<const float4*>(smem + sU + u_cell(cg * 4 + x, v));
+            uu[4 * x] = wk.use_u ? u4.x : 0.0f; uu[4 * x + 1] = wk.use_u ? u4.y : 0.0f; uu[4 * x + 2] = wk.use_u ? u4.z : 0.0f; uu[4 * x + 3] = wk.use_u ? u4.w : 0.0f;
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars[bEmptyU]);  // U is consumed
+        if (!wait(bWS, c)) { leave(); break; }
+        tc::fence_after_sync();
+        {
+            uint32_t r[16], wh[8], wl[8];
+            tc::tmem_ld16(tc::tmem_addr(tm, quad, tWS + i0), r);
+            tc::tmem_ld_wait();
+#pragma unroll
+            for (int x = 0; x < 8; ++x) tc::split_bf16x2(uu[2 * x] - __uint_as_float(r[2 * x]), uu[2 * x + 1] - __uint_as_float(r[2 * x + 1]), wh[x], wl[x]);
+            tc::tmem_st8(tc::tmem_addr(tm, quad, tDhi + i0 / 2), wh);
+            tc::tmem_st8(tc::tmem_addr(tm, quad, tDlo + i0 / 2), wl);
+            tc::tmem_st_wait();
+            arrive(bD);
+        }
+        // The outputs of the chunk before leave while the state's product runs.
+        if (wk.emit && c > 0 && !emit(c - 1)) { alive = false; break; }
+        if (!wait(bSNew, c)) { leave(); break; }
+        tc::fence_after_sync();
+        if (c + 1 < count && !begin_chunk(c + 1)) { leave(); break; }
+    }
+    if (alive && wk.emit && count > 0 && !emit(count - 1)) alive = false;
 
     // ---- the outgoing state ---------------------------------------------------------------------------------------------
-    if (alive) {
-        uint32_t r[C];
-        tc::tmem_ld<C>(tc::tmem_addr(tm, quad, tS + cg * C), r);
+    if (alive && wk.fin != 2) {
+        uint32_t r[32];
+        tc::tmem_ld32(tc::tmem_addr(tm, quad, tS + k_first), r);
         tc::tmem_ld_wait();
+        if (wk.fin == 0 && p.state_bf16) {
+            uint16_t* at = reinterpret_cast<uint16_t*>(p.state_out) + s_at;
+            uint32_t pr[16];
 #pragma unroll
-        for (int j = 0; j < C; ++j) {
-            const long long at = s_elem + (long long)(v0 + cg * C + j) * DK + lane_row128;
-            if (wk.fin == 2) continue;
-            if (wk.fin == 1) wk.to[(v0 + cg * C + j) * DK + lane_row128] = __uint_as_float(r[j]);
-            else if (p.state_bf16) reinterpret_cast<uint16_t*>(p.state_out)[at] = f32_to_bf16_bits(__uint_as_float(r[j]));
-            else reinterpret_cast<float*>(p.state_out)[at] = __uint_as_float(r[j]);
+            for (int x = 0; x < 16; ++x) pr[x] = tc::bf16x2(__uint_as_float(r[2 * x]), __uint_as_float(r[2 * x + 1]));
+            if ((reinterpret_cast<uintptr_t>(at) & 15) == 0) {
+#pragma unroll
+                for (int x = 0; x < 4; ++x) reinterpret_cast<uint4*>(at)[x] = make_uint4(pr[4 * x], pr[4 * x + 1], pr[4 * x + 2], pr[4 * x + 3]);
+            } else {
+#pragma unroll
+                for (int x = 0; x < 16; ++x) {
+                    at[2 * x] = (uint16_t)pr[x];
+                    at[2 * x + 1] = (uint16_t)(pr[x] >> 16);
+                }
+            }
+        } else {
+            float* at = wk.fin == 1 ? wk.to + b_at : reinterpret_cast<float*>(p.state_out) + s_at;
+            if ((reinterpret_cast<uintptr_t>(at) & 15) == 0) {
+#pragma unroll
+                for (int x = 0; x < 8; ++x) reinterpret_cast<uint4*>(at)[x] = make_uint4(r[4 * x], r[4 * x + 1], r[4 * x + 2], r[4 * x + 3]);
+            } else {
+#pragma unroll
+                for (int x = 0; x < 32; ++x) at[x] = __uint_as_float(r[x]);
+            }
         }
     }
     tc::fence_before_sync();
@@ -957,7 +1006,7 @@ __global__ void __launch_bounds__(kThreadsSp, 1) prefill_sp_kernel(const __grid_
             const int end = last ? (p.scan_open ? 0x7fffffff : hi) : min(p.state_chunk0 + (sg + 1) * p.scan_chunks, hi);
             const Walk wk{min(p.state_chunk0 + sg * p.scan_chunks, hi), end, kind ? 2 : 1, nullptr, 1,
                           p.scan_ab + (((size_t)chain * p.scan_p1 + sg) * 2 + kind) * DV * DK, kind == 0, false};
-            state_role<DV>(p, smem, tm, chain, 0, wk);
+            state_role(p, smem, tm, chain, wk);
         }
     } else if (p.scan_pass == 2) {  // (chain, segment): the walk with outputs from the segment's true incoming state
         const int sg = blockIdx.x % p.scan_k, chain = blockIdx.x / p.scan_k;
@@ -966,16 +1015,13 @@ __global__ void __launch_bounds__(kThreadsSp, 1) prefill_sp_kernel(const __grid_
             const bool last = sg == p.scan_k - 1;
             const int hi = p.state_chunk0 + p.seg_chunks;
             const int end = last ? (p.scan_open ? 0x7fffffff : hi) : min(p.state_chunk0 + (sg + 1) * p.scan_chunks, hi);
-            const bool carried = sg == 0 && p.scan_carry_in != nullptr;  // a later super-block: its incoming state is a composed one
-            const Walk wk{min(p.state_chunk0 + sg * p.scan_chunks, hi), end, sg == 0 && !carried ? 0 : 3,
-                          carried ? p.scan_carry_in + (size_t)chain * DV * DK : p.scan_start + ((size_t)chain * p.scan_k + sg) * DV * DK,
+            const Walk wk{min(p.state_chunk0 + sg * p.scan_chunks, hi), end, 3, p.scan_start + ((size_t)chain * p.scan_k + sg) * DV * DK,
                           last ? 0 : 2, nullptr, true, true};
-            state_role<DV>(p, smem, tm, chain, 0, wk);
+            state_role(p, smem, tm, chain, wk);
         }
-    } else if (p.has_state && blockIdx.x < (unsigned)(chains * p.parts)) {
+    } else if (p.has_state && blockIdx.x < (unsigned)chains) {
         const Walk wk{p.state_chunk0, p.state_chunk0 + p.seg_chunks, 0, nullptr, 0, nullptr, true, true};
-        if (p.parts == 2) state_role<64>(p, smem, tm, (int)(blockIdx.x >> 1), (int)(blockIdx.x & 1), wk);
-        else state_role<DV>(p, smem, tm, (int)blockIdx.x, 0, wk);
+        state_role(p, smem, tm, (int)blockIdx.x, wk);
         tc::fence_after_sync();
     }
     if (p.has_intra && ctl[1] == 0u) intra_role(p, smem, tm);
@@ -996,8 +1042,13 @@ __global__ void __launch_bounds__(128) scan_compose_kernel(const __grid_constant
     const int b = chain / p.H, h = chain % p.H;
     const float* s0 = p.scan_carry_in != nullptr ? p.scan_carry_in + (size_t)chain * DV * DK
                                                  : reinterpret_cast<const float*>(p.state_in) + p.state_off[b] + (long long)h * DV * DK;
+    // Segment 0 starts from a copy: in place, the last segment of a sequence that ends early writes the final state over the
+    // caller's before segment 0 may have read it.
 #pragma unroll
-    for (int vi = 0; vi < kCols; ++vi) S[vi][k] = s0[(v0 + vi) * DK + k];
+    for (int vi = 0; vi < kCols; ++vi) {
+        S[vi][k] = s0[(v0 + vi) * DK + k];
+        p.scan_start[(size_t)chain * p.scan_k * DV * DK + (v0 + vi) * DK + k] = S[vi][k];
+    }
     __syncthreads();
     for (int sg = 0; sg < p.scan_p1; ++sg) {
         const float* B = p.scan_ab + ((size_t)chain * p.scan_p1 + sg) * 2 * DV * DK;
@@ -1131,9 +1182,6 @@ int core_prefill_sp_launch(int32_t heads, int32_t batch, const int32_t* cu_seqle
     } else if (out == nullptr) {
         return kInvalid;
     }
-    // Few chains: the serial walk over a chain's chunks is the critical path, so two blocks share each chain.  (Not with
-    // the fused output norm, which needs a row's every value channel in one block.)
-    p.parts = (gate == nullptr && chains * 2 <= 64) ? 2 : 1;
     p.seg_chunks = (int)seg;
     unsigned char* base = reinterpret_cast<unsigned char*>(workspace);
     unsigned char* half[2] = {base, overlap ? base + chains * seg * kSlotBytes : base};
@@ -1201,7 +1249,6 @@ int core_prefill_sp_launch(int32_t heads, int32_t batch, const int32_t* cu_seqle
                     const long long c0 = b * sb, cnt = (need - c0) < sb ? (need - c0) : sb;
                     if (cnt <= 0) break;
                     const long long Kb = cnt >= min_seg * Ks ? Ks : (cnt / min_seg > 1 ? cnt / min_seg : 1);
-                    p.parts = 1;
                     p.seg_chunks = (int)cnt;
                     p.intra_chunk0 = p.state_chunk0 = (int)c0;
                     p.ws_intra = p.ws_state = base + b * chains * sb * kSlotBytes;
@@ -1247,7 +1294,6 @@ int core_prefill_sp_launch(int32_t heads, int32_t batch, const int32_t* cu_seqle
         const long long scratch = chains * (3 * K - 2) * (long long)(DV * DK * sizeof(float));
         if (K >= 2 && !bf16_state && chains * need * kSlotBytes + scratch <= usable) {
             p.seg_chunks = (int)need;
-            p.parts = 1;
             p.ws_intra = p.ws_state = base;
             p.intra_chunk0 = p.state_chunk0 = 0;
             p.ctr = 0;
@@ -1282,7 +1328,7 @@ int core_prefill_sp_launch(int32_t heads, int32_t batch, const int32_t* cu_seqle
         p.ws_intra = half[intra_seg & 1];
         p.ws_state = half[state_seg & 1];
         p.ctr = launch_no++ & 1;
-        long long grid = p.has_state ? chains * p.parts : 0;
+        long long grid = p.has_state ? chains : 0;
         if (p.has_intra) {
             const long long items = chains * seg, want = items < sms ? items : sms;
             if (grid < want) grid = want;
