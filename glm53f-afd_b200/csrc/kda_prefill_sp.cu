@@ -853,65 +853,102 @@ __device__ void state_role(const SpParams& p, unsigned char* smem, const uint32_
     };
     if (count > 0 && !begin_chunk(0)) leave();
 
-    const float nw = votes ? bf16_bits_to_f32(p.norm_w[v]) : 0.0f;
     // ---- a chunk's outputs: bf16(y), or the gated RMSNorm of bf16(y) ---------------------------------------------------
-    auto emit = [&](int c) -> bool {
+    // O^T is read in the fragment layout, from which a transposing matrix store puts rows of the output into the tile: this
+    // thread's values are (channel fv + 8 q, row fi + 8 g + e), q < 4, g < 2, e < 2.
+    const int fv = quad * 32 + (lane >> 2), fi = i0 + 2 * (lane & 3);
+    float nw[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    if (votes)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) nw[q] = bf16_bits_to_f32(p.norm_w[fv + 8 * q]);
+    // With the norm fused a chunk's gate values are fetched before D is formed, so that their latency is not in the walk.
+    uint16_t gt[2][2][4];
+    auto fetch_gate = [&](int c) {
         const int i_first = (j0 + c) * CH, n = min(CH, T - i_first);
-        const long long gr0 = row0 + i_first;
+        const uint16_t* at = p.gate + ((row0 + i_first + fi) * H + h) * DV + fv;
+#pragma unroll
+        for (int g = 0; g < 2; ++g)
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) gt[g][e][q] = fi + 8 * g + e < n ? at[(long long)(8 * g + e) * H * DV + 8 * q] : (uint16_t)0;
+    };
+    auto emit = [&](int c) -> bool {
         bool ok = wait(bO + (c & 1), c >> 1);
         tc::fence_after_sync();
-        uint32_t r[16];
-        tc::tmem_ld16(tc::tmem_addr(tm, quad, tO + (uint32_t)(c & 1) * 64 + i0), r);
+        uint32_t ra[8], rb[8];
+        const uint32_t at = tc::tmem_addr(tm, quad, tO + (uint32_t)(c & 1) * 64 + i0);
+        tc::tmem_ld_frag(at, ra);
+        tc::tmem_ld_frag(at + (16u << 16), rb);
         tc::tmem_ld_wait();
         arrive(bOFree + (c & 1));
         ok = ok && wait(bOutEmpty + (c & 1), (c >> 1) ^ 1);
-        if (votes) {  // the norm needs a row's every value channel: whole-head blocks only
-            float y[16], gt[16], sq[16];
+        uint32_t y2[2][4];  // [g][q]: rows fi + 8 g and the next of channel fv + 8 q
 #pragma unroll
-            for (int x = 0; x < 16; ++x) {
-                y[x] = bf16_round(__uint_as_float(r[x]));
-                sq[x] = y[x] * y[x];
-                gt[x] = i0 + x < n ? bf16_bits_to_f32(p.gate[((gr0 + i0 + x) * H + h) * DV + v]) : 0.0f;
-            }
-            // The sixteen rows' sums over the warp's 32 channels: lane l ends with row l / 2's.
-#pragma unroll
-            for (int half = 8; half >= 1; half >>= 1) {
-                const bool up = (lane & (2 * half)) != 0;
-#pragma unroll
-                for (int x = 0; x < half; ++x) sq[x] = (up ? sq[half + x] : sq[x]) + __shfl_xor_sync(0xffffffffu, up ? sq[x] : sq[half + x], 2 * half);
-            }
-            sq[0] += __shfl_xor_sync(0xffffffffu, sq[0], 1);
-            float* red = reinterpret_cast<float*>(smem + sRed) + (c & 1) * 4 * CH;
-            if ((lane & 1) == 0) red[quad * CH + i0 + (lane >> 1)] = sq[0];
-            ok = named_bar_all(4 + cg, 128, ok);
-            float rinv = 0.0f;
-            if (lane < 16) {
-                const float tot = (red[i0 + lane] + red[CH + i0 + lane]) + (red[2 * CH + i0 + lane] + red[3 * CH + i0 + lane]);
-                rinv = 1.0f / sqrtf(tot / (float)DV + p.eps);
-            }
-#pragma unroll
-            for (int x = 0; x < 16; ++x)
-                r[x] = __float_as_uint(nw * (y[x] * __shfl_sync(0xffffffffu, rinv, x)) * __fdividef(1.0f, 1.0f + __expf(-gt[x])));
+        for (int g = 0; g < 2; ++g) {
+            y2[g][0] = tc::bf16x2(__uint_as_float(ra[4 * g]), __uint_as_float(ra[4 * g + 1]));
+            y2[g][1] = tc::bf16x2(__uint_as_float(ra[4 * g + 2]), __uint_as_float(ra[4 * g + 3]));
+            y2[g][2] = tc::bf16x2(__uint_as_float(rb[4 * g]), __uint_as_float(rb[4 * g + 1]));
+            y2[g][3] = tc::bf16x2(__uint_as_float(rb[4 * g + 2]), __uint_as_float(rb[4 * g + 3]));
         }
-        // Into the output tile (the output warp takes it from there).
+        if (votes) {
+            float sq[2][2];
+#pragma unroll
+            for (int g = 0; g < 2; ++g) {
+                sq[g][0] = sq[g][1] = 0.0f;
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const float lo = __uint_as_float(y2[g][q] << 16), hi = __uint_as_float(y2[g][q] & 0xffff0000u);
+                    sq[g][0] = fmaf(lo, lo, sq[g][0]);
+                    sq[g][1] = fmaf(hi, hi, sq[g][1]);
+                }
+#pragma unroll
+                for (int o = 4; o <= 16; o <<= 1) {
+                    sq[g][0] += __shfl_xor_sync(0xffffffffu, sq[g][0], o);
+                    sq[g][1] += __shfl_xor_sync(0xffffffffu, sq[g][1], o);
+                }
+            }
+            float* red = reinterpret_cast<float*>(smem + sRed) + (c & 1) * 4 * CH + fi;
+            if (lane < 4)
+#pragma unroll
+                for (int g = 0; g < 2; ++g) *reinterpret_cast<float2*>(red + quad * CH + 8 * g) = make_float2(sq[g][0], sq[g][1]);
+            ok = named_bar_all(4 + cg, 128, ok);
+#pragma unroll
+            for (int g = 0; g < 2; ++g) {
+                float tot[2] = {0.0f, 0.0f}, rinv[2];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const float2 s2 = *reinterpret_cast<const float2*>(red + q * CH + 8 * g);
+                    tot[0] += s2.x;
+                    tot[1] += s2.y;
+                }
+#pragma unroll
+                for (int e = 0; e < 2; ++e) rinv[e] = 1.0f / sqrtf(tot[e] / (float)DV + p.eps);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const float lo = __uint_as_float(y2[g][q] << 16), hi = __uint_as_float(y2[g][q] & 0xffff0000u);
+                    y2[g][q] = tc::bf16x2(nw[q] * (lo * rinv[0]) * __fdividef(1.0f, 1.0f + __expf(-bf16_bits_to_f32(gt[g][0][q]))),
+                                          nw[q] * (hi * rinv[1]) * __fdividef(1.0f, 1.0f + __expf(-bf16_bits_to_f32(gt[g][1][q]))));
+                }
+            }
+        }
+        // Into the output tile (the output warp takes it from there): a lane names the row (lane % 8) of matrix lane / 8, the
+        // matrices being (channels 8 (m % 2), rows 8 (m / 2)) of the two halves of the warp's channels.
         if (!ok) return false;
         unsigned char* dst = smem + sOut + (c & 1) * kOutTile;
-        {
-#pragma unroll
-            for (int x = 0; x < 16; x += 2) {
-                const uint32_t two = tc::bf16x2(__uint_as_float(r[x]), __uint_as_float(r[x + 1]));
-                *reinterpret_cast<uint16_t*>(dst + box_piece(i0 + x, v >> 3) + (v & 7) * 2) = (uint16_t)two;
-                *reinterpret_cast<uint16_t*>(dst + box_piece(i0 + x + 1, v >> 3) + (v & 7) * 2) = (uint16_t)(two >> 16);
-            }
-        }
+        const int row = i0 + (lane >> 4) * 8 + (lane & 7), piece = quad * 4 + ((lane >> 3) & 1);
+        tc::stmatrix_t4(dst + box_piece(row, piece), y2[0][0], y2[0][1], y2[1][0], y2[1][1]);
+        tc::stmatrix_t4(dst + box_piece(row, piece + 2), y2[0][2], y2[0][3], y2[1][2], y2[1][3]);
         fence_proxy_async_smem();  // the tensor stores read the tile through the async proxy
         __syncwarp();
         if (lane == 0) mbar_arrive(&bars[bOutFull + (c & 1)]);
         return true;
     };
+
     for (int c = 0; alive && c < count; ++c) {
         // ---- D^T = U^T - (W S)^T as bf16 hi + lo pairs of rows ------------------------------------------------------------
         float uu[16];
+        if (votes && c > 0) fetch_gate(c - 1);
         if (!wait(bFullU, c)) { leave(); break; }
 #pragma unroll
         for (int x = 0; x < 4; ++x) {
@@ -939,7 +976,10 @@ __device__ void state_role(const SpParams& p, unsigned char* smem, const uint32_
         tc::fence_after_sync();
         if (c + 1 < count && !begin_chunk(c + 1)) { leave(); break; }
     }
-    if (alive && wk.emit && count > 0 && !emit(count - 1)) alive = false;
+    if (alive && wk.emit && count > 0) {
+        if (votes) fetch_gate(count - 1);
+        alive = emit(count - 1);
+    }
 
     // ---- the outgoing state ---------------------------------------------------------------------------------------------
     if (alive && wk.fin != 2) {
