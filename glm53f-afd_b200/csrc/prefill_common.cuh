@@ -49,6 +49,38 @@ __device__ __forceinline__ void compute_sync() { named_bar_sync(1, kCompute); }
 
 __device__ __forceinline__ unsigned char* cell(unsigned char* tile, int R, int c, int r) { return tile + ((size_t)c * R + r) * 16; }
 
+// Two-wide FP32 products (each half rounded once).
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+    unsigned long long r, x, y;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(x) : "f"(a.x), "f"(a.y));
+    asm("mov.b64 %0, {%1, %2};" : "=l"(y) : "f"(b.x), "f"(b.y));
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(x), "l"(y));
+    float2 c;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(c.x), "=f"(c.y) : "l"(r));
+    return c;
+}
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 d) {
+    unsigned long long r, x, y, z;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(x) : "f"(a.x), "f"(a.y));
+    asm("mov.b64 %0, {%1, %2};" : "=l"(y) : "f"(b.x), "f"(b.y));
+    asm("mov.b64 %0, {%1, %2};" : "=l"(z) : "f"(d.x), "f"(d.y));
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(x), "l"(y), "l"(z));
+    float2 c;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(c.x), "=f"(c.y) : "l"(r));
+    return c;
+}
+__device__ __forceinline__ float rcp_approx(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float ex2_approx(float x) {
+    float r;
+    asm("ex2.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+constexpr float kLog2e = 1.4426950408889634f;
+
 // Eight FP32 values (TMEM words) to one 16-byte cell of bf16.
 __device__ __forceinline__ uint4 pack8(const uint32_t* r) {
     return make_uint4(tc::bf16x2(__uint_as_float(r[0]), __uint_as_float(r[1])), tc::bf16x2(__uint_as_float(r[2]), __uint_as_float(r[3])),
@@ -60,49 +92,47 @@ __device__ __forceinline__ uint4 pack8(const uint32_t* r) {
 // diagonal blocks come by substitution; then the lower-left sz x sz block of every 2sz x 2sz diagonal block is
 // -T22 (L21 T11), sz = 16 and 32.
 //
-// The merges run on the warp-level tensor instruction (m16n8k8, tf32) with every operand split into two tf32 halves and three
-// products, 21 bits of operand mantissa: these contractions are too small for a round through tensor memory (publish, issue,
-// wait, read back: about 1,000 cycles), and as multiply-adds from shared memory they took 6,500 of an item's 31,000 cycles.
-__device__ __forceinline__ uint32_t tf32_of(float x) {
-    uint32_t r;
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
-    return r;
+// The merges are FP32 multiply-adds throughout.  A lane holds a 4 x 4 tile of the result over a quarter of the k range (kp = lane >> 3
+// picks four of every sixteen, so that eight lanes read one row: no bank conflicts); two 16-byte reads feed sixteen products.  The
+// four quarters meet by shuffles, after which kp is the tile's row.  The whole inverse, four blocks of 256 threads per SM: 5,500 cycles;
+// rows of four columns a thread over all of k, 5,900 to 7,500; the warp-level tensor instruction with operands split into two tf32
+// halves, 5,300, but at 2.2 to 2.7 times the FP32 error in the merged blocks.
+__device__ __forceinline__ void row_fma(float2 (&c)[2], float a, const float4& b) {
+    c[0] = fma2({a, a}, {b.x, b.y}, c[0]);
+    c[1] = fma2({a, a}, {b.z, b.w}, c[1]);
 }
-__device__ __forceinline__ void split_tf32(float x, uint32_t& hi, uint32_t& lo) {
-    hi = tf32_of(x);
-    lo = tf32_of(x - __uint_as_float(hi));
-}
-__device__ __forceinline__ void mma_tf32(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
-    asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
-}
-// c += A B over k in [k0, k1) (multiples of 8), c a 16 x 8 tile of one warp: element (i, k) of A at A[i * AI + k * AK], (k, j) of B at
-// B[k * BK + j].
-template <int AI, int AK, int BK>
-__device__ __forceinline__ void tile_product(float (&c)[4], const float* A, const float* B, int k0, int k1, int lane) {
-    const int g = lane >> 2, t = lane & 3;
-#pragma unroll 2
-    for (int k = k0; k < k1; k += 8) {
-        uint32_t ah[4], al[4], bh[2], bl[2];
-        split_tf32(A[g * AI + (k + t) * AK], ah[0], al[0]);
-        split_tf32(A[(g + 8) * AI + (k + t) * AK], ah[1], al[1]);
-        split_tf32(A[g * AI + (k + t + 4) * AK], ah[2], al[2]);
-        split_tf32(A[(g + 8) * AI + (k + t + 4) * AK], ah[3], al[3]);
-        split_tf32(B[(k + t) * BK + g], bh[0], bl[0]);
-        split_tf32(B[(k + t + 4) * BK + g], bh[1], bl[1]);
-        mma_tf32(c, al, bh);
-        mma_tf32(c, ah, bl);
-        mma_tf32(c, ah, bh);
+__device__ __forceinline__ float pick(const float4& x, int s) { return s == 0 ? x.x : s == 1 ? x.y : s == 2 ? x.z : x.w; }
+// Sixteen of k.  A transposed (AT): element (i, k) at A[k * LS + i]; else at A[i * LS + k].  (k, j) of B at B[k * BK + j].
+template <bool AT, int BK>
+__device__ __forceinline__ void tile_step(float2 (&c)[4][2], const float* A, const float* B, int kp) {
+    A += AT ? kp * 4 * LS : kp * 4;
+    B += kp * 4 * BK;
+    float4 a[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) a[u] = *reinterpret_cast<const float4*>(A + u * LS);
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+        const float4 b = *reinterpret_cast<const float4*>(B + s * BK);
+        const float col[4] = {AT ? a[s].x : pick(a[0], s), AT ? a[s].y : pick(a[1], s), AT ? a[s].z : pick(a[2], s), AT ? a[s].w : pick(a[3], s)};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) row_fma(c[i], col[i], b);
     }
 }
-template <int LD>
-__device__ __forceinline__ void tile_store(float* C, const float (&c)[4], float sign, int lane) {
-    const int g = lane >> 2, t = lane & 3;
-    *reinterpret_cast<float2*>(C + g * LD + 2 * t) = make_float2(sign * c[0], sign * c[1]);
-    *reinterpret_cast<float2*>(C + (g + 8) * LD + 2 * t) = make_float2(sign * c[2], sign * c[3]);
+__device__ __forceinline__ float4 tile_row(const float2 (&c)[4][2], int kp) {
+    float h[2][4], r[4];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+            const float lo = v & 1 ? c[i][v >> 1].y : c[i][v >> 1].x, hi = v & 1 ? c[2 + i][v >> 1].y : c[2 + i][v >> 1].x;
+            h[i][v] = ((kp & 2) ? hi : lo) + __shfl_xor_sync(0xffffffffu, (kp & 2) ? lo : hi, 16);
+        }
+    }
+#pragma unroll
+    for (int v = 0; v < 4; ++v) r[v] = ((kp & 1) ? h[1][v] : h[0][v]) + __shfl_xor_sync(0xffffffffu, (kp & 1) ? h[0][v] : h[1][v], 8);
+    return make_float4(r[0], r[1], r[2], r[3]);
 }
-constexpr int PS = 40;  // row stride of the merges' intermediate product (32 x 32): conflict-free as a B operand
+constexpr int PS = 36;  // row stride of the merges' intermediate product
 
 // NT threads (numbered tid = 0 .. NT-1, at least eight warps) take part and meet at named barrier `bar`; ends with a barrier.
 template <int NT = kCompute>
@@ -134,29 +164,34 @@ __device__ __forceinline__ void invert(const float* Lm, float* Tm, float* Pm, in
         }
     }
     named_bar_sync(bar, NT);
+    const int kp = lane >> 3;
     if (warp < 4) {  // sz = 16: a warp has eight columns of one of the two blocks, which need nothing of the other columns
-        const int r0 = (warp >> 1) * 32 + 16, c0 = r0 - 16, j0 = (warp & 1) * 8;
-        float* P = Pm + warp * 16 * 8;
-        float c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-        tile_product<1, LS, LS>(c, Lm + c0 * LS + r0, Tm + c0 * LS + c0 + j0, j0, 16, lane);  // T11 is lower triangular
-        tile_store<8>(P, c, 1.0f, lane);
+        const int r0 = (warp >> 1) * 32 + 16, c0 = r0 - 16, j0 = (warp & 1) * 8 + (lane & 1) * 4, i0 = ((lane >> 1) & 3) * 4;
+        float* P = Pm + (warp >> 1) * 16 * PS;
+        float2 c[4][2] = {};
+        tile_step<true, LS>(c, Lm + c0 * LS + r0 + i0, Tm + c0 * LS + c0 + j0, kp);
+        *reinterpret_cast<float4*>(P + (i0 + kp) * PS + j0) = tile_row(c, kp);
         __syncwarp();
-        c[0] = c[1] = c[2] = c[3] = 0.0f;
-        tile_product<LS, 1, 8>(c, Tm + r0 * LS + r0, P, 0, 16, lane);
-        tile_store<LS>(Tm + r0 * LS + c0 + j0, c, -1.0f, lane);
+        float2 d[4][2] = {};
+        tile_step<false, PS>(d, Tm + (r0 + i0) * LS + r0, P + j0, kp);
+        const float4 t = tile_row(d, kp);
+        *reinterpret_cast<float4*>(Tm + (r0 + i0 + kp) * LS + c0 + j0) = make_float4(-t.x, -t.y, -t.z, -t.w);
     }
     named_bar_sync(bar, NT);
-    const int i0 = (warp >> 2) * 16, j0 = (warp & 3) * 8;  // sz = 32: eight warps, a 16 x 8 tile each
+    const int i0 = (warp >> 1) * 8 + ((lane >> 2) & 1) * 4, j0 = (warp & 1) * 16 + (lane & 3) * 4;  // sz = 32: eight warps, 8 x 16 each
     if (warp < 8) {
-        float c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-        tile_product<1, LS, LS>(c, Lm + 32 + i0, Tm + j0, j0, 32, lane);
-        tile_store<PS>(Pm + i0 * PS + j0, c, 1.0f, lane);
+        float2 c[4][2] = {};
+        if (!(warp & 1)) tile_step<true, LS>(c, Lm + 32 + i0, Tm + j0, kp);  // T11 is lower triangular
+        tile_step<true, LS>(c, Lm + 16 * LS + 32 + i0, Tm + 16 * LS + j0, kp);
+        *reinterpret_cast<float4*>(Pm + (i0 + kp) * PS + j0) = tile_row(c, kp);
     }
     named_bar_sync(bar, NT);
     if (warp < 8) {
-        float c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-        tile_product<LS, 1, PS>(c, Tm + (32 + i0) * LS + 32, Pm + j0, 0, i0 + 16, lane);  // T22 is lower triangular
-        tile_store<LS>(Tm + (32 + i0) * LS + j0, c, -1.0f, lane);
+        float2 c[4][2] = {};
+        tile_step<false, PS>(c, Tm + (32 + i0) * LS + 32, Pm + j0, kp);
+        if (warp >= 4) tile_step<false, PS>(c, Tm + (32 + i0) * LS + 48, Pm + 16 * PS + j0, kp);  // T22 is lower triangular
+        const float4 t = tile_row(c, kp);
+        *reinterpret_cast<float4*>(Tm + (32 + i0 + kp) * LS + j0) = make_float4(-t.x, -t.y, -t.z, -t.w);
     }
     named_bar_sync(bar, NT);
 }
