@@ -204,7 +204,7 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
             float run[32], acc = 0.0f;
 #pragma unroll
             for (int r = 0; r < 32; ++r) {
-                acc += *reinterpret_cast<const float*>(col + r * 128 + ((pc ^ (r & 7)) << 4));
+                acc = fmaf(*reinterpret_cast<const float*>(col + r * 128 + ((pc ^ (r & 7)) << 4)), kLog2e, acc);  // in powers of two from here on
                 run[r] = acc;
             }
             tmp[part * 128 + d] = acc;
@@ -213,7 +213,7 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
             float amax = 0.0f;
 #pragma unroll
             for (int r = 0; r < 32; ++r) {
-                const float av = __expf(run[r] - run[(r & 16) | 8]);
+                const float av = ex2_approx(run[r] - run[(r & 16) | 8]);
                 amax = fmaxf(amax, av);
                 *reinterpret_cast<float*>(col + r * 128 + ((pc ^ (r & 7)) << 4)) = av;
             }
@@ -225,18 +225,18 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
             const float gl = base1 + tmp[128 + d];
             float* tab = reinterpret_cast<float*>(gs + gTab) + d;
             if (part == 0) {
-                tab[(tE0 + 0) * 128] = __expf(gm0); tab[(tE0 + 1) * 128] = __expf(gm1); tab[(tE0 + 2) * 128] = __expf(gm2); tab[(tE0 + 3) * 128] = __expf(gm3);
-                tab[(tEL + 0) * 128] = __expf(gl - gm0); tab[(tEL + 1) * 128] = __expf(gl - gm1);
-                tab[(tEL + 2) * 128] = __expf(gl - gm2); tab[(tEL + 3) * 128] = __expf(gl - gm3);
+                tab[(tE0 + 0) * 128] = ex2_approx(gm0); tab[(tE0 + 1) * 128] = ex2_approx(gm1); tab[(tE0 + 2) * 128] = ex2_approx(gm2); tab[(tE0 + 3) * 128] = ex2_approx(gm3);
+                tab[(tEL + 0) * 128] = ex2_approx(gl - gm0); tab[(tEL + 1) * 128] = ex2_approx(gl - gm1);
+                tab[(tEL + 2) * 128] = ex2_approx(gl - gm2); tab[(tEL + 3) * 128] = ex2_approx(gl - gm3);
             } else {
-                tab[(tF + 0) * 128] = __expf(gm1 - gm0);
-                tab[(tF + 1) * 128] = __expf(gm2 - gm0); tab[(tF + 2) * 128] = __expf(gm2 - gm1);
-                tab[(tF + 3) * 128] = __expf(gm3 - gm0); tab[(tF + 4) * 128] = __expf(gm3 - gm1); tab[(tF + 5) * 128] = __expf(gm3 - gm2);
-                const float egl = __expf(gl);
+                tab[(tF + 0) * 128] = ex2_approx(gm1 - gm0);
+                tab[(tF + 1) * 128] = ex2_approx(gm2 - gm0); tab[(tF + 2) * 128] = ex2_approx(gm2 - gm1);
+                tab[(tF + 3) * 128] = ex2_approx(gm3 - gm0); tab[(tF + 4) * 128] = ex2_approx(gm3 - gm1); tab[(tF + 5) * 128] = ex2_approx(gm3 - gm2);
+                const float egl = ex2_approx(gl);
                 reinterpret_cast<float*>(slot + wEgl)[d] = egl;
                 reinterpret_cast<float*>(gs + gGl)[d] = egl;
             }
-            mild = gl > -60.0f;
+            mild = gl > -60.0f * kLog2e;
         }
         // A chunk whose whole decay stays above e^-60 in every channel needs no block-wise references: exp(G) and exp(-G) from
         // the chunk's start are both representable with room for small q and k, one column-side tile serves every row, and L^T,
@@ -266,25 +266,20 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
                 const uint4 k8 = *reinterpret_cast<const uint4*>(gs + gK + box_piece(r, c));
                 const float4 e0a = *reinterpret_cast<const float4*>(tabs + (tE0 + J) * 128 + c * 8), e0b = *reinterpret_cast<const float4*>(tabs + (tE0 + J) * 128 + c * 8 + 4);
                 const float4 gla = *reinterpret_cast<const float4*>(gs + gGl + c * 32), glb = *reinterpret_cast<const float4*>(gs + gGl + c * 32 + 16);
-                const float E0[8] = {e0a.x, e0a.y, e0a.z, e0a.w, e0b.x, e0b.y, e0b.z, e0b.w};
-                const float GL[8] = {gla.x, gla.y, gla.z, gla.w, glb.x, glb.y, glb.z, glb.w};
+                const float2 E0[4] = {{e0a.x, e0a.y}, {e0a.z, e0a.w}, {e0b.x, e0b.y}, {e0b.z, e0b.w}};
+                const float2 GL[4] = {{gla.x, gla.y}, {gla.z, gla.w}, {glb.x, glb.y}, {glb.z, glb.w}};
                 const uint32_t kw[4] = {k8.x, k8.y, k8.z, k8.w};
                 uint32_t kg[4], ki[4], dh[4], dl[4];
 #pragma unroll
                 for (int u2 = 0; u2 < 4; ++u2) {
-                    const float kf[2] = {__uint_as_float(kw[u2] << 16), __uint_as_float(kw[u2] & 0xffff0000u)};
-                    float v_kg[2], v_ki[2], hi[2], lo[2];
-#pragma unroll
-                    for (int u = 0; u < 2; ++u) {
-                        const float e = a[cc * 8 + 2 * u2 + u] * E0[2 * u2 + u], einv = __fdividef(1.0f, e);
-                        v_kg[u] = kf[u] * e;
-                        v_ki[u] = kf[u] * einv;
-                        tc::split_bf16(kf[u] * (GL[2 * u2 + u] * einv), hi[u], lo[u]);
-                    }
-                    kg[u2] = tc::bf16x2(v_kg[0], v_kg[1]);
-                    ki[u2] = tc::bf16x2(v_ki[0], v_ki[1]);
-                    dh[u2] = tc::bf16x2(hi[0], hi[1]);
-                    dl[u2] = tc::bf16x2(lo[0], lo[1]);
+                    const float2 kf = {__uint_as_float(kw[u2] << 16), __uint_as_float(kw[u2] & 0xffff0000u)};
+                    const float2 e = mul2({a[cc * 8 + 2 * u2], a[cc * 8 + 2 * u2 + 1]}, E0[u2]);
+                    a[cc * 8 + 2 * u2] = e.x;  // exp(G): what the tiles made from q need
+                    a[cc * 8 + 2 * u2 + 1] = e.y;
+                    const float2 v_kg = mul2(kf, e), v_ki = mul2(kf, {rcp_approx(e.x), rcp_approx(e.y)}), v_kd = mul2(v_ki, GL[u2]);
+                    kg[u2] = tc::bf16x2(v_kg.x, v_kg.y);
+                    ki[u2] = tc::bf16x2(v_ki.x, v_ki.y);
+                    tc::split_bf16x2(v_kd.x, v_kd.y, dh[u2], dl[u2]);
                 }
                 *reinterpret_cast<uint4*>(gs + gK + box_piece(r, c)) = make_uint4(kg[0], kg[1], kg[2], kg[3]);
                 *reinterpret_cast<uint4*>(gs + gKc + kc_piece(3, r, c)) = make_uint4(ki[0], ki[1], ki[2], ki[3]);
@@ -362,19 +357,27 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
         for (int cc = 0; cc < 4; ++cc) {
             const int c = cq * 4 + cc;
             const uint4 q8 = *reinterpret_cast<const uint4*>(gs + gQ + box_piece(r, c));
-            const float4 e0a = *reinterpret_cast<const float4*>(tabs + (tE0 + J) * 128 + c * 8), e0b = *reinterpret_cast<const float4*>(tabs + (tE0 + J) * 128 + c * 8 + 4);
-            const float E0[8] = {e0a.x, e0a.y, e0a.z, e0a.w, e0b.x, e0b.y, e0b.z, e0b.w};
             const uint32_t qw[4] = {q8.x, q8.y, q8.z, q8.w};
             uint32_t qg[4], qgb[4];
+            if (narrow) {
 #pragma unroll
-            for (int u2 = 0; u2 < 4; ++u2) {
-                const float q0 = __uint_as_float(qw[u2] << 16), q1 = __uint_as_float(qw[u2] & 0xffff0000u);
-                const float a0 = a[cc * 8 + 2 * u2], a1 = a[cc * 8 + 2 * u2 + 1];
-                qgb[u2] = tc::bf16x2(q0 * a0, q1 * a1);
-                qg[u2] = tc::bf16x2(q0 * (a0 * E0[2 * u2]), q1 * (a1 * E0[2 * u2 + 1]));
+                for (int u2 = 0; u2 < 4; ++u2) {
+                    const float2 x = mul2({__uint_as_float(qw[u2] << 16), __uint_as_float(qw[u2] & 0xffff0000u)}, {a[cc * 8 + 2 * u2], a[cc * 8 + 2 * u2 + 1]});
+                    qg[u2] = qgb[u2] = tc::bf16x2(x.x, x.y);
+                }
+            } else {
+                const float4 e0a = *reinterpret_cast<const float4*>(tabs + (tE0 + J) * 128 + c * 8), e0b = *reinterpret_cast<const float4*>(tabs + (tE0 + J) * 128 + c * 8 + 4);
+                const float E0[8] = {e0a.x, e0a.y, e0a.z, e0a.w, e0b.x, e0b.y, e0b.z, e0b.w};
+#pragma unroll
+                for (int u2 = 0; u2 < 4; ++u2) {
+                    const float q0 = __uint_as_float(qw[u2] << 16), q1 = __uint_as_float(qw[u2] & 0xffff0000u);
+                    const float a0 = a[cc * 8 + 2 * u2], a1 = a[cc * 8 + 2 * u2 + 1];
+                    qgb[u2] = tc::bf16x2(q0 * a0, q1 * a1);
+                    qg[u2] = tc::bf16x2(q0 * (a0 * E0[2 * u2]), q1 * (a1 * E0[2 * u2 + 1]));
+                }
             }
             // narrow: Qg itself is M's row side
-            *reinterpret_cast<uint4*>(gs + gQ + box_piece(r, c)) = narrow ? make_uint4(qg[0], qg[1], qg[2], qg[3]) : make_uint4(qgb[0], qgb[1], qgb[2], qgb[3]);
+            *reinterpret_cast<uint4*>(gs + gQ + box_piece(r, c)) = make_uint4(qgb[0], qgb[1], qgb[2], qgb[3]);
             *reinterpret_cast<uint4*>(cell(slot + wQg, CH, c, r)) = make_uint4(qg[0], qg[1], qg[2], qg[3]);
         }
         publish();
@@ -443,12 +446,10 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
                 const int c = cq + cc * 4;
                 uint32_t wh[4], wl[4];
 #pragma unroll
-                for (int j2 = 0; j2 < 4; ++j2) {
-                    float h0, l0, h1, l1;
-                    tc::split_bf16(Tm[i * LS + c * 8 + 2 * j2] * betas[c * 8 + 2 * j2], h0, l0);
-                    tc::split_bf16(Tm[i * LS + c * 8 + 2 * j2 + 1] * betas[c * 8 + 2 * j2 + 1], h1, l1);
-                    wh[j2] = tc::bf16x2(h0, h1);
-                    wl[j2] = tc::bf16x2(l0, l1);
+                for (int j2 = 0; j2 < 2; ++j2) {
+                    const float4 t4 = *reinterpret_cast<const float4*>(Tm + i * LS + c * 8 + 4 * j2), b4 = *reinterpret_cast<const float4*>(betas + c * 8 + 4 * j2);
+                    tc::split_bf16x2(t4.x * b4.x, t4.y * b4.y, wh[2 * j2], wl[2 * j2]);
+                    tc::split_bf16x2(t4.z * b4.z, t4.w * b4.w, wh[2 * j2 + 1], wl[2 * j2 + 1]);
                 }
                 *reinterpret_cast<uint4*>(gs + gTp + box_piece(i, c)) = make_uint4(wh[0], wh[1], wh[2], wh[3]);
                 *reinterpret_cast<uint4*>(gs + gTp + kBox + box_piece(i, c)) = make_uint4(wl[0], wl[1], wl[2], wl[3]);
@@ -529,6 +530,13 @@ __device__ __forceinline__ void intra_loader(const SpParams& p, unsigned char* s
         float b0 = 0.0f, b1 = 0.0f;
         if (lane < n) b0 = p.beta[(gr0 + lane) * H + h];
         if (lane + 32 < n) b1 = p.beta[(gr0 + lane + 32) * H + h];
+        if (!last && n == CH && lane == 0) {  // on their way into L2 while the group is still busy with the item before
+            const int row = (int)gr0;
+            for (int x = 0; x < 4; ++x) tensor_prefetch_3d(&p.tm_g, x * 32, h, row);
+            for (int x = 0; x < 2; ++x) tensor_prefetch_3d(&p.tm_k, x * 64, h, row);
+            for (int x = 0; x < 2; ++x) tensor_prefetch_3d(&p.tm_q, x * 64, h, row);
+            for (int x = 0; x < 2; ++x) tensor_prefetch_3d(&p.tm_v, x * 64, h, row);
+        }
         if (it > 0) {
             if (!mbar_wait(bar_free, free_phase, ctx, kStatusWaitPrefill)) break;
             free_phase ^= 1u;
@@ -608,7 +616,7 @@ __device__ void intra_role(const SpParams& p, unsigned char* smem, const uint32_
 // are A operands that never leave tensor memory; what comes from the workspace is the B side, so shared memory has room for
 // two chunks of it and a load has a whole chunk's time to arrive.
 // Measured per chunk at 64 chains: 5,800 cycles with products of 64 rows, S and D through shared memory and block barriers
-// around every step; MEASURE_ME so.
+// around every step; 3,700 to 4,000 so.
 // =====================================================================================================================
 // Shared memory: two buffers of [Qg | W], two of [M | Kdec hi | Kdec lo] and exp(G_last), one of U, each with a full / empty pair.
 // Finished output rows (bf16) wait in one of two tiles for the output warp: two boxes of 64 rows x 128 bytes each (value
