@@ -57,20 +57,21 @@ int conv_shift_launch(int32_t channels, int32_t layers, int32_t batch, const int
                       int32_t keep1, int32_t rows1, glm53f_bf16* conv, int64_t conv_stride, const int64_t* conv_off,
                       const glm53f_bf16* p, int64_t p_layer_stride, int64_t p_stride, cudaStream_t stream);
 
-// One pass of a layer prefill through the core kernel: sequence b's inputs are rows b * pass_rows .. of q, k, v, g, beta
-// (its rows row_shift .. row_shift + pass_rows - 1, as many of them as it has); its outputs and gate rows are rows
-// cu[b] + row_shift .. of `out` and `gate`, gate rows gate_stride elements apart.
-struct PrefillWindow {
-    int pass_rows = 0, row_shift = 0;
-    long long gate_stride = 0;
-    bool qk_fp16 = false;  // q and k hold fp16 bits (the layer prologue's), not bf16
-};
+// A workspace slot of one (chain, chunk) item of the two-pass prefill (kda_prefill_sp.cu).  Before its first pass a layer
+// prefill's slot holds the chunk's inputs: q and k as fp16 bits, v bf16, the log decays f32, as boxes of 64 rows x 128 bytes in
+// the 128-byte swizzle (the 16-byte piece p of row r at box p / 8, piece (p % 8) ^ (r % 8)), then beta.
+constexpr int kPrefillSlotBytes = 107008, kPrefillTailBytes = 256;
+// The workspace's last 256 bytes, as words: two item counters | a single request's metadata (an offset, cu_rows) | from word 8
+// on two sets, which consecutive launches use in turn: items and chains handed out, and finished items per group of chains.
+constexpr int kTailMeta = 2, kTailSets = 8, kTailSet = 28, kTailGroups = kTailSet - 2;
+constexpr int kSlotInK = 0, kSlotInV = 16384, kSlotInQ = 32768, kSlotInG = 49152, kSlotInBeta = 81920;
+__host__ __device__ inline int prefill_box_piece(int r, int piece) { return (piece >> 3) * 8192 + r * 128 + (((piece & 7) ^ (r & 7)) << 4); }
 
 // The chunk-64 tensor-core prefill (kda_prefill_tc.cu).  q, k, v, g, out (and norm_w) must be 16-byte aligned.
 int core_prefill_tc_launch(int32_t heads, int32_t batch, const int32_t* cu_seqlens, const glm53f_bf16* q, const glm53f_bf16* k,
                            const glm53f_bf16* v, const float* g, const float* beta, const void* state_in, void* state_out,
                            const int64_t* state_off, bool bf16_state, const glm53f_bf16* gate, const glm53f_bf16* norm_w,
-                           float eps, glm53f_bf16* out, cudaStream_t stream, const PrefillWindow* win = nullptr);
+                           float eps, glm53f_bf16* out, cudaStream_t stream);
 
 // Draft verification as one 16-row chunk on the tensor cores (kda_verify_tc.cu): bf16 states, read only; outputs to the
 // rounding of bf16 operands, replay saves as the exact path writes them.  q, k, v, g must be 16-byte aligned.
@@ -96,15 +97,18 @@ int commit_tc_launch(int32_t heads, int32_t layers, int32_t batch, const int32_t
                      void* state_out, int64_t state_stride, const int64_t* state_off, const float* k_save, const glm53f_bf16* v_save,
                      const float* g_save, const float* b_save, int64_t kv_stride, int64_t b_stride, cudaStream_t stream);
 
-// The layer prologue of a prefill pass (kda_prologue.cu): for rows row_shift .. row_shift + pass_rows - 1 of every request,
-// the short convolution + SiLU, the L2 norms, the log decay and beta, with the chain's arithmetic, written as core inputs
-// (q, k as fp16 bits, v bf16, g f32 log decay [batch * pass_rows][H][128]; beta f32 [batch * pass_rows][H]).  p, a, conv must be
-// 8-byte aligned with strides that are multiples of 4 elements.
-int layer_prologue_launch(int32_t heads, int32_t batch, const int32_t* cu_rows, int32_t pass_rows, int32_t row_shift,
+// The layer prologue of a prefill pass (kda_prologue.cu): for chunks chunk0 .. chunk0 + chunks - 1 (of 64 rows) of every
+// request, the short convolution + SiLU, the L2 norms, the log decay and beta, written as core inputs into the slots
+// [batch][heads][chunks].  p, a, conv must be 8-byte aligned with strides that are multiples of 4 elements.
+int layer_prologue_launch(int32_t heads, int32_t batch, const int32_t* cu_rows, int32_t chunks, int32_t chunk0,
                           const glm53f_bf16* p, int64_t p_stride, int64_t b_off, const glm53f_bf16* a, int64_t a_stride,
                           const glm53f_bf16* conv, const int64_t* conv_off, const glm53f_bf16* conv_w, const float* a_log,
-                          const float* dt_bias, float lower, glm53f_bf16* q, glm53f_bf16* k, glm53f_bf16* v, float* g, float* beta,
-                          cudaStream_t stream);
+                          const float* dt_bias, float lower, unsigned char* slots, cudaStream_t stream);
+// The pass itself, both roles, from those slots (kda_prefill_sp.cu).  `tail`: the workspace's
+// tail, its sets zero before the first pass.
+int layer_pass_launch(int32_t heads, int32_t batch, const int32_t* cu_rows, int32_t chunks, int32_t chunk0, unsigned char* slots,
+                      unsigned int* tail, const void* state_in, void* state_out, const int64_t* state_off, bool bf16_state,
+                      const glm53f_bf16* gate, int64_t gate_stride, const glm53f_bf16* norm_w, float eps, glm53f_bf16* out, cudaStream_t stream);
 
 // The two-pass tensor-core prefill over a workspace (kda_prefill_sp.cu).
 int64_t core_prefill_workspace_bytes(int32_t heads, int32_t batch, int32_t chunks_per_pass);

@@ -9,9 +9,9 @@
 //   exact (default)   the row-by-row recurrence, the chain's results bit for bit: passes of (layer prologue -> recurrence of
 //                     kda_rows.cu) over the caller's workspace and one launch of the output norm; short or unaligned calls
 //                     run the chain of kda_chain.cu itself;
-//   chunked           passes of (layer prologue -> chunk-64 tcgen05 kernel of kda_prefill_tc.cu with the gated norm
-//                     fused) over the caller's workspace, which holds one pass's core inputs; agrees with the chain
-//                     to the rounding of bf16 operands, like every chunked form.  The kernels cover the whole gate
+//   chunked           passes of (layer prologue -> the two roles of kda_prefill_sp.cu with the gated norm fused) over the
+//                     caller's workspace, whose slots hold a pass's core inputs and then what the recurrence takes;
+//                     agrees with the chain to the rounding of bf16 operands, like every chunked form.  The kernels cover the whole gate
 //                     domain of the entry points (lower in [-5.8, 0]).
 // The core entry point runs the chunk-64 tcgen05 kernel directly.
 
@@ -35,19 +35,20 @@ std::atomic<int> g_layer_prefill_mode{[] {
 }()};
 
 constexpr int kNotEligible = -1;
-constexpr int64_t kCoreBytesPerRowHead = 3 * DK * 2 + DK * 4 + 4;  // q, k, v bf16, log decay f32, beta f32
 
-// Batch metadata of a single-request call, written into the workspace (the kernels read metadata on the device).
-__global__ void single_request_meta(int32_t* cu, long long* zeros, int32_t rows) {
-    cu[0] = 0;
-    cu[1] = rows;
-    zeros[0] = 0;
+// The workspace's tail: the passes' item counters, and the batch metadata of a single-request call (the kernels read metadata
+// on the device).
+__global__ void prefill_tail(unsigned int* tail, int32_t rows) {
+    static_assert(kPrefillTailBytes == 4 * 64 && kTailSets + 2 * kTailSet == 64, "the workspace's tail");
+    tail[threadIdx.x] = threadIdx.x == kTailMeta + 3 ? (unsigned)rows : 0u;
 }
 
-// The chunked form.  The workspace holds the core inputs of one pass: P rows of every request, P the largest multiple
-// of 64 that fits (chunks count from a request's first row, so passes cut at chunk boundaries and the results do not
-// depend on the workspace size).  Returns kNotEligible when the call does not meet the kernels' layout requirements
-// (dense output rows, aligned rows, room for 64 rows a pass); the caller then runs the exact form.
+// The chunked form.  The workspace holds the slots of one pass: as many 64-row chunks of every request as fit, the passes of
+// equal length (chunks count from a request's first row, so the results do not depend on the workspace size).  Returns
+// kNotEligible when the call does not meet the kernels' layout requirements (dense output rows, aligned rows, room for
+// one chunk a pass); the caller then runs the exact form.
+// 4 requests x 2,048 rows x 64 heads with 256-row workspaces: 1,800 us with one block doing all of a chain
+// (kda_prefill_tc.cu, passes of six chunks), 1,216 so.
 int chunked_layer_prefill(int32_t heads, int32_t batch, const int32_t* cu_rows, int32_t max_rows, const glm53f_bf16* p,
                           int64_t p_stride, int64_t b_off, const glm53f_bf16* a, int64_t a_stride, const glm53f_bf16* g,
                           int64_t g_stride, const glm53f_bf16* conv, const int64_t* conv_off, const glm53f_bf16* conv_w,
@@ -58,36 +59,26 @@ int chunked_layer_prefill(int32_t heads, int32_t batch, const int32_t* cu_rows, 
     if (out_stride != (int64_t)heads * DV || !al(out, 16) || !al(workspace, 16) || !al(p, 8) || !al(a, 8) || !al(conv, 8) || !al(conv_w, 16) ||
         !al(dt_bias, 16) || p_stride % 4 || a_stride % 4 || g_stride < (int64_t)heads * DV)
         return kNotEligible;
-    constexpr int64_t kMeta = 256;
-    int64_t pass = (workspace_bytes - kMeta) / ((int64_t)batch * heads * kCoreBytesPerRowHead) / 64 * 64;
-    const int64_t need = ((int64_t)max_rows + 63) / 64 * 64;
+    const int64_t chains = (int64_t)batch * heads, need = ((int64_t)max_rows + 63) / 64;
+    const int64_t usable = (workspace_bytes - kPrefillTailBytes) / 16 * 16;
+    int64_t pass = usable / (chains * kPrefillSlotBytes);
     if (pass > need) pass = need;
-    if (pass < 64 || (int64_t)batch * pass > 0x7fffffffll) return kNotEligible;
-    const int64_t cap = (int64_t)batch * pass * heads;  // (row, head) pairs a pass holds
-    unsigned char* w = reinterpret_cast<unsigned char*>(workspace);
-    glm53f_bf16* q = reinterpret_cast<glm53f_bf16*>(w);
-    glm53f_bf16* k = q + cap * DK;
-    glm53f_bf16* v = k + cap * DK;
-    float* lg = reinterpret_cast<float*>(v + cap * DK);
-    float* beta = lg + cap * DK;
+    if (pass < 1 || chains * pass * 16 > 0x7fffffffll) return kNotEligible;
+    const int64_t passes = (need + pass - 1) / pass;
+    pass = (need + passes - 1) / passes;
+    unsigned char* slots = reinterpret_cast<unsigned char*>(workspace);
+    unsigned int* tail = reinterpret_cast<unsigned int*>(slots + usable);
+    prefill_tail<<<1, 64, 0, st>>>(tail, max_rows);
     if (cu_rows == nullptr) {
-        int32_t* cu = reinterpret_cast<int32_t*>(beta + cap);
-        long long* zeros = reinterpret_cast<long long*>(w + ((reinterpret_cast<unsigned char*>(cu + 2) - w + 15) / 16) * 16);
-        single_request_meta<<<1, 1, 0, st>>>(cu, zeros, max_rows);
-        cu_rows = cu;
-        conv_off = state_off = reinterpret_cast<const int64_t*>(zeros);
+        cu_rows = reinterpret_cast<int32_t*>(tail + kTailMeta + 2);
+        conv_off = state_off = reinterpret_cast<const int64_t*>(tail + kTailMeta);
     }
-    PrefillWindow win;
-    win.pass_rows = (int)pass;
-    win.gate_stride = g_stride;
-    win.qk_fp16 = true;
-    for (int64_t shift = 0; shift < max_rows; shift += pass) {
-        win.row_shift = (int)shift;
-        int rc = layer_prologue_launch(heads, batch, cu_rows, (int)pass, (int)shift, p, p_stride, b_off, a, a_stride, conv, conv_off, conv_w,
-                                       a_log, dt_bias, lower, q, k, v, lg, beta, st);
+    for (int64_t chunk0 = 0; chunk0 < need; chunk0 += pass) {
+        int rc = layer_prologue_launch(heads, batch, cu_rows, (int)pass, (int)chunk0, p, p_stride, b_off, a, a_stride, conv, conv_off, conv_w, a_log,
+                                       dt_bias, lower, slots, st);
         if (rc != 0) return rc;
-        rc = core_prefill_tc_launch(heads, batch, cu_rows, q, k, v, lg, beta, shift == 0 ? state_in : state_out, state_out, state_off,
-                                    bf16_state, g, norm_w, eps, out, st, &win);
+        rc = layer_pass_launch(heads, batch, cu_rows, (int)pass, (int)chunk0, slots, tail, state_in, state_out, state_off, bf16_state, g, g_stride, norm_w,
+                               eps, out, st);
         if (rc != 0) return rc;
     }
     return 0;

@@ -1,5 +1,5 @@
-// Chunk-64 tensor-core prefill in two passes over a caller-provided workspace, for launches with few (sequence,
-// head) chains: a single long sequence, or a GPU's shard of heads.
+// Chunk-64 tensor-core prefill in two passes over a caller-provided workspace: the core entry points that take one, and the
+// chunked form of the layer prefill.
 //
 // The arithmetic is that of kda_prefill_tc.cu (same operand tiles, same products, same precision mix).  What
 // changes is where it runs.  Everything of a chunk that does not need the recurrent state -- the decay scan, the
@@ -13,16 +13,18 @@
 // The sequence is cut into segments sized by the workspace.  One kernel launch runs the state role for segment s-1
 // (blocks 0..chains-1) and the intra role for segment s (every block, the chain blocks after their state work; items
 // are handed out through a counter in the workspace), on two halves of the workspace that swap from launch to
-// launch.  Stream order between launches is the only synchronisation: no block ever waits on another block.
+// launch; stream order between launches is the only synchronisation.  With more chains than SMs, and for the layer entry
+// points, one persistent launch a pass runs both roles over all the slots (fused_roles).
 //
 // Workspace slot of one (chain, chunk) item, bytes: Qg 0 | W 16,384 (cells of eight rows, [8][128 key channels]) | M 32,768 | Kdec hi 40,960 | Kdec lo 57,344 |
 // U 73,728 (FP32, cells of four rows, [2][16][64 value channels]) | E_last 106,496 (128 floats); 107,008 per slot = 1,672 per row and head, inside
 // the 2,176 the reference's prefill workspace formula provides (kernels/kda_prefill.cu:40-43, 695-698).  The last
-// 256 bytes of the workspace hold the two item counters.
+// 256 bytes of the workspace hold the counters (kda_internal.h).
 
 #include <cstdlib>
 
 #include <cuda.h>
+#include <cuda_fp16.h>
 
 #include "common.cuh"
 #include "glm53f_kda.h"
@@ -40,14 +42,23 @@ using namespace pf;
 __device__ __forceinline__ int u_cell(int row4, int v) { return (((v >> 6) * 16 + row4) * 64 + (v & 63)) * 16; }
 constexpr int wQg = 0, wW = kTile, wMm = 2 * kTile, wKdHi = wMm + kTile / 2, wKdLo = wKdHi + kTile, wU = wKdLo + kTile;
 constexpr int kUBytes = CH * DV * 4, wEgl = wU + kUBytes, kSlotBytes = wEgl + 512;
-static_assert(kSlotBytes == 107008 && wU == 73728, "workspace slot layout");
+static_assert(kSlotBytes == kPrefillSlotBytes && wU == 73728, "workspace slot layout");
 
 // Staging of a chunk's raw rows in the intra kernel: dense boxes of 64 rows x 128 bytes written by tiled tensor copies
 // with the 128-byte swizzle (16-byte piece p of row r sits at piece p ^ (r & 7)), so that threads walking down the
 // rows of one column spread over all banks.  q, k, v: two boxes each (channels 0-63, 64-127); the log decays: four.
 constexpr int kBox = CH * 128;  // 8 KiB
 // Byte offset inside a tensor's staging of the 16-byte piece `piece` (0..15 for bf16 rows, 0..31 for f32 rows) of row r.
-__device__ __forceinline__ int box_piece(int r, int piece) { return (piece >> 3) * kBox + r * 128 + (((piece & 7) ^ (r & 7)) << 4); }
+__device__ __forceinline__ int box_piece(int r, int piece) { return prefill_box_piece(r, piece); }
+
+// Two 16-bit values of a q or k row to FP32: bf16 (the core entry points' inputs), or fp16 where the layer prologue produced
+// them (normalised q and k lie in [-1, 1]; eleven mantissa bits instead of eight keep the rounding of k, which goes into
+// the state through Kdec, below the state's error budget).
+template <bool LAYER>
+__device__ __forceinline__ float2 widen2(uint32_t w) {
+    if constexpr (LAYER) return __half22float2(*reinterpret_cast<const __half2*>(&w));
+    else return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
+}
 
 struct SpParams {
     alignas(64) CUtensorMap tm_q, tm_k, tm_v, tm_g;  // [rows][H][128] as (128, H, rows); boxes of 64 rows x 128 bytes, 128-byte swizzle
@@ -63,6 +74,7 @@ struct SpParams {
     const long long* state_off;
     int state_bf16;
     const uint16_t* gate;
+    long long gate_stride;  // elements between consecutive gate rows
     const uint16_t* norm_w;
     float eps;
     uint16_t* out;
@@ -75,6 +87,10 @@ struct SpParams {
     int ranks, heads_total, head0;
     unsigned int* counters;  // [2] item counters: this launch hands items out of counters[ctr], and zeroes the other
     int ctr;
+    // One persistent launch for both roles (fused != 0): items, then chains, are handed out from tail set ctr; chains form groups
+    // of `group`, and a chain's state role starts when all items of its group are finished.
+    int fused, group;
+    unsigned int* sets;
     int* status;
     // The scan over segments of the sequence (scan_pass != 0; FP32 states; the workspace holds every chunk).  Segment s of
     // a chain covers chunks [s * scan_chunks, (s + 1) * scan_chunks).
@@ -95,6 +111,17 @@ struct SpParams {
 
 __device__ __forceinline__ unsigned char* slot_of(unsigned char* ws, int seg_chunks, int chain, int jj) {
     return ws + ((size_t)chain * seg_chunks + jj) * kSlotBytes;
+}
+
+struct Item {
+    int chain, jj, group;
+};
+// Chunk-major, neighbouring chains next to each other; in a fused launch so within each group of chains.
+__device__ __forceinline__ Item item_of(const SpParams& p, int item) {
+    const int chains = p.batch * p.H;
+    if (!p.fused) return {item % chains, item / chains, 0};
+    const int per = p.group * p.seg_chunks, g = item / per, rem = item - g * per, n = min(p.group, chains - g * p.group);
+    return {g * p.group + rem % n, rem / n, g};
 }
 
 // The state role's barriers sit behind every tile (set up once at kernel entry, never repurposed).  The intra role's
@@ -133,18 +160,21 @@ constexpr int kKcBytes = 2 * 128 * (16 + 32 + 48 + 64);  // the four column-side
 __device__ __forceinline__ int kc_piece(int I, int r, int piece) {
     return kc_tile(I) + (piece >> 3) * (I + 1) * 2048 + r * 128 + (((piece & 7) ^ (r & 7)) << 4);
 }
-constexpr int gQ = 0, gK = kTile, gV = 2 * kTile, gKb = 3 * kTile, gG = 4 * kTile, gKc = gG;  // Q/Qgb | K/Kg | V | Kgb | g/G, then the column-side tiles
-constexpr int gT = gKc, gL = gT + CH * LS * 4, gP = gL + CH * LS * 4, gTp = gL;              // inverse scratch over the column-side tiles; T' (hi | lo box) over L
+constexpr int gK = 0, gV = kTile, gQ = 2 * kTile, gKb = 3 * kTile, gKc = 4 * kTile;  // K/Kg | V | Q/Qgb | Kgb | the column-side tiles
+// The log decays lie over the column-side tiles; the inverse's scratch and T' (hi | lo box, over L) over Q, Kgb and the 8 KiB before
+// the log decays, so that the next item's log decays can arrive as soon as L and M are formed.
+constexpr int gG = gKc + 8192, gT = gQ, gL = gT + CH * LS * 4, gTp = gL;
 static_assert(gTp % 1024 == 0 && gKc % 1024 == 0, "swizzled tiles are 1024-byte aligned");
 // Per-block decay factors, 128 channels each: E0[J] = exp(Gm_J), EL[J] = exp(G_last - Gm_J), F[I(I-1)/2 + J] =
 // exp(Gm_I - Gm_J) for I > J.  The scan's totals use the first two rows before the tables are written.
-constexpr int gTab = gKc + kKcBytes, gBeta = gTab + kTabs * 512, gBars = gBeta + CH * 4, gItem = gBars + 32, gGl = gItem + 16;  // gGl: exp(G_last) [128]
+constexpr int gTab = gKc + kKcBytes, gP = gTab, gBeta = gTab + kTabs * 512, gBars = gBeta + CH * 4, kGroupBars = 6, gItem = gBars + kGroupBars * 8, gGl = gItem + 16;  // gGl: exp(G_last) [128]
 constexpr int kGroupBytes = 114688;
-static_assert(4 * kBox <= kKcBytes && gP + 32 * PS * 4 <= gTab && gTp + kTile <= gP && gGl + 512 <= kGroupBytes && kGroupBytes % 1024 == 0, "group map");
+static_assert(gG + 4 * kBox <= gTab && gG % 1024 == 0 && 32 * PS * 4 <= kTabs * 512 && gL + CH * LS * 4 <= gG && gGl + 512 <= kGroupBytes && kGroupBytes % 1024 == 0, "group map");
 static_assert(kGroups * kGroupBytes <= oCtl, "two groups must fit below the block's control words");
 constexpr uint32_t gcL = 0, gcM = 64, gcW = 0, gcU = 64, kGroupCols = 128;
 
-// G = 0 or 1, a runtime value: both groups run the same instructions (one copy of this code in the instruction cache).
+// LAYER: the items' inputs are in their slots (kda_internal.h), which the results then replace.  G = 0 or 1, a runtime value: both groups run the same instructions (one copy of this code in the instruction cache).
+template <bool LAYER>
 __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* smem, const uint32_t tm_block, const WaitCtx& ctx, const int G) {
     const int BAR = 2 + G;
     unsigned char* gs = smem + G * kGroupBytes;
@@ -152,13 +182,12 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
     uint64_t* bar_raw = reinterpret_cast<uint64_t*>(gs + gBars);
     uint64_t* bar_mma = bar_raw + 1;
     uint64_t* bar_lm = bar_raw + 2;  // the eight products of L^T and M^T: eight issuing threads arrive
-    uint64_t* bar_free = bar_raw + 3;
+    uint64_t *bar_free = bar_raw + 3, *bar_g = bar_raw + 4, *bar_gfree = bar_raw + 5;
     volatile int* item_slot = reinterpret_cast<volatile int*>(gs + gItem);
     float* betas = reinterpret_cast<float*>(gs + gBeta);
     const int gt = threadIdx.x - G * kGroupThreads, gw = gt >> 5, lane = gt & 31;
     const int quad = gw & 3, cg = gw >> 2;  // a warp reaches tensor-memory lanes 32 * (warp % 4)..; cg picks a half of the columns
     const int lane_row64 = quad * 16 + lane;
-    const int H = p.H, chains = p.batch * H;
     auto group_sync = [&]() { named_bar_sync(BAR, kGroupThreads); };
     auto publish = [&]() {
         fence_proxy_async_smem();
@@ -184,12 +213,11 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
     };
 
     for (;;) {
-        if (!mbar_wait(bar_raw, raw_phase, ctx, kStatusWaitPrefill)) break;
-        raw_phase ^= 1u;
+        if (!mbar_wait(bar_g, raw_phase, ctx, kStatusWaitPrefill)) break;
         const int item = *item_slot;
         if (item < 0) break;
-        const int chain = item % chains, jj = item / chains;
-        unsigned char* slot = slot_of(p.ws_intra, p.seg_chunks, chain, jj);
+        const Item at_item = item_of(p, item);
+        unsigned char* slot = slot_of(p.ws_intra, p.seg_chunks, at_item.chain, at_item.jj);
 
         bool mild;
         // ---- 1. per key channel: the cumulative log decay; a = exp(G - Gm), every row relative to the middle row of its block of
@@ -253,6 +281,8 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
             a[pp * 4 + 0] = x.x; a[pp * 4 + 1] = x.y; a[pp * 4 + 2] = x.z; a[pp * 4 + 3] = x.w;
         }
         group_sync();  // nobody reads the staged a (or the scan's scratch) any more: the tiles may go over them
+        if (!mbar_wait(bar_raw, raw_phase, ctx, kStatusWaitPrefill)) break;
+        raw_phase ^= 1u;
 
         // ---- 3. operand tiles, first those made from k.  Row side Kgb = K a; Kg = K exp(G) (over K) for W; Kdec =
         // K exp(G_last - G) as bf16 hi + lo out to the workspace; column sides K exp(Gm_I - G) into the tiles I >= J.
@@ -272,7 +302,7 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
                 uint32_t kg[4], ki[4], dh[4], dl[4];
 #pragma unroll
                 for (int u2 = 0; u2 < 4; ++u2) {
-                    const float2 kf = {__uint_as_float(kw[u2] << 16), __uint_as_float(kw[u2] & 0xffff0000u)};
+                    const float2 kf = widen2<LAYER>(kw[u2]);
                     const float2 e = mul2({a[cc * 8 + 2 * u2], a[cc * 8 + 2 * u2 + 1]}, E0[u2]);
                     a[cc * 8 + 2 * u2] = e.x;  // exp(G): what the tiles made from q need
                     a[cc * 8 + 2 * u2 + 1] = e.y;
@@ -300,7 +330,8 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
             float kc[8];  // K exp(Gm_J - G): the column side inside the row's own block
 #pragma unroll
             for (int u2 = 0; u2 < 4; ++u2) {
-                const float kf[2] = {__uint_as_float(kw[u2] << 16), __uint_as_float(kw[u2] & 0xffff0000u)};
+                const float2 k2 = widen2<LAYER>(kw[u2]);
+                const float kf[2] = {k2.x, k2.y};
                 float v_kg[2], v_kgb[2], hi[2], lo[2];
 #pragma unroll
                 for (int u = 0; u < 2; ++u) {
@@ -362,7 +393,7 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
             if (narrow) {
 #pragma unroll
                 for (int u2 = 0; u2 < 4; ++u2) {
-                    const float2 x = mul2({__uint_as_float(qw[u2] << 16), __uint_as_float(qw[u2] & 0xffff0000u)}, {a[cc * 8 + 2 * u2], a[cc * 8 + 2 * u2 + 1]});
+                    const float2 x = mul2(widen2<LAYER>(qw[u2]), {a[cc * 8 + 2 * u2], a[cc * 8 + 2 * u2 + 1]});
                     qg[u2] = qgb[u2] = tc::bf16x2(x.x, x.y);
                 }
             } else {
@@ -370,7 +401,8 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
                 const float E0[8] = {e0a.x, e0a.y, e0a.z, e0a.w, e0b.x, e0b.y, e0b.z, e0b.w};
 #pragma unroll
                 for (int u2 = 0; u2 < 4; ++u2) {
-                    const float q0 = __uint_as_float(qw[u2] << 16), q1 = __uint_as_float(qw[u2] & 0xffff0000u);
+                    const float2 q2 = widen2<LAYER>(qw[u2]);
+                    const float q0 = q2.x, q1 = q2.y;
                     const float a0 = a[cc * 8 + 2 * u2], a1 = a[cc * 8 + 2 * u2 + 1];
                     qgb[u2] = tc::bf16x2(q0 * a0, q1 * a1);
                     qg[u2] = tc::bf16x2(q0 * (a0 * E0[2 * u2]), q1 * (a1 * E0[2 * u2 + 1]));
@@ -401,6 +433,7 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
             __syncwarp();
         }
         if (!mma_wait(bar_lm, lm_phase)) break;
+        if (gt == 0) mbar_arrive(bar_gfree);  // nothing is left over the log decays' place
 
         // ---- 4. from L^T and M^T (lane = column j, tensor-memory column = row i): L (FP32, strictly lower, times beta_i) into
         // the scratch; M (lower with the diagonal) out as bf16 cells of eight consecutive rows i, [8 cells][64 columns j] ----------
@@ -491,9 +524,14 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
             for (int j2 = 0; j2 < 8; ++j2)
                 *reinterpret_cast<uint4*>(slot + wU + u_cell(cg * 8 + j2, ch)) = make_uint4(r[j2 * 4], r[j2 * 4 + 1], r[j2 * 4 + 2], r[j2 * 4 + 3]);
         }
+        if (p.fused) fence_proxy_async_global();  // another block's bulk copies read the slot
         tc::fence_before_sync();
         group_sync();
         tc::fence_after_sync();
+        if (p.fused && gt == 0) {
+            __threadfence();
+            atomicAdd(p.sets + p.ctr * kTailSet + 2 + at_item.group, 1u);
+        }
     }
 }
 
@@ -501,10 +539,11 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
 // chunk arrives by ten tiled tensor copies issued by one lane; a sequence's last, partial chunk is copied by the
 // warp's own loads and stores (rows past the sequence's end are not read, they become zero), so no copy ever reaches
 // past the rows the caller's metadata names.
+template <bool LAYER>
 __device__ __forceinline__ void intra_loader(const SpParams& p, unsigned char* smem, const WaitCtx& ctx, const int G) {
     unsigned char* gs = smem + G * kGroupBytes;
     uint64_t* bar_raw = reinterpret_cast<uint64_t*>(gs + gBars);
-    uint64_t* bar_free = bar_raw + 3;
+    uint64_t *bar_free = bar_raw + 3, *bar_g = bar_raw + 4, *bar_gfree = bar_raw + 5;
     volatile int* item_slot = reinterpret_cast<volatile int*>(gs + gItem);
     float* betas = reinterpret_cast<float*>(gs + gBeta);
     const int lane = threadIdx.x & 31;
@@ -513,69 +552,87 @@ __device__ __forceinline__ void intra_loader(const SpParams& p, unsigned char* s
     uint32_t free_phase = 0;
     for (int it = 0;;) {
         long long item = 0;
-        if (lane == 0) item = atomicAdd(&p.counters[p.ctr], 1u);
+        if (lane == 0) item = atomicAdd(p.fused ? p.sets + p.ctr * kTailSet : p.counters + p.ctr, 1u);
         item = __shfl_sync(0xffffffffu, item, 0);
         const bool last = item >= items;
         int h = 0, n = 0;
         long long gr0 = 0;
+        const unsigned char* in = nullptr;
         if (!last) {
-            const int chain = (int)(item % chains), j = p.intra_chunk0 + (int)(item / chains);
-            const int b = chain / H;
-            h = chain % H;
+            const Item at = item_of(p, (int)item);
+            const int j = p.intra_chunk0 + at.jj, b = at.chain / H;
+            h = at.chain % H;
             const int r0 = p.cu[b], T = p.cu[b + 1] - r0;
-            if ((long long)j * CH >= T) continue;  // the sequence has no such chunk
+            if ((long long)j * CH >= T) {  // the sequence has no such chunk
+                if (p.fused && lane == 0) atomicAdd(p.sets + p.ctr * kTailSet + 2 + at.group, 1u);
+                continue;
+            }
             gr0 = (long long)r0 + (long long)j * CH;
             n = min(CH, T - j * CH);
+            if constexpr (LAYER) in = slot_of(p.ws_intra, p.seg_chunks, at.chain, at.jj);
         }
         float b0 = 0.0f, b1 = 0.0f;
-        if (lane < n) b0 = p.beta[(gr0 + lane) * H + h];
-        if (lane + 32 < n) b1 = p.beta[(gr0 + lane + 32) * H + h];
-        if (!last && n == CH && lane == 0) {  // on their way into L2 while the group is still busy with the item before
+        if (lane < n) b0 = LAYER ? reinterpret_cast<const float*>(in + kSlotInBeta)[lane] : p.beta[(gr0 + lane) * H + h];
+        if (lane + 32 < n) b1 = LAYER ? reinterpret_cast<const float*>(in + kSlotInBeta)[lane + 32] : p.beta[(gr0 + lane + 32) * H + h];
+        if (!LAYER && !last && n == CH && lane == 0) {  // on their way into L2 while the group is still busy with the item before
             const int row = (int)gr0;
             for (int x = 0; x < 4; ++x) tensor_prefetch_3d(&p.tm_g, x * 32, h, row);
             for (int x = 0; x < 2; ++x) tensor_prefetch_3d(&p.tm_k, x * 64, h, row);
             for (int x = 0; x < 2; ++x) tensor_prefetch_3d(&p.tm_q, x * 64, h, row);
             for (int x = 0; x < 2; ++x) tensor_prefetch_3d(&p.tm_v, x * 64, h, row);
         }
+        const int row = (int)gr0;
+        const uint4 z = make_uint4(0, 0, 0, 0);
+        // The log decays, as soon as the item before has formed its L and M; then the other rows, when it is through with its own.
+        if (it > 0 && !mbar_wait(bar_gfree, free_phase, ctx, kStatusWaitPrefill)) break;
+        if (lane == 0) *item_slot = last ? -1 : (int)item;
+        if (last) {  // tell the compute warps that there is nothing more
+            if (lane == 0) mbar_arrive(bar_g);
+            break;
+        }
+        if (n == CH) {
+            if (lane == 0) {
+                mbar_arrive_expect_tx(bar_g, 4u * kBox);
+                if constexpr (LAYER) bulk_load(gs + gG, in + kSlotInG, 4 * kBox, bar_g);
+                else
+                    for (int x = 0; x < 4; ++x) tensor_load_3d(gs + gG + x * kBox, &p.tm_g, x * 32, h, row, bar_g);
+            }
+        } else {
+            for (int e = lane; e < CH * 32; e += 32) {
+                const int r = e >> 5, piece = e & 31;
+                const void* src = LAYER ? (const void*)(in + kSlotInG + box_piece(r, piece)) : (const void*)(p.g + ((gr0 + r) * H + h) * DK + piece * 4);
+                *reinterpret_cast<uint4*>(gs + gG + box_piece(r, piece)) = r < n ? *reinterpret_cast<const uint4*>(src) : z;
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_g);
+        }
         if (it > 0) {
             if (!mbar_wait(bar_free, free_phase, ctx, kStatusWaitPrefill)) break;
             free_phase ^= 1u;
         }
         ++it;
-        if (last) {  // tell the compute warps that there is nothing more
-            if (lane == 0) {
-                *item_slot = -1;
-                mbar_arrive(bar_raw);
-            }
-            break;
-        }
         betas[lane] = b0;
         betas[lane + 32] = b1;
-        if (lane == 0) *item_slot = (int)item;
         if (n == CH) {
             __syncwarp();
             if (lane == 0) {
-                mbar_arrive_expect_tx(bar_raw, 3u * kTile + 4u * kBox);
-                const int row = (int)gr0;
-                for (int x = 0; x < 4; ++x) tensor_load_3d(gs + gG + x * kBox, &p.tm_g, x * 32, h, row, bar_raw);
-                for (int x = 0; x < 2; ++x) tensor_load_3d(gs + gK + x * kBox, &p.tm_k, x * 64, h, row, bar_raw);
-                for (int x = 0; x < 2; ++x) tensor_load_3d(gs + gQ + x * kBox, &p.tm_q, x * 64, h, row, bar_raw);
-                for (int x = 0; x < 2; ++x) tensor_load_3d(gs + gV + x * kBox, &p.tm_v, x * 64, h, row, bar_raw);
+                mbar_arrive_expect_tx(bar_raw, 3u * kTile);
+                if constexpr (LAYER) {
+                    bulk_load(gs + gK, in + kSlotInK, 3 * kTile, bar_raw);
+                } else {
+                    for (int x = 0; x < 2; ++x) tensor_load_3d(gs + gK + x * kBox, &p.tm_k, x * 64, h, row, bar_raw);
+                    for (int x = 0; x < 2; ++x) tensor_load_3d(gs + gQ + x * kBox, &p.tm_q, x * 64, h, row, bar_raw);
+                    for (int x = 0; x < 2; ++x) tensor_load_3d(gs + gV + x * kBox, &p.tm_v, x * 64, h, row, bar_raw);
+                }
             }
         } else {
-            const uint4 z = make_uint4(0, 0, 0, 0);
             for (int e = lane; e < CH * 16; e += 32) {
-                const int r = e >> 4, c = e & 15;
+                const int r = e >> 4, c = e & 15, box = box_piece(r, c);
                 const long long at = ((gr0 + r) * H + h) * DK + c * 8;
-                const bool in = r < n;
-                *reinterpret_cast<uint4*>(gs + gQ + box_piece(r, c)) = in ? *reinterpret_cast<const uint4*>(p.q + at) : z;
-                *reinterpret_cast<uint4*>(gs + gK + box_piece(r, c)) = in ? *reinterpret_cast<const uint4*>(p.k + at) : z;
-                *reinterpret_cast<uint4*>(gs + gV + box_piece(r, c)) = in ? *reinterpret_cast<const uint4*>(p.v + at) : z;
-            }
-            for (int e = lane; e < CH * 32; e += 32) {
-                const int r = e >> 5, piece = e & 31;
-                const long long at = ((gr0 + r) * H + h) * DK + piece * 4;
-                *reinterpret_cast<uint4*>(gs + gG + box_piece(r, piece)) = r < n ? *reinterpret_cast<const uint4*>(p.g + at) : z;
+                const bool live = r < n;
+                *reinterpret_cast<uint4*>(gs + gK + box) = live ? *reinterpret_cast<const uint4*>(LAYER ? (const void*)(in + kSlotInK + box) : (const void*)(p.k + at)) : z;
+                *reinterpret_cast<uint4*>(gs + gV + box) = live ? *reinterpret_cast<const uint4*>(LAYER ? (const void*)(in + kSlotInV + box) : (const void*)(p.v + at)) : z;
+                *reinterpret_cast<uint4*>(gs + gQ + box) = live ? *reinterpret_cast<const uint4*>(LAYER ? (const void*)(in + kSlotInQ + box) : (const void*)(p.q + at)) : z;
             }
             fence_proxy_async_smem();  // V is read by the tensor core as it stands
             __syncwarp();
@@ -584,6 +641,7 @@ __device__ __forceinline__ void intra_loader(const SpParams& p, unsigned char* s
     }
 }
 
+template <bool LAYER>
 __device__ void intra_role(const SpParams& p, unsigned char* smem, const uint32_t tm) {
     volatile uint32_t* ctl = reinterpret_cast<volatile uint32_t*>(smem + oCtl);
     const WaitCtx ctx{ctl, ctl + 1, p.status};
@@ -591,13 +649,13 @@ __device__ void intra_role(const SpParams& p, unsigned char* smem, const uint32_
     if (tid == 0) {
         for (int g = 0; g < kGroups; ++g) {
             uint64_t* b = reinterpret_cast<uint64_t*>(smem + g * kGroupBytes + gBars);
-            for (int i = 0; i < 4; ++i) mbar_init(b + i, i == 2 ? 8 : 1);  // raw, mma, L^T/M^T (eight issuers), free
+            for (int i = 0; i < kGroupBars; ++i) mbar_init(b + i, i == 2 ? 8 : 1);  // raw, mma, L^T/M^T (eight issuers), free, log decays, their place free
         }
         mbar_init_fence();
     }
     __syncthreads();
-    if (warp == kLoaderWarp || warp == kOutWarp) intra_loader(p, smem, ctx, warp == kLoaderWarp ? 0 : 1);
-    else if (warp != kMmaWarp) intra_group(p, smem, tm, ctx, warp < kGroupThreads / 32 ? 0 : 1);
+    if (warp == kLoaderWarp || warp == kOutWarp) intra_loader<LAYER>(p, smem, ctx, warp == kLoaderWarp ? 0 : 1);
+    else if (warp != kMmaWarp) intra_group<LAYER>(p, smem, tm, ctx, warp < kGroupThreads / 32 ? 0 : 1);
     tc::fence_before_sync();
     __syncthreads();
 }
@@ -637,6 +695,26 @@ __device__ __forceinline__ int state_bar_count(int i) {
     return warps ? kCompute / 32 : 1;
 }
 static_assert(kStateBars * 8 <= 192, "state role barriers");
+
+// Waits until a count in global memory has reached `want`; gives up when it has stood still for the waits' limit.
+__device__ __forceinline__ bool count_wait(const unsigned int* at, unsigned want, const WaitCtx& ctx, int code) {
+    unsigned seen = 0;
+    uint64_t t0 = global_timer_ns();
+    for (;;) {
+        unsigned v;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(at) : "memory");
+        if (v >= want) return true;
+        const uint64_t now = global_timer_ns();
+        if (v != seen) {
+            seen = v;
+            t0 = now;
+        } else if (now - t0 > ctx.limit_ns) {
+            atomicCAS(ctx.status, 0, code);
+            return false;
+        }
+        __nanosleep(100);
+    }
+}
 
 // What one walk of the state role covers: chunks [ja, jb) of its chain, where the state comes from and goes to, whether
 // U takes part (not in the walk that yields a segment's transition) and whether outputs are produced.
@@ -763,6 +841,9 @@ __device__ void state_role(const SpParams& p, unsigned char* smem, const uint32_
             if (leader) atomicAdd(const_cast<uint32_t*>(ctl), 1u);
             __syncwarp();
         }
+        // Nobody else waits for the last two chunks' buffers; a block that goes on to another chain sets its barriers up again.
+        for (int c = max(count - 2, 0); c < count; ++c)
+            if (!ready(bEmptyQW + (c & 1), c >> 1) || !ready(bEmptyMKd + (c & 1), c >> 1)) break;
         tc::fence_before_sync();
         __syncthreads();
         return;
@@ -873,13 +954,13 @@ __device__ void state_role(const SpParams& p, unsigned char* smem, const uint32_
     uint16_t gt[2][2][4];
     auto fetch_gate = [&](int c) {
         const int i_first = (j0 + c) * CH, n = min(CH, T - i_first);
-        const uint16_t* at = p.gate + ((row0 + i_first + fi) * H + h) * DV + fv;
+        const uint16_t* at = p.gate + (row0 + i_first + fi) * p.gate_stride + h * DV + fv;
 #pragma unroll
         for (int g = 0; g < 2; ++g)
 #pragma unroll
             for (int e = 0; e < 2; ++e)
 #pragma unroll
-                for (int q = 0; q < 4; ++q) gt[g][e][q] = fi + 8 * g + e < n ? at[(long long)(8 * g + e) * H * DV + 8 * q] : (uint16_t)0;
+                for (int q = 0; q < 4; ++q) gt[g][e][q] = fi + 8 * g + e < n ? at[(8 * g + e) * p.gate_stride + 8 * q] : (uint16_t)0;
     };
     auto emit = [&](int c) -> bool {
         bool ok = wait(bO + (c & 1), c >> 1);
@@ -1024,7 +1105,48 @@ __device__ void state_role(const SpParams& p, unsigned char* smem, const uint32_
     __syncthreads();
 }
 
+// Both roles of a pass in one launch: every block takes items until there are none, then chains.  A block waits for other blocks'
+// items only when every item has been handed out, that is to blocks that are running and wait for nobody.
+template <bool LAYER>
+__device__ void fused_roles(const SpParams& p, unsigned char* smem, const uint32_t tm) {
+    volatile uint32_t* ctl = reinterpret_cast<volatile uint32_t*>(smem + oCtl);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + oBarsState);
+    unsigned int* set = p.sets + p.ctr * kTailSet;
+    const int tid = threadIdx.x, chains = p.batch * p.H;
+    intra_role<LAYER>(p, smem, tm);
+    if (ctl[1] != 0u) return;
+    if (tid < kGroupBars * kGroups) mbar_inval(reinterpret_cast<uint64_t*>(smem + tid / kGroupBars * kGroupBytes + gBars) + tid % kGroupBars);
+    for (bool first = true;; first = false) {
+        fence_proxy_async_smem();  // what the role before left in shared memory is overwritten by bulk copies
+        tc::fence_before_sync();
+        __syncthreads();
+        if (tid == 0) {
+            const int chain = (int)atomicAdd(set + 1, 1u);
+            if (chain < chains) {
+                const int g = chain / p.group, want = min(p.group, chains - g * p.group) * p.seg_chunks;
+                if (!count_wait(set + 2 + g, (unsigned)want, WaitCtx{ctl, ctl + 1, p.status}, kStatusWaitPrefill)) ctl[1] = 1u;
+                if (!first)
+                    for (int i = 0; i < kStateBars; ++i) {
+                        mbar_inval(bars + i);
+                        mbar_init(bars + i, state_bar_count(i));
+                    }
+                mbar_init_fence();
+            }
+            ctl[3] = (uint32_t)chain;
+        }
+        __syncthreads();
+        tc::fence_after_sync();
+        fence_proxy_async_global();
+        const int chain = (int)ctl[3];
+        if (chain >= chains || ctl[1] != 0u) break;
+        const Walk wk{p.state_chunk0, p.state_chunk0 + p.seg_chunks, 0, nullptr, 0, nullptr, true, true};
+        state_role(p, smem, tm, chain, wk);
+        if (ctl[1] != 0u) break;
+    }
+}
+
 // One launch: the state role of one segment on the chain blocks, then the intra role of the next segment on all blocks.
+template <bool LAYER>
 __global__ void __launch_bounds__(kThreadsSp, 1) prefill_sp_kernel(const __grid_constant__ SpParams p) {
     extern __shared__ __align__(1024) unsigned char smem[];
     volatile uint32_t* ctl = reinterpret_cast<volatile uint32_t*>(smem + oCtl);
@@ -1038,15 +1160,18 @@ __global__ void __launch_bounds__(kThreadsSp, 1) prefill_sp_kernel(const __grid_
         mbar_init_fence();
         // the next launch's counter; nobody reads it during this launch.  (A scan pass leaves the counters alone: it may run
         // beside the next super-block's intra launch on another stream.)
-        if (blockIdx.x == 0 && p.scan_pass == 0) p.counters[p.ctr ^ 1] = 0u;
+        if (blockIdx.x == 0 && p.scan_pass == 0 && !p.fused) p.counters[p.ctr ^ 1] = 0u;
     }
+    if (p.fused && blockIdx.x == 0 && tid < kTailSet) p.sets[(p.ctr ^ 1) * kTailSet + tid] = 0u;  // likewise
     if (warp == 0) tc::tmem_alloc(tmem_slot, kTmemCols);
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
     const uint32_t tm = *tmem_slot;
     const int chains = p.batch * p.H;
-    if (p.scan_pass == 1) {  // (chain, segment s < scan_p1, kind): the segment's offset and transition
+    if (p.fused) {
+        fused_roles<LAYER>(p, smem, tm);
+    } else if (p.scan_pass == 1) {  // (chain, segment s < scan_p1, kind): the segment's offset and transition
         const int kind = blockIdx.x & 1, sg = (blockIdx.x >> 1) % p.scan_p1, chain = (blockIdx.x >> 1) / p.scan_p1;
         if (chain < chains) {
             const int hi = p.state_chunk0 + p.seg_chunks;  // the launch's chunk range ends here
@@ -1072,7 +1197,7 @@ __global__ void __launch_bounds__(kThreadsSp, 1) prefill_sp_kernel(const __grid_
         state_role(p, smem, tm, (int)blockIdx.x, wk);
         tc::fence_after_sync();
     }
-    if (p.has_intra && ctl[1] == 0u) intra_role(p, smem, tm);
+    if (!p.fused && p.has_intra && ctl[1] == 0u) intra_role<LAYER>(p, smem, tm);
     tc::fence_before_sync();
     __syncthreads();
     if (warp == 0) tc::tmem_dealloc(tm, kTmemCols);
@@ -1150,11 +1275,27 @@ static bool row_tensor_map(CUtensorMap* tm, const void* base, int elem, int H, l
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-constexpr long long kCounterBytes = 256;  // tail of the workspace: the two item counters
+constexpr long long kCounterBytes = kPrefillTailBytes;  // tail of the workspace: the two item counters
 
 int64_t core_prefill_workspace_bytes(int32_t heads, int32_t batch, int32_t chunks_per_pass) {
     if (heads < 1 || batch < 1 || chunks_per_pass < 1) return 0;
     return (int64_t)heads * batch * chunks_per_pass * kSlotBytes + kCounterBytes;
+}
+
+// A fused launch over chunks [chunk0, chunk0 + chunks) of every sequence; pass = its number in the call.
+template <bool LAYER>
+static int fused_launch(SpParams& p, unsigned char* slots, unsigned int* tail, int pass, int chunks, int chunk0, cudaStream_t stream) {
+    const long long chains = (long long)p.H * p.batch, items = chains * chunks, sms = sm_count(), most = items > chains ? items : chains;
+    p.seg_chunks = chunks;
+    p.intra_chunk0 = p.state_chunk0 = chunk0;
+    p.ws_intra = p.ws_state = slots;
+    p.counters = tail;
+    p.sets = tail + kTailSets;
+    p.ctr = pass & 1;
+    p.fused = 1;
+    p.group = (int)((chains + kTailGroups - 1) / kTailGroups);
+    prefill_sp_kernel<LAYER><<<(unsigned)(most < sms ? most : sms), kThreadsSp, kSmemSp, stream>>>(p);
+    return (int)cudaGetLastError();
 }
 
 // The launches over every segment of the longest sequence, in stream order.  A workspace of two or more chunks per
@@ -1200,7 +1341,7 @@ int core_prefill_sp_launch(int32_t heads, int32_t batch, const int32_t* cu_seqle
     int dev = 0;
     cudaGetDevice(&dev);
     if (configured_dev != dev) {
-        const cudaError_t e = cudaFuncSetAttribute(prefill_sp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemSp);
+        const cudaError_t e = cudaFuncSetAttribute(prefill_sp_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemSp);
         if (e != cudaSuccess) return (int)e;
         configured_dev = dev;
     }
@@ -1219,7 +1360,7 @@ int core_prefill_sp_launch(int32_t heads, int32_t batch, const int32_t* cu_seqle
     p.state_in = state_in; p.state_out = state_out;
     p.state_off = reinterpret_cast<const long long*>(state_off);
     p.state_bf16 = bf16_state ? 1 : 0;
-    p.gate = gate; p.norm_w = norm_w; p.eps = eps; p.out = out;
+    p.gate = gate; p.gate_stride = (long long)heads * DV; p.norm_w = norm_w; p.eps = eps; p.out = out;
     if (scatter != nullptr) {
         if (scatter->ranks < 1 || scatter->ranks > 8 || scatter->head0 < 0 || scatter->head0 + heads > scatter->heads_total) return kInvalid;
         for (int r = 0; r < scatter->ranks; ++r) {
@@ -1246,7 +1387,7 @@ int core_prefill_sp_launch(int32_t heads, int32_t batch, const int32_t* cu_seqle
     if (out != nullptr && !row_tensor_map(&p.tm_out, out, 2, heads, rows_cap)) return (int)cudaErrorNotSupported;
     for (int r = 0; r < p.ranks; ++r)
         if (!row_tensor_map(&p.tm_full[r], p.full[r], 2, p.heads_total, rows_cap)) return (int)cudaErrorNotSupported;
-    cudaError_t e = cudaMemsetAsync(p.counters, 0, 2 * sizeof(unsigned int), stream);
+    cudaError_t e = cudaMemsetAsync(p.counters, 0, kCounterBytes, stream);
     if (e != cudaSuccess) return (int)e;
     const long long sms = sm_count();
     // Few chains and a long sequence: the serial walk over a chain's chunks is the critical path whatever the number of
@@ -1317,10 +1458,10 @@ int core_prefill_sp_launch(int32_t heads, int32_t batch, const int32_t* cu_seqle
                     // which is ready about now, off the machine until they are done, and the links idle.  From the second
                     // super-block on they leave that pass its SMs (measured on 8 GPUs, 2^20 tokens: 28.6 -> 26.1 ms).
                     const long long items = chains * cnt, room = b == 0 ? sms : (sms - Kb * chains > sms / 2 ? sms - Kb * chains : sms / 2);
-                    prefill_sp_kernel<<<(unsigned)(items < room ? items : room), kThreadsSp, kSmemSp, side->a>>>(p);
+                    prefill_sp_kernel<false><<<(unsigned)(items < room ? items : room), kThreadsSp, kSmemSp, side->a>>>(p);
                     if ((e = cudaGetLastError()) != cudaSuccess) return (int)e;
                     p.has_intra = 0; p.has_state = 1; p.scan_pass = 1;
-                    prefill_sp_kernel<<<(unsigned)(2 * Kb * chains), kThreadsSp, kSmemSp, side->a>>>(p);
+                    prefill_sp_kernel<false><<<(unsigned)(2 * Kb * chains), kThreadsSp, kSmemSp, side->a>>>(p);
                     if ((e = cudaGetLastError()) != cudaSuccess) return (int)e;
                     scan_compose_kernel<<<(unsigned)(chains * (DV / kComposeCols)), 128, 0, side->a>>>(p);
                     if ((e = cudaGetLastError()) != cudaSuccess) return (int)e;
@@ -1328,7 +1469,7 @@ int core_prefill_sp_launch(int32_t heads, int32_t batch, const int32_t* cu_seqle
                     // the other: the walks with the outputs (and the stores to the peers), super-block after super-block
                     cudaStreamWaitEvent(side->b, side->ready[b], 0);
                     p.scan_pass = 2;
-                    prefill_sp_kernel<<<(unsigned)(Kb * chains), kThreadsSp, kSmemSp, side->b>>>(p);
+                    prefill_sp_kernel<false><<<(unsigned)(Kb * chains), kThreadsSp, kSmemSp, side->b>>>(p);
                     if ((e = cudaGetLastError()) != cudaSuccess) return (int)e;
                     carry = p.scan_carry_out;
                 }
@@ -1354,17 +1495,28 @@ int core_prefill_sp_launch(int32_t heads, int32_t batch, const int32_t* cu_seqle
             p.scan_carry_in = nullptr; p.scan_carry_out = nullptr;
             p.has_intra = 1; p.has_state = 0; p.scan_pass = 0;
             const long long items = chains * need;
-            prefill_sp_kernel<<<(unsigned)(items < sms ? items : sms), kThreadsSp, kSmemSp, stream>>>(p);
+            prefill_sp_kernel<false><<<(unsigned)(items < sms ? items : sms), kThreadsSp, kSmemSp, stream>>>(p);
             if ((e = cudaGetLastError()) != cudaSuccess) return (int)e;
             p.has_intra = 0; p.has_state = 1; p.scan_pass = 1;
-            prefill_sp_kernel<<<(unsigned)(2 * (K - 1) * chains), kThreadsSp, kSmemSp, stream>>>(p);
+            prefill_sp_kernel<false><<<(unsigned)(2 * (K - 1) * chains), kThreadsSp, kSmemSp, stream>>>(p);
             if ((e = cudaGetLastError()) != cudaSuccess) return (int)e;
             scan_compose_kernel<<<(unsigned)(chains * (DV / kComposeCols)), 128, 0, stream>>>(p);
             if ((e = cudaGetLastError()) != cudaSuccess) return (int)e;
             p.scan_pass = 2;
-            prefill_sp_kernel<<<(unsigned)(K * chains), kThreadsSp, kSmemSp, stream>>>(p);
+            prefill_sp_kernel<false><<<(unsigned)(K * chains), kThreadsSp, kSmemSp, stream>>>(p);
             return (int)cudaGetLastError();
         }
+    }
+    // More chains than SMs: the state role fills the machine by itself, there is nothing to run beside it, and a fused launch over
+    // all the slots needs half as many launches as two halves that swap.  64 heads x 8
+    // sequences, 8,192 rows, a workspace of 32 chunks a chain: 641 -> 570 us.
+    if (chains > sms && need > 0) {
+        const long long passes = (need + whole - 1) / whole, n = (need + passes - 1) / passes;
+        for (long long c = 0; c < need; c += n) {
+            const int rc = fused_launch<false>(p, base, p.counters, (int)(c / n), (int)n, (int)c, stream);
+            if (rc != 0) return rc;
+        }
+        return 0;
     }
     const long long segs = need > 0 ? (need + seg - 1) / seg : 0;
     int launch_no = 0;
@@ -1381,7 +1533,7 @@ int core_prefill_sp_launch(int32_t heads, int32_t batch, const int32_t* cu_seqle
             const long long items = chains * seg, want = items < sms ? items : sms;
             if (grid < want) grid = want;
         }
-        prefill_sp_kernel<<<(unsigned)grid, kThreadsSp, kSmemSp, stream>>>(p);
+        prefill_sp_kernel<false><<<(unsigned)grid, kThreadsSp, kSmemSp, stream>>>(p);
         return (int)cudaGetLastError();
     };
     if (segs == 0) return launch(-1, 0);  // nothing but empty sequences: their states are copied
@@ -1398,6 +1550,32 @@ int core_prefill_sp_launch(int32_t heads, int32_t batch, const int32_t* cu_seqle
         }
     }
     return 0;
+}
+
+// A pass of a layer prefill.  No halves that swap: a slot's inputs and results share its bytes, so a pass takes all the chunks
+// that the workspace has slots for, both roles in one launch.
+int layer_pass_launch(int32_t heads, int32_t batch, const int32_t* cu_rows, int32_t chunks, int32_t chunk0, unsigned char* slots,
+                      unsigned int* tail, const void* state_in, void* state_out, const int64_t* state_off, bool bf16_state,
+                      const glm53f_bf16* gate, int64_t gate_stride, const glm53f_bf16* norm_w, float eps, glm53f_bf16* out, cudaStream_t stream) {
+    static int configured_dev = -1;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (configured_dev != dev) {
+        const cudaError_t e = cudaFuncSetAttribute(prefill_sp_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemSp);
+        if (e != cudaSuccess) return (int)e;
+        configured_dev = dev;
+    }
+    SpParams p{};
+    p.H = heads; p.batch = batch; p.cu = cu_rows;
+    p.state_in = state_in; p.state_out = state_out;
+    p.state_off = reinterpret_cast<const long long*>(state_off);
+    p.state_bf16 = bf16_state ? 1 : 0;
+    p.gate = gate; p.gate_stride = gate_stride; p.norm_w = norm_w; p.eps = eps; p.out = out;
+    p.status = status_word();
+    if (p.status == nullptr) return (int)cudaErrorUnknown;
+    // Only full chunks leave by tensor stores, and the metadata vouches for their rows: the map's extent bounds nothing.
+    if (!row_tensor_map(&p.tm_out, out, 2, heads, 0x7fffffffll)) return (int)cudaErrorNotSupported;
+    return fused_launch<true>(p, slots, tail, chunk0 / chunks, chunks, chunk0, stream);
 }
 
 // ---------------------------------------------------------------------------------------------------------------------

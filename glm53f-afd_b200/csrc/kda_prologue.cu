@@ -7,17 +7,18 @@
 // without multiply-add contraction like the chain): four taps summed in order, one bf16 rounding after the SiLU, decay
 // exp(lower * sigmoid(exp(A_log) (a + dt_bias))), beta = bf16(sigmoid(b)), each L2 norm as a lane's four consecutive
 // channels summed in order, then the xor butterfly.  (Bit for bit in the verify sink; the prefill sink uses the
-// hardware's approximate division, exponential and reciprocal root, see sigmoid_ below.)
+// hardware's approximate division, exponential and reciprocal root, four rows a warp, and multiply-adds.)
 //
-// One warp per (request, head, row); a lane owns four consecutive channels, so the norms need no shared memory.  The
-// work is bound by instruction issue (about 850 instructions per row and lane, most of them IEEE divisions and
+// A lane owns four consecutive channels, so the norms need no shared memory.  With the chain's arithmetic (verify and exact
+// sinks): one warp per (request, head, row).  The work is bound by instruction issue (about 850 instructions per row and lane, most of them IEEE divisions and
 // exponentials), so a warp takes ONE row and reads its three predecessors again (the four warps of a block take four
 // consecutive rows; the predecessors come from L1/L2): every load of a warp is in flight at once and 79 registers
 // allow 24 resident warps per SM.  (A warp that walks 16 rows with the three earlier rows sliding in registers needs
 // 143 registers and was half as fast.)
 //
 // Three sinks:
-//  * a prefill pass: dense core inputs for one pass of rows in the caller's workspace.  q and k are rounded to fp16
+//  * a prefill pass: core inputs for one pass of chunks, in the caller's workspace as the slots of kda_prefill_sp.cu take
+//    them (a chunk's rows together, already in the swizzle that one bulk copy brings to the tensor core).  q and k are rounded to fp16
 //    (they lie in [-1, 1]; eleven mantissa bits), the one place where the chunked prefill departs from the chain's
 //    FP32 q and k before the tensor-core products: with bf16's eight bits the rounding of k alone, which reaches the
 //    state through K^T D, would take the state's whole error budget when few rows dominate it.  The decay is kept as
@@ -29,6 +30,7 @@
 //  * a pass of the exact prefill (kda_rows.cu): as the verify sink, q in f32 with the chain's arithmetic too, all of it in
 //    the caller's workspace.
 
+#include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
 #include "common.cuh"
@@ -54,26 +56,21 @@ struct ProParams {
     const float* a_log;
     const float* dt_bias;
     float lower;
-    // prefill pass: [batch * pass_rows][H][128] (beta [batch * pass_rows][H])
-    uint16_t *q, *k, *v;
-    float *g, *beta;
-    // verify: q as fp16 into the output rows (through `q`), the rest into the replay saves
+    unsigned char* slots;  // prefill pass: [batch][H][pass_rows / 64]
+    // verify: q as fp16 into the output rows, the rest into the replay saves
+    uint16_t* q;
     long long out_stride;
     float *k_save, *g_save, *b_save;
     uint16_t* v_save;
     float* qf;  // exact sink: q in f32 (k, decay multiplier, v and beta through the saves' pointers)
     int rows1;  // cu == nullptr: one request of rows1 rows
 };
-enum Sink : int { kFast = 0, kVerify = 1, kExact = 2 };
+enum Sink : int { kVerify = 1, kExact = 2 };
 
-// The verify sink keeps the chain's IEEE arithmetic (its results are the replay saves, bit for bit); the prefill sink
-// feeds tensor-core products that round every operand to bf16 anyway, so there the divisions, exponentials and
-// reciprocal roots are the hardware approximations (a few ulp of FP32): a third of the instructions.
-template <bool FAST>
-__device__ __forceinline__ float sigmoid_(float x) {
-    if constexpr (FAST) return __fdividef(1.0f, 1.0f + __expf(-x));
-    else return 1.0f / (1.0f + expf(-x));
-}
+// IEEE arithmetic is the chain's (its results are the replay saves, bit for bit).  q of the verify sink and everything of the
+// prefill sink feed tensor-core products that round every operand to bf16 or fp16 anyway, so there the divisions, exponentials
+// and reciprocal roots are the hardware approximations (a few ulp of FP32).
+__device__ __forceinline__ float sigmoid_(float x) { return 1.0f / (1.0f + expf(-x)); }
 template <bool FAST>
 __device__ __forceinline__ float silu_(float x) {
     if constexpr (FAST) return __fdividef(x, 1.0f + __expf(-x));
@@ -106,7 +103,7 @@ __device__ __forceinline__ uint2 pack4(const float (&x)[4]) {
 
 template <int SINK>
 __global__ void __launch_bounds__(128, 6) layer_prologue_kernel(const ProParams p) {
-    constexpr bool VERIFY = SINK == kVerify, EXACT = SINK == kExact, FAST = SINK == kFast;
+    constexpr bool VERIFY = SINK == kVerify, EXACT = SINK == kExact;
     if constexpr (EXACT) {
         asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
         asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -160,7 +157,7 @@ __global__ void __launch_bounds__(128, 6) layer_prologue_kernel(const ProParams 
             acc = acc + __uint_as_float(ww[2 * c + 1] << 16) * xv[2][c];
             acc = acc + __uint_as_float(ww[2 * c + 1] & 0xffff0000u) * xv[3][c];
             // q reaches only the outputs, which carry bf16-operand rounding in both chunked forms: the fast form there
-            act[part][c] = bf16_round(part == 0 ? silu_<!EXACT>(acc) : silu_<FAST>(acc));
+            act[part][c] = bf16_round(part == 0 ? silu_<!EXACT>(acc) : silu_<false>(acc));
         }
     }
     // L2 norms of q and k (eps 1e-6 inside the root), q also times 128^-0.5.
@@ -174,7 +171,7 @@ __global__ void __launch_bounds__(128, 6) layer_prologue_kernel(const ProParams 
         }
         sq = butterfly(sq);
         sk = butterfly(sk);
-        const float iq = inv_norm_<!EXACT>(sq), ik = inv_norm_<FAST>(sk);
+        const float iq = inv_norm_<!EXACT>(sq), ik = inv_norm_<false>(sk);
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
             qn[c] = (act[0][c] * iq) * (1.0f / sqrtf((float)DK));
@@ -185,8 +182,8 @@ __global__ void __launch_bounds__(128, 6) layer_prologue_kernel(const ProParams 
     unpack4(a_bits, a4);
     const float dtb[4] = {dtb4.x, dtb4.y, dtb4.z, dtb4.w};
 #pragma unroll
-    for (int c = 0; c < 4; ++c) lg[c] = p.lower * sigmoid_<FAST>(decay_rate * (a4[c] + dtb[c]));
-    const float bt = bf16_round(sigmoid_<FAST>(blogit));
+    for (int c = 0; c < 4; ++c) lg[c] = p.lower * sigmoid_(decay_rate * (a4[c] + dtb[c]));
+    const float bt = bf16_round(sigmoid_(blogit));
     if constexpr (VERIFY) {
         const long long sv = (gr * H + h) * DK + c0;
         if (j < p.pass_rows) *reinterpret_cast<uint2*>(p.q + gr * p.out_stride + (long long)h * DK + c0) = pack4_fp16(qn);  // rows past 16 get no output: leave theirs alone
@@ -201,14 +198,111 @@ __global__ void __launch_bounds__(128, 6) layer_prologue_kernel(const ProParams 
         *reinterpret_cast<float4*>(p.g_save + at) = make_float4(expf(lg[0]), expf(lg[1]), expf(lg[2]), expf(lg[3]));
         *reinterpret_cast<uint2*>(p.v_save + at) = pack4(act[2]);
         if (lane == 0) p.b_save[orow * H + h] = bt;
-    } else {
-        const long long orow = (long long)b * p.pass_rows + j, at = (orow * H + h) * DK + c0;
-        *reinterpret_cast<uint2*>(p.q + at) = pack4_fp16(qn);
-        *reinterpret_cast<uint2*>(p.k + at) = pack4_fp16(kn);
-        *reinterpret_cast<uint2*>(p.v + at) = pack4(act[2]);
-        *reinterpret_cast<float4*>(p.g + at) = make_float4(lg[0], lg[1], lg[2], lg[3]);
-        if (lane == 0) p.beta[orow * H + h] = bt;
     }
+    }
+}
+
+// ---- the prefill sink ---------------------------------------------------------------------------------------------------
+// Bound by instruction issue before it is bound by memory (a row and head: 1 KiB in, 1.3 KiB out).  A warp takes four consecutive
+// rows: seven rows of inputs instead of sixteen, the weights once, and everything in pairs of channels (two-wide multiply-adds).
+// 1,280 rows x 64 heads: 79 us with a warp per row as in the kernel above, 52 so.
+constexpr int kRowsPer = 4;
+__device__ __forceinline__ float2 lo_hi(uint32_t w) { return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)); }
+__device__ __forceinline__ float2 add2(float2 a, float2 b) { return fma2(a, {1.0f, 1.0f}, b); }
+// 1 / (1 + e^-x)
+__device__ __forceinline__ float2 sigmoid2(float2 x) {
+    const float2 t = mul2(x, {-kLog2e, -kLog2e}), d = add2({ex2_approx(t.x), ex2_approx(t.y)}, {1.0f, 1.0f});
+    return make_float2(rcp_approx(d.x), rcp_approx(d.y));
+}
+__device__ __forceinline__ uint32_t fp16x2(float2 x) {
+    const __half2 h = __float22half2_rn(x);
+    return *reinterpret_cast<const uint32_t*>(&h);
+}
+
+__global__ void __launch_bounds__(128, 4) prefill_prologue_kernel(const ProParams p) {
+    const int lane = threadIdx.x & 31, H = p.H, groups = p.pass_rows / (4 * kRowsPer), c0 = lane * 4;
+    // heads innermost: neighbouring blocks read neighbouring pieces of the same rows
+    const int h = (int)(blockIdx.x % H), b = (int)(blockIdx.x / H / groups), j0 = (int)(blockIdx.x / H % groups) * 4 * kRowsPer + (threadIdx.x >> 5) * kRowsPer;
+    const int r0 = p.cu[b], n = min(p.cu[b + 1] - r0 - p.row_shift, p.pass_rows);
+    if (j0 >= n) return;
+    const int first = p.row_shift + j0, last = p.row_shift + n - 1;  // rows of the request; rows before its first come from the conv window
+    const long long C = 3LL * H * DK;
+    const uint16_t* window = p.conv + (p.conv_off ? p.conv_off[b] : 0);
+    uint2 x[3][kRowsPer + 3];
+#pragma unroll
+    for (int d = 0; d < kRowsPer + 3; ++d) {
+        const int rr = min(first - 3 + d, last);
+        const uint16_t* row = (rr < 0 ? window + (long long)(WINDOW + rr) * C : p.P + ((long long)r0 + rr) * p.p_stride) + (long long)h * DK + c0;
+#pragma unroll
+        for (int part = 0; part < 3; ++part) x[part][d] = *reinterpret_cast<const uint2*>(row + (long long)part * H * DK);
+    }
+    uint2 a_bits[kRowsPer];
+    float bl[kRowsPer];
+#pragma unroll
+    for (int i = 0; i < kRowsPer; ++i) {
+        const long long gr = (long long)r0 + min(first + i, last);
+        a_bits[i] = *reinterpret_cast<const uint2*>(p.A + gr * p.a_stride + (long long)h * DK + c0);
+        bl[i] = bf16_bits_to_f32(p.P[gr * p.p_stride + p.b_off + h]);
+    }
+    const float4 dtb = *reinterpret_cast<const float4*>(p.dt_bias + (long long)h * DK + c0);
+    const float rate = expf(p.a_log[h]);
+    unsigned char* slot = p.slots + (((long long)b * H + h) * (p.pass_rows / 64) + (j0 >> 6)) * kPrefillSlotBytes;
+    const int r = j0 & 63;
+
+#pragma unroll
+    for (int part = 0; part < 3; ++part) {
+        const uint4* src = reinterpret_cast<const uint4*>(p.cw + (((long long)part * H + h) * DK + c0) * TAPS);
+        const uint4 wa = src[0], wb = src[1];  // a channel's four taps in two words
+        const float2 w01[TAPS] = {{__uint_as_float(wa.x << 16), __uint_as_float(wa.z << 16)}, {__uint_as_float(wa.x & 0xffff0000u), __uint_as_float(wa.z & 0xffff0000u)},
+                                  {__uint_as_float(wa.y << 16), __uint_as_float(wa.w << 16)}, {__uint_as_float(wa.y & 0xffff0000u), __uint_as_float(wa.w & 0xffff0000u)}};
+        const float2 w23[TAPS] = {{__uint_as_float(wb.x << 16), __uint_as_float(wb.z << 16)}, {__uint_as_float(wb.x & 0xffff0000u), __uint_as_float(wb.z & 0xffff0000u)},
+                                  {__uint_as_float(wb.y << 16), __uint_as_float(wb.w << 16)}, {__uint_as_float(wb.y & 0xffff0000u), __uint_as_float(wb.w & 0xffff0000u)}};
+        float2 acc[kRowsPer][2];
+#pragma unroll
+        for (int d = 0; d < kRowsPer + 3; ++d) {  // input row d is tap d - i of output row i
+            const float2 x01 = lo_hi(x[part][d].x), x23 = lo_hi(x[part][d].y);
+#pragma unroll
+            for (int i = 0; i < kRowsPer; ++i) {
+                const int t = d - i;
+                if (t == 0) acc[i][0] = mul2(w01[0], x01), acc[i][1] = mul2(w23[0], x23);
+                else if (t > 0 && t < TAPS) acc[i][0] = fma2(w01[t], x01, acc[i][0]), acc[i][1] = fma2(w23[t], x23, acc[i][1]);
+            }
+        }
+        float ss[kRowsPer];
+        uint2 y[kRowsPer];  // bf16(silu)
+#pragma unroll
+        for (int i = 0; i < kRowsPer; ++i) {
+            const float2 s01 = mul2(acc[i][0], sigmoid2(acc[i][0])), s23 = mul2(acc[i][1], sigmoid2(acc[i][1]));
+            const __nv_bfloat162 p01 = __float22bfloat162_rn(s01), p23 = __float22bfloat162_rn(s23);
+            y[i] = make_uint2(*reinterpret_cast<const uint32_t*>(&p01), *reinterpret_cast<const uint32_t*>(&p23));
+            if (part < 2) {
+                const float2 f01 = lo_hi(y[i].x), f23 = lo_hi(y[i].y), q = fma2(f23, f23, mul2(f01, f01));
+                ss[i] = q.x + q.y;
+            }
+        }
+        if (part < 2) {  // L2 norms of q and k (eps 1e-6 inside the root), q also times 128^-0.5
+#pragma unroll
+            for (int o = 16; o; o >>= 1)
+#pragma unroll
+                for (int i = 0; i < kRowsPer; ++i) ss[i] += __shfl_xor_sync(FULL, ss[i], o);
+#pragma unroll
+            for (int i = 0; i < kRowsPer; ++i) {
+                const float s = rsqrtf(ss[i] + 1e-6f) * (part == 0 ? 0.08838834764831845f : 1.0f);
+                y[i] = make_uint2(fp16x2(mul2(lo_hi(y[i].x), {s, s})), fp16x2(mul2(lo_hi(y[i].y), {s, s})));
+            }
+        }
+        unsigned char* to = slot + (part == 0 ? kSlotInQ : part == 1 ? kSlotInK : kSlotInV) + (lane & 1) * 8;
+#pragma unroll
+        for (int i = 0; i < kRowsPer; ++i)
+            if (j0 + i < n) *reinterpret_cast<uint2*>(to + prefill_box_piece(r + i, lane >> 1)) = y[i];
+    }
+#pragma unroll
+    for (int i = 0; i < kRowsPer; ++i) {
+        if (j0 + i >= n) break;
+        const float2 s01 = sigmoid2(mul2(add2(lo_hi(a_bits[i].x), {dtb.x, dtb.y}), {rate, rate})), s23 = sigmoid2(mul2(add2(lo_hi(a_bits[i].y), {dtb.z, dtb.w}), {rate, rate}));
+        const float2 g01 = mul2(s01, {p.lower, p.lower}), g23 = mul2(s23, {p.lower, p.lower});
+        *reinterpret_cast<float4*>(slot + kSlotInG + prefill_box_piece(r + i, lane)) = make_float4(g01.x, g01.y, g23.x, g23.y);
+        if (lane == 0) reinterpret_cast<float*>(slot + kSlotInBeta)[r + i] = bf16_round(sigmoid2({bl[i], bl[i]}).x);
     }
 }
 
@@ -230,21 +324,22 @@ int launch(const ProParams& pp, cudaStream_t stream) {
 
 }  // namespace
 
-int layer_prologue_launch(int32_t heads, int32_t batch, const int32_t* cu_rows, int32_t pass_rows, int32_t row_shift,
+int layer_prologue_launch(int32_t heads, int32_t batch, const int32_t* cu_rows, int32_t chunks, int32_t chunk0,
                           const glm53f_bf16* p, int64_t p_stride, int64_t b_off, const glm53f_bf16* a, int64_t a_stride,
                           const glm53f_bf16* conv, const int64_t* conv_off, const glm53f_bf16* conv_w, const float* a_log,
-                          const float* dt_bias, float lower, glm53f_bf16* q, glm53f_bf16* k, glm53f_bf16* v, float* g, float* beta,
-                          cudaStream_t stream) {
-    if (pass_rows < 16 || pass_rows % 16 != 0) return kInvalid;
+                          const float* dt_bias, float lower, unsigned char* slots, cudaStream_t stream) {
     ProParams pp{};
-    pp.H = heads; pp.batch = batch; pp.pass_rows = pass_rows; pp.row_shift = row_shift;
+    pp.H = heads; pp.batch = batch; pp.pass_rows = chunks * 64; pp.row_shift = chunk0 * 64;
     pp.cu = cu_rows;
     pp.P = p; pp.p_stride = p_stride; pp.b_off = b_off;
     pp.A = a; pp.a_stride = a_stride;
     pp.conv = conv; pp.conv_off = reinterpret_cast<const long long*>(conv_off); pp.cw = conv_w;
     pp.a_log = a_log; pp.dt_bias = dt_bias; pp.lower = lower;
-    pp.q = q; pp.k = k; pp.v = v; pp.g = g; pp.beta = beta;
-    return launch<kFast>(pp, stream);
+    pp.slots = slots;
+    const long long blocks = (long long)batch * heads * (pp.pass_rows / (4 * kRowsPer));
+    if (blocks > 0x7fffffffLL) return kInvalid;
+    prefill_prologue_kernel<<<(unsigned)blocks, 128, 0, stream>>>(pp);
+    return (int)cudaGetLastError();
 }
 
 int exact_prologue_launch(int32_t heads, int32_t batch, const int32_t* cu_rows, int32_t rows1, int32_t pass_rows, int32_t row_shift,

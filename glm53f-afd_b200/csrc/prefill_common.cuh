@@ -49,38 +49,6 @@ __device__ __forceinline__ void compute_sync() { named_bar_sync(1, kCompute); }
 
 __device__ __forceinline__ unsigned char* cell(unsigned char* tile, int R, int c, int r) { return tile + ((size_t)c * R + r) * 16; }
 
-// Two-wide FP32 products (each half rounded once).
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
-    unsigned long long r, x, y;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(x) : "f"(a.x), "f"(a.y));
-    asm("mov.b64 %0, {%1, %2};" : "=l"(y) : "f"(b.x), "f"(b.y));
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(x), "l"(y));
-    float2 c;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(c.x), "=f"(c.y) : "l"(r));
-    return c;
-}
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 d) {
-    unsigned long long r, x, y, z;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(x) : "f"(a.x), "f"(a.y));
-    asm("mov.b64 %0, {%1, %2};" : "=l"(y) : "f"(b.x), "f"(b.y));
-    asm("mov.b64 %0, {%1, %2};" : "=l"(z) : "f"(d.x), "f"(d.y));
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(x), "l"(y), "l"(z));
-    float2 c;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(c.x), "=f"(c.y) : "l"(r));
-    return c;
-}
-__device__ __forceinline__ float rcp_approx(float x) {
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
-}
-__device__ __forceinline__ float ex2_approx(float x) {
-    float r;
-    asm("ex2.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
-}
-constexpr float kLog2e = 1.4426950408889634f;
-
 // Eight FP32 values (TMEM words) to one 16-byte cell of bf16.
 __device__ __forceinline__ uint4 pack8(const uint32_t* r) {
     return make_uint4(tc::bf16x2(__uint_as_float(r[0]), __uint_as_float(r[1])), tc::bf16x2(__uint_as_float(r[2]), __uint_as_float(r[3])),
