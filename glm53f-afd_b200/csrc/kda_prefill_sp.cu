@@ -205,6 +205,16 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
         }
     };
     uint32_t raw_phase = 0, mma_phase = 0, lm_phase = 0;
+    // Fused launches count finished items.  The fence has to wait for the group's last stores, so an item is counted during the next
+    // one's last products, when they have long landed.
+    int unreported = -1;
+    auto report = [&]() {
+        if (p.fused && unreported >= 0 && gt == kGroupThreads - 1) {
+            __threadfence();
+            atomicAdd(p.sets + p.ctr * kTailSet + 2 + unreported, 1u);
+        }
+        unreported = -1;
+    };
     auto mma_wait = [&](uint64_t* bar, uint32_t& phase) -> bool {
         if (!mbar_wait(bar, phase, ctx, kStatusWaitPrefill)) return false;
         phase ^= 1u;
@@ -506,6 +516,7 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
             for (int k0 = 0; k0 < CH; k0 += 16)
                 tc::mma_bf16_if(leader, tm + gcU, tc::desc_sw128_mnmajor(gs + gV, CH, k0), tc::desc_sw128_kmajor(tpl, CH, k0), id, true);
         });
+        report();
         if (!mma_wait(bar_mma, mma_phase)) break;
         // Nothing of this item is left in the group's shared memory: the loader may bring the next item in.
         if (gt == 0) mbar_arrive(bar_free);
@@ -528,11 +539,9 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
         tc::fence_before_sync();
         group_sync();
         tc::fence_after_sync();
-        if (p.fused && gt == 0) {
-            __threadfence();
-            atomicAdd(p.sets + p.ctr * kTailSet + 2 + at_item.group, 1u);
-        }
+        unreported = at_item.group;
     }
+    report();
 }
 
 // The loader warp of group G: takes items off the counter and brings each one's rows into the group's staging.  A full
