@@ -132,11 +132,9 @@ struct Params {
 // Raw-row slot layouts, byte offsets.
 struct RawLayer {
     static constexpr int X = 0;                 // bf16 [4 taps][3 parts][128]
-    static constexpr int W = X + 4 * 3 * 256;   // bf16 [3 parts][128][4]
-    static constexpr int A = W + 3 * 1024;      // bf16 [128]
+    static constexpr int A = X + 4 * 3 * 256;   // bf16 [128]
     static constexpr int GATE = A + 256;        // bf16 [128]
-    static constexpr int DTB = GATE + 256;      // f32 [128]
-    static constexpr int B = DTB + 512;         // the 16 aligned bytes that hold the beta logit
+    static constexpr int B = GATE + 256;        // the 16 aligned bytes that hold the beta logit
     static constexpr int BYTES = B + 16;
 };
 struct RawCore {
@@ -170,12 +168,19 @@ struct Cooked {
     int pad[3];
 };
 
+// What the recurrence needs to know of a unit, left by the mover beside its state; rows < 0: no more units.  (Read from global
+// memory by the sixteen warps themselves, it queued behind their own stores of the state before.)
+struct __align__(16) UnitInfo {
+    long long s_elem;
+    int rows;
+};
+
 template <typename S, int MODE>
 struct Smem {
     static constexpr int kStateBytes = DV * DK * (int)sizeof(S);
     static constexpr int kStateSlots = sizeof(S) == 4 ? 3 : 5;
-    static constexpr int kRawSlots = sizeof(S) == 4 ? 3 : 4;  // raw-row ring depth
-    static constexpr int kRowSlots = sizeof(S) == 4 ? 3 : 4;  // cooked-row ring depth
+    static constexpr int kRawSlots = MODE == kLayer ? (sizeof(S) == 4 ? 5 : 8) : sizeof(S) == 4 ? 3 : 4;  // raw-row ring depth
+    static constexpr int kRowSlots = MODE == kLayer ? (sizeof(S) == 4 ? 5 : 8) : sizeof(S) == 4 ? 3 : 4;  // cooked-row ring depth
     static constexpr int kRawBytes = align_up(RawOf<MODE>::T::BYTES, 128);
     static constexpr int oState = 0;
     static constexpr int oRaw = oState + kStateSlots * kStateBytes;
@@ -185,7 +190,9 @@ struct Smem {
     // barriers: st_full[S], st_empty[S], raw_full[R], raw_empty[R], row_full[C], y_full[C], row_empty[C]
     static constexpr int kBars = 2 * kStateSlots + 2 * kRawSlots + 3 * kRowSlots;
     static constexpr int oCtl = oBars + kBars * 8;  // progress, abort
-    static constexpr int kBytes = oCtl + 16;
+    static constexpr int oUnits = oCtl + 16;        // UnitInfo per state slot
+    static constexpr int kBytes = oUnits + kStateSlots * 16;
+    static_assert(kBytes <= 232448, "shared memory budget");
 };
 
 struct Unit {
@@ -198,14 +205,17 @@ struct Unit {
 
 // The units of this block, u = blockIdx.x, blockIdx.x + gridDim.x, ...: (request, head) with the head fastest, or
 // (request, layer, head) for the replay.  Indices advance by 32-bit arithmetic; the metadata of the next unit
-// (row range, state and window offsets: loads from global memory) is fetched while the current one is processed.
+// (row range, state and window offsets: loads from global memory) is fetched while the current one is processed, and stays as
+// loaded until that unit's turn: arithmetic on it right after the loads would wait for them there, 1,500 cycles a unit and role.
 template <int MODE>
 struct UnitIter {
     unsigned long long u;
     unsigned b, h, layer;
     unsigned step_b, step_h;  // gridDim.x = step_b * H + step_h
     bool ok;
-    Unit nxt;
+    int r0, r1, kept;
+    long long s_off, c_off;
+    float a_log;
 
     __device__ __forceinline__ explicit UnitIter(const Params& p) {
         u = blockIdx.x;
@@ -217,42 +227,42 @@ struct UnitIter {
         const unsigned q = blockIdx.x / H;
         layer = MODE == kReplay ? q % L : 0u;
         b = MODE == kReplay ? q / L : q;
-        if (ok) nxt = fetch(p);
+        r0 = r1 = kept = 0;
+        s_off = c_off = 0;
+        a_log = 0.0f;
+        if (ok) fetch(p);
     }
-    __device__ __forceinline__ Unit fetch(const Params& p) const {
-        Unit x;
-        x.b = (int)b;
-        x.h = (int)h;
-        x.layer = (int)layer;
-        if (MODE == kReplay) {
-            x.row0 = p.cu_rows ? p.cu_rows[b] : 0;
-            x.rows = p.keep ? p.keep[b] : p.rows1;
-        } else if (p.cu_rows) {
-            const int r0 = p.cu_rows[b];
-            x.row0 = r0;
-            x.rows = p.cu_rows[b + 1] - r0;
-            if (MODE == kLayer && p.keep) {  // a commit by recomputation: only the request's first keep[b] rows
-                const int kept = p.keep[b];
-                if (kept < x.rows) x.rows = kept;
-            }
-        } else {
-            x.row0 = 0;
-            x.rows = p.rows1;
+    __device__ __forceinline__ void fetch(const Params& p) {
+        if (p.cu_rows) {
+            r0 = p.cu_rows[b];
+            if (MODE != kReplay) r1 = p.cu_rows[b + 1];
         }
-        if (x.rows < 0) x.rows = 0;
-        x.s_elem = (long long)layer * p.state_stride + (p.state_off ? p.state_off[b] : 0) + (long long)h * DV * DK;
-        x.conv_off = 0;
-        x.a_log = 0.0f;
+        if (MODE != kCore && p.keep) kept = p.keep[b];
+        if (p.state_off) s_off = p.state_off[b];
         if (MODE == kLayer) {
-            x.conv_off = p.conv_off ? p.conv_off[b] : 0;
-            x.a_log = p.a_log[h];
+            if (p.conv_off) c_off = p.conv_off[b];
+            a_log = p.a_log[h];
         }
-        return x;
     }
     __device__ __forceinline__ bool valid() const { return ok; }
     // The current unit; advances to the next one and starts fetching its metadata.
     __device__ __forceinline__ Unit take(const Params& p) {
-        const Unit cur = nxt;
+        Unit cur;
+        cur.b = (int)b;
+        cur.h = (int)h;
+        cur.layer = (int)layer;
+        cur.row0 = p.cu_rows ? r0 : 0;
+        if (MODE == kReplay) {
+            cur.rows = p.keep ? kept : p.rows1;
+        } else {
+            cur.rows = p.cu_rows ? r1 - r0 : p.rows1;
+            // a commit by recomputation: only the request's first keep[b] rows
+            if (MODE == kLayer && p.cu_rows && p.keep && kept < cur.rows) cur.rows = kept;
+        }
+        if (cur.rows < 0) cur.rows = 0;
+        cur.s_elem = (long long)layer * p.state_stride + s_off + (long long)h * DV * DK;
+        cur.conv_off = c_off;
+        cur.a_log = a_log;
         u += gridDim.x;
         ok = u < (unsigned long long)p.units;
         const unsigned H = (unsigned)p.H;
@@ -270,7 +280,7 @@ struct UnitIter {
                 ++b;
             }
         }
-        if (ok) nxt = fetch(p);
+        if (ok) fetch(p);
         return cur;
     }
 };
@@ -290,45 +300,52 @@ struct Ring {
 };
 
 // ---- the mover -----------------------------------------------------------------------------------------------
-// Calls f(dst_offset, src, bytes, is_scalar_chunk) for every piece of a row's raw inputs.  Pieces are 16-byte
-// multiples except the "scalar chunk" (beta or its logit): for that one `src` is the element's own address and the
-// mover copies the aligned 16 bytes around it, so the element lands at dst_offset + (address & 15).
-template <int MODE, typename F>
-__device__ __forceinline__ void for_each_piece(const Params& p, const Unit& u, int r, F&& f) {
+// The pieces of a row's raw inputs, one per lane: a lane works out its own piece's address and issues its own copy.  (Issued one
+// after the other by one lane, the twenty pieces of a layer row took 3,500 cycles a row, longer than any other stage of a
+// single-row launch.)  Pieces are 16-byte multiples except the "scalar chunk" (beta or its logit): for that one `src` is the
+// element's own address and the mover copies the aligned 16 bytes around it, so the element lands at off + (address & 15).
+struct Piece {
+    int off, bytes;  // bytes == 0: this lane has none
+    const void* src;
+    bool scalar;
+};
+template <int MODE>
+__device__ __forceinline__ Piece piece_of(const Params& p, const Unit& u, int r, int lane) {
     const long long gr = u.row0 + r;
+    Piece x{0, 0, nullptr, false};
     if constexpr (MODE == kLayer) {
-        const long long C = 3LL * p.H * DK;
-        const uint16_t* cs = p.conv + u.conv_off;
-#pragma unroll
-        for (int tap = 0; tap < TAPS; ++tap) {
-            const int at = r + tap;
-            const uint16_t* src_row = at < WINDOW ? cs + (long long)at * C : p.P + (u.row0 + at - WINDOW) * p.p_stride;
-#pragma unroll
-            for (int part = 0; part < 3; ++part)
-                f(RawLayer::X + (tap * 3 + part) * 256, src_row + ((long long)part * p.H + u.h) * DK, 256, false);
+        if (lane < 3 * TAPS) {
+            const int tap = lane / 3, part = lane - tap * 3, at = r + tap;
+            const uint16_t* row = at < WINDOW ? p.conv + u.conv_off + (long long)at * 3 * p.H * DK : p.P + (u.row0 + at - WINDOW) * p.p_stride;
+            x = {RawLayer::X + lane * 256, 256, row + ((long long)part * p.H + u.h) * DK, false};
+        } else if (lane == 3 * TAPS) {
+            x = {RawLayer::A, 256, p.A + gr * p.a_stride + (long long)u.h * DK, false};
+        } else if (lane == 3 * TAPS + 1) {
+            x = {RawLayer::GATE, 256, p.G + gr * p.g_stride + (long long)u.h * DV, false};
+        } else if (lane == 3 * TAPS + 2) {
+            x = {RawLayer::B, 2, p.P + gr * p.p_stride + p.b_off + u.h, true};
         }
-#pragma unroll
-        for (int part = 0; part < 3; ++part)
-            f(RawLayer::W + part * 1024, p.cw + (((long long)part * p.H + u.h) * DK) * TAPS, 1024, false);
-        f(RawLayer::A, p.A + gr * p.a_stride + (long long)u.h * DK, 256, false);
-        f(RawLayer::GATE, p.G + gr * p.g_stride + (long long)u.h * DV, 256, false);
-        f(RawLayer::DTB, p.dt_bias + (long long)u.h * DK, 512, false);
-        f(RawLayer::B, p.P + gr * p.p_stride + p.b_off + u.h, 2, true);
     } else if constexpr (MODE == kCore) {
         const long long at = (gr * p.H + u.h) * DK;
-        f(RawCore::Q, p.q + at, 256, false);
-        f(RawCore::K, p.k + at, 256, false);
-        f(RawCore::V, p.v + at, 256, false);
-        f(RawCore::GLOG, p.glog + at, 512, false);
-        if (p.G) f(RawCore::GATE, p.G + at, 256, false);
-        f(RawCore::B, p.beta + gr * p.H + u.h, 4, true);
+        if (lane == 0) x = {RawCore::Q, 256, p.q + at, false};
+        else if (lane == 1) x = {RawCore::K, 256, p.k + at, false};
+        else if (lane == 2) x = {RawCore::V, 256, p.v + at, false};
+        else if (lane == 3) x = {RawCore::GLOG, 512, p.glog + at, false};
+        else if (lane == 4) x = {RawCore::B, 4, p.beta + gr * p.H + u.h, true};
+        else if (lane == 5 && p.G) x = {RawCore::GATE, 256, p.G + at, false};
     } else {
         const long long at = (gr * p.H + u.h) * DK;
-        f(RawReplay::K, p.k_save + u.layer * p.kv_stride + at, 512, false);
-        f(RawReplay::G, p.g_save + u.layer * p.kv_stride + at, 512, false);
-        f(RawReplay::V, p.v_save + u.layer * p.kv_stride + at, 256, false);
-        f(RawReplay::B, p.b_save + u.layer * p.b_stride + gr * p.H + u.h, 4, true);
+        if (lane == 0) x = {RawReplay::K, 512, p.k_save + u.layer * p.kv_stride + at, false};
+        else if (lane == 1) x = {RawReplay::G, 512, p.g_save + u.layer * p.kv_stride + at, false};
+        else if (lane == 2) x = {RawReplay::V, 256, p.v_save + u.layer * p.kv_stride + at, false};
+        else if (lane == 3) x = {RawReplay::B, 4, p.b_save + u.layer * p.b_stride + gr * p.H + u.h, true};
     }
+    return x;
+}
+
+template <int MODE>
+__device__ __forceinline__ uint32_t raw_row_bytes(const Params& p) {
+    return MODE == kLayer ? (3 * TAPS + 2) * 256 + 16 : MODE == kCore ? 3 * 256 + 512 + 16 + (p.G ? 256 : 0) : 2 * 512 + 256 + 16;
 }
 
 template <typename S, int MODE>
@@ -338,6 +355,7 @@ __device__ void mover_role(const Params& p, unsigned char* smem, uint64_t* bars,
     uint64_t* st_empty = st_full + L::kStateSlots;
     uint64_t* raw_full = st_empty + L::kStateSlots;
     uint64_t* raw_empty = raw_full + L::kRawSlots;
+    UnitInfo* info = reinterpret_cast<UnitInfo*>(smem + L::oUnits);
     Ring st, raw;
     const bool copy0 = copies_state(p);
     UnitIter<MODE> units(p);
@@ -347,6 +365,7 @@ __device__ void mover_role(const Params& p, unsigned char* smem, uint64_t* bars,
         if (un.rows == 0 && !copy0) continue;
         // The unit's state.
         if (!mbar_wait(&st_empty[st.idx], st.phase ^ 1u, ctx, kStatusWaitStateEmpty)) return;
+        if (lane == 0) info[st.idx] = {un.s_elem, un.rows};
         if (p.skip_first_state && blockIdx.x == 0 && first) {
             // Diagnostic launch: nothing is copied and nobody is told, so the recurrence's wait for this state runs out.
         } else {
@@ -370,35 +389,27 @@ __device__ void mover_role(const Params& p, unsigned char* smem, uint64_t* bars,
         for (int r = 0; r < un.rows; ++r) {
             if (!mbar_wait(&raw_empty[raw.idx], raw.phase ^ 1u, ctx, kStatusWaitRawEmpty)) return;
             unsigned char* dst = smem + L::oRaw + raw.idx * L::kRawBytes;
-            uintptr_t low = 0;
-            uint32_t bytes = 0;
-            for_each_piece<MODE>(p, un, r, [&](int, const void* src, int n, bool scalar) {
-                if (!scalar) low |= reinterpret_cast<uintptr_t>(src);
-                bytes += scalar ? 16 : n;
-            });
-            if ((low & 15) == 0) {
-                if (lane == 0) {
-                    mbar_arrive_expect_tx(&raw_full[raw.idx], bytes);
-                    for_each_piece<MODE>(p, un, r, [&](int off, const void* src, int n, bool scalar) {
-                        if (scalar)
-                            bulk_load(dst + off, reinterpret_cast<const void*>(reinterpret_cast<uintptr_t>(src) & ~uintptr_t(15)), 16,
-                                      &raw_full[raw.idx]);
-                        else
-                            bulk_load(dst + off, src, n, &raw_full[raw.idx]);
-                    });
-                }
-            } else {  // unaligned rows: 2-byte copies by the whole warp
-                for_each_piece<MODE>(p, un, r, [&](int off, const void* src, int n, bool scalar) {
-                    const uint16_t* s = reinterpret_cast<const uint16_t*>(src);
-                    uint16_t* d = reinterpret_cast<uint16_t*>(dst + off + (scalar ? (int)(reinterpret_cast<uintptr_t>(src) & 15) : 0));
-                    for (int e = lane; e < n / 2; e += 32) d[e] = s[e];
-                });
+            const Piece x = piece_of<MODE>(p, un, r, lane);
+            const uintptr_t src = reinterpret_cast<uintptr_t>(x.src);
+            if (!__any_sync(0xffffffffu, !x.scalar && (src & 15) != 0)) {
+                if (lane == 0) mbar_arrive_expect_tx(&raw_full[raw.idx], raw_row_bytes<MODE>(p));
+                __syncwarp();
+                if (x.bytes) bulk_load(dst + x.off, reinterpret_cast<const void*>(src & ~uintptr_t(15)), x.scalar ? 16 : x.bytes, &raw_full[raw.idx]);
+            } else {  // unaligned rows: 2-byte copies, a lane its piece
+                uint16_t* d = reinterpret_cast<uint16_t*>(dst + x.off + (x.scalar ? (int)(src & 15) : 0));
+                for (int e = 0; e < x.bytes / 2; ++e) d[e] = reinterpret_cast<const uint16_t*>(x.src)[e];
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&raw_full[raw.idx]);
             }
+            __syncwarp();
             raw.next(L::kRawSlots);
             if (lane == 0) atomicAdd(const_cast<uint32_t*>(ctx.progress), 1u);
         }
+    }
+    if (!mbar_wait(&st_empty[st.idx], st.phase ^ 1u, ctx, kStatusWaitStateEmpty)) return;
+    if (lane == 0) {
+        info[st.idx] = {0, -1};
+        mbar_arrive(&st_full[st.idx]);
     }
 }
 
@@ -435,13 +446,11 @@ __device__ void prologue_role(const Params& p, unsigned char* smem, uint64_t* ba
     Ring raw, row;
     const bool copy0 = copies_state(p);
     // Whether the role's threads meet at barriers in every row (the L2 norms go through shared scratch).
-    const bool syncs = MODE == kLayer || (MODE == kCore && (p.flags & GLM53F_KDA_CORE_L2NORM) != 0);
+    const bool syncs = MODE == kCore && (p.flags & GLM53F_KDA_CORE_L2NORM) != 0;
     UnitIter<MODE> units(p);
     while (units.valid()) {
         const Unit un = units.take(p);
         if (un.rows == 0 && !copy0) continue;
-        float decay_rate = 0.0f;
-        if constexpr (MODE == kLayer) decay_rate = expf(un.a_log);
         for (int r = 0; r < un.rows; ++r) {
             // A thread that gave up on a wait may not simply leave when the role synchronises below: the threads that got
             // through would wait for it at the role's barrier for ever.  There the decision is taken by all at that barrier.
@@ -454,33 +463,6 @@ __device__ void prologue_role(const Params& p, unsigned char* smem, uint64_t* ba
             bool normalise = true;
             if (!ready) {
                 // nothing to read: go to the vote
-            } else if constexpr (MODE == kLayer) {
-                // Short conv + SiLU, one bf16 rounding (kda.cu:129-142): channel c of q, k and v.
-                const uint16_t* x = reinterpret_cast<const uint16_t*>(in + RawLayer::X);
-                const uint16_t* w = reinterpret_cast<const uint16_t*>(in + RawLayer::W);
-                for (int c = t; c < DK; c += kProThreads) {
-#pragma unroll
-                    for (int part = 0; part < 3; ++part) {
-                        float acc = 0.0f;
-#pragma unroll
-                        for (int tap = 0; tap < TAPS; ++tap)
-                            acc = acc + bf16_bits_to_f32(w[(part * DK + c) * TAPS + tap]) * bf16_bits_to_f32(x[(tap * 3 + part) * DK + c]);
-                        const float act = bf16_round(acc / (1.0f + expf(-acc)));
-                        if (part == 0) scratch[c] = act;
-                        else if (part == 1) scratch[DK + c] = act;
-                        else ck.v[c] = act;
-                    }
-                    // Decay multiplier (kda.cu:143-146) and sigmoid of the output gate (kda.cu:199-200).
-                    const float a = bf16_bits_to_f32(reinterpret_cast<const uint16_t*>(in + RawLayer::A)[c]) +
-                                    reinterpret_cast<const float*>(in + RawLayer::DTB)[c];
-                    ck.g[c] = expf(p.lower * sigmoidf_(decay_rate * a));
-                    ck.sg[c] = sigmoidf_(bf16_bits_to_f32(reinterpret_cast<const uint16_t*>(in + RawLayer::GATE)[c]));
-                }
-                if (t == 0) {
-                    const uintptr_t addr = reinterpret_cast<uintptr_t>(p.P + gr * p.p_stride + p.b_off + un.h);
-                    const uint16_t logit = *reinterpret_cast<const uint16_t*>(in + RawLayer::B + (addr & 15));
-                    ck.beta = bf16_round(sigmoidf_(bf16_bits_to_f32(logit)));  // kda.cu:147-149
-                }
             } else if constexpr (MODE == kCore) {
                 normalise = (p.flags & GLM53F_KDA_CORE_L2NORM) != 0;
                 for (int c = t; c < DK; c += kProThreads) {
@@ -527,6 +509,159 @@ __device__ void prologue_role(const Params& p, unsigned char* smem, uint64_t* ba
     }
 }
 
+// The layer entry points' prologue.  Windows of several rows: a warp cooks a whole row (a lane four consecutive channels, so the
+// norms stay in the warp and nothing meets at a barrier), the warps take rows in turn.  A row is a chain of about 1,000
+// instructions, most of them divisions and exponentials; with all four warps on the same row a row left every 4,500 cycles and the
+// recurrence, 1,600 a row, waited (6 slots x 4 to 8 rows, f32: 37 -> 32 us a layer).
+template <typename S>
+__device__ void layer_prologue_role(const Params& p, unsigned char* smem, uint64_t* bars, const WaitCtx& ctx, int warp, int lane) {
+    using L = Smem<S, kLayer>;
+    uint64_t* raw_full = bars + 2 * L::kStateSlots;
+    uint64_t* raw_empty = raw_full + L::kRawSlots;
+    uint64_t* row_full = raw_empty + L::kRawSlots;
+    uint64_t* row_empty = row_full + 2 * L::kRowSlots;
+    Ring raw, row;
+    const bool copy0 = copies_state(p);
+    const bool vec = ((reinterpret_cast<uintptr_t>(p.cw) | reinterpret_cast<uintptr_t>(p.dt_bias)) & 15) == 0;
+    UnitIter<kLayer> units(p);
+    int turn = 0;
+    auto widen = [](uint2 w, float (&x)[4]) {
+        x[0] = __uint_as_float(w.x << 16);
+        x[1] = __uint_as_float(w.x & 0xffff0000u);
+        x[2] = __uint_as_float(w.y << 16);
+        x[3] = __uint_as_float(w.y & 0xffff0000u);
+    };
+    while (units.valid()) {
+        const Unit un = units.take(p);
+        if (un.rows == 0 && !copy0) continue;
+        if (un.rows == 1) {
+            // A single row is cooked by all four warps, a thread a channel: with one row a unit the next state is waited for anyway,
+            // and the row's latency counts (16 slots, bf16: 0.670 ms a step of 34 layers, 0.696 with a row per warp; 1 slot 0.215
+            // against 0.263).
+            const int c = warp * 32 + lane;
+            uint2 w[3];
+#pragma unroll
+            for (int part = 0; part < 3; ++part) {
+                const uint16_t* cw = p.cw + (((long long)part * p.H + un.h) * DK + c) * TAPS;
+                w[part] = vec ? *reinterpret_cast<const uint2*>(cw) : make_uint2((uint32_t)cw[0] | ((uint32_t)cw[1] << 16), (uint32_t)cw[2] | ((uint32_t)cw[3] << 16));
+            }
+            const float db = p.dt_bias[(long long)un.h * DK + c], decay_rate = expf(un.a_log);
+            const bool ready = mbar_wait(&raw_full[raw.idx], raw.phase, ctx, kStatusWaitRawFull) && mbar_wait(&row_empty[row.idx], row.phase ^ 1u, ctx, kStatusWaitRowEmpty);
+            const unsigned char* in = smem + L::oRaw + raw.idx * L::kRawBytes;
+            Cooked& ck = *reinterpret_cast<Cooked*>(smem + L::oCooked + row.idx * sizeof(Cooked));
+            float* scratch = reinterpret_cast<float*>(smem + L::oScratch);
+            if (ready) {
+                const uint16_t* x = reinterpret_cast<const uint16_t*>(in + RawLayer::X);
+#pragma unroll
+                for (int part = 0; part < 3; ++part) {
+                    float wt[TAPS], acc = 0.0f;
+                    widen(w[part], wt);
+#pragma unroll
+                    for (int tap = 0; tap < TAPS; ++tap) acc = acc + wt[tap] * bf16_bits_to_f32(x[(tap * 3 + part) * DK + c]);
+                    (part == 2 ? ck.v : scratch + part * DK)[c] = bf16_round(acc / (1.0f + expf(-acc)));
+                }
+            }
+            if (!named_bar_all(1, kProThreadsOf<kLayer>, ready)) return;  // one that gave up does not leave the others waiting
+            if (warp == 0) l2norm_warp(scratch, ck.q, lane, true);
+            else if (warp == 1) l2norm_warp(scratch + DK, ck.k, lane, false);
+            else if (warp == 2 && lane == 0) {
+                const uintptr_t addr = reinterpret_cast<uintptr_t>(p.P + un.row0 * p.p_stride + p.b_off + un.h);
+                ck.beta = bf16_round(sigmoidf_(bf16_bits_to_f32(*reinterpret_cast<const uint16_t*>(in + RawLayer::B + (addr & 15)))));
+            }
+            ck.g[c] = expf(p.lower * sigmoidf_(decay_rate * (bf16_bits_to_f32(reinterpret_cast<const uint16_t*>(in + RawLayer::A)[c]) + db)));
+            ck.sg[c] = sigmoidf_(bf16_bits_to_f32(reinterpret_cast<const uint16_t*>(in + RawLayer::GATE)[c]));
+            named_bar_sync(2, kProThreadsOf<kLayer>);
+            if (warp == 0 && lane == 0) {
+                mbar_arrive(&row_full[row.idx]);
+                mbar_arrive(&raw_empty[raw.idx]);
+            }
+            raw.next(L::kRawSlots);
+            row.next(L::kRowSlots);
+            continue;
+        }
+        for (int r = 0; r < un.rows; ++r, raw.next(L::kRawSlots), row.next(L::kRowSlots)) {
+            if ((turn++ & (kProWarpsOf<kLayer> - 1)) != warp) continue;
+            // The head's weights come straight from global memory, on their way while the row's inputs are waited for.
+            uint4 w[3][2];
+            float4 dtb;
+            {
+                const uint16_t* cw = p.cw + ((long long)un.h * DK + lane * 4) * TAPS;
+                const float* db = p.dt_bias + (long long)un.h * DK + lane * 4;
+#pragma unroll
+                for (int part = 0; part < 3; ++part, cw += (long long)p.H * DK * TAPS) {
+                    if (vec) {
+                        w[part][0] = reinterpret_cast<const uint4*>(cw)[0];
+                        w[part][1] = reinterpret_cast<const uint4*>(cw)[1];
+                    } else {
+                        auto two = [&](int e) { return (uint32_t)cw[e] | ((uint32_t)cw[e + 1] << 16); };
+                        w[part][0] = make_uint4(two(0), two(2), two(4), two(6));
+                        w[part][1] = make_uint4(two(8), two(10), two(12), two(14));
+                    }
+                }
+                dtb = vec ? *reinterpret_cast<const float4*>(db) : make_float4(db[0], db[1], db[2], db[3]);
+            }
+            if (!mbar_wait(&raw_full[raw.idx], raw.phase, ctx, kStatusWaitRawFull)) return;
+            if (!mbar_wait(&row_empty[row.idx], row.phase ^ 1u, ctx, kStatusWaitRowEmpty)) return;
+            const unsigned char* in = smem + L::oRaw + raw.idx * L::kRawBytes;
+            Cooked& ck = *reinterpret_cast<Cooked*>(smem + L::oCooked + row.idx * sizeof(Cooked));
+            // Short conv + SiLU, one bf16 rounding (kda.cu:129-142); q and k then through the L2 norm (kda.cu:151-165).
+#pragma unroll
+            for (int part = 0; part < 3; ++part) {
+                const uint32_t ww[8] = {w[part][0].x, w[part][0].y, w[part][0].z, w[part][0].w, w[part][1].x, w[part][1].y, w[part][1].z, w[part][1].w};
+                float act[4], acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+                for (int tap = 0; tap < TAPS; ++tap) {
+                    float x[4];
+                    widen(*reinterpret_cast<const uint2*>(in + RawLayer::X + (tap * 3 + part) * 256 + lane * 8), x);
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        const uint32_t t2 = ww[2 * c + (tap >> 1)];
+                        acc[c] = acc[c] + __uint_as_float(tap & 1 ? t2 & 0xffff0000u : t2 << 16) * x[c];
+                    }
+                }
+#pragma unroll
+                for (int c = 0; c < 4; ++c) act[c] = bf16_round(acc[c] / (1.0f + expf(-acc[c])));
+                if (part == 2) {
+                    *reinterpret_cast<float4*>(&ck.v[lane * 4]) = make_float4(act[0], act[1], act[2], act[3]);
+                } else {
+                    float ss = 0.0f;
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) ss = ss + act[c] * act[c];
+                    const float inv = 1.0f / sqrtf(butterfly1(ss) + 1e-6f);
+                    float y[4];
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        y[c] = act[c] * inv;
+                        if (part == 0) y[c] = y[c] * (1.0f / sqrtf((float)DK));
+                    }
+                    *reinterpret_cast<float4*>(part == 0 ? &ck.q[lane * 4] : &ck.k[lane * 4]) = make_float4(y[0], y[1], y[2], y[3]);
+                }
+            }
+            // Decay multiplier (kda.cu:143-146), sigmoid of the output gate (kda.cu:199-200) and beta (kda.cu:147-149).
+            float a[4], gt[4], d[4], sg[4];
+            widen(*reinterpret_cast<const uint2*>(in + RawLayer::A + lane * 8), a);
+            widen(*reinterpret_cast<const uint2*>(in + RawLayer::GATE + lane * 8), gt);
+            const float db[4] = {dtb.x, dtb.y, dtb.z, dtb.w}, decay_rate = expf(un.a_log);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                d[c] = expf(p.lower * sigmoidf_(decay_rate * (a[c] + db[c])));
+                sg[c] = sigmoidf_(gt[c]);
+            }
+            *reinterpret_cast<float4*>(&ck.g[lane * 4]) = make_float4(d[0], d[1], d[2], d[3]);
+            *reinterpret_cast<float4*>(&ck.sg[lane * 4]) = make_float4(sg[0], sg[1], sg[2], sg[3]);
+            if (lane == 0) {
+                const uintptr_t addr = reinterpret_cast<uintptr_t>(p.P + (un.row0 + r) * p.p_stride + p.b_off + un.h);
+                ck.beta = bf16_round(sigmoidf_(bf16_bits_to_f32(*reinterpret_cast<const uint16_t*>(in + RawLayer::B + (addr & 15)))));
+            }
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive(&row_full[row.idx]);
+                mbar_arrive(&raw_empty[raw.idx]);
+            }
+        }
+    }
+}
+
 // ---- the recurrence ------------------------------------------------------------------------------------------
 template <typename S, int MODE>
 __device__ void recurrence_role(const Params& p, unsigned char* smem, uint64_t* bars, const WaitCtx& ctx, int warp, int lane) {
@@ -537,12 +672,11 @@ __device__ void recurrence_role(const Params& p, unsigned char* smem, uint64_t* 
     uint64_t* y_full = row_full + L::kRowSlots;
     uint64_t* row_empty = y_full + L::kRowSlots;
     Ring st, row;
-    const bool copy0 = copies_state(p);
-    UnitIter<MODE> units(p);
-    while (units.valid()) {
-        const Unit un = units.take(p);
-        if (un.rows == 0 && !copy0) continue;
+    const UnitInfo* info = reinterpret_cast<const UnitInfo*>(smem + L::oUnits);
+    for (;;) {
         if (!mbar_wait(&st_full[st.idx], st.phase, ctx, kStatusWaitStateFull)) return;
+        const UnitInfo un = info[st.idx];
+        if (un.rows < 0) return;
         unsigned char* slot = smem + L::oState + st.idx * L::kStateBytes;
         f32x2 s[kPairs][4];
         load_rows<S>(slot, warp, lane, s);
@@ -670,8 +804,8 @@ __global__ void __launch_bounds__(kThreadsOf<MODE>, 1) recurrent_kernel(const __
         for (int i = 0; i < L::kStateSlots; ++i) mbar_init(b++, 1);                                // st_full
         for (int i = 0; i < L::kStateSlots; ++i) mbar_init(b++, kRecWarps);                        // st_empty
         for (int i = 0; i < L::kRawSlots; ++i) mbar_init(b++, 1);                                     // raw_full
-        for (int i = 0; i < L::kRawSlots; ++i) mbar_init(b++, kProThreads);                           // raw_empty
-        for (int i = 0; i < L::kRowSlots; ++i) mbar_init(b++, kProThreads);                           // row_full
+        for (int i = 0; i < L::kRawSlots; ++i) mbar_init(b++, MODE == kLayer ? 1 : kProThreads);         // raw_empty
+        for (int i = 0; i < L::kRowSlots; ++i) mbar_init(b++, MODE == kLayer ? 1 : kProThreads);         // row_full
         for (int i = 0; i < L::kRowSlots; ++i) mbar_init(b++, kRecWarps);                             // y_full
         for (int i = 0; i < L::kRowSlots; ++i) mbar_init(b++, MODE == kReplay ? kRecWarps : 1);       // row_empty
         ctl[0] = 0u;
@@ -688,7 +822,8 @@ __global__ void __launch_bounds__(kThreadsOf<MODE>, 1) recurrent_kernel(const __
     if (warp < kRecWarps) {
         recurrence_role<S, MODE>(p, smem, bars, ctx, warp, lane);
     } else if (warp < kRecWarps + kProWarps) {
-        prologue_role<S, MODE>(p, smem, bars, ctx, tid - kRecThreads);
+        if constexpr (MODE == kLayer) layer_prologue_role<S>(p, smem, bars, ctx, warp - kRecWarps, lane);
+        else prologue_role<S, MODE>(p, smem, bars, ctx, tid - kRecThreads);
     } else if (warp == kRecWarps + kProWarps) {
         if (MODE != kReplay) epilogue_role<S, MODE>(p, smem, bars, ctx, lane);
     } else {
