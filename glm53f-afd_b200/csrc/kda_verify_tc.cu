@@ -42,11 +42,11 @@ constexpr int WIN = 16, kVThreads = 128;
 // Shared memory map (bytes).  Tiles are boxes of R rows x 128 bytes in the 128-byte swizzle (16-byte piece p of row r at
 // piece p ^ (r & 7)), two boxes per tile (channels 0-63, 64-127).  The column-side tile Kc comes first: as the M = 128
 // operand of L^T and M^T its descriptor walks 128 rows although 16 are real, and what follows it is the state tile.
-// Once those two products are done Kc is dead, and L and M (FP32, 2.1 KB) take its place until the unit ends.
+// Once those two products are done Kc is dead, and L and M (FP32, 3 KB) take its place until the unit ends.
 constexpr int vKc = 0, vS = 4096, vKgb = vS + 32768, vQgb = vKgb + 4096, vQg = vQgb + 4096, vRaw = vQg + 4096;
 constexpr int vW = vKgb;                                                 // W replaces Kgb once L^T is done
 constexpr int vStage = vKgb;                                             // layer form: FP32 outputs [16][128] over W and Qgb
-constexpr int vL = vKc, vM = vL + WIN * 17 * 4;
+constexpr int vL = vKc, vM = vL + WIN * WIN * 8;  // L twice in a row (see substitute), M transposed
 static_assert(vM + WIN * WIN * 4 <= vS, "L and M fit the dead column-side tile");
 // Raw rows of a unit.  Core form: q, k, v bf16 (256 bytes a row), log decay f32 (512), beta.  Layer form: q fp16, v bf16,
 // k f32, the decay multiplier f32, beta.
@@ -99,20 +99,70 @@ __device__ __forceinline__ int sw_elem(int R, int r, int c) {
 // and division do (the file's other divisions and exponentials keep IEEE arithmetic for the replay saves).
 __device__ __forceinline__ float sigmoid_(float x) { return __fdividef(1.0f, 1.0f + __expf(-x)); }
 
+// (W, U) by forward substitution down the 16 rows, two-wide: x[i] = (beta_i kg_i, beta_i v_i) - sum_j L[i][j] x[j].  -L[i][j] lies
+// twice in a row at Ln[i * LN + j], so one 16-byte read feeds two of the 136 two-wide multiply-adds.
+constexpr int LN = WIN;
+__device__ __forceinline__ void substitute(const float2* Ln, const float* betas, const float (&kg)[WIN], const float (&vv)[WIN], float2 (&x)[WIN]) {
+#pragma unroll
+    for (int i = 0; i < WIN; ++i) {
+        const float bi = betas[i];
+        float2 x0 = mul2({bi, bi}, {kg[i], vv[i]}), x1 = {0.0f, 0.0f};
+#pragma unroll
+        for (int j = 0; j < i; j += 2) {
+            const float4 l = *reinterpret_cast<const float4*>(Ln + i * LN + j);
+            x0 = fma2({l.x, l.y}, x[j], x0);
+            if (j + 1 < i) x1 = fma2({l.z, l.w}, x[j + 1], x1);
+        }
+        x[i] = i > 1 ? fma2(x1, {1.0f, 1.0f}, x0) : x0;
+    }
+}
+
 struct Unit {
     int b, h, n;
     long long row0, s_elem;
 };
-__device__ __forceinline__ Unit unit_of(const VParams& p, long long u) {
-    Unit x;
-    x.b = (int)(u / p.H);
-    x.h = (int)(u % p.H);
-    const int r0 = p.cu[x.b];
-    x.row0 = r0;
-    x.n = p.cu[x.b + 1] - r0;
-    x.s_elem = p.state_off[x.b] + (long long)x.h * DV * DK;
-    return x;
-}
+// The block's units, u = blockIdx.x, blockIdx.x + gridDim.x, ...  A unit's metadata is read two units ahead and stays as loaded until
+// then: arithmetic right after the loads would wait for them behind the stores of a unit's results (1,900 cycles a unit).
+struct Units {
+    unsigned b, h, step_b, step_h;
+    long long left;  // units from the one in the registers on
+    int r0, r1;
+    long long off;
+    __device__ __forceinline__ explicit Units(const VParams& p) {
+        const unsigned H = (unsigned)p.H;
+        b = blockIdx.x / H;
+        h = blockIdx.x % H;
+        step_b = gridDim.x / H;
+        step_h = gridDim.x % H;
+        left = p.units - blockIdx.x;
+        r0 = r1 = 0;
+        off = 0;
+        fetch(p);
+    }
+    __device__ __forceinline__ void fetch(const VParams& p) {
+        if (left <= 0) return;
+        r0 = p.cu[b];
+        r1 = p.cu[b + 1];
+        off = p.state_off[b];
+    }
+    __device__ __forceinline__ bool take(const VParams& p, Unit& x) {
+        if (left <= 0) return false;
+        x.b = (int)b;
+        x.h = (int)h;
+        x.row0 = r0;
+        x.n = r1 - r0;
+        x.s_elem = off + (long long)h * DV * DK;
+        left -= gridDim.x;
+        h += step_h;
+        b += step_b;
+        if (h >= (unsigned)p.H) {
+            h -= (unsigned)p.H;
+            ++b;
+        }
+        fetch(p);
+        return true;
+    }
+};
 
 // The unit's raw rows; rows past the window's end become zero.
 template <bool LAYER>
@@ -197,7 +247,7 @@ __global__ void __launch_bounds__(kVThreads, 3) verify_tc_kernel(const __grid_co
     const uint32_t tm = *tmem_slot;
     const WaitCtx ctx{ctl, ctl + 1, p.status};
     uint32_t phase = 0;
-    float* Lf = reinterpret_cast<float*>(smem + vL);
+    float2* Ln = reinterpret_cast<float2*>(smem + vL);
     float* Mf = reinterpret_cast<float*>(smem + vM);
     float* betas = reinterpret_cast<float*>(smem + MP::vBeta);
     float nw[4] = {0.0f, 0.0f, 0.0f, 0.0f};
@@ -206,18 +256,16 @@ __global__ void __launch_bounds__(kVThreads, 3) verify_tc_kernel(const __grid_co
         for (int i = 0; i < 4; ++i) nw[i] = bf16_bits_to_f32(p.norm_w[lane * 4 + i]);
     }
 
-    long long u = blockIdx.x;
-    if (u < p.units) {
-        const Unit first = unit_of(p, u);
-        fetch_rows<LAYER>(p, smem, first, t);
-        fetch_state(p, smem, first, t);
+    Units units(p);
+    Unit un, nxt;
+    bool more = units.take(p, nxt);
+    if (more) {
+        fetch_rows<LAYER>(p, smem, nxt, t);
+        fetch_state(p, smem, nxt, t);
     }
-    for (; u < p.units; u += gridDim.x) {
-        const Unit un = unit_of(p, u);
-        const long long u_next = u + gridDim.x;
-        const bool more = u_next < p.units;
-        Unit nxt = un;
-        if (more) nxt = unit_of(p, u_next);
+    while (more) {
+        un = nxt;
+        more = units.take(p, nxt);
         if (un.n > WIN && t == 0) atomicCAS(p.status, 0, kStatusVerifyWindow);
         const int n = min(max(un.n, 0), WIN);
 
@@ -311,9 +359,12 @@ __global__ void __launch_bounds__(kVThreads, 3) verify_tc_kernel(const __grid_co
                 const int j = lane;
 #pragma unroll
                 for (int i = 0; i < WIN; ++i) {
-                    Lf[i * 17 + j] = i > j ? betas[i] * __uint_as_float(l16[i]) : 0.0f;
-                    Mf[i * WIN + j] = i >= j ? __uint_as_float(m16[i]) : 0.0f;
+                    const float l = i > j ? -betas[i] * __uint_as_float(l16[i]) : 0.0f;
+                    Ln[i * LN + j] = make_float2(l, l);
+                    if (i < j) m16[i] = 0u;
                 }
+#pragma unroll
+                for (int i = 0; i < WIN; i += 4) *reinterpret_cast<uint4*>(Mf + j * WIN + i) = make_uint4(m16[i], m16[i + 1], m16[i + 2], m16[i + 3]);
             }
         }
         tc::fence_before_sync();
@@ -323,29 +374,10 @@ __global__ void __launch_bounds__(kVThreads, 3) verify_tc_kernel(const __grid_co
         // ---- C. W = (I + L)^-1 diag(beta) Kg into its tile (thread = channel), U = (I + L)^-1 diag(beta) V in registers
         //         (thread = value channel), both by forward substitution down the 16 rows: the same multiply-adds as a product
         //         with an explicit inverse, without the inverse
-        float U[WIN];
-        {
-            float W[WIN];
+        float2 wu[WIN];
+        substitute(Ln, betas, kg, vv, wu);
 #pragma unroll
-            for (int i = 0; i < WIN; ++i) {
-                const float bi = betas[i];
-                float w0 = bi * kg[i], w1 = 0.0f, u0 = bi * vv[i], u1 = 0.0f;
-#pragma unroll
-                for (int j = 0; j < i; ++j) {
-                    const float l = Lf[i * 17 + j];
-                    if (j & 1) {
-                        w1 = fmaf(-l, W[j], w1);
-                        u1 = fmaf(-l, U[j], u1);
-                    } else {
-                        w0 = fmaf(-l, W[j], w0);
-                        u0 = fmaf(-l, U[j], u0);
-                    }
-                }
-                W[i] = w0 + w1;
-                U[i] = u0 + u1;
-                *reinterpret_cast<uint16_t*>(smem + vW + sw_elem(WIN, i, t)) = f32_to_bf16_bits(W[i]);
-            }
-        }
+        for (int i = 0; i < WIN; ++i) *reinterpret_cast<uint16_t*>(smem + vW + sw_elem(WIN, i, t)) = f32_to_bf16_bits(wu[i].x);
         cp_async_wait<1>();  // this unit's state has landed (the next unit's rows may still be on the way)
         fence_proxy_async_smem();
         tc::fence_before_sync();
@@ -378,16 +410,24 @@ __global__ void __launch_bounds__(kVThreads, 3) verify_tc_kernel(const __grid_co
             tc::tmem_ld16(tc::tmem_addr(tm, warp, 0), ws);
             tc::tmem_ld16(tc::tmem_addr(tm, warp, 16), qs);
             tc::tmem_ld_wait();
-            float D[WIN];
+            float2 o[WIN / 2];  // rows 2 p and 2 p + 1
 #pragma unroll
-            for (int j = 0; j < WIN; ++j) D[j] = U[j] - __uint_as_float(ws[j]);
+            for (int q = 0; q < WIN / 2; ++q) o[q] = {__uint_as_float(qs[2 * q]), __uint_as_float(qs[2 * q + 1])};
+#pragma unroll
+            for (int j = 0; j < WIN; ++j) {  // M's column j: rows j .. 15, zero above
+                const float d = wu[j].y - __uint_as_float(ws[j]);
+#pragma unroll
+                for (int i = j / 4 * 4; i < WIN; i += 4) {
+                    const float4 m = *reinterpret_cast<const float4*>(Mf + j * WIN + i);
+                    if (i + 1 >= j) o[i / 2] = fma2({m.x, m.y}, {d, d}, o[i / 2]);
+                    o[i / 2 + 1] = fma2({m.z, m.w}, {d, d}, o[i / 2 + 1]);
+                }
+            }
 #pragma unroll
             for (int i = 0; i < WIN; ++i) {
-                float o = __uint_as_float(qs[i]);
-#pragma unroll
-                for (int j = 0; j <= i; ++j) o = fmaf(Mf[i * WIN + j], D[j], o);
-                if constexpr (LAYER) reinterpret_cast<float*>(smem + vStage)[i * DV + t] = o;  // W and Qgb are dead
-                else if (i < n) p.out[(un.row0 + i) * p.out_stride + (long long)un.h * DV + t] = f32_to_bf16_bits(o);
+                const float x = i & 1 ? o[i / 2].y : o[i / 2].x;
+                if constexpr (LAYER) reinterpret_cast<float*>(smem + vStage)[i * DV + t] = x;  // W and Qgb are dead
+                else if (i < n) p.out[(un.row0 + i) * p.out_stride + (long long)un.h * DV + t] = f32_to_bf16_bits(x);
             }
         }
         tc::fence_before_sync();  // the next unit's products overwrite these tensor-memory columns
@@ -437,16 +477,19 @@ __global__ void __launch_bounds__(kVThreads, 3) verify_tc_kernel(const __grid_co
 // chunk's state or is copied out.  Unlike the exact replay this rounds the state to bf16 once per chunk instead of
 // after every row, and its sums run in another order: the committed state agrees with serial decode steps to the last
 // bits of bf16, not bit for bit (glm53f_kda_commit_mode).
-// Four blocks per SM (128 registers a thread, all 512 columns of tensor memory, 52.6 KB of shared memory each): the stages
-// of a unit are serial, so what overlaps one unit's waits is the other resident blocks' work.  To fit, the hi half of D^T
-// shares its 4 KB with Kc and L: Kc is read by the L^T product only, L by the forward substitution only, and D^T is written
-// after the (W S)^T product, which comes after both.
+// Three blocks per SM: the stages of a unit are serial, so what overlaps one unit's waits is the other resident blocks' work.  A
+// chunk's saved rows arrive in shared memory by asynchronous copies issued one chunk (or unit) ahead, and the unit's metadata is
+// read a unit ahead: taken straight from global memory, queued behind the state before's stores, they were 15,000 of a unit's
+// 25,800 cycles, which a fourth block (no room for the rows) did not cover. 
+// The hi half of D^T shares its 4 KB with Kc and L: Kc is read by the L^T product only, L by the forward substitution only, and
+// D^T is written after the (W S)^T product, which comes after both.
 constexpr int cS = 0, cDT = 32768, cKc = cDT, cKgb = cDT + 8192, cKdT = cKgb + 4096, cE = cKdT + 8192, cBeta = cE + 512;
-constexpr int cBar = cBeta + 64, cCtl = cBar + 16, kCSmem = cCtl + 16;
+constexpr int cBar = cBeta + 64, cCtl = cBar + 16, cRawK = cCtl + 16, cRawG = cRawK + WIN * DK * 4, cRawV = cRawG + WIN * DK * 4, kCSmem = cRawV + WIN * DV * 2;
 constexpr int cW = cKgb, cL = cKc;                    // W replaces Kgb, L replaces Kc once L^T is done
 constexpr uint32_t kCCols = 128;                      // tensor memory: L^T, then (W S)^T, then the 128 x 128 update
-constexpr int kCBlocks = 4;
-static_assert(kCBlocks * (kCSmem + 1024) <= 228 * 1024 && kCBlocks * kCCols <= 512, "four blocks per SM");
+constexpr int kCBlocks = 3;
+static_assert(kCBlocks * (kCSmem + 1024) <= 228 * 1024 && kCBlocks * kCCols <= 512, "three blocks per SM");
+static_assert(cRawK % 16 == 0 && WIN * LN * 8 <= 4096, "");
 
 struct CParams {
     int H, layers, rows1;
@@ -486,21 +529,68 @@ __global__ void __launch_bounds__(kVThreads, kCBlocks) commit_tc_kernel(const __
     const uint32_t tm = *tmem_slot;
     const WaitCtx ctx{ctl, ctl + 1, p.status};
     uint32_t phase = 0;
-    float* Lf = reinterpret_cast<float*>(smem + cL);
+    float2* Ln = reinterpret_cast<float2*>(smem + cL);
     float* En = reinterpret_cast<float*>(smem + cE);
     float* betas = reinterpret_cast<float*>(smem + cBeta);
     bool ok = true;
 
+    // A unit's place and metadata; those of the next one are read a unit ahead, as they come (arithmetic would wait for them).
+    const unsigned H = (unsigned)p.H, NL = (unsigned)p.layers;
+    unsigned h = blockIdx.x % H, layer = blockIdx.x / H % NL, b = blockIdx.x / H / NL;
+    int m_row = 0, m_keep = p.rows1;
+    long long m_off = 0;
+    auto fetch_meta = [&]() {
+        if (p.cu) m_row = p.cu[b];
+        if (p.keep) m_keep = p.keep[b];
+        if (p.state_off) m_off = p.state_off[b];
+    };
+    const bool vec_rows = ((reinterpret_cast<uintptr_t>(p.k_save) | reinterpret_cast<uintptr_t>(p.v_save) | reinterpret_cast<uintptr_t>(p.g_save)) & 15) == 0 && p.kv_stride % 8 == 0;
+    // Rows row .. row + n - 1 (n <= 16) of the saves; the places of the others keep what they hold.
+    auto fetch_saves = [&](unsigned lay, unsigned head, long long row, int n) {
+        const long long base = (long long)lay * p.kv_stride + (row * H + head) * DK;
+        if (vec_rows) {
+            for (int e = t; e < n * 32; e += kVThreads) {
+                const long long at = base + (long long)(e >> 5) * H * DK + (e & 31) * 4;
+                cp_async16(smem + cRawK + e * 16, p.k_save + at);
+                cp_async16(smem + cRawG + e * 16, p.g_save + at);
+            }
+            for (int e = t; e < n * 16; e += kVThreads) cp_async16(smem + cRawV + e * 16, p.v_save + base + (long long)(e >> 4) * H * DK + (e & 15) * 8);
+        } else {
+            for (int r = 0; r < n; ++r) {
+                const long long at = base + (long long)r * H * DK + t;
+                reinterpret_cast<float*>(smem + cRawK)[r * DK + t] = p.k_save[at];
+                reinterpret_cast<float*>(smem + cRawG)[r * DK + t] = p.g_save[at];
+                reinterpret_cast<uint16_t*>(smem + cRawV)[r * DV + t] = p.v_save[at];
+            }
+        }
+        cp_async_commit();
+    };
+    if (blockIdx.x < p.units) {
+        fetch_meta();
+        fetch_saves(layer, h, m_row, min(max(m_keep, 0), WIN));
+    }
+
     for (long long u = blockIdx.x; u < p.units && ok; u += gridDim.x) {
-        const int h = (int)(u % p.H), layer = (int)((u / p.H) % p.layers), b = (int)(u / ((long long)p.H * p.layers));
-        const long long row0 = p.cu ? p.cu[b] : 0;
-        int n = p.keep ? p.keep[b] : p.rows1;
-        if (n < 0) n = 0;
-        const long long s_elem = (long long)layer * p.state_stride + (p.state_off ? p.state_off[b] : 0) + (long long)h * DV * DK;
+        const long long row0 = m_row;
+        const int n = max(m_keep, 0);
+        const unsigned uh = h, ul = layer;
+        const long long s_elem = (long long)ul * p.state_stride + m_off + (long long)uh * DV * DK;
         const uint16_t* src = p.state_in + s_elem;
         uint16_t* dst = p.state_out + s_elem;
-        if (n == 0 && dst == src) continue;
-        const long long kv_base = (long long)layer * p.kv_stride, b_base = (long long)layer * p.b_stride;
+        const bool more = u + gridDim.x < p.units;
+        {
+            const unsigned nh = h + gridDim.x, dq = nh / H, nl = layer + dq, lq = nl / NL;
+            h = nh - dq * H;
+            layer = nl - lq * NL;
+            b += lq;
+        }
+        if (more) fetch_meta();
+        auto fetch_next = [&]() { fetch_saves(layer, h, m_row, more ? min(max(m_keep, 0), WIN) : 0); };
+        if (n == 0 && dst == src) {
+            fetch_next();
+            continue;
+        }
+        const long long b_base = (long long)ul * p.b_stride;
         __syncthreads();  // the previous unit's tile has been copied out
         // The unit's state into the swizzled tile.
         const bool vec = ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0;
@@ -514,20 +604,24 @@ __global__ void __launch_bounds__(kVThreads, kCBlocks) commit_tc_kernel(const __
             for (int e = t; e < DV * DK; e += kVThreads) *reinterpret_cast<uint16_t*>(smem + cS + sw_elem(DV, e >> 7, e & 127)) = src[e];
         }
         cp_async_commit();
+        if (n == 0) fetch_next();
 
         for (int c0 = 0; c0 < n && ok; c0 += WIN) {
             const int nr = min(WIN, n - c0);
+            const float bt = t < nr ? p.b_save[b_base + (row0 + c0 + t) * H + uh] : 0.0f;  // (t < 16 uses it)
+            if (c0 == 0) cp_async_wait<1>();  // its rows are there (the state may still be on the way)
+            else cp_async_wait<0>();
+            __syncthreads();
             // ---- A. thread = channel: the decay scan and the operand tiles; thread = value channel: v ----------------------
             float kg[WIN], vv[WIN];
             {
                 float kf[WIN], G[WIN], acc = 0.0f;
 #pragma unroll
                 for (int r = 0; r < WIN; ++r) {
-                    const long long at = kv_base + ((row0 + c0 + r) * p.H + h) * DK + t;
                     const bool live = r < nr;
-                    kf[r] = live ? p.k_save[at] : 0.0f;
-                    vv[r] = live ? bf16_bits_to_f32(p.v_save[at]) : 0.0f;
-                    acc += live ? __logf(p.g_save[at]) : 0.0f;
+                    kf[r] = live ? reinterpret_cast<const float*>(smem + cRawK)[r * DK + t] : 0.0f;
+                    vv[r] = live ? bf16_bits_to_f32(reinterpret_cast<const uint16_t*>(smem + cRawV)[r * DV + t]) : 0.0f;
+                    acc += live ? __logf(reinterpret_cast<const float*>(smem + cRawG)[r * DK + t]) : 0.0f;
                     G[r] = acc;
                 }
                 const float gm = G[WIN / 2], gl = G[WIN - 1];
@@ -535,7 +629,7 @@ __global__ void __launch_bounds__(kVThreads, kCBlocks) commit_tc_kernel(const __
                 uint32_t dh[WIN / 2], dl[WIN / 2];
 #pragma unroll
                 for (int r = 0; r < WIN; r += 2) {
-                    float hi[2], lo[2];
+                    float kd[2];
 #pragma unroll
                     for (int x = 0; x < 2; ++x) {
                         const float a = __expf(G[r + x] - gm);
@@ -543,10 +637,9 @@ __global__ void __launch_bounds__(kVThreads, kCBlocks) commit_tc_kernel(const __
                         kg[r + x] = kf[r + x] * __expf(G[r + x]);
                         *reinterpret_cast<uint16_t*>(smem + cKgb + sw_elem(WIN, r + x, t)) = f32_to_bf16_bits(kf[r + x] * a);
                         *reinterpret_cast<uint16_t*>(smem + cKc + sw_elem(WIN, r + x, t)) = f32_to_bf16_bits(kf[r + x] * __fdividef(1.0f, a));
-                        tc::split_bf16(kf[r + x] * __expf(gl - G[r + x]), hi[x], lo[x]);
+                        kd[x] = kf[r + x] * __expf(gl - G[r + x]);
                     }
-                    dh[r / 2] = tc::bf16x2(hi[0], hi[1]);
-                    dl[r / 2] = tc::bf16x2(lo[0], lo[1]);
+                    tc::split_bf16x2(kd[0], kd[1], dh[r / 2], dl[r / 2]);
                 }
                 // Kdec^T: row = key channel t, 16 row indices along K = two 16-byte cells
                 *reinterpret_cast<uint4*>(smem + cKdT + (0 * DK + t) * 16) = make_uint4(dh[0], dh[1], dh[2], dh[3]);
@@ -555,12 +648,16 @@ __global__ void __launch_bounds__(kVThreads, kCBlocks) commit_tc_kernel(const __
                 *reinterpret_cast<uint4*>(smem + cKdT + 4096 + (1 * DK + t) * 16) = make_uint4(dl[4], dl[5], dl[6], dl[7]);
                 En[t] = __expf(gl);
                 if (!(amax < 1e37f)) atomicCAS(p.status, 0, kStatusPrefillRange);
-                if (t < WIN) betas[t] = t < nr ? p.b_save[b_base + (row0 + c0 + t) * p.H + h] : 0.0f;
+                if (t < WIN) betas[t] = bt;
             }
             fence_proxy_async_smem();
             tc::fence_before_sync();
             __syncthreads();
             tc::fence_after_sync();
+
+            // The saved rows are consumed: the next chunk's, or the next unit's first, may come in.
+            if (c0 + WIN < n) fetch_saves(ul, uh, row0 + c0 + WIN, min(WIN, n - c0 - WIN));
+            else fetch_next();
 
             // ---- B. L^T ---------------------------------------------------------------------------------------------------
             if (warp == 0) {
@@ -583,7 +680,10 @@ __global__ void __launch_bounds__(kVThreads, kCBlocks) commit_tc_kernel(const __
                 tc::tmem_ld_wait();
                 if (lane < WIN) {
 #pragma unroll
-                    for (int i = 0; i < WIN; ++i) Lf[i * 17 + lane] = i > lane ? betas[i] * __uint_as_float(l16[i]) : 0.0f;
+                    for (int i = 0; i < WIN; ++i) {
+                        const float l = i > lane ? -betas[i] * __uint_as_float(l16[i]) : 0.0f;
+                        Ln[i * LN + lane] = make_float2(l, l);
+                    }
                 }
             }
             tc::fence_before_sync();
@@ -591,30 +691,11 @@ __global__ void __launch_bounds__(kVThreads, kCBlocks) commit_tc_kernel(const __
             tc::fence_after_sync();
 
             // ---- C. W and U by forward substitution ---------------------------------------------------------------------------
-            float U[WIN];
-            {
-                float W[WIN];
+            float2 wu[WIN];
+            substitute(Ln, betas, kg, vv, wu);
 #pragma unroll
-                for (int i = 0; i < WIN; ++i) {
-                    const float bi = betas[i];
-                    float w0 = bi * kg[i], w1 = 0.0f, u0 = bi * vv[i], u1 = 0.0f;
-#pragma unroll
-                    for (int j = 0; j < i; ++j) {
-                        const float l = Lf[i * 17 + j];
-                        if (j & 1) {
-                            w1 = fmaf(-l, W[j], w1);
-                            u1 = fmaf(-l, U[j], u1);
-                        } else {
-                            w0 = fmaf(-l, W[j], w0);
-                            u0 = fmaf(-l, U[j], u0);
-                        }
-                    }
-                    W[i] = w0 + w1;
-                    U[i] = u0 + u1;
-                    *reinterpret_cast<uint16_t*>(smem + cW + sw_elem(WIN, i, t)) = f32_to_bf16_bits(W[i]);  // over Kgb, which is consumed
-                }
-            }
-            cp_async_wait<0>();  // the state has landed (first chunk)
+            for (int i = 0; i < WIN; ++i) *reinterpret_cast<uint16_t*>(smem + cW + sw_elem(WIN, i, t)) = f32_to_bf16_bits(wu[i].x);  // over Kgb, which is consumed
+            cp_async_wait<1>();  // the state has landed (the next rows may still be on the way)
             fence_proxy_async_smem();
             tc::fence_before_sync();
             __syncthreads();
@@ -644,11 +725,7 @@ __global__ void __launch_bounds__(kVThreads, kCBlocks) commit_tc_kernel(const __
                 uint32_t dh[WIN / 2], dl[WIN / 2];
 #pragma unroll
                 for (int i = 0; i < WIN; i += 2) {
-                    float hi[2], lo[2];
-                    tc::split_bf16(U[i] - __uint_as_float(ws[i]), hi[0], lo[0]);
-                    tc::split_bf16(U[i + 1] - __uint_as_float(ws[i + 1]), hi[1], lo[1]);
-                    dh[i / 2] = tc::bf16x2(hi[0], hi[1]);
-                    dl[i / 2] = tc::bf16x2(lo[0], lo[1]);
+                    tc::split_bf16x2(wu[i].y - __uint_as_float(ws[i]), wu[i + 1].y - __uint_as_float(ws[i + 1]), dh[i / 2], dl[i / 2]);
                 }
                 *reinterpret_cast<uint4*>(smem + cDT + (0 * DV + t) * 16) = make_uint4(dh[0], dh[1], dh[2], dh[3]);
                 *reinterpret_cast<uint4*>(smem + cDT + (1 * DV + t) * 16) = make_uint4(dh[4], dh[5], dh[6], dh[7]);
@@ -706,7 +783,7 @@ __global__ void __launch_bounds__(kVThreads, kCBlocks) commit_tc_kernel(const __
             tc::fence_after_sync();
         }
         if (!ok) break;
-        cp_async_wait<0>();  // a unit without rows: its state is only copied
+        if (n == 0) cp_async_wait<1>();  // a unit without rows: its state is only copied
         __syncthreads();
         // ---- the tile back to global memory, coalesced ------------------------------------------------------------------------
         if (vec) {
