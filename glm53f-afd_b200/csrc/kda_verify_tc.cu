@@ -99,6 +99,33 @@ __device__ __forceinline__ int sw_elem(int R, int r, int c) {
 // and division do (the file's other divisions and exponentials keep IEEE arithmetic for the replay saves).
 __device__ __forceinline__ float sigmoid_(float x) { return __fdividef(1.0f, 1.0f + __expf(-x)); }
 
+// The operand tiles are made two channels and eight rows a thread (lanes 16-31 have rows 8-15): four-byte shared-memory accesses,
+// packed conversions.  What a lane of the other half holds:
+__device__ __forceinline__ float2 other_half(float2 x) {
+    return make_float2(__shfl_xor_sync(0xffffffffu, x.x, 16), __shfl_xor_sync(0xffffffffu, x.y, 16));
+}
+__device__ __forceinline__ float2 widen_bf16x2(uint32_t w) { return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)); }
+__device__ __forceinline__ float2 exp2f_(float2 x) { return make_float2(__expf(x.x), __expf(x.y)); }
+// The cumulative sums g of a thread's eight rows to those of the chunk; returns row 8's (Gm) and row 15's (G_last).
+__device__ __forceinline__ void join_halves(float2 (&G)[WIN / 2], bool upper, float2& gm, float2& gl) {
+    const float2 o = other_half(G[WIN / 2 - 1]);
+    if (upper)
+#pragma unroll
+        for (int r = 0; r < WIN / 2; ++r) G[r] = make_float2(G[r].x + o.x, G[r].y + o.y);
+    const float2 m = other_half(G[0]), l = other_half(G[WIN / 2 - 1]);
+    gm = upper ? G[0] : m;
+    gl = upper ? G[WIN / 2 - 1] : l;
+}
+// All 16 rows of one channel (c0 + upper) from the two halves' pairs of channels.
+__device__ __forceinline__ void all_rows(const float2 (&x)[WIN / 2], bool upper, float (&y)[WIN]) {
+#pragma unroll
+    for (int r = 0; r < WIN / 2; ++r) {
+        const float got = __shfl_xor_sync(0xffffffffu, upper ? x[r].x : x[r].y, 16);
+        y[r] = upper ? got : x[r].x;
+        y[WIN / 2 + r] = upper ? x[r].y : got;
+    }
+}
+
 // (W, U) by forward substitution down the 16 rows, two-wide: x[i] = (beta_i kg_i, beta_i v_i) - sum_j L[i][j] x[j].  -L[i][j] lies
 // twice in a row at Ln[i * LN + j], so one 16-byte read feeds two of the 136 two-wide multiply-adds.
 constexpr int LN = WIN;
@@ -164,6 +191,9 @@ struct Units {
     }
 };
 
+// Offset in the state tile of the 16-byte piece pk of row v.
+__device__ __forceinline__ int state_piece(int v, int pk) { return (pk >> 3) * 16384 + v * 128 + (((pk & 7) ^ (v & 7)) << 4); }
+
 // The unit's raw rows; rows past the window's end become zero.
 template <bool LAYER>
 __device__ __forceinline__ void fetch_rows(const VParams& p, unsigned char* smem, const Unit& un, int t) {
@@ -171,37 +201,41 @@ __device__ __forceinline__ void fetch_rows(const VParams& p, unsigned char* smem
     const int n = min(max(un.n, 0), WIN);
     unsigned char* raw = smem + vRaw;
     const uint4 z = make_uint4(0, 0, 0, 0);
-    for (int e = t; e < WIN * 16; e += kVThreads) {  // 16-byte pieces of the 256-byte rows
-        const int r = e >> 4, pc = e & 15;
-        const long long at = ((un.row0 + r) * p.H + un.h) * DK + pc * 8;
-        if (r < n) {
-            if constexpr (LAYER) {
-                cp_async16(raw + R::Q + e * 16, p.out + (un.row0 + r) * p.out_stride + (long long)un.h * DK + pc * 8);
-                cp_async16(raw + R::V + e * 16, p.v_save + at);
+    const long long rs = (long long)p.H * DK, unit = (un.row0 * p.H + un.h) * DK;
+    {  // 16-byte pieces of the 256-byte rows, eight rows a step
+        const int r0 = t >> 4, pc = t & 15;
+        const long long at = unit + r0 * rs + pc * 8;
+        const uint16_t* qs = LAYER ? p.out + (un.row0 + r0) * p.out_stride + (long long)un.h * DK + pc * 8 : p.q + at;
+        const uint16_t* vs = (LAYER ? p.v_save : p.v) + at;
+        const uint16_t* ks = p.k + at;  // core form
+#pragma unroll
+        for (int i = 0; i < WIN / 8; ++i) {
+            unsigned char* to = raw + (t + i * kVThreads) * 16;
+            if (r0 + 8 * i < n) {
+                cp_async16(to + R::Q, qs + i * 8 * (LAYER ? p.out_stride : rs));
+                if constexpr (!LAYER) cp_async16(to + R::K, ks + i * 8 * rs);
+                cp_async16(to + R::V, vs + i * 8 * rs);
             } else {
-                cp_async16(raw + R::Q + e * 16, p.q + at);
-                cp_async16(raw + R::K + e * 16, p.k + at);
-                cp_async16(raw + R::V + e * 16, p.v + at);
+                *reinterpret_cast<uint4*>(to + R::Q) = z;
+                if constexpr (!LAYER) *reinterpret_cast<uint4*>(to + R::K) = z;
+                *reinterpret_cast<uint4*>(to + R::V) = z;
             }
-        } else {
-            *reinterpret_cast<uint4*>(raw + R::Q + e * 16) = z;
-            if constexpr (!LAYER) *reinterpret_cast<uint4*>(raw + R::K + e * 16) = z;
-            *reinterpret_cast<uint4*>(raw + R::V + e * 16) = z;
         }
     }
-    for (int e = t; e < WIN * 32; e += kVThreads) {  // and of the 512-byte rows
-        const int r = e >> 5, pc = e & 31;
-        const long long at = ((un.row0 + r) * p.H + un.h) * DK + pc * 4;
-        if (r < n) {
-            if constexpr (LAYER) {
-                cp_async16(raw + R::K + e * 16, p.k_save + at);
-                cp_async16(raw + R::G + e * 16, p.g_save + at);
+    {  // and of the 512-byte rows, four a step
+        const int r0 = t >> 5;
+        const long long at = unit + r0 * rs + (t & 31) * 4;
+        const float *gs = (LAYER ? p.g_save : p.g) + at, *ks = p.k_save + at;
+#pragma unroll
+        for (int i = 0; i < WIN / 4; ++i) {
+            unsigned char* to = raw + (t + i * kVThreads) * 16;
+            if (r0 + 4 * i < n) {
+                cp_async16(to + R::G, gs + i * 4 * rs);
+                if constexpr (LAYER) cp_async16(to + R::K, ks + i * 4 * rs);
             } else {
-                cp_async16(raw + R::G + e * 16, p.g + at);
+                *reinterpret_cast<uint4*>(to + R::G) = z;
+                if constexpr (LAYER) *reinterpret_cast<uint4*>(to + R::K) = z;
             }
-        } else {
-            if constexpr (LAYER) *reinterpret_cast<uint4*>(raw + R::K + e * 16) = z;
-            *reinterpret_cast<uint4*>(raw + R::G + e * 16) = z;
         }
     }
     if (t < WIN) {
@@ -214,11 +248,10 @@ __device__ __forceinline__ void fetch_rows(const VParams& p, unsigned char* smem
 __device__ __forceinline__ void fetch_state(const VParams& p, unsigned char* smem, const Unit& un, int t) {
     const uint16_t* src = p.state + un.s_elem;
     if ((reinterpret_cast<uintptr_t>(src) & 15) == 0) {
+        unsigned char* to = smem + vS + state_piece(t >> 4, t & 15);  // eight rows a step: the swizzle stays
+        src += t * 8;
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            const int e = t + i * kVThreads, v = e >> 4, pk = e & 15;
-            cp_async16(smem + vS + (pk >> 3) * 16384 + v * 128 + (((pk & 7) ^ (v & 7)) << 4), src + (long long)e * 8);
-        }
+        for (int i = 0; i < 16; ++i) cp_async16(to + i * 1024, src + i * kVThreads * 8);
     } else {  // a state that is not 16-byte aligned: element by element
         for (int e = t; e < DV * DK; e += kVThreads) *reinterpret_cast<uint16_t*>(smem + vS + sw_elem(DV, e >> 7, e & 127)) = src[e];
     }
@@ -256,6 +289,7 @@ __global__ void __launch_bounds__(kVThreads, 3) verify_tc_kernel(const __grid_co
         for (int i = 0; i < 4; ++i) nw[i] = bf16_bits_to_f32(p.norm_w[lane * 4 + i]);
     }
 
+    const bool pair_saves = ((reinterpret_cast<uintptr_t>(p.k_save) | reinterpret_cast<uintptr_t>(p.g_save)) & 7) == 0 && (reinterpret_cast<uintptr_t>(p.v_save) & 3) == 0;
     Units units(p);
     Unit un, nxt;
     bool more = units.take(p, nxt);
@@ -272,49 +306,69 @@ __global__ void __launch_bounds__(kVThreads, 3) verify_tc_kernel(const __grid_co
         cp_async_wait<1>();  // this unit's rows have landed (its state may still be on the way)
         __syncthreads();     // and every thread is done with the previous unit's L, M and staged outputs
 
-        // ---- A. thread = channel c: the decay scan, the operand tiles, the replay saves ----------------------------------
-        float kg[WIN], vv[WIN], qe[WIN];
+        // ---- A. the decay scan, the operand tiles, the replay saves: channels c0 and c0 + 1, rows rb .. rb + 7 ---------------
+        float kg[WIN], vv[WIN];
+        float2 qe[WIN / 2];
+        const bool upper = lane >= 16;
+        const int c0 = warp * 32 + (lane & 15) * 2, rb = upper ? WIN / 2 : 0;
         {
-            const int c = t;
             const unsigned char* raw = smem + vRaw;
-            float G[WIN], acc = 0.0f;
+            float2 G[WIN / 2], acc = {0.0f, 0.0f}, gm, gl;
 #pragma unroll
-            for (int r = 0; r < WIN; ++r) {
-                const float x = reinterpret_cast<const float*>(raw + R::G)[r * DK + c];
+            for (int r = 0; r < WIN / 2; ++r) {
+                float2 x = *reinterpret_cast<const float2*>(raw + R::G + ((rb + r) * DK + c0) * 4);
                 // layer form: the saved multiplier exp(log decay) in (0, 1]; the rows past the window decay by nothing
-                acc += LAYER ? (r < n ? __logf(x) : 0.0f) : x;
+                if constexpr (LAYER) x = rb + r < n ? make_float2(__logf(x.x), __logf(x.y)) : make_float2(0.0f, 0.0f);
+                acc = make_float2(acc.x + x.x, acc.y + x.y);
                 G[r] = acc;
             }
-            const float gm = G[WIN / 2];
+            join_halves(G, upper, gm, gl);
             float amax = 0.0f;
+            float2 kgp[WIN / 2];
 #pragma unroll
-            for (int r = 0; r < WIN; ++r) {
-                float kf, qf;
+            for (int r = 0; r < WIN / 2; ++r) {
+                const int row = rb + r, at2 = (row * DK + c0) * 2;
+                float2 kf, qf;
+                const uint32_t qw = *reinterpret_cast<const uint32_t*>(raw + R::Q + at2);
                 if constexpr (LAYER) {
-                    kf = reinterpret_cast<const float*>(raw + R::K)[r * DK + c];
-                    qf = __half2float(reinterpret_cast<const __half*>(raw + R::Q)[r * DK + c]);
+                    kf = *reinterpret_cast<const float2*>(raw + R::K + at2 * 2);
+                    qf = __half22float2(*reinterpret_cast<const __half2*>(&qw));
                 } else {
-                    kf = bf16_bits_to_f32(reinterpret_cast<const uint16_t*>(raw + R::K)[r * DK + c]);
-                    qf = bf16_bits_to_f32(reinterpret_cast<const uint16_t*>(raw + R::Q)[r * DK + c]);
+                    kf = widen_bf16x2(*reinterpret_cast<const uint32_t*>(raw + R::K + at2));
+                    qf = widen_bf16x2(qw);
                 }
-                const uint16_t vb = reinterpret_cast<const uint16_t*>(raw + R::V)[r * DK + c];
-                const float a = __expf(G[r] - gm), e = __expf(G[r]);
-                amax = fmaxf(amax, a);
-                kg[r] = kf * e;
-                vv[r] = bf16_bits_to_f32(vb);
-                *reinterpret_cast<uint16_t*>(smem + vKgb + sw_elem(WIN, r, c)) = f32_to_bf16_bits(kf * a);
-                *reinterpret_cast<uint16_t*>(smem + vQgb + sw_elem(WIN, r, c)) = f32_to_bf16_bits(qf * a);
-                *reinterpret_cast<uint16_t*>(smem + vKc + sw_elem(WIN, r, c)) = f32_to_bf16_bits(kf * __fdividef(1.0f, a));
-                qe[r] = qf * e;  // the Qg tile is written while the first products run
+                const float2 a = exp2f_({G[r].x - gm.x, G[r].y - gm.y}), e = exp2f_(G[r]);
+                amax = fmaxf(amax, fmaxf(a.x, a.y));
+                kgp[r] = mul2(kf, e);
+                qe[r] = mul2(qf, e);  // the Qg tile is written while the first products run
+                const float2 kb = mul2(kf, a), qb = mul2(qf, a), kc = mul2(kf, {__fdividef(1.0f, a.x), __fdividef(1.0f, a.y)});
+                const int to = sw_elem(WIN, row, c0);
+                *reinterpret_cast<uint32_t*>(smem + vKgb + to) = tc::bf16x2(kb.x, kb.y);
+                *reinterpret_cast<uint32_t*>(smem + vQgb + to) = tc::bf16x2(qb.x, qb.y);
+                *reinterpret_cast<uint32_t*>(smem + vKc + to) = tc::bf16x2(kc.x, kc.y);
                 if constexpr (!LAYER) {
-                    if (r < n && p.k_save != nullptr) {
-                        const long long at = ((un.row0 + r) * p.H + un.h) * DK + c;
-                        p.k_save[at] = kf;
-                        p.v_save[at] = vb;
-                        p.g_save[at] = expf(reinterpret_cast<const float*>(raw + R::G)[r * DK + c]);
+                    if (row < n && p.k_save != nullptr) {
+                        const long long at = ((un.row0 + row) * p.H + un.h) * DK + c0;
+                        const float2 gx = *reinterpret_cast<const float2*>(raw + R::G + at2 * 2);
+                        const uint32_t vw = *reinterpret_cast<const uint32_t*>(raw + R::V + at2);
+                        if (pair_saves) {
+                            *reinterpret_cast<float2*>(p.k_save + at) = kf;
+                            *reinterpret_cast<uint32_t*>(p.v_save + at) = vw;
+                            *reinterpret_cast<float2*>(p.g_save + at) = make_float2(expf(gx.x), expf(gx.y));
+                        } else {
+                            p.k_save[at] = kf.x;
+                            p.k_save[at + 1] = kf.y;
+                            p.v_save[at] = (uint16_t)vw;
+                            p.v_save[at + 1] = (uint16_t)(vw >> 16);
+                            p.g_save[at] = expf(gx.x);
+                            p.g_save[at + 1] = expf(gx.y);
+                        }
                     }
                 }
             }
+            all_rows(kgp, upper, kg);
+#pragma unroll
+            for (int r = 0; r < WIN; ++r) vv[r] = bf16_bits_to_f32(reinterpret_cast<const uint16_t*>(raw + R::V)[r * DK + t]);
             if (!(amax < 1e37f)) atomicCAS(p.status, 0, kStatusPrefillRange);
             if (t < WIN) {
                 const float bt = reinterpret_cast<const float*>(raw + R::B)[t];
@@ -345,7 +399,7 @@ __global__ void __launch_bounds__(kVThreads, 3) verify_tc_kernel(const __grid_co
             __syncwarp();
         }
 #pragma unroll
-        for (int r = 0; r < WIN; ++r) *reinterpret_cast<uint16_t*>(smem + vQg + sw_elem(WIN, r, t)) = f32_to_bf16_bits(qe[r]);
+        for (int r = 0; r < WIN / 2; ++r) *reinterpret_cast<uint32_t*>(smem + vQg + sw_elem(WIN, rb + r, c0)) = tc::bf16x2(qe[r].x, qe[r].y);
         bool ok = mbar_wait(bar, phase, ctx, kStatusWaitPrefill);
         phase ^= 1u;
         if (!__syncthreads_and(ok)) break;
@@ -371,13 +425,13 @@ __global__ void __launch_bounds__(kVThreads, 3) verify_tc_kernel(const __grid_co
         __syncthreads();
         tc::fence_after_sync();
 
-        // ---- C. W = (I + L)^-1 diag(beta) Kg into its tile (thread = channel), U = (I + L)^-1 diag(beta) V in registers
+        // ---- C. W = (I + L)^-1 diag(beta) Kg into its tile (thread = channel c0 + upper), U = (I + L)^-1 diag(beta) V in registers
         //         (thread = value channel), both by forward substitution down the 16 rows: the same multiply-adds as a product
         //         with an explicit inverse, without the inverse
         float2 wu[WIN];
         substitute(Ln, betas, kg, vv, wu);
 #pragma unroll
-        for (int i = 0; i < WIN; ++i) *reinterpret_cast<uint16_t*>(smem + vW + sw_elem(WIN, i, t)) = f32_to_bf16_bits(wu[i].x);
+        for (int i = 0; i < WIN; ++i) *reinterpret_cast<uint16_t*>(smem + vW + sw_elem(WIN, i, c0 + upper)) = f32_to_bf16_bits(wu[i].x);
         cp_async_wait<1>();  // this unit's state has landed (the next unit's rows may still be on the way)
         fence_proxy_async_smem();
         tc::fence_before_sync();
@@ -508,7 +562,7 @@ struct CParams {
     int* status;
 };
 
-__device__ __forceinline__ int state_piece(int v, int pk) { return cS + (pk >> 3) * 16384 + v * 128 + (((pk & 7) ^ (v & 7)) << 4); }
+static_assert(cS == 0, "state_piece() is the place in the tile");
 
 __global__ void __launch_bounds__(kVThreads, kCBlocks) commit_tc_kernel(const __grid_constant__ CParams p) {
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -549,12 +603,17 @@ __global__ void __launch_bounds__(kVThreads, kCBlocks) commit_tc_kernel(const __
     auto fetch_saves = [&](unsigned lay, unsigned head, long long row, int n) {
         const long long base = (long long)lay * p.kv_stride + (row * H + head) * DK;
         if (vec_rows) {
-            for (int e = t; e < n * 32; e += kVThreads) {
-                const long long at = base + (long long)(e >> 5) * H * DK + (e & 31) * 4;
-                cp_async16(smem + cRawK + e * 16, p.k_save + at);
-                cp_async16(smem + cRawG + e * 16, p.g_save + at);
-            }
-            for (int e = t; e < n * 16; e += kVThreads) cp_async16(smem + cRawV + e * 16, p.v_save + base + (long long)(e >> 4) * H * DK + (e & 15) * 8);
+            const long long rs = (long long)H * DK, at = base + (t >> 5) * rs + (t & 31) * 4;  // four rows a step
+#pragma unroll
+            for (int i = 0; i < WIN / 4; ++i)
+                if ((t >> 5) + 4 * i < n) {
+                    cp_async16(smem + cRawK + (t + i * kVThreads) * 16, p.k_save + at + i * 4 * rs);
+                    cp_async16(smem + cRawG + (t + i * kVThreads) * 16, p.g_save + at + i * 4 * rs);
+                }
+            const uint16_t* vs = p.v_save + base + (t >> 4) * rs + (t & 15) * 8;  // eight
+#pragma unroll
+            for (int i = 0; i < WIN / 8; ++i)
+                if ((t >> 4) + 8 * i < n) cp_async16(smem + cRawV + (t + i * kVThreads) * 16, vs + i * 8 * rs);
         } else {
             for (int r = 0; r < n; ++r) {
                 const long long at = base + (long long)r * H * DK + t;
@@ -595,11 +654,9 @@ __global__ void __launch_bounds__(kVThreads, kCBlocks) commit_tc_kernel(const __
         // The unit's state into the swizzled tile.
         const bool vec = ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0;
         if (vec) {
+            unsigned char* to = smem + state_piece(t >> 4, t & 15);
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                const int e = t + i * kVThreads;
-                cp_async16(smem + state_piece(e >> 4, e & 15), src + (long long)e * 8);
-            }
+            for (int i = 0; i < 16; ++i) cp_async16(to + i * 1024, src + (t + i * kVThreads) * 8);
         } else {
             for (int e = t; e < DV * DK; e += kVThreads) *reinterpret_cast<uint16_t*>(smem + cS + sw_elem(DV, e >> 7, e & 127)) = src[e];
         }
@@ -612,41 +669,54 @@ __global__ void __launch_bounds__(kVThreads, kCBlocks) commit_tc_kernel(const __
             if (c0 == 0) cp_async_wait<1>();  // its rows are there (the state may still be on the way)
             else cp_async_wait<0>();
             __syncthreads();
-            // ---- A. thread = channel: the decay scan and the operand tiles; thread = value channel: v ----------------------
+            // ---- A. the decay scan and the operand tiles: channels ch0 and ch0 + 1, rows rb .. rb + 7; thread = value channel: v ------
             float kg[WIN], vv[WIN];
+            const bool upper = lane >= 16;
+            const int ch0 = warp * 32 + (lane & 15) * 2, rb = upper ? WIN / 2 : 0;
             {
-                float kf[WIN], G[WIN], acc = 0.0f;
+                float2 kf[WIN / 2], G[WIN / 2], acc = {0.0f, 0.0f}, gm, gl;
 #pragma unroll
-                for (int r = 0; r < WIN; ++r) {
-                    const bool live = r < nr;
-                    kf[r] = live ? reinterpret_cast<const float*>(smem + cRawK)[r * DK + t] : 0.0f;
-                    vv[r] = live ? bf16_bits_to_f32(reinterpret_cast<const uint16_t*>(smem + cRawV)[r * DV + t]) : 0.0f;
-                    acc += live ? __logf(reinterpret_cast<const float*>(smem + cRawG)[r * DK + t]) : 0.0f;
+                for (int r = 0; r < WIN / 2; ++r) {
+                    kf[r] = make_float2(0.0f, 0.0f);
+                    if (rb + r < nr) {
+                        kf[r] = *reinterpret_cast<const float2*>(smem + cRawK + ((rb + r) * DK + ch0) * 4);
+                        const float2 x = *reinterpret_cast<const float2*>(smem + cRawG + ((rb + r) * DK + ch0) * 4);
+                        acc = make_float2(acc.x + __logf(x.x), acc.y + __logf(x.y));
+                    }
                     G[r] = acc;
                 }
-                const float gm = G[WIN / 2], gl = G[WIN - 1];
+                join_halves(G, upper, gm, gl);
                 float amax = 0.0f;
-                uint32_t dh[WIN / 2], dl[WIN / 2];
+                float2 kgp[WIN / 2];
+                uint32_t dh[2][WIN / 4], dl[2][WIN / 4];
 #pragma unroll
-                for (int r = 0; r < WIN; r += 2) {
-                    float kd[2];
+                for (int r = 0; r < WIN / 2; r += 2) {
+                    float2 kd[2];
 #pragma unroll
                     for (int x = 0; x < 2; ++x) {
-                        const float a = __expf(G[r + x] - gm);
-                        amax = fmaxf(amax, a);
-                        kg[r + x] = kf[r + x] * __expf(G[r + x]);
-                        *reinterpret_cast<uint16_t*>(smem + cKgb + sw_elem(WIN, r + x, t)) = f32_to_bf16_bits(kf[r + x] * a);
-                        *reinterpret_cast<uint16_t*>(smem + cKc + sw_elem(WIN, r + x, t)) = f32_to_bf16_bits(kf[r + x] * __fdividef(1.0f, a));
-                        kd[x] = kf[r + x] * __expf(gl - G[r + x]);
+                        const float2 a = exp2f_({G[r + x].x - gm.x, G[r + x].y - gm.y});
+                        amax = fmaxf(amax, fmaxf(a.x, a.y));
+                        kgp[r + x] = mul2(kf[r + x], exp2f_(G[r + x]));
+                        kd[x] = mul2(kf[r + x], exp2f_({gl.x - G[r + x].x, gl.y - G[r + x].y}));
+                        const float2 kb = mul2(kf[r + x], a), kc = mul2(kf[r + x], {__fdividef(1.0f, a.x), __fdividef(1.0f, a.y)});
+                        const int to = sw_elem(WIN, rb + r + x, ch0);
+                        *reinterpret_cast<uint32_t*>(smem + cKgb + to) = tc::bf16x2(kb.x, kb.y);
+                        *reinterpret_cast<uint32_t*>(smem + cKc + to) = tc::bf16x2(kc.x, kc.y);
                     }
-                    tc::split_bf16x2(kd[0], kd[1], dh[r / 2], dl[r / 2]);
+                    tc::split_bf16x2(kd[0].x, kd[1].x, dh[0][r / 2], dl[0][r / 2]);
+                    tc::split_bf16x2(kd[0].y, kd[1].y, dh[1][r / 2], dl[1][r / 2]);
                 }
-                // Kdec^T: row = key channel t, 16 row indices along K = two 16-byte cells
-                *reinterpret_cast<uint4*>(smem + cKdT + (0 * DK + t) * 16) = make_uint4(dh[0], dh[1], dh[2], dh[3]);
-                *reinterpret_cast<uint4*>(smem + cKdT + (1 * DK + t) * 16) = make_uint4(dh[4], dh[5], dh[6], dh[7]);
-                *reinterpret_cast<uint4*>(smem + cKdT + 4096 + (0 * DK + t) * 16) = make_uint4(dl[0], dl[1], dl[2], dl[3]);
-                *reinterpret_cast<uint4*>(smem + cKdT + 4096 + (1 * DK + t) * 16) = make_uint4(dl[4], dl[5], dl[6], dl[7]);
-                En[t] = __expf(gl);
+                // Kdec^T: row = key channel, 16 row indices along K = two 16-byte cells, of which this thread has one
+#pragma unroll
+                for (int x = 0; x < 2; ++x) {
+                    unsigned char* to = smem + cKdT + ((upper ? DK : 0) + ch0 + x) * 16;
+                    *reinterpret_cast<uint4*>(to) = make_uint4(dh[x][0], dh[x][1], dh[x][2], dh[x][3]);
+                    *reinterpret_cast<uint4*>(to + 4096) = make_uint4(dl[x][0], dl[x][1], dl[x][2], dl[x][3]);
+                }
+                if (!upper) *reinterpret_cast<float2*>(&En[ch0]) = exp2f_(gl);
+                all_rows(kgp, upper, kg);
+#pragma unroll
+                for (int r = 0; r < WIN; ++r) vv[r] = r < nr ? bf16_bits_to_f32(reinterpret_cast<const uint16_t*>(smem + cRawV)[r * DV + t]) : 0.0f;
                 if (!(amax < 1e37f)) atomicCAS(p.status, 0, kStatusPrefillRange);
                 if (t < WIN) betas[t] = bt;
             }
@@ -694,7 +764,7 @@ __global__ void __launch_bounds__(kVThreads, kCBlocks) commit_tc_kernel(const __
             float2 wu[WIN];
             substitute(Ln, betas, kg, vv, wu);
 #pragma unroll
-            for (int i = 0; i < WIN; ++i) *reinterpret_cast<uint16_t*>(smem + cW + sw_elem(WIN, i, t)) = f32_to_bf16_bits(wu[i].x);  // over Kgb, which is consumed
+            for (int i = 0; i < WIN; ++i) *reinterpret_cast<uint16_t*>(smem + cW + sw_elem(WIN, i, ch0 + upper)) = f32_to_bf16_bits(wu[i].x);  // over Kgb, which is consumed
             cp_async_wait<1>();  // the state has landed (the next rows may still be on the way)
             fence_proxy_async_smem();
             tc::fence_before_sync();
@@ -767,12 +837,13 @@ __global__ void __launch_bounds__(kVThreads, kCBlocks) commit_tc_kernel(const __
                     const uint32_t sw[4] = {sv.x, sv.y, sv.z, sv.w};
                     uint32_t out[4];
 #pragma unroll
-                    for (int x = 0; x < 4; ++x) {
-                        const int k = cg * 32 + half * 8 + 2 * x;
-                        const float2 e2 = *reinterpret_cast<const float2*>(&En[k]);
-                        const float lo = fmaf(e2.x, __uint_as_float(sw[x] << 16), __uint_as_float(a16[half * 8 + 2 * x]));
-                        const float hi = fmaf(e2.y, __uint_as_float(sw[x] & 0xffff0000u), __uint_as_float(a16[half * 8 + 2 * x + 1]));
-                        out[x] = tc::bf16x2(lo, hi);
+                    for (int x = 0; x < 4; x += 2) {
+                        const float4 e4 = *reinterpret_cast<const float4*>(&En[cg * 32 + half * 8 + 2 * x]);
+                        const uint32_t* a4 = a16 + half * 8 + 2 * x;
+                        const float2 s0 = fma2({e4.x, e4.y}, widen_bf16x2(sw[x]), {__uint_as_float(a4[0]), __uint_as_float(a4[1])});
+                        const float2 s1 = fma2({e4.z, e4.w}, widen_bf16x2(sw[x + 1]), {__uint_as_float(a4[2]), __uint_as_float(a4[3])});
+                        out[x] = tc::bf16x2(s0.x, s0.y);
+                        out[x + 1] = tc::bf16x2(s1.x, s1.y);
                     }
                     *reinterpret_cast<uint4*>(at) = make_uint4(out[0], out[1], out[2], out[3]);
                 }
@@ -787,11 +858,9 @@ __global__ void __launch_bounds__(kVThreads, kCBlocks) commit_tc_kernel(const __
         __syncthreads();
         // ---- the tile back to global memory, coalesced ------------------------------------------------------------------------
         if (vec) {
+            const unsigned char* from = smem + state_piece(t >> 4, t & 15);
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                const int e = t + i * kVThreads;
-                *reinterpret_cast<uint4*>(dst + (long long)e * 8) = *reinterpret_cast<const uint4*>(smem + state_piece(e >> 4, e & 15));
-            }
+            for (int i = 0; i < 16; ++i) *reinterpret_cast<uint4*>(dst + (t + i * kVThreads) * 8) = *reinterpret_cast<const uint4*>(from + i * 1024);
         } else {
             for (int e = t; e < DV * DK; e += kVThreads) dst[e] = *reinterpret_cast<const uint16_t*>(smem + cS + sw_elem(DV, e >> 7, e & 127));
         }
