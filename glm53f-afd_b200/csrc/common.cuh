@@ -212,4 +212,25 @@ __device__ __forceinline__ float ex2_approx(float x) {
 }
 constexpr float kLog2e = 1.4426950408889634f;
 
+// A launch that may begin while its predecessor in the stream drains; the kernel calls grid_ready() before its first access to
+// global memory, so the order of effects is a plain launch's.
+template <typename P>
+inline int launch_early(void (*kernel)(P), unsigned grid, unsigned threads, size_t smem, cudaStream_t stream, const P& p) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return (int)cudaLaunchKernelEx(&cfg, kernel, p);
+}
+__device__ __forceinline__ void grid_ready() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 }  // namespace kda

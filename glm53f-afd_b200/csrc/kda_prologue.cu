@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(128, 6) layer_prologue_kernel(const ProParams 
 // ---- the prefill sink ---------------------------------------------------------------------------------------------------
 // Bound by instruction issue before it is bound by memory (a row and head: 1 KiB in, 1.3 KiB out).  A warp takes four consecutive
 // rows: seven rows of inputs instead of sixteen, the weights once, and everything in pairs of channels (two-wide multiply-adds).
-// 1,280 rows x 64 heads: 79 us with a warp per row as in the kernel above, 52 so.
+// 1,280 rows x 64 heads: 79 us with a warp per row as in the kernel above, 52 so with four blocks an SM; five take another 4 us off a pass of the whole call.
 constexpr int kRowsPer = 4;
 __device__ __forceinline__ float2 lo_hi(uint32_t w) { return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)); }
 __device__ __forceinline__ float2 add2(float2 a, float2 b) { return fma2(a, {1.0f, 1.0f}, b); }
@@ -219,7 +219,7 @@ __device__ __forceinline__ uint32_t fp16x2(float2 x) {
     return *reinterpret_cast<const uint32_t*>(&h);
 }
 
-__global__ void __launch_bounds__(128, 4) prefill_prologue_kernel(const ProParams p) {
+__global__ void __launch_bounds__(128, 5) prefill_prologue_kernel(const ProParams p) {
     const int lane = threadIdx.x & 31, H = p.H, groups = p.pass_rows / (4 * kRowsPer), c0 = lane * 4;
     // heads innermost: neighbouring blocks read neighbouring pieces of the same rows
     const int h = (int)(blockIdx.x % H), b = (int)(blockIdx.x / H / groups), j0 = (int)(blockIdx.x / H % groups) * 4 * kRowsPer + (threadIdx.x >> 5) * kRowsPer;

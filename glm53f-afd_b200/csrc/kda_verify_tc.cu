@@ -278,6 +278,7 @@ __global__ void __launch_bounds__(kVThreads, 3) verify_tc_kernel(const __grid_co
     __syncthreads();
     tc::fence_after_sync();
     const uint32_t tm = *tmem_slot;
+    grid_ready();
     const WaitCtx ctx{ctl, ctl + 1, p.status};
     uint32_t phase = 0;
     float2* Ln = reinterpret_cast<float2*>(smem + vL);
@@ -581,6 +582,7 @@ __global__ void __launch_bounds__(kVThreads, kCBlocks) commit_tc_kernel(const __
     __syncthreads();
     tc::fence_after_sync();
     const uint32_t tm = *tmem_slot;
+    grid_ready();
     const WaitCtx ctx{ctl, ctl + 1, p.status};
     uint32_t phase = 0;
     float2* Ln = reinterpret_cast<float2*>(smem + cL);
@@ -883,8 +885,7 @@ int launch_verify(const VParams& p, cudaStream_t stream) {
     }
     if (p.status == nullptr) return (int)cudaErrorUnknown;
     const long long cap = 3LL * sm_count();
-    verify_tc_kernel<LAYER><<<(unsigned)(p.units < cap ? p.units : cap), kVThreads, Map<LAYER>::kSmem, stream>>>(p);
-    return (int)cudaGetLastError();
+    return launch_early(verify_tc_kernel<LAYER>, (unsigned)(p.units < cap ? p.units : cap), kVThreads, Map<LAYER>::kSmem, stream, p);
 }
 
 }  // namespace
@@ -952,8 +953,7 @@ int commit_tc_launch(int32_t heads, int32_t layers, int32_t batch, const int32_t
     p.status = status_word();
     if (p.status == nullptr) return (int)cudaErrorUnknown;
     const long long cap = (long long)kCBlocks * sm_count();
-    commit_tc_kernel<<<(unsigned)(p.units < cap ? p.units : cap), kVThreads, kCSmem, stream>>>(p);
-    return (int)cudaGetLastError();
+    return launch_early(commit_tc_kernel, (unsigned)(p.units < cap ? p.units : cap), kVThreads, kCSmem, stream, p);
 }
 
 }  // namespace kda
