@@ -21,11 +21,8 @@
 // the final state is within 5e-4 rel-L2 of the FP32 recurrence (limit 1e-3) and the bf16 outputs within 4e-3
 // (limit 5e-3).
 //
-// Every exponent the scheme evaluates stays representable only while a chunk's cumulative log decay stays above
-// about -80 per channel (1/E is formed explicitly).  The benchmark's gates (log sigmoid(N(3,1)), about -4.5 per
-// chunk) are far inside that range; the model's gate bound of -5 per row is not, so the layer entry points
-// (glm53f_kda_prefill*) keep the exact row-by-row path, and this kernel records kStatusPrefillRange when a chunk
-// leaves the range.
+// The decay factors are split at reference rows as in kda_prefill_sp.cu ("Decay range" there): one reference for a chunk with
+// mild gates, one per 16 rows otherwise; kStatusPrefillRange records a chunk that leaves even that range.
 //
 // Raw inputs arrive by bulk asynchronous copies (one per row and tensor) into padded row-major staging buffers;
 // operands are written in the un-swizzled "cell" layout of tc.cuh.  All waits are bounded.

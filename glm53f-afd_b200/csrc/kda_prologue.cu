@@ -10,16 +10,16 @@
 // hardware's approximate division, exponential and reciprocal root, four rows a warp, and multiply-adds.)
 //
 // A lane owns four consecutive channels, so the norms need no shared memory.  With the chain's arithmetic (verify and exact
-// sinks): one warp per (request, head, row).  The work is bound by instruction issue (about 850 instructions per row and lane, most of them IEEE divisions and
-// exponentials), so a warp takes ONE row and reads its three predecessors again (the four warps of a block take four
+// sinks): one warp per (request, head, row).  The work is bound by instruction issue (about 850 instructions per row and lane,
+// most of them IEEE divisions and exponentials), so a warp takes ONE row and reads its three predecessors again (the four warps of a block take four
 // consecutive rows; the predecessors come from L1/L2): every load of a warp is in flight at once and 79 registers
 // allow 24 resident warps per SM.  (A warp that walks 16 rows with the three earlier rows sliding in registers needs
 // 143 registers and was half as fast.)
 //
 // Three sinks:
 //  * a prefill pass: core inputs for one pass of chunks, in the caller's workspace as the slots of kda_prefill_sp.cu take
-//    them (a chunk's rows together, already in the swizzle that one bulk copy brings to the tensor core).  q and k are rounded to fp16
-//    (they lie in [-1, 1]; eleven mantissa bits), the one place where the chunked prefill departs from the chain's
+//    them (a chunk's rows together, already in the swizzle that one bulk copy brings to the tensor core).  q and k are rounded
+//    to fp16 (they lie in [-1, 1]; eleven mantissa bits), the one place where the chunked prefill departs from the chain's
 //    FP32 q and k before the tensor-core products: with bf16's eight bits the rounding of k alone, which reaches the
 //    state through K^T D, would take the state's whole error budget when few rows dominate it.  The decay is kept as
 //    its logarithm.

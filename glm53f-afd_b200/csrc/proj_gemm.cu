@@ -7,7 +7,7 @@
 // low-rank gate pair 4096 -> 256 -> 2 x 8192; 3772-3790: o_proj 8192 -> 4096).
 //
 // Shape of the kernel.  The weight is the M operand: a tile is 128 output features x NR activation rows, NR in
-// {16, 32, 64, 128, 256} chosen from the row count, so a decode step's 16 rows waste nothing and the weight -- which
+// {16, 32, 64} chosen from the row count (more rows: proj_gemm_pair.cu), so a decode step's 16 rows waste nothing and the weight -- which
 // dominates the traffic at few rows (202 MB for the fused projection) -- streams through once.  Both operands are
 // K-major in global memory ([o][k] and [r][k]), so tiled tensor copies in the 128-byte swizzle feed tcgen05.mma
 // in place: a stage is 64 k of the weight tile (16 KiB) and of the row tile (NR x 128 bytes).  Roles per block:

@@ -75,20 +75,8 @@ __device__ __forceinline__ uint32_t elect_one() {
 // stays converged, so what it computes from uniform inputs stays in uniform registers.
 __device__ __forceinline__ bool warp_all(bool ok) { return __all_sync(0xffffffffu, ok); }
 
-// D[tmem] (+)= A[smem] * B[smem], issued by one thread.
-__device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, bool accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"((uint32_t)accumulate)
-        : "memory");
-}
-// Makes `bar` complete once every MMA issued so far by this thread has finished (implies fence::before_thread_sync).
-__device__ __forceinline__ void mma_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-
-// The same two issued by a converged warp with `leader` set in one lane (elect_one).  Inside an `if` of one lane the compiler
+// D[tmem] (+)= A[smem] * B[smem], and the commit that makes a barrier complete once every MMA issued so far has finished (implies
+// fence::before_thread_sync), issued by a converged warp with `leader` set in one lane (elect_one).  Inside an `if` of one lane the compiler
 // moves every operand of every MMA over from that lane's registers, about 90 cycles an instruction; issued so, descriptors
 // computed from uniform values are uniform registers already.
 __device__ __forceinline__ void mma_bf16_if(uint32_t leader, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, bool accumulate) {
@@ -169,17 +157,6 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32
         "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]),
         "r"(r[31])
         : "memory");
-}
-// 32 lanes x C columns (C = 16 or 32).
-template <int C>
-__device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[C]) {
-    if constexpr (C == 32) tmem_ld32(taddr, r);
-    else tmem_ld16(taddr, r);
-}
-template <int C>
-__device__ __forceinline__ void tmem_st(uint32_t taddr, const uint32_t (&r)[C]) {
-    if constexpr (C == 32) tmem_st32(taddr, r);
-    else tmem_st16(taddr, r);
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
