@@ -101,6 +101,13 @@ __device__ __forceinline__ uint2 pack4(const float (&x)[4]) {
                       (uint32_t)f32_to_bf16_bits(x[2]) | ((uint32_t)f32_to_bf16_bits(x[3]) << 16));
 }
 
+// Four consecutive channels of a row.  Rows of the projections are aligned for it (the callers check); a request's conv window
+// starts at any element of the arena its offset names, and is read element by element where that is not a multiple of four.
+__device__ __forceinline__ uint2 load4(const uint16_t* at, bool whole) {
+    if (whole) return *reinterpret_cast<const uint2*>(at);
+    return make_uint2((uint32_t)at[0] | ((uint32_t)at[1] << 16), (uint32_t)at[2] | ((uint32_t)at[3] << 16));
+}
+
 template <int SINK>
 __global__ void __launch_bounds__(128, 6) layer_prologue_kernel(const ProParams p) {
     constexpr bool VERIFY = SINK == kVerify, EXACT = SINK == kExact;
@@ -122,13 +129,14 @@ __global__ void __launch_bounds__(128, 6) layer_prologue_kernel(const ProParams 
     const int c0 = lane * 4, jj = p.row_shift + j;  // row of the request
     const long long C = 3LL * H * DK, gr = (long long)r0 + jj;
     const uint16_t* window = p.conv + (p.conv_off ? p.conv_off[b] : 0);
+    const bool odd = (reinterpret_cast<uintptr_t>(window) & 7) != 0;
     uint2 x[TAPS][3];  // [tap: rows jj-3 .. jj][part]; rows before the request's first come from the conv window
 #pragma unroll
     for (int d = 0; d < TAPS; ++d) {
         const int rr = jj - 3 + d;
         const uint16_t* row = rr < 0 ? window + (long long)(WINDOW + rr) * C : p.P + ((long long)r0 + rr) * p.p_stride;
 #pragma unroll
-        for (int part = 0; part < 3; ++part) x[d][part] = *reinterpret_cast<const uint2*>(row + ((long long)part * H + h) * DK + c0);
+        for (int part = 0; part < 3; ++part) x[d][part] = load4(row + ((long long)part * H + h) * DK + c0, rr >= 0 || !odd);
     }
     uint4 wq[3][2];
 #pragma unroll
@@ -228,13 +236,14 @@ __global__ void __launch_bounds__(128, 5) prefill_prologue_kernel(const ProParam
     const int first = p.row_shift + j0, last = p.row_shift + n - 1;  // rows of the request; rows before its first come from the conv window
     const long long C = 3LL * H * DK;
     const uint16_t* window = p.conv + (p.conv_off ? p.conv_off[b] : 0);
+    const bool odd = (reinterpret_cast<uintptr_t>(window) & 7) != 0;
     uint2 x[3][kRowsPer + 3];
 #pragma unroll
     for (int d = 0; d < kRowsPer + 3; ++d) {
         const int rr = min(first - 3 + d, last);
         const uint16_t* row = (rr < 0 ? window + (long long)(WINDOW + rr) * C : p.P + ((long long)r0 + rr) * p.p_stride) + (long long)h * DK + c0;
 #pragma unroll
-        for (int part = 0; part < 3; ++part) x[part][d] = *reinterpret_cast<const uint2*>(row + (long long)part * H * DK);
+        for (int part = 0; part < 3; ++part) x[part][d] = load4(row + (long long)part * H * DK, d >= 3 || rr >= 0 || !odd);  // d >= 3 is never a window row
     }
     uint2 a_bits[kRowsPer];
     float bl[kRowsPer];
