@@ -364,7 +364,7 @@ __device__ void mover_role(const Params& p, unsigned char* smem, uint64_t* bars,
         const Unit un = units.take(p);
         if (un.rows == 0 && !copy0) continue;
         // The unit's state.
-        if (!mbar_wait(&st_empty[st.idx], st.phase ^ 1u, ctx, kStatusWaitStateEmpty)) return;
+        if (!__all_sync(FULL, mbar_wait(&st_empty[st.idx], st.phase ^ 1u, ctx, kStatusWaitStateEmpty))) return;
         if (lane == 0) info[st.idx] = {un.s_elem, un.rows};
         if (p.skip_first_state && blockIdx.x == 0 && first) {
             // Diagnostic launch: nothing is copied and nobody is told, so the recurrence's wait for this state runs out.
@@ -387,7 +387,7 @@ __device__ void mover_role(const Params& p, unsigned char* smem, uint64_t* bars,
         st.next(L::kStateSlots);
         // Its rows' raw inputs.
         for (int r = 0; r < un.rows; ++r) {
-            if (!mbar_wait(&raw_empty[raw.idx], raw.phase ^ 1u, ctx, kStatusWaitRawEmpty)) return;
+            if (!__all_sync(FULL, mbar_wait(&raw_empty[raw.idx], raw.phase ^ 1u, ctx, kStatusWaitRawEmpty))) return;
             unsigned char* dst = smem + L::oRaw + raw.idx * L::kRawBytes;
             const Piece x = piece_of<MODE>(p, un, r, lane);
             const uintptr_t src = reinterpret_cast<uintptr_t>(x.src);
@@ -525,6 +525,9 @@ __device__ void layer_prologue_role(const Params& p, unsigned char* smem, uint64
     const bool vec = ((reinterpret_cast<uintptr_t>(p.cw) | reinterpret_cast<uintptr_t>(p.dt_bias)) & 15) == 0;
     UnitIter<kLayer> units(p);
     int turn = 0;
+    // A warp whose wait gave up does not leave: the single-row units further on are cooked by all four warps, which meet there at
+    // barriers.  It takes no more rows and goes on through the units to the next vote, which then sends all four home.
+    bool dead = false;
     auto widen = [](uint2 w, float (&x)[4]) {
         x[0] = __uint_as_float(w.x << 16);
         x[1] = __uint_as_float(w.x & 0xffff0000u);
@@ -546,7 +549,7 @@ __device__ void layer_prologue_role(const Params& p, unsigned char* smem, uint64
                 w[part] = vec ? *reinterpret_cast<const uint2*>(cw) : make_uint2((uint32_t)cw[0] | ((uint32_t)cw[1] << 16), (uint32_t)cw[2] | ((uint32_t)cw[3] << 16));
             }
             const float db = p.dt_bias[(long long)un.h * DK + c], decay_rate = expf(un.a_log);
-            const bool ready = mbar_wait(&raw_full[raw.idx], raw.phase, ctx, kStatusWaitRawFull) && mbar_wait(&row_empty[row.idx], row.phase ^ 1u, ctx, kStatusWaitRowEmpty);
+            const bool ready = !dead && mbar_wait(&raw_full[raw.idx], raw.phase, ctx, kStatusWaitRawFull) && mbar_wait(&row_empty[row.idx], row.phase ^ 1u, ctx, kStatusWaitRowEmpty);
             const unsigned char* in = smem + L::oRaw + raw.idx * L::kRawBytes;
             Cooked& ck = *reinterpret_cast<Cooked*>(smem + L::oCooked + row.idx * sizeof(Cooked));
             float* scratch = reinterpret_cast<float*>(smem + L::oScratch);
@@ -561,7 +564,7 @@ __device__ void layer_prologue_role(const Params& p, unsigned char* smem, uint64
                     (part == 2 ? ck.v : scratch + part * DK)[c] = bf16_round(acc / (1.0f + expf(-acc)));
                 }
             }
-            if (!named_bar_all(1, kProThreadsOf<kLayer>, ready)) return;  // one that gave up does not leave the others waiting
+            if (!named_bar_all(1, kProThreadsOf<kLayer>, ready)) return;  // all four leave together
             if (warp == 0) l2norm_warp(scratch, ck.q, lane, true);
             else if (warp == 1) l2norm_warp(scratch + DK, ck.k, lane, false);
             else if (warp == 2 && lane == 0) {
@@ -580,7 +583,7 @@ __device__ void layer_prologue_role(const Params& p, unsigned char* smem, uint64
             continue;
         }
         for (int r = 0; r < un.rows; ++r, raw.next(L::kRawSlots), row.next(L::kRowSlots)) {
-            if ((turn++ & (kProWarpsOf<kLayer> - 1)) != warp) continue;
+            if ((turn++ & (kProWarpsOf<kLayer> - 1)) != warp || dead) continue;
             // The head's weights come straight from global memory, on their way while the row's inputs are waited for.
             uint4 w[3][2];
             float4 dtb;
@@ -600,8 +603,11 @@ __device__ void layer_prologue_role(const Params& p, unsigned char* smem, uint64
                 }
                 dtb = vec ? *reinterpret_cast<const float4*>(db) : make_float4(db[0], db[1], db[2], db[3]);
             }
-            if (!mbar_wait(&raw_full[raw.idx], raw.phase, ctx, kStatusWaitRawFull)) return;
-            if (!mbar_wait(&row_empty[row.idx], row.phase ^ 1u, ctx, kStatusWaitRowEmpty)) return;
+            const bool ready = mbar_wait(&raw_full[raw.idx], raw.phase, ctx, kStatusWaitRawFull) && mbar_wait(&row_empty[row.idx], row.phase ^ 1u, ctx, kStatusWaitRowEmpty);
+            if (!__all_sync(FULL, ready)) {  // the warp as a whole: the norms below shuffle across it
+                dead = true;
+                continue;
+            }
             const unsigned char* in = smem + L::oRaw + raw.idx * L::kRawBytes;
             Cooked& ck = *reinterpret_cast<Cooked*>(smem + L::oCooked + row.idx * sizeof(Cooked));
             // Short conv + SiLU, one bf16 rounding (kda.cu:129-142); q and k then through the L2 norm (kda.cu:151-165).
