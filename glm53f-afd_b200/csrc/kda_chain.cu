@@ -188,6 +188,7 @@ struct Smem {
     static constexpr int oScratch = oCooked + kRowSlots * (int)sizeof(Cooked);  // prologue scratch: q, k before norm
     static constexpr int oBars = oScratch + 2 * DK * 4;
     // barriers: st_full[S], st_empty[S], raw_full[R], raw_empty[R], row_full[C], y_full[C], row_empty[C]
+    static_assert(MODE != kLayer || kRawSlots == kRowSlots, "layer_prologue_role: a free cooked slot implies a finished raw slot");
     static constexpr int kBars = 2 * kStateSlots + 2 * kRawSlots + 3 * kRowSlots;
     static constexpr int oCtl = oBars + kBars * 8;  // progress, abort
     static constexpr int oUnits = oCtl + 16;        // UnitInfo per state slot
@@ -513,6 +514,9 @@ __device__ void prologue_role(const Params& p, unsigned char* smem, uint64_t* ba
 // norms stay in the warp and nothing meets at a barrier), the warps take rows in turn.  A row is a chain of about 1,000
 // instructions, most of them divisions and exponentials; with all four warps on the same row a row left every 4,500 cycles and the
 // recurrence, 1,600 a row, waited (6 slots x 4 to 8 rows, f32: 37 -> 32 us a layer).
+// A warp skips the others' rows, so it has not itself seen the row that held the raw slot before, whose copy may land after later
+// rows' copies: raw_full can be a phase behind what its parity says.  So every row waits for its cooked slot first.  The two rings
+// are equally deep, and that slot is free only when the row before has been through the whole pipeline, its raw copy included.
 template <typename S>
 __device__ void layer_prologue_role(const Params& p, unsigned char* smem, uint64_t* bars, const WaitCtx& ctx, int warp, int lane) {
     using L = Smem<S, kLayer>;
@@ -549,7 +553,7 @@ __device__ void layer_prologue_role(const Params& p, unsigned char* smem, uint64
                 w[part] = vec ? *reinterpret_cast<const uint2*>(cw) : make_uint2((uint32_t)cw[0] | ((uint32_t)cw[1] << 16), (uint32_t)cw[2] | ((uint32_t)cw[3] << 16));
             }
             const float db = p.dt_bias[(long long)un.h * DK + c], decay_rate = expf(un.a_log);
-            const bool ready = !dead && mbar_wait(&raw_full[raw.idx], raw.phase, ctx, kStatusWaitRawFull) && mbar_wait(&row_empty[row.idx], row.phase ^ 1u, ctx, kStatusWaitRowEmpty);
+            const bool ready = !dead && mbar_wait(&row_empty[row.idx], row.phase ^ 1u, ctx, kStatusWaitRowEmpty) && mbar_wait(&raw_full[raw.idx], raw.phase, ctx, kStatusWaitRawFull);
             const unsigned char* in = smem + L::oRaw + raw.idx * L::kRawBytes;
             Cooked& ck = *reinterpret_cast<Cooked*>(smem + L::oCooked + row.idx * sizeof(Cooked));
             float* scratch = reinterpret_cast<float*>(smem + L::oScratch);
@@ -603,7 +607,7 @@ __device__ void layer_prologue_role(const Params& p, unsigned char* smem, uint64
                 }
                 dtb = vec ? *reinterpret_cast<const float4*>(db) : make_float4(db[0], db[1], db[2], db[3]);
             }
-            const bool ready = mbar_wait(&raw_full[raw.idx], raw.phase, ctx, kStatusWaitRawFull) && mbar_wait(&row_empty[row.idx], row.phase ^ 1u, ctx, kStatusWaitRowEmpty);
+            const bool ready = mbar_wait(&row_empty[row.idx], row.phase ^ 1u, ctx, kStatusWaitRowEmpty) && mbar_wait(&raw_full[raw.idx], raw.phase, ctx, kStatusWaitRawFull);
             if (!__all_sync(FULL, ready)) {  // the warp as a whole: the norms below shuffle across it
                 dead = true;
                 continue;
