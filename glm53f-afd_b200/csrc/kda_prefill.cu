@@ -100,6 +100,10 @@ int exact_layer_prefill(int32_t heads, int32_t batch, const int32_t* cu_rows, in
     if (max_rows < kExactMinRows || !al(out, 8) || !al(g, 8) || !al(norm_w, 8) || !al(workspace, 16) || !al(p, 8) || !al(a, 8) || !al(conv, 8) ||
         !al(conv_w, 16) || !al(dt_bias, 16) || p_stride % 4 || a_stride % 4 || g_stride % 4 || out_stride % 4)
         return kNotEligible;
+    // In place, or shifted back by whole rows: the only ways for the two to meet in which the chain's results are defined.
+    const int64_t apart = ((int64_t)reinterpret_cast<uintptr_t>(g) - (int64_t)reinterpret_cast<uintptr_t>(out)) / (int64_t)sizeof(glm53f_bf16);
+    if (out_stride == g_stride && (apart == 0 || (out_stride != 0 && apart % out_stride == 0 && apart / out_stride >= 0 && apart / out_stride < max_rows)))
+        return kNotEligible;
     int64_t pass = workspace_bytes / ((int64_t)batch * heads * kExactBytesPerRowHead) / 16 * 16;
     const int64_t need = ((int64_t)max_rows + 15) / 16 * 16;
     if (pass > need) pass = need;

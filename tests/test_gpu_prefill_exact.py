@@ -48,3 +48,24 @@ def test_passes_leave_the_chains_bits(K, lens, pass_rows, state, in_place):
         got.append((out, st if in_place else other, cv))
     for a, b in zip(*got):
         assert torch.equal(a.view(torch.int16), b.view(torch.int16))
+
+
+@pytest.mark.parametrize("back", [0, 1, 40])  # rows by which the outputs lie before the gate rows of the same buffer
+def test_outputs_over_the_gate_rows(K, back):
+    h, rows, g = 2, 70, torch.Generator(device="cuda").manual_seed(back)
+    c, width = K.channels(h), h * DK
+    rn = lambda m, s=1.0, d=torch.bfloat16: (torch.randn(m, device="cuda", generator=g) * s).to(d)
+    buf = lambda t: K.DeviceBuffer(t.view(torch.uint8))
+    w = K.Weights(h, buf(rn(c * 4, 0.5)), buf(rn(h, 0.5, torch.float32)), buf(rn(width, 1.0, torch.float32)), buf(1 + rn(DK, 0.1)), 1e-5, -5.0)
+    p, a, gate, conv, state = rn(rows * (c + h * 4)), rn(rows * width), rn((back + rows) * width), rn(3 * c), rn(K.state_len(h), 0.3, torch.float32)
+    meta, stream, got = K.BatchMeta.new(1), K.Stream(), []
+    meta.set([K.Request(rows, 0, 0)])
+    for over in (False, True):
+        gates, st, cv = gate.clone(), state.clone(), conv.clone()
+        out = gates if over else torch.zeros(rows * width, dtype=torch.bfloat16, device="cuda")
+        K.PrefillBatch(w, K.RowView.dense(buf(p), c + h * 4), c, K.RowView.dense(buf(a), width), K.RowView.new(buf(gates), back * width, width), buf(cv), buf(st),
+                       K.StateOut.InPlace, K.RowView.dense(buf(out), width), 0, K.PrefillWorkspace.new(h, 1, 32)).launch(meta, stream)
+        torch.cuda.synchronize()
+        got.append((out[:rows * width].clone(), st, cv))
+    for x, y in zip(*got):
+        assert torch.equal(x.view(torch.int16), y.view(torch.int16))
