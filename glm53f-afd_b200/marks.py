@@ -220,6 +220,8 @@ class KvPool:
             raise Invalid("a mark or a slot of another pool")
         if len({kv.slot for kv in kvs}) != len(kvs):
             raise Invalid("the same slot twice in one batch")
+        for m in marks_:
+            m._check_whole()
         n = len(kvs)
         lists = torch.from_numpy(np.concatenate([m._pages for m in marks_])).to(self.pages.t.device)
         slots = torch.tensor([kv.slot for kv in kvs], dtype=torch.int32).to(self.pages.t.device)
@@ -279,6 +281,11 @@ class KvMark:
 
     def pages(self) -> int:
         return len(self._pages)
+
+    def _check_whole(self) -> None:
+        """The copies read as many entries of the page list as the pool's layout has pages, whatever the list holds."""
+        if len(self._pages) != self._pool.mark_pages:
+            raise Invalid(f"a mark of {len(self._pages)} pages (dropped?), the layout has {self._pool.mark_pages}")
 
     def page_list(self) -> list[int]:
         return self._pages.tolist()
@@ -369,6 +376,7 @@ class GlmKv:
         """The positional state into `mark`'s pages (`save`) or out of them into the slot (kv.rs:412-476)."""
         if mark._pool is not self.pool:
             raise Invalid("a mark of another pool")
+        mark._check_whole()
         torch = kernel._torch()
         l, p = self.layout(), self.pool
         pb = l.page_bytes

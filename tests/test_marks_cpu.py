@@ -147,3 +147,16 @@ def test_error_behaviour_needs_no_launch(marks, pkg, monkeypatch):
     assert b.conv_elem_offset() == l.conv_bytes() // 2 and b.tail_row(0) == 1
     b.release()
     assert pool.free_slots() == 1
+
+
+def test_a_dropped_mark_is_refused_before_any_copy(marks, monkeypatch):
+    kernel = importlib.import_module("glm53f-afd_b200.kernel")
+    monkeypatch.setattr(kernel, "DEVICE", "cpu")
+    l = marks.KvLayout.new(1, 1).with_kda_state_bf16(True)
+    pool = marks.KvPool(marks.KvConfig(l, 2, 2 * l.mark_pages()))
+    a, b = pool.slot(), pool.slot()
+    whole, dropped = (marks.KvMark(0, pool.alloc.alloc_many(l.mark_pages()), pool) for _ in range(2))
+    dropped.drop()
+    for call in (lambda: a.rewind(0, dropped), lambda: pool.rewind_many([a, b], [whole, dropped]), lambda: pool.rewind_many([a], [dropped])):
+        with pytest.raises(marks.Invalid, match="a mark of 0 pages"):
+            call()
