@@ -443,10 +443,15 @@ class GlmKv:
         if mark._pool is not self.pool:
             self.reset()
             raise Invalid("a mark of another pool")
-        # The slot's state is not cleared first: the copy covers every byte of it.
+        # The slot's state is not cleared first: the copy covers every byte of it.  Without the copy it is: the slot then holds no
+        # tokens, and a prefill into it has to start from nothing.
         self._tokens = 0
         self.pending = 0
-        self._copy_mark(mark, False)
+        try:
+            self._copy_mark(mark, False)
+        except Exception:
+            self._clear_state()
+            raise
         self._tokens = to
 
     # ---- host images ------------------------------------------------------------------------------------------

@@ -160,3 +160,26 @@ def test_a_dropped_mark_is_refused_before_any_copy(marks, monkeypatch):
     for call in (lambda: a.rewind(0, dropped), lambda: pool.rewind_many([a, b], [whole, dropped]), lambda: pool.rewind_many([a], [dropped])):
         with pytest.raises(marks.Invalid, match="a mark of 0 pages"):
             call()
+
+
+def test_a_fork_that_fails_leaves_an_empty_slot(marks, monkeypatch):
+    kernel = importlib.import_module("glm53f-afd_b200.kernel")
+    monkeypatch.setattr(kernel, "DEVICE", "cpu")
+    l = marks.KvLayout.new(1, 1).with_kda_state_bf16(True)
+    pool = marks.KvPool(marks.KvConfig(l, 3, 2 * l.mark_pages()))
+    a, b, c = pool.slot(), pool.slot(), pool.slot()
+    dropped = marks.KvMark(0, pool.alloc.alloc_many(l.mark_pages()), pool)
+    dropped.drop()
+    whole = marks.KvMark(0, pool.alloc.alloc_many(l.mark_pages()), pool)
+    for mark in (dropped, whole):  # the second one fails in the launch itself: there is no GPU
+        for t in (pool.state.t, pool.conv.t, pool.tails.t):
+            t.fill_(7)
+        b.advance(5)
+        if mark is whole:
+            monkeypatch.setattr(marks.GlmKv, "_copy_mark", lambda *_: (_ for _ in ()).throw(marks.CudaError(999, "mark pages")))
+        with pytest.raises((marks.Invalid, marks.CudaError)):
+            b.fork(a, 0, mark)
+        assert (b.tokens(), b.pending) == (0, 0)
+        arenas = ((pool.state.t, l.kda_state_bytes()), (pool.conv.t, l.conv_bytes()), (pool.tails.t, max(l.tails_bytes(), 16)))
+        for t, n in arenas:  # slot 1's part is cleared, its neighbours are not touched
+            assert not t[n:n + n // 16 * 16].any() and (t[:n] == 7).all() and (t[2 * n:] == 7).all()
