@@ -23,7 +23,7 @@ from __future__ import annotations
 
 import ctypes as C
 from dataclasses import dataclass, replace
-from typing import Optional
+from typing import Optional, Sequence
 
 import numpy as np
 
@@ -271,9 +271,9 @@ class KvMark:
     """A slot's positional state at `tokens`, held in pages of the pool (kv.rs:207-236).  `drop()` (or garbage
     collection) gives the pages back."""
 
-    def __init__(self, tokens: int, pages: np.ndarray, pool: KvPool):
+    def __init__(self, tokens: int, pages: Sequence[int], pool: KvPool):
         self.tokens = tokens
-        self._pages = pages
+        self._pages = np.ascontiguousarray(pages, np.int32)
         self._pool = pool
 
     def bytes(self) -> int:

@@ -183,3 +183,16 @@ def test_a_fork_that_fails_leaves_an_empty_slot(marks, monkeypatch):
         arenas = ((pool.state.t, l.kda_state_bytes()), (pool.conv.t, l.conv_bytes()), (pool.tails.t, max(l.tails_bytes(), 16)))
         for t, n in arenas:  # slot 1's part is cleared, its neighbours are not touched
             assert not t[n:n + n // 16 * 16].any() and (t[:n] == 7).all() and (t[2 * n:] == 7).all()
+
+
+def test_a_mark_takes_any_sequence_of_pages(marks, monkeypatch):
+    kernel = importlib.import_module("glm53f-afd_b200.kernel")
+    monkeypatch.setattr(kernel, "DEVICE", "cpu")
+    l = marks.KvLayout.new(1, 0).with_kda_state_bf16(True)
+    pool = marks.KvPool(marks.KvConfig(l, 1, l.mark_pages()))
+    for kind in (list, tuple, np.asarray):
+        m = marks.KvMark(3, kind([pool.alloc.alloc() for _ in range(l.mark_pages())]), pool)
+        assert sorted(m.page_list()) == list(range(l.mark_pages())) and m.pages() == l.mark_pages() and pool.free_pages() == 0
+        m.drop()
+        m.drop()
+        assert pool.free_pages() == l.mark_pages() and m.page_list() == []
