@@ -212,6 +212,15 @@ class KvPool:
     def bytes(self) -> int:
         return self.pages.bytes()
 
+    def _after_current(self) -> None:
+        """With a stream of the pool's own: a copy on it comes after the work of torch's current stream, where slots are cleared and
+        images imported.  (The copies that upload a page list first wait for that stream on the host.)"""
+        if self.stream.stream is not None:
+            cuda = kernel._torch().cuda
+            current, own = cuda.current_stream(), self.stream.stream.cuda_stream
+            if own != current.cuda_stream:
+                cuda.ExternalStream(own).wait_stream(current)
+
     # ---- several slots in one launch (an addition: the reference marks slot by slot) -------------------------------
     def _copy_marks(self, kvs, marks_, save: bool) -> None:
         torch = kernel._torch()
@@ -382,6 +391,7 @@ class GlmKv:
         pb = l.page_bytes
         n_idx = len(mark._pages)
         if p.fused and n_idx <= INLINE_PAGES and p.pages.t.is_cuda:
+            p._after_current()
             parts = (C.c_void_p * 3)(*[a.as_ptr() + at for a, at in self._arenas()])
             return _launched(ffi.load().glm53f_kda_mark_copy_list(p.pages.as_ptr(), pb, mark._pages.ctypes.data, n_idx, parts, p.mark_sizes, 1 if save else 0, p.stream.raw()),
                              "mark pages")

@@ -287,3 +287,24 @@ def test_marks_of_several_slots_in_one_launch(marks, bf16):
     with pytest.raises(marks.OutOfMemory):
         pool.mark_many(kvs)
     assert pool.mark_many([]) == []
+
+
+def test_copies_on_the_pools_own_stream_follow_the_current_one(marks, G):
+    K = importlib.import_module("glm53f-afd_b200.kernel")
+    l = marks.KvLayout.new(1, 1).with_kda_state_bf16(True)
+    pool = marks.KvPool(marks.KvConfig(l, 2, 2 * l.mark_pages()), K.Stream(torch.cuda.Stream()))
+    a, n = pool.slot(), l.kda_state_bytes()
+    a.advance(64)
+    torch.cuda.synchronize()
+    torch.cuda._sleep(20_000_000)  # 10 ms: what follows on this stream is still to come when the copies are launched
+    pool.state.t[:n] = 5
+    m = a.mark()
+    b = pool.slot()  # cleared on the current stream
+    b.fork(a, 64, m)
+    torch.cuda.synchronize()
+    assert (pool.state.t[n:] == 5).all()
+    torch.cuda._sleep(20_000_000)
+    pool.state.t[:n] = 6
+    a.rewind(64, m)
+    torch.cuda.synchronize()
+    assert (pool.state.t[:n] == 5).all()
