@@ -101,12 +101,13 @@ __device__ __forceinline__ uint2 pack4(const float (&x)[4]) {
                       (uint32_t)f32_to_bf16_bits(x[2]) | ((uint32_t)f32_to_bf16_bits(x[3]) << 16));
 }
 
-// Four consecutive channels of a row.  Rows of the projections are aligned for it (the callers check); a request's conv window
-// starts at any element of the arena its offset names, and is read element by element where that is not a multiple of four.
-__device__ __forceinline__ uint2 load4(const uint16_t* at, bool whole) {
-    if (whole) return *reinterpret_cast<const uint2*>(at);
+// Four consecutive channels of a row, element by element.  Rows of the projections are aligned for vector loads (the callers check);
+// a request's conv window starts at any element of the arena its offset names, and the few warps that read one take a way of
+// their own where it is not aligned: a choice at every load costs the loads their overlap (701 rows exact: 403 -> 408 us).
+__device__ __forceinline__ uint2 load4(const uint16_t* at) {
     return make_uint2((uint32_t)at[0] | ((uint32_t)at[1] << 16), (uint32_t)at[2] | ((uint32_t)at[3] << 16));
 }
+__device__ __forceinline__ bool unaligned8(const void* at) { return (reinterpret_cast<uintptr_t>(at) & 7) != 0; }
 
 template <int SINK>
 __global__ void __launch_bounds__(128, 6) layer_prologue_kernel(const ProParams p) {
@@ -129,15 +130,18 @@ __global__ void __launch_bounds__(128, 6) layer_prologue_kernel(const ProParams 
     const int c0 = lane * 4, jj = p.row_shift + j;  // row of the request
     const long long C = 3LL * H * DK, gr = (long long)r0 + jj;
     const uint16_t* window = p.conv + (p.conv_off ? p.conv_off[b] : 0);
-    const bool odd = (reinterpret_cast<uintptr_t>(window) & 7) != 0;
     uint2 x[TAPS][3];  // [tap: rows jj-3 .. jj][part]; rows before the request's first come from the conv window
+    auto fetch = [&](auto&& load) {
 #pragma unroll
-    for (int d = 0; d < TAPS; ++d) {
-        const int rr = jj - 3 + d;
-        const uint16_t* row = rr < 0 ? window + (long long)(WINDOW + rr) * C : p.P + ((long long)r0 + rr) * p.p_stride;
+        for (int d = 0; d < TAPS; ++d) {
+            const int rr = jj - 3 + d;
+            const uint16_t* row = rr < 0 ? window + (long long)(WINDOW + rr) * C : p.P + ((long long)r0 + rr) * p.p_stride;
 #pragma unroll
-        for (int part = 0; part < 3; ++part) x[d][part] = load4(row + ((long long)part * H + h) * DK + c0, rr >= 0 || !odd);
-    }
+            for (int part = 0; part < 3; ++part) x[d][part] = load(row + ((long long)part * H + h) * DK + c0);
+        }
+    };
+    if (jj < WINDOW && unaligned8(window)) fetch([](const uint16_t* at) { return load4(at); });
+    else fetch([](const uint16_t* at) { return *reinterpret_cast<const uint2*>(at); });
     uint4 wq[3][2];
 #pragma unroll
     for (int part = 0; part < 3; ++part) {
@@ -227,6 +231,8 @@ __device__ __forceinline__ uint32_t fp16x2(float2 x) {
     return *reinterpret_cast<const uint32_t*>(&h);
 }
 
+// FIRST: the pass with the requests' first rows, which reach back into the conv windows.
+template <bool FIRST>
 __global__ void __launch_bounds__(128, 5) prefill_prologue_kernel(const ProParams p) {
     const int lane = threadIdx.x & 31, H = p.H, groups = p.pass_rows / (4 * kRowsPer), c0 = lane * 4;
     // heads innermost: neighbouring blocks read neighbouring pieces of the same rows
@@ -235,15 +241,23 @@ __global__ void __launch_bounds__(128, 5) prefill_prologue_kernel(const ProParam
     if (j0 >= n) return;
     const int first = p.row_shift + j0, last = p.row_shift + n - 1;  // rows of the request; rows before its first come from the conv window
     const long long C = 3LL * H * DK;
-    const uint16_t* window = p.conv + (p.conv_off ? p.conv_off[b] : 0);
-    const bool odd = (reinterpret_cast<uintptr_t>(window) & 7) != 0;
     uint2 x[3][kRowsPer + 3];
+    auto fetch = [&](const uint16_t* window, auto&& load) {
 #pragma unroll
-    for (int d = 0; d < kRowsPer + 3; ++d) {
-        const int rr = min(first - 3 + d, last);
-        const uint16_t* row = (rr < 0 ? window + (long long)(WINDOW + rr) * C : p.P + ((long long)r0 + rr) * p.p_stride) + (long long)h * DK + c0;
+        for (int d = 0; d < kRowsPer + 3; ++d) {
+            const int rr = min(first - 3 + d, last);
+            const uint16_t* row = (FIRST && rr < 0 ? window + (long long)(WINDOW + rr) * C : p.P + ((long long)r0 + rr) * p.p_stride) + (long long)h * DK + c0;
 #pragma unroll
-        for (int part = 0; part < 3; ++part) x[part][d] = load4(row + (long long)part * H * DK, d >= 3 || rr >= 0 || !odd);  // d >= 3 is never a window row
+            for (int part = 0; part < 3; ++part) x[part][d] = load(row + (long long)part * H * DK);
+        }
+    };
+    auto vec = [](const uint16_t* at) { return *reinterpret_cast<const uint2*>(at); };
+    if constexpr (FIRST) {
+        const uint16_t* window = p.conv + (p.conv_off ? p.conv_off[b] : 0);
+        if (first < WINDOW && unaligned8(window)) fetch(window, [](const uint16_t* at) { return load4(at); });
+        else fetch(window, vec);
+    } else {
+        fetch(nullptr, vec);
     }
     uint2 a_bits[kRowsPer];
     float bl[kRowsPer];
@@ -347,7 +361,8 @@ int layer_prologue_launch(int32_t heads, int32_t batch, const int32_t* cu_rows, 
     pp.slots = slots;
     const long long blocks = (long long)batch * heads * (pp.pass_rows / (4 * kRowsPer));
     if (blocks > 0x7fffffffLL) return kInvalid;
-    prefill_prologue_kernel<<<(unsigned)blocks, 128, 0, stream>>>(pp);
+    if (chunk0 == 0) prefill_prologue_kernel<true><<<(unsigned)blocks, 128, 0, stream>>>(pp);
+    else prefill_prologue_kernel<false><<<(unsigned)blocks, 128, 0, stream>>>(pp);
     return (int)cudaGetLastError();
 }
 
