@@ -450,11 +450,14 @@ class BatchMeta:
         if self._all.t.is_cuda:
             torch.cuda.synchronize()
 
-    def set_on(self, requests: Sequence[Request], keep: Optional[Sequence[int]], stream: Stream) -> None:
-        """`set` in the order of `stream`, without waiting for it: for launches on that stream."""
+    def set_on(self, requests: Sequence[Request], keep: Optional[Sequence[int]], stream: Stream, wait=None) -> None:
+        """`set` in the order of `stream`, without waiting for it: for launches on that stream.  `wait(stream)`, if given, is what
+        the launch still has to wait for; it is called last, when all that is left to do is the launch."""
         if not self._all.t.is_cuda:
             return self.set(requests, keep)
         image = self._set(requests, keep)
+        if wait is not None:
+            wait(stream)
         _launched(ffi.glm53f_kda_store_words(self._all.ptr(), image.ctypes.data, image.size, stream.raw()), "glm53f_kda_store_words")
 
     def _set(self, requests: Sequence[Request], keep: Optional[Sequence[int]]) -> np.ndarray:

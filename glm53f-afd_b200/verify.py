@@ -99,20 +99,27 @@ class KdaVerify:
             raise Invalid(f"{sum(rows)} verify rows exceed the scratch of {self.v.rows}")
         if any(kv.pool is not self.pool for kv, _ in windows):
             raise Invalid("a slot of another pool")
-        self._set_meta([K.Request(r, kv.conv_elem_offset(), kv.state_elem_offset()) for kv, r in windows], None, self.pool.stream)
+        requests = [K.Request(r, kv.conv_elem_offset(), kv.state_elem_offset()) for kv, r in windows]
+        self._set_meta(requests, None, self.pool.stream, self._wait_for_all)
         self.pending = [_Req(kv.slot, kv.tokens(), r) for kv, r in windows]
         for kv, r in windows:
             kv.pending = r
 
-    def _set_meta(self, requests, keep, stream: K.Stream) -> None:
-        """The batch metadata in the order of `stream`: the host runs on while earlier launches are still queued."""
-        self._order(stream)
-        self.meta.set_on(requests, keep, stream)
+    def _set_meta(self, requests, keep, stream: K.Stream, wait) -> None:
+        """The batch metadata in the order of `stream`, after `wait(stream)`."""
+        self.meta.set_on(requests, keep, stream, wait)
         self._meta_on = K.raw_stream(stream) if self.pool.state.t.is_cuda else None
 
+    def _wait_for_all(self, _stream) -> None:
+        """A round opens behind everything queued on the device: a prefill of its slots, or the commit of another round over the pool,
+        may be on any stream.  (Inside a graph's capture the order is the captured one.)"""
+        cuda = K._torch().cuda
+        if not cuda.is_current_stream_capturing():
+            cuda.synchronize()
+
     def _order(self, stream: K.Stream) -> None:
-        """Before work on `stream`: when the round so far is on another stream, wait for it (from then on before every call
-        of the round, since its launches are on several streams)."""
+        """Before work of an open round on `stream`: when the round so far is on another stream, wait for it (from then on before
+        every call of the round, since its launches are on several streams)."""
         if self._meta_on is not None and K.raw_stream(stream) != self._meta_on:
             K._torch().cuda.synchronize()
             self._meta_on = -1
@@ -157,7 +164,7 @@ class KdaVerify:
                 raise Invalid(f"commit of {k} rows does not match the pending verify of slot {kv.slot}")
         l = self.pool.cfg.layout
         stream = stream or self.pool.stream
-        self._set_meta(self.meta.requests(), list(keep), stream)
+        self._set_meta(self.meta.requests(), list(keep), stream, self._order)  # the host runs on while the layers are still queued
         # The arenas are slot-major ([slot][layer]...): layer strides of one layer's elements, request offsets of whole
         # slots.  The checked wrappers of kernel.py assume layer-major arenas, so, like the reference's forward, this goes
         # to the entry points directly (forward.rs:1972-2031).

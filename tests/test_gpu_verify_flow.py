@@ -126,3 +126,35 @@ def test_verify_then_commit_equals_serial_decode(mods, oracle, bf16, recompute):
     for (j, r), out in serial_out.items():
         got = outs[j].buf.download(np.uint16, H * DK, r * H * DK)
         assert np.array_equal(got, out.buf.download(np.uint16, H * DK)), (j, r)
+
+
+def test_a_round_opens_behind_work_on_other_streams(mods):
+    K, marks, verify = mods["kernel"], mods["marks"], mods["verify"]
+    l = marks.KvLayout.new(1, 0)
+    pool = marks.KvPool(marks.KvConfig(l, 1, 1))
+    kv, g = pool.slot(), torch.Generator(device="cuda").manual_seed(4)
+    rn = lambda m, s=1.0, d=torch.bfloat16: (torch.randn(m, device="cuda", generator=g) * s).to(d)
+    buf = lambda t: K.DeviceBuffer(t.view(torch.uint8))
+    c, width = K.channels(H), H * DK
+    w = K.Weights(H, buf(rn(c * 4, 0.5)), buf(rn(H, 0.5, torch.float32)), buf(rn(width, 1.0, torch.float32)), buf(1 + rn(DK, 0.1)), 1e-5, -5.0)
+    vf = verify.KdaVerify(pool, [w], 2, 1)
+    vf.v.p.t.view(torch.bfloat16).copy_(rn(2 * (c + H)))
+    gates, state, outs = buf(rn(2 * 2 * width)), rn(K.state_len(H), 0.3, torch.float32), []
+    for late in (False, True):
+        pool.state.t.zero_()
+        pool.conv.t.zero_()
+        torch.cuda.synchronize()
+        side = torch.cuda.Stream()
+        with torch.cuda.stream(side):  # the slot's prefill, say
+            if late:
+                torch.cuda._sleep(20_000_000)  # 10 ms
+            pool.state.t.view(torch.float32).copy_(state)
+        if not late:
+            torch.cuda.synchronize()
+        out = torch.zeros(2 * width, dtype=torch.bfloat16, device="cuda")
+        vf.verify([(kv, 2)])
+        vf.layer(0, K.RowView.new(gates, 0, 2 * width), K.RowView.new(gates, width, 2 * width), K.RowView.dense(buf(out), width))
+        vf.commit([kv], [1])
+        torch.cuda.synchronize()
+        outs.append((out, pool.state.t.clone()))
+    assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
