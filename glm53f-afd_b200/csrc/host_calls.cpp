@@ -81,9 +81,15 @@ inline Buffer get_buffer(PyObject* o, PyObject* name) {
     Ref r(get(o, name));
     return buffer(r.o);
 }
+// a * b + c, exactly.
+inline int64_t mul_add(int64_t a, int64_t b, int64_t c) {
+    int64_t r;
+    if (__builtin_mul_overflow(a, b, &r) || __builtin_add_overflow(r, c, &r)) throw Miss{};
+    return r;
+}
 // Elements [offset, offset + n) of `size` bytes lie inside the buffer.
 inline void region(const Buffer& b, int64_t size, int64_t offset, int64_t n) {
-    if (offset < 0 || offset + n > b.bytes / size) throw Miss{};
+    if (offset < 0 || mul_add(offset, 1, n) > b.bytes / size) throw Miss{};
 }
 
 struct Rows {
@@ -96,7 +102,7 @@ inline Rows rows_of(PyObject* owner, PyObject* name, int64_t rows, int64_t lo, i
     is_exactly(v.o, T_view);
     const Buffer b = get_buffer(v.o, N.buf);
     const int64_t offset = get_i64(v.o, N.offset), stride = get_i64(v.o, N.stride);
-    if (rows > 0 && (offset + lo < 0 || offset + (rows - 1) * stride + hi > b.bytes / 2)) throw Miss{};
+    if (rows > 0 && (mul_add(offset, 1, lo) < 0 || mul_add(rows - 1, stride, mul_add(offset, 1, hi)) > b.bytes / 2)) throw Miss{};
     return {reinterpret_cast<glm53f_bf16*>(b.ptr) + offset, stride};
 }
 
@@ -125,7 +131,8 @@ int chain_batch(PyObject* cb, PyObject* meta, PyObject* stream, bool bf16) {
     if (heads < 1 || heads > 65535 || batch < 1) throw Miss{};
     const int64_t channels = 3 * heads * kD, width = heads * kD, state_len = heads * kD * kD;
     const int64_t b_off = get_i64(cb, N.b_off);
-    const Rows p = rows_of(cb, N.p, total, b_off < 0 ? b_off : 0, b_off + heads > channels ? b_off + heads : channels);
+    const int64_t b_end = mul_add(b_off, 1, heads);
+    const Rows p = rows_of(cb, N.p, total, b_off < 0 ? b_off : 0, b_end > channels ? b_end : channels);
     const Rows a = rows_of(cb, N.a, total, 0, width), g = rows_of(cb, N.g, total, 0, width), out = rows_of(cb, N.out, total, 0, width);
     if (total > 1 && out.stride < width) throw Miss{};
     const Buffer conv = get_buffer(cb, N.conv), state = get_buffer(cb, N.state);
@@ -204,7 +211,7 @@ int core_decode(PyObject* const* a) {
     if (!state.is_cuda()) throw Miss{};
     const int32_t kind = sd == at::kFloat ? 0 : sd == at::kBFloat16 || sd == at::kShort || sd == at::kUInt16 ? 1 : -1;
     if (kind < 0) throw Miss{};
-    if (a[17] != Py_None && state.numel() < to_i64(a[17]) + heads * kD * kD) throw Miss{};
+    if (a[17] != Py_None && state.numel() < mul_add(to_i64(a[17]), 1, heads * kD * kD)) throw Miss{};
     void* so = nullptr;
     if (PyUnicode_Check(a[10])) so = state.data_ptr();
     else if (a[10] != Py_None) {

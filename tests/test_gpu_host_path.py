@@ -61,3 +61,31 @@ def test_calls_with_an_error_keep_their_errors(pkg):
             core.decode_batch(**{**ok, **bad})
     torch.cuda.synchronize()
     assert core.device_status() == 0
+
+
+BIG = 1 << 62
+
+
+@pytest.mark.parametrize("what, text", [
+    (dict(conv_offset=(1 << 63) - 1), "conv: elements"), (dict(state_offset=(1 << 63) - 8), "state: elements"), (dict(conv_offset=-1), "conv: elements"),
+    (dict(b_off=(1 << 63) - 1), "p"), (dict(rows=2, p_stride=BIG), "p"), (dict(p_stride=BIG), "p"), (dict(a_stride=BIG), "a"), (dict(g_stride=3 * BIG // 2), "g"), (dict(p_offset=(1 << 63) - 4), "p"),
+    (dict(out_stride=255), "out"), (dict(state_offset=1), "state: "), (dict(rows=3), "p"), (dict(saves=1), "saves hold")])
+def test_a_chain_call_with_an_error_keeps_its_error(pkg, what, text):
+    """Extents that 64 bits cannot hold among them: the checks on the native path may not wrap."""
+    K = importlib.import_module("glm53f-afd_b200.kernel")
+    h, rows, n = 2, 2, 2
+    c, width = K.channels(h), h * 128
+    buf = lambda elems, size=2: K.DeviceBuffer(torch.zeros(elems * size, dtype=torch.uint8, device="cuda"))
+    w = K.Weights(h, buf(c * 4), buf(h, 4), buf(width, 4), buf(128), 1e-5, -5.0)
+    meta = K.BatchMeta.new(n)
+
+    def call(conv_offset=0, state_offset=K.state_len(h), b_off=c, p_stride=c + h, a_stride=width, g_stride=width, out_stride=width, p_offset=0, rows=1, saves=0):
+        meta.set([K.Request(rows, 0, 0), K.Request(1, conv_offset, state_offset)])
+        K.ChainBatch(w, K.RowView.new(buf(2 * (c + h)), p_offset, p_stride), b_off, K.RowView.new(buf(2 * width), 0, a_stride), K.RowView.new(buf(2 * width), 0, g_stride),
+                     buf(3 * c), buf(n * K.state_len(h), 4), K.StateOut.InPlace, K.RowView.new(buf(2 * width), 0, out_stride),
+                     K.Saves.alloc(h, saves) if saves else None).launch(meta, K.Stream())
+
+    call()
+    with pytest.raises(K.Invalid, match="^" + text):
+        call(**what)
+    torch.cuda.synchronize()
