@@ -60,26 +60,51 @@ inline double get_f64(PyObject* o, PyObject* name) {
 inline void is_exactly(PyObject* o, PyObject* type) {
     if (reinterpret_cast<PyObject*>(Py_TYPE(o)) != type) throw Miss{};
 }
+// A launch without the interpreter's lock, as a foreign call makes it: a full launch queue blocks the caller, and what it waits for
+// may be a host function that needs the lock.  Everything Python has been read by then.
+template <typename F>
+int unlocked(F&& launch) {
+    int rc;
+    Py_BEGIN_ALLOW_THREADS
+    rc = launch();
+    Py_END_ALLOW_THREADS
+    return rc;
+}
+
 inline const at::Tensor& tensor(PyObject* o) {
     if (!THPVariable_Check(o)) throw Miss{};
     return THPVariable_Unpack(o);
 }
 
+// The tensors whose addresses a launch takes, held until it is out: another thread may let go of them meanwhile.
+struct Held {
+    PyObject* o[24];
+    int n = 0;
+    PyObject* add(PyObject* x) {
+        if (n == 24) throw Miss{};
+        Py_INCREF(x);
+        return o[n++] = x;
+    }
+    ~Held() {
+        while (n > 0) Py_DECREF(o[--n]);
+    }
+};
+
 struct Buffer {  // a DeviceBuffer: address and bytes
     unsigned char* ptr;
     int64_t bytes;
 };
-inline Buffer buffer(PyObject* o) {
+inline Buffer buffer(PyObject* o, Held& held) {
     is_exactly(o, T_buffer);
     Ref t(get(o, N.t));
-    const at::Tensor& x = tensor(t.o);
+    const at::Tensor& x = tensor(held.add(t.o));
     if (!x.is_cuda()) throw Miss{};
     const int64_t n = x.numel();
     return {n != 0 ? static_cast<unsigned char*>(x.data_ptr()) : nullptr, n};
 }
-inline Buffer get_buffer(PyObject* o, PyObject* name) {
+inline Buffer get_buffer(PyObject* o, PyObject* name, Held& held) {
     Ref r(get(o, name));
-    return buffer(r.o);
+    return buffer(r.o, held);
 }
 // a * b + c, exactly.
 inline int64_t mul_add(int64_t a, int64_t b, int64_t c) {
@@ -97,10 +122,10 @@ struct Rows {
     int64_t stride;
 };
 // A RowView of bf16 rows whose columns [lo, hi) lie inside its buffer for `rows` rows.
-inline Rows rows_of(PyObject* owner, PyObject* name, int64_t rows, int64_t lo, int64_t hi) {
+inline Rows rows_of(PyObject* owner, PyObject* name, int64_t rows, int64_t lo, int64_t hi, Held& held) {
     Ref v(get(owner, name));
     is_exactly(v.o, T_view);
-    const Buffer b = get_buffer(v.o, N.buf);
+    const Buffer b = get_buffer(v.o, N.buf, held);
     const int64_t offset = get_i64(v.o, N.offset), stride = get_i64(v.o, N.stride);
     if (rows > 0 && (mul_add(offset, 1, lo) < 0 || mul_add(rows - 1, stride, mul_add(offset, 1, hi)) > b.bytes / 2)) throw Miss{};
     return {reinterpret_cast<glm53f_bf16*>(b.ptr) + offset, stride};
@@ -125,6 +150,7 @@ int chain_batch(PyObject* cb, PyObject* meta, PyObject* stream, bool bf16) {
     int64_t m[8];
     for (int i = 0; i < 8; ++i) m[i] = to_i64(PyTuple_GET_ITEM(fast.o, i));
     const int64_t batch = m[0], total = m[1];
+    Held held;
     Ref w(get(cb, N.weights));
     is_exactly(w.o, T_weights);
     const int64_t heads = get_i64(w.o, N.heads), es = bf16 ? 2 : 4;
@@ -132,10 +158,10 @@ int chain_batch(PyObject* cb, PyObject* meta, PyObject* stream, bool bf16) {
     const int64_t channels = 3 * heads * kD, width = heads * kD, state_len = heads * kD * kD;
     const int64_t b_off = get_i64(cb, N.b_off);
     const int64_t b_end = mul_add(b_off, 1, heads);
-    const Rows p = rows_of(cb, N.p, total, b_off < 0 ? b_off : 0, b_end > channels ? b_end : channels);
-    const Rows a = rows_of(cb, N.a, total, 0, width), g = rows_of(cb, N.g, total, 0, width), out = rows_of(cb, N.out, total, 0, width);
+    const Rows p = rows_of(cb, N.p, total, b_off < 0 ? b_off : 0, b_end > channels ? b_end : channels, held);
+    const Rows a = rows_of(cb, N.a, total, 0, width, held), g = rows_of(cb, N.g, total, 0, width, held), out = rows_of(cb, N.out, total, 0, width, held);
     if (total > 1 && out.stride < width) throw Miss{};
-    const Buffer conv = get_buffer(cb, N.conv), state = get_buffer(cb, N.state);
+    const Buffer conv = get_buffer(cb, N.conv, held), state = get_buffer(cb, N.state, held);
     region(conv, 2, m[2], kWindow * channels);
     region(conv, 2, m[3], kWindow * channels);
     region(state, es, m[5], state_len);
@@ -155,25 +181,27 @@ int chain_batch(PyObject* cb, PyObject* meta, PyObject* stream, bool bf16) {
         if (s.o != Py_None) {
             is_exactly(s.o, T_saves);
             if (get_i64(s.o, N.heads) != heads || get_i64(s.o, N.rows) < total) throw Miss{};
-            ks = get_buffer(s.o, N.k).ptr;
-            vs = get_buffer(s.o, N.v).ptr;
-            gs = get_buffer(s.o, N.g).ptr;
-            bs = get_buffer(s.o, N.b).ptr;
+            ks = get_buffer(s.o, N.k, held).ptr;
+            vs = get_buffer(s.o, N.v, held).ptr;
+            gs = get_buffer(s.o, N.g, held).ptr;
+            bs = get_buffer(s.o, N.b, held).ptr;
         }
     }
-    const auto* cu = reinterpret_cast<const int32_t*>(get_buffer(meta, N.cu_rows).ptr);
-    const auto* conv_off = reinterpret_cast<const int64_t*>(get_buffer(meta, N.conv_off).ptr);
-    const auto* state_off = reinterpret_cast<const int64_t*>(get_buffer(meta, N.state_off).ptr);
-    const auto* conv_w = reinterpret_cast<const glm53f_bf16*>(get_buffer(w.o, N.conv_w).ptr);
-    const auto* a_log = reinterpret_cast<const float*>(get_buffer(w.o, N.a_log).ptr);
-    const auto* dt_bias = reinterpret_cast<const float*>(get_buffer(w.o, N.dt_bias).ptr);
-    const auto* norm_w = reinterpret_cast<const glm53f_bf16*>(get_buffer(w.o, N.norm_w).ptr);
+    const auto* cu = reinterpret_cast<const int32_t*>(get_buffer(meta, N.cu_rows, held).ptr);
+    const auto* conv_off = reinterpret_cast<const int64_t*>(get_buffer(meta, N.conv_off, held).ptr);
+    const auto* state_off = reinterpret_cast<const int64_t*>(get_buffer(meta, N.state_off, held).ptr);
+    const auto* conv_w = reinterpret_cast<const glm53f_bf16*>(get_buffer(w.o, N.conv_w, held).ptr);
+    const auto* a_log = reinterpret_cast<const float*>(get_buffer(w.o, N.a_log, held).ptr);
+    const auto* dt_bias = reinterpret_cast<const float*>(get_buffer(w.o, N.dt_bias, held).ptr);
+    const auto* norm_w = reinterpret_cast<const glm53f_bf16*>(get_buffer(w.o, N.norm_w, held).ptr);
     const float eps = (float)get_f64(w.o, N.eps), lower = (float)get_f64(w.o, N.lower);
     const glm53f_stream_t st = stream_of(stream);
     auto launch = [&](auto fn, auto* s_in, auto* s_out) {
-        return fn((int32_t)heads, (int32_t)batch, cu, p.ptr, p.stride, b_off, a.ptr, a.stride, g.ptr, g.stride, reinterpret_cast<const glm53f_bf16*>(conv.ptr),
-                  conv_off, conv_w, s_in, s_out, state_off, a_log, dt_bias, norm_w, eps, lower, out.ptr, out.stride, static_cast<float*>(ks),
-                  static_cast<glm53f_bf16*>(vs), static_cast<float*>(gs), static_cast<float*>(bs), st);
+        return unlocked([&] {
+            return fn((int32_t)heads, (int32_t)batch, cu, p.ptr, p.stride, b_off, a.ptr, a.stride, g.ptr, g.stride, reinterpret_cast<const glm53f_bf16*>(conv.ptr),
+                      conv_off, conv_w, s_in, s_out, state_off, a_log, dt_bias, norm_w, eps, lower, out.ptr, out.stride, static_cast<float*>(ks),
+                      static_cast<glm53f_bf16*>(vs), static_cast<float*>(gs), static_cast<float*>(bs), st);
+        });
     };
     if (bf16) return launch(glm53f_kda_chain_batch_bf16state, reinterpret_cast<const glm53f_bf16*>(state.ptr), static_cast<glm53f_bf16*>(state_out));
     return launch(glm53f_kda_chain_batch, reinterpret_cast<const float*>(state.ptr), static_cast<float*>(state_out));
@@ -230,16 +258,21 @@ int core_decode(PyObject* const* a) {
     const float eps = (float)PyFloat_AS_DOUBLE(a[14]);
     auto* out = need<glm53f_bf16>(a[15], kBf16, n);
     const auto st = reinterpret_cast<glm53f_stream_t>(c10::cuda::getCurrentCUDAStream().stream());
+    const void* si = state.data_ptr();
+    // (the caller's frame holds the tensors)
     if (a[16] == Py_None)
-        return glm53f_kda_core_decode_batch((int32_t)heads, (int32_t)batch, cu, q, k, v, g, beta, state.data_ptr(), so, off, kind, (int32_t)flags, gate, norm_w,
-                                            eps, out, st);
+        return unlocked([&] {
+            return glm53f_kda_core_decode_batch((int32_t)heads, (int32_t)batch, cu, q, k, v, g, beta, si, so, off, kind, (int32_t)flags, gate, norm_w, eps, out, st);
+        });
     if (!PyTuple_CheckExact(a[16]) || PyTuple_GET_SIZE(a[16]) != 4) throw Miss{};
     auto* ks = need<float>(PyTuple_GET_ITEM(a[16], 0), kF32, n);
     auto* vs = need<glm53f_bf16>(PyTuple_GET_ITEM(a[16], 1), kBf16, n);
     auto* gs = need<float>(PyTuple_GET_ITEM(a[16], 2), kF32, n);
     auto* bs = need<float>(PyTuple_GET_ITEM(a[16], 3), kF32, rows * heads);
-    return glm53f_kda_core_verify_batch((int32_t)heads, (int32_t)batch, cu, q, k, v, g, beta, state.data_ptr(), so, off, kind, (int32_t)flags, gate, norm_w, eps,
-                                        out, ks, vs, gs, bs, st);
+    return unlocked([&] {
+        return glm53f_kda_core_verify_batch((int32_t)heads, (int32_t)batch, cu, q, k, v, g, beta, si, so, off, kind, (int32_t)flags, gate, norm_w, eps, out, ks, vs,
+                                            gs, bs, st);
+    });
 }
 
 template <typename F>

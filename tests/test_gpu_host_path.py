@@ -89,3 +89,52 @@ def test_a_chain_call_with_an_error_keeps_its_error(pkg, what, text):
     with pytest.raises(K.Invalid, match="^" + text):
         call(**what)
     torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("entry", ["core", "chain"])
+def test_a_blocked_launch_does_not_stop_other_threads(pkg, entry):
+    """More launches than the queue holds behind a kernel of 0.6 s: the launch that finds it full blocks, its thread alone."""
+    import threading
+    import time
+
+    core, K = (importlib.import_module("glm53f-afd_b200." + m) for m in ("core", "kernel"))
+    h = 1
+    z = lambda n, d=torch.bfloat16: torch.zeros(n, dtype=d, device="cuda")
+    if entry == "core":
+        cu, off, q, k, v, g, beta = torch.tensor([0, 1], dtype=torch.int32, device="cuda"), z(1, torch.int64), z(128), z(128), z(128), z(128, torch.float32), z(1, torch.float32)
+        state, out = z(128 * 128, torch.float32), z(128)
+        launch = lambda: core.decode_batch(h, 1, cu, q, k, v, g, beta, state, off, out=out)
+    else:
+        c, buf = K.channels(h), lambda n, size=2: K.DeviceBuffer(z(n * size, torch.uint8))
+        w, meta, s = K.Weights(h, buf(c * 4), buf(h, 4), buf(128, 4), buf(128), 1e-5, -5.0), K.BatchMeta.new(1), K.Stream()
+        meta.set([K.Request(1, 0, 0)])
+        call = K.ChainBatch(w, K.RowView.dense(buf(c + h), c + h), c, K.RowView.dense(buf(128), 128), K.RowView.dense(buf(128), 128), buf(3 * c),
+                            buf(K.state_len(h), 4), K.StateOut.InPlace, K.RowView.dense(buf(128), 128))
+        launch = lambda: call.launch(meta, s)
+    launch()
+    torch.cuda.synchronize()
+    gaps, stop = [], threading.Event()
+
+    def tick():
+        last = time.perf_counter()
+        while not stop.is_set():
+            time.sleep(0.001)
+            now = time.perf_counter()
+            gaps.append(now - last)
+            last = now
+
+    thread = threading.Thread(target=tick)
+    thread.start()
+    try:
+        torch.cuda._sleep(1_100_000_000)
+        t0 = time.perf_counter()
+        for _ in range(6000):
+            launch()
+        blocked = time.perf_counter() - t0
+    finally:
+        stop.set()
+        thread.join()
+        torch.cuda.synchronize()
+    if blocked < 0.4:
+        pytest.skip("the queue held every launch")
+    assert max(gaps) < 0.15
