@@ -365,7 +365,7 @@ __device__ void mover_role(const Params& p, unsigned char* smem, uint64_t* bars,
         const Unit un = units.take(p);
         if (un.rows == 0 && !copy0) continue;
         // The unit's state.
-        if (!__all_sync(FULL, mbar_wait(&st_empty[st.idx], st.phase ^ 1u, ctx, kStatusWaitStateEmpty))) return;
+        if (!mbar_wait(&st_empty[st.idx], st.phase ^ 1u, ctx, kStatusWaitStateEmpty)) return;
         if (lane == 0) info[st.idx] = {un.s_elem, un.rows};
         if (p.skip_first_state && blockIdx.x == 0 && first) {
             // Diagnostic launch: nothing is copied and nobody is told, so the recurrence's wait for this state runs out.
@@ -388,7 +388,7 @@ __device__ void mover_role(const Params& p, unsigned char* smem, uint64_t* bars,
         st.next(L::kStateSlots);
         // Its rows' raw inputs.
         for (int r = 0; r < un.rows; ++r) {
-            if (!__all_sync(FULL, mbar_wait(&raw_empty[raw.idx], raw.phase ^ 1u, ctx, kStatusWaitRawEmpty))) return;
+            if (!mbar_wait(&raw_empty[raw.idx], raw.phase ^ 1u, ctx, kStatusWaitRawEmpty)) return;
             unsigned char* dst = smem + L::oRaw + raw.idx * L::kRawBytes;
             const Piece x = piece_of<MODE>(p, un, r, lane);
             const uintptr_t src = reinterpret_cast<uintptr_t>(x.src);
