@@ -61,17 +61,32 @@ def build(force: bool = False, verbose: bool = False) -> str:
     return LIB
 
 
+def host_built_for() -> str:
+    """What the host module's binary interface depends on beside its own source."""
+    import importlib.metadata
+    import sys
+
+    return f"torch {importlib.metadata.version('torch')}, python {sys.version_info.major}.{sys.version_info.minor}"
+
+
+def _host_stale(src: str) -> bool:
+    if _stale(HOST, [src, LIB, os.path.join(INCLUDE, "glm53f_kda.h")]):
+        return True
+    with open(HOST, "rb") as f:
+        return host_built_for().encode() + b"\0" not in f.read()
+
+
 def build_host(force: bool = False) -> str:
     """csrc/host_calls.cpp against Python's and torch's headers, linked to the library beside it."""
     src = os.path.join(CSRC, "host_calls.cpp")
-    if force or _stale(HOST, [src, os.path.join(INCLUDE, "glm53f_kda.h")]):
+    if force or _host_stale(src):
         import sysconfig
 
         import torch
 
         t = os.path.dirname(torch.__file__)
         cuda = os.path.dirname(os.path.dirname(nvcc()))
-        subprocess.check_call(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-I" + INCLUDE,
+        subprocess.check_call(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", f'-DHOST_BUILT_FOR="{host_built_for()}"', "-I" + INCLUDE,
                                "-I" + sysconfig.get_paths()["include"], "-isystem", os.path.join(t, "include"), "-isystem", os.path.join(cuda, "include"), src,
                                "-o", HOST, "-L" + HERE, "-l:" + os.path.basename(LIB), "-L" + os.path.join(t, "lib"), "-lc10", "-lc10_cuda", "-ltorch_python",
                                "-ltorch_cpu", "-Wl,-rpath,$ORIGIN"])

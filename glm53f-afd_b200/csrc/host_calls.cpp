@@ -340,5 +340,10 @@ PyMODINIT_FUNC PyInit__host(void) {
     NAME(kind, "kind"); NAME(rows, "rows"); NAME(k, "k"); NAME(v, "v"); NAME(b, "b"); NAME(fast, "_extent"); NAME(cu_rows, "cu_rows");
     NAME(conv_off, "conv_off"); NAME(state_off, "state_off"); NAME(stream, "stream"); NAME(cuda_stream, "cuda_stream");
 #undef NAME
-    return PyModule_Create(&module);
+    PyObject* m = PyModule_Create(&module);
+    if (m != nullptr && PyModule_AddStringConstant(m, "built_for", HOST_BUILT_FOR) != 0) {
+        Py_DECREF(m);
+        return nullptr;
+    }
+    return m;
 }

@@ -7,6 +7,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import warnings
 
 from . import _build
 
@@ -101,18 +102,33 @@ def load(path: str | None = None):
 _native = None
 
 
+class _PythonPath:
+    """Stands in for the native host path: it takes no call, so every launch goes through the Python checks and ctypes."""
+
+    core_decode = chain_batch = staticmethod(lambda *_: -1)
+    raw_stream = staticmethod(lambda _: None)
+
+
 def host():
-    """The native host path of the per-layer launches (csrc/host_calls.cpp).  Raises if it has not been built."""
+    """The native host path of the per-layer launches (csrc/host_calls.cpp).  It only saves host time: where it has not been built,
+    or for another torch or Python, the launches go the Python way, with a warning."""
     global _native
     if _native is None:
-        if not os.path.exists(_build.HOST):
-            raise RuntimeError(f"{_build.HOST} is missing: build it with `python -c 'import __graft_entry__ as g; g.build()'`")
-        import torch  # noqa: F401  its libraries are what the module links
+        try:
+            import torch  # noqa: F401  its libraries are what the module links
 
-        from . import _host as module, kernel as K
+            if not os.path.exists(_build.HOST):
+                raise ImportError(f"{_build.HOST} is missing")
+            from . import _host as module, kernel as K
 
-        module.bind(K.DeviceBuffer, K.RowView, K.Weights, K.Saves, K.ChainBatch, K.BatchMeta, K.Stream)
-        _native = module
+            if module.built_for != _build.host_built_for():
+                raise ImportError(f"built for {module.built_for}")
+            module.bind(K.DeviceBuffer, K.RowView, K.Weights, K.Saves, K.ChainBatch, K.BatchMeta, K.Stream)
+            _native = module
+        except (ImportError, AttributeError) as e:
+            warnings.warn(f"native host path not available ({e}): launches go through ctypes; build it with "
+                          "`python -c 'import __graft_entry__ as g; g.build()'`", RuntimeWarning, stacklevel=2)
+            _native = _PythonPath
     return _native
 
 

@@ -138,3 +138,24 @@ def test_a_blocked_launch_does_not_stop_other_threads(pkg, entry):
     if blocked < 0.4:
         pytest.skip("the queue held every launch")
     assert max(gaps) < 0.15
+
+
+def test_launches_without_the_native_module(pkg, monkeypatch):
+    """The same call through the native path and through the Python checks and ctypes."""
+    ffi, K = (importlib.import_module("glm53f-afd_b200." + m) for m in ("ffi", "kernel"))
+    h, got = 2, []
+    g = torch.Generator(device="cuda").manual_seed(1)
+    c, width = K.channels(h), h * 128
+    buf = lambda m, s=1.0, d=torch.bfloat16: K.DeviceBuffer((torch.randn(m, device="cuda", generator=g) * s).to(d).view(torch.uint8))
+    w = K.Weights(h, buf(c * 4, 0.5), buf(h, 0.5, torch.float32), buf(width, 1.0, torch.float32), buf(128), 1e-5, -5.0)
+    p, gates, conv, state, meta = buf(c + h), buf(2 * width), buf(3 * c), buf(K.state_len(h), 0.3, torch.float32), K.BatchMeta.new(1)
+    meta.set([K.Request(1, 0, 0)])
+    for native in (True, False):
+        if not native:
+            monkeypatch.setattr(ffi, "_native", ffi._PythonPath)
+        st, out = K.DeviceBuffer(state.t.clone()), K.DeviceBuffer.zeroed(2 * width)
+        K.ChainBatch(w, K.RowView.dense(p, c + h), c, K.RowView.new(gates, 0, width), K.RowView.new(gates, width, width), conv, st, K.StateOut.InPlace,
+                     K.RowView.dense(out, width)).launch(meta, K.Stream())
+        torch.cuda.synchronize()
+        got.append((out.t, st.t))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1]) and got[0][0].any()
