@@ -335,7 +335,7 @@ constexpr int kFewRows = 64;        // launches of up to this many rows run here
 // ... and a K-split shape by itself up to here: its splits run side by side on a cluster, on a pair one after another (o_proj at
 // 128 rows: 36 us on pairs, 24 so)
 constexpr int kFewRowsSplit = 128;
-constexpr int kSplitRowsMax = 512;  // ... and up to this many keep the K split's summation order
+constexpr int kSplitRowsMax = 512;  // ... and every launch of up to this many keeps the K split's summation order (see k_segments)
 
 // A [groups][rows][k] bf16 matrix (row stride ld, group stride gstride, in elements) as a 3-D map with boxes of
 // 64 k x box_rows rows in the 128-byte swizzle; rows past the extent read as zero.  The dimensions are ordered by
@@ -446,8 +446,13 @@ int pick_row_tile(long long feature_tiles, int rows, int kblocks, int most) {
     return best;
 }
 
+// The parts k is summed in.  Above 512 rows a launch whose tiles of 128 features x 256 rows fill the GPU runs k in one go; the others
+// keep the parts of a small launch, and with them its bits (the 4096 -> 256 factor at any row count, o_proj up to 1,024 rows: 41 to
+// 44 us for 513 to 768 rows and 64 us for 1,024, against 38 to 41 and 50 in one go).
 int k_segments(const glm53f_proj_job& j) {
-    return j.rows <= kSplitRowsMax ? pick_ksplit((long long)j.groups * ((j.n + kBM - 1) / kBM), j.k / kBK, sm_count()) : 1;
+    const long long feature_tiles = (long long)j.groups * ((j.n + kBM - 1) / kBM);
+    if (j.rows > kSplitRowsMax && feature_tiles * ((j.rows + 255) / 256) >= sm_count()) return 1;
+    return pick_ksplit(feature_tiles, j.k / kBK, sm_count());
 }
 
 bool pair_problem(PairProblem& q, const glm53f_proj_job& j) {
@@ -461,7 +466,8 @@ bool pair_problem(PairProblem& q, const glm53f_proj_job& j) {
     q.out_f32 = j.out_f32 != 0;
     q.segments = k_segments(j);
     q.n_tiles = (j.n + 2 * kBM - 1) / (2 * kBM);
-    q.row_tile = pick_row_tile((long long)j.groups * q.n_tiles, j.rows, q.kblocks, q.segments > 1 ? 128 : 256);
+    // Segmented tiles of more than 128 rows have a slower instance of the kernel: only where one round of them replaces two or more.
+    q.row_tile = pick_row_tile((long long)j.groups * q.n_tiles, j.rows, q.kblocks, q.segments == 1 ? 256 : j.rows > kSplitRowsMax ? kPairSplitRows : 128);
     q.r_tiles = (j.rows + q.row_tile - 1) / q.row_tile;
     q.tiles = (long long)j.groups * q.n_tiles * q.r_tiles;
     if (q.tiles > 0x3fffffff) return false;

@@ -21,6 +21,7 @@ struct PairProblem {
 };
 
 constexpr int kPairProblems = 2;
+constexpr int kPairSplitRows = 192;  // rows per tile at most when k runs in segments
 // proj_gemm_pair.cu: launches the tiles of n (1 or 2) problems.
 int proj_gemm_pair_launch(const PairProblem* problems, int n, int* status, cudaStream_t stream);
 
