@@ -55,14 +55,13 @@ def bf16(x: torch.Tensor, ldx: int, x_gstride: int, w: Bf16Mat, rows: int, out: 
     """out[g][m][o] = sum_k x[g][m][k] w[g][o][k] (Gemm::bf16, gemm.rs:212-235); offsets in elements of x / out."""
     if rows == 0:
         return
-    j = _job(x, ldx, x_gstride, w, rows, out, ldo, o_gstride, out_f32, x_offset, out_offset)
-    stream = torch.cuda.current_stream().cuda_stream
-    code = ffi.glm53f_kda_proj_bf16(*(getattr(j, f) for f, _ in j._fields_), stream)
+    job = _job(x, ldx, x_gstride, w, rows, out, ldo, o_gstride, out_f32, x_offset, out_offset)
+    code = ffi.load().glm53f_kda_proj_bf16(*job, torch.cuda.current_stream().cuda_stream)
     _launched(code, "glm53f_kda_proj_bf16")
 
 
-def _job(x, ldx, x_gstride, w: Bf16Mat, rows, out, ldo, o_gstride, out_f32=False, x_offset=0, out_offset=0) -> ffi.ProjJob:
-    """The checked arguments of one GEMM."""
+def _job(x, ldx, x_gstride, w: Bf16Mat, rows, out, ldo, o_gstride, out_f32=False, x_offset=0, out_offset=0) -> tuple:
+    """The checked arguments of one GEMM: those of glm53f_kda_proj_bf16 before the stream, the fields of ffi.ProjJob."""
     if x.dtype not in (torch.bfloat16, torch.int16, torch.uint16) or w.t.dtype not in (torch.bfloat16, torch.int16, torch.uint16):
         raise Invalid("x and the weight are bf16")
     if out.dtype != (torch.float32 if out_f32 else x.dtype) and not (not out_f32 and out.element_size() == 2):
@@ -71,8 +70,8 @@ def _job(x, ldx, x_gstride, w: Bf16Mat, rows, out, ldo, o_gstride, out_f32=False
     need_o = out_offset + (w.groups - 1) * o_gstride + (rows - 1) * ldo + w.n
     if x.numel() < need_x or out.numel() < need_o or w.t.numel() < (w.groups - 1) * w.gstride + (w.n - 1) * w.ld + w.k:
         raise Invalid("a buffer is smaller than the shapes named")
-    return ffi.ProjJob(x.data_ptr() + 2 * x_offset, ldx, x_gstride, w.t.data_ptr(), w.ld, w.gstride, w.groups, rows, w.n, w.k,
-                       out.data_ptr() + out_offset * out.element_size(), 1 if out_f32 else 0, ldo, o_gstride)
+    return (x.data_ptr() + 2 * x_offset, ldx, x_gstride, w.t.data_ptr(), w.ld, w.gstride, w.groups, rows, w.n, w.k,
+            out.data_ptr() + out_offset * out.element_size(), 1 if out_f32 else 0, ldo, o_gstride)
 
 
 @dataclass
@@ -95,7 +94,7 @@ def kda_input_projections(normed: torch.Tensor, rows: int, w: KdaProjW, p: torch
     apart = _disjoint(p, fga) and _disjoint(p, normed) and _disjoint(fga, normed)
     stream = torch.cuda.current_stream().cuda_stream
     if apart:  # the first gate factor beside the fused projection of the same rows
-        _launched(ffi.glm53f_kda_proj_bf16_many((ffi.ProjJob * 2)(*both), 2, stream), "glm53f_kda_proj_bf16_many")
+        _launched(ffi.glm53f_kda_proj_bf16_many((ffi.ProjJob * 2)(*(ffi.ProjJob(*j) for j in both)), 2, stream), "glm53f_kda_proj_bf16_many")
     else:
         bf16(normed, HIDDEN, 0, w.qkvb, rows, p, KDA_P_COLS, 0)
         bf16(normed, HIDDEN, 0, w.fga, rows, fga, 2 * KDA_DIM, 0)
