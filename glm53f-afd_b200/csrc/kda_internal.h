@@ -64,6 +64,7 @@ constexpr int kPrefillSlotBytes = 107008, kPrefillTailBytes = 256;
 // The workspace's last 256 bytes, as words: two item counters | a single request's metadata (an offset, cu_rows) | from word 8
 // on two sets, which consecutive launches use in turn: items and chains handed out, and finished items per group of chains.
 constexpr int kTailMeta = 2, kTailSets = 8, kTailSet = 28, kTailGroups = kTailSet - 2;
+static_assert(kPrefillTailBytes == 4 * 64 && kTailSets + 2 * kTailSet == 64, "the workspace's tail");
 constexpr int kSlotInK = 0, kSlotInV = 16384, kSlotInQ = 32768, kSlotInG = 49152, kSlotInBeta = 81920;
 __host__ __device__ inline int prefill_box_piece(int r, int piece) { return (piece >> 3) * 8192 + r * 128 + (((piece & 7) ^ (r & 7)) << 4); }
 
@@ -99,11 +100,12 @@ int commit_tc_launch(int32_t heads, int32_t layers, int32_t batch, const int32_t
 
 // The layer prologue of a prefill pass (kda_prologue.cu): for chunks chunk0 .. chunk0 + chunks - 1 (of 64 rows) of every
 // request, the short convolution + SiLU, the L2 norms, the log decay and beta, written as core inputs into the slots
-// [batch][heads][chunks].  p, a, conv must be 8-byte aligned with strides that are multiples of 4 elements.
+// [batch][heads][chunks].  p and a must be 8-byte aligned with strides that are multiples of 4 elements.  The first pass also clears
+// the counters in the workspace's tail.
 int layer_prologue_launch(int32_t heads, int32_t batch, const int32_t* cu_rows, int32_t chunks, int32_t chunk0,
                           const glm53f_bf16* p, int64_t p_stride, int64_t b_off, const glm53f_bf16* a, int64_t a_stride,
                           const glm53f_bf16* conv, const int64_t* conv_off, const glm53f_bf16* conv_w, const float* a_log,
-                          const float* dt_bias, float lower, unsigned char* slots, cudaStream_t stream);
+                          const float* dt_bias, float lower, unsigned char* slots, unsigned int* tail, cudaStream_t stream);
 // The pass itself, both roles, from those slots (kda_prefill_sp.cu).  `tail`: the workspace's
 // tail, its sets zero before the first pass.
 int layer_pass_launch(int32_t heads, int32_t batch, const int32_t* cu_rows, int32_t chunks, int32_t chunk0, unsigned char* slots,

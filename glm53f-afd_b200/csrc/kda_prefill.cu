@@ -36,12 +36,9 @@ std::atomic<int> g_layer_prefill_mode{[] {
 
 constexpr int kNotEligible = -1;
 
-// The workspace's tail: the passes' item counters, and the batch metadata of a single-request call (the kernels read metadata
-// on the device).
-__global__ void prefill_tail(unsigned int* tail, int32_t rows) {
-    static_assert(kPrefillTailBytes == 4 * 64 && kTailSets + 2 * kTailSet == 64, "the workspace's tail");
-    tail[threadIdx.x] = threadIdx.x == kTailMeta + 3 ? (unsigned)rows : 0u;
-}
+// The batch metadata of a single-request call, in the workspace's tail (the kernels read metadata on the device): an offset of zero,
+// cu_rows.
+__global__ void single_request_meta(unsigned int* meta, int32_t rows) { meta[threadIdx.x] = threadIdx.x == 3 ? (unsigned)rows : 0u; }
 
 // The chunked form.  The workspace holds the slots of one pass: as many 64-row chunks of every request as fit, the passes of
 // equal length (chunks count from a request's first row, so the results do not depend on the workspace size).  Returns
@@ -68,14 +65,14 @@ int chunked_layer_prefill(int32_t heads, int32_t batch, const int32_t* cu_rows, 
     pass = (need + passes - 1) / passes;
     unsigned char* slots = reinterpret_cast<unsigned char*>(workspace);
     unsigned int* tail = reinterpret_cast<unsigned int*>(slots + usable);
-    prefill_tail<<<1, 64, 0, st>>>(tail, max_rows);
     if (cu_rows == nullptr) {
+        single_request_meta<<<1, 4, 0, st>>>(tail + kTailMeta, max_rows);
         cu_rows = reinterpret_cast<int32_t*>(tail + kTailMeta + 2);
         conv_off = state_off = reinterpret_cast<const int64_t*>(tail + kTailMeta);
     }
     for (int64_t chunk0 = 0; chunk0 < need; chunk0 += pass) {
         int rc = layer_prologue_launch(heads, batch, cu_rows, (int)pass, (int)chunk0, p, p_stride, b_off, a, a_stride, conv, conv_off, conv_w, a_log,
-                                       dt_bias, lower, slots, st);
+                                       dt_bias, lower, slots, tail, st);
         if (rc != 0) return rc;
         rc = layer_pass_launch(heads, batch, cu_rows, (int)pass, (int)chunk0, slots, tail, state_in, state_out, state_off, bf16_state, g, g_stride, norm_w,
                                eps, out, st);

@@ -57,6 +57,7 @@ struct ProParams {
     const float* dt_bias;
     float lower;
     unsigned char* slots;  // prefill pass: [batch][H][pass_rows / 64]
+    unsigned int* tail;    // the workspace's tail
     // verify: q as fp16 into the output rows, the rest into the replay saves
     uint16_t* q;
     long long out_stride;
@@ -238,6 +239,8 @@ __global__ void __launch_bounds__(128, 5) prefill_prologue_kernel(const ProParam
     // heads innermost: neighbouring blocks read neighbouring pieces of the same rows
     const int h = (int)(blockIdx.x % H), b = (int)(blockIdx.x / H / groups), j0 = (int)(blockIdx.x / H % groups) * 4 * kRowsPer + (threadIdx.x >> 5) * kRowsPer;
     const int r0 = p.cu[b], n = min(p.cu[b + 1] - r0 - p.row_shift, p.pass_rows);
+    // The passes' counters start from zero (as a launch of its own this was 2 us of a short prompt's 50).
+    if (FIRST && blockIdx.x == 0 && threadIdx.x < 2 * kTailSet) p.tail[kTailSets + threadIdx.x] = 0u;
     if (j0 >= n) return;
     const int first = p.row_shift + j0, last = p.row_shift + n - 1;  // rows of the request; rows before its first come from the conv window
     const long long C = 3LL * H * DK;
@@ -350,7 +353,7 @@ int launch(const ProParams& pp, cudaStream_t stream) {
 int layer_prologue_launch(int32_t heads, int32_t batch, const int32_t* cu_rows, int32_t chunks, int32_t chunk0,
                           const glm53f_bf16* p, int64_t p_stride, int64_t b_off, const glm53f_bf16* a, int64_t a_stride,
                           const glm53f_bf16* conv, const int64_t* conv_off, const glm53f_bf16* conv_w, const float* a_log,
-                          const float* dt_bias, float lower, unsigned char* slots, cudaStream_t stream) {
+                          const float* dt_bias, float lower, unsigned char* slots, unsigned int* tail, cudaStream_t stream) {
     ProParams pp{};
     pp.H = heads; pp.batch = batch; pp.pass_rows = chunks * 64; pp.row_shift = chunk0 * 64;
     pp.cu = cu_rows;
@@ -359,6 +362,7 @@ int layer_prologue_launch(int32_t heads, int32_t batch, const int32_t* cu_rows, 
     pp.conv = conv; pp.conv_off = reinterpret_cast<const long long*>(conv_off); pp.cw = conv_w;
     pp.a_log = a_log; pp.dt_bias = dt_bias; pp.lower = lower;
     pp.slots = slots;
+    pp.tail = tail;
     const long long blocks = (long long)batch * heads * (pp.pass_rows / (4 * kRowsPer));
     if (blocks > 0x7fffffffLL) return kInvalid;
     if (chunk0 == 0) prefill_prologue_kernel<true><<<(unsigned)blocks, 128, 0, stream>>>(pp);
