@@ -517,7 +517,12 @@ __device__ void prologue_role(const Params& p, unsigned char* smem, uint64_t* ba
 // A warp skips the others' rows, so it has not itself seen the row that held the raw slot before, whose copy may land after later
 // rows' copies: raw_full can be a phase behind what its parity says.  So every row waits for its cooked slot first.  The two rings
 // are equally deep, and that slot is free only when the row before has been through the whole pipeline, its raw copy included.
-template <typename S>
+//
+// A launch of one unit a block (ONE_UNIT, an instance of the kernel to itself: the rule inside cost 16 single-row slots 1.5 %) waits for its
+// first rows, and there four warps on a row are the shorter way: windows of 2, 4 and 8 rows of one slot 7.9, 10.6 and 15.4 us with
+// a row per warp, 6.6, 9.3 and 14.7 so (two units a block, 4 rows: 16.4 against 17.2).
+constexpr int kTogetherRows = 8;
+template <typename S, bool ONE_UNIT>
 __device__ void layer_prologue_role(const Params& p, unsigned char* smem, uint64_t* bars, const WaitCtx& ctx, int warp, int lane) {
     using L = Smem<S, kLayer>;
     uint64_t* raw_full = bars + 2 * L::kStateSlots;
@@ -528,6 +533,7 @@ __device__ void layer_prologue_role(const Params& p, unsigned char* smem, uint64
     const bool copy0 = copies_state(p);
     const bool vec = ((reinterpret_cast<uintptr_t>(p.cw) | reinterpret_cast<uintptr_t>(p.dt_bias)) & 15) == 0;
     UnitIter<kLayer> units(p);
+    constexpr int together = ONE_UNIT ? kTogetherRows : 1;
     int turn = 0;
     // A warp whose wait gave up does not leave: the single-row units further on are cooked by all four warps, which meet there at
     // barriers.  It takes no more rows and goes on through the units to the next vote, which then sends all four home.
@@ -541,10 +547,10 @@ __device__ void layer_prologue_role(const Params& p, unsigned char* smem, uint64
     while (units.valid()) {
         const Unit un = units.take(p);
         if (un.rows == 0 && !copy0) continue;
-        if (un.rows == 1) {
+        if (un.rows <= together) {
             // A single row is cooked by all four warps, a thread a channel: with one row a unit the next state is waited for anyway,
             // and the row's latency counts (16 slots, bf16: 0.670 ms a step of 34 layers, 0.696 with a row per warp; 1 slot 0.215
-            // against 0.263).
+            // against 0.263).  ONE_UNIT: so are up to eight, there being no other unit's rows to work on meanwhile.
             const int c = warp * 32 + lane;
             uint2 w[3];
 #pragma unroll
@@ -553,37 +559,37 @@ __device__ void layer_prologue_role(const Params& p, unsigned char* smem, uint64
                 w[part] = vec ? *reinterpret_cast<const uint2*>(cw) : make_uint2((uint32_t)cw[0] | ((uint32_t)cw[1] << 16), (uint32_t)cw[2] | ((uint32_t)cw[3] << 16));
             }
             const float db = p.dt_bias[(long long)un.h * DK + c], decay_rate = expf(un.a_log);
-            const bool ready = !dead && mbar_wait(&row_empty[row.idx], row.phase ^ 1u, ctx, kStatusWaitRowEmpty) && mbar_wait(&raw_full[raw.idx], raw.phase, ctx, kStatusWaitRawFull);
-            const unsigned char* in = smem + L::oRaw + raw.idx * L::kRawBytes;
-            Cooked& ck = *reinterpret_cast<Cooked*>(smem + L::oCooked + row.idx * sizeof(Cooked));
-            float* scratch = reinterpret_cast<float*>(smem + L::oScratch);
-            if (ready) {
-                const uint16_t* x = reinterpret_cast<const uint16_t*>(in + RawLayer::X);
+            for (int r = 0; r < un.rows; ++r, raw.next(L::kRawSlots), row.next(L::kRowSlots)) {
+                const bool ready = !dead && mbar_wait(&row_empty[row.idx], row.phase ^ 1u, ctx, kStatusWaitRowEmpty) && mbar_wait(&raw_full[raw.idx], raw.phase, ctx, kStatusWaitRawFull);
+                const unsigned char* in = smem + L::oRaw + raw.idx * L::kRawBytes;
+                Cooked& ck = *reinterpret_cast<Cooked*>(smem + L::oCooked + row.idx * sizeof(Cooked));
+                float* scratch = reinterpret_cast<float*>(smem + L::oScratch);
+                if (ready) {
+                    const uint16_t* x = reinterpret_cast<const uint16_t*>(in + RawLayer::X);
 #pragma unroll
-                for (int part = 0; part < 3; ++part) {
-                    float wt[TAPS], acc = 0.0f;
-                    widen(w[part], wt);
+                    for (int part = 0; part < 3; ++part) {
+                        float wt[TAPS], acc = 0.0f;
+                        widen(w[part], wt);
 #pragma unroll
-                    for (int tap = 0; tap < TAPS; ++tap) acc = acc + wt[tap] * bf16_bits_to_f32(x[(tap * 3 + part) * DK + c]);
-                    (part == 2 ? ck.v : scratch + part * DK)[c] = bf16_round(acc / (1.0f + expf(-acc)));
+                        for (int tap = 0; tap < TAPS; ++tap) acc = acc + wt[tap] * bf16_bits_to_f32(x[(tap * 3 + part) * DK + c]);
+                        (part == 2 ? ck.v : scratch + part * DK)[c] = bf16_round(acc / (1.0f + expf(-acc)));
+                    }
+                }
+                if (!named_bar_all(1, kProThreadsOf<kLayer>, ready)) return;  // all four leave together
+                if (warp == 0) l2norm_warp(scratch, ck.q, lane, true);
+                else if (warp == 1) l2norm_warp(scratch + DK, ck.k, lane, false);
+                else if (warp == 2 && lane == 0) {
+                    const uintptr_t addr = reinterpret_cast<uintptr_t>(p.P + (un.row0 + r) * p.p_stride + p.b_off + un.h);
+                    ck.beta = bf16_round(sigmoidf_(bf16_bits_to_f32(*reinterpret_cast<const uint16_t*>(in + RawLayer::B + (addr & 15)))));
+                }
+                ck.g[c] = expf(p.lower * sigmoidf_(decay_rate * (bf16_bits_to_f32(reinterpret_cast<const uint16_t*>(in + RawLayer::A)[c]) + db)));
+                ck.sg[c] = sigmoidf_(bf16_bits_to_f32(reinterpret_cast<const uint16_t*>(in + RawLayer::GATE)[c]));
+                named_bar_sync(2, kProThreadsOf<kLayer>);
+                if (warp == 0 && lane == 0) {
+                    mbar_arrive(&row_full[row.idx]);
+                    mbar_arrive(&raw_empty[raw.idx]);
                 }
             }
-            if (!named_bar_all(1, kProThreadsOf<kLayer>, ready)) return;  // all four leave together
-            if (warp == 0) l2norm_warp(scratch, ck.q, lane, true);
-            else if (warp == 1) l2norm_warp(scratch + DK, ck.k, lane, false);
-            else if (warp == 2 && lane == 0) {
-                const uintptr_t addr = reinterpret_cast<uintptr_t>(p.P + un.row0 * p.p_stride + p.b_off + un.h);
-                ck.beta = bf16_round(sigmoidf_(bf16_bits_to_f32(*reinterpret_cast<const uint16_t*>(in + RawLayer::B + (addr & 15)))));
-            }
-            ck.g[c] = expf(p.lower * sigmoidf_(decay_rate * (bf16_bits_to_f32(reinterpret_cast<const uint16_t*>(in + RawLayer::A)[c]) + db)));
-            ck.sg[c] = sigmoidf_(bf16_bits_to_f32(reinterpret_cast<const uint16_t*>(in + RawLayer::GATE)[c]));
-            named_bar_sync(2, kProThreadsOf<kLayer>);
-            if (warp == 0 && lane == 0) {
-                mbar_arrive(&row_full[row.idx]);
-                mbar_arrive(&raw_empty[raw.idx]);
-            }
-            raw.next(L::kRawSlots);
-            row.next(L::kRowSlots);
             continue;
         }
         for (int r = 0; r < un.rows; ++r, raw.next(L::kRawSlots), row.next(L::kRowSlots)) {
@@ -801,7 +807,7 @@ __device__ void epilogue_role(const Params& p, unsigned char* smem, uint64_t* ba
 }
 
 // ---- the kernel ----------------------------------------------------------------------------------------------
-template <typename S, int MODE>
+template <typename S, int MODE, bool ONE_UNIT = false>
 __global__ void __launch_bounds__(kThreadsOf<MODE>, 1) recurrent_kernel(const __grid_constant__ Params p) {
     using L = Smem<S, MODE>;
     constexpr int kProWarps = kProWarpsOf<MODE>, kProThreads = kProThreadsOf<MODE>;
@@ -832,7 +838,7 @@ __global__ void __launch_bounds__(kThreadsOf<MODE>, 1) recurrent_kernel(const __
     if (warp < kRecWarps) {
         recurrence_role<S, MODE>(p, smem, bars, ctx, warp, lane);
     } else if (warp < kRecWarps + kProWarps) {
-        if constexpr (MODE == kLayer) layer_prologue_role<S>(p, smem, bars, ctx, warp - kRecWarps, lane);
+        if constexpr (MODE == kLayer) layer_prologue_role<S, ONE_UNIT>(p, smem, bars, ctx, warp - kRecWarps, lane);
         else prologue_role<S, MODE>(p, smem, bars, ctx, tid - kRecThreads);
     } else if (warp == kRecWarps + kProWarps) {
         if (MODE != kReplay) epilogue_role<S, MODE>(p, smem, bars, ctx, lane);
@@ -1016,20 +1022,23 @@ int launch_replay_small(const Params& p, cudaStream_t stream) {
     return (int)cudaLaunchKernelEx(&cfg, replay_small_kernel<S>, q);
 }
 
-template <typename S, int MODE>
+template <typename S, int MODE, bool ONE_UNIT = false>
 int launch(const Params& p, cudaStream_t stream) {
     using L = Smem<S, MODE>;
+    const long long sms = sm_count();
+    if constexpr (MODE == kLayer && !ONE_UNIT) {
+        if (p.units <= sms) return launch<S, MODE, true>(p, stream);
+    }
     static bool configured = false;  // per process; the attribute is per device, so set it on every device change
     static int configured_dev = -1;
     int dev = 0;
     cudaGetDevice(&dev);
     if (!configured || configured_dev != dev) {
-        const cudaError_t e = cudaFuncSetAttribute(recurrent_kernel<S, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kBytes);
+        const cudaError_t e = cudaFuncSetAttribute(recurrent_kernel<S, MODE, ONE_UNIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kBytes);
         if (e != cudaSuccess) return (int)e;
         configured = true;
         configured_dev = dev;
     }
-    const long long sms = sm_count();
     const unsigned grid = (unsigned)(p.units < sms ? p.units : sms);
     Params q = p;
     q.neg_zero2 = 0x8000000080000000ull;
@@ -1052,7 +1061,7 @@ int launch(const Params& p, cudaStream_t stream) {
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl ? 1 : 0;
-    return (int)cudaLaunchKernelEx(&cfg, recurrent_kernel<S, MODE>, q);
+    return (int)cudaLaunchKernelEx(&cfg, recurrent_kernel<S, MODE, ONE_UNIT>, q);
 }
 
 template <int MODE>

@@ -11,9 +11,10 @@ DK = 128
 
 
 # As many heads as SMs: block 0 has (0, head 0) and then a unit of the next request.  Rows beyond the ring
-# (5 rows with f32 states, 8 with bf16) put the waits that run out into different warps; [2, 1, 9] ends among single rows.
+# (5 rows with f32 states, 8 with bf16) put the waits that run out into different warps; [2, 1, 9] ends among single rows; one request alone
+# is a launch of one unit a block.
 @pytest.mark.parametrize("state", ["f32", "bf16"])
-@pytest.mark.parametrize("lens", [[6, 1], [9, 1, 1], [11, 1], [2, 1, 9], [8, 3, 1]])
+@pytest.mark.parametrize("lens", [[6, 1], [9, 1, 1], [11, 1], [2, 1, 9], [8, 3, 1], [8], [9]])
 def test_every_warp_leaves_when_a_wait_runs_out(pkg, lens, state):
     if not torch.cuda.is_available():
         pytest.skip("no CUDA device")
