@@ -398,7 +398,8 @@ int glm53f_kda_gather_close(const glm53f_kda_gather_handle* handle, void* full);
  *      workspace; results agree with the chain to the rounding of bf16 operands (the task's tolerances: bf16 outputs
  *      within 2e-2 max-abs / 5e-3 rel-L2, state within 1e-3 rel-L2) and do not depend on the workspace size or the
  *      batching; `value_blocks` is not used.  Calls the chunked kernels cannot take (output rows that are not dense,
- *      rows not 8-byte aligned, a workspace below 64 rows a pass) run the exact form.
+ *      rows not 8-byte aligned, a workspace of fewer than 33 rows a pass by glm53f_kda_prefill_workspace_bytes, or for
+ *      one or two requests fewer than 49) run the exact form.
  * Any other value only queries.  Returns the mode that was in force.  The environment variable
  * GLM53F_KDA_PREFILL=chunked makes 1 the initial mode.  Process-wide; set it before the launches it should affect. */
 int32_t glm53f_kda_prefill_mode(int32_t mode);
