@@ -417,6 +417,9 @@ class Request:
     state_offset: int
 
 
+STORE_WORDS = 4000  # glm53f_kda_store_words carries 1,000 a launch (2 us); a copy that waits takes about 20 us
+
+
 class BatchMeta:
     """Batch metadata on the device -- row ranges, offsets and kept rows -- with a host copy for the checks
     (kernel.rs:409-526)."""
@@ -444,7 +447,9 @@ class BatchMeta:
     def set(self, requests: Sequence[Request], keep: Optional[Sequence[int]] = None) -> None:
         """Set the requests and, for replays and conv shifts, the rows each keeps (None: all).  Copies to the device
         synchronously."""
-        image = self._set(requests, keep)
+        self._upload(self._set(requests, keep))
+
+    def _upload(self, image: np.ndarray) -> None:
         torch = _torch()
         self._all.t.copy_(torch.from_numpy(image.view(np.uint8)))
         if self._all.t.is_cuda:
@@ -458,6 +463,9 @@ class BatchMeta:
         image = self._set(requests, keep)
         if wait is not None:
             wait(stream)
+        if image.size > STORE_WORDS:  # capacities of many hundreds of requests: one copy, when the launches before have run
+            _torch().cuda.synchronize()
+            return self._upload(image)
         _launched(ffi.glm53f_kda_store_words(self._all.ptr(), image.ctypes.data, image.size, stream.raw()), "glm53f_kda_store_words")
 
     def _set(self, requests: Sequence[Request], keep: Optional[Sequence[int]]) -> np.ndarray:

@@ -159,3 +159,24 @@ def test_launches_without_the_native_module(pkg, monkeypatch):
         torch.cuda.synchronize()
         got.append((out.t, st.t))
     assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1]) and got[0][0].any()
+
+
+@pytest.mark.parametrize("capacity", [1, 3, 166, 167, 700, 5000])
+def test_metadata_in_stream_order(pkg, capacity):
+    """BatchMeta.set_on at the edges of what a launch and a few launches carry: the device holds what `set` puts there, and a
+    launch queued before still reads what was there then."""
+    K = importlib.import_module("glm53f-afd_b200.kernel")
+    n = min(capacity, 600)
+    first, second = ([K.Request(1 + (i + s) % 3, 8 * i + s, 64 * i + s) for i in range(n)] for s in (0, 5))
+    metas = [K.BatchMeta.new(capacity) for _ in range(2)]
+    metas[0].set(first)
+    metas[1].set(first)
+    was = metas[0]._all.t.clone()
+    torch.cuda.synchronize()
+    torch.cuda._sleep(20_000_000)
+    seen = metas[0]._all.t.clone()  # in stream order, ahead of the new metadata
+    metas[0].set_on(second, [1] * n, K.Stream())
+    metas[1].set(second, [1] * n)
+    torch.cuda.synchronize()
+    assert torch.equal(seen, was) and torch.equal(metas[0]._all.t, metas[1]._all.t) and not torch.equal(was, seen.new_zeros(()).expand_as(was))
+    assert metas[0]._extent == metas[1]._extent and metas[0].requests() == second
