@@ -1091,11 +1091,11 @@ int chain_entry(int32_t heads, int32_t batch, bool batched, const int32_t* cu_ro
         return kInvalid;
     }
     if (batched && bf16_state && state_out == nullptr && k_save != nullptr && keep == nullptr && g_layer_verify_mode.load() == 1) {
-        // The chunked form of a verify call: eligible when every row the two kernels touch by vector is aligned; any
-        // other call runs the exact form below.
+        // The chunked form of a verify call: eligible when every row the two kernels touch by vector is aligned and the outputs,
+        // which hold q between them, do not go over the gate rows; any other call runs the exact form below.
         auto al = [](const void* x, int bytes) { return (reinterpret_cast<uintptr_t>(x) & (bytes - 1)) == 0; };
         if (al(p, 8) && al(a, 8) && al(g, 8) && al(conv, 8) && al(conv_w, 16) && al(dt_bias, 16) && al(out, 16) && al(k_save, 16) && al(v_save, 16) &&
-            al(g_save, 16) && al(state_in, 16) && p_stride % 4 == 0 && a_stride % 4 == 0 && g_stride % 4 == 0 && out_stride % 8 == 0) {
+            al(g_save, 16) && al(state_in, 16) && (out != g || out_stride != g_stride) && p_stride % 4 == 0 && a_stride % 4 == 0 && g_stride % 4 == 0 && out_stride % 8 == 0) {
             cudaStream_t st = (cudaStream_t)stream;
             const int rc = verify_prologue_launch(heads, batch, cu_rows, p, p_stride, b_off, a, a_stride, conv, conv_off, conv_w, a_log, dt_bias,
                                                   lower, out, out_stride, k_save, v_save, g_save, b_save, st);

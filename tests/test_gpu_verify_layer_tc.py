@@ -10,6 +10,7 @@ bf16 path, 5e-2 of max|ref| (crates/glm53f-kda/src/goldens.rs:756-761), and with
 gates as in crates/glm53f-kda/tests/cpu_reference.rs:399-450.
 """
 import ctypes as C
+import importlib
 
 import numpy as np
 import pytest
@@ -184,3 +185,26 @@ def test_the_mode_switch_reports_and_restores(G):
     assert lib.glm53f_kda_verify_mode(7) == 1    # any other value only queries
     assert lib.glm53f_kda_verify_mode(0) == 1
     assert lib.glm53f_kda_verify_mode(-1) == 0
+
+
+def test_outputs_over_the_gate_rows_run_the_exact_form():
+    K = importlib.import_module("glm53f-afd_b200.kernel")
+    h, lens, g = 2, [3, 8], torch.Generator(device="cuda").manual_seed(2)
+    c, width, total = K.channels(h), h * 128, sum(lens)
+    rn = lambda m, s=1.0, d=torch.bfloat16: (torch.randn(m, device="cuda", generator=g) * s).to(d)
+    buf = lambda t: K.DeviceBuffer(t.view(torch.uint8))
+    w = K.Weights(h, buf(rn(c * 4, 0.5)), buf(rn(h, 0.5, torch.float32)), buf(rn(width, 1.0, torch.float32)), buf(1 + rn(128, 0.1)), 1e-5, -5.0)
+    p, a, gate, conv, state = rn(total * (c + 8)), rn(total * width), rn(total * width), rn(2 * 3 * c), rn(2 * K.state_len(h), 0.3)
+    meta, outs = K.BatchMeta.new(2), []
+    meta.set([K.Request(r, i * 3 * c, i * K.state_len(h)) for i, r in enumerate(lens)])
+    for form, over in ((K.Form.EXACT, False), (K.Form.CHUNKED, True)):
+        before, gates = K.set_verify_form(form), gate.clone()
+        out = gates if over else torch.zeros_like(gates)
+        try:
+            K.ChainBatch(w, K.RowView.dense(buf(p), c + 8), c, K.RowView.dense(buf(a), width), K.RowView.dense(buf(gates), width), buf(conv), buf(state),
+                         K.StateOut.Skip, K.RowView.dense(buf(out), width), K.Saves.alloc(h, total)).launch_bf16_state(meta, K.Stream())
+            torch.cuda.synchronize()
+        finally:
+            K.set_verify_form(before)
+        outs.append(out)
+    assert torch.equal(outs[0].view(torch.int16), outs[1].view(torch.int16))
