@@ -1215,6 +1215,11 @@ __global__ void __launch_bounds__(kThreadsSp, 1) prefill_sp_kernel(const __grid_
         tc::fence_after_sync();
     }
     if (!p.fused && p.has_intra && ctl[1] == 0u) intra_role<LAYER>(p, smem, tm);
+    if (ctl[1] != 0u) {  // after an abort copies into this block's shared memory may still be in flight: give them a bounded time
+        const uint64_t t0 = global_timer_ns();
+        while (global_timer_ns() - t0 < 2000000ull) {
+        }
+    }
     tc::fence_before_sync();
     __syncthreads();
     if (warp == 0) tc::tmem_dealloc(tm, kTmemCols);
