@@ -127,7 +127,7 @@ __device__ __forceinline__ void bulk_store(void* gmem_dst, const void* smem_src,
                  "r"(bytes)
                  : "memory");
 }
-// A piece of global memory on its way into L2 (16-byte aligned, a multiple of 16 bytes), and a tensor map's box likewise.
+// A tensor map's box on its way into L2.
 __device__ __forceinline__ void tensor_prefetch_3d(const void* tmap, int x, int y, int z) {
     asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];" ::"l"(reinterpret_cast<uint64_t>(tmap)), "r"(x), "r"(y), "r"(z)
                  : "memory");

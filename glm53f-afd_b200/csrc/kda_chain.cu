@@ -5,15 +5,17 @@
 //
 //   mover (1 warp)      bulk-copies (cp.async.bulk) each unit's 128x128 state and each row's raw inputs from global
 //                       memory into shared-memory rings, several units ahead of the arithmetic;
-//   prologue (2 warps)  turns a row's raw inputs into q, k, v, the decay multipliers, beta and sigmoid(gate)
-//                       (short conv + SiLU, L2 norms, gates for the layer entry points; exp(g) for the core ones);
+//   prologue (2 or 4 warps)  turns a row's raw inputs into q, k, v, the decay multipliers, beta and sigmoid(gate)
+//                       (short conv + SiLU, L2 norms, gates for the layer entry points, on four warps; exp(g) for the core ones,
+//                       on two);
 //   recurrence (16 warps) keeps the unit's state in registers across its rows: warp w owns value rows 8w..8w+7,
 //                       lane l key columns 4l..4l+3; per row the delta rule and the read-out; afterwards each warp
 //                       stores its own 8 rows, a whole contiguous row per instruction;
 //   epilogue (1 warp)   gated RMSNorm, bf16 outputs, replay saves.
 //
 // The state therefore crosses HBM once in each direction -- in as bulk transfers that are always several units deep
-// in flight, out as coalesced vector stores from the registers -- and no role ever waits on a global load.
+// in flight, out as coalesced vector stores from the registers.  What roles load from global memory themselves (a unit's metadata, the
+// layer prologue's conv weights and biases) is fetched ahead of the wait for the row or unit it belongs to.
 //
 // Arithmetic contract (what makes this a drop-in for the reference's kernels/kda.cu): every sum over the 128 key
 // channels is formed as the reference forms it -- a lane's four consecutive channels added in order from zero,

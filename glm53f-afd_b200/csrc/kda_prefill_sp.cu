@@ -31,6 +31,7 @@
 #include "kda_internal.h"
 #include "prefill_common.cuh"
 #include "tc.cuh"
+#include "tensor_map.cuh"
 
 namespace kda {
 namespace {
@@ -1271,19 +1272,6 @@ __global__ void __launch_bounds__(128) scan_compose_kernel(const __grid_constant
 
 }  // namespace
 
-// The driver's tensor-map encoder, looked up once through the runtime (the library does not link libcuda).
-using EncodeTiled = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                                 const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-static EncodeTiled encode_tiled() {
-    static EncodeTiled fn = [] {
-        void* f = nullptr;
-        cudaDriverEntryPointQueryResult qr;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &qr) != cudaSuccess || qr != cudaDriverEntryPointSuccess) f = nullptr;
-        return reinterpret_cast<EncodeTiled>(f);
-    }();
-    return fn;
-}
-
 // A [rows][H][128] tensor of `elem`-byte elements as (128, H, rows) with boxes of 64 rows of one head, 128 bytes wide.
 static bool row_tensor_map(CUtensorMap* tm, const void* base, int elem, int H, long long rows) {
     EncodeTiled enc = encode_tiled();
@@ -1297,7 +1285,7 @@ static bool row_tensor_map(CUtensorMap* tm, const void* base, int elem, int H, l
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-constexpr long long kCounterBytes = kPrefillTailBytes;  // tail of the workspace: the two item counters
+constexpr long long kCounterBytes = kPrefillTailBytes;  // tail of the workspace: the launches' counters (kda_internal.h)
 
 int64_t core_prefill_workspace_bytes(int32_t heads, int32_t batch, int32_t chunks_per_pass) {
     if (heads < 1 || batch < 1 || chunks_per_pass < 1) return 0;
@@ -1423,7 +1411,7 @@ int core_prefill_sp_launch(int32_t heads, int32_t batch, const int32_t* cu_seqle
     {
         long long K = 1;
         if (const char* env = getenv("GLM53F_KDA_PREFILL_SEGMENTS")) K = atoll(env);
-        else if (chains <= 16) {  // measured, 2^20 tokens: 8 chains 41.0 -> 17.0 ms, 16 chains 42.1 -> 33.8 ms, 32 chains 55.3 -> 61.9 ms
+        else if (chains <= 16) {  // measured, 2^18 tokens: 8 chains 7.5 -> 2.7 ms, 16 chains 8.4 -> 5.6, 24 (four segments) 9.2 -> 8.2, 32 (three) 10.1 -> 10.8
             const long long ka = sms / (2 * chains) + 1, kc = sms / chains;
             K = ka < kc ? ka : kc;
             if (K > 16) K = 16;
@@ -1531,8 +1519,8 @@ int core_prefill_sp_launch(int32_t heads, int32_t batch, const int32_t* cu_seqle
         }
     }
     // More chains than SMs: the state role fills the machine by itself, there is nothing to run beside it, and a fused launch over
-    // all the slots needs half as many launches as two halves that swap.  64 heads x 8
-    // sequences, 8,192 rows, a workspace of 32 chunks a chain: 641 -> 570 us.
+    // all the slots needs half as many launches as two halves that swap.  Workspaces of 32 chunks a chain: 150 chains (3 x 1,365
+    // rows) 309 -> 233 us, 192 (3 x 2,731 rows) 674 -> 567, 512 (8 x 1,024 rows) 608 -> 540.
     if (chains > sms && need > 0) {
         const long long passes = (need + whole - 1) / whole, n = (need + passes - 1) / passes;
         for (long long c = 0; c < need; c += n) {

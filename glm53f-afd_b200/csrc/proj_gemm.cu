@@ -12,8 +12,8 @@
 // K-major in global memory ([o][k] and [r][k]), so tiled tensor copies in the 128-byte swizzle feed tcgen05.mma
 // in place: a stage is 64 k of the weight tile (16 KiB) and of the row tile (NR x 128 bytes).  Roles per block:
 //   warp 0  producer: tensor copies into a ring of stages, each completing a stage's mbarrier;
-//   warp 1  one elected thread issues 4 MMAs (K = 16) per stage and commits the stage back to the producer, and the
-//           tile's accumulator to the epilogue when its last stage is in; owns the TMEM allocation;
+//   warp 1  issues 4 MMAs (K = 16) per stage, the warp converged and one lane elected (tc::mma_bf16_if), and commits the stage
+//           back to the producer, and the tile's accumulator to the epilogue when its last stage is in; owns the TMEM allocation;
 //   warps 2-5  epilogue: tcgen05.ld of the finished accumulator (lane = feature, column = row), convert, store.
 // Two accumulators alternate, so the epilogue of a tile overlaps the MMAs of the next; blocks walk the tile list with
 // the row tile fastest (blocks that run together share a weight tile in L2).  A block stays under
@@ -39,6 +39,7 @@
 #include "kda_internal.h"
 #include "proj_gemm.cuh"
 #include "tc.cuh"
+#include "tensor_map.cuh"
 
 namespace kda {
 namespace {
@@ -317,18 +318,6 @@ done:
         if (!opened) cluster_wait();  // the threads that never needed the opening barrier complete it here
         cluster_sync_all();
     }
-}
-
-using EncodeTiled = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                                 const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-EncodeTiled encode_tiled() {
-    static EncodeTiled fn = [] {
-        void* f = nullptr;
-        cudaDriverEntryPointQueryResult qr;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &qr) != cudaSuccess || qr != cudaDriverEntryPointSuccess) f = nullptr;
-        return reinterpret_cast<EncodeTiled>(f);
-    }();
-    return fn;
 }
 
 constexpr int kFewRows = 64;        // launches of up to this many rows run here, larger ones on SM pairs
