@@ -81,12 +81,13 @@ constexpr int kRecThreads = kRecWarps * 32;
 // the layer symbol 0.746 -> 0.657 ms per step with four, the exact verify 24.5 -> 19.1 ms, an exact prefill lane
 // 2.05 -> 1.57 ms, the replay 4.97 -> 4.72 ms); the core prologue is a widening and one exponential per channel, and
 // there two more warps only take registers and issue slots from the recurrence (0.538 -> 0.566 ms).
-template <int MODE>
-constexpr int kProWarpsOf = MODE == 1 /* kCore */ ? 2 : 4;
-template <int MODE>
-constexpr int kProThreadsOf = kProWarpsOf<MODE> * 32;
-template <int MODE>
-constexpr int kThreadsOf = kRecThreads + kProThreadsOf<MODE> + 64;  // + epilogue warp + mover warp
+// Single rows of bf16 states are cooked by two teams of four, a unit each in turn: a unit's 64 KiB take an SM 1.4 us at the copy rate, its row
+// four warps as long or longer (16 slots bf16: 674 -> 594 us a step of 34 layers; f32 states, 2.9 us a unit, 916 -> 937 with two teams,
+// and the exact verify's windows 1,346 -> 1,420, its recurrence being short of issue slots; one unit a block: 191 -> 203).
+template <typename S, int MODE, bool ONE_UNIT = false>
+constexpr int kProWarpsOf = MODE == 1 /* kCore */ ? 2 : MODE == 0 /* kLayer */ && sizeof(S) == 2 && !ONE_UNIT ? 8 : 4;
+template <typename S, int MODE, bool ONE_UNIT = false>
+constexpr int kThreadsOf = kRecThreads + kProWarpsOf<S, MODE, ONE_UNIT> * 32 + 64;  // + epilogue warp + mover warp
 
 struct Params {
     int H, layers;
@@ -128,6 +129,7 @@ struct Params {
     long long kv_stride, b_stride;
     unsigned long long neg_zero2;  // two -0.0f: see mul2
     unsigned long long wait_limit_ns;  // bound of every device-side wait (no progress for this long: give up)
+    int late_release;      // core: a state's slot is given back when its rows are through, not when the state is in registers
     int skip_first_state;  // diagnostic (glm53f_kda_debug_wait_test): block 0 does not fetch its first unit's state
 };
 
@@ -180,15 +182,17 @@ struct __align__(16) UnitInfo {
 template <typename S, int MODE>
 struct Smem {
     static constexpr int kStateBytes = DV * DK * (int)sizeof(S);
-    static constexpr int kStateSlots = sizeof(S) == 4 ? 3 : 5;
-    static constexpr int kRawSlots = MODE == kLayer ? (sizeof(S) == 4 ? 5 : 8) : sizeof(S) == 4 ? 3 : 4;  // raw-row ring depth
-    static constexpr int kRowSlots = MODE == kLayer ? (sizeof(S) == 4 ? 5 : 8) : sizeof(S) == 4 ? 3 : 4;  // cooked-row ring depth
+    // States in flight: 96 KiB (bf16) or 128 KiB (f32).  More slow a long launch down, its reads then crowd out its writes (bf16 core, 5 and
+    // 3 slots of the ring: 48 requests 1,303 and 1,220 us a step of 34 layers, 16 requests 462 and 459; 2: 1,214 and 488).
+    static constexpr int kStateSlots = MODE == kReplay ? (sizeof(S) == 4 ? 3 : 5) : sizeof(S) == 4 ? 2 : 3;
+    static constexpr int kRawSlots = MODE == kLayer ? (sizeof(S) == 4 ? 6 : 8) : sizeof(S) == 4 ? 3 : 4;  // raw-row ring depth
+    static constexpr int kRowSlots = MODE == kLayer ? (sizeof(S) == 4 ? 6 : 8) : sizeof(S) == 4 ? 3 : 4;  // cooked-row ring depth
     static constexpr int kRawBytes = align_up(RawOf<MODE>::T::BYTES, 128);
     static constexpr int oState = 0;
     static constexpr int oRaw = oState + kStateSlots * kStateBytes;
     static constexpr int oCooked = oRaw + kRawSlots * kRawBytes;
     static constexpr int oScratch = oCooked + kRowSlots * (int)sizeof(Cooked);  // prologue scratch: q, k before norm
-    static constexpr int oBars = oScratch + 2 * DK * 4;
+    static constexpr int oBars = oScratch + 4 * DK * 4;
     // barriers: st_full[S], st_empty[S], raw_full[R], raw_empty[R], row_full[C], y_full[C], row_empty[C]
     static_assert(MODE != kLayer || kRawSlots == kRowSlots, "layer_prologue_role: a free cooked slot implies a finished raw slot");
     static constexpr int kBars = 2 * kStateSlots + 2 * kRawSlots + 3 * kRowSlots;
@@ -210,6 +214,10 @@ struct Unit {
 // (request, layer, head) for the replay.  Indices advance by 32-bit arithmetic; the metadata of the next unit
 // (row range, state and window offsets: loads from global memory) is fetched while the current one is processed, and stays as
 // loaded until that unit's turn: arithmetic on it right after the loads would wait for them there, 1,500 cycles a unit and role.
+// Every role waits for itself, behind what it can work out from the launch's parameters alone: with the index arithmetic and the
+// first reads of the parameters behind the wait, a unit's metadata came 930 ns after it, 300 ns so.
+__device__ __forceinline__ void predecessors_done() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 template <int MODE>
 struct UnitIter {
     unsigned long long u;
@@ -233,6 +241,10 @@ struct UnitIter {
         r0 = r1 = kept = 0;
         s_off = c_off = 0;
         a_log = 0.0f;
+    }
+    // Behind the launch's predecessors: nothing global is read before this.
+    __device__ __forceinline__ void begin(const Params& p) {
+        predecessors_done();
         if (ok) fetch(p);
     }
     __device__ __forceinline__ void fetch(const Params& p) {
@@ -308,40 +320,56 @@ struct Ring {
 // single-row launch.)  Pieces are 16-byte multiples except the "scalar chunk" (beta or its logit): for that one `src` is the
 // element's own address and the mover copies the aligned 16 bytes around it, so the element lands at off + (address & 15).
 struct Piece {
-    int off, bytes;  // bytes == 0: this lane has none
-    const void* src;
+    int off, bytes;  // its place in the slot; bytes == 0: this lane has none
     bool scalar;
+    int tap;                        // conv inputs: the tap; others 3, the row itself
+    const unsigned char* base;      // the piece of row 0, head 0, layer 0
+    long long row, head, layer;     // bytes from one row, head, layer to the next
+    const unsigned char* window;    // conv inputs: the piece of head 0 in the first row of the window at offset 0
+    long long window_row;
+    __device__ __forceinline__ const unsigned char* at(const Unit& u, int r) const {
+        const int x = r + tap;
+        return (x < WINDOW ? window + u.conv_off * 2 + x * window_row : base + (u.row0 + x - WINDOW) * row) + u.h * head + u.layer * layer;
+    }
 };
+// What does not depend on the unit, worked out while the launch's predecessors finish; a row is then one address a lane.  (As a branch
+// for every kind of piece behind the metadata, 1 slot 204 -> 186 us a step of 34 layers, 16 slots core 495 -> 464.)
 template <int MODE>
-__device__ __forceinline__ Piece piece_of(const Params& p, const Unit& u, int r, int lane) {
-    const long long gr = u.row0 + r;
-    Piece x{0, 0, nullptr, false};
+__device__ __forceinline__ Piece piece_of(const Params& p, int lane) {
+    Piece x{0, 0, false, WINDOW, nullptr, 0, 0, 0, nullptr, 0};
+    auto set = [&](int off, int bytes, bool scalar, const void* base, long long row, long long head, long long layer) {
+        x.off = off; x.bytes = bytes; x.scalar = scalar;
+        x.base = reinterpret_cast<const unsigned char*>(base);
+        x.row = row; x.head = head; x.layer = layer;
+    };
     if constexpr (MODE == kLayer) {
         if (lane < 3 * TAPS) {
-            const int tap = lane / 3, part = lane - tap * 3, at = r + tap;
-            const uint16_t* row = at < WINDOW ? p.conv + u.conv_off + (long long)at * 3 * p.H * DK : p.P + (u.row0 + at - WINDOW) * p.p_stride;
-            x = {RawLayer::X + lane * 256, 256, row + ((long long)part * p.H + u.h) * DK, false};
+            const long long from = (long long)(lane % 3) * p.H * DK;
+            set(RawLayer::X + lane * 256, 256, false, p.P + from, p.p_stride * 2, 2 * DK, 0);
+            x.tap = lane / 3;
+            x.window = reinterpret_cast<const unsigned char*>(p.conv + from);
+            x.window_row = 3LL * p.H * DK * 2;
         } else if (lane == 3 * TAPS) {
-            x = {RawLayer::A, 256, p.A + gr * p.a_stride + (long long)u.h * DK, false};
+            set(RawLayer::A, 256, false, p.A, p.a_stride * 2, 2 * DK, 0);
         } else if (lane == 3 * TAPS + 1) {
-            x = {RawLayer::GATE, 256, p.G + gr * p.g_stride + (long long)u.h * DV, false};
+            set(RawLayer::GATE, 256, false, p.G, p.g_stride * 2, 2 * DV, 0);
         } else if (lane == 3 * TAPS + 2) {
-            x = {RawLayer::B, 2, p.P + gr * p.p_stride + p.b_off + u.h, true};
+            set(RawLayer::B, 2, true, p.P + p.b_off, p.p_stride * 2, 2, 0);
         }
     } else if constexpr (MODE == kCore) {
-        const long long at = (gr * p.H + u.h) * DK;
-        if (lane == 0) x = {RawCore::Q, 256, p.q + at, false};
-        else if (lane == 1) x = {RawCore::K, 256, p.k + at, false};
-        else if (lane == 2) x = {RawCore::V, 256, p.v + at, false};
-        else if (lane == 3) x = {RawCore::GLOG, 512, p.glog + at, false};
-        else if (lane == 4) x = {RawCore::B, 4, p.beta + gr * p.H + u.h, true};
-        else if (lane == 5 && p.G) x = {RawCore::GATE, 256, p.G + at, false};
+        const long long row2 = 2LL * p.H * DK;
+        if (lane == 0) set(RawCore::Q, 256, false, p.q, row2, 2 * DK, 0);
+        else if (lane == 1) set(RawCore::K, 256, false, p.k, row2, 2 * DK, 0);
+        else if (lane == 2) set(RawCore::V, 256, false, p.v, row2, 2 * DK, 0);
+        else if (lane == 3) set(RawCore::GLOG, 512, false, p.glog, 2 * row2, 4 * DK, 0);
+        else if (lane == 4) set(RawCore::B, 4, true, p.beta, 4LL * p.H, 4, 0);
+        else if (lane == 5 && p.G) set(RawCore::GATE, 256, false, p.G, row2, 2 * DK, 0);
     } else {
-        const long long at = (gr * p.H + u.h) * DK;
-        if (lane == 0) x = {RawReplay::K, 512, p.k_save + u.layer * p.kv_stride + at, false};
-        else if (lane == 1) x = {RawReplay::G, 512, p.g_save + u.layer * p.kv_stride + at, false};
-        else if (lane == 2) x = {RawReplay::V, 256, p.v_save + u.layer * p.kv_stride + at, false};
-        else if (lane == 3) x = {RawReplay::B, 4, p.b_save + u.layer * p.b_stride + gr * p.H + u.h, true};
+        const long long row2 = 2LL * p.H * DK;
+        if (lane == 0) set(RawReplay::K, 512, false, p.k_save, 2 * row2, 4 * DK, 4 * p.kv_stride);
+        else if (lane == 1) set(RawReplay::G, 512, false, p.g_save, 2 * row2, 4 * DK, 4 * p.kv_stride);
+        else if (lane == 2) set(RawReplay::V, 256, false, p.v_save, row2, 2 * DK, 2 * p.kv_stride);
+        else if (lane == 3) set(RawReplay::B, 4, true, p.b_save, 4LL * p.H, 4, 4 * p.b_stride);
     }
     return x;
 }
@@ -362,10 +390,35 @@ __device__ void mover_role(const Params& p, unsigned char* smem, uint64_t* bars,
     Ring st, raw;
     const bool copy0 = copies_state(p);
     UnitIter<MODE> units(p);
+    const Piece x = piece_of<MODE>(p, lane);
+    units.begin(p);
+    auto row_in = [&](const Unit& un, int r) -> bool {
+        if (!mbar_wait(&raw_empty[raw.idx], raw.phase ^ 1u, ctx, kStatusWaitRawEmpty)) return false;
+        unsigned char* dst = smem + L::oRaw + raw.idx * L::kRawBytes;
+        const uintptr_t src = reinterpret_cast<uintptr_t>(x.at(un, r));
+        if (!__any_sync(0xffffffffu, !x.scalar && (src & 15) != 0)) {
+            if (lane == 0) mbar_arrive_expect_tx(&raw_full[raw.idx], raw_row_bytes<MODE>(p));
+            __syncwarp();
+            if (x.bytes) bulk_load(dst + x.off, reinterpret_cast<const void*>(src & ~uintptr_t(15)), x.scalar ? 16 : x.bytes, &raw_full[raw.idx]);
+        } else {  // unaligned rows: 2-byte copies, a lane its piece
+            uint16_t* d = reinterpret_cast<uint16_t*>(dst + x.off + (x.scalar ? (int)(src & 15) : 0));
+            for (int e = 0; e < x.bytes / 2; ++e) d[e] = reinterpret_cast<const uint16_t*>(src)[e];
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&raw_full[raw.idx]);
+        }
+        __syncwarp();
+        raw.next(L::kRawSlots);
+        if (lane == 0) atomicAdd(const_cast<uint32_t*>(ctx.progress), 1u);
+        return true;
+    };
+    constexpr bool kRowFirst = MODE == kLayer;  // a core row is cooked in no time (16 slots 459 us a step; 473 with the row first)
     bool first = true;
     for (; units.valid(); first = false) {
         const Unit un = units.take(p);
         if (un.rows == 0 && !copy0) continue;
+        // A layer call's first row goes ahead of its state: the row has to be cooked before the state is wanted (5 slots 352 us a step, behind
+        // it 369).
+        if (kRowFirst && first && un.rows > 0 && !row_in(un, 0)) return;
         // The unit's state.
         if (!mbar_wait(&st_empty[st.idx], st.phase ^ 1u, ctx, kStatusWaitStateEmpty)) return;
         if (lane == 0) info[st.idx] = {un.s_elem, un.rows};
@@ -388,26 +441,9 @@ __device__ void mover_role(const Params& p, unsigned char* smem, uint64_t* bars,
             }
         }
         st.next(L::kStateSlots);
-        // Its rows' raw inputs.
-        for (int r = 0; r < un.rows; ++r) {
-            if (!mbar_wait(&raw_empty[raw.idx], raw.phase ^ 1u, ctx, kStatusWaitRawEmpty)) return;
-            unsigned char* dst = smem + L::oRaw + raw.idx * L::kRawBytes;
-            const Piece x = piece_of<MODE>(p, un, r, lane);
-            const uintptr_t src = reinterpret_cast<uintptr_t>(x.src);
-            if (!__any_sync(0xffffffffu, !x.scalar && (src & 15) != 0)) {
-                if (lane == 0) mbar_arrive_expect_tx(&raw_full[raw.idx], raw_row_bytes<MODE>(p));
-                __syncwarp();
-                if (x.bytes) bulk_load(dst + x.off, reinterpret_cast<const void*>(src & ~uintptr_t(15)), x.scalar ? 16 : x.bytes, &raw_full[raw.idx]);
-            } else {  // unaligned rows: 2-byte copies, a lane its piece
-                uint16_t* d = reinterpret_cast<uint16_t*>(dst + x.off + (x.scalar ? (int)(src & 15) : 0));
-                for (int e = 0; e < x.bytes / 2; ++e) d[e] = reinterpret_cast<const uint16_t*>(x.src)[e];
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&raw_full[raw.idx]);
-            }
-            __syncwarp();
-            raw.next(L::kRawSlots);
-            if (lane == 0) atomicAdd(const_cast<uint32_t*>(ctx.progress), 1u);
-        }
+        // The other rows.
+        for (int r = kRowFirst && first ? 1 : 0; r < un.rows; ++r)
+            if (!row_in(un, r)) return;
     }
     if (!mbar_wait(&st_empty[st.idx], st.phase ^ 1u, ctx, kStatusWaitStateEmpty)) return;
     if (lane == 0) {
@@ -439,7 +475,7 @@ __device__ __forceinline__ void l2norm_warp(const float* x, float* y, int lane, 
 template <typename S, int MODE>
 __device__ void prologue_role(const Params& p, unsigned char* smem, uint64_t* bars, const WaitCtx& ctx, int t) {
     using L = Smem<S, MODE>;
-    constexpr int kProThreads = kProThreadsOf<MODE>;
+    constexpr int kProThreads = kProWarpsOf<S, MODE> * 32;
     uint64_t* raw_full = bars + 2 * L::kStateSlots;
     uint64_t* raw_empty = raw_full + L::kRawSlots;
     uint64_t* row_full = raw_empty + L::kRawSlots;
@@ -451,6 +487,7 @@ __device__ void prologue_role(const Params& p, unsigned char* smem, uint64_t* ba
     // Whether the role's threads meet at barriers in every row (the L2 norms go through shared scratch).
     const bool syncs = MODE == kCore && (p.flags & GLM53F_KDA_CORE_L2NORM) != 0;
     UnitIter<MODE> units(p);
+    units.begin(p);
     while (units.valid()) {
         const Unit un = units.take(p);
         if (un.rows == 0 && !copy0) continue;
@@ -523,7 +560,7 @@ __device__ void prologue_role(const Params& p, unsigned char* smem, uint64_t* ba
 // A launch of one unit a block (ONE_UNIT, an instance of the kernel to itself: the rule inside cost 16 single-row slots 1.5 %) waits for its
 // first rows, and there four warps on a row are the shorter way: windows of 2, 4 and 8 rows of one slot 7.9, 10.6 and 15.4 us with
 // a row per warp, 6.6, 9.3 and 14.7 so (two units a block, 4 rows: 16.4 against 17.2).
-constexpr int kTogetherRows = 8;
+constexpr int kTogetherRows = 8, kTeamWarps = 4;
 template <typename S, bool ONE_UNIT>
 __device__ void layer_prologue_role(const Params& p, unsigned char* smem, uint64_t* bars, const WaitCtx& ctx, int warp, int lane) {
     using L = Smem<S, kLayer>;
@@ -535,8 +572,10 @@ __device__ void layer_prologue_role(const Params& p, unsigned char* smem, uint64
     const bool copy0 = copies_state(p);
     const bool vec = ((reinterpret_cast<uintptr_t>(p.cw) | reinterpret_cast<uintptr_t>(p.dt_bias)) & 15) == 0;
     UnitIter<kLayer> units(p);
+    units.begin(p);
     constexpr int together = ONE_UNIT ? kTogetherRows : 1;
-    int turn = 0;
+    constexpr int kTeams = kProWarpsOf<S, kLayer, ONE_UNIT> / kTeamWarps;
+    int turn = 0, team_turn = 0;
     // A warp whose wait gave up does not leave: the single-row units further on are cooked by all four warps, which meet there at
     // barriers.  It takes no more rows and goes on through the units to the next vote, which then sends all four home.
     bool dead = false;
@@ -553,19 +592,27 @@ __device__ void layer_prologue_role(const Params& p, unsigned char* smem, uint64
             // A single row is cooked by all four warps, a thread a channel: with one row a unit the next state is waited for anyway,
             // and the row's latency counts (16 slots, bf16: 0.670 ms a step of 34 layers, 0.696 with a row per warp; 1 slot 0.215
             // against 0.263).  ONE_UNIT: so are up to eight, there being no other unit's rows to work on meanwhile.
-            const int c = warp * 32 + lane;
+            if (kTeams > 1 && (team_turn++ & (kTeams - 1)) != (warp >> 2)) {
+                for (int r = 0; r < un.rows; ++r) {
+                    raw.next(L::kRawSlots);
+                    row.next(L::kRowSlots);
+                }
+                continue;
+            }
+            const int tw = warp & (kTeamWarps - 1), c = tw * 32 + lane, bar = 1 + 2 * (warp >> 2);
             uint2 w[3];
 #pragma unroll
             for (int part = 0; part < 3; ++part) {
                 const uint16_t* cw = p.cw + (((long long)part * p.H + un.h) * DK + c) * TAPS;
                 w[part] = vec ? *reinterpret_cast<const uint2*>(cw) : make_uint2((uint32_t)cw[0] | ((uint32_t)cw[1] << 16), (uint32_t)cw[2] | ((uint32_t)cw[3] << 16));
             }
-            const float db = p.dt_bias[(long long)un.h * DK + c], decay_rate = expf(un.a_log);
+            const float* dtb = p.dt_bias + (long long)un.h * DK + (c & (DK / 2 - 1));
+            const float db[2] = {dtb[0], dtb[DK / 2]}, decay_rate = expf(un.a_log);
             for (int r = 0; r < un.rows; ++r, raw.next(L::kRawSlots), row.next(L::kRowSlots)) {
                 const bool ready = !dead && mbar_wait(&row_empty[row.idx], row.phase ^ 1u, ctx, kStatusWaitRowEmpty) && mbar_wait(&raw_full[raw.idx], raw.phase, ctx, kStatusWaitRawFull);
                 const unsigned char* in = smem + L::oRaw + raw.idx * L::kRawBytes;
                 Cooked& ck = *reinterpret_cast<Cooked*>(smem + L::oCooked + row.idx * sizeof(Cooked));
-                float* scratch = reinterpret_cast<float*>(smem + L::oScratch);
+                float* scratch = reinterpret_cast<float*>(smem + L::oScratch) + (warp >> 2) * 2 * DK;
                 if (ready) {
                     const uint16_t* x = reinterpret_cast<const uint16_t*>(in + RawLayer::X);
 #pragma unroll
@@ -577,17 +624,23 @@ __device__ void layer_prologue_role(const Params& p, unsigned char* smem, uint64
                         (part == 2 ? ck.v : scratch + part * DK)[c] = bf16_round(acc / (1.0f + expf(-acc)));
                     }
                 }
-                if (!named_bar_all(1, kProThreadsOf<kLayer>, ready)) return;  // all four leave together
-                if (warp == 0) l2norm_warp(scratch, ck.q, lane, true);
-                else if (warp == 1) l2norm_warp(scratch + DK, ck.k, lane, false);
-                else if (warp == 2 && lane == 0) {
-                    const uintptr_t addr = reinterpret_cast<uintptr_t>(p.P + (un.row0 + r) * p.p_stride + p.b_off + un.h);
-                    ck.beta = bf16_round(sigmoidf_(bf16_bits_to_f32(*reinterpret_cast<const uint16_t*>(in + RawLayer::B + (addr & 15)))));
+                if (!named_bar_all(bar, kTeamWarps * 32, ready)) return;  // all four leave together
+                if (tw == 0) l2norm_warp(scratch, ck.q, lane, true);
+                else if (tw == 1) l2norm_warp(scratch + DK, ck.k, lane, false);
+                else {  // meanwhile the other two warps: decay, gate and beta, two channels a thread
+#pragma unroll
+                    for (int half = 0; half < 2; ++half) {
+                        const int d = (c & (DK / 2 - 1)) + half * (DK / 2);
+                        ck.g[d] = expf(p.lower * sigmoidf_(decay_rate * (bf16_bits_to_f32(reinterpret_cast<const uint16_t*>(in + RawLayer::A)[d]) + db[half])));
+                        ck.sg[d] = sigmoidf_(bf16_bits_to_f32(reinterpret_cast<const uint16_t*>(in + RawLayer::GATE)[d]));
+                    }
+                    if (tw == 2 && lane == 0) {
+                        const uintptr_t addr = reinterpret_cast<uintptr_t>(p.P + (un.row0 + r) * p.p_stride + p.b_off + un.h);
+                        ck.beta = bf16_round(sigmoidf_(bf16_bits_to_f32(*reinterpret_cast<const uint16_t*>(in + RawLayer::B + (addr & 15)))));
+                    }
                 }
-                ck.g[c] = expf(p.lower * sigmoidf_(decay_rate * (bf16_bits_to_f32(reinterpret_cast<const uint16_t*>(in + RawLayer::A)[c]) + db)));
-                ck.sg[c] = sigmoidf_(bf16_bits_to_f32(reinterpret_cast<const uint16_t*>(in + RawLayer::GATE)[c]));
-                named_bar_sync(2, kProThreadsOf<kLayer>);
-                if (warp == 0 && lane == 0) {
+                named_bar_sync(bar + 1, kTeamWarps * 32);
+                if (tw == 0 && lane == 0) {
                     mbar_arrive(&row_full[row.idx]);
                     mbar_arrive(&raw_empty[raw.idx]);
                 }
@@ -595,7 +648,7 @@ __device__ void layer_prologue_role(const Params& p, unsigned char* smem, uint64
             continue;
         }
         for (int r = 0; r < un.rows; ++r, raw.next(L::kRawSlots), row.next(L::kRowSlots)) {
-            if ((turn++ & (kProWarpsOf<kLayer> - 1)) != warp || dead) continue;
+            if ((turn++ & (kProWarpsOf<S, kLayer, ONE_UNIT> - 1)) != warp || dead) continue;
             // The head's weights come straight from global memory, on their way while the row's inputs are waited for.
             uint4 w[3][2];
             float4 dtb;
@@ -691,6 +744,7 @@ __device__ void recurrence_role(const Params& p, unsigned char* smem, uint64_t* 
     uint64_t* row_empty = y_full + L::kRowSlots;
     Ring st, row;
     const UnitInfo* info = reinterpret_cast<const UnitInfo*>(smem + L::oUnits);
+    predecessors_done();
     for (;;) {
         if (!mbar_wait(&st_full[st.idx], st.phase, ctx, kStatusWaitStateFull)) return;
         const UnitInfo un = info[st.idx];
@@ -700,7 +754,8 @@ __device__ void recurrence_role(const Params& p, unsigned char* smem, uint64_t* 
         load_rows<S>(slot, warp, lane, s);
         const bool writes = p.state_out != nullptr;
         __syncwarp();  // the slot is free as soon as every lane's registers hold the state
-        if (lane == 0) mbar_arrive(&st_empty[st.idx]);
+        const bool late = MODE == kCore && p.late_release;
+        if (!late && lane == 0) mbar_arrive(&st_empty[st.idx]);
         for (int r = 0; r < un.rows; ++r) {
             if (!mbar_wait(&row_full[row.idx], row.phase, ctx, kStatusWaitRowFull)) return;
             Cooked& ck = *reinterpret_cast<Cooked*>(smem + L::oCooked + row.idx * sizeof(Cooked));
@@ -731,6 +786,10 @@ __device__ void recurrence_role(const Params& p, unsigned char* smem, uint64_t* 
             }
             row.next(L::kRowSlots);
         }
+        if (late) {  // see late_release
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&st_empty[st.idx]);
+        }
         if (writes) {
             // Straight from the registers: per row a lane stores its 4 consecutive elements (8 or 16 bytes), a warp a
             // whole contiguous row.  Each warp wrote nothing but the rows it read, so in place is safe.
@@ -751,10 +810,11 @@ __device__ void epilogue_role(const Params& p, unsigned char* smem, uint64_t* ba
     const bool copy0 = copies_state(p);
     const bool gated = MODE == kLayer || p.G != nullptr;
     float nw[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    UnitIter<MODE> units(p);
+    units.begin(p);
     if (gated)
 #pragma unroll
         for (int i = 0; i < 4; ++i) nw[i] = bf16_bits_to_f32(p.norm_w[lane * 4 + i]);
-    UnitIter<MODE> units(p);
     while (units.valid()) {
         const Unit un = units.take(p);
         if (un.rows == 0 && !copy0) continue;
@@ -810,9 +870,9 @@ __device__ void epilogue_role(const Params& p, unsigned char* smem, uint64_t* ba
 
 // ---- the kernel ----------------------------------------------------------------------------------------------
 template <typename S, int MODE, bool ONE_UNIT = false>
-__global__ void __launch_bounds__(kThreadsOf<MODE>, 1) recurrent_kernel(const __grid_constant__ Params p) {
+__global__ void __launch_bounds__(kThreadsOf<S, MODE, ONE_UNIT>, 1) recurrent_kernel(const __grid_constant__ Params p) {
     using L = Smem<S, MODE>;
-    constexpr int kProWarps = kProWarpsOf<MODE>, kProThreads = kProThreadsOf<MODE>;
+    constexpr int kProWarps = kProWarpsOf<S, MODE, ONE_UNIT>, kProThreads = kProWarps * 32;
     extern __shared__ __align__(128) unsigned char smem[];
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::oBars);
     volatile uint32_t* ctl = reinterpret_cast<volatile uint32_t*>(smem + L::oCtl);
@@ -832,10 +892,9 @@ __global__ void __launch_bounds__(kThreadsOf<MODE>, 1) recurrent_kernel(const __
     }
     __syncthreads();
     // Programmatic dependent launch: let the next kernel of the stream be scheduled onto SMs as this grid's blocks
-    // retire (its block set-up then overlaps this grid's tail), and do not touch global memory before every earlier
-    // grid of the stream has completed and flushed.  Both are no-ops for a launch without the attribute.
+    // retire (its block set-up then overlaps this grid's tail); the roles touch no global memory before every earlier
+    // grid of the stream has completed and flushed (predecessors_done).  Both are no-ops for a launch without the attribute.
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
     const WaitCtx ctx{ctl, ctl + 1, &g_status, p.wait_limit_ns};
     if (warp < kRecWarps) {
         recurrence_role<S, MODE>(p, smem, bars, ctx, warp, lane);
@@ -1024,6 +1083,13 @@ int launch_replay_small(const Params& p, cudaStream_t stream) {
     return (int)cudaLaunchKernelEx(&cfg, replay_small_kernel<S>, q);
 }
 
+// Core launches: when a state's slot is free for the next one.  At once, the next read is as early as can be, which is what a launch of few
+// units a block wants (bf16, 16 slots 460 us a step of 34 layers against 485; 30 slots 780 against 795); many units are through
+// sooner when reads keep less far ahead of the writes (48 slots 1,219 against 1,204; f32 states, 5, 16 and 40 slots: 371, 850 and 2,013
+// against 385, 843 and 1,945).  The line lies between 13 and 21 bf16 units a block, 2 and 7 f32 ones.
+template <typename S>
+bool late_release(long long units, long long sms) { return units * DV * DK * (long long)sizeof(S) > sms * 432 * 1024; }
+
 template <typename S, int MODE, bool ONE_UNIT = false>
 int launch(const Params& p, cudaStream_t stream) {
     using L = Smem<S, MODE>;
@@ -1045,6 +1111,7 @@ int launch(const Params& p, cudaStream_t stream) {
     Params q = p;
     q.neg_zero2 = 0x8000000080000000ull;
     q.wait_limit_ns = g_wait_limit_ns;
+    q.late_release = MODE == kCore && late_release<S>(p.units, sms);
     q.skip_first_state = g_skip_first_state;
     g_skip_first_state = 0;
     // Launched with programmatic stream serialization: the kernel itself waits for its predecessors before its first
@@ -1055,7 +1122,7 @@ int launch(const Params& p, cudaStream_t stream) {
     }();
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(kThreadsOf<MODE>);
+    cfg.blockDim = dim3(kThreadsOf<S, MODE, ONE_UNIT>);
     cfg.dynamicSmemBytes = L::kBytes;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
