@@ -129,7 +129,6 @@ struct Params {
     long long kv_stride, b_stride;
     unsigned long long neg_zero2;  // two -0.0f: see mul2
     unsigned long long wait_limit_ns;  // bound of every device-side wait (no progress for this long: give up)
-    int late_release;      // core: a state's slot is given back when its rows are through, not when the state is in registers
     int skip_first_state;  // diagnostic (glm53f_kda_debug_wait_test): block 0 does not fetch its first unit's state
 };
 
@@ -734,7 +733,7 @@ __device__ void layer_prologue_role(const Params& p, unsigned char* smem, uint64
 }
 
 // ---- the recurrence ------------------------------------------------------------------------------------------
-template <typename S, int MODE>
+template <typename S, int MODE, bool LATE>
 __device__ void recurrence_role(const Params& p, unsigned char* smem, uint64_t* bars, const WaitCtx& ctx, int warp, int lane) {
     using L = Smem<S, MODE>;
     uint64_t* st_full = bars;
@@ -754,8 +753,7 @@ __device__ void recurrence_role(const Params& p, unsigned char* smem, uint64_t* 
         load_rows<S>(slot, warp, lane, s);
         const bool writes = p.state_out != nullptr;
         __syncwarp();  // the slot is free as soon as every lane's registers hold the state
-        const bool late = MODE == kCore && p.late_release;
-        if (!late && lane == 0) mbar_arrive(&st_empty[st.idx]);
+        if (!LATE && lane == 0) mbar_arrive(&st_empty[st.idx]);
         for (int r = 0; r < un.rows; ++r) {
             if (!mbar_wait(&row_full[row.idx], row.phase, ctx, kStatusWaitRowFull)) return;
             Cooked& ck = *reinterpret_cast<Cooked*>(smem + L::oCooked + row.idx * sizeof(Cooked));
@@ -786,7 +784,7 @@ __device__ void recurrence_role(const Params& p, unsigned char* smem, uint64_t* 
             }
             row.next(L::kRowSlots);
         }
-        if (late) {  // see late_release
+        if constexpr (LATE) {  // see late_release
             __syncwarp();
             if (lane == 0) mbar_arrive(&st_empty[st.idx]);
         }
@@ -869,7 +867,7 @@ __device__ void epilogue_role(const Params& p, unsigned char* smem, uint64_t* ba
 }
 
 // ---- the kernel ----------------------------------------------------------------------------------------------
-template <typename S, int MODE, bool ONE_UNIT = false>
+template <typename S, int MODE, bool ONE_UNIT = false, bool LATE = false>
 __global__ void __launch_bounds__(kThreadsOf<S, MODE, ONE_UNIT>, 1) recurrent_kernel(const __grid_constant__ Params p) {
     using L = Smem<S, MODE>;
     constexpr int kProWarps = kProWarpsOf<S, MODE, ONE_UNIT>, kProThreads = kProWarps * 32;
@@ -897,7 +895,7 @@ __global__ void __launch_bounds__(kThreadsOf<S, MODE, ONE_UNIT>, 1) recurrent_ke
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const WaitCtx ctx{ctl, ctl + 1, &g_status, p.wait_limit_ns};
     if (warp < kRecWarps) {
-        recurrence_role<S, MODE>(p, smem, bars, ctx, warp, lane);
+        recurrence_role<S, MODE, LATE>(p, smem, bars, ctx, warp, lane);
     } else if (warp < kRecWarps + kProWarps) {
         if constexpr (MODE == kLayer) layer_prologue_role<S, ONE_UNIT>(p, smem, bars, ctx, warp - kRecWarps, lane);
         else prologue_role<S, MODE>(p, smem, bars, ctx, tid - kRecThreads);
@@ -1087,22 +1085,26 @@ int launch_replay_small(const Params& p, cudaStream_t stream) {
 // units a block wants (bf16, 16 slots 460 us a step of 34 layers against 485; 30 slots 780 against 795); many units are through
 // sooner when reads keep less far ahead of the writes (48 slots 1,219 against 1,204; f32 states, 5, 16 and 40 slots: 371, 850 and 2,013
 // against 385, 843 and 1,945).  The line lies between 13 and 21 bf16 units a block, 2 and 7 f32 ones.
+// (An instance of the kernel to itself: the choice inside cost 16 slots 1 %.)
 template <typename S>
 bool late_release(long long units, long long sms) { return units * DV * DK * (long long)sizeof(S) > sms * 432 * 1024; }
 
-template <typename S, int MODE, bool ONE_UNIT = false>
+template <typename S, int MODE, bool ONE_UNIT = false, bool LATE = false>
 int launch(const Params& p, cudaStream_t stream) {
     using L = Smem<S, MODE>;
     const long long sms = sm_count();
     if constexpr (MODE == kLayer && !ONE_UNIT) {
         if (p.units <= sms) return launch<S, MODE, true>(p, stream);
     }
+    if constexpr (MODE == kCore && !LATE) {
+        if (late_release<S>(p.units, sms)) return launch<S, MODE, false, true>(p, stream);
+    }
     static bool configured = false;  // per process; the attribute is per device, so set it on every device change
     static int configured_dev = -1;
     int dev = 0;
     cudaGetDevice(&dev);
     if (!configured || configured_dev != dev) {
-        const cudaError_t e = cudaFuncSetAttribute(recurrent_kernel<S, MODE, ONE_UNIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kBytes);
+        const cudaError_t e = cudaFuncSetAttribute(recurrent_kernel<S, MODE, ONE_UNIT, LATE>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kBytes);
         if (e != cudaSuccess) return (int)e;
         configured = true;
         configured_dev = dev;
@@ -1111,7 +1113,6 @@ int launch(const Params& p, cudaStream_t stream) {
     Params q = p;
     q.neg_zero2 = 0x8000000080000000ull;
     q.wait_limit_ns = g_wait_limit_ns;
-    q.late_release = MODE == kCore && late_release<S>(p.units, sms);
     q.skip_first_state = g_skip_first_state;
     g_skip_first_state = 0;
     // Launched with programmatic stream serialization: the kernel itself waits for its predecessors before its first
@@ -1130,7 +1131,7 @@ int launch(const Params& p, cudaStream_t stream) {
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl ? 1 : 0;
-    return (int)cudaLaunchKernelEx(&cfg, recurrent_kernel<S, MODE, ONE_UNIT>, q);
+    return (int)cudaLaunchKernelEx(&cfg, recurrent_kernel<S, MODE, ONE_UNIT, LATE>, q);
 }
 
 template <int MODE>
