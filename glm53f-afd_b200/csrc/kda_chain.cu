@@ -36,6 +36,7 @@
 #include "glm53f_kda.h"
 #include "kda_internal.h"
 #include "recurrence.cuh"
+#include "recurrence_octet.cuh"
 
 namespace kda {
 
@@ -916,72 +917,77 @@ __global__ void __launch_bounds__(kThreadsOf<S, MODE, ONE_UNIT>, 1) recurrent_ke
 }
 
 // ---- the core step on many small blocks ------------------------------------------------------------------------
-// The same arithmetic (delta_rule, rows_dot, round_rows: the bits are those of the kernel above and of the reference)
-// for the core entry points without fused norms, arranged for few units: a block of four warps owns a QUARTER of a
-// unit -- 32 of its 128 value rows, 8 a warp, which never interact with the others -- loads that part of the state
-// straight from global memory into registers (a lane's four consecutive key channels of a row are 8 or 16 contiguous
-// bytes, a warp's a whole row), cooks each row's inputs itself (128 threads, one channel each: widen q, k, v, exp of
-// the log decay, beta), steps through the request's rows and stores its rows of the state back.  No rings, no bulk
-// copies: with eight such blocks resident on an SM, and blocks handed out as SMs free up, the loads of some cover the
-// arithmetic and stores of others, a launch's last blocks end within one small block's time of each other, and the
-// next launch's blocks move in as room appears (programmatic dependent launch).  Used for the exact verify, whose 16
-// serial rows a unit want many warps; for single-row decode the persistent kernel above streams faster.  (A variant
-// without shared memory, every warp cooking its own lanes' pieces of a row as the replay below does, was slower: the
-// sixteen warps of a unit each repeat the row's exponentials -- exact verify 12.0 against 11.1 ms, decode 3,567 GB/s.)
-constexpr int kSmallWarps = 4, kSmallThreads = kSmallWarps * 32, kSmallParts = kRecWarps / kSmallWarps;
+// The same arithmetic (recurrence_octet.cuh: the bits are those of the kernel above and of the reference) for the core entry
+// points without fused norms, arranged for windows: a block of four warps owns HALF of a unit -- 64 of its 128 value rows, 16 a
+// warp, which never interact with the others -- loads that part of the state straight from global memory into registers, cooks
+// each row's inputs itself (128 threads, one channel each: widen q, k, v, exp of the log decay, beta; loaded a row ahead, into the other
+// of two buffers, so a row takes one barrier), steps through the request's rows and stores its rows of the state back.  No rings, no
+// bulk copies: four such blocks on an SM are two units' serial rows at once.  Used for the exact verify; for single-row
+// decode the persistent kernel above streams faster.
+constexpr int kSmallWarps = 4, kSmallThreads = kSmallWarps * 32, kR = 4, kSmallParts = DV / (4 * kR * kSmallWarps);
 
 template <typename S>
-__global__ void __launch_bounds__(kSmallThreads, 8) core_small_kernel(const __grid_constant__ Params p) {
-    __shared__ __align__(16) float sq[DK], sk[DK], sg[DK], sv[DV];
-    __shared__ float sbeta;
+__global__ void __launch_bounds__(kSmallThreads, 4) core_small_kernel(const __grid_constant__ Params p) {
+    __shared__ __align__(16) float sq[2][DK], sk[2][DK], sg[2][DK], sv[2][DV];
+    __shared__ float sbeta[2];
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     const long long unit = blockIdx.x / kSmallParts;
-    const int part = blockIdx.x % kSmallParts, uw = part * kSmallWarps + warp;  // this warp's place among the unit's 16
+    const int part = blockIdx.x % kSmallParts, uw = part * kSmallWarps + warp;  // this warp's place among the unit's
     const int b = (int)(unit / p.H), h = (int)(unit % p.H);
     const int r0 = p.cu_rows[b], rows = max(p.cu_rows[b + 1] - r0, 0);
     const bool writes = p.state_out != nullptr;
     if (rows == 0 && !copies_state(p)) return;
     const long long s_elem = p.state_off[b] + (long long)h * DV * DK;
-    f32x2 s[kPairs][4];
-    load_rows_global<S>(reinterpret_cast<const S*>(p.state_in) + s_elem, uw, lane, s);
+    f32x2 s[kR][oct::kRowPairs];
+    oct::load_rows(reinterpret_cast<const S*>(p.state_in) + s_elem, uw, lane, s);
+    const int mine = uw * 4 * kR + oct::row_of_lane<kR>(lane);
+    struct Raw {  // a row's inputs, this thread's channel
+        uint16_t q, k, v;
+        float g, beta;
+    } next{};
+    auto fetch = [&](int r) {
+        const long long gr = (long long)r0 + r, at = (gr * p.H + h) * DK + t;
+        next.q = p.q[at];
+        next.k = p.k[at];
+        next.v = p.v[at];
+        next.g = p.glog[at];
+        if (t == 0) next.beta = p.beta[gr * p.H + h];
+    };
+    if (rows > 0) fetch(0);
     for (int r = 0; r < rows; ++r) {
         const long long gr = (long long)r0 + r, at = (gr * p.H + h) * DK + t;
-        // The row's inputs, one channel a thread (the prologue of the kernel above for the core entry points).
-        const float kf = bf16_bits_to_f32(p.k[at]), gf = expf(p.glog[at]);
-        const uint16_t vb = p.v[at];
-        sq[t] = bf16_bits_to_f32(p.q[at]);
-        sk[t] = kf;
-        sg[t] = gf;
-        sv[t] = bf16_bits_to_f32(vb);
-        float bt = 0.0f;
-        if (t == 0) sbeta = bt = p.beta[gr * p.H + h];
+        const int buf = r & 1;  // the row before may still be read from the other buffer
+        const float kf = bf16_bits_to_f32(next.k), gf = expf(next.g);
+        sq[buf][t] = bf16_bits_to_f32(next.q);
+        sk[buf][t] = kf;
+        sg[buf][t] = gf;
+        sv[buf][t] = bf16_bits_to_f32(next.v);
+        if (t == 0) sbeta[buf] = next.beta;
         if (p.k_save != nullptr && part == 0) {
             p.k_save[at] = kf;
             p.g_save[at] = gf;
-            p.v_save[at] = vb;
-            if (t == 0) p.b_save[gr * p.H + h] = bt;
+            p.v_save[at] = next.v;
+            if (t == 0) p.b_save[gr * p.H + h] = next.beta;
         }
         __syncthreads();
-        f32x2 kk[4], gg[4];
+        if (r + 1 < rows) fetch(r + 1);
         {
-            const float4 k4 = *reinterpret_cast<const float4*>(&sk[lane * 4]);
-            const float4 g4 = *reinterpret_cast<const float4*>(&sg[lane * 4]);
-            kk[0] = pack2(k4.x, k4.x); kk[1] = pack2(k4.y, k4.y); kk[2] = pack2(k4.z, k4.z); kk[3] = pack2(k4.w, k4.w);
-            gg[0] = pack2(g4.x, g4.x); gg[1] = pack2(g4.y, g4.y); gg[2] = pack2(g4.z, g4.z); gg[3] = pack2(g4.w, g4.w);
+            f32x2 kk[oct::kRowPairs], gg[oct::kRowPairs];
+            oct::load_leaves(sg[buf], lane, gg);
+            oct::load_leaves(sk[buf], lane, kk);
+            oct::delta_rule(s, kk, gg, sv[buf][mine], lane, sbeta[buf], p.neg_zero2);
         }
-        delta_rule(s, kk, gg, sv, uw, lane, sbeta, p.neg_zero2);
-        const float4 q4 = *reinterpret_cast<const float4*>(&sq[lane * 4]);
-        const f32x2 qq[4] = {pack2(q4.x, q4.x), pack2(q4.y, q4.y), pack2(q4.z, q4.z), pack2(q4.w, q4.w)};
-        const float o = rows_dot(s, qq, lane, p.neg_zero2);
-        if ((lane & 3) == 0) p.out[gr * p.out_stride + (long long)h * DV + uw * kRowsPerLane + (lane >> 2)] = f32_to_bf16_bits(o);
+        f32x2 qq[oct::kRowPairs];
+        oct::load_leaves(sq[buf], lane, qq);
+        const float o = oct::rows_dot(s, qq, lane, p.neg_zero2);
+        if (oct::first_of_row<kR>(lane)) p.out[gr * p.out_stride + (long long)h * DV + mine] = f32_to_bf16_bits(o);
         if constexpr (sizeof(S) == 2) {
-            if (r + 1 < rows || !writes) round_rows(s);
+            if (r + 1 < rows || !writes) oct::round_rows(s);
         }
-        __syncthreads();  // the cooked row is overwritten by the next one
     }
-    if (writes) store_rows_global<S>(reinterpret_cast<S*>(p.state_out) + s_elem, uw, lane, s);
+    if (writes) oct::store_rows(reinterpret_cast<S*>(p.state_out) + s_elem, uw, lane, s);
 }
 
 template <typename S>
@@ -1006,35 +1012,27 @@ int launch_small(const Params& p, cudaStream_t stream) {
 }
 
 // ---- the replay on many small blocks ---------------------------------------------------------------------------
-// A commit replays keep[b] saved rows onto every (request, layer, head) state: no read-out, no norms, inputs that are
-// already cooked.  Eight of a unit's value rows never interact with the others, and what a lane needs of a saved row is
-// exactly a 16-byte piece of k and of the decay (its four key channels), one v and beta: so a WARP is the unit of work
-// here -- no shared memory, no barrier, the next row's inputs loaded into registers while the current row's delta rule
-// runs -- and 32 such warps are resident on an SM where the persistent kernel has one unit's 16.  Same delta_rule, same
-// rounding points (a bf16 state is rounded after every row), so the bits are the persistent kernel's and the
-// reference's.  Measured at 48 slots x 34 layers, accepted prefixes drawn from 0..16: 3.63 ms a commit against 4.71 ms.
-struct ReplayRow {
-    float4 k, g;
-    uint16_t v;  // bf16 bits, widened when the row's turn comes: a conversion at the load would wait for it there and then
+// A commit replays keep[b] saved rows onto every (request, layer, head) state: no read-out, no norms, inputs that are already
+// cooked.  As above a block of four warps takes half of a unit; a row's saves come into shared memory by asynchronous copies, three
+// rows ahead.  Same delta rule, same rounding points (a bf16 state is rounded after every row), so the bits are the persistent
+// kernel's and the reference's.  Measured at 48 slots x 34 layers, accepted prefixes drawn from 0..16, bf16: 4.71 ms on the persistent
+// kernel, 3.63 ms with eight value rows a warp read straight from global memory; see recurrence_octet.cuh for the step.
+constexpr int kReplayAhead = 3;
+struct __align__(16) ReplayRow {
+    float k[DK], g[DK];
+    uint16_t v[DV];
     float beta;
 };
-__device__ __forceinline__ ReplayRow replay_row(const Params& p, long long kv_base, long long b_base, long long gr, int h, int uw, int lane) {
-    ReplayRow x;
-    const long long at = kv_base + (gr * p.H + h) * DK;
-    x.k = *reinterpret_cast<const float4*>(p.k_save + at + lane * 4);
-    x.g = *reinterpret_cast<const float4*>(p.g_save + at + lane * 4);
-    x.v = p.v_save[at + uw * kRowsPerLane + (lane >> 2)];
-    x.beta = p.b_save[b_base + gr * p.H + h];
-    return x;
-}
 
 template <typename S>
-__global__ void __launch_bounds__(kSmallThreads, sizeof(S) == 4 ? 6 : 8) replay_small_kernel(const __grid_constant__ Params p) {
+__global__ void __launch_bounds__(kSmallThreads, 4) replay_small_kernel(const __grid_constant__ Params p) {
+    static_assert((kReplayAhead & (kReplayAhead + 1)) == 0, "ring index");
+    __shared__ ReplayRow ring[kReplayAhead + 1];
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     const long long unit = blockIdx.x / kSmallParts;
-    const int uw = (int)(blockIdx.x % kSmallParts) * kSmallWarps + warp;  // this warp's place among the unit's 16
+    const int uw = (int)(blockIdx.x % kSmallParts) * kSmallWarps + warp;  // this warp's place among the unit's
     const int h = (int)(unit % p.H), layer = (int)((unit / p.H) % p.layers), b = (int)(unit / ((long long)p.H * p.layers));
     const long long r0 = p.cu_rows ? p.cu_rows[b] : 0;
     int rows = p.keep ? p.keep[b] : p.rows1;
@@ -1042,22 +1040,36 @@ __global__ void __launch_bounds__(kSmallThreads, sizeof(S) == 4 ? 6 : 8) replay_
     if (rows == 0 && !copies_state(p)) return;
     const long long s_elem = (long long)layer * p.state_stride + (p.state_off ? p.state_off[b] : 0) + (long long)h * DV * DK;
     const long long kv_base = (long long)layer * p.kv_stride, b_base = (long long)layer * p.b_stride;
-    f32x2 s[kPairs][4];
-    load_rows_global<S>(reinterpret_cast<const S*>(p.state_in) + s_elem, uw, lane, s);
-    ReplayRow cur{};
-    if (rows > 0) cur = replay_row(p, kv_base, b_base, r0, h, uw, lane);
-    for (int r = 0; r < rows; ++r) {
-        ReplayRow nxt = cur;
-        if (r + 1 < rows) nxt = replay_row(p, kv_base, b_base, r0 + r + 1, h, uw, lane);
-        const f32x2 kk[4] = {pack2(cur.k.x, cur.k.x), pack2(cur.k.y, cur.k.y), pack2(cur.k.z, cur.k.z), pack2(cur.k.w, cur.k.w)};
-        const f32x2 gg[4] = {pack2(cur.g.x, cur.g.x), pack2(cur.g.y, cur.g.y), pack2(cur.g.z, cur.g.z), pack2(cur.g.w, cur.g.w)};
-        delta_rule_v(s, kk, gg, bf16_bits_to_f32(cur.v), lane, cur.beta, p.neg_zero2);
-        if constexpr (sizeof(S) == 2) {
-            if (r + 1 < rows) round_rows(s);  // the last row's rounding is the store's
+    auto fetch = [&](int r) {  // 16 bytes of k or of the decay a thread, 8 of v; beta
+        if (r < rows) {
+            const long long rh = (r0 + r) * p.H + h, at = kv_base + rh * DK;
+            ReplayRow& x = ring[r & kReplayAhead];
+            if (t < 32) oct::copy16(&x.k[t * 4], p.k_save + at + t * 4);
+            else if (t < 64) oct::copy16(&x.g[(t - 32) * 4], p.g_save + at + (t - 32) * 4);
+            else if (t < 96) oct::copy8(&x.v[(t - 64) * 4], p.v_save + at + (t - 64) * 4);
+            else if (t == 96) oct::copy4(&x.beta, p.b_save + b_base + rh);
         }
-        cur = nxt;
+        oct::copies_commit();
+    };
+#pragma unroll
+    for (int r = 0; r < kReplayAhead; ++r) fetch(r);
+    f32x2 s[kR][oct::kRowPairs];
+    oct::load_rows(reinterpret_cast<const S*>(p.state_in) + s_elem, uw, lane, s);
+    const int mine = uw * 4 * kR + oct::row_of_lane<kR>(lane);
+    for (int r = 0; r < rows; ++r) {
+        oct::copies_wait<kReplayAhead - 1>();
+        __syncthreads();  // row r is there for all, and nobody reads row r - 1 any more
+        fetch(r + kReplayAhead);
+        const ReplayRow& x = ring[r & kReplayAhead];
+        f32x2 kk[oct::kRowPairs], gg[oct::kRowPairs];
+        oct::load_leaves(x.g, lane, gg);
+        oct::load_leaves(x.k, lane, kk);
+        oct::delta_rule(s, kk, gg, bf16_bits_to_f32(x.v[mine]), lane, x.beta, p.neg_zero2);
+        if constexpr (sizeof(S) == 2) {
+            if (r + 1 < rows) oct::round_rows(s);  // the last row's rounding is the store's
+        }
     }
-    store_rows_global<S>(reinterpret_cast<S*>(p.state_out) + s_elem, uw, lane, s);
+    oct::store_rows(reinterpret_cast<S*>(p.state_out) + s_elem, uw, lane, s);
 }
 
 template <typename S>
@@ -1217,14 +1229,14 @@ int replay_entry(int32_t heads, int32_t layers, int32_t batch, bool batched, con
     if (bf16_state && g_commit_mode.load() == 1)
         return commit_tc_launch(heads, layers, batch, cu_rows, keep, rows, state_in, state_out, state_stride, state_off, k_save, v_save, g_save,
                                 b_save, kv_stride, b_stride, (cudaStream_t)stream);
-    // The warp-per-eight-rows kernel takes aligned saves and grids that fit; GLM53F_KDA_REPLAY=pipeline keeps the
+    // The small-block kernel takes aligned saves and grids that fit; GLM53F_KDA_REPLAY=pipeline keeps the
     // persistent kernel.
     static const bool small = [] {
         const char* e = getenv("GLM53F_KDA_REPLAY");
         return !(e != nullptr && strcmp(e, "pipeline") == 0);
     }();
     auto al16 = [](const void* x) { return (reinterpret_cast<uintptr_t>(x) & 15) == 0; };
-    if (small && al16(k_save) && al16(g_save) && kv_stride % 4 == 0 && q.units * kSmallParts <= 0x7fffffffLL)
+    if (small && al16(k_save) && al16(g_save) && (reinterpret_cast<uintptr_t>(v_save) & 7) == 0 && kv_stride % 4 == 0 && q.units * kSmallParts <= 0x7fffffffLL)
         return bf16_state ? launch_replay_small<__nv_bfloat16>(q, (cudaStream_t)stream) : launch_replay_small<float>(q, (cudaStream_t)stream);
     return launch_typed<kReplay>(q, bf16_state, (cudaStream_t)stream);
 }
