@@ -260,8 +260,7 @@ struct UnitIter {
         }
     }
     __device__ __forceinline__ bool valid() const { return ok; }
-    // The current unit; advances to the next one and starts fetching its metadata.
-    __device__ __forceinline__ Unit take(const Params& p) {
+    __device__ __forceinline__ Unit current(const Params& p) const {
         Unit cur;
         cur.b = (int)b;
         cur.h = (int)h;
@@ -278,6 +277,11 @@ struct UnitIter {
         cur.s_elem = (long long)layer * p.state_stride + s_off + (long long)h * DV * DK;
         cur.conv_off = c_off;
         cur.a_log = a_log;
+        return cur;
+    }
+    // The current unit; advances to the next one and starts fetching its metadata.
+    __device__ __forceinline__ Unit take(const Params& p) {
+        const Unit cur = current(p);
         u += gridDim.x;
         ok = u < (unsigned long long)p.units;
         const unsigned H = (unsigned)p.H;
@@ -379,7 +383,22 @@ __device__ __forceinline__ uint32_t raw_row_bytes(const Params& p) {
     return MODE == kLayer ? (3 * TAPS + 2) * 256 + 16 : MODE == kCore ? 3 * 256 + 512 + 16 + (p.G ? 256 : 0) : 2 * 512 + 256 + 16;
 }
 
-template <typename S, int MODE>
+// A block's first row (layer calls), issued by the prologue's first four warps, four pieces each, as soon as they know the unit: bulk copies
+// of several lanes are issued one after the other, and the fifteen of a row took the mover 0.7 us, the state behind them (5 slots 338 ->
+// 326 us a step of 34 layers, 16 slots 593 -> 578).  The mover counts their bytes (before or after they land); a row that is not
+// aligned it copies itself, and all of a launch of one unit a block, whose prologue has the weights to fetch meanwhile (2 slots 205,
+// so 223).
+template <typename L>
+__device__ __forceinline__ void first_row(const Params& p, unsigned char* smem, uint64_t* raw_full, const Piece& x, const Unit& un, int warp, int lane) {
+    if (un.rows == 0 || warp >= 4) return;
+    const uintptr_t src = reinterpret_cast<uintptr_t>(x.at(un, 0));
+    if (__any_sync(0xffffffffu, !x.scalar && (src & 15) != 0)) return;
+    if (x.bytes && (lane >> 2) == warp)
+        bulk_load(smem + L::oRaw + x.off, reinterpret_cast<const void*>(src & ~uintptr_t(15)), x.scalar ? 16 : x.bytes, raw_full);
+    __syncwarp();
+}
+
+template <typename S, int MODE, bool ONE_UNIT>
 __device__ void mover_role(const Params& p, unsigned char* smem, uint64_t* bars, const WaitCtx& ctx, int lane) {
     using L = Smem<S, MODE>;
     uint64_t* st_full = bars;
@@ -418,7 +437,16 @@ __device__ void mover_role(const Params& p, unsigned char* smem, uint64_t* bars,
         if (un.rows == 0 && !copy0) continue;
         // A layer call's first row goes ahead of its state: the row has to be cooked before the state is wanted (5 slots 352 us a step, behind
         // it 369).
-        if (kRowFirst && first && un.rows > 0 && !row_in(un, 0)) return;
+        if (kRowFirst && first && un.rows > 0) {
+            const uintptr_t src = reinterpret_cast<uintptr_t>(x.at(un, 0));
+            if (ONE_UNIT || __any_sync(0xffffffffu, !x.scalar && (src & 15) != 0)) {
+                if (!row_in(un, 0)) return;
+            } else {  // the prologue's warps issue its copies (first_row)
+                if (lane == 0) mbar_arrive_expect_tx(&raw_full[raw.idx], raw_row_bytes<MODE>(p));
+                __syncwarp();
+                raw.next(L::kRawSlots);
+            }
+        }
         // The unit's state.
         if (!mbar_wait(&st_empty[st.idx], st.phase ^ 1u, ctx, kStatusWaitStateEmpty)) return;
         if (lane == 0) info[st.idx] = {un.s_elem, un.rows};
@@ -572,7 +600,13 @@ __device__ void layer_prologue_role(const Params& p, unsigned char* smem, uint64
     const bool copy0 = copies_state(p);
     const bool vec = ((reinterpret_cast<uintptr_t>(p.cw) | reinterpret_cast<uintptr_t>(p.dt_bias)) & 15) == 0;
     UnitIter<kLayer> units(p);
-    units.begin(p);
+    if constexpr (ONE_UNIT) {
+        units.begin(p);
+    } else {
+        const Piece x = piece_of<kLayer>(p, lane);
+        units.begin(p);
+        if (units.valid()) first_row<L>(p, smem, raw_full, x, units.current(p), warp, lane);
+    }
     constexpr int together = ONE_UNIT ? kTogetherRows : 1;
     constexpr int kTeams = kProWarpsOf<S, kLayer, ONE_UNIT> / kTeamWarps;
     int turn = 0, team_turn = 0;
@@ -903,7 +937,7 @@ __global__ void __launch_bounds__(kThreadsOf<S, MODE, ONE_UNIT>, 1) recurrent_ke
     } else if (warp == kRecWarps + kProWarps) {
         if (MODE != kReplay) epilogue_role<S, MODE>(p, smem, bars, ctx, lane);
     } else {
-        mover_role<S, MODE>(p, smem, bars, ctx, lane);
+        mover_role<S, MODE, ONE_UNIT>(p, smem, bars, ctx, lane);
     }
     // No thread leaves while bulk loads into this block's shared memory may still be in flight: the mover issues a
     // load only after its consumers freed the slot, and every consumer role waits for every load before it ends,
