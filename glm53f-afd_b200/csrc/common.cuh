@@ -215,9 +215,9 @@ constexpr float kLog2e = 1.4426950408889634f;
 // A launch that may begin while its predecessor in the stream drains; the kernel calls grid_ready() before its first access to
 // global memory, so the order of effects is a plain launch's.
 template <typename P>
-inline int launch_early(void (*kernel)(P), unsigned grid, unsigned threads, size_t smem, cudaStream_t stream, const P& p) {
+inline int launch_early(void (*kernel)(P), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream, const P& p) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
+    cfg.gridDim = grid;
     cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;

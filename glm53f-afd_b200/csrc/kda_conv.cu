@@ -33,6 +33,7 @@ __device__ __forceinline__ const uint16_t* stacked_row(const uint16_t* window, c
 }
 
 __global__ void __launch_bounds__(kThreadsShift) conv_shift_kernel(const ShiftJob job) {
+    grid_ready();
     const long long ch = ((long long)blockIdx.x * kThreadsShift + threadIdx.x) * kVec;
     if (ch >= job.channels) return;
     const int layer = blockIdx.y, req = blockIdx.z;
@@ -84,8 +85,7 @@ int conv_shift_launch(int32_t channels, int32_t layers, int32_t batch, const int
     job.windows = conv; job.window_layer_pitch = conv_stride; job.window_at = reinterpret_cast<const long long*>(conv_off);
     job.fresh = p; job.fresh_layer_pitch = p_layer_stride; job.fresh_row_pitch = p_stride;
     const dim3 grid(((channels + kVec - 1) / kVec + kThreadsShift - 1) / kThreadsShift, layers, batch);
-    conv_shift_kernel<<<grid, kThreadsShift, 0, stream>>>(job);
-    return (int)cudaGetLastError();
+    return launch_early(conv_shift_kernel, grid, kThreadsShift, 0, stream, job);
 }
 
 }  // namespace kda
