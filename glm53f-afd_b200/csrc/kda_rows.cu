@@ -16,6 +16,8 @@
 // states: 1,087 -> 402 us (0.5 us a row); four prompts: 1,222 us.  Measured against it at 701 rows: three rows in flight 406,
 // five blocks an SM (96 registers, spills) 515, four value rows a warp 451, rows through shared memory by asynchronous copies 457.
 //
+// Two prompts and more run rows_octet_kernel: there the work of an SM's warps counts, not a row's latency.
+//
 // Same arithmetic in the same order with the same rounding points (a bf16 state is rounded after every row, the read-out
 // before the norm): the chain's bits.
 
@@ -23,6 +25,7 @@
 #include "glm53f_kda.h"
 #include "kda_internal.h"
 #include "recurrence.cuh"
+#include "recurrence_octet.cuh"
 
 namespace kda {
 namespace {
@@ -115,6 +118,91 @@ __global__ void __launch_bounds__(kRowsThreads, kPerSm) rows_kernel(const __grid
     store_rows_global<S>(reinterpret_cast<S*>(p.state_out) + s_elem, uw, lane, s);
 }
 
+// The same for launches of more units than a row's latency matters to: eight lanes to a value row (recurrence_octet.cuh), four rows a thread,
+// so half a unit a block of four warps, the cooked rows through shared memory, four at a time.  701 rows of 2, 3 and 4 prompts, f32:
+// 699 -> 656, 1,037 -> 930 and 1,240 -> 1,206 us (bf16, 3: 1,187 -> 1,037); one prompt 403 -> 419, hence the line in rows_launch.
+constexpr int kOctR = 4, kOctParts = DV / (4 * kOctR * kRowsWarps);
+constexpr int kStageRows = 4, kStages = 3;  // rows that arrive and are waited for together, such groups in shared memory
+struct __align__(16) StagedRow {
+    float k[DK], g[DK], q[DK];
+    uint16_t v[DV];
+    float beta;
+};
+
+template <typename S>
+__global__ void __launch_bounds__(kRowsThreads, kPerSm) rows_octet_kernel(const __grid_constant__ RowsParams p) {
+    constexpr int R = kOctR;
+    __shared__ StagedRow ring[kStages][kStageRows];
+    grid_ready();
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    const unsigned unit = blockIdx.x / kOctParts;
+    const int uw = (int)(blockIdx.x % kOctParts) * kRowsWarps + warp;  // this warp's place among the unit's
+    const int h = (int)(unit % (unsigned)p.H), b = (int)(unit / (unsigned)p.H);
+    const int r0 = p.cu ? p.cu[b] : 0, all = p.cu ? p.cu[b + 1] - r0 : p.rows1;
+    const int n = min(max(all - p.row_shift, 0), p.pass_rows);
+    if (n == 0 && p.state_in == p.state_out) return;
+    const long long s_elem = (p.state_off ? p.state_off[b] : 0) + (long long)h * DV * DK;
+    const long long first = (long long)b * p.pass_rows * p.H + h;  // (row, head) index of the pass's row 0
+    auto fetch = [&](int stage) {  // 16 or 8 bytes a thread and row
+#pragma unroll
+        for (int i = 0; i < kStageRows; ++i) {
+            const int r = stage * kStageRows + i;
+            if (r >= n) break;
+            StagedRow& x = ring[stage % kStages][i];
+            const long long rh = first + (long long)r * p.H, at = rh * DK;
+            if (t < 32) oct::copy16(&x.k[t * 4], p.k + at + t * 4);
+            else if (t < 64) oct::copy16(&x.g[(t - 32) * 4], p.g + at + (t - 32) * 4);
+            else if (t < 96) oct::copy16(&x.q[(t - 64) * 4], p.q + at + (t - 64) * 4);
+            else oct::copy8(&x.v[(t - 96) * 4], p.v + at + (t - 96) * 4);
+            if (t == 0) oct::copy4(&x.beta, p.beta + rh);
+        }
+        oct::copies_commit();
+    };
+#pragma unroll
+    for (int i = 0; i < kStages - 1; ++i) fetch(i);
+    f32x2 s[R][oct::kRowPairs];
+    oct::load_rows(reinterpret_cast<const S*>(p.state_in) + s_elem, uw, lane, s);
+    // As above, a row's read-out is reduced together with the next row's k-product: lanes 0-3 of a group receive its four rows' k-products, lanes
+    // 4-7 the previous row's read-outs.
+    float sums[2 * R] = {};
+    const int mine = uw * 4 * R + (lane >> 3) * R + (lane & 3);  // the value row whose sums this lane receives
+    const bool reads_out = (lane & 4) != 0;
+    uint16_t* out = p.out + ((long long)r0 + p.row_shift) * p.out_stride + (long long)h * DV + mine;
+    for (int stage = 0; stage * kStageRows < n; ++stage) {
+        oct::copies_wait<kStages - 2>();
+        __syncthreads();  // the group is there for all, and nobody reads the one before any more
+        fetch(stage + kStages - 1);
+#pragma unroll
+        for (int i = 0; i < kStageRows; ++i) {
+            const int r = stage * kStageRows + i;
+            if (r >= n) break;
+            const StagedRow& x = ring[stage % kStages][i];
+            f32x2 kk[oct::kRowPairs], gg[oct::kRowPairs], qq[oct::kRowPairs];
+            oct::load_leaves(x.g, lane, gg);
+            oct::load_leaves(x.k, lane, kk);
+            const float v = bf16_bits_to_f32(x.v[mine]), beta = x.beta;
+            if constexpr (sizeof(S) == 2) {
+                if (r != 0) oct::round_rows(s);  // after a row's read-out; the last row's rounding is the store's
+            }
+            oct::decay_rows(s, gg, p.neg_zero2);
+            oct::rows_partial(s, kk, sums, p.neg_zero2);
+            const float sum = butterfly_of<2 * R>(sums, lane, 4);
+            if (r != 0) {
+                if (reads_out) *out = f32_to_bf16_bits(sum);
+                out += p.out_stride;
+            }
+            oct::update_rows<R, 1>(s, kk, (v - sum) * beta, lane, p.neg_zero2);
+            oct::load_leaves(x.q, lane, qq);
+            oct::rows_partial(s, qq, sums + R, p.neg_zero2);
+        }
+    }
+    if (n > 0) {
+        const float o = butterfly_of<2 * R>(sums, lane, 4);
+        if (reads_out) *out = f32_to_bf16_bits(o);
+    }
+    oct::store_rows(reinterpret_cast<S*>(p.state_out) + s_elem, uw, lane, s);
+}
+
 // The gated RMSNorm of every row (kda.cu:188-201), one warp per (row, head): `out` holds bf16(y) and receives the output.
 __global__ void __launch_bounds__(128) rows_norm_kernel(const __grid_constant__ RowsParams p) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -165,21 +253,27 @@ int launch(void (*kernel)(RowsParams), unsigned grid, const RowsParams& p, cudaS
 
 int rows_launch(RowsParams p, int batch, bool bf16_state, cudaStream_t stream) {
     p.neg_zero2 = 0x8000000080000000ull;
-    const long long blocks = (long long)p.H * batch * kParts;
-    if (blocks > 0x7fffffffLL) return kInvalid;
-    auto* kernel = bf16_state ? rows_kernel<__nv_bfloat16> : rows_kernel<float>;
+    const long long units = (long long)p.H * batch;
+    const bool many = units * kParts > 2LL * sm_count();  // more than two blocks of rows_kernel an SM, two warps a scheduler
+    const long long blocks = units * (many ? kOctParts : kParts);
+    if (units * kParts > 0x7fffffffLL) return kInvalid;
+    using Kernel = void (*)(RowsParams);
+    static const Kernel kernels[2][2] = {{rows_kernel<float>, rows_kernel<__nv_bfloat16>}, {rows_octet_kernel<float>, rows_octet_kernel<__nv_bfloat16>}};
+    const Kernel kernel = kernels[many][bf16_state];
     // Blocks that start while the prologue before them still fills most SMs would crowd onto the SMs that free up first, and
-    // a row takes as long as the fullest SM needs: shared memory nobody uses keeps a launch to its fair share of blocks per SM.
-    constexpr size_t kSmemPerSm = 227 * 1024;
+    // a row takes as long as the fullest SM needs: shared memory nobody uses keeps a launch to its fair share of blocks per SM (701 rows
+    // of two prompts without it 1,074 us, so 656).
+    constexpr size_t kSmemPerSm = 227 * 1024, kRing = kStages * kStageRows * sizeof(StagedRow);
+    const size_t own = many ? kRing : 0;
     const long long share = (blocks + sm_count() - 1) / sm_count();
-    const size_t pad = share < kPerSm ? kSmemPerSm / (size_t)(share + 1) + 1024 : 0;
-    static int configured[2] = {-1, -1};
+    const size_t pad = share < kPerSm ? kSmemPerSm / (size_t)(share + 1) + 1024 - own : 0;
+    static int configured[2][2] = {{-1, -1}, {-1, -1}};
     int dev = 0;
     cudaGetDevice(&dev);
-    if (configured[bf16_state] != dev) {
-        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemPerSm);
+    if (configured[many][bf16_state] != dev) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kSmemPerSm - own));
         if (e != cudaSuccess) return (int)e;
-        configured[bf16_state] = dev;
+        configured[many][bf16_state] = dev;
     }
     return launch(kernel, (unsigned)blocks, p, stream, pad);
 }

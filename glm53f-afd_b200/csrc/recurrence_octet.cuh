@@ -1,5 +1,5 @@
 // The exact recurrence step of recurrence.cuh with EIGHT lanes to a value row, for kernels in which many warps of several units share an
-// SM (the core entry points' exact verify, the commit replay).
+// SM (the core entry points' exact verify, the commit replay, the exact prefill of several prompts).
 //
 // The reference forms a sum over the 128 key channels as a warp does: a lane adds its four consecutive channels (a leaf) in order
 // from zero, then the xor butterfly 16, 8, 4, 2, 1 adds the 32 leaves.  Here lane 8g + j holds leaves j, j + 8, j + 16 and j + 24 of R
@@ -164,22 +164,30 @@ __device__ __forceinline__ float rows_dot(const f32x2 (&s)[R][kRowPairs], const 
     rows_partial(s, x, part, nz);
     return butterfly_of<R>(part, lane, 4);
 }
-// Reference kda.cu:38-53: decay, read with k, correct toward v.  `v_mine` is v at the value row whose sums the lane receives.
 template <int R>
-__device__ __forceinline__ void delta_rule(f32x2 (&s)[R][kRowPairs], const f32x2 (&kk)[kRowPairs], const f32x2 (&gg)[kRowPairs], float v_mine,
-                                           int lane, float beta, f32x2 nz) {
+__device__ __forceinline__ void decay_rows(f32x2 (&s)[R][kRowPairs], const f32x2 (&gg)[kRowPairs], f32x2 nz) {
 #pragma unroll
     for (int r = 0; r < R; ++r)
 #pragma unroll
         for (int i = 0; i < kRowPairs; ++i) s[r][i] = mul2(s[r][i], gg[i], nz);
-    const float mine = (v_mine - rows_dot(s, kk, lane, nz)) * beta;
+}
+// `d` is (v - k-product) * beta of the lane's group's row r in its lane r * STEP.
+template <int R, int STEP>
+__device__ __forceinline__ void update_rows(f32x2 (&s)[R][kRowPairs], const f32x2 (&kk)[kRowPairs], float d, int lane, f32x2 nz) {
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-        const float x = __shfl_sync(FULL, mine, (lane & 24) + r * (8 / R));
+        const float x = __shfl_sync(FULL, d, (lane & 24) + r * STEP);
         const f32x2 delta = pack2(x, x);
 #pragma unroll
         for (int i = 0; i < kRowPairs; ++i) s[r][i] = add2(s[r][i], mul2(kk[i], delta, nz));
     }
+}
+// Reference kda.cu:38-53: decay, read with k, correct toward v.  `v_mine` is v at the value row whose sums the lane receives.
+template <int R>
+__device__ __forceinline__ void delta_rule(f32x2 (&s)[R][kRowPairs], const f32x2 (&kk)[kRowPairs], const f32x2 (&gg)[kRowPairs], float v_mine,
+                                           int lane, float beta, f32x2 nz) {
+    decay_rows(s, gg, nz);
+    update_rows<R, 8 / R>(s, kk, (v_mine - rows_dot(s, kk, lane, nz)) * beta, lane, nz);
 }
 
 }  // namespace oct
