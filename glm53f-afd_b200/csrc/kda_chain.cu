@@ -4,17 +4,17 @@
 // (request, layer, head) for the commit replay).  Four roles, connected by mbarrier rings in shared memory:
 //
 //   mover (1 warp)      bulk-copies (cp.async.bulk) each unit's 128x128 state and each row's raw inputs from global
-//                       memory into shared-memory rings, several units ahead of the arithmetic;
-//   prologue (2 or 4 warps)  turns a row's raw inputs into q, k, v, the decay multipliers, beta and sigmoid(gate)
-//                       (short conv + SiLU, L2 norms, gates for the layer entry points, on four warps; exp(g) for the core ones,
-//                       on two);
+//                       memory into shared-memory rings, two or three units ahead of the arithmetic;
+//   prologue (2 to 8 warps)  turns a row's raw inputs into q, k, v, the decay multipliers, beta and sigmoid(gate)
+//                       (short conv + SiLU, L2 norms, gates for the layer entry points, on four or eight warps; exp(g) for the core
+//                       ones, on two; see kProWarpsOf);
 //   recurrence (16 warps) keeps the unit's state in registers across its rows: warp w owns value rows 8w..8w+7,
 //                       lane l key columns 4l..4l+3; per row the delta rule and the read-out; afterwards each warp
 //                       stores its own 8 rows, a whole contiguous row per instruction;
 //   epilogue (1 warp)   gated RMSNorm, bf16 outputs, replay saves.
 //
-// The state therefore crosses HBM once in each direction -- in as bulk transfers that are always several units deep
-// in flight, out as coalesced vector stores from the registers.  What roles load from global memory themselves (a unit's metadata, the
+// The state therefore crosses HBM once in each direction -- in as bulk transfers that are always two or three
+// units deep in flight, out as coalesced vector stores from the registers.  What roles load from global memory themselves (a unit's metadata, the
 // layer prologue's conv weights and biases) is fetched ahead of the wait for the row or unit it belongs to.
 //
 // Arithmetic contract (what makes this a drop-in for the reference's kernels/kda.cu): every sum over the 128 key
@@ -22,8 +22,9 @@
 // then the five-step xor butterfly over 32 lanes -- and nothing is contracted into an FMA (this file is compiled
 // with --fmad=false --ftz=false --prec-div=true --prec-sqrt=true, the reference's build.rs flags).  The butterfly
 // is evaluated as a reduce-scatter (kda.cu:30-33 applied to eight rows at once): the same additions in the same
-// pairing, so the same bits, with 9 shuffles for eight rows instead of 40.  decode, verify and replay share
-// `delta_rule`, so a replayed prefix of a window has the bits of serial single-row steps
+// pairing, so the same bits, with 9 shuffles for eight rows instead of 40.  The kernels on small blocks further down lay a row
+// across eight lanes (recurrence_octet.cuh) and add the same numbers in the same pairs, so a replayed prefix of a
+// window has the bits of serial single-row steps
 // (reference kernels/glm53f_kda.h:111-116, 166-168).
 //
 // Reference lines restated here: kernels/kda.cu:38-53 (update), 98-210 (chain_kernel), 214-253 (replay_kernel),
@@ -1305,9 +1306,9 @@ int core_entry(int32_t heads, int32_t batch, const int32_t* cu_rows, const glm53
     x.state_off = reinterpret_cast<const long long*>(state_off);
     x.out = out; x.out_stride = (long long)heads * DV;
     x.k_save = k_save; x.v_save = v_save; x.g_save = g_save; x.b_save = b_save;
-    // The exact verify (saves requested, inputs used as given, no fused output norm) runs on the small-block kernel: 16
-    // serial rows a unit are bound by instruction issue, and 32 resident warps an SM issue more than the persistent
-    // kernel's 16 (11.1 against 12.3 ms per step of 48 slots x 16 rows x 34 layers).  Single-row decode stays on the
+    // The exact verify (saves requested, inputs used as given, no fused output norm) runs on the small-block kernel: two
+    // units' serial rows at once wait less on their own latencies than the persistent kernel's one (before the present step 11.1
+    // against 12.3 ms per step of 48 slots x 16 rows x 34 layers).  Single-row decode stays on the
     // persistent kernel, which streams faster (4,263 against 3,500 GB/s at 16 slots: small blocks keep too few bytes in
     // flight).  GLM53F_KDA_DECODE=pipeline / small forces one or the other; the bits are the same either way.
     static const int forced = [] {

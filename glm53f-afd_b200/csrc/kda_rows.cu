@@ -7,13 +7,13 @@
 //   rows_norm_kernel                          the gated RMSNorm over every row, in place in `out`
 //
 // The persistent pipeline (kda_chain.cu) cooks, steps and normalises row after row on one SM per (request, head): 1.55 us a
-// row, 64 of 148 SMs busy for one prompt.  Here, as in the commit replay, a WARP is the unit of work -- eight of a unit's
+// row, 64 of 148 SMs busy for one prompt.  Here a WARP is the unit of work -- eight of a unit's
 // value rows never interact with the others --, reads what its lanes need of a cooked row straight into registers, rows
 // ahead, and meets no barrier; a unit's sixteen warps are four blocks, so a prompt of 64 heads puts work on every SM.
 //
 // What bounds it: a row is a chain of dependent steps (decayed state, k-product, five shuffles, update) with two warps a
-// scheduler for one prompt, the FP32 pipe (112 two-wide operations a row and warp) for four.  One prompt of 701 rows, f32
-// states: 1,087 -> 402 us (0.5 us a row); four prompts: 1,222 us.  Measured against it at 701 rows: three rows in flight 406,
+// scheduler (340 issue slots a row and warp, two-wide operations at 2.5 cycles).  One prompt of 701 rows, f32
+// states: 1,087 -> 402 us (0.5 us a row).  Measured against it at 701 rows: three rows in flight 406,
 // five blocks an SM (96 registers, spills) 515, four value rows a warp 451, rows through shared memory by asynchronous copies 457.
 //
 // Two prompts and more run rows_octet_kernel: there the work of an SM's warps counts, not a row's latency.
