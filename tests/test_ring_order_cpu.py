@@ -18,25 +18,27 @@ def waits():
     return [tuple(x) for x in lines if x]
 
 
-def stale_read(slots, order, seed, rows=40, single=0.0):
-    """One random run; whether a row was cooked before its copy had landed.  `single`: the share of rows cooked by all four warps."""
+def stale_read(slots, order, seed, rows=40, single=0.0, teams=1):
+    """One random run; whether a row was cooked before its copy had landed.  `single`: the share of rows cooked by a team of four warps,
+    the teams in turn."""
     r = random.Random(seed)
-    cooks, turn = [], 0
+    cooks, turn, team, warps = [], 0, 0, 4 * teams
     for _ in range(rows):
         if r.random() < single:
-            cooks.append((0, 1, 2, 3))
+            cooks.append(tuple(range(4 * (team % teams), 4 * (team % teams) + 4)))
+            team += 1
         else:
-            cooks.append((turn & 3,))
+            cooks.append((turn % warps,))
             turn += 1
     phases = {"raw_full": [0] * slots, "row_empty": [0] * slots}  # phases completed
-    raw_free, issued, released, landed, cooked, seen, at = [0] * slots, 0, 0, set(), set(), {}, [0] * 4
+    raw_free, issued, released, landed, cooked, seen, at = [0] * slots, 0, 0, set(), set(), {}, [0] * warps
     while released < rows:
         moves = [("land", x) for x in range(issued) if x not in landed]
         if issued < rows and raw_free[issued % slots] >= issued // slots:
             moves.append(("issue", issued))
         if released in cooked:
             moves.append(("release", released))
-        for w in range(4):
+        for w in range(warps):
             while at[w] < rows and w not in cooks[at[w]]:
                 at[w] += 1
             if at[w] < rows:
@@ -77,3 +79,10 @@ def test_no_row_is_read_before_it_has_landed(slots, single):
     assert len(orders) == 2 and all(len(o) == 2 for o in orders)  # rows cooked together, rows by one warp
     for order in set(orders):
         assert not any(stale_read(slots, order, seed, single=single) for seed in range(300)), order
+
+
+@pytest.mark.parametrize("slots", [6, 8])
+@pytest.mark.parametrize("single", [0.5, 0.9, 1.0])
+def test_two_teams_read_no_row_before_it_has_landed(slots, single):
+    for order in set(waits()):
+        assert not any(stale_read(slots, order, seed, single=single, teams=2) for seed in range(150)), order
