@@ -186,8 +186,8 @@ struct Smem {
     // States in flight: 96 KiB (bf16) or 128 KiB (f32).  More slow a long launch down, its reads then crowd out its writes (bf16 core, 5 and
     // 3 slots of the ring: 48 requests 1,303 and 1,220 us a step of 34 layers, 16 requests 462 and 459; 2: 1,214 and 488).
     static constexpr int kStateSlots = MODE == kReplay ? (sizeof(S) == 4 ? 3 : 5) : sizeof(S) == 4 ? 2 : 3;
-    static constexpr int kRawSlots = MODE == kLayer ? (sizeof(S) == 4 ? 6 : 8) : sizeof(S) == 4 ? 3 : 4;  // raw-row ring depth
-    static constexpr int kRowSlots = MODE == kLayer ? (sizeof(S) == 4 ? 6 : 8) : sizeof(S) == 4 ? 3 : 4;  // cooked-row ring depth
+    static constexpr int kRawSlots = MODE == kLayer ? (sizeof(S) == 4 ? 6 : 10) : sizeof(S) == 4 ? 3 : 4;  // raw-row ring depth
+    static constexpr int kRowSlots = MODE == kLayer ? (sizeof(S) == 4 ? 6 : 10) : sizeof(S) == 4 ? 3 : 4;  // cooked-row ring depth
     static constexpr int kRawBytes = align_up(RawOf<MODE>::T::BYTES, 128);
     static constexpr int oState = 0;
     static constexpr int oRaw = oState + kStateSlots * kStateBytes;
@@ -196,6 +196,9 @@ struct Smem {
     static constexpr int oBars = oScratch + 4 * DK * 4;
     // barriers: st_full[S], st_empty[S], raw_full[R], raw_empty[R], row_full[C], y_full[C], row_empty[C]
     static_assert(MODE != kLayer || kRawSlots == kRowSlots, "layer_prologue_role: a free cooked slot implies a finished raw slot");
+    // A warp sees its slots' parities only at its own rows; between two of them lie at most the other warps' windows' rows and a
+    // single row of the other team, and no parity may come round in that time.
+    static_assert(MODE != kLayer || kRowSlots > kProWarpsOf<S, kLayer>, "layer_prologue_role: rows between two of a warp's own");
     static constexpr int kBars = 2 * kStateSlots + 2 * kRawSlots + 3 * kRowSlots;
     static constexpr int oCtl = oBars + kBars * 8;  // progress, abort
     static constexpr int oUnits = oCtl + 16;        // UnitInfo per state slot

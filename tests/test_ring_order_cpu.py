@@ -81,8 +81,13 @@ def test_no_row_is_read_before_it_has_landed(slots, single):
         assert not any(stale_read(slots, order, seed, single=single) for seed in range(300)), order
 
 
-@pytest.mark.parametrize("slots", [6, 8])
-@pytest.mark.parametrize("single", [0.5, 0.9, 1.0])
+def test_the_model_finds_rings_too_short_for_two_teams():
+    order = ("row_empty", "raw_full")
+    assert any(stale_read(6, order, seed, single=0.5, teams=2) for seed in range(150))
+
+
+@pytest.mark.parametrize("slots", [9, 10])  # more than the eight warps: the rows between two of a warp's own
+@pytest.mark.parametrize("single", [0.1, 0.5, 0.9, 1.0])
 def test_two_teams_read_no_row_before_it_has_landed(slots, single):
     for order in set(waits()):
         assert not any(stale_read(slots, order, seed, single=single, teams=2) for seed in range(150)), order
