@@ -201,8 +201,9 @@ struct Smem {
     static_assert(MODE != kLayer || kRowSlots > kProWarpsOf<S, kLayer>, "layer_prologue_role: rows between two of a warp's own");
     static constexpr int kBars = 2 * kStateSlots + 2 * kRawSlots + 3 * kRowSlots;
     static constexpr int oCtl = oBars + kBars * 8;  // progress, abort
-    static constexpr int oUnits = oCtl + 16;        // UnitInfo per state slot
-    static constexpr int kBytes = oUnits + kStateSlots * 16;
+    static constexpr int oUnits = align_up(oCtl + 16, (int)alignof(UnitInfo));  // UnitInfo per state slot
+    static constexpr int kBytes = oUnits + kStateSlots * (int)sizeof(UnitInfo);
+    static_assert(oUnits % alignof(UnitInfo) == 0, "a UnitInfo is read and written whole");
     static_assert(kBytes <= 232448, "shared memory budget");
 };
 
