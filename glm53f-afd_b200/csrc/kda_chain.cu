@@ -1059,7 +1059,7 @@ int launch_small(const Params& p, cudaStream_t stream) {
 constexpr int kReplayAhead = 3;
 struct __align__(16) ReplayRow {
     float k[DK], g[DK];
-    uint16_t v[DV];
+    uint16_t v[DV + 4];  // the 8-byte words that hold the row's values: they begin v_lead elements in
     float beta;
 };
 
@@ -1079,14 +1079,16 @@ __global__ void __launch_bounds__(kSmallThreads, 4) replay_small_kernel(const __
     if (rows == 0 && !copies_state(p)) return;
     const long long s_elem = (long long)layer * p.state_stride + (p.state_off ? p.state_off[b] : 0) + (long long)h * DV * DK;
     const long long kv_base = (long long)layer * p.kv_stride, b_base = (long long)layer * p.b_stride;
+    // Values at any element: the aligned words around them are copied (rows and layers are multiples of four elements apart).
+    const int v_lead = (int)((reinterpret_cast<uintptr_t>(p.v_save) & 7) / 2);
     auto fetch = [&](int r) {  // 16 bytes of k or of the decay a thread, 8 of v; beta
         if (r < rows) {
             const long long rh = (r0 + r) * p.H + h, at = kv_base + rh * DK;
             ReplayRow& x = ring[r & kReplayAhead];
             if (t < 32) oct::copy16(&x.k[t * 4], p.k_save + at + t * 4);
             else if (t < 64) oct::copy16(&x.g[(t - 32) * 4], p.g_save + at + (t - 32) * 4);
-            else if (t < 96) oct::copy8(&x.v[(t - 64) * 4], p.v_save + at + (t - 64) * 4);
-            else if (t == 96) oct::copy4(&x.beta, p.b_save + b_base + rh);
+            else if (t < 96 || (t == 96 && v_lead != 0)) oct::copy8(&x.v[(t - 64) * 4], p.v_save + at - v_lead + (t - 64) * 4);
+            else if (t == 97) oct::copy4(&x.beta, p.b_save + b_base + rh);
         }
         oct::copies_commit();
     };
@@ -1103,7 +1105,7 @@ __global__ void __launch_bounds__(kSmallThreads, 4) replay_small_kernel(const __
         f32x2 kk[oct::kRowPairs], gg[oct::kRowPairs];
         oct::load_leaves(x.g, lane, gg);
         oct::load_leaves(x.k, lane, kk);
-        oct::delta_rule(s, kk, gg, bf16_bits_to_f32(x.v[mine]), lane, x.beta, p.neg_zero2);
+        oct::delta_rule(s, kk, gg, bf16_bits_to_f32(x.v[v_lead + mine]), lane, x.beta, p.neg_zero2);
         if constexpr (sizeof(S) == 2) {
             if (r + 1 < rows) oct::round_rows(s);  // the last row's rounding is the store's
         }
@@ -1268,14 +1270,14 @@ int replay_entry(int32_t heads, int32_t layers, int32_t batch, bool batched, con
     if (bf16_state && g_commit_mode.load() == 1)
         return commit_tc_launch(heads, layers, batch, cu_rows, keep, rows, state_in, state_out, state_stride, state_off, k_save, v_save, g_save,
                                 b_save, kv_stride, b_stride, (cudaStream_t)stream);
-    // The small-block kernel takes aligned saves and grids that fit; GLM53F_KDA_REPLAY=pipeline keeps the
+    // The small-block kernel takes k and decays on 16 bytes and grids that fit; GLM53F_KDA_REPLAY=pipeline keeps the
     // persistent kernel.
     static const bool small = [] {
         const char* e = getenv("GLM53F_KDA_REPLAY");
         return !(e != nullptr && strcmp(e, "pipeline") == 0);
     }();
     auto al16 = [](const void* x) { return (reinterpret_cast<uintptr_t>(x) & 15) == 0; };
-    if (small && al16(k_save) && al16(g_save) && (reinterpret_cast<uintptr_t>(v_save) & 7) == 0 && kv_stride % 4 == 0 && q.units * kSmallParts <= 0x7fffffffLL)
+    if (small && al16(k_save) && al16(g_save) && kv_stride % 4 == 0 && q.units * kSmallParts <= 0x7fffffffLL)
         return bf16_state ? launch_replay_small<__nv_bfloat16>(q, (cudaStream_t)stream) : launch_replay_small<float>(q, (cudaStream_t)stream);
     return launch_typed<kReplay>(q, bf16_state, (cudaStream_t)stream);
 }

@@ -1,5 +1,5 @@
-"""The commit replay whose saved values start at any element: those on 8 bytes run on the small-block kernel (csrc/kda_chain.cu,
-replay_entry), the others on the persistent one, with the same bits.  Prefix lengths around the rows kept in flight."""
+"""The commit replay whose saved values start at any element: all run on the small-block kernel (csrc/kda_chain.cu,
+replay_entry), with the bits of aligned values.  Prefix lengths around the rows kept in flight."""
 import ctypes
 import importlib
 
@@ -36,3 +36,35 @@ def test_values_at_any_element(rows, shift):
     moved[shift:shift + n * DK] = v
     got, want = run(moved[shift:]), run(v)
     assert torch.equal(got, want) and (rows > 0 or torch.equal(got, state))
+
+
+@pytest.mark.parametrize("state", ["f32", "bf16"])
+@pytest.mark.parametrize("shift", [0, 1, 2, 3, 4])
+def test_a_batch_of_layers_on_the_small_block_kernel(shift, state):
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from captured import launches
+
+    core = importlib.import_module("glm53f-afd_b200.core")
+    h, layers, keep = 3, 2, [4, 0, 7, 1]
+    rows, n, per = [5, 2, 7, 3], 17 * h, h * DK * DK
+    gen = torch.Generator(device="cuda").manual_seed(shift)
+    rn = lambda m: torch.randn(m, device="cuda", generator=gen)
+    k = torch.nn.functional.normalize(rn(layers * n * DK).view(-1, DK)).view(-1)
+    v, g, beta = rn(layers * n * DK).bfloat16(), torch.exp(torch.nn.functional.logsigmoid(rn(layers * n * DK) + 3)), torch.sigmoid(rn(layers * n))
+    states = rn(layers * len(rows) * per).to(torch.bfloat16 if state == "bf16" else torch.float32)
+    cu = torch.tensor([0, 5, 7, 14, 17], dtype=torch.int32, device="cuda")
+    kept = torch.tensor(keep, dtype=torch.int32, device="cuda")
+    off = torch.arange(len(rows), dtype=torch.int64, device="cuda") * per
+    moved = torch.zeros(v.numel() + 8, dtype=torch.bfloat16, device="cuda")
+    moved[shift:shift + v.numel()] = v
+
+    def run(vv, st):
+        core.commit_batch(h, layers, cu, kept, st, len(rows) * per, off, (k, vv, g, beta), n * DK, n)
+        return st
+
+    got, want = run(moved[shift:], states.clone()), run(v, states.clone())
+    torch.cuda.synchronize()
+    assert torch.equal(got, want) and not torch.equal(got, states)
+    names, _ = launches(lambda: run(moved[shift:], got))
+    assert len(names) == 1 and "replay_small_kernel" in names[0], names
