@@ -254,7 +254,10 @@ int launch(void (*kernel)(RowsParams), unsigned grid, const RowsParams& p, cudaS
 int rows_launch(RowsParams p, int batch, bool bf16_state, cudaStream_t stream) {
     p.neg_zero2 = 0x8000000080000000ull;
     const long long units = (long long)p.H * batch;
-    const bool many = units * kParts > 2LL * sm_count();  // more than two blocks of rows_kernel an SM, two warps a scheduler
+    // From four blocks of rows_kernel on some SM, four warps a scheduler.  Up to three a row's latency still counts: 256 rows, f32, 80, 96 and
+    // 104 units 192, 199 and 209 us on rows_kernel, 222, 227 and 234 on the other; 112, 128 and 208 units 246, 256 and 391 against 235, 242 and 348
+    // (bf16 219, 224 and 232 against 250, 255 and 261; 280, 287 and 439 against 263, 269 and 384).
+    const bool many = units * kParts > 3LL * sm_count();
     const long long blocks = units * (many ? kOctParts : kParts);
     if (units * kParts > 0x7fffffffLL) return kInvalid;
     using Kernel = void (*)(RowsParams);

@@ -37,3 +37,27 @@ def test_many_units_have_the_chains_bits(lens, pass_rows, state, in_place):
         got.append((out, st if in_place else other))
     for a, b in zip(*got):
         assert torch.equal(a.view(torch.int16), b.view(torch.int16))
+
+
+@pytest.mark.parametrize("quarters, octet", [(3, False), (4, True)])
+def test_which_kernel_takes_how_many_units(quarters, octet):
+    """A unit is four blocks of rows_kernel: up to three of them on an SM a row's latency counts, beyond that the work of its warps."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from captured import launches
+
+    K = importlib.import_module("glm53f-afd_b200.kernel")
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    h, n = (quarters * sms // 4 - (0 if octet else 1)) // 2, 2
+    c, width, total = K.channels(h), h * DK, 16 * n
+    zb = lambda m: K.DeviceBuffer(torch.zeros(m, dtype=torch.bfloat16, device="cuda").view(torch.uint8))
+    zf = lambda m: K.DeviceBuffer(torch.zeros(m, device="cuda").view(torch.uint8))
+    w = K.Weights(h, zb(c * 4), zf(h), zf(width), zb(DK), 1e-5, -5.0)
+    meta, gates, stride = K.BatchMeta.new(n), zb(total * 2 * width), (c + h + 7) // 8 * 8
+    meta.set([K.Request(16, i * 3 * c, i * K.state_len(h)) for i in range(n)])
+    call = K.PrefillBatch(w, K.RowView.dense(zb(total * stride), stride), c, K.RowView.new(gates, 0, 2 * width), K.RowView.new(gates, width, 2 * width),
+                          zb(n * 3 * c), zf(n * K.state_len(h)), K.StateOut.InPlace, K.RowView.dense(zb(total * width), width), 0,
+                          K.PrefillWorkspace.new(h, n, 16))
+    call.launch(meta, K.Stream())
+    names, _ = launches(lambda: call.launch(meta, K.Stream()))
+    assert any("rows_octet_kernel" in x for x in names) == octet and any("rows_kernel" in x for x in names) != octet, names
