@@ -983,10 +983,10 @@ __global__ void __launch_bounds__(kThreadsOf<S, MODE, ONE_UNIT>, 1) recurrent_ke
 // of two buffers, so a row takes one barrier), steps through the request's rows and stores its rows of the state back.  No rings, no
 // bulk copies: four such blocks on an SM are two units' serial rows at once.  Used for the exact verify; for single-row
 // decode the persistent kernel above streams faster.
-constexpr int kSmallWarps = 4, kSmallThreads = kSmallWarps * 32, kR = 4, kSmallParts = DV / (4 * kR * kSmallWarps);
+constexpr int kSmallWarps = 4, kSmallThreads = kSmallWarps * 32, kR = 4, kSmallParts = DV / (4 * kR * kSmallWarps), kSmallPerSm = 4;
 
 template <typename S>
-__global__ void __launch_bounds__(kSmallThreads, 4) core_small_kernel(const __grid_constant__ Params p) {
+__global__ void __launch_bounds__(kSmallThreads, kSmallPerSm) core_small_kernel(const __grid_constant__ Params p) {
     __shared__ __align__(16) float sq[2][DK], sk[2][DK], sg[2][DK], sv[2][DV];
     __shared__ float sbeta[2];
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -1086,7 +1086,7 @@ struct __align__(16) ReplayRow {
 };
 
 template <typename S>
-__global__ void __launch_bounds__(kSmallThreads, 4) replay_small_kernel(const __grid_constant__ Params p) {
+__global__ void __launch_bounds__(kSmallThreads, kSmallPerSm) replay_small_kernel(const __grid_constant__ Params p) {
     static_assert((kReplayAhead & (kReplayAhead + 1)) == 0, "ring index");
     __shared__ ReplayRow ring[kReplayAhead + 1];
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -1135,6 +1135,57 @@ __global__ void __launch_bounds__(kSmallThreads, 4) replay_small_kernel(const __
     oct::store_rows(reinterpret_cast<S*>(p.state_out) + s_elem, uw, lane, s);
 }
 
+// A launch whose blocks find an SM each -- a layer's replay of a few heads -- is over when its longest chain of rows is.  A warp then
+// takes eight value rows on the step of recurrence.cuh: what a lane needs of a saved row is a 16-byte piece of k and of the decay, one v and
+// beta, loaded into registers while the row before is worked on; nothing is shared, so no row waits at a barrier.  (16 rows, 16 units, 34
+// launches: 225 us f32, 265 bf16; on replay_small_kernel 340 and 382; rows two or three ahead in registers 240 to 270 and 272 to 406.)
+constexpr int kFewParts = kRecWarps / kSmallWarps;
+struct FewRow {
+    float4 k, g;
+    uint16_t v;  // bf16 bits, widened when the row's turn comes: a conversion at the load would wait for it there and then
+    float beta;
+};
+__device__ __forceinline__ FewRow few_row(const Params& p, long long kv_base, long long b_base, long long gr, int h, int uw, int lane) {
+    FewRow x;
+    const long long at = kv_base + (gr * p.H + h) * DK;
+    x.k = *reinterpret_cast<const float4*>(p.k_save + at + lane * 4);
+    x.g = *reinterpret_cast<const float4*>(p.g_save + at + lane * 4);
+    x.v = p.v_save[at + uw * kRowsPerLane + (lane >> 2)];
+    x.beta = p.b_save[b_base + gr * p.H + h];
+    return x;
+}
+
+template <typename S>
+__global__ void __launch_bounds__(kSmallThreads, sizeof(S) == 4 ? 6 : 8) replay_few_kernel(const __grid_constant__ Params p) {
+    grid_ready();
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    const long long unit = blockIdx.x / kFewParts;
+    const int uw = (int)(blockIdx.x % kFewParts) * kSmallWarps + warp;  // this warp's place among the unit's 16
+    const int h = (int)(unit % p.H), layer = (int)((unit / p.H) % p.layers), b = (int)(unit / ((long long)p.H * p.layers));
+    const long long r0 = p.cu_rows ? p.cu_rows[b] : 0;
+    int rows = p.keep ? p.keep[b] : p.rows1;
+    if (rows < 0) rows = 0;
+    if (rows == 0 && !copies_state(p)) return;
+    const long long s_elem = (long long)layer * p.state_stride + (p.state_off ? p.state_off[b] : 0) + (long long)h * DV * DK;
+    const long long kv_base = (long long)layer * p.kv_stride, b_base = (long long)layer * p.b_stride;
+    f32x2 s[kPairs][4];
+    load_rows_global<S>(reinterpret_cast<const S*>(p.state_in) + s_elem, uw, lane, s);
+    FewRow cur{};
+    if (rows > 0) cur = few_row(p, kv_base, b_base, r0, h, uw, lane);
+    for (int r = 0; r < rows; ++r) {
+        FewRow nxt = cur;
+        if (r + 1 < rows) nxt = few_row(p, kv_base, b_base, r0 + r + 1, h, uw, lane);
+        const f32x2 kk[4] = {pack2(cur.k.x, cur.k.x), pack2(cur.k.y, cur.k.y), pack2(cur.k.z, cur.k.z), pack2(cur.k.w, cur.k.w)};
+        const f32x2 gg[4] = {pack2(cur.g.x, cur.g.x), pack2(cur.g.y, cur.g.y), pack2(cur.g.z, cur.g.z), pack2(cur.g.w, cur.g.w)};
+        delta_rule_v(s, kk, gg, bf16_bits_to_f32(cur.v), lane, cur.beta, p.neg_zero2);
+        if constexpr (sizeof(S) == 2) {
+            if (r + 1 < rows) round_rows(s);  // the last row's rounding is the store's
+        }
+        cur = nxt;
+    }
+    store_rows_global<S>(reinterpret_cast<S*>(p.state_out) + s_elem, uw, lane, s);
+}
+
 template <typename S>
 int launch_replay_small(const Params& p, cudaStream_t stream) {
     Params q = p;
@@ -1143,17 +1194,38 @@ int launch_replay_small(const Params& p, cudaStream_t stream) {
         const char* v = getenv("GLM53F_KDA_PDL");
         return !(v && v[0] == '0');
     }();
+    // Up to a block an SM with bf16 states, to three on four SMs with f32 ones.  34 launches of 16 rows, bf16, 37 and 38 units: 319 and (three rounds
+    // of four blocks) 805 us on the one, 374 and 374 on the other; f32, 24 and 32: 288 and 426 against 332 and 346.
+    const long long sms = sm_count();
+    const bool few = p.units * kFewParts * (sizeof(S) == 4 ? 4 : 3) <= 3 * sms;
+    const long long blocks = p.units * (few ? kFewParts : kSmallParts);
+    auto* kernel = few ? replay_few_kernel<S> : replay_small_kernel<S>;
+    // Blocks that start while the launch before them still runs would crowd onto the SMs that it left free, and a launch takes as
+    // long as the fullest SM: shared memory that nobody uses keeps it to its fair share of blocks an SM (34 launches of 16 rows, 64 units, f32 and
+    // bf16: 729 and 800 us without it, 368 and 396 so).
+    constexpr size_t kSmemPerSm = 227 * 1024, kMostPad = kSmemPerSm / 2 + 1024;
+    const size_t own = few ? 0 : (kReplayAhead + 1) * sizeof(ReplayRow);
+    const long long share = (blocks + sms - 1) / sms;
+    const size_t pad = share < kSmallPerSm ? kSmemPerSm / (size_t)(share + 1) + 1024 - own : 0;
+    static int configured[2] = {-1, -1};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (configured[few] != dev) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMostPad);
+        if (e != cudaSuccess) return (int)e;
+        configured[few] = dev;
+    }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(p.units * kSmallParts));
+    cfg.gridDim = dim3((unsigned)blocks);
     cfg.blockDim = dim3(kSmallThreads);
-    cfg.dynamicSmemBytes = 0;
+    cfg.dynamicSmemBytes = pad;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl ? 1 : 0;
-    return (int)cudaLaunchKernelEx(&cfg, replay_small_kernel<S>, q);
+    return (int)cudaLaunchKernelEx(&cfg, kernel, q);
 }
 
 // Core launches: when a state's slot is free for the next one.  At once, the next read is as early as can be, which is what a launch of few

@@ -46,7 +46,7 @@ def test_a_batch_of_layers_on_the_small_block_kernel(shift, state):
     from captured import launches
 
     core = importlib.import_module("glm53f-afd_b200.core")
-    h, layers, keep = 3, 2, [4, 0, 7, 1]
+    h, layers, keep = 3, 4, [4, 0, 7, 1]  # 48 units: more than find an SM for each of their blocks
     rows, n, per = [5, 2, 7, 3], 17 * h, h * DK * DK
     gen = torch.Generator(device="cuda").manual_seed(shift)
     rn = lambda m: torch.randn(m, device="cuda", generator=gen)
@@ -68,3 +68,37 @@ def test_a_batch_of_layers_on_the_small_block_kernel(shift, state):
     assert torch.equal(got, want) and not torch.equal(got, states)
     names, _ = launches(lambda: run(moved[shift:], got))
     assert len(names) == 1 and "replay_small_kernel" in names[0], names
+
+
+@pytest.mark.parametrize("state", ["f32", "bf16"])
+@pytest.mark.parametrize("rows", [0, 1, 2, 3, 4, 5, 17])
+def test_few_units_have_the_bits_of_many(rows, state):
+    """Launches whose blocks find an SM each run replay_few_kernel: layer by layer the bits of all layers in one launch."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from captured import launches
+
+    core = importlib.import_module("glm53f-afd_b200.core")
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    h = 3 * sms // 16 if state == "f32" else sms // 4  # the most units that run there
+    layers, n, per = 3, max(rows, 1) * h, h * DK * DK
+    gen = torch.Generator(device="cuda").manual_seed(rows)
+    rn = lambda m: torch.randn(m, device="cuda", generator=gen)
+    k = torch.nn.functional.normalize(rn(layers * n * DK).view(-1, DK)).view(-1)
+    v, g, beta = rn(layers * n * DK).bfloat16(), torch.exp(torch.nn.functional.logsigmoid(rn(layers * n * DK) + 3)), torch.sigmoid(rn(layers * n))
+    states = rn(layers * per).to(torch.bfloat16 if state == "bf16" else torch.float32)
+    cu, kept, off = (torch.tensor(x, dtype=d, device="cuda") for x, d in (([0, rows], torch.int32), ([rows], torch.int32), ([0], torch.int64)))
+
+    def run(st, first, count):
+        a, b = slice(first * n * DK, (first + count) * n * DK), slice(first * n, (first + count) * n)
+        core.commit_batch(h, count, cu, kept, st[first * per:], per, off, (k[a], v[a], g[a], beta[b]), n * DK, n)
+
+    many, few = states.clone(), states.clone()
+    run(many, 0, layers)
+    for layer in range(layers):
+        run(few, layer, 1)
+    torch.cuda.synchronize()
+    assert torch.equal(many, few) and torch.equal(many, states) == (rows == 0)
+    for count, kernel in ((1, "replay_few_kernel"), (layers, "replay_small_kernel")):
+        names, _ = launches(lambda: run(few, 0, count))
+        assert len(names) == 1 and kernel in names[0], names
