@@ -1229,12 +1229,13 @@ int launch_replay_small(const Params& p, cudaStream_t stream) {
 }
 
 // Core launches: when a state's slot is free for the next one.  At once, the next read is as early as can be, which is what a launch of few
-// units a block wants (bf16, 16 slots 460 us a step of 34 layers against 485; 30 slots 780 against 795); many units are through
-// sooner when reads keep less far ahead of the writes (48 slots 1,219 against 1,204; f32 states, 5, 16 and 40 slots: 371, 850 and 2,013
-// against 385, 843 and 1,945).  The line lies between 13 and 21 bf16 units a block, 2 and 7 f32 ones.
+// units a block wants; many units are through sooner when reads keep less far ahead of the writes.  Single rows, us a step of 34 layers,
+// early and late: bf16, 16, 32, 40 and 44 slots 458 and 484, 833 and 845, 1,031 and 1,038, 1,121 and 1,124; 46 slots 1,165 and
+// 1,160; 48 and 56 the same within 0.2 %; 64 slots 1,587 and 1,558.  f32, 8, 12 and 15 slots 460 and 504, 657 and 687, 817 and 819; 16, 20 and 32 slots 852 and 844, 1,067 and
+// 1,045, 1,655 and 1,599.  So the lines: 19.5 bf16 units a block (44 slots of 64 heads are 19.0, 46 are 19.9) and 6.75 f32 ones (15 are 6.5, 16 are 6.9).
 // (An instance of the kernel to itself: the choice inside cost 16 slots 1 %.)
 template <typename S>
-bool late_release(long long units, long long sms) { return units * DV * DK * (long long)sizeof(S) > sms * 432 * 1024; }
+bool late_release(long long units, long long sms) { return 4 * units > sms * (sizeof(S) == 4 ? 27 : 78); }
 
 template <typename S, int MODE, bool ONE_UNIT = false, bool LATE = false>
 int launch(const Params& p, cudaStream_t stream) {
