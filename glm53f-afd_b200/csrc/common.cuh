@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <cstdlib>
+
 namespace kda {
 
 constexpr int DK = 128, DV = 128, TAPS = 4, WINDOW = 3;
@@ -212,8 +214,19 @@ __device__ __forceinline__ float ex2_approx(float x) {
 }
 constexpr float kLog2e = 1.4426950408889634f;
 
-// A launch that may begin while its predecessor in the stream drains; the kernel calls grid_ready() before its first access to
-// global memory, so the order of effects is a plain launch's.
+// The attribute of a launch that may begin while its predecessor in the stream drains, and how many attributes that are: none with
+// GLM53F_KDA_PDL=0, which makes every launch of the library a plain one.  The kernel waits (griddepcontrol.wait) before its first
+// access to global memory, so the order of effects is a plain launch's.
+inline unsigned early_attribute(cudaLaunchAttribute& at) {
+    static const bool early = [] {
+        const char* e = getenv("GLM53F_KDA_PDL");
+        return !(e != nullptr && e[0] == '0');
+    }();
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    return early ? 1 : 0;
+}
+// Such a launch of a kernel that calls grid_ready().
 template <typename P>
 inline int launch_early(void (*kernel)(P), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream, const P& p) {
     cudaLaunchConfig_t cfg = {};
@@ -222,10 +235,8 @@ inline int launch_early(void (*kernel)(P), dim3 grid, unsigned threads, size_t s
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = early_attribute(attr[0]);
     return (int)cudaLaunchKernelEx(&cfg, kernel, p);
 }
 __device__ __forceinline__ void grid_ready() {

@@ -1055,20 +1055,14 @@ template <typename S>
 int launch_small(const Params& p, cudaStream_t stream) {
     Params q = p;
     q.neg_zero2 = 0x8000000080000000ull;
-    static const bool pdl = [] {
-        const char* v = getenv("GLM53F_KDA_PDL");
-        return !(v && v[0] == '0');
-    }();
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(p.units * kSmallParts));
     cfg.blockDim = dim3(kSmallThreads);
     cfg.dynamicSmemBytes = 0;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
+    cfg.numAttrs = early_attribute(attr[0]);
     return (int)cudaLaunchKernelEx(&cfg, core_small_kernel<S>, q);
 }
 
@@ -1190,10 +1184,6 @@ template <typename S>
 int launch_replay_small(const Params& p, cudaStream_t stream) {
     Params q = p;
     q.neg_zero2 = 0x8000000080000000ull;
-    static const bool pdl = [] {
-        const char* v = getenv("GLM53F_KDA_PDL");
-        return !(v && v[0] == '0');
-    }();
     // Up to a block an SM with bf16 states, to three on four SMs with f32 ones.  34 launches of 16 rows, bf16, 37 and 38 units: 319 and (three rounds
     // of four blocks) 805 us on the one, 374 and 374 on the other; f32, 24 and 32: 288 and 426 against 332 and 346.
     const long long sms = sm_count();
@@ -1221,10 +1211,8 @@ int launch_replay_small(const Params& p, cudaStream_t stream) {
     cfg.dynamicSmemBytes = pad;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
+    cfg.numAttrs = early_attribute(attr[0]);
     return (int)cudaLaunchKernelEx(&cfg, kernel, q);
 }
 
@@ -1264,21 +1252,15 @@ int launch(const Params& p, cudaStream_t stream) {
     q.skip_first_state = g_skip_first_state;
     g_skip_first_state = 0;
     // Launched with programmatic stream serialization: the kernel itself waits for its predecessors before its first
-    // global access, so ordering is what a plain launch gives.  GLM53F_KDA_PDL=0 selects a plain launch.
-    static const bool pdl = [] {
-        const char* v = getenv("GLM53F_KDA_PDL");
-        return !(v && v[0] == '0');
-    }();
+    // global access, so ordering is what a plain launch gives.
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(kThreadsOf<S, MODE, ONE_UNIT>);
     cfg.dynamicSmemBytes = L::kBytes;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
+    cfg.numAttrs = early_attribute(attr[0]);
     return (int)cudaLaunchKernelEx(&cfg, recurrent_kernel<S, MODE, ONE_UNIT, LATE>, q);
 }
 

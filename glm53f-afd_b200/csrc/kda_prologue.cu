@@ -333,8 +333,8 @@ template <int SINK>
 int launch(const ProParams& pp, cudaStream_t stream) {
     const long long blocks = (long long)pp.batch * pp.H * (pp.pass_rows / 4);
     if (blocks > 0x7fffffffLL) return kInvalid;
-    // Begun while the launch before drains: a chunked round of 4 slots 755 -> 703 us, of 12 slots x 8 rows 1,600 -> 1,565.  (The prefill
-    // sink below is the faster for a plain launch.)
+    // Begun while the launch before drains: a chunked round of 4 slots 755 -> 703 us, of 12 slots x 8 rows 1,600 -> 1,565.  (The prefill's
+    // prologue, launched further down, is the faster for a plain launch.)
     return launch_early(layer_prologue_kernel<SINK>, (unsigned)blocks, 128, 0, stream, pp);
 }
 

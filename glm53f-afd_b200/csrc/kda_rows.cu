@@ -235,20 +235,6 @@ __global__ void __launch_bounds__(128) rows_norm_kernel(const __grid_constant__ 
     *reinterpret_cast<uint2*>(dst) = make_uint2((uint32_t)o[0] | ((uint32_t)o[1] << 16), (uint32_t)o[2] | ((uint32_t)o[3] << 16));
 }
 
-int launch(void (*kernel)(RowsParams), unsigned grid, const RowsParams& p, cudaStream_t stream, size_t smem = 0) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.dynamicSmemBytes = smem;
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(kRowsThreads);
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // the kernels wait for their predecessors themselves
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return (int)cudaLaunchKernelEx(&cfg, kernel, p);
-}
-
 }  // namespace
 
 int rows_launch(RowsParams p, int batch, bool bf16_state, cudaStream_t stream) {
@@ -278,13 +264,13 @@ int rows_launch(RowsParams p, int batch, bool bf16_state, cudaStream_t stream) {
         if (e != cudaSuccess) return (int)e;
         configured[many][bf16_state] = dev;
     }
-    return launch(kernel, (unsigned)blocks, p, stream, pad);
+    return launch_early(kernel, (unsigned)blocks, kRowsThreads, pad, stream, p);
 }
 
 int rows_norm_launch(const RowsParams& p, int batch, cudaStream_t stream) {
     const long long blocks = (long long)p.H * batch * ((p.max_rows + 3) / 4);
     if (blocks > 0x7fffffffLL) return kInvalid;
-    return blocks == 0 ? 0 : launch(rows_norm_kernel, (unsigned)blocks, p, stream);
+    return blocks == 0 ? 0 : launch_early(rows_norm_kernel, (unsigned)blocks, kRowsThreads, 0, stream, p);
 }
 
 }  // namespace kda

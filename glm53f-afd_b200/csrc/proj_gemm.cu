@@ -32,7 +32,6 @@
 
 #include <cuda.h>
 
-#include <cstdlib>
 
 #include "common.cuh"
 #include "glm53f_proj.h"
@@ -373,17 +372,8 @@ int launch_one(GemmParams& p, long long clusters, cudaStream_t stream) {
     cfg.stream = stream;
     // Programmatic stream serialization: the kernel waits for its predecessors itself (grid_dependency_wait) before its
     // first global access, so its blocks' set-up (barriers, tensor memory, descriptor fetch) overlaps their tail.
-    static const bool pdl = [] {
-        const char* v = getenv("GLM53F_KDA_PDL");
-        return !(v && v[0] == '0');
-    }();
     cudaLaunchAttribute attr[2];
-    int na = 0;
-    if (pdl) {
-        attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[na].val.programmaticStreamSerializationAllowed = 1;
-        ++na;
-    }
+    unsigned na = early_attribute(attr[0]);
     if (KS > 1) {
         attr[na].id = cudaLaunchAttributeClusterDimension;
         attr[na].val.clusterDim.x = (unsigned)KS;

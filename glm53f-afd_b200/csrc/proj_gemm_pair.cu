@@ -381,10 +381,8 @@ int proj_gemm_pair_launch(const PairProblem* problems, int n, int* status, cudaS
     attr[0].val.clusterDim.x = 2;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
-    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 2;
+    cfg.numAttrs = 1 + early_attribute(attr[1]);
     return (int)cudaLaunchKernelEx(&cfg, kernel, p);
 }
 
