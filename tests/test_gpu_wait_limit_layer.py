@@ -11,10 +11,12 @@ DK = 128
 
 
 # As many heads as SMs: block 0 has (0, head 0) and then a unit of the next request.  Rows beyond the ring
-# (5 rows with f32 states, 8 with bf16) put the waits that run out into different warps; [2, 1, 9] ends among single rows; one request alone
-# is a launch of one unit a block.
+# (6 rows with f32 states, 10 with bf16) put the waits that run out into different warps; [2, 1, 9] ends among single rows; one request alone
+# is a launch of one unit a block.  bf16 launches of several units a block have two teams of four warps, which take single rows in turn: in
+# [13, 1, 1] and [15, 1, 1, 1] rows 12 to 14 of the window, stuck behind the ring, are those of warps 4 to 6, which then meet their
+# own team's vote.
 @pytest.mark.parametrize("state", ["f32", "bf16"])
-@pytest.mark.parametrize("lens", [[6, 1], [9, 1, 1], [11, 1], [2, 1, 9], [8, 3, 1], [8], [9]])
+@pytest.mark.parametrize("lens", [[6, 1], [9, 1, 1], [11, 1], [2, 1, 9], [8, 3, 1], [8], [9], [11], [12], [13, 1, 1], [15, 1, 1, 1]])
 def test_every_warp_leaves_when_a_wait_runs_out(pkg, lens, state):
     if not torch.cuda.is_available():
         pytest.skip("no CUDA device")
