@@ -18,6 +18,15 @@ def waits():
     return [tuple(x) for x in lines if x]
 
 
+def depths():
+    """The rings' depths with f32 and with bf16 states, in layer calls."""
+    with open(SOURCE) as f:
+        text = f.read()
+    rings = [re.search(r"%s = MODE == kLayer \? \(sizeof\(S\) == 4 \? (\d+) : (\d+)\)" % ring, text).groups() for ring in ("kRawSlots", "kRowSlots")]
+    assert rings[0] == rings[1]
+    return tuple(int(x) for x in rings[0])
+
+
 def stale_read(slots, order, seed, rows=40, single=0.0, teams=1):
     """One random run; whether a row was cooked before its copy had landed.  `single`: the share of rows cooked by a team of four warps,
     the teams in turn."""
@@ -72,7 +81,7 @@ def test_the_model_finds_the_order_that_fails():
     assert any(stale_read(5, ("raw_full", "row_empty"), seed) for seed in range(40))
 
 
-@pytest.mark.parametrize("slots", [5, 8])
+@pytest.mark.parametrize("slots", [5, 8, *depths()])
 @pytest.mark.parametrize("single", [0.0, 0.3])
 def test_no_row_is_read_before_it_has_landed(slots, single):
     orders = waits()
@@ -86,7 +95,7 @@ def test_the_model_finds_rings_too_short_for_two_teams():
     assert any(stale_read(6, order, seed, single=0.5, teams=2) for seed in range(150))
 
 
-@pytest.mark.parametrize("slots", [9, 10])  # more than the eight warps: the rows between two of a warp's own
+@pytest.mark.parametrize("slots", [9, depths()[1]])  # more than the eight warps: the rows between two of a warp's own
 @pytest.mark.parametrize("single", [0.1, 0.5, 0.9, 1.0])
 def test_two_teams_read_no_row_before_it_has_landed(slots, single):
     for order in set(waits()):
