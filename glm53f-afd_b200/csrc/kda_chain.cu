@@ -703,7 +703,11 @@ __device__ void layer_prologue_role(const Params& p, unsigned char* smem, uint64
                 }
                 return true;
             };
-            if (ONE_UNIT && un.rows > 1 ? !cook(std::false_type{}) : !cook(std::true_type{})) return;
+            if (!ONE_UNIT || un.rows == 1) {
+                if (!cook(std::true_type{})) return;
+            } else {
+                if (!cook(std::false_type{})) return;
+            }
             continue;
         }
         for (int r = 0; r < un.rows; ++r, raw.next(L::kRawSlots), row.next(L::kRowSlots)) {
