@@ -4,7 +4,7 @@
 // (request, layer, head) for the commit replay).  Four roles, connected by mbarrier rings in shared memory:
 //
 //   mover (1 warp)      bulk-copies (cp.async.bulk) each unit's 128x128 state and each row's raw inputs from global
-//                       memory into shared-memory rings, two or three units ahead of the arithmetic;
+//                       memory into shared-memory rings, two or three units ahead of the arithmetic (replay: three or five);
 //   prologue (2 to 8 warps)  turns a row's raw inputs into q, k, v, the decay multipliers, beta and sigmoid(gate)
 //                       (short conv + SiLU, L2 norms, gates for the layer entry points, on four or eight warps; exp(g) for the core
 //                       ones, on two; see kProWarpsOf);
@@ -13,7 +13,7 @@
 //                       stores its own 8 rows, a whole contiguous row per instruction;
 //   epilogue (1 warp)   gated RMSNorm, bf16 outputs, replay saves.
 //
-// The state therefore crosses HBM once in each direction -- in as bulk transfers that are always two or three
+// The state therefore crosses HBM once in each direction -- in as bulk transfers that are always that many
 // units deep in flight, out as coalesced vector stores from the registers.  What roles load from global memory themselves (a unit's metadata, the
 // layer prologue's conv weights and biases) is fetched ahead of the wait for the row or unit it belongs to.
 //
@@ -184,7 +184,7 @@ struct __align__(16) UnitInfo {
 template <typename S, int MODE>
 struct Smem {
     static constexpr int kStateBytes = DV * DK * (int)sizeof(S);
-    // States in flight: 96 KiB (bf16) or 128 KiB (f32).  More slow a long launch down, its reads then crowd out its writes (bf16 core, 5 and
+    // States in flight: 96 KiB (bf16) or 128 KiB (f32); the replay of saves off their 16 bytes has 160 and 192.  More slow a long launch down, its reads then crowd out its writes (bf16 core, 5 and
     // 3 slots of the ring: 48 requests 1,303 and 1,220 us a step of 34 layers, 16 requests 462 and 459; 2: 1,214 and 488).
     static constexpr int kStateSlots = MODE == kReplay ? (sizeof(S) == 4 ? 3 : 5) : sizeof(S) == 4 ? 2 : 3;
     static constexpr int kRawSlots = MODE == kLayer ? (sizeof(S) == 4 ? 6 : 10) : sizeof(S) == 4 ? 3 : 4;  // raw-row ring depth
@@ -985,8 +985,8 @@ __global__ void __launch_bounds__(kThreadsOf<S, MODE, ONE_UNIT>, 1) recurrent_ke
 // warp, which never interact with the others -- loads that part of the state straight from global memory into registers, cooks
 // each row's inputs itself (128 threads, one channel each: widen q, k, v, exp of the log decay, beta; loaded a row ahead, into the other
 // of two buffers, so a row takes one barrier), steps through the request's rows and stores its rows of the state back.  No rings, no
-// bulk copies: four such blocks on an SM are two units' serial rows at once.  Used for the exact verify; for single-row
-// decode the persistent kernel above streams faster.
+// bulk copies: four such blocks on an SM are two units' serial rows at once.  Used for the exact verify; single-row decode runs on the
+// persistent kernel above (core_entry).
 constexpr int kSmallWarps = 4, kSmallThreads = kSmallWarps * 32, kR = 4, kSmallParts = DV / (4 * kR * kSmallWarps), kSmallPerSm = 4;
 
 template <typename S>
@@ -1394,10 +1394,11 @@ int core_entry(int32_t heads, int32_t batch, const int32_t* cu_rows, const glm53
     x.out = out; x.out_stride = (long long)heads * DV;
     x.k_save = k_save; x.v_save = v_save; x.g_save = g_save; x.b_save = b_save;
     // The exact verify (saves requested, inputs used as given, no fused output norm) runs on the small-block kernel: two
-    // units' serial rows at once wait less on their own latencies than the persistent kernel's one (before the present step 11.1
-    // against 12.3 ms per step of 48 slots x 16 rows x 34 layers).  Single-row decode stays on the
-    // persistent kernel, which streams faster (4,263 against 3,500 GB/s at 16 slots: small blocks keep too few bytes in
-    // flight).  GLM53F_KDA_DECODE=pipeline / small forces one or the other; the bits are the same either way.
+    // units' serial rows at once wait less on their own latencies than the persistent kernel's one (48 slots x 16 rows x 34 layers, bf16,
+    // 9.6 against 11.9 ms; 6 slots x 8 rows 841 against 990 us, f32 757 and 901; a single slot's windows are the exception, four rows
+    // 335 against 254).  Single-row decode stays on the persistent kernel, which keeps more bytes in flight (bf16, 16 slots 458
+    // against 635 us, 48 slots 1,208 and 1,704; f32 845 and 786, 2,335 and 2,117, not so).  GLM53F_KDA_DECODE=pipeline / small forces one or
+    // the other; the bits are the same either way.
     static const int forced = [] {
         const char* e = getenv("GLM53F_KDA_DECODE");
         return e == nullptr ? 0 : (strcmp(e, "pipeline") == 0 ? 1 : (strcmp(e, "small") == 0 ? 2 : 0));

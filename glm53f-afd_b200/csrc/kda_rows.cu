@@ -16,7 +16,8 @@
 // states: 1,087 -> 402 us (0.5 us a row).  Measured against it at 701 rows: three rows in flight 406,
 // five blocks an SM (96 registers, spills) 515, four value rows a warp 451, rows through shared memory by asynchronous copies 457.
 //
-// Two prompts and more run rows_octet_kernel: there the work of an SM's warps counts, not a row's latency.
+// Launches of more units (rows_launch: from 112 on, two prompts of 64 heads) run rows_octet_kernel: there the work of an SM's warps counts, not a
+// row's latency.
 //
 // Same arithmetic in the same order with the same rounding points (a bf16 state is rounded after every row, the read-out
 // before the norm): the chain's bits.

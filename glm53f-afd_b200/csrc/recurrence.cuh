@@ -16,9 +16,8 @@ constexpr unsigned FULL = 0xffffffffu;
 
 // ---- packed FP32 pairs -----------------------------------------------------------------------------------------
 // sm_100 has two-wide FP32 instructions (mul.f32x2, add.f32x2): each half is an IEEE round-to-nearest operation,
-// so a pair gives the bits of two scalar instructions for half the issue slots.  The recurrence is bound by
-// instruction issue, not by the FP32 pipe, so the state is held as pairs: pair jp of a lane holds value rows
-// 2jp and 2jp+1 of its warp at one key column.
+// so a pair gives the bits of two scalar instructions for half the issue slots (the pipe's time stays).  The state is
+// held as pairs: pair jp of a lane holds value rows 2jp and 2jp+1 of its warp at one key column.
 using f32x2 = unsigned long long;
 __device__ __forceinline__ f32x2 pack2(float lo, float hi) {
     f32x2 r;

@@ -1,17 +1,19 @@
 // The exact recurrence step of recurrence.cuh with EIGHT lanes to a value row, for kernels in which many warps of several units share an
-// SM (the core entry points' exact verify, the commit replay, the exact prefill of several prompts).
+// SM (the core entry points' exact verify, the commit replay of many units, the exact prefill of several prompts).
 //
 // The reference forms a sum over the 128 key channels as a warp does: a lane adds its four consecutive channels (a leaf) in order
 // from zero, then the xor butterfly 16, 8, 4, 2, 1 adds the 32 leaves.  Here lane 8g + j holds leaves j, j + 8, j + 16 and j + 24 of R
 // rows, so that the butterfly's first two levels are additions within the thread and only three cross lanes.  Same additions,
 // same pairing, hence the same bits.  A warp owns 4R consecutive value rows, rows gR .. gR + R - 1 of them with lane group g.
 //
-// What bounds it: the FP32 pipe.  Seven separately rounded operations a state element and row are 896 cycles of an SM's 128 lanes;
-// two-wide instructions halve the issue slots, not the pipe's time.  With a row's 32 leaves in 32 lanes a unit and row cost 1,340 issue
-// slots a scheduler: 18 shuffles and 8 broadcasts for eight rows, and 24 moves that double k, decay and q.  Here 8 shuffles
+// What bounds it: no unit is full.  Seven separately rounded operations a state element and row are 896 cycles of an SM's 128 lanes, and
+// two-wide instructions halve the issue slots, not the pipe's time; with four warps a scheduler the FP32 pipe is 59 % active, issue 69 to
+// 74 %, and warps wait for the pipe, for their turn and for fixed latencies about equally.  With a row's 32 leaves in 32 lanes a unit
+// and row cost 1,340 issue slots a scheduler: 18 shuffles and 8 broadcasts for eight rows, and 24 moves that double k, decay and q.  Here 8 shuffles
 // and 4 broadcasts for sixteen rows (R = 4), and k, decay and q are used in the pairs in which they lie, for four times the
-// shared-memory reads.  Exact verify and replay of 48 slots x up to 16 rows x 34 layers: 11.16 -> 10.19 ms.  With few warps an SM the
-// reads' latency shows instead (one prompt of 701 rows: 405 against 417 us), so the others keep the layout of recurrence.cuh.
+// shared-memory reads.  Exact verify and replay of 48 slots x up to 16 rows x 34 layers: 11.16 -> 10.04 ms.  With few warps an SM the
+// reads' latency shows instead (one prompt of 701 rows: 405 against 417 us; the replay of few units, launch_replay_small), so the
+// others keep the layout of recurrence.cuh.
 #pragma once
 
 #include "recurrence.cuh"
