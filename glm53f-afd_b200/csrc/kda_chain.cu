@@ -438,10 +438,10 @@ __device__ void mover_role(const Params& p, unsigned char* smem, uint64_t* bars,
     };
     constexpr bool kRowFirst = MODE == kLayer;  // a core row is cooked in no time (16 slots 459 us a step; 473 with the row first)
     // A block's second f32 state waits for its first one: windows of two or three rows leave room in the ring of rows, so that it is asked for at
-    // once, and every SM's first state is then late (4 slots x 3 rows core 404 us a step of 34 layers, 421 without, 6 x 2 440 and 461; single
-    // rows, where the second state is wanted soon, 318 both ways).
+    // once, and every SM's first state is then late (4 slots x 3 rows core 402 us a step of 34 layers, 420 without, 6 x 2 441 and 461; single
+    // rows, where the second state is wanted soon, 319 both ways).
     constexpr bool kPaced = MODE == kCore && sizeof(S) == 4;
-    bool first = true, pace = false;
+    bool first = true;
     for (; units.valid(); first = false) {
         const Unit un = units.take(p);
         if (un.rows == 0 && !copy0) continue;
@@ -457,8 +457,6 @@ __device__ void mover_role(const Params& p, unsigned char* smem, uint64_t* bars,
                 raw.next(L::kRawSlots);
             }
         }
-        if (pace && !mbar_wait(&st_full[0], 0, ctx, kStatusWaitStateFull)) return;
-        pace = kPaced && first && un.rows > 1;
         // The unit's state.
         if (!mbar_wait(&st_empty[st.idx], st.phase ^ 1u, ctx, kStatusWaitStateEmpty)) return;
         if (lane == 0) info[st.idx] = {un.s_elem, un.rows};
@@ -484,6 +482,9 @@ __device__ void mover_role(const Params& p, unsigned char* smem, uint64_t* bars,
         // The other rows.
         for (int r = kRowFirst && first ? 1 : 0; r < un.rows; ++r)
             if (!row_in(un, r)) return;
+        if constexpr (kPaced) {
+            if (first && un.rows > 1 && !mbar_wait(&st_full[0], 0, ctx, kStatusWaitStateFull)) return;
+        }
     }
     if (!mbar_wait(&st_empty[st.idx], st.phase ^ 1u, ctx, kStatusWaitStateEmpty)) return;
     if (lane == 0) {
