@@ -1017,11 +1017,14 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallPerSm) core_small_kernel(
         next.g = p.glog[at];
         if (t == 0) next.beta = p.beta[gr * p.H + h];
     };
-    // Ahead of the state, and no rounding of a state that nobody reads: windows of one row of 6 bf16 slots 287 -> 246 us a step of 34
-    // layers, of four rows 530 -> 491 (a quarter of a unit a block on the step of recurrence.cuh: 272 and 553).
-    if (rows > 0) fetch(0);
+    // bf16: ahead of the state, and no rounding of a state that nobody reads: windows of one row of 6 slots 287 -> 246 us a step of 34
+    // layers, of four rows 530 -> 491 (a quarter of a unit a block on the step of recurrence.cuh: 272 and 553).  f32: behind it (2 slots x
+    // 16 rows 808 us, ahead 841).
+    constexpr bool kRowFirst = sizeof(S) == 2;
+    if (kRowFirst && rows > 0) fetch(0);
     f32x2 s[kR][oct::kRowPairs];
     oct::load_rows(reinterpret_cast<const S*>(p.state_in) + s_elem, uw, lane, s);
+    if (!kRowFirst && rows > 0) fetch(0);
     for (int r = 0; r < rows; ++r) {
         const long long gr = (long long)r0 + r, at = (gr * p.H + h) * DK + t;
         const int buf = r & 1;  // the row before may still be read from the other buffer
