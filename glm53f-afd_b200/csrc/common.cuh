@@ -129,6 +129,9 @@ __device__ __forceinline__ void bulk_store(void* gmem_dst, const void* smem_src,
                  "r"(bytes)
                  : "memory");
 }
+__device__ __forceinline__ void bulk_prefetch(const void* gmem_src, uint32_t bytes) {  // into L2
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(gmem_src), "r"(bytes) : "memory");
+}
 // A tensor map's box on its way into L2.
 __device__ __forceinline__ void tensor_prefetch_3d(const void* tmap, int x, int y, int z) {
     asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];" ::"l"(reinterpret_cast<uint64_t>(tmap)), "r"(x), "r"(y), "r"(z)
@@ -210,6 +213,12 @@ __device__ __forceinline__ float rcp_approx(float x) {
 __device__ __forceinline__ float ex2_approx(float x) {
     float r;
     asm("ex2.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+// The same where a result below 2^-126 may as well be 0: one instruction instead of four.
+__device__ __forceinline__ float ex2_ftz(float x) {
+    float r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
 constexpr float kLog2e = 1.4426950408889634f;

@@ -64,6 +64,7 @@ __device__ __forceinline__ float2 widen2(uint32_t w) {
 struct SpParams {
     alignas(64) CUtensorMap tm_q, tm_k, tm_v, tm_g;  // [rows][H][128] as (128, H, rows); boxes of 64 rows x 128 bytes, 128-byte swizzle
     alignas(64) CUtensorMap tm_out;                  // the shard-local output, the same way
+    alignas(64) CUtensorMap tm_gate;                 // the gate rows, the same way (gate_boxes != 0)
     alignas(64) CUtensorMap tm_full[8];              // every rank's full output buffer: (128, heads_total, rows)
     int H, batch;
     const int32_t* cu;
@@ -76,6 +77,7 @@ struct SpParams {
     int state_bf16;
     const uint16_t* gate;
     long long gate_stride;  // elements between consecutive gate rows
+    int gate_boxes;         // full chunks' gate values come by tiled tensor copies (base and stride on 16 bytes)
     const uint16_t* norm_w;
     float eps;
     uint16_t* out;
@@ -128,7 +130,7 @@ __device__ __forceinline__ Item item_of(const SpParams& p, int item) {
 // The state role's barriers sit behind every tile (set up once at kernel entry, never repurposed).  The intra role's
 // live inside its two groups' areas, which the state role -- it runs first in a block -- uses as tile space, so they are
 // set up when the intra role starts.
-constexpr int oBarsState = kSmemTc, kSmemSp = kSmemTc + 192;
+constexpr int oBarsState = kSmemTc, oChain = oBarsState + 240, kSmemSp = oChain + 64;
 // 16 compute warps, the loader warp, and (state role only) a warp that moves finished output rows to global memory and one that
 // issues the tensor-core products.
 constexpr int kThreadsSp = kCompute + 96, kLoaderWarp = kCompute / 32, kOutWarp = kCompute / 32 + 1, kMmaWarp = kCompute / 32 + 2;
@@ -252,7 +254,7 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
             float amax = 0.0f;
 #pragma unroll
             for (int r = 0; r < 32; ++r) {
-                const float av = ex2_approx(run[r] - run[(r & 16) | 8]);
+                const float av = ex2_ftz(fmaxf(run[r] - run[(r & 16) | 8], -126.0f));  // never 0: its reciprocal is taken
                 amax = fmaxf(amax, av);
                 *reinterpret_cast<float*>(col + r * 128 + ((pc ^ (r & 7)) << 4)) = av;
             }
@@ -264,14 +266,14 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
             const float gl = base1 + tmp[128 + d];
             float* tab = reinterpret_cast<float*>(gs + gTab) + d;
             if (part == 0) {
-                tab[(tE0 + 0) * 128] = ex2_approx(gm0); tab[(tE0 + 1) * 128] = ex2_approx(gm1); tab[(tE0 + 2) * 128] = ex2_approx(gm2); tab[(tE0 + 3) * 128] = ex2_approx(gm3);
-                tab[(tEL + 0) * 128] = ex2_approx(gl - gm0); tab[(tEL + 1) * 128] = ex2_approx(gl - gm1);
-                tab[(tEL + 2) * 128] = ex2_approx(gl - gm2); tab[(tEL + 3) * 128] = ex2_approx(gl - gm3);
+                tab[(tE0 + 0) * 128] = ex2_ftz(gm0); tab[(tE0 + 1) * 128] = ex2_ftz(gm1); tab[(tE0 + 2) * 128] = ex2_ftz(gm2); tab[(tE0 + 3) * 128] = ex2_ftz(gm3);
+                tab[(tEL + 0) * 128] = ex2_ftz(gl - gm0); tab[(tEL + 1) * 128] = ex2_ftz(gl - gm1);
+                tab[(tEL + 2) * 128] = ex2_ftz(gl - gm2); tab[(tEL + 3) * 128] = ex2_ftz(gl - gm3);
             } else {
-                tab[(tF + 0) * 128] = ex2_approx(gm1 - gm0);
-                tab[(tF + 1) * 128] = ex2_approx(gm2 - gm0); tab[(tF + 2) * 128] = ex2_approx(gm2 - gm1);
-                tab[(tF + 3) * 128] = ex2_approx(gm3 - gm0); tab[(tF + 4) * 128] = ex2_approx(gm3 - gm1); tab[(tF + 5) * 128] = ex2_approx(gm3 - gm2);
-                const float egl = ex2_approx(gl);
+                tab[(tF + 0) * 128] = ex2_ftz(gm1 - gm0);
+                tab[(tF + 1) * 128] = ex2_ftz(gm2 - gm0); tab[(tF + 2) * 128] = ex2_ftz(gm2 - gm1);
+                tab[(tF + 3) * 128] = ex2_ftz(gm3 - gm0); tab[(tF + 4) * 128] = ex2_ftz(gm3 - gm1); tab[(tF + 5) * 128] = ex2_ftz(gm3 - gm2);
+                const float egl = ex2_ftz(gl);
                 reinterpret_cast<float*>(slot + wEgl)[d] = egl;
                 reinterpret_cast<float*>(gs + gGl)[d] = egl;
             }
@@ -346,7 +348,7 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
                 float v_kg[2], v_kgb[2], hi[2], lo[2];
 #pragma unroll
                 for (int u = 0; u < 2; ++u) {
-                    const float av = a[cc * 8 + 2 * u2 + u], inva = __fdividef(1.0f, av);
+                    const float av = a[cc * 8 + 2 * u2 + u], inva = rcp_approx(av);
                     v_kgb[u] = kf[u] * av;
                     v_kg[u] = kf[u] * (av * E0[2 * u2 + u]);
                     kc[2 * u2 + u] = kf[u] * inva;
@@ -691,7 +693,8 @@ __device__ void intra_role(const SpParams& p, unsigned char* smem, const uint32_
 // are A operands that never leave tensor memory; what comes from the workspace is the B side, so shared memory has room for
 // two chunks of it and a load has a whole chunk's time to arrive.
 // Measured per chunk at 64 chains: 5,800 cycles with products of 64 rows, S and D through shared memory and block barriers
-// around every step; 3,700 to 4,000 so.
+// around every step; 3,700 to 4,000 so; 3,500 with U asked into L2 a chunk ahead.  With the gated norm 5,400: 16,384 exponentials and
+// reciprocals a chunk are 1,000 cycles of the units that do them (before U and D instead of behind D they are as long, and cost registers).
 // =====================================================================================================================
 // Shared memory: two buffers of [Qg | W], two of [M | Kdec hi | Kdec lo] and exp(G_last), one of U, each with a full / empty pair.
 // Finished output rows (bf16) wait in one of two tiles for the output warp: two boxes of 64 rows x 128 bytes each (value
@@ -705,13 +708,13 @@ constexpr uint32_t tS = 0, tS16 = 128, tWS = 192, tO = 256, tDhi = 384, tDlo = 4
 // The state role's barriers and their arrival counts.  Those of a buffer that alternates between chunks come in pairs, so that
 // no barrier can complete a phase while somebody still has to see the one before.
 enum : int { bFullQW = 0, bFullMKd = 2, bFullU = 4, bEmptyQW = 5, bEmptyMKd = 7, bEmptyU = 9, bWS = 10, bSNew = 11, bS16 = 12, bSDec = 13, bD = 14, bO = 15, bOFree = 17,
-             bOutFull = 19, bOutEmpty = 21, kStateBars = 23 };
+             bOutFull = 19, bOutEmpty = 21, bChainFull = 23, bChainEmpty = 25, bGate = 27, kStateBars = 29 };
 __device__ __forceinline__ int state_bar_count(int i) {
     // one arrival per compute warp, or one in all
     const bool warps = i == bEmptyU || i == bS16 || i == bSDec || i == bD || i == bOFree || i == bOFree + 1 || i == bOutFull || i == bOutFull + 1;
-    return warps ? kCompute / 32 : 1;
+    return warps ? kCompute / 32 : i == bChainEmpty || i == bChainEmpty + 1 ? kCompute / 32 + 2 : 1;  // a chain is read by the MMA and the output warp too
 }
-static_assert(kStateBars * 8 <= 192, "state role barriers");
+static_assert(kStateBars * 8 <= oChain - oBarsState && oChain % 16 == 0, "state role barriers");
 
 // Waits until a count in global memory has reached `want`; gives up when it has stood still for the waits' limit.
 __device__ __forceinline__ bool count_wait(const unsigned int* at, unsigned want, const WaitCtx& ctx, int code) {
@@ -744,33 +747,159 @@ struct Walk {
     bool use_u, emit;
 };
 
+// What the roles of a block need to know of a chain they walk: `count` chunks from row `row` of the whole batch on, of head h; `rows`
+// rows are left of the sequence there.  The loader warp writes it; the others read it from shared memory whenever they want some of it.
+struct Chain {
+    int count, rows, h, start;  // count < 0: no more chains; start: the sequence begins here
+    long long row, s_elem;
+};
+__device__ __forceinline__ Chain chain_of(const SpParams& p, const Walk& wk, int chain) {
+    const int b = chain / p.H, h = chain % p.H, T = p.cu[b + 1] - p.cu[b];
+    const int nch = (T + CH - 1) / CH, j0 = min(wk.ja, nch);
+    return {max(min(nch, wk.jb) - j0, 0), T - j0 * CH, h, j0 == 0, p.cu[b] + (long long)j0 * CH, p.state_off[b] + (long long)h * DV * DK};
+}
+// A chain with no chunk in this range: only the first segment has anything to do (an empty sequence copies its state); a scan
+// walk always delivers its end state.
+__device__ __forceinline__ bool nothing_to_do(const SpParams& p, const Chain& c) {
+    return p.scan_pass == 0 && c.count == 0 && !(c.start && p.state_out != p.state_in);
+}
+
+// A warp's 32 x 32 piece of the state between tensor memory and a state buffer on 16 bytes (rows of 128 elements).  A thread that moves
+// its own row's 32 values touches a line of its own with every 16 bytes (2,000 cycles a state of bf16, 4,000 of FP32); from the fragment
+// layout, in which four lanes hold a row's neighbouring columns, two or four lanes trade halves and a row's 64 bytes go at once.
+__device__ __forceinline__ uint32_t trade(bool up, uint32_t lo, uint32_t hi, int lanes) { return __shfl_xor_sync(0xffffffffu, up ? lo : hi, lanes); }
+__device__ __forceinline__ void state_from_tmem(uint32_t at, float* to, int lane) {  // to: row 0, column 0 of the piece
+    const int q = lane & 3;
+    const bool odd = q & 1;
+    to += (lane >> 2) * DK + (odd ? 6 + 2 * q : 2 * q);
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {  // sixteen rows (x / 2) and sixteen columns (x % 2)
+        uint32_t f[8];
+        tc::tmem_ld_frag(at + ((uint32_t)(x >> 1) << 20) + (x & 1) * 16, f);
+        tc::tmem_ld_wait();
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {  // eight rows
+            const uint32_t r0 = trade(odd, f[2 * h], f[4 + 2 * h], 1), r1 = trade(odd, f[2 * h + 1], f[5 + 2 * h], 1);
+            *reinterpret_cast<uint4*>(to + ((x >> 1) * 16 + h * 8) * DK + (x & 1) * 16) = odd ? make_uint4(r0, r1, f[4 + 2 * h], f[5 + 2 * h]) : make_uint4(f[2 * h], f[2 * h + 1], r0, r1);
+        }
+    }
+}
+__device__ __forceinline__ void state_to_tmem(uint32_t at, const float* from, int lane) {
+    const int q = lane & 3;
+    const bool odd = q & 1;
+    from += (lane >> 2) * DK + (odd ? 6 + 2 * q : 2 * q);
+    uint4 w[8];
+#pragma unroll
+    for (int x = 0; x < 8; ++x) w[x] = *reinterpret_cast<const uint4*>(from + ((x >> 2) * 16 + (x & 1) * 8) * DK + ((x >> 1) & 1) * 16);
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+        uint32_t f[8];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const uint4 v = w[2 * x + h];
+            const uint32_t r0 = trade(odd, v.x, v.z, 1), r1 = trade(odd, v.y, v.w, 1);
+            f[2 * h] = odd ? r0 : v.x; f[2 * h + 1] = odd ? r1 : v.y;
+            f[4 + 2 * h] = odd ? v.z : r0; f[5 + 2 * h] = odd ? v.w : r1;
+        }
+        tc::tmem_st_frag(at + ((uint32_t)(x >> 1) << 20) + (x & 1) * 16, f);
+    }
+}
+__device__ __forceinline__ void state_from_tmem(uint32_t at, uint16_t* to, int lane) {
+    const int q = lane & 3;
+    const bool odd = q & 1, up = q & 2;
+    to += (lane >> 2) * DK + q * 8;
+#pragma unroll
+    for (int x = 0; x < 2; ++x) {  // sixteen rows
+        uint32_t f[2][8];
+        tc::tmem_ld_frag(at + ((uint32_t)x << 20), f[0]);
+        tc::tmem_ld_frag(at + ((uint32_t)x << 20) + 16, f[1]);
+        tc::tmem_ld_wait();
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            uint32_t w[4], pr[2][2];  // w[g]: columns 8 g + 2 q and the next; pr: of g = 2 i + odd, those of lanes (q & 2) and (q & 2) + 1
+#pragma unroll
+            for (int g = 0; g < 4; ++g) w[g] = tc::bf16x2(__uint_as_float(f[g >> 1][4 * (g & 1) + 2 * h]), __uint_as_float(f[g >> 1][4 * (g & 1) + 2 * h + 1]));
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const uint32_t r = trade(odd, w[2 * i], w[2 * i + 1], 1);
+                pr[i][0] = odd ? r : w[2 * i];
+                pr[i][1] = odd ? w[2 * i + 1] : r;
+            }
+            const uint32_t r0 = trade(up, pr[0][0], pr[1][0], 2), r1 = trade(up, pr[0][1], pr[1][1], 2);
+            *reinterpret_cast<uint4*>(to + (x * 16 + h * 8) * DK) = up ? make_uint4(r0, r1, pr[1][0], pr[1][1]) : make_uint4(pr[0][0], pr[0][1], r0, r1);
+        }
+    }
+}
+__device__ __forceinline__ void state_to_tmem(uint32_t at, const uint16_t* from, int lane) {
+    const int q = lane & 3;
+    const bool odd = q & 1, up = q & 2;
+    from += (lane >> 2) * DK + q * 8;
+    uint4 v[4];
+#pragma unroll
+    for (int x = 0; x < 4; ++x) v[x] = *reinterpret_cast<const uint4*>(from + x * 8 * DK);
+#pragma unroll
+    for (int x = 0; x < 2; ++x) {
+        uint32_t f[2][8];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const uint4 y = v[2 * x + h];
+            const uint32_t r0 = trade(up, y.x, y.z, 2), r1 = trade(up, y.y, y.w, 2);
+            const uint32_t pr[2][2] = {{up ? r0 : y.x, up ? r1 : y.y}, {up ? y.z : r0, up ? y.w : r1}};
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const uint32_t r = trade(odd, pr[i][0], pr[i][1], 1), w0 = odd ? r : pr[i][0], w1 = odd ? pr[i][1] : r;
+                f[i][2 * h] = w0 << 16; f[i][2 * h + 1] = w0 & 0xffff0000u;
+                f[i][4 + 2 * h] = w1 << 16; f[i][5 + 2 * h] = w1 & 0xffff0000u;
+            }
+        }
+        tc::tmem_st_frag(at + ((uint32_t)x << 20), f[0]);
+        tc::tmem_st_frag(at + ((uint32_t)x << 20) + 16, f[1]);
+    }
+}
+
+// Walks `chain`, or (MANY) the chains of a fused launch that this block's loader warp takes off the counter, until there are none.
+// Nothing is set up or drained between two of these: the buffers, accumulators and barriers go on alternating with the chunks, whichever
+// chain they belong to, the next chain's first chunks are loaded behind the last ones of the chain before, and the outputs of a chain's
+// last chunk leave behind the next chain's first D.  A walk that began and ended by itself took 23 us for five chunks, 13 of them beside the
+// chunks: counter, metadata, barriers and first loads one after another, the state a line per 16 bytes, the last chunk's gate.  Whole
+// calls, us: chunked layer prefill of 4 x 2,048 rows 1,136 -> 1,043, of 3 x 700 342 -> 301; core prefill of 8,192 rows in 8 sequences 525 -> 504, with
+// the norm in 3 sequences 663 -> 582; 8 chains of 1,024 chunks (one walk each) 1,968 -> 1,845.
+template <bool MANY>
 __device__ void state_role(const SpParams& p, unsigned char* smem, const uint32_t tm, const int chain, const Walk wk) {
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + oBarsState);
     volatile uint32_t* ctl = reinterpret_cast<volatile uint32_t*>(smem + oCtl);
+    volatile Chain* recs = reinterpret_cast<volatile Chain*>(smem + oChain);  // the chain that is walked, and the one before or after it
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int quad = warp & 3, cg = warp >> 2;
-    const int H = p.H, b = chain / H, h = chain % H;
-    const long long row0 = p.cu[b];
-    const int T = p.cu[b + 1] - p.cu[b];
-    const int nch = (T + CH - 1) / CH;
-    const int j0 = min(wk.ja, nch), j1 = min(nch, wk.jb), count = j1 - j0;
-    const long long s_elem = p.state_off[b] + (long long)h * DV * DK;
-    // A chain with no chunk in this range: only the first segment has anything to do (an empty sequence copies its state);
-    // a scan walk always delivers its end state.
-    if (p.scan_pass == 0 && j0 >= j1 && !(j0 == 0 && p.state_out != p.state_in)) return;
+    if (!MANY && nothing_to_do(p, chain_of(p, wk, chain))) return;
     const WaitCtx ctx{ctl, ctl + 1, p.status};
     auto wait = [&](int i, int phase) { return mbar_wait(&bars[i], (uint32_t)(phase & 1), ctx, kStatusWaitPrefill); };
+    // This block's chain number n lies in record n & 1 until everyone has released it; its number of chunks, -1 where there are no more
+    // chains, -2 where a wait gave up.
+    auto chain_count = [&](int n) -> int { return wait(bChainFull + (n & 1), n >> 1) ? recs[n & 1].count : -2; };
+    auto release = [&](int n) {
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars[bChainEmpty + (n & 1)]);
+    };
+    // In every role C counts the chunks of all the block's chains: it selects the buffers and gives the phases.
 
     if (warp == kOutWarp) {
         // The output warp: each finished tile of rows goes to the shard-local `out` and, for a head-sharded launch, into
         // every rank's full buffer -- the all-gather, done here: a peer's buffer is reached over NVLink.  A full chunk
         // leaves by tiled tensor stores (two per destination), off the compute warps' path; a sequence's last, partial
         // chunk by the warp's own stores, so that no row beyond the sequence is touched.
-        for (int c = 0; wk.emit && c < count; ++c) {
-            const int n = min(CH, T - (j0 + c) * CH);
-            const long long gr0 = row0 + (long long)(j0 + c) * CH;
-            if (!wait(bOutFull + (c & 1), c >> 1)) break;
-            const unsigned char* tile = smem + sOut + (c & 1) * kOutTile;
+        bool alive = wk.emit;
+        for (int seq = 0, C = 0; alive; ++seq) {
+        const int count = chain_count(seq);
+        if (count < 0) break;
+        const int rows = recs[seq & 1].rows, h = recs[seq & 1].h;
+        const long long row = recs[seq & 1].row;
+        release(seq);
+        for (int c = 0; c < count; ++c, ++C) {
+            const int n = min(CH, rows - c * CH);
+            const long long gr0 = row + (long long)c * CH;
+            if (!wait(bOutFull + (C & 1), C >> 1)) { alive = false; break; }
+            const unsigned char* tile = smem + sOut + (C & 1) * kOutTile;
             if (n == CH) {
                 if (lane == 0) {
                     for (int x = 0; x < 2; ++x) {
@@ -784,13 +913,14 @@ __device__ void state_role(const SpParams& p, unsigned char* smem, const uint32_
                 for (int e = lane; e < n * 16; e += 32) {
                     const int r = e >> 4, piece = e & 15;
                     const uint4 v4 = *reinterpret_cast<const uint4*>(tile + box_piece(r, piece));
-                    if (p.out != nullptr) *reinterpret_cast<uint4*>(p.out + ((gr0 + r) * H + h) * DV + piece * 8) = v4;
+                    if (p.out != nullptr) *reinterpret_cast<uint4*>(p.out + ((gr0 + r) * p.H + h) * DV + piece * 8) = v4;
                     const long long at_full = ((gr0 + r) * p.heads_total + p.head0 + h) * DV + piece * 8;
                     for (int pe = 0; pe < p.ranks; ++pe) *reinterpret_cast<uint4*>(p.full[pe] + at_full) = v4;
                 }
             }
             __syncwarp();
-            if (lane == 0) mbar_arrive(&bars[bOutEmpty + (c & 1)]);
+            if (lane == 0) mbar_arrive(&bars[bOutEmpty + (C & 1)]);
+        }
         }
         if (lane == 0) bulk_wait_all<0>();
         tc::fence_before_sync();
@@ -799,20 +929,87 @@ __device__ void state_role(const SpParams& p, unsigned char* smem, const uint32_
     }
     if (warp == kLoaderWarp) {
         if (lane == 0) {
-            for (int c = 0; c < count; ++c) {
-                const unsigned char* slot = slot_of(p.ws_state, p.seg_chunks, chain, j0 + c - p.state_chunk0);
-                const int x = c & 1;
-                if (!wait(bEmptyQW + x, (c >> 1) ^ 1)) break;  // an empty barrier starts released
-                mbar_arrive_expect_tx(&bars[bFullQW + x], kQW);
-                bulk_load(smem + sQW + x * kQW, slot + wQg, kQW, &bars[bFullQW + x]);
-                if (!wait(bEmptyMKd + x, (c >> 1) ^ 1)) break;
-                mbar_arrive_expect_tx(&bars[bFullMKd + x], kMKd + 512);
-                bulk_load(smem + sE + x * 512, slot + wEgl, 512, &bars[bFullMKd + x]);
-                bulk_load(smem + sMKd + x * kMKd, slot + wMm, kMKd, &bars[bFullMKd + x]);
-                if (!wait(bEmptyU, c ^ 1)) break;
-                mbar_arrive_expect_tx(&bars[bFullU], kUBytes);
-                bulk_load(smem + sU, slot + wU, kUBytes, &bars[bFullU]);
+            unsigned int* set = p.sets + p.ctr * kTailSet;
+            const int chains = p.batch * p.H;
+            auto take = [&]() { return MANY ? (int)min(atomicAdd(set + 1, 1u), (unsigned)chains) : chain; };
+            // Record number n; -1 chunks end the list.
+            auto publish = [&](int n, const Chain& c) -> bool {
+                if (!wait(bChainEmpty + (n & 1), (n >> 1) ^ 1)) return false;
+                volatile Chain& to = recs[n & 1];
+                to.count = c.count; to.rows = c.rows; to.h = c.h; to.start = c.start; to.row = c.row; to.s_elem = c.s_elem;
+                mbar_arrive(&bars[bChainFull + (n & 1)]);
+                return true;
+            };
+            // A chunk's gate values, for a chunk that the norm is fused into: into the tile that its outputs will take, when the chunk two before
+            // has left it, and asked for behind the rows of the chunk after, so that nothing waits for that.
+            bool gate_due = false;
+            int gate_row = 0, gate_h = 0;
+            auto load_gate = [&](int C) -> bool {  // of chunk C
+                if (!wait(bOutEmpty + (C & 1), (C >> 1) ^ 1)) return false;
+                if (gate_row < 0) {  // a partial chunk's are read by the threads that want them
+                    mbar_arrive(&bars[bGate + (C & 1)]);
+                    return true;
+                }
+                mbar_arrive_expect_tx(&bars[bGate + (C & 1)], kOutTile);
+                for (int x = 0; x < 2; ++x) tensor_load_3d(smem + sOut + (C & 1) * kOutTile + x * kBox, &p.tm_gate, x * 64, gate_h, gate_row, &bars[bGate + (C & 1)]);
+                return true;
+            };
+            int next = take(), C = 0;
+            for (int seq = 0;;) {
+                const int ch = next;
+                if ((MANY && ch >= chains) || (!MANY && seq > 0)) {
+                    publish(seq, Chain{-1, 0, 0, 0, 0, 0});
+                    break;
+                }
+                const Chain at = chain_of(p, wk, ch);
+                if constexpr (MANY) {
+                    if (nothing_to_do(p, at)) {
+                        next = take();
+                        continue;
+                    }
+                    // Its state on the way into L2, and the chain's items, finished by whichever blocks took them: they lie in its group.
+                    const int elem = p.state_bf16 ? 2 : 4;
+                    const char* state = reinterpret_cast<const char*>(at.start ? p.state_in : p.state_out) + at.s_elem * elem;
+                    if ((reinterpret_cast<uintptr_t>(state) & 15) == 0) bulk_prefetch(state, DV * DK * elem);
+                    const int g = ch / p.group, want = min(p.group, chains - g * p.group) * p.seg_chunks;
+                    if (!count_wait(set + 2 + g, (unsigned)want, ctx, kStatusWaitPrefill)) {
+                        ctl[1] = 1u;
+                        break;
+                    }
+                    fence_proxy_async_global();
+                }
+                if (!publish(seq, at)) break;
+                ++seq;
+                if (at.count == 0 && gate_due) {  // no rows behind which the gate of the chunk before would be asked for
+                    if (!load_gate(C - 1)) break;
+                    gate_due = false;
+                }
+                const int j0 = (wk.ja - p.state_chunk0);
+                bool ok = true;
+                for (int c = 0; ok && c < at.count; ++c, ++C) {
+                    const unsigned char* slot = slot_of(p.ws_state, p.seg_chunks, ch, j0 + c);
+                    const int x = C & 1;
+                    if (!(ok = wait(bEmptyQW + x, (C >> 1) ^ 1))) break;  // an empty barrier starts released
+                    mbar_arrive_expect_tx(&bars[bFullQW + x], kQW);
+                    bulk_load(smem + sQW + x * kQW, slot + wQg, kQW, &bars[bFullQW + x]);
+                    if (!(ok = wait(bEmptyMKd + x, (C >> 1) ^ 1))) break;
+                    mbar_arrive_expect_tx(&bars[bFullMKd + x], kMKd + 512);
+                    bulk_load(smem + sE + x * 512, slot + wEgl, 512, &bars[bFullMKd + x]);
+                    bulk_load(smem + sMKd + x * kMKd, slot + wMm, kMKd, &bars[bFullMKd + x]);
+                    if (!(ok = wait(bEmptyU, C ^ 1))) break;
+                    mbar_arrive_expect_tx(&bars[bFullU], kUBytes);
+                    bulk_load(smem + sU, slot + wU, kUBytes, &bars[bFullU]);
+                    // U has one buffer, so its load is on the walk: from L2.
+                    if (c + 1 < at.count) bulk_prefetch(slot + kSlotBytes + wU, kUBytes);
+                    if (gate_due && !(ok = load_gate(C - 1))) break;
+                    gate_due = wk.emit && p.gate_boxes != 0;
+                    gate_row = at.rows - c * CH >= CH ? (int)(at.row + c * CH) : -1;
+                    gate_h = at.h;
+                }
+                if (!ok) break;
+                next = take();  // a chunk and a half before it is wanted; any earlier, and blocks that come late find too few left
             }
+            if (gate_due) load_gate(C - 1);
         }
         tc::fence_before_sync();
         __syncthreads();
@@ -822,25 +1019,32 @@ __device__ void state_role(const SpParams& p, unsigned char* smem, const uint32_
         const uint32_t leader = tc::elect_one();
         auto ready = [&](int i, int phase) { return tc::warp_all(wait(i, phase)); };
         constexpr uint32_t idw = tc::idesc_bf16(DV, CH, 0, 1, 0), idq = tc::idesc_bf16(DV, CH, 0, 0, 0), ids = tc::idesc_bf16(DV, DK, 0, 1, 0);
-        for (int c = 0; c < count; ++c) {
-            const int x = c & 1;
+        bool alive = true;
+        int C = 0;
+        for (int seq = 0; alive; ++seq) {
+        const int count = chain_count(seq);
+        if (!tc::warp_all(count >= 0)) break;
+        release(seq);
+        for (int c = 0; tc::warp_all(c < count); ++c, ++C) {
+            alive = false;
+            const int x = C & 1;
             const uint32_t acc = tm + tO + (uint32_t)x * 64;
             const unsigned char *qw = smem + sQW + x * kQW, *mm = smem + sMKd + x * kMKd, *kdhi = mm + kTile / 2, *kdlo = kdhi + kTile;
-            if (!ready(bFullQW + x, c >> 1) || !ready(bS16, c)) break;
+            if (!ready(bFullQW + x, C >> 1) || !ready(bS16, C)) break;
             tc::fence_after_sync();
 #pragma unroll
             for (int k0 = 0; k0 < DK; k0 += 16)
                 tc::mma_bf16_ts_if(leader, tm + tWS, tm + tS16 + k0 / 2, tc::desc_mnmajor_bf16(qw + kTile, DK, 0, k0), idw, k0 > 0);
             tc::mma_commit_if(leader, &bars[bWS]);
             if (wk.emit) {
-                if (c >= 2 && !ready(bOFree + x, (c >> 1) - 1)) break;  // chunk c - 2's outputs have left this accumulator
+                if (C >= 2 && !ready(bOFree + x, (C >> 1) - 1)) break;  // chunk C - 2's outputs have left this accumulator
                 tc::fence_after_sync();
 #pragma unroll
                 for (int k0 = 0; k0 < DK; k0 += 16)
                     tc::mma_bf16_ts_if(leader, acc, tm + tS16 + k0 / 2, tc::desc_kmajor_bf16(qw, CH, 0, k0), idq, k0 > 0);
             }
             tc::mma_commit_if(leader, &bars[bEmptyQW + x]);
-            if (!ready(bFullMKd + x, c >> 1) || !ready(bSDec, c) || !ready(bD, c)) break;
+            if (!ready(bFullMKd + x, C >> 1) || !ready(bSDec, C) || !ready(bD, C)) break;
             tc::fence_after_sync();
 #pragma unroll
             for (int k0 = 0; k0 < CH; k0 += 16) tc::mma_bf16_ts_if(leader, tm + tS, tm + tDhi + k0 / 2, tc::desc_mnmajor_bf16(kdhi, CH, 0, k0), ids, true);
@@ -857,9 +1061,11 @@ __device__ void state_role(const SpParams& p, unsigned char* smem, const uint32_
             tc::mma_commit_if(leader, &bars[bEmptyMKd + x]);
             if (leader) atomicAdd(const_cast<uint32_t*>(ctl), 1u);
             __syncwarp();
+            alive = true;
         }
-        // Nobody else waits for the last two chunks' buffers; a block that goes on to another chain sets its barriers up again.
-        for (int c = max(count - 2, 0); c < count; ++c)
+        }
+        // Nobody else waits for the last two chunks' buffers.
+        for (int c = max(C - 2, 0); c < C; ++c)
             if (!ready(bEmptyQW + (c & 1), c >> 1) || !ready(bEmptyMKd + (c & 1), c >> 1)) break;
         tc::fence_before_sync();
         __syncthreads();
@@ -909,55 +1115,44 @@ __device__ void state_role(const SpParams& p, unsigned char* smem, const uint32_
     };
 
     // ---- the incoming state into tensor memory; a thread's 32 key channels are consecutive in every state buffer ------------
-    const long long s_at = s_elem + (long long)v * DK + k_first;
     const int b_at = v * DK + k_first;
-    {
-        const void* src = j0 == 0 ? p.state_in : p.state_out;
+    auto piece_aligned = [](const void* at) { return (reinterpret_cast<uintptr_t>(at) & 15) == 0; };  // for all lanes or none
+    auto state_in = [&](bool start, long long s_elem) {
+        const void* src = start ? p.state_in : p.state_out;
+        const long long s_at = s_elem + b_at;
         uint32_t r[32];
         if (wk.init == 1 || wk.init == 2) {
 #pragma unroll
             for (int x = 0; x < 32; ++x) r[x] = wk.init == 2 && k_first + x == v ? __float_as_uint(1.0f) : 0u;
         } else if (wk.init == 0 && p.state_bf16) {
             const uint16_t* at = reinterpret_cast<const uint16_t*>(src) + s_at;
-            if ((reinterpret_cast<uintptr_t>(at) & 15) == 0) {
-#pragma unroll
-                for (int x = 0; x < 4; ++x) {
-                    const uint4 w = reinterpret_cast<const uint4*>(at)[x];
-                    const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-                    for (int y = 0; y < 4; ++y) {
-                        r[8 * x + 2 * y] = ww[y] << 16;
-                        r[8 * x + 2 * y + 1] = ww[y] & 0xffff0000u;
-                    }
-                }
-            } else {
-#pragma unroll
-                for (int x = 0; x < 32; ++x) r[x] = (uint32_t)at[x] << 16;
+            if (piece_aligned(at)) {
+                state_to_tmem(tc::tmem_addr(tm, quad, tS + k_first), at - lane * DK, lane);
+                tc::tmem_st_wait();
+                return;
             }
+#pragma unroll
+            for (int x = 0; x < 32; ++x) r[x] = (uint32_t)at[x] << 16;
         } else {
             const float* at = wk.init == 3 ? wk.from + b_at : reinterpret_cast<const float*>(src) + s_at;
-            if ((reinterpret_cast<uintptr_t>(at) & 15) == 0) {
-#pragma unroll
-                for (int x = 0; x < 8; ++x) {
-                    const uint4 w = reinterpret_cast<const uint4*>(at)[x];
-                    r[4 * x] = w.x; r[4 * x + 1] = w.y; r[4 * x + 2] = w.z; r[4 * x + 3] = w.w;
-                }
-            } else {
-#pragma unroll
-                for (int x = 0; x < 32; ++x) r[x] = __float_as_uint(at[x]);
+            if (piece_aligned(at)) {
+                state_to_tmem(tc::tmem_addr(tm, quad, tS + k_first), at - lane * DK, lane);
+                tc::tmem_st_wait();
+                return;
             }
+#pragma unroll
+            for (int x = 0; x < 32; ++x) r[x] = __float_as_uint(at[x]);
         }
         tc::tmem_st32(tc::tmem_addr(tm, quad, tS + k_first), r);
         tc::tmem_st_wait();
-    }
-    // The four warps that share output rows vote at a barrier in every chunk when the norm is fused; one that gives up before
-    // it still takes part.
+    };
+    // The four warps that share output rows vote at a barrier in every chunk when the norm is fused, and before every chain of
+    // several; one that gives up before it still takes part.
     const bool votes = wk.emit && p.gate != nullptr;
     auto leave = [&] {
-        if (votes) named_bar_all(4 + cg, 128, false);
+        if (MANY || votes) named_bar_all(4 + cg, 128, false);
         alive = false;
     };
-    if (count > 0 && !begin_chunk(0)) leave();
 
     // ---- a chunk's outputs: bf16(y), or the gated RMSNorm of bf16(y) ---------------------------------------------------
     // O^T is read in the fragment layout, from which a transposing matrix store puts rows of the output into the tile: this
@@ -967,19 +1162,24 @@ __device__ void state_role(const SpParams& p, unsigned char* smem, const uint32_
     if (votes)
 #pragma unroll
         for (int q = 0; q < 4; ++q) nw[q] = bf16_bits_to_f32(p.norm_w[fv + 8 * q]);
-    // With the norm fused a chunk's gate values are fetched before D is formed, so that their latency is not in the walk.
-    uint16_t gt[2][2][4];
-    auto fetch_gate = [&](int c) {
-        const int i_first = (j0 + c) * CH, n = min(CH, T - i_first);
-        const uint16_t* at = p.gate + (row0 + i_first + fi) * p.gate_stride + h * DV + fv;
+    // Into (and, with the gate, out of) the output tile: a lane names the row (lane % 8) of matrix lane / 8, the matrices being
+    // (channels 8 (m % 2), rows 8 (m / 2)) of the two halves of the warp's channels.
+    const int tile_row = i0 + (lane >> 4) * 8 + (lane & 7), tile_piece = quad * 4 + ((lane >> 3) & 1);
+    // A chunk's gate values, laid out as y2 below.  They lie in the tile that the outputs go to (the loader's copy), or, in a partial chunk
+    // or where the rows are not on 16 bytes, are fetched before D is formed, so that their latency is not in the walk.
+    uint32_t gt[2][4];
+    auto fetch_gate = [&](const volatile Chain& of, int c) {
+        const int n = of.rows - c * CH;
+        const uint16_t* at = p.gate + (of.row + c * CH + fi) * p.gate_stride + of.h * DV + fv;
 #pragma unroll
         for (int g = 0; g < 2; ++g)
 #pragma unroll
-            for (int e = 0; e < 2; ++e)
-#pragma unroll
-                for (int q = 0; q < 4; ++q) gt[g][e][q] = fi + 8 * g + e < n ? at[(8 * g + e) * p.gate_stride + 8 * q] : (uint16_t)0;
+            for (int q = 0; q < 4; ++q) {
+                const uint32_t lo = fi + 8 * g < n ? at[8 * g * p.gate_stride + 8 * q] : 0u, hi = fi + 8 * g + 1 < n ? at[(8 * g + 1) * p.gate_stride + 8 * q] : 0u;
+                gt[g][q] = lo | hi << 16;
+            }
     };
-    auto emit = [&](int c) -> bool {
+    auto emit = [&](int c, bool boxes) -> bool {  // boxes: the gate values come from the tile
         bool ok = wait(bO + (c & 1), c >> 1);
         tc::fence_after_sync();
         uint32_t ra[8], rb[8];
@@ -997,65 +1197,95 @@ __device__ void state_role(const SpParams& p, unsigned char* smem, const uint32_
             y2[g][2] = tc::bf16x2(__uint_as_float(rb[4 * g]), __uint_as_float(rb[4 * g + 1]));
             y2[g][3] = tc::bf16x2(__uint_as_float(rb[4 * g + 2]), __uint_as_float(rb[4 * g + 3]));
         }
+        unsigned char* dst = smem + sOut + (c & 1) * kOutTile;
         if (votes) {
-            float sq[2][2];
+            float sq[4];  // [2 g + e]
 #pragma unroll
             for (int g = 0; g < 2; ++g) {
-                sq[g][0] = sq[g][1] = 0.0f;
+                float2 s2 = {0.0f, 0.0f};
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
-                    const float lo = __uint_as_float(y2[g][q] << 16), hi = __uint_as_float(y2[g][q] & 0xffff0000u);
-                    sq[g][0] = fmaf(lo, lo, sq[g][0]);
-                    sq[g][1] = fmaf(hi, hi, sq[g][1]);
+                    const float2 y = {__uint_as_float(y2[g][q] << 16), __uint_as_float(y2[g][q] & 0xffff0000u)};
+                    s2 = fma2(y, y, s2);
                 }
-#pragma unroll
-                for (int o = 4; o <= 16; o <<= 1) {
-                    sq[g][0] += __shfl_xor_sync(0xffffffffu, sq[g][0], o);
-                    sq[g][1] += __shfl_xor_sync(0xffffffffu, sq[g][1], o);
-                }
+                sq[2 * g] = s2.x;
+                sq[2 * g + 1] = s2.y;
             }
-            float* red = reinterpret_cast<float*>(smem + sRed) + (c & 1) * 4 * CH + fi;
-            if (lane < 4)
-#pragma unroll
-                for (int g = 0; g < 2; ++g) *reinterpret_cast<float2*>(red + quad * CH + 8 * g) = make_float2(sq[g][0], sq[g][1]);
+            // The sum over the eight lanes of a row; at the first two steps a lane gives away the rows that it does not go on with.
+            const bool up4 = lane & 4, up8 = lane & 8;
+            const float a0 = (up4 ? sq[2] : sq[0]) + __shfl_xor_sync(0xffffffffu, up4 ? sq[0] : sq[2], 4);
+            const float a1 = (up4 ? sq[3] : sq[1]) + __shfl_xor_sync(0xffffffffu, up4 ? sq[1] : sq[3], 4);
+            float a = (up8 ? a1 : a0) + __shfl_xor_sync(0xffffffffu, up8 ? a0 : a1, 8);
+            a += __shfl_xor_sync(0xffffffffu, a, 16);
+            if (lane < 16) reinterpret_cast<float*>(smem + sRed)[((c & 1) * 4 + quad) * CH + fi + 8 * (up4 ? 1 : 0) + (up8 ? 1 : 0)] = a;
+            if (boxes) ok = ok && wait(bGate + (c & 1), c >> 1);
             ok = named_bar_all(4 + cg, 128, ok);
+            if (boxes && ok) {
+                tc::ldmatrix_t4(dst + box_piece(tile_row, tile_piece), gt[0][0], gt[0][1], gt[1][0], gt[1][1]);
+                tc::ldmatrix_t4(dst + box_piece(tile_row, tile_piece + 2), gt[0][2], gt[0][3], gt[1][2], gt[1][3]);
+            }
+            // A row's factor is formed by one lane of each of the first two quarters (a square root and a division, both IEEE).
+            float rinv;
+            {
+                const float* at = reinterpret_cast<const float*>(smem + sRed) + (c & 1) * 4 * CH + i0 + (lane & 15);
+                rinv = 1.0f / sqrtf((((at[0] + at[CH]) + at[2 * CH]) + at[3 * CH]) / (float)DV + p.eps);
+            }
 #pragma unroll
             for (int g = 0; g < 2; ++g) {
-                float tot[2] = {0.0f, 0.0f}, rinv[2];
+                const float2 rv = {__shfl_sync(0xffffffffu, rinv, 2 * (lane & 3) + 8 * g), __shfl_sync(0xffffffffu, rinv, 2 * (lane & 3) + 8 * g + 1)};
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
-                    const float2 s2 = *reinterpret_cast<const float2*>(red + q * CH + 8 * g);
-                    tot[0] += s2.x;
-                    tot[1] += s2.y;
-                }
-#pragma unroll
-                for (int e = 0; e < 2; ++e) rinv[e] = 1.0f / sqrtf(tot[e] / (float)DV + p.eps);
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const float lo = __uint_as_float(y2[g][q] << 16), hi = __uint_as_float(y2[g][q] & 0xffff0000u);
-                    y2[g][q] = tc::bf16x2(nw[q] * (lo * rinv[0]) * __fdividef(1.0f, 1.0f + __expf(-bf16_bits_to_f32(gt[g][0][q]))),
-                                          nw[q] * (hi * rinv[1]) * __fdividef(1.0f, 1.0f + __expf(-bf16_bits_to_f32(gt[g][1][q]))));
+                    const float2 sig = {rcp_approx(1.0f + ex2_ftz(-kLog2e * __uint_as_float(gt[g][q] << 16))), rcp_approx(1.0f + ex2_ftz(-kLog2e * __uint_as_float(gt[g][q] & 0xffff0000u)))};
+                    const float2 y = mul2(mul2({nw[q], nw[q]}, mul2({__uint_as_float(y2[g][q] << 16), __uint_as_float(y2[g][q] & 0xffff0000u)}, rv)), sig);
+                    y2[g][q] = tc::bf16x2(y.x, y.y);
                 }
             }
         }
-        // Into the output tile (the output warp takes it from there): a lane names the row (lane % 8) of matrix lane / 8, the
-        // matrices being (channels 8 (m % 2), rows 8 (m / 2)) of the two halves of the warp's channels.
-        if (!ok) return false;
-        unsigned char* dst = smem + sOut + (c & 1) * kOutTile;
-        const int row = i0 + (lane >> 4) * 8 + (lane & 7), piece = quad * 4 + ((lane >> 3) & 1);
-        tc::stmatrix_t4(dst + box_piece(row, piece), y2[0][0], y2[0][1], y2[1][0], y2[1][1]);
-        tc::stmatrix_t4(dst + box_piece(row, piece + 2), y2[0][2], y2[0][3], y2[1][2], y2[1][3]);
+        if (!ok) return false;  // else the output warp takes it from there
+        tc::stmatrix_t4(dst + box_piece(tile_row, tile_piece), y2[0][0], y2[0][1], y2[1][0], y2[1][1]);
+        tc::stmatrix_t4(dst + box_piece(tile_row, tile_piece + 2), y2[0][2], y2[0][3], y2[1][2], y2[1][3]);
         fence_proxy_async_smem();  // the tensor stores read the tile through the async proxy
         __syncwarp();
         if (lane == 0) mbar_arrive(&bars[bOutFull + (c & 1)]);
         return true;
     };
 
-    for (int c = 0; alive && c < count; ++c) {
+    // The outputs of a chunk leave behind the next chunk's D, be that chunk of the same chain or of the next; a chain's record is released
+    // with its last outputs.
+    int C = 0, due = -1, due_seq = 0;  // due: the chunk of chain due_seq whose outputs are still to leave
+    int held = -1;                     // the chain before, while its record is
+    auto out_boxes = [&] { return p.gate_boxes != 0 && recs[due_seq & 1].rows - due * CH >= CH; };
+    auto emit_due = [&]() -> bool {
+        const bool ok = emit(C - 1, votes && out_boxes());
+        due = -1;
+        if (ok) return true;
+        if (votes) alive = false;  // it has voted
+        else leave();
+        return false;
+    };
+    auto emit_last = [&]() -> bool {  // where no D is on its way
+        if (votes && !out_boxes()) fetch_gate(recs[due_seq & 1], due);
+        return emit_due();
+    };
+    for (int seq = 0;; ++seq) {
+    const int count = chain_count(seq);
+    if (MANY) {
+        if (!named_bar_all(4 + cg, 128, count != -2)) { alive = false; break; }
+    } else if (count == -2) { leave(); break; }
+    if (count < 0) break;
+    state_in(recs[seq & 1].start, recs[seq & 1].s_elem);
+    // A sequence of no rows has no D to wait for, and the output warp, which has to read its record too, may wait for these.
+    if (count == 0 && held >= 0) {
+        if (due >= 0 && !emit_last()) break;
+        release(held);
+        held = -1;
+    }
+    if (count > 0 && !begin_chunk(C)) { leave(); break; }
+    for (int c = 0; c < count; ++c, ++C) {
         // ---- D^T = U^T - (W S)^T as bf16 hi + lo pairs of rows ------------------------------------------------------------
         float uu[16];
-        if (votes && c > 0) fetch_gate(c - 1);
-        if (!wait(bFullU, c)) { leave(); break; }
+        if (votes && due >= 0 && !out_boxes()) fetch_gate(recs[due_seq & 1], due);
+        if (!wait(bFullU, C)) { leave(); break; }
 #pragma unroll
         for (int x = 0; x < 4; ++x) {
             const float4 u4 = *reinterpret_cast<const float4*>(smem + sU + u_cell(cg * 4 + x, v));
@@ -1063,7 +1293,7 @@ __device__ void state_role(const SpParams& p, unsigned char* smem, const uint32_
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(&bars[bEmptyU]);  // U is consumed
-        if (!wait(bWS, c)) { leave(); break; }
+        if (!wait(bWS, C)) { leave(); break; }
         tc::fence_after_sync();
         {
             uint32_t r[16], wh[8], wl[8];
@@ -1077,47 +1307,45 @@ __device__ void state_role(const SpParams& p, unsigned char* smem, const uint32_
             arrive(bD);
         }
         // The outputs of the chunk before leave while the state's product runs.
-        if (wk.emit && c > 0 && !emit(c - 1)) { alive = false; break; }
-        if (!wait(bSNew, c)) { leave(); break; }
+        if (due >= 0 && !emit_due()) break;
+        if (held >= 0) release(held);
+        held = -1;
+        if (wk.emit) due = c;
+        due_seq = seq;
+        if (!wait(bSNew, C)) { leave(); break; }
         tc::fence_after_sync();
-        if (c + 1 < count && !begin_chunk(c + 1)) { leave(); break; }
-    }
-    if (alive && wk.emit && count > 0) {
-        if (votes) fetch_gate(count - 1);
-        alive = emit(count - 1);
+        if (c + 1 < count && !begin_chunk(C + 1)) { leave(); break; }
     }
 
     // ---- the outgoing state ---------------------------------------------------------------------------------------------
-    if (alive && wk.fin != 2) {
-        uint32_t r[32];
-        tc::tmem_ld32(tc::tmem_addr(tm, quad, tS + k_first), r);
-        tc::tmem_ld_wait();
-        if (wk.fin == 0 && p.state_bf16) {
-            uint16_t* at = reinterpret_cast<uint16_t*>(p.state_out) + s_at;
-            uint32_t pr[16];
+    if (!alive) break;
+    const long long s_out = recs[seq & 1].s_elem + b_at;
+    if (wk.fin != 2) {
+        const uint32_t from = tc::tmem_addr(tm, quad, tS + k_first);
+        uint16_t* to16 = reinterpret_cast<uint16_t*>(p.state_out) + s_out;
+        float* to32 = wk.fin == 1 ? wk.to + b_at : reinterpret_cast<float*>(p.state_out) + s_out;
+        const bool to_bf16 = wk.fin == 0 && p.state_bf16;
+        if (piece_aligned(to_bf16 ? (const void*)to16 : (const void*)to32)) {
+            if (to_bf16) state_from_tmem(from, to16 - lane * DK, lane);
+            else state_from_tmem(from, to32 - lane * DK, lane);
+        } else {
 #pragma unroll
-            for (int x = 0; x < 16; ++x) pr[x] = tc::bf16x2(__uint_as_float(r[2 * x]), __uint_as_float(r[2 * x + 1]));
-            if ((reinterpret_cast<uintptr_t>(at) & 15) == 0) {
-#pragma unroll
-                for (int x = 0; x < 4; ++x) reinterpret_cast<uint4*>(at)[x] = make_uint4(pr[4 * x], pr[4 * x + 1], pr[4 * x + 2], pr[4 * x + 3]);
-            } else {
+            for (int half = 0; half < 2; ++half) {
+                uint32_t r[16];
+                tc::tmem_ld16(from + half * 16, r);
+                tc::tmem_ld_wait();
 #pragma unroll
                 for (int x = 0; x < 16; ++x) {
-                    at[2 * x] = (uint16_t)pr[x];
-                    at[2 * x + 1] = (uint16_t)(pr[x] >> 16);
+                    if (to_bf16) to16[half * 16 + x] = f32_to_bf16_bits(__uint_as_float(r[x]));
+                    else to32[half * 16 + x] = __uint_as_float(r[x]);
                 }
-            }
-        } else {
-            float* at = wk.fin == 1 ? wk.to + b_at : reinterpret_cast<float*>(p.state_out) + s_at;
-            if ((reinterpret_cast<uintptr_t>(at) & 15) == 0) {
-#pragma unroll
-                for (int x = 0; x < 8; ++x) reinterpret_cast<uint4*>(at)[x] = make_uint4(r[4 * x], r[4 * x + 1], r[4 * x + 2], r[4 * x + 3]);
-            } else {
-#pragma unroll
-                for (int x = 0; x < 32; ++x) at[x] = __uint_as_float(r[x]);
             }
         }
     }
+    if (count == 0) release(seq);
+    else held = seq;
+    }
+    if (alive && due >= 0) emit_last();
     tc::fence_before_sync();
     __syncthreads();
 }
@@ -1127,39 +1355,15 @@ __device__ void state_role(const SpParams& p, unsigned char* smem, const uint32_
 template <bool LAYER>
 __device__ void fused_roles(const SpParams& p, unsigned char* smem, const uint32_t tm) {
     volatile uint32_t* ctl = reinterpret_cast<volatile uint32_t*>(smem + oCtl);
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + oBarsState);
-    unsigned int* set = p.sets + p.ctr * kTailSet;
-    const int tid = threadIdx.x, chains = p.batch * p.H;
+    const int tid = threadIdx.x;
     intra_role<LAYER>(p, smem, tm);
     if (ctl[1] != 0u) return;
     if (tid < kGroupBars * kGroups) mbar_inval(reinterpret_cast<uint64_t*>(smem + tid / kGroupBars * kGroupBytes + gBars) + tid % kGroupBars);
-    for (bool first = true;; first = false) {
-        fence_proxy_async_smem();  // what the role before left in shared memory is overwritten by bulk copies
-        tc::fence_before_sync();
-        __syncthreads();
-        if (tid == 0) {
-            const int chain = (int)atomicAdd(set + 1, 1u);
-            if (chain < chains) {
-                const int g = chain / p.group, want = min(p.group, chains - g * p.group) * p.seg_chunks;
-                if (!count_wait(set + 2 + g, (unsigned)want, WaitCtx{ctl, ctl + 1, p.status}, kStatusWaitPrefill)) ctl[1] = 1u;
-                if (!first)
-                    for (int i = 0; i < kStateBars; ++i) {
-                        mbar_inval(bars + i);
-                        mbar_init(bars + i, state_bar_count(i));
-                    }
-                mbar_init_fence();
-            }
-            ctl[3] = (uint32_t)chain;
-        }
-        __syncthreads();
-        tc::fence_after_sync();
-        fence_proxy_async_global();
-        const int chain = (int)ctl[3];
-        if (chain >= chains || ctl[1] != 0u) break;
-        const Walk wk{p.state_chunk0, p.state_chunk0 + p.seg_chunks, 0, nullptr, 0, nullptr, true, true};
-        state_role(p, smem, tm, chain, wk);
-        if (ctl[1] != 0u) break;
-    }
+    fence_proxy_async_smem();  // what the intra role left in shared memory is overwritten by bulk copies
+    tc::fence_before_sync();
+    __syncthreads();
+    tc::fence_after_sync();
+    state_role<true>(p, smem, tm, 0, Walk{p.state_chunk0, p.state_chunk0 + p.seg_chunks, 0, nullptr, 0, nullptr, true, true});
 }
 
 // One launch: the state role of one segment on the chain blocks, then the intra role of the next segment on all blocks.
@@ -1186,34 +1390,36 @@ __global__ void __launch_bounds__(kThreadsSp, 1) prefill_sp_kernel(const __grid_
     // beside the next super-block's intra launch on another stream.)
     if (p.fused && blockIdx.x == 0 && tid < kTailSet) p.sets[(p.ctr ^ 1) * kTailSet + tid] = 0u;
     if (!p.fused && blockIdx.x == 0 && tid == 0 && p.scan_pass == 0) p.counters[p.ctr ^ 1] = 0u;
-    const int chains = p.batch * p.H;
     if (p.fused) {
         fused_roles<LAYER>(p, smem, tm);
-    } else if (p.scan_pass == 1) {  // (chain, segment s < scan_p1, kind): the segment's offset and transition
-        const int kind = blockIdx.x & 1, sg = (blockIdx.x >> 1) % p.scan_p1, chain = (blockIdx.x >> 1) / p.scan_p1;
-        if (chain < chains) {
+    } else if (p.has_state) {
+        // Block (chain); (chain, segment s < scan_p1, kind) in scan pass 1: the segment's offset and transition; (chain, segment) in
+        // scan pass 2: the walk with outputs from the segment's true incoming state, of which only the last delivers the sequence's
+        // final state (the others end where the next one starts).
+        const int pass = p.scan_pass, kind = blockIdx.x & 1, per = pass == 1 ? p.scan_p1 : pass == 2 ? p.scan_k : 1;
+        const int at = pass == 1 ? blockIdx.x >> 1 : blockIdx.x, sg = at % per, chain = at / per;
+        if (chain < p.batch * p.H) {
             const int hi = p.state_chunk0 + p.seg_chunks;  // the launch's chunk range ends here
-            const bool last = sg == p.scan_k - 1;
-            const int end = last ? (p.scan_open ? 0x7fffffff : hi) : min(p.state_chunk0 + (sg + 1) * p.scan_chunks, hi);
-            const Walk wk{min(p.state_chunk0 + sg * p.scan_chunks, hi), end, kind ? 2 : 1, nullptr, 1,
-                          p.scan_ab + (((size_t)chain * p.scan_p1 + sg) * 2 + kind) * DV * DK, kind == 0, false};
-            state_role(p, smem, tm, chain, wk);
+            Walk wk{p.state_chunk0, hi, 0, nullptr, 0, nullptr, true, true};
+            if (pass != 0) {
+                const bool last = sg == p.scan_k - 1;
+                wk.ja = min(p.state_chunk0 + sg * p.scan_chunks, hi);
+                wk.jb = last ? (p.scan_open ? 0x7fffffff : hi) : min(p.state_chunk0 + (sg + 1) * p.scan_chunks, hi);
+                if (pass == 1) {
+                    wk.init = kind ? 2 : 1;
+                    wk.fin = 1;
+                    wk.to = p.scan_ab + (((size_t)chain * p.scan_p1 + sg) * 2 + kind) * DV * DK;
+                    wk.use_u = kind == 0;
+                    wk.emit = false;
+                } else {
+                    wk.init = 3;
+                    wk.from = p.scan_start + ((size_t)chain * p.scan_k + sg) * DV * DK;
+                    wk.fin = last ? 0 : 2;
+                }
+            }
+            state_role<false>(p, smem, tm, chain, wk);
+            tc::fence_after_sync();
         }
-    } else if (p.scan_pass == 2) {  // (chain, segment): the walk with outputs from the segment's true incoming state
-        const int sg = blockIdx.x % p.scan_k, chain = blockIdx.x / p.scan_k;
-        if (chain < chains) {
-            // Only the last segment delivers the sequence's final state; the others end where the next one starts.
-            const bool last = sg == p.scan_k - 1;
-            const int hi = p.state_chunk0 + p.seg_chunks;
-            const int end = last ? (p.scan_open ? 0x7fffffff : hi) : min(p.state_chunk0 + (sg + 1) * p.scan_chunks, hi);
-            const Walk wk{min(p.state_chunk0 + sg * p.scan_chunks, hi), end, 3, p.scan_start + ((size_t)chain * p.scan_k + sg) * DV * DK,
-                          last ? 0 : 2, nullptr, true, true};
-            state_role(p, smem, tm, chain, wk);
-        }
-    } else if (p.has_state && blockIdx.x < (unsigned)chains) {
-        const Walk wk{p.state_chunk0, p.state_chunk0 + p.seg_chunks, 0, nullptr, 0, nullptr, true, true};
-        state_role(p, smem, tm, (int)blockIdx.x, wk);
-        tc::fence_after_sync();
     }
     if (!p.fused && p.has_intra && ctl[1] == 0u) intra_role<LAYER>(p, smem, tm);
     if (ctl[1] != 0u) {  // after an abort copies into this block's shared memory may still be in flight: give them a bounded time
@@ -1272,17 +1478,25 @@ __global__ void __launch_bounds__(128) scan_compose_kernel(const __grid_constant
 
 }  // namespace
 
-// A [rows][H][128] tensor of `elem`-byte elements as (128, H, rows) with boxes of 64 rows of one head, 128 bytes wide.
-static bool row_tensor_map(CUtensorMap* tm, const void* base, int elem, int H, long long rows) {
+// A [rows][H][128] tensor of `elem`-byte elements, its rows row_bytes apart (0: dense), as (128, H, rows) with boxes of 64 rows of one
+// head, 128 bytes wide.
+static bool row_tensor_map(CUtensorMap* tm, const void* base, int elem, int H, long long rows, long long row_bytes = 0) {
     EncodeTiled enc = encode_tiled();
     if (enc == nullptr) return false;
     const cuuint64_t dims[3] = {(cuuint64_t)DK, (cuuint64_t)H, (cuuint64_t)rows};
-    const cuuint64_t strides[2] = {(cuuint64_t)DK * elem, (cuuint64_t)H * DK * elem};
+    const cuuint64_t strides[2] = {(cuuint64_t)DK * elem, row_bytes != 0 ? (cuuint64_t)row_bytes : (cuuint64_t)H * DK * elem};
     const cuuint32_t box[3] = {(cuuint32_t)(128 / elem), 1u, (cuuint32_t)CH};
     const cuuint32_t estr[3] = {1u, 1u, 1u};
     return enc(tm, elem == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<void*>(base), dims, strides, box, estr,
                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// The gate rows' map, where they are on 16 bytes; else the walk reads them value by value.
+static void gate_tensor_map(SpParams& p, long long rows) {
+    const long long bytes = p.gate_stride * 2;
+    p.gate_boxes = p.gate != nullptr && ((reinterpret_cast<uintptr_t>(p.gate) | (uintptr_t)bytes) & 15) == 0 && bytes >= (long long)p.H * DV * 2 &&
+                   row_tensor_map(&p.tm_gate, p.gate, 2, p.H, rows, bytes);
 }
 
 constexpr long long kCounterBytes = kPrefillTailBytes;  // tail of the workspace: the launches' counters (kda_internal.h)
@@ -1396,6 +1610,7 @@ int core_prefill_sp_launch(int32_t heads, int32_t batch, const int32_t* cu_seqle
         !row_tensor_map(&p.tm_v, v, 2, heads, rows_cap) || !row_tensor_map(&p.tm_g, g, 4, heads, rows_cap))
         return (int)cudaErrorNotSupported;
     if (out != nullptr && !row_tensor_map(&p.tm_out, out, 2, heads, rows_cap)) return (int)cudaErrorNotSupported;
+    gate_tensor_map(p, rows_cap);
     for (int r = 0; r < p.ranks; ++r)
         if (!row_tensor_map(&p.tm_full[r], p.full[r], 2, p.heads_total, rows_cap)) return (int)cudaErrorNotSupported;
     cudaError_t e = cudaMemsetAsync(p.counters, 0, kCounterBytes, stream);
@@ -1585,6 +1800,7 @@ int layer_pass_launch(int32_t heads, int32_t batch, const int32_t* cu_rows, int3
     if (p.status == nullptr) return (int)cudaErrorUnknown;
     // Only full chunks leave by tensor stores, and the metadata vouches for their rows: the map's extent bounds nothing.
     if (!row_tensor_map(&p.tm_out, out, 2, heads, 0x7fffffffll)) return (int)cudaErrorNotSupported;
+    gate_tensor_map(p, 0x7fffffffll);
     return fused_launch<true>(p, slots, tail, chunk0 / chunks, chunks, chunk0, stream);
 }
 

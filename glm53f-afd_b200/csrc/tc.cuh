@@ -130,10 +130,19 @@ __device__ __forceinline__ void tmem_ld_frag(uint32_t taddr, uint32_t (&r)[8]) {
                  : "r"(taddr)
                  : "memory");
 }
+__device__ __forceinline__ void tmem_st_frag(uint32_t taddr, const uint32_t (&r)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.16x256b.x2.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]),
+                 "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+                 : "memory");
+}
 // Four 8 x 8 bf16 matrices, each register a fragment as above (row l / 4, two columns), stored transposed: column j of matrix m
 // goes to the 16 bytes that lane 8 m + j names.
 __device__ __forceinline__ void stmatrix_t4(void* row, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
     asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(smem_u32(row)), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+// And back: the fragments of the four matrices that stmatrix_t4 with these addresses would have stored.
+__device__ __forceinline__ void ldmatrix_t4(const void* row, uint32_t& a, uint32_t& b, uint32_t& c, uint32_t& d) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(a), "=r"(b), "=r"(c), "=r"(d) : "r"(smem_u32(row)) : "memory");
 }
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
     asm volatile(
