@@ -90,9 +90,9 @@ struct SpParams {
     int ranks, heads_total, head0;
     unsigned int* counters;  // [2] item counters: this launch hands items out of counters[ctr], and zeroes the other
     int ctr;
-    // One persistent launch for both roles (fused != 0): items, then chains, are handed out from tail set ctr; chains form groups
+    // One persistent launch for both roles: items, then chains, are handed out from tail set ctr; chains form groups
     // of `group`, and a chain's state role starts when all items of its group are finished.
-    int fused, group;
+    int group;
     unsigned int* sets;
     int* status;
     // The scan over segments of the sequence (scan_pass != 0; FP32 states; the workspace holds every chunk).  Segment s of
@@ -120,9 +120,10 @@ struct Item {
     int chain, jj, group;
 };
 // Chunk-major, neighbouring chains next to each other; in a fused launch so within each group of chains.
+template <bool FUSED>
 __device__ __forceinline__ Item item_of(const SpParams& p, int item) {
     const int chains = p.batch * p.H;
-    if (!p.fused) return {item % chains, item / chains, 0};
+    if (!FUSED) return {item % chains, item / chains, 0};
     const int per = p.group * p.seg_chunks, g = item / per, rem = item - g * per, n = min(p.group, chains - g * p.group);
     return {g * p.group + rem % n, rem / n, g};
 }
@@ -177,8 +178,11 @@ static_assert(kGroups * kGroupBytes <= oCtl, "two groups must fit below the bloc
 constexpr uint32_t gcL = 0, gcM = 64, gcW = 0, gcU = 64, kGroupCols = 128;
 
 // LAYER: the items' inputs are in their slots (kda_internal.h), which the results then replace.  G = 0 or 1, a runtime value: both groups run the same instructions (one copy of this code in the instruction cache).
-template <bool LAYER>
+template <bool LAYER, bool FUSED>
 __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* smem, const uint32_t tm_block, const WaitCtx& ctx, const int G) {
+    // The layer form's items take the block-wise branch, whose instructions are the most: there the issue loops stay loops (4 x 2,048 rows
+    // 985 -> 955 us), which on the one-product branch of the core form costs more than it saves (8,192 rows 480 -> 494).
+    constexpr int kIssue = LAYER ? 1 : 8;
     const int BAR = 2 + G;
     unsigned char* gs = smem + G * kGroupBytes;
     const uint32_t tm = tm_block + G * kGroupCols;
@@ -190,7 +194,6 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
     float* betas = reinterpret_cast<float*>(gs + gBeta);
     const int gt = threadIdx.x - G * kGroupThreads, gw = gt >> 5, lane = gt & 31;
     const int quad = gw & 3, cg = gw >> 2;  // a warp reaches tensor-memory lanes 32 * (warp % 4)..; cg picks a half of the columns
-    const int lane_row64 = quad * 16 + lane;
     auto group_sync = [&]() { named_bar_sync(BAR, kGroupThreads); };
     auto publish = [&]() {
         fence_proxy_async_smem();
@@ -212,7 +215,7 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
     // one's last products, when they have long landed.
     int unreported = -1;
     auto report = [&]() {
-        if (p.fused && unreported >= 0 && gt == kGroupThreads - 1) {
+        if (FUSED && unreported >= 0 && gt == kGroupThreads - 1) {
             __threadfence();
             atomicAdd(p.sets + p.ctr * kTailSet + 2 + unreported, 1u);
         }
@@ -229,7 +232,7 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
         if (!mbar_wait(bar_g, raw_phase, ctx, kStatusWaitPrefill)) break;
         const int item = *item_slot;
         if (item < 0) break;
-        const Item at_item = item_of(p, item);
+        const Item at_item = item_of<FUSED>(p, item);
         unsigned char* slot = slot_of(p.ws_intra, p.seg_chunks, at_item.chain, at_item.jj);
 
         bool mild;
@@ -285,94 +288,103 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
         // own gates only, so it is the same however the call is batched or cut into passes.
         const bool narrow = named_bar_all(BAR, kGroupThreads, mild);
 
-        // ---- 2. a of this thread's row and 32 channels into registers -----------------------------------------------------------
-        const int r = gt & 63, cq = gt >> 6, J = r >> 4;
-        float a[32];
-#pragma unroll
-        for (int pp = 0; pp < 8; ++pp) {
-            const float4 x = *reinterpret_cast<const float4*>(gs + gG + box_piece(r, cq * 8 + pp));
-            a[pp * 4 + 0] = x.x; a[pp * 4 + 1] = x.y; a[pp * 4 + 2] = x.z; a[pp * 4 + 3] = x.w;
-        }
-        group_sync();  // nobody reads the staged a (or the scan's scratch) any more: the tiles may go over them
-        if (!mbar_wait(bar_raw, raw_phase, ctx, kStatusWaitPrefill)) break;
-        raw_phase ^= 1u;
-
-        // ---- 3. operand tiles, first those made from k.  Row side Kgb = K a; Kg = K exp(G) (over K) for W; Kdec =
-        // K exp(G_last - G) as bf16 hi + lo out to the workspace; column sides K exp(Gm_I - G) into the tiles I >= J.
+        // ---- 2., 3. operand tiles -------------------------------------------------------------------------------------------------
         const float* tabs = reinterpret_cast<const float*>(gs + gTab);
+        float a[32];
+        // The block-wise form's share of a thread: a row of blocks J and 3 - J, sixteen channels each, so that every warp makes as many
+        // column-side pieces (3 - J a piece; with one row of 32 channels a thread, half of the warps made three times the others').
+        auto block = [&](int t) { return t < 2 ? gw & 1 : 3 - (gw & 1); };
+        auto row = [&](int t) { return block(t) * 16 + (lane & 15); };
+        auto piece = [&](int t) { return (gw >> 1) * 4 + (lane >> 4) * 2 + (t & 1); };
         if (narrow) {
             // One reference (the chunk's start): Kg = K exp(G) (over K) is the row side of L and the operand of W, Kinv = K exp(-G)
-            // the one column-side tile (the 64-row tile), Kdec = Kinv exp(G_last).
-#pragma unroll
-            for (int cc = 0; cc < 4; ++cc) {
-                const int c = cq * 4 + cc;
-                const uint4 k8 = *reinterpret_cast<const uint4*>(gs + gK + box_piece(r, c));
+            // (in Kgb's place) the one column-side tile, Kdec = Kinv exp(G_last) as bf16 hi + lo out to the workspace, Qg = Q exp(G) (over Q and
+            // out) the row side of M.  All from one read of a, in a loop that stays a loop: the group's instructions are more than
+            // the cache next to the warps holds.
+            if (!mbar_wait(bar_raw, raw_phase, ctx, kStatusWaitPrefill)) break;
+            raw_phase ^= 1u;
+            const int r = gt & 63, cq = gt >> 6, J = r >> 4;
+#pragma unroll 1
+            for (int c = cq * 4; c < cq * 4 + 4; ++c) {
+                const uint4 k8 = *reinterpret_cast<const uint4*>(gs + gK + box_piece(r, c)), q8 = *reinterpret_cast<const uint4*>(gs + gQ + box_piece(r, c));
+                const float4 aa = *reinterpret_cast<const float4*>(gs + gG + box_piece(r, 2 * c)), ab = *reinterpret_cast<const float4*>(gs + gG + box_piece(r, 2 * c + 1));
                 const float4 e0a = *reinterpret_cast<const float4*>(tabs + (tE0 + J) * 128 + c * 8), e0b = *reinterpret_cast<const float4*>(tabs + (tE0 + J) * 128 + c * 8 + 4);
                 const float4 gla = *reinterpret_cast<const float4*>(gs + gGl + c * 32), glb = *reinterpret_cast<const float4*>(gs + gGl + c * 32 + 16);
+                const float2 A[4] = {{aa.x, aa.y}, {aa.z, aa.w}, {ab.x, ab.y}, {ab.z, ab.w}};
                 const float2 E0[4] = {{e0a.x, e0a.y}, {e0a.z, e0a.w}, {e0b.x, e0b.y}, {e0b.z, e0b.w}};
                 const float2 GL[4] = {{gla.x, gla.y}, {gla.z, gla.w}, {glb.x, glb.y}, {glb.z, glb.w}};
-                const uint32_t kw[4] = {k8.x, k8.y, k8.z, k8.w};
-                uint32_t kg[4], ki[4], dh[4], dl[4];
+                const uint32_t kw[4] = {k8.x, k8.y, k8.z, k8.w}, qw[4] = {q8.x, q8.y, q8.z, q8.w};
+                uint32_t kg[4], ki[4], dh[4], dl[4], qg[4];
 #pragma unroll
                 for (int u2 = 0; u2 < 4; ++u2) {
-                    const float2 kf = widen2<LAYER>(kw[u2]);
-                    const float2 e = mul2({a[cc * 8 + 2 * u2], a[cc * 8 + 2 * u2 + 1]}, E0[u2]);
-                    a[cc * 8 + 2 * u2] = e.x;  // exp(G): what the tiles made from q need
-                    a[cc * 8 + 2 * u2 + 1] = e.y;
-                    const float2 v_kg = mul2(kf, e), v_ki = mul2(kf, {rcp_approx(e.x), rcp_approx(e.y)}), v_kd = mul2(v_ki, GL[u2]);
+                    const float2 kf = widen2<LAYER>(kw[u2]), e = mul2(A[u2], E0[u2]);
+                    const float2 v_kg = mul2(kf, e), v_ki = mul2(kf, {rcp_approx(e.x), rcp_approx(e.y)}), v_kd = mul2(v_ki, GL[u2]), v_qg = mul2(widen2<LAYER>(qw[u2]), e);
                     kg[u2] = tc::bf16x2(v_kg.x, v_kg.y);
                     ki[u2] = tc::bf16x2(v_ki.x, v_ki.y);
+                    qg[u2] = tc::bf16x2(v_qg.x, v_qg.y);
                     tc::split_bf16x2(v_kd.x, v_kd.y, dh[u2], dl[u2]);
                 }
                 *reinterpret_cast<uint4*>(gs + gK + box_piece(r, c)) = make_uint4(kg[0], kg[1], kg[2], kg[3]);
-                *reinterpret_cast<uint4*>(gs + gKc + kc_piece(3, r, c)) = make_uint4(ki[0], ki[1], ki[2], ki[3]);
+                *reinterpret_cast<uint4*>(gs + gKb + box_piece(r, c)) = make_uint4(ki[0], ki[1], ki[2], ki[3]);
+                *reinterpret_cast<uint4*>(gs + gQ + box_piece(r, c)) = make_uint4(qg[0], qg[1], qg[2], qg[3]);
                 *reinterpret_cast<uint4*>(cell(slot + wKdHi, CH, c, r)) = make_uint4(dh[0], dh[1], dh[2], dh[3]);
                 *reinterpret_cast<uint4*>(cell(slot + wKdLo, CH, c, r)) = make_uint4(dl[0], dl[1], dl[2], dl[3]);
+                *reinterpret_cast<uint4*>(cell(slot + wQg, CH, c, r)) = make_uint4(qg[0], qg[1], qg[2], qg[3]);
             }
         } else {
+            // a into registers: the column-side tiles go over it.  Then the tiles made from k: row side Kgb = K a; Kg = K exp(G)
+            // (over K) for W; Kdec = K exp(G_last - G) as bf16 hi + lo out to the workspace; column sides K exp(Gm_I - G) into the
+            // tiles I >= J.
 #pragma unroll
-        for (int cc = 0; cc < 4; ++cc) {
-            const int c = cq * 4 + cc;
-            const uint4 k8 = *reinterpret_cast<const uint4*>(gs + gK + box_piece(r, c));
-            const float4 e0a = *reinterpret_cast<const float4*>(tabs + (tE0 + J) * 128 + c * 8), e0b = *reinterpret_cast<const float4*>(tabs + (tE0 + J) * 128 + c * 8 + 4);
-            const float4 ela = *reinterpret_cast<const float4*>(tabs + (tEL + J) * 128 + c * 8), elb = *reinterpret_cast<const float4*>(tabs + (tEL + J) * 128 + c * 8 + 4);
-            const float E0[8] = {e0a.x, e0a.y, e0a.z, e0a.w, e0b.x, e0b.y, e0b.z, e0b.w};
-            const float EL[8] = {ela.x, ela.y, ela.z, ela.w, elb.x, elb.y, elb.z, elb.w};
-            const uint32_t kw[4] = {k8.x, k8.y, k8.z, k8.w};
-            uint32_t kg[4], kgb[4], kcd[4], dh[4], dl[4];
-            float kc[8];  // K exp(Gm_J - G): the column side inside the row's own block
+            for (int t = 0; t < 4; ++t)
 #pragma unroll
-            for (int u2 = 0; u2 < 4; ++u2) {
-                const float2 k2 = widen2<LAYER>(kw[u2]);
-                const float kf[2] = {k2.x, k2.y};
-                float v_kg[2], v_kgb[2], hi[2], lo[2];
-#pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                    const float av = a[cc * 8 + 2 * u2 + u], inva = rcp_approx(av);
-                    v_kgb[u] = kf[u] * av;
-                    v_kg[u] = kf[u] * (av * E0[2 * u2 + u]);
-                    kc[2 * u2 + u] = kf[u] * inva;
-                    tc::split_bf16(kc[2 * u2 + u] * EL[2 * u2 + u], hi[u], lo[u]);
+                for (int h = 0; h < 2; ++h) {
+                    const float4 x = *reinterpret_cast<const float4*>(gs + gG + box_piece(row(t), 2 * piece(t) + h));
+                    a[t * 8 + 4 * h + 0] = x.x; a[t * 8 + 4 * h + 1] = x.y; a[t * 8 + 4 * h + 2] = x.z; a[t * 8 + 4 * h + 3] = x.w;
                 }
-                kg[u2] = tc::bf16x2(v_kg[0], v_kg[1]);
-                kgb[u2] = tc::bf16x2(v_kgb[0], v_kgb[1]);
-                kcd[u2] = tc::bf16x2(kc[2 * u2], kc[2 * u2 + 1]);
-                dh[u2] = tc::bf16x2(hi[0], hi[1]);
-                dl[u2] = tc::bf16x2(lo[0], lo[1]);
+            group_sync();  // nobody reads the staged a (or the scan's scratch) any more: the tiles may go over them
+            if (!mbar_wait(bar_raw, raw_phase, ctx, kStatusWaitPrefill)) break;
+            raw_phase ^= 1u;
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                const int c = piece(t), J = block(t), r = row(t);
+                const uint4 k8 = *reinterpret_cast<const uint4*>(gs + gK + box_piece(r, c));
+                const float4 e0a = *reinterpret_cast<const float4*>(tabs + (tE0 + J) * 128 + c * 8), e0b = *reinterpret_cast<const float4*>(tabs + (tE0 + J) * 128 + c * 8 + 4);
+                const float4 ela = *reinterpret_cast<const float4*>(tabs + (tEL + J) * 128 + c * 8), elb = *reinterpret_cast<const float4*>(tabs + (tEL + J) * 128 + c * 8 + 4);
+                const float2 E0[4] = {{e0a.x, e0a.y}, {e0a.z, e0a.w}, {e0b.x, e0b.y}, {e0b.z, e0b.w}};
+                const float2 EL[4] = {{ela.x, ela.y}, {ela.z, ela.w}, {elb.x, elb.y}, {elb.z, elb.w}};
+                const uint32_t kw[4] = {k8.x, k8.y, k8.z, k8.w};
+                uint32_t kg[4], kgb[4], kcd[4], dh[4], dl[4];
+                float2 kc[4];  // K exp(Gm_J - G): the column side inside the row's own block
+#pragma unroll
+                for (int u2 = 0; u2 < 4; ++u2) {
+                    const float2 kf = widen2<LAYER>(kw[u2]), av = {a[t * 8 + 2 * u2], a[t * 8 + 2 * u2 + 1]};
+                    const float2 v_kgb = mul2(kf, av), v_kg = mul2(kf, mul2(av, E0[u2]));
+                    kc[u2] = mul2(kf, {rcp_approx(av.x), rcp_approx(av.y)});
+                    const float2 v_kd = mul2(kc[u2], EL[u2]);
+                    kg[u2] = tc::bf16x2(v_kg.x, v_kg.y);
+                    kgb[u2] = tc::bf16x2(v_kgb.x, v_kgb.y);
+                    kcd[u2] = tc::bf16x2(kc[u2].x, kc[u2].y);
+                    tc::split_bf16x2(v_kd.x, v_kd.y, dh[u2], dl[u2]);
+                }
+                *reinterpret_cast<uint4*>(gs + gK + box_piece(r, c)) = make_uint4(kg[0], kg[1], kg[2], kg[3]);
+                *reinterpret_cast<uint4*>(gs + gKb + box_piece(r, c)) = make_uint4(kgb[0], kgb[1], kgb[2], kgb[3]);
+                *reinterpret_cast<uint4*>(cell(slot + wKdHi, CH, c, r)) = make_uint4(dh[0], dh[1], dh[2], dh[3]);
+                *reinterpret_cast<uint4*>(cell(slot + wKdLo, CH, c, r)) = make_uint4(dl[0], dl[1], dl[2], dl[3]);
+                *reinterpret_cast<uint4*>(gs + gKc + kc_piece(J, r, c)) = make_uint4(kcd[0], kcd[1], kcd[2], kcd[3]);
+                for (int I = J + 1; I < 4; ++I) {  // the later row blocks see this row through exp(Gm_I - Gm_J) <= 1
+                    const float* f = tabs + (tF + I * (I - 1) / 2 + J) * 128 + c * 8;
+                    const float4 fa = *reinterpret_cast<const float4*>(f), fb = *reinterpret_cast<const float4*>(f + 4);
+                    const float2 F[4] = {{fa.x, fa.y}, {fa.z, fa.w}, {fb.x, fb.y}, {fb.z, fb.w}};
+                    uint32_t kcf[4];
+#pragma unroll
+                    for (int u2 = 0; u2 < 4; ++u2) {
+                        const float2 x = mul2(kc[u2], F[u2]);
+                        kcf[u2] = tc::bf16x2(x.x, x.y);
+                    }
+                    *reinterpret_cast<uint4*>(gs + gKc + kc_piece(I, r, c)) = make_uint4(kcf[0], kcf[1], kcf[2], kcf[3]);
+                }
             }
-            *reinterpret_cast<uint4*>(gs + gK + box_piece(r, c)) = make_uint4(kg[0], kg[1], kg[2], kg[3]);
-            *reinterpret_cast<uint4*>(gs + gKb + box_piece(r, c)) = make_uint4(kgb[0], kgb[1], kgb[2], kgb[3]);
-            *reinterpret_cast<uint4*>(cell(slot + wKdHi, CH, c, r)) = make_uint4(dh[0], dh[1], dh[2], dh[3]);
-            *reinterpret_cast<uint4*>(cell(slot + wKdLo, CH, c, r)) = make_uint4(dl[0], dl[1], dl[2], dl[3]);
-            *reinterpret_cast<uint4*>(gs + gKc + kc_piece(J, r, c)) = make_uint4(kcd[0], kcd[1], kcd[2], kcd[3]);
-            for (int I = J + 1; I < 4; ++I) {  // the later row blocks see this row through exp(Gm_I - Gm_J) <= 1
-                const float* f = tabs + (tF + I * (I - 1) / 2 + J) * 128 + c * 8;
-                const float4 fa = *reinterpret_cast<const float4*>(f), fb = *reinterpret_cast<const float4*>(f + 4);
-                *reinterpret_cast<uint4*>(gs + gKc + kc_piece(I, r, c)) =
-                    make_uint4(tc::bf16x2(kc[0] * fa.x, kc[1] * fa.y), tc::bf16x2(kc[2] * fa.z, kc[3] * fa.w),
-                               tc::bf16x2(kc[4] * fb.x, kc[5] * fb.y), tc::bf16x2(kc[6] * fb.z, kc[7] * fb.w));
-            }
-        }
         }
         publish();
         // ---- 3a. L^T, one block column of 16 rows i a warp: [64 j x 16 i] = column side (tile I) x row side (block I)^T.  The
@@ -383,12 +395,14 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
             if (narrow) {  // one product, all 64 rows i at once, row side Kg (a commit with nothing pending arrives at once)
                 constexpr uint32_t id64 = tc::idesc_bf16(64, 64, 0, 0, 0);
                 if (gw == 0)
+#pragma unroll kIssue
                     for (int k0 = 0; k0 < DK; k0 += 16)
-                        tc::mma_bf16_if(leader, tm + gcL, tc::desc_sw128_kmajor(gs + gKc + kc_tile(3), CH, k0), tc::desc_sw128_kmajor(gs + gK, CH, k0), id64, k0 > 0);
+                        tc::mma_bf16_if(leader, tm + gcL, tc::desc_sw128_kmajor(gs + gKb, CH, k0), tc::desc_sw128_kmajor(gs + gK, CH, k0), id64, k0 > 0);
             } else {
             constexpr uint32_t id = tc::idesc_bf16(64, 16, 0, 0, 0);
             const int I = gw;
             const unsigned char* kct = gs + gKc + kc_tile(I);
+#pragma unroll kIssue
             for (int k0 = 0; k0 < DK; k0 += 16)
                 tc::mma_bf16_if(leader, tm + gcL + 16 * I, tc::desc_sw128_kmajor(kct, 16 * (I + 1), k0), tc::desc_sw128_kmajor(gs + gKb + I * 2048, CH, k0), id, k0 > 0);
             }
@@ -396,48 +410,41 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
             if (leader) atomicAdd(const_cast<uint32_t*>(ctx.progress), 1u);
             __syncwarp();
         }
-        // ---- 3b. the tiles made from q, while L^T runs: row side Qgb = Q a (over Q); Qg = Q exp(G) out to the workspace -------
+        // ---- 3b. the block-wise form's tiles made from q, while L^T runs: row side Qgb = Q a (over Q); Qg = Q exp(G) out to the workspace
+        if (!narrow) {
 #pragma unroll
-        for (int cc = 0; cc < 4; ++cc) {
-            const int c = cq * 4 + cc;
-            const uint4 q8 = *reinterpret_cast<const uint4*>(gs + gQ + box_piece(r, c));
-            const uint32_t qw[4] = {q8.x, q8.y, q8.z, q8.w};
-            uint32_t qg[4], qgb[4];
-            if (narrow) {
-#pragma unroll
-                for (int u2 = 0; u2 < 4; ++u2) {
-                    const float2 x = mul2(widen2<LAYER>(qw[u2]), {a[cc * 8 + 2 * u2], a[cc * 8 + 2 * u2 + 1]});
-                    qg[u2] = qgb[u2] = tc::bf16x2(x.x, x.y);
-                }
-            } else {
+            for (int t = 0; t < 4; ++t) {
+                const int c = piece(t), J = block(t), r = row(t);
+                const uint4 q8 = *reinterpret_cast<const uint4*>(gs + gQ + box_piece(r, c));
+                const uint32_t qw[4] = {q8.x, q8.y, q8.z, q8.w};
+                uint32_t qg[4], qgb[4];
                 const float4 e0a = *reinterpret_cast<const float4*>(tabs + (tE0 + J) * 128 + c * 8), e0b = *reinterpret_cast<const float4*>(tabs + (tE0 + J) * 128 + c * 8 + 4);
-                const float E0[8] = {e0a.x, e0a.y, e0a.z, e0a.w, e0b.x, e0b.y, e0b.z, e0b.w};
+                const float2 E0[4] = {{e0a.x, e0a.y}, {e0a.z, e0a.w}, {e0b.x, e0b.y}, {e0b.z, e0b.w}};
 #pragma unroll
                 for (int u2 = 0; u2 < 4; ++u2) {
-                    const float2 q2 = widen2<LAYER>(qw[u2]);
-                    const float q0 = q2.x, q1 = q2.y;
-                    const float a0 = a[cc * 8 + 2 * u2], a1 = a[cc * 8 + 2 * u2 + 1];
-                    qgb[u2] = tc::bf16x2(q0 * a0, q1 * a1);
-                    qg[u2] = tc::bf16x2(q0 * (a0 * E0[2 * u2]), q1 * (a1 * E0[2 * u2 + 1]));
+                    const float2 qf = widen2<LAYER>(qw[u2]), av = {a[t * 8 + 2 * u2], a[t * 8 + 2 * u2 + 1]}, x = mul2(qf, av), y = mul2(qf, mul2(av, E0[u2]));
+                    qgb[u2] = tc::bf16x2(x.x, x.y);
+                    qg[u2] = tc::bf16x2(y.x, y.y);
                 }
+                *reinterpret_cast<uint4*>(gs + gQ + box_piece(r, c)) = make_uint4(qgb[0], qgb[1], qgb[2], qgb[3]);
+                *reinterpret_cast<uint4*>(cell(slot + wQg, CH, c, r)) = make_uint4(qg[0], qg[1], qg[2], qg[3]);
             }
-            // narrow: Qg itself is M's row side
-            *reinterpret_cast<uint4*>(gs + gQ + box_piece(r, c)) = make_uint4(qgb[0], qgb[1], qgb[2], qgb[3]);
-            *reinterpret_cast<uint4*>(cell(slot + wQg, CH, c, r)) = make_uint4(qg[0], qg[1], qg[2], qg[3]);
+            publish();
         }
-        publish();
         // ---- 3c. M^T the same way, by the other four warps ------------------------------------------------------------------------
         if (gw >= 4) {
             const uint32_t leader = tc::elect_one();
             if (narrow) {
                 constexpr uint32_t id64 = tc::idesc_bf16(64, 64, 0, 0, 0);
                 if (gw == 4)
+#pragma unroll kIssue
                     for (int k0 = 0; k0 < DK; k0 += 16)
-                        tc::mma_bf16_if(leader, tm + gcM, tc::desc_sw128_kmajor(gs + gKc + kc_tile(3), CH, k0), tc::desc_sw128_kmajor(gs + gQ, CH, k0), id64, k0 > 0);
+                        tc::mma_bf16_if(leader, tm + gcM, tc::desc_sw128_kmajor(gs + gKb, CH, k0), tc::desc_sw128_kmajor(gs + gQ, CH, k0), id64, k0 > 0);
             } else {
             constexpr uint32_t id = tc::idesc_bf16(64, 16, 0, 0, 0);
             const int I = gw - 4;
             const unsigned char* kct = gs + gKc + kc_tile(I);
+#pragma unroll kIssue
             for (int k0 = 0; k0 < DK; k0 += 16)
                 tc::mma_bf16_if(leader, tm + gcM + 16 * I, tc::desc_sw128_kmajor(kct, 16 * (I + 1), k0), tc::desc_sw128_kmajor(gs + gQ + I * 2048, CH, k0), id, k0 > 0);
             }
@@ -451,30 +458,33 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
         // ---- 4. from L^T and M^T (lane = column j, tensor-memory column = row i): L (FP32, strictly lower, times beta_i) into
         // the scratch; M (lower with the diagonal) out as bf16 cells of eight consecutive rows i, [8 cells][64 columns j] ----------
         {
-            const int j = lane_row64;
+            // In the fragment layout: columns j and j + 8, rows i = 16 x + 8 g + 2 (lane % 4) and the next.
+            const int j = quad * 16 + (lane >> 2), i0 = 2 * (lane & 3);
+            uint32_t f[4][8];
 #pragma unroll
-            for (int half = 0; half < 2; ++half) {
-                uint32_t rr[32];
-                tc::tmem_ld32(tc::tmem_addr(tm, quad, (cg == 0 ? gcL : gcM) + half * 32), rr);
-                tc::tmem_ld_wait();
-                if (lane < 16) {
-                    if (cg == 0) {  // L stays transposed: this thread's column j, 32 consecutive rows i
-                        float* Lt = reinterpret_cast<float*>(gs + gL) + j * LS + half * 32;
+            for (int x = 0; x < 4; ++x) tc::tmem_ld_frag(tc::tmem_addr(tm, quad, (cg == 0 ? gcL : gcM) + 16 * x), f[x]);
+            tc::tmem_ld_wait();
+            if (cg == 0) {  // L stays transposed
+                float* Lt = reinterpret_cast<float*>(gs + gL) + j * LS + i0;
 #pragma unroll
-                        for (int i4 = 0; i4 < 8; ++i4) {
-                            const float4 b4 = *reinterpret_cast<const float4*>(betas + half * 32 + i4 * 4);
-                            const int i = half * 32 + i4 * 4;
-                            *reinterpret_cast<float4*>(Lt + i4 * 4) = make_float4(i > j ? b4.x * __uint_as_float(rr[i4 * 4]) : 0.0f, i + 1 > j ? b4.y * __uint_as_float(rr[i4 * 4 + 1]) : 0.0f,
-                                                                                  i + 2 > j ? b4.z * __uint_as_float(rr[i4 * 4 + 2]) : 0.0f, i + 3 > j ? b4.w * __uint_as_float(rr[i4 * 4 + 3]) : 0.0f);
-                        }
-                    } else {
+                for (int x = 0; x < 8; ++x) {
+                    const float2 b2 = *reinterpret_cast<const float2*>(betas + x * 8 + i0);
 #pragma unroll
-                        for (int i2 = 0; i2 < 32; ++i2)
-                            if (half * 32 + i2 < j) rr[i2] = 0u;
-#pragma unroll
-                        for (int cc = 0; cc < 4; ++cc) *reinterpret_cast<uint4*>(cell(slot + wMm, CH, half * 4 + cc, j)) = pack8(rr + cc * 8);
+                    for (int h = 0; h < 2; ++h) {
+                        const int i = x * 8 + i0, jh = j + 8 * h;
+                        const float l0 = __uint_as_float(f[x >> 1][4 * (x & 1) + 2 * h]), l1 = __uint_as_float(f[x >> 1][4 * (x & 1) + 2 * h + 1]);
+                        *reinterpret_cast<float2*>(Lt + h * 8 * LS + x * 8) = make_float2(i > jh ? b2.x * l0 : 0.0f, i + 1 > jh ? b2.y * l1 : 0.0f);
                     }
                 }
+            } else {  // four lanes' pairs are a cell
+#pragma unroll
+                for (int x = 0; x < 8; ++x)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const int i = x * 8 + i0, jh = j + 8 * h;
+                        const float m0 = __uint_as_float(f[x >> 1][4 * (x & 1) + 2 * h]), m1 = __uint_as_float(f[x >> 1][4 * (x & 1) + 2 * h + 1]);
+                        *reinterpret_cast<uint32_t*>(cell(slot + wMm, CH, x, jh) + 2 * i0) = tc::bf16x2(i >= jh ? m0 : 0.0f, i + 1 >= jh ? m1 : 0.0f);
+                    }
             }
         }
         tc::fence_before_sync();
@@ -509,13 +519,13 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
             constexpr uint32_t id = tc::idesc_bf16(128, 64, 1, 0, 0);
             const unsigned char* tph = gs + gTp;
             const unsigned char* tpl = gs + gTp + kBox;
-#pragma unroll
+#pragma unroll kIssue
             for (int k0 = 0; k0 < CH; k0 += 16)
                 tc::mma_bf16_if(leader, tm + gcW, tc::desc_sw128_mnmajor(gs + gK, CH, k0), tc::desc_sw128_kmajor(tph, CH, k0), id, k0 > 0);
-#pragma unroll
+#pragma unroll kIssue
             for (int k0 = 0; k0 < CH; k0 += 16)
                 tc::mma_bf16_if(leader, tm + gcU, tc::desc_sw128_mnmajor(gs + gV, CH, k0), tc::desc_sw128_kmajor(tph, CH, k0), id, k0 > 0);
-#pragma unroll
+#pragma unroll kIssue
             for (int k0 = 0; k0 < CH; k0 += 16)
                 tc::mma_bf16_if(leader, tm + gcU, tc::desc_sw128_mnmajor(gs + gV, CH, k0), tc::desc_sw128_kmajor(tpl, CH, k0), id, true);
         });
@@ -538,7 +548,7 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
             for (int j2 = 0; j2 < 8; ++j2)
                 *reinterpret_cast<uint4*>(slot + wU + u_cell(cg * 8 + j2, ch)) = make_uint4(r[j2 * 4], r[j2 * 4 + 1], r[j2 * 4 + 2], r[j2 * 4 + 3]);
         }
-        if (p.fused) fence_proxy_async_global();  // another block's bulk copies read the slot
+        if (FUSED) fence_proxy_async_global();  // another block's bulk copies read the slot
         tc::fence_before_sync();
         group_sync();
         tc::fence_after_sync();
@@ -558,7 +568,7 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // 16-byte copies (rows past the sequence's end are not read, they become zero), so no copy ever reaches
 // past the rows the caller's metadata names.  They are asynchronous, all in flight at once: as loads and stores, a row's after
 // the other's, they were 8 to 12 us of a launch (33 rows x 64 heads by the chunked layer prefill: 59 us, 64 rows 52).
-template <bool LAYER>
+template <bool LAYER, bool FUSED>
 __device__ __forceinline__ void intra_loader(const SpParams& p, unsigned char* smem, const WaitCtx& ctx, const int G) {
     unsigned char* gs = smem + G * kGroupBytes;
     uint64_t* bar_raw = reinterpret_cast<uint64_t*>(gs + gBars);
@@ -571,19 +581,19 @@ __device__ __forceinline__ void intra_loader(const SpParams& p, unsigned char* s
     uint32_t free_phase = 0;
     for (int it = 0;;) {
         long long item = 0;
-        if (lane == 0) item = atomicAdd(p.fused ? p.sets + p.ctr * kTailSet : p.counters + p.ctr, 1u);
+        if (lane == 0) item = atomicAdd(FUSED ? p.sets + p.ctr * kTailSet : p.counters + p.ctr, 1u);
         item = __shfl_sync(0xffffffffu, item, 0);
         const bool last = item >= items;
         int h = 0, n = 0;
         long long gr0 = 0;
         const unsigned char* in = nullptr;
         if (!last) {
-            const Item at = item_of(p, (int)item);
+            const Item at = item_of<FUSED>(p, (int)item);
             const int j = p.intra_chunk0 + at.jj, b = at.chain / H;
             h = at.chain % H;
             const int r0 = p.cu[b], T = p.cu[b + 1] - r0;
             if ((long long)j * CH >= T) {  // the sequence has no such chunk
-                if (p.fused && lane == 0) atomicAdd(p.sets + p.ctr * kTailSet + 2 + at.group, 1u);
+                if (FUSED && lane == 0) atomicAdd(p.sets + p.ctr * kTailSet + 2 + at.group, 1u);
                 continue;
             }
             gr0 = (long long)r0 + (long long)j * CH;
@@ -660,7 +670,7 @@ __device__ __forceinline__ void intra_loader(const SpParams& p, unsigned char* s
     }
 }
 
-template <bool LAYER>
+template <bool LAYER, bool FUSED>
 __device__ void intra_role(const SpParams& p, unsigned char* smem, const uint32_t tm) {
     volatile uint32_t* ctl = reinterpret_cast<volatile uint32_t*>(smem + oCtl);
     const WaitCtx ctx{ctl, ctl + 1, p.status};
@@ -673,8 +683,8 @@ __device__ void intra_role(const SpParams& p, unsigned char* smem, const uint32_
         mbar_init_fence();
     }
     __syncthreads();
-    if (warp == kLoaderWarp || warp == kOutWarp) intra_loader<LAYER>(p, smem, ctx, warp == kLoaderWarp ? 0 : 1);
-    else if (warp != kMmaWarp) intra_group<LAYER>(p, smem, tm, ctx, warp < kGroupThreads / 32 ? 0 : 1);
+    if (warp == kLoaderWarp || warp == kOutWarp) intra_loader<LAYER, FUSED>(p, smem, ctx, warp == kLoaderWarp ? 0 : 1);
+    else if (warp != kMmaWarp) intra_group<LAYER, FUSED>(p, smem, tm, ctx, warp < kGroupThreads / 32 ? 0 : 1);
     tc::fence_before_sync();
     __syncthreads();
 }
@@ -864,7 +874,7 @@ __device__ __forceinline__ void state_to_tmem(uint32_t at, const uint16_t* from,
 // chunks: counter, metadata, barriers and first loads one after another, the state a line per 16 bytes, the last chunk's gate.  Whole
 // calls, us: chunked layer prefill of 4 x 2,048 rows 1,136 -> 1,043, of 3 x 700 342 -> 301; core prefill of 8,192 rows in 8 sequences 525 -> 504, with
 // the norm in 3 sequences 663 -> 582; 8 chains of 1,024 chunks (one walk each) 1,968 -> 1,845.
-template <bool MANY>
+template <bool MANY, bool GATED>
 __device__ void state_role(const SpParams& p, unsigned char* smem, const uint32_t tm, const int chain, const Walk wk) {
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + oBarsState);
     volatile uint32_t* ctl = reinterpret_cast<volatile uint32_t*>(smem + oCtl);
@@ -1002,7 +1012,7 @@ __device__ void state_role(const SpParams& p, unsigned char* smem, const uint32_
                     // U has one buffer, so its load is on the walk: from L2.
                     if (c + 1 < at.count) bulk_prefetch(slot + kSlotBytes + wU, kUBytes);
                     if (gate_due && !(ok = load_gate(C - 1))) break;
-                    gate_due = wk.emit && p.gate_boxes != 0;
+                    gate_due = GATED && wk.emit && p.gate_boxes != 0;
                     gate_row = at.rows - c * CH >= CH ? (int)(at.row + c * CH) : -1;
                     gate_h = at.h;
                 }
@@ -1148,7 +1158,7 @@ __device__ void state_role(const SpParams& p, unsigned char* smem, const uint32_
     };
     // The four warps that share output rows vote at a barrier in every chunk when the norm is fused, and before every chain of
     // several; one that gives up before it still takes part.
-    const bool votes = wk.emit && p.gate != nullptr;
+    const bool votes = GATED && wk.emit;
     auto leave = [&] {
         if (MANY || votes) named_bar_all(4 + cg, 128, false);
         alive = false;
@@ -1352,22 +1362,25 @@ __device__ void state_role(const SpParams& p, unsigned char* smem, const uint32_
 
 // Both roles of a pass in one launch: every block takes items until there are none, then chains.  A block waits for other blocks'
 // items only when every item has been handed out, that is to blocks that are running and wait for nobody.
-template <bool LAYER>
+template <bool LAYER, bool GATED>
 __device__ void fused_roles(const SpParams& p, unsigned char* smem, const uint32_t tm) {
     volatile uint32_t* ctl = reinterpret_cast<volatile uint32_t*>(smem + oCtl);
     const int tid = threadIdx.x;
-    intra_role<LAYER>(p, smem, tm);
+    intra_role<LAYER, true>(p, smem, tm);
     if (ctl[1] != 0u) return;
     if (tid < kGroupBars * kGroups) mbar_inval(reinterpret_cast<uint64_t*>(smem + tid / kGroupBars * kGroupBytes + gBars) + tid % kGroupBars);
     fence_proxy_async_smem();  // what the intra role left in shared memory is overwritten by bulk copies
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
-    state_role<true>(p, smem, tm, 0, Walk{p.state_chunk0, p.state_chunk0 + p.seg_chunks, 0, nullptr, 0, nullptr, true, true});
+    state_role<true, GATED>(p, smem, tm, 0, Walk{p.state_chunk0, p.state_chunk0 + p.seg_chunks, 0, nullptr, 0, nullptr, true, true});
 }
 
 // One launch: the state role of one segment on the chain blocks, then the intra role of the next segment on all blocks.
-template <bool LAYER>
+// (An instance for each set of roles and for the norm: both roles are bound by their own instructions, and what an instance does not run costs
+// it registers and room in the instruction caches.  Against one for all of the core form: 2 sequences of 10,000 rows x 32 heads 980 -> 865 us,
+// 8 chains of 1,024 chunks 1,880 -> 1,680; 4 x 2,048 rows of the layer form 1,011 -> 985.)
+template <bool LAYER, bool FUSED, bool GATED>
 __global__ void __launch_bounds__(kThreadsSp, 1) prefill_sp_kernel(const __grid_constant__ SpParams p) {
     extern __shared__ __align__(1024) unsigned char smem[];
     volatile uint32_t* ctl = reinterpret_cast<volatile uint32_t*>(smem + oCtl);
@@ -1388,10 +1401,10 @@ __global__ void __launch_bounds__(kThreadsSp, 1) prefill_sp_kernel(const __grid_
     grid_ready();
     // the next launch's counters; nobody reads them during this launch.  (A scan pass leaves the counters alone: it may run
     // beside the next super-block's intra launch on another stream.)
-    if (p.fused && blockIdx.x == 0 && tid < kTailSet) p.sets[(p.ctr ^ 1) * kTailSet + tid] = 0u;
-    if (!p.fused && blockIdx.x == 0 && tid == 0 && p.scan_pass == 0) p.counters[p.ctr ^ 1] = 0u;
-    if (p.fused) {
-        fused_roles<LAYER>(p, smem, tm);
+    if (FUSED && blockIdx.x == 0 && tid < kTailSet) p.sets[(p.ctr ^ 1) * kTailSet + tid] = 0u;
+    if (!FUSED && blockIdx.x == 0 && tid == 0 && p.scan_pass == 0) p.counters[p.ctr ^ 1] = 0u;
+    if constexpr (FUSED) {
+        fused_roles<LAYER, GATED>(p, smem, tm);
     } else if (p.has_state) {
         // Block (chain); (chain, segment s < scan_p1, kind) in scan pass 1: the segment's offset and transition; (chain, segment) in
         // scan pass 2: the walk with outputs from the segment's true incoming state, of which only the last delivers the sequence's
@@ -1417,11 +1430,11 @@ __global__ void __launch_bounds__(kThreadsSp, 1) prefill_sp_kernel(const __grid_
                     wk.fin = last ? 0 : 2;
                 }
             }
-            state_role<false>(p, smem, tm, chain, wk);
+            state_role<false, GATED>(p, smem, tm, chain, wk);
             tc::fence_after_sync();
         }
     }
-    if (!p.fused && p.has_intra && ctl[1] == 0u) intra_role<LAYER>(p, smem, tm);
+    if (!FUSED && p.has_intra && ctl[1] == 0u) intra_role<LAYER, false>(p, smem, tm);
     if (ctl[1] != 0u) {  // after an abort copies into this block's shared memory may still be in flight: give them a bounded time
         const uint64_t t0 = global_timer_ns();
         while (global_timer_ns() - t0 < 2000000ull) {
@@ -1516,11 +1529,10 @@ static int fused_launch(SpParams& p, unsigned char* slots, unsigned int* tail, i
     p.counters = tail;
     p.sets = tail + kTailSets;
     p.ctr = pass & 1;
-    p.fused = 1;
     p.group = (int)((chains + kTailGroups - 1) / kTailGroups);
     // (The prologue in front is a plain launch: begun early too, its blocks crowd onto the SMs that come free first, 1,243 against
     // 1,203 us for 4 requests x 2,048 rows.)
-    return launch_early(prefill_sp_kernel<LAYER>, (unsigned)(most < sms ? most : sms), kThreadsSp, kSmemSp, stream, p);
+    return launch_early(LAYER || p.gate != nullptr ? prefill_sp_kernel<LAYER, true, true> : prefill_sp_kernel<LAYER, true, LAYER>, (unsigned)(most < sms ? most : sms), kThreadsSp, kSmemSp, stream, p);
 }
 
 // The launches over every segment of the longest sequence, in stream order.  A workspace of two or more chunks per
@@ -1566,7 +1578,9 @@ int core_prefill_sp_launch(int32_t heads, int32_t batch, const int32_t* cu_seqle
     int dev = 0;
     cudaGetDevice(&dev);
     if (configured_dev != dev) {
-        const cudaError_t e = cudaFuncSetAttribute(prefill_sp_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemSp);
+        cudaError_t e = cudaSuccess;
+        for (auto kernel : {prefill_sp_kernel<false, false, false>, prefill_sp_kernel<false, false, true>, prefill_sp_kernel<false, true, false>, prefill_sp_kernel<false, true, true>})
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemSp);
         if (e != cudaSuccess) return (int)e;
         configured_dev = dev;
     }
@@ -1613,6 +1627,7 @@ int core_prefill_sp_launch(int32_t heads, int32_t batch, const int32_t* cu_seqle
     gate_tensor_map(p, rows_cap);
     for (int r = 0; r < p.ranks; ++r)
         if (!row_tensor_map(&p.tm_full[r], p.full[r], 2, p.heads_total, rows_cap)) return (int)cudaErrorNotSupported;
+    const auto kernel = gate != nullptr ? prefill_sp_kernel<false, false, true> : prefill_sp_kernel<false, false, false>;
     cudaError_t e = cudaMemsetAsync(p.counters, 0, kCounterBytes, stream);
     if (e != cudaSuccess) return (int)e;
     const long long sms = sm_count();
@@ -1684,10 +1699,10 @@ int core_prefill_sp_launch(int32_t heads, int32_t batch, const int32_t* cu_seqle
                     // which is ready about now, off the machine until they are done, and the links idle.  From the second
                     // super-block on they leave that pass its SMs (measured on 8 GPUs, 2^20 tokens: 28.6 -> 26.1 ms).
                     const long long items = chains * cnt, room = b == 0 ? sms : (sms - Kb * chains > sms / 2 ? sms - Kb * chains : sms / 2);
-                    prefill_sp_kernel<false><<<(unsigned)(items < room ? items : room), kThreadsSp, kSmemSp, side->a>>>(p);
+                    kernel<<<(unsigned)(items < room ? items : room), kThreadsSp, kSmemSp, side->a>>>(p);
                     if ((e = cudaGetLastError()) != cudaSuccess) return (int)e;
                     p.has_intra = 0; p.has_state = 1; p.scan_pass = 1;
-                    prefill_sp_kernel<false><<<(unsigned)(2 * Kb * chains), kThreadsSp, kSmemSp, side->a>>>(p);
+                    kernel<<<(unsigned)(2 * Kb * chains), kThreadsSp, kSmemSp, side->a>>>(p);
                     if ((e = cudaGetLastError()) != cudaSuccess) return (int)e;
                     scan_compose_kernel<<<(unsigned)(chains * (DV / kComposeCols)), 128, 0, side->a>>>(p);
                     if ((e = cudaGetLastError()) != cudaSuccess) return (int)e;
@@ -1695,7 +1710,7 @@ int core_prefill_sp_launch(int32_t heads, int32_t batch, const int32_t* cu_seqle
                     // the other: the walks with the outputs (and the stores to the peers), super-block after super-block
                     cudaStreamWaitEvent(side->b, side->ready[b], 0);
                     p.scan_pass = 2;
-                    prefill_sp_kernel<false><<<(unsigned)(Kb * chains), kThreadsSp, kSmemSp, side->b>>>(p);
+                    kernel<<<(unsigned)(Kb * chains), kThreadsSp, kSmemSp, side->b>>>(p);
                     if ((e = cudaGetLastError()) != cudaSuccess) return (int)e;
                     carry = p.scan_carry_out;
                 }
@@ -1721,15 +1736,15 @@ int core_prefill_sp_launch(int32_t heads, int32_t batch, const int32_t* cu_seqle
             p.scan_carry_in = nullptr; p.scan_carry_out = nullptr;
             p.has_intra = 1; p.has_state = 0; p.scan_pass = 0;
             const long long items = chains * need;
-            prefill_sp_kernel<false><<<(unsigned)(items < sms ? items : sms), kThreadsSp, kSmemSp, stream>>>(p);
+            kernel<<<(unsigned)(items < sms ? items : sms), kThreadsSp, kSmemSp, stream>>>(p);
             if ((e = cudaGetLastError()) != cudaSuccess) return (int)e;
             p.has_intra = 0; p.has_state = 1; p.scan_pass = 1;
-            prefill_sp_kernel<false><<<(unsigned)(2 * (K - 1) * chains), kThreadsSp, kSmemSp, stream>>>(p);
+            kernel<<<(unsigned)(2 * (K - 1) * chains), kThreadsSp, kSmemSp, stream>>>(p);
             if ((e = cudaGetLastError()) != cudaSuccess) return (int)e;
             scan_compose_kernel<<<(unsigned)(chains * (DV / kComposeCols)), 128, 0, stream>>>(p);
             if ((e = cudaGetLastError()) != cudaSuccess) return (int)e;
             p.scan_pass = 2;
-            prefill_sp_kernel<false><<<(unsigned)(K * chains), kThreadsSp, kSmemSp, stream>>>(p);
+            kernel<<<(unsigned)(K * chains), kThreadsSp, kSmemSp, stream>>>(p);
             return (int)cudaGetLastError();
         }
     }
@@ -1759,7 +1774,7 @@ int core_prefill_sp_launch(int32_t heads, int32_t batch, const int32_t* cu_seqle
             const long long items = chains * seg, want = items < sms ? items : sms;
             if (grid < want) grid = want;
         }
-        return launch_early(prefill_sp_kernel<false>, (unsigned)grid, kThreadsSp, kSmemSp, stream, p);
+        return launch_early(kernel, (unsigned)grid, kThreadsSp, kSmemSp, stream, p);
     };
     if (segs == 0) return launch(-1, 0);  // nothing but empty sequences: their states are copied
     if (overlap) {
@@ -1786,7 +1801,7 @@ int layer_pass_launch(int32_t heads, int32_t batch, const int32_t* cu_rows, int3
     int dev = 0;
     cudaGetDevice(&dev);
     if (configured_dev != dev) {
-        const cudaError_t e = cudaFuncSetAttribute(prefill_sp_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemSp);
+        const cudaError_t e = cudaFuncSetAttribute(prefill_sp_kernel<true, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemSp);
         if (e != cudaSuccess) return (int)e;
         configured_dev = dev;
     }
