@@ -221,6 +221,11 @@ __device__ __forceinline__ float ex2_ftz(float x) {
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
+__device__ __forceinline__ float max_nan(float a, float b) {  // NaN where either is
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
 constexpr float kLog2e = 1.4426950408889634f;
 
 // The attribute of a launch that may begin while its predecessor in the stream drains, and how many attributes that are: none with

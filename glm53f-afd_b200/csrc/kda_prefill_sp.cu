@@ -257,7 +257,7 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
             float amax = 0.0f;
 #pragma unroll
             for (int r = 0; r < 32; ++r) {
-                const float av = ex2_ftz(fmaxf(run[r] - run[(r & 16) | 8], -126.0f));  // never 0: its reciprocal is taken
+                const float av = ex2_ftz(max_nan(run[r] - run[(r & 16) | 8], -126.0f));  // never 0: its reciprocal is taken
                 amax = fmaxf(amax, av);
                 *reinterpret_cast<float*>(col + r * 128 + ((pc ^ (r & 7)) << 4)) = av;
             }
@@ -267,16 +267,17 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
             const float base1 = tmp[d];
             const float gm0 = tmp[2 * 128 + d], gm1 = tmp[3 * 128 + d], gm2 = base1 + tmp[4 * 128 + d], gm3 = base1 + tmp[5 * 128 + d];
             const float gl = base1 + tmp[128 + d];
+            // (Denormals are wanted here: sixteen rows at the gate's bound decay by e^-93, and their factor meets others of e^+40 and e^+46.)
             float* tab = reinterpret_cast<float*>(gs + gTab) + d;
             if (part == 0) {
-                tab[(tE0 + 0) * 128] = ex2_ftz(gm0); tab[(tE0 + 1) * 128] = ex2_ftz(gm1); tab[(tE0 + 2) * 128] = ex2_ftz(gm2); tab[(tE0 + 3) * 128] = ex2_ftz(gm3);
-                tab[(tEL + 0) * 128] = ex2_ftz(gl - gm0); tab[(tEL + 1) * 128] = ex2_ftz(gl - gm1);
-                tab[(tEL + 2) * 128] = ex2_ftz(gl - gm2); tab[(tEL + 3) * 128] = ex2_ftz(gl - gm3);
+                tab[(tE0 + 0) * 128] = ex2_approx(gm0); tab[(tE0 + 1) * 128] = ex2_approx(gm1); tab[(tE0 + 2) * 128] = ex2_approx(gm2); tab[(tE0 + 3) * 128] = ex2_approx(gm3);
+                tab[(tEL + 0) * 128] = ex2_approx(gl - gm0); tab[(tEL + 1) * 128] = ex2_approx(gl - gm1);
+                tab[(tEL + 2) * 128] = ex2_approx(gl - gm2); tab[(tEL + 3) * 128] = ex2_approx(gl - gm3);
             } else {
-                tab[(tF + 0) * 128] = ex2_ftz(gm1 - gm0);
-                tab[(tF + 1) * 128] = ex2_ftz(gm2 - gm0); tab[(tF + 2) * 128] = ex2_ftz(gm2 - gm1);
-                tab[(tF + 3) * 128] = ex2_ftz(gm3 - gm0); tab[(tF + 4) * 128] = ex2_ftz(gm3 - gm1); tab[(tF + 5) * 128] = ex2_ftz(gm3 - gm2);
-                const float egl = ex2_ftz(gl);
+                tab[(tF + 0) * 128] = ex2_approx(gm1 - gm0);
+                tab[(tF + 1) * 128] = ex2_approx(gm2 - gm0); tab[(tF + 2) * 128] = ex2_approx(gm2 - gm1);
+                tab[(tF + 3) * 128] = ex2_approx(gm3 - gm0); tab[(tF + 4) * 128] = ex2_approx(gm3 - gm1); tab[(tF + 5) * 128] = ex2_approx(gm3 - gm2);
+                const float egl = ex2_approx(gl);
                 reinterpret_cast<float*>(slot + wEgl)[d] = egl;
                 reinterpret_cast<float*>(gs + gGl)[d] = egl;
             }
