@@ -7,10 +7,10 @@
 // the model's gate bound of -5.8 per row) and S the window's incoming state [v][k]:
 //
 //   L = beta_i (k_i a_i).(k_j / a_j) for j < i,  M = (q_i a_i).(k_j / a_j) for j <= i,   a = exp(G - Gm)
-//                         as L^T, M^T = Kc x Kgb^T, Kc x Qgb^T (tcgen05, M = 128 of which 16 rows are real, N = 16)
+//                         as L^T | M^T = Kc x [Kgb | Qgb]^T (tcgen05, M = 64 of which 16 rows are real, N = 32)
 //   W = (I + L)^-1 diag(beta) Kg,  U = (I + L)^-1 diag(beta) V   forward substitution down the 16 rows, FP32 on the CUDA
 //                         cores (thread = channel: 136 multiply-adds each; no explicit inverse), Kg = k exp(G)
-//   (W S)^T, (Qg S)^T     = S x W^T, S x Qg^T: tcgen05, M = 128 value channels, N = 16 rows, K = 128 key channels; the
+//   (W S)^T | (Qg S)^T    = S x [W | Qg]^T: tcgen05, M = 128 value channels, N = 2 x 16 rows, K = 128 key channels; the
 //                         bf16 state tile is the A operand exactly as it lies in HBM (rows of 128 key channels)
 //   D = U - W S,  O = Qg S + M D   FP32, thread = value channel (its tensor-memory lane)
 //
@@ -27,6 +27,12 @@
 // One block of 128 threads per (request, head) unit, three blocks per SM, blocks walk the units persistently.  A unit's
 // rows and state arrive by asynchronous 16-byte copies issued one unit ahead (the state straight into the 128-byte
 // swizzle the tensor core reads), so one unit's arithmetic covers the next one's loads.  All waits are bounded.
+//
+// A unit's serial stages bound it, at twelve warps an SM.  What they took and take, cycles of a unit of the core form (48 requests of 8 to
+// 16 rows): operand tiles 4,400 with two exponentials and a division an element and the saves between them, 1,800 as products of
+// multipliers; the saves 1,300, beside the first products; the next rows' copies 1,800 with a load of beta to wait for, 570 without;
+// products 870 + 880 as eight of N = 32 each instead of sixteen of N = 16; outputs 3,000 as two-byte stores, now sixteen bytes a unit
+// later.  Verify and commit of 34 layers together: 3,806 -> 3,183 us, 20 requests of 4 to 8 rows 1,625 -> 1,371.
 
 #include <cuda_fp16.h>
 
@@ -41,11 +47,11 @@ namespace {
 constexpr int WIN = 16, kVThreads = 128;
 // Shared memory map (bytes).  Tiles are boxes of R rows x 128 bytes in the 128-byte swizzle (16-byte piece p of row r at
 // piece p ^ (r & 7)), two boxes per tile (channels 0-63, 64-127).  The column-side tile Kc comes first: as the M = 128
-// operand of L^T and M^T its descriptor walks 128 rows although 16 are real, and what follows it is the state tile.
+// operand of L^T and M^T (M = 64) its descriptor walks 64 rows although 16 are real, and what follows it is the state tile.
 // Once those two products are done Kc is dead, and L and M (FP32, 3 KB) take its place until the unit ends.
-constexpr int vKc = 0, vS = 4096, vKgb = vS + 32768, vQgb = vKgb + 4096, vQg = vQgb + 4096, vRaw = vQg + 4096;
-constexpr int vW = vKgb;                                                 // W replaces Kgb once L^T is done
-constexpr int vStage = vKgb;                                             // layer form: FP32 outputs [16][128] over W and Qgb
+constexpr int vKc = 0, vS = 4096, vRow = vS + 32768, vRaw = vRow + 8192;
+constexpr int kRowR = 2 * WIN;   // the row side: one tile of 32 rows, Kgb | Qgb and, once L^T and M^T are formed, W | Qg
+constexpr int vStage = vRow;     // layer form: FP32 outputs [16][128] over W | Qg
 constexpr int vL = vKc, vM = vL + WIN * WIN * 8;  // L twice in a row (see substitute), M transposed
 static_assert(vM + WIN * WIN * 4 <= vS, "L and M fit the dead column-side tile");
 // Raw rows of a unit.  Core form: q, k, v bf16 (256 bytes a row), log decay f32 (512), beta.  Layer form: q fp16, v bf16,
@@ -56,7 +62,8 @@ struct Raw {
 };
 template <bool LAYER>
 struct Map {
-    static constexpr int vBeta = vRaw + Raw<LAYER>::kBytes, vBar = vBeta + 64, vCtl = vBar + 16, kSmem = vCtl + 16;
+    static constexpr int vOut = vRaw + Raw<LAYER>::kBytes;  // core form: a unit's outputs, bf16 [16][128], on their way out
+    static constexpr int vBeta = vOut + (LAYER ? 0 : WIN * DV * 2), vBar = vBeta + 64, vCtl = vBar + 16, kSmem = vCtl + 16;
     static_assert(vBar % 8 == 0 && kSmem <= 75 * 1024, "three blocks per SM");
 };
 constexpr uint32_t kVCols = 32;  // tensor memory: [0, 16) L^T then (W S)^T, [16, 32) M^T then (Qg S)^T
@@ -86,6 +93,13 @@ struct VParams {
 __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem_dst)), "l"(gmem_src) : "memory");
 }
+// Zeros where !read (nothing is read then).
+__device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src, bool read) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(smem_dst)), "l"(gmem_src), "r"(read ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async4(void* smem_dst, const void* gmem_src, bool read) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(smem_dst)), "l"(gmem_src), "r"(read ? 4 : 0) : "memory");
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() {
@@ -99,30 +113,55 @@ __device__ __forceinline__ int sw_elem(int R, int r, int c) {
 // and division do (the file's other divisions and exponentials keep IEEE arithmetic for the replay saves).
 __device__ __forceinline__ float sigmoid_(float x) { return __fdividef(1.0f, 1.0f + __expf(-x)); }
 
-// The operand tiles are made two channels and eight rows a thread (lanes 16-31 have rows 8-15): four-byte shared-memory accesses,
-// packed conversions.  What a lane of the other half holds:
+// The operand tiles are made two channels and eight rows a thread, outwards from the chunk's middle: lanes 0-15 have rows 7, 6, .. 0, lanes
+// 16-31 rows 8, 9, .. 15.  Four-byte shared-memory accesses, packed conversions.  What a lane of the other half holds:
 __device__ __forceinline__ float2 other_half(float2 x) {
     return make_float2(__shfl_xor_sync(0xffffffffu, x.x, 16), __shfl_xor_sync(0xffffffffu, x.y, 16));
 }
 __device__ __forceinline__ float2 widen_bf16x2(uint32_t w) { return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)); }
-__device__ __forceinline__ float2 exp2f_(float2 x) { return make_float2(__expf(x.x), __expf(x.y)); }
-// The cumulative sums g of a thread's eight rows to those of the chunk; returns row 8's (Gm) and row 15's (G_last).
-__device__ __forceinline__ void join_halves(float2 (&G)[WIN / 2], bool upper, float2& gm, float2& gl) {
-    const float2 o = other_half(G[WIN / 2 - 1]);
-    if (upper)
+__device__ __forceinline__ int row_of(int s, bool upper) { return upper ? WIN / 2 + s : WIN / 2 - 1 - s; }
+
+// The decay factors of a thread's rows from their multipliers m[s] (the exponentials of the log decays): products of at most sixteen of
+// them, no logarithms and no exponentials of sums.  Relative to the middle row (8), a row's factor is the product of the multipliers
+// between, on the lower half its reciprocal.
+struct Factors {
+    float2 between[WIN / 2], out[WIN / 2];  // products of the rows from the middle up to a row, without the further end; from a row outwards
+    float2 to_middle, beyond, all;
+    bool upper;
+    __device__ __forceinline__ Factors(const float2 (&m)[WIN / 2], bool up) : upper(up) {
+        between[0] = {1.0f, 1.0f};
+        out[WIN / 2 - 1] = m[WIN / 2 - 1];
 #pragma unroll
-        for (int r = 0; r < WIN / 2; ++r) G[r] = make_float2(G[r].x + o.x, G[r].y + o.y);
-    const float2 m = other_half(G[0]), l = other_half(G[WIN / 2 - 1]);
-    gm = upper ? G[0] : m;
-    gl = upper ? G[WIN / 2 - 1] : l;
-}
+        for (int s = 1; s < WIN / 2; ++s) between[s] = mul2(between[s - 1], {up ? m[s].x : m[s - 1].x, up ? m[s].y : m[s - 1].y});
+#pragma unroll
+        for (int s = WIN / 2 - 2; s >= 0; --s) out[s] = mul2(out[s + 1], m[s]);
+        const float2 m8 = other_half(m[0]), rest = other_half(out[0]), x = mul2(rest, m[0]);
+        to_middle = {up ? 1.0f : m8.x, up ? 1.0f : m8.y};
+        beyond = {up ? x.x : rest.x, up ? x.y : rest.y};
+        all = mul2(rest, out[0]);
+    }
+    // a = exp(G - G_8) and its reciprocal.  The smaller of the two stops at 2^-126, so that the other is finite (NaN stays NaN).
+    __device__ __forceinline__ void relative(int s, float2& a, float2& inva) const {
+        const float2 p = mul2(to_middle, between[s]), r = {rcp_approx(max_nan(p.x, 0x1p-126f)), rcp_approx(max_nan(p.y, 0x1p-126f))};
+        a = {upper ? p.x : r.x, upper ? p.y : r.y};
+        inva = {upper ? r.x : p.x, upper ? r.y : p.y};
+    }
+    __device__ __forceinline__ float2 from_start(int s) const {  // exp(G)
+        const float2 x = mul2(beyond, between[s]);
+        return {upper ? x.x : out[s].x, upper ? x.y : out[s].y};
+    }
+    __device__ __forceinline__ float2 to_end(int s) const {  // exp(G_last - G)
+        const float2 x = mul2(beyond, between[s]), o = s + 1 < WIN / 2 ? out[s + 1] : float2{1.0f, 1.0f};
+        return {upper ? o.x : x.x, upper ? o.y : x.y};
+    }
+};
 // All 16 rows of one channel (c0 + upper) from the two halves' pairs of channels.
 __device__ __forceinline__ void all_rows(const float2 (&x)[WIN / 2], bool upper, float (&y)[WIN]) {
 #pragma unroll
-    for (int r = 0; r < WIN / 2; ++r) {
-        const float got = __shfl_xor_sync(0xffffffffu, upper ? x[r].x : x[r].y, 16);
-        y[r] = upper ? got : x[r].x;
-        y[WIN / 2 + r] = upper ? x[r].y : got;
+    for (int s = 0; s < WIN / 2; ++s) {
+        const float got = __shfl_xor_sync(0xffffffffu, upper ? x[s].x : x[s].y, 16);
+        y[WIN / 2 - 1 - s] = upper ? got : x[s].x;
+        y[WIN / 2 + s] = upper ? x[s].y : got;
     }
 }
 
@@ -200,7 +239,6 @@ __device__ __forceinline__ void fetch_rows(const VParams& p, unsigned char* smem
     using R = Raw<LAYER>;
     const int n = min(max(un.n, 0), WIN);
     unsigned char* raw = smem + vRaw;
-    const uint4 z = make_uint4(0, 0, 0, 0);
     const long long rs = (long long)p.H * DK, unit = (un.row0 * p.H + un.h) * DK;
     {  // 16-byte pieces of the 256-byte rows, eight rows a step
         const int r0 = t >> 4, pc = t & 15;
@@ -211,15 +249,10 @@ __device__ __forceinline__ void fetch_rows(const VParams& p, unsigned char* smem
 #pragma unroll
         for (int i = 0; i < WIN / 8; ++i) {
             unsigned char* to = raw + (t + i * kVThreads) * 16;
-            if (r0 + 8 * i < n) {
-                cp_async16(to + R::Q, qs + i * 8 * (LAYER ? p.out_stride : rs));
-                if constexpr (!LAYER) cp_async16(to + R::K, ks + i * 8 * rs);
-                cp_async16(to + R::V, vs + i * 8 * rs);
-            } else {
-                *reinterpret_cast<uint4*>(to + R::Q) = z;
-                if constexpr (!LAYER) *reinterpret_cast<uint4*>(to + R::K) = z;
-                *reinterpret_cast<uint4*>(to + R::V) = z;
-            }
+            const bool in = r0 + 8 * i < n;
+            cp_async16(to + R::Q, in ? qs + i * 8 * (LAYER ? p.out_stride : rs) : qs, in);
+            if constexpr (!LAYER) cp_async16(to + R::K, in ? ks + i * 8 * rs : ks, in);
+            cp_async16(to + R::V, in ? vs + i * 8 * rs : vs, in);
         }
     }
     {  // and of the 512-byte rows, four a step
@@ -229,18 +262,14 @@ __device__ __forceinline__ void fetch_rows(const VParams& p, unsigned char* smem
 #pragma unroll
         for (int i = 0; i < WIN / 4; ++i) {
             unsigned char* to = raw + (t + i * kVThreads) * 16;
-            if (r0 + 4 * i < n) {
-                cp_async16(to + R::G, gs + i * 4 * rs);
-                if constexpr (LAYER) cp_async16(to + R::K, ks + i * 4 * rs);
-            } else {
-                *reinterpret_cast<uint4*>(to + R::G) = z;
-                if constexpr (LAYER) *reinterpret_cast<uint4*>(to + R::K) = z;
-            }
+            const bool in = r0 + 4 * i < n;
+            cp_async16(to + R::G, in ? gs + i * 4 * rs : gs, in);
+            if constexpr (LAYER) cp_async16(to + R::K, in ? ks + i * 4 * rs : ks, in);
         }
     }
     if (t < WIN) {
         const float* src = LAYER ? p.b_save : p.beta;
-        reinterpret_cast<float*>(raw + R::B)[t] = t < n ? src[(un.row0 + t) * p.H + un.h] : 0.0f;
+        cp_async4(raw + R::B + t * 4, t < n ? src + (un.row0 + t) * p.H + un.h : src, t < n);
     }
     cp_async_commit();
 }
@@ -256,6 +285,40 @@ __device__ __forceinline__ void fetch_state(const VParams& p, unsigned char* sme
         for (int e = t; e < DV * DK; e += kVThreads) *reinterpret_cast<uint16_t*>(smem + vS + sw_elem(DV, e >> 7, e & 127)) = src[e];
     }
     cp_async_commit();
+}
+
+// The core form's replay saves of a unit's n rows, the exact path's bits: k widened, v, exp(g), which stage A has left in place of g, beta.
+__device__ __forceinline__ void save_rows(const VParams& p, const unsigned char* smem, const Unit& un, int n, int t, bool vec) {
+    using R = Raw<false>;
+    if (p.k_save == nullptr) return;
+    const unsigned char* raw = smem + vRaw;
+    const long long rs = (long long)p.H * DK, unit = (un.row0 * p.H + un.h) * DK;
+    if (t < n) p.b_save[(un.row0 + t) * p.H + un.h] = reinterpret_cast<const float*>(raw + R::B)[t];
+    if (vec) {
+#pragma unroll
+        for (int i = 0; i < WIN / 4; ++i) {  // four channels a thread, four rows a step
+            const int r = (t >> 5) + 4 * i, c = (t & 31) * 4;
+            if (r < n) {
+                const uint2 kw = *reinterpret_cast<const uint2*>(raw + R::K + (r * DK + c) * 2);
+                const float2 k0 = widen_bf16x2(kw.x), k1 = widen_bf16x2(kw.y);
+                const float4 g4 = *reinterpret_cast<const float4*>(raw + R::G + (r * DK + c) * 4);
+                *reinterpret_cast<float4*>(p.k_save + unit + r * rs + c) = make_float4(k0.x, k0.y, k1.x, k1.y);
+                *reinterpret_cast<float4*>(p.g_save + unit + r * rs + c) = g4;
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < WIN / 8; ++i) {
+            const int r = (t >> 4) + 8 * i, c = (t & 15) * 8;
+            if (r < n) *reinterpret_cast<uint4*>(p.v_save + unit + r * rs + c) = *reinterpret_cast<const uint4*>(raw + R::V + (r * DK + c) * 2);
+        }
+    } else {
+        for (int r = 0; r < n; ++r) {
+            const long long at = unit + r * rs + t;
+            p.k_save[at] = bf16_bits_to_f32(reinterpret_cast<const uint16_t*>(raw + R::K)[r * DK + t]);
+            p.g_save[at] = reinterpret_cast<const float*>(raw + R::G)[r * DK + t];
+            p.v_save[at] = reinterpret_cast<const uint16_t*>(raw + R::V)[r * DK + t];
+        }
+    }
 }
 
 template <bool LAYER>
@@ -290,7 +353,18 @@ __global__ void __launch_bounds__(kVThreads, 3) verify_tc_kernel(const __grid_co
         for (int i = 0; i < 4; ++i) nw[i] = bf16_bits_to_f32(p.norm_w[lane * 4 + i]);
     }
 
-    const bool pair_saves = ((reinterpret_cast<uintptr_t>(p.k_save) | reinterpret_cast<uintptr_t>(p.g_save)) & 7) == 0 && (reinterpret_cast<uintptr_t>(p.v_save) & 3) == 0;
+    const bool vec_saves = ((reinterpret_cast<uintptr_t>(p.k_save) | reinterpret_cast<uintptr_t>(p.g_save) | reinterpret_cast<uintptr_t>(p.v_save)) & 15) == 0;
+    // The core form's outputs leave sixteen bytes a thread (two bytes a thread, sixteen stores each, held up whatever came after them),
+    // behind the next unit's first barrier.
+    long long out_at = 0;
+    int out_n = 0;
+    auto out_rows = [&] {
+#pragma unroll
+        for (int i = 0; i < WIN / 8; ++i) {
+            const int r = (t >> 4) + 8 * i, c = (t & 15) * 8;
+            if (r < out_n) *reinterpret_cast<uint4*>(p.out + out_at + (long long)r * p.H * DV + c) = *reinterpret_cast<const uint4*>(smem + MP::vOut + (r * DV + c) * 2);
+        }
+    };
     Units units(p);
     Unit un, nxt;
     bool more = units.take(p, nxt);
@@ -306,30 +380,35 @@ __global__ void __launch_bounds__(kVThreads, 3) verify_tc_kernel(const __grid_co
 
         cp_async_wait<1>();  // this unit's rows have landed (its state may still be on the way)
         __syncthreads();     // and every thread is done with the previous unit's L, M and staged outputs
+        if constexpr (!LAYER) out_rows();
+        out_at = (un.row0 * p.H + un.h) * DV;
+        out_n = n;
 
-        // ---- A. the decay scan, the operand tiles, the replay saves: channels c0 and c0 + 1, rows rb .. rb + 7 ---------------
+        // ---- A. the decay factors and the operand tiles: channels c0 and c0 + 1, eight rows -------------------------------------
         float kg[WIN], vv[WIN];
         float2 qe[WIN / 2];
         const bool upper = lane >= 16;
-        const int c0 = warp * 32 + (lane & 15) * 2, rb = upper ? WIN / 2 : 0;
+        const int c0 = warp * 32 + (lane & 15) * 2;
         {
-            const unsigned char* raw = smem + vRaw;
-            float2 G[WIN / 2], acc = {0.0f, 0.0f}, gm, gl;
+            unsigned char* raw = smem + vRaw;
+            float2 m[WIN / 2], kgp[WIN / 2];
 #pragma unroll
-            for (int r = 0; r < WIN / 2; ++r) {
-                float2 x = *reinterpret_cast<const float2*>(raw + R::G + ((rb + r) * DK + c0) * 4);
-                // layer form: the saved multiplier exp(log decay) in (0, 1]; the rows past the window decay by nothing
-                if constexpr (LAYER) x = rb + r < n ? make_float2(__logf(x.x), __logf(x.y)) : make_float2(0.0f, 0.0f);
-                acc = make_float2(acc.x + x.x, acc.y + x.y);
-                G[r] = acc;
+            for (int s = 0; s < WIN / 2; ++s) {
+                float2* x = reinterpret_cast<float2*>(raw + R::G + (row_of(s, upper) * DK + c0) * 4);
+                m[s] = *x;
+                if constexpr (LAYER) {  // the saved multipliers; the rows past the window decay by nothing
+                    if (row_of(s, upper) >= n) m[s] = {1.0f, 1.0f};
+                } else {  // of the log decays, by the exact path's expf; save_rows() takes them from here
+                    m[s] = {expf(m[s].x), expf(m[s].y)};
+                    *x = m[s];
+                }
             }
-            join_halves(G, upper, gm, gl);
+            const Factors fac(m, upper);
             float amax = 0.0f;
-            float2 kgp[WIN / 2];
 #pragma unroll
-            for (int r = 0; r < WIN / 2; ++r) {
-                const int row = rb + r, at2 = (row * DK + c0) * 2;
-                float2 kf, qf;
+            for (int s = 0; s < WIN / 2; ++s) {
+                const int row = row_of(s, upper), at2 = (row * DK + c0) * 2;
+                float2 kf, qf, a, inva;
                 const uint32_t qw = *reinterpret_cast<const uint32_t*>(raw + R::Q + at2);
                 if constexpr (LAYER) {
                     kf = *reinterpret_cast<const float2*>(raw + R::K + at2 * 2);
@@ -338,34 +417,15 @@ __global__ void __launch_bounds__(kVThreads, 3) verify_tc_kernel(const __grid_co
                     kf = widen_bf16x2(*reinterpret_cast<const uint32_t*>(raw + R::K + at2));
                     qf = widen_bf16x2(qw);
                 }
-                const float2 a = exp2f_({G[r].x - gm.x, G[r].y - gm.y}), e = exp2f_(G[r]);
+                fac.relative(s, a, inva);
+                const float2 e = fac.from_start(s);
                 amax = fmaxf(amax, fmaxf(a.x, a.y));
-                kgp[r] = mul2(kf, e);
-                qe[r] = mul2(qf, e);  // the Qg tile is written while the first products run
-                const float2 kb = mul2(kf, a), qb = mul2(qf, a), kc = mul2(kf, {__fdividef(1.0f, a.x), __fdividef(1.0f, a.y)});
-                const int to = sw_elem(WIN, row, c0);
-                *reinterpret_cast<uint32_t*>(smem + vKgb + to) = tc::bf16x2(kb.x, kb.y);
-                *reinterpret_cast<uint32_t*>(smem + vQgb + to) = tc::bf16x2(qb.x, qb.y);
-                *reinterpret_cast<uint32_t*>(smem + vKc + to) = tc::bf16x2(kc.x, kc.y);
-                if constexpr (!LAYER) {
-                    if (row < n && p.k_save != nullptr) {
-                        const long long at = ((un.row0 + row) * p.H + un.h) * DK + c0;
-                        const float2 gx = *reinterpret_cast<const float2*>(raw + R::G + at2 * 2);
-                        const uint32_t vw = *reinterpret_cast<const uint32_t*>(raw + R::V + at2);
-                        if (pair_saves) {
-                            *reinterpret_cast<float2*>(p.k_save + at) = kf;
-                            *reinterpret_cast<uint32_t*>(p.v_save + at) = vw;
-                            *reinterpret_cast<float2*>(p.g_save + at) = make_float2(expf(gx.x), expf(gx.y));
-                        } else {
-                            p.k_save[at] = kf.x;
-                            p.k_save[at + 1] = kf.y;
-                            p.v_save[at] = (uint16_t)vw;
-                            p.v_save[at + 1] = (uint16_t)(vw >> 16);
-                            p.g_save[at] = expf(gx.x);
-                            p.g_save[at + 1] = expf(gx.y);
-                        }
-                    }
-                }
+                kgp[s] = mul2(kf, e);
+                qe[s] = mul2(qf, e);  // the Qg rows are written when Qgb's have been read
+                const float2 kb = mul2(kf, a), qb = mul2(qf, a), kc = mul2(kf, inva);
+                *reinterpret_cast<uint32_t*>(smem + vRow + sw_elem(kRowR, row, c0)) = tc::bf16x2(kb.x, kb.y);
+                *reinterpret_cast<uint32_t*>(smem + vRow + sw_elem(kRowR, WIN + row, c0)) = tc::bf16x2(qb.x, qb.y);
+                *reinterpret_cast<uint32_t*>(smem + vKc + sw_elem(WIN, row, c0)) = tc::bf16x2(kc.x, kc.y);
             }
             all_rows(kgp, upper, kg);
 #pragma unroll
@@ -374,54 +434,53 @@ __global__ void __launch_bounds__(kVThreads, 3) verify_tc_kernel(const __grid_co
             if (t < WIN) {
                 const float bt = reinterpret_cast<const float*>(raw + R::B)[t];
                 betas[t] = bt;
-                if constexpr (!LAYER) {
-                    if (t < n && p.b_save != nullptr) p.b_save[(un.row0 + t) * p.H + un.h] = bt;
-                }
             }
         }
         fence_proxy_async_smem();
         tc::fence_before_sync();
         __syncthreads();
         tc::fence_after_sync();
-        // The raw rows are consumed: the next unit's may come in.
-        if (more) fetch_rows<LAYER>(p, smem, nxt, t);
-        else cp_async_commit();
+        if constexpr (LAYER) {  // the raw rows are consumed: the next unit's may come in
+            if (more) fetch_rows<LAYER>(p, smem, nxt, t);
+            else cp_async_commit();
+        }
 
         // ---- B. L^T and M^T -------------------------------------------------------------------------------------------------
         if (warp == 0) {
             const uint32_t leader = tc::elect_one();
-            constexpr uint32_t id = tc::idesc_bf16(128, WIN, 0, 0, 0);
+            constexpr uint32_t id = tc::idesc_bf16(64, kRowR, 0, 0, 0);
+#pragma unroll
             for (int k0 = 0; k0 < DK; k0 += 16)
-                tc::mma_bf16_if(leader, tm, tc::desc_sw128_kmajor(smem + vKc, WIN, k0), tc::desc_sw128_kmajor(smem + vKgb, WIN, k0), id, k0 > 0);
-            for (int k0 = 0; k0 < DK; k0 += 16)
-                tc::mma_bf16_if(leader, tm + 16, tc::desc_sw128_kmajor(smem + vKc, WIN, k0), tc::desc_sw128_kmajor(smem + vQgb, WIN, k0), id, k0 > 0);
+                tc::mma_bf16_if(leader, tm, tc::desc_sw128_kmajor(smem + vKc, WIN, k0), tc::desc_sw128_kmajor(smem + vRow, kRowR, k0), id, k0 > 0);
             tc::mma_commit_if(leader, bar);
             if (leader) atomicAdd(const_cast<uint32_t*>(ctl), 1u);
             __syncwarp();
         }
-#pragma unroll
-        for (int r = 0; r < WIN / 2; ++r) *reinterpret_cast<uint32_t*>(smem + vQg + sw_elem(WIN, rb + r, c0)) = tc::bf16x2(qe[r].x, qe[r].y);
+        if constexpr (!LAYER) save_rows(p, smem, un, n, t, vec_saves);  // while the products run
         bool ok = mbar_wait(bar, phase, ctx, kStatusWaitPrefill);
         phase ^= 1u;
         if (!__syncthreads_and(ok)) break;
         tc::fence_after_sync();
-        if (warp == 0) {  // lanes 0..15 hold column j of L and of M; tensor-memory column = row i.  Kc is dead: L, M go over it.
-            uint32_t l16[16], m16[16];
-            tc::tmem_ld16(tc::tmem_addr(tm, 0, 0), l16);
-            tc::tmem_ld16(tc::tmem_addr(tm, 0, 16), m16);
+        if constexpr (!LAYER) {  // the raw rows are consumed
+            if (more) fetch_rows<LAYER>(p, smem, nxt, t);
+            else cp_async_commit();
+        }
+        if (warp == 0) {  // tensor-memory lane = column j, column = row i of L, then of M.  Kc is dead: L, M go over it.
+            uint32_t l16[8], m16[8];  // the fragment layout: columns j and j + 8, rows i = 8 g + 2 (lane % 4) and the next
+            tc::tmem_ld_frag(tm, l16);
+            tc::tmem_ld_frag(tm + 16, m16);
             tc::tmem_ld_wait();
-            if (lane < WIN) {
-                const int j = lane;
 #pragma unroll
-                for (int i = 0; i < WIN; ++i) {
-                    const float l = i > j ? -betas[i] * __uint_as_float(l16[i]) : 0.0f;
-                    Ln[i * LN + j] = make_float2(l, l);
-                    if (i < j) m16[i] = 0u;
-                }
-#pragma unroll
-                for (int i = 0; i < WIN; i += 4) *reinterpret_cast<uint4*>(Mf + j * WIN + i) = make_uint4(m16[i], m16[i + 1], m16[i + 2], m16[i + 3]);
+            for (int x = 0; x < 4; ++x) {
+                const int j = (lane >> 2) + 8 * (x & 1), i = 8 * (x >> 1) + 2 * (lane & 3);
+                const float l0 = i > j ? -betas[i] * __uint_as_float(l16[2 * x]) : 0.0f, l1 = i + 1 > j ? -betas[i + 1] * __uint_as_float(l16[2 * x + 1]) : 0.0f;
+                Ln[i * LN + j] = make_float2(l0, l0);
+                Ln[(i + 1) * LN + j] = make_float2(l1, l1);
+                *reinterpret_cast<uint2*>(Mf + j * WIN + i) = make_uint2(i < j ? 0u : m16[2 * x], i + 1 < j ? 0u : m16[2 * x + 1]);
             }
         }
+#pragma unroll
+        for (int s = 0; s < WIN / 2; ++s) *reinterpret_cast<uint32_t*>(smem + vRow + sw_elem(kRowR, WIN + row_of(s, upper), c0)) = tc::bf16x2(qe[s].x, qe[s].y);
         tc::fence_before_sync();
         __syncthreads();
         tc::fence_after_sync();
@@ -432,7 +491,7 @@ __global__ void __launch_bounds__(kVThreads, 3) verify_tc_kernel(const __grid_co
         float2 wu[WIN];
         substitute(Ln, betas, kg, vv, wu);
 #pragma unroll
-        for (int i = 0; i < WIN; ++i) *reinterpret_cast<uint16_t*>(smem + vW + sw_elem(WIN, i, c0 + upper)) = f32_to_bf16_bits(wu[i].x);
+        for (int i = 0; i < WIN; ++i) *reinterpret_cast<uint16_t*>(smem + vRow + sw_elem(kRowR, i, c0 + upper)) = f32_to_bf16_bits(wu[i].x);
         cp_async_wait<1>();  // this unit's state has landed (the next unit's rows may still be on the way)
         fence_proxy_async_smem();
         tc::fence_before_sync();
@@ -442,11 +501,10 @@ __global__ void __launch_bounds__(kVThreads, 3) verify_tc_kernel(const __grid_co
         // ---- D. (W S)^T and (Qg S)^T: the state tile as it lies in memory is the M operand ---------------------------------------
         if (warp == 0) {
             const uint32_t leader = tc::elect_one();
-            constexpr uint32_t id = tc::idesc_bf16(128, WIN, 0, 0, 0);
+            constexpr uint32_t id = tc::idesc_bf16(128, kRowR, 0, 0, 0);
+#pragma unroll
             for (int k0 = 0; k0 < DK; k0 += 16)
-                tc::mma_bf16_if(leader, tm, tc::desc_sw128_kmajor(smem + vS, DV, k0), tc::desc_sw128_kmajor(smem + vW, WIN, k0), id, k0 > 0);
-            for (int k0 = 0; k0 < DK; k0 += 16)
-                tc::mma_bf16_if(leader, tm + 16, tc::desc_sw128_kmajor(smem + vS, DV, k0), tc::desc_sw128_kmajor(smem + vQg, WIN, k0), id, k0 > 0);
+                tc::mma_bf16_if(leader, tm, tc::desc_sw128_kmajor(smem + vS, DV, k0), tc::desc_sw128_kmajor(smem + vRow, kRowR, k0), id, k0 > 0);
             tc::mma_commit_if(leader, bar);
             if (leader) atomicAdd(const_cast<uint32_t*>(ctl), 1u);
             __syncwarp();
@@ -481,8 +539,8 @@ __global__ void __launch_bounds__(kVThreads, 3) verify_tc_kernel(const __grid_co
 #pragma unroll
             for (int i = 0; i < WIN; ++i) {
                 const float x = i & 1 ? o[i / 2].y : o[i / 2].x;
-                if constexpr (LAYER) reinterpret_cast<float*>(smem + vStage)[i * DV + t] = x;  // W and Qgb are dead
-                else if (i < n) p.out[(un.row0 + i) * p.out_stride + (long long)un.h * DV + t] = f32_to_bf16_bits(x);
+                if constexpr (LAYER) reinterpret_cast<float*>(smem + vStage)[i * DV + t] = x;  // W and Qg are dead
+                else reinterpret_cast<uint16_t*>(smem + MP::vOut)[i * DV + t] = f32_to_bf16_bits(x);
             }
         }
         tc::fence_before_sync();  // the next unit's products overwrite these tensor-memory columns
@@ -519,6 +577,9 @@ __global__ void __launch_bounds__(kVThreads, 3) verify_tc_kernel(const __grid_co
     cp_async_wait<0>();
     tc::fence_before_sync();
     __syncthreads();
+    if constexpr (!LAYER) {
+        if (ctl[1] == 0u) out_rows();
+    }
     if (warp == 0) tc::tmem_dealloc(tm, kVCols);
 }
 
@@ -671,51 +732,49 @@ __global__ void __launch_bounds__(kVThreads, kCBlocks) commit_tc_kernel(const __
             if (c0 == 0) cp_async_wait<1>();  // its rows are there (the state may still be on the way)
             else cp_async_wait<0>();
             __syncthreads();
-            // ---- A. the decay scan and the operand tiles: channels ch0 and ch0 + 1, rows rb .. rb + 7; thread = value channel: v ------
+            // ---- A. the decay factors and the operand tiles: channels ch0 and ch0 + 1, eight rows; thread = value channel: v ---------
             float kg[WIN], vv[WIN];
             const bool upper = lane >= 16;
-            const int ch0 = warp * 32 + (lane & 15) * 2, rb = upper ? WIN / 2 : 0;
+            const int ch0 = warp * 32 + (lane & 15) * 2;
             {
-                float2 kf[WIN / 2], G[WIN / 2], acc = {0.0f, 0.0f}, gm, gl;
-#pragma unroll
-                for (int r = 0; r < WIN / 2; ++r) {
-                    kf[r] = make_float2(0.0f, 0.0f);
-                    if (rb + r < nr) {
-                        kf[r] = *reinterpret_cast<const float2*>(smem + cRawK + ((rb + r) * DK + ch0) * 4);
-                        const float2 x = *reinterpret_cast<const float2*>(smem + cRawG + ((rb + r) * DK + ch0) * 4);
-                        acc = make_float2(acc.x + __logf(x.x), acc.y + __logf(x.y));
-                    }
-                    G[r] = acc;
-                }
-                join_halves(G, upper, gm, gl);
+                float2 m[WIN / 2], kgp[WIN / 2];
                 float amax = 0.0f;
-                float2 kgp[WIN / 2];
+#pragma unroll
+                for (int s = 0; s < WIN / 2; ++s) {
+                    m[s] = {1.0f, 1.0f};
+                    if (row_of(s, upper) < nr) m[s] = *reinterpret_cast<const float2*>(smem + cRawG + (row_of(s, upper) * DK + ch0) * 4);
+                }
+                const Factors fac(m, upper);
                 uint32_t dh[2][WIN / 4], dl[2][WIN / 4];
 #pragma unroll
                 for (int r = 0; r < WIN / 2; r += 2) {
                     float2 kd[2];
 #pragma unroll
                     for (int x = 0; x < 2; ++x) {
-                        const float2 a = exp2f_({G[r + x].x - gm.x, G[r + x].y - gm.y});
+                        const int s = r + x, row = row_of(s, upper), to = sw_elem(WIN, row, ch0);
+                        const float2 kf = row < nr ? *reinterpret_cast<const float2*>(smem + cRawK + (row * DK + ch0) * 4) : float2{0.0f, 0.0f};
+                        float2 a, inva;
+                        fac.relative(s, a, inva);
                         amax = fmaxf(amax, fmaxf(a.x, a.y));
-                        kgp[r + x] = mul2(kf[r + x], exp2f_(G[r + x]));
-                        kd[x] = mul2(kf[r + x], exp2f_({gl.x - G[r + x].x, gl.y - G[r + x].y}));
-                        const float2 kb = mul2(kf[r + x], a), kc = mul2(kf[r + x], {__fdividef(1.0f, a.x), __fdividef(1.0f, a.y)});
-                        const int to = sw_elem(WIN, rb + r + x, ch0);
+                        kgp[s] = mul2(kf, fac.from_start(s));
+                        kd[x] = mul2(kf, fac.to_end(s));
+                        const float2 kb = mul2(kf, a), kc = mul2(kf, inva);
                         *reinterpret_cast<uint32_t*>(smem + cKgb + to) = tc::bf16x2(kb.x, kb.y);
                         *reinterpret_cast<uint32_t*>(smem + cKc + to) = tc::bf16x2(kc.x, kc.y);
                     }
-                    tc::split_bf16x2(kd[0].x, kd[1].x, dh[0][r / 2], dl[0][r / 2]);
-                    tc::split_bf16x2(kd[0].y, kd[1].y, dh[1][r / 2], dl[1][r / 2]);
+                    // in the order of the rows: the lower half counts down
+                    const float2 d0 = upper ? kd[0] : kd[1], d1 = upper ? kd[1] : kd[0];
+                    tc::split_bf16x2(d0.x, d1.x, dh[0][r / 2], dl[0][r / 2]);
+                    tc::split_bf16x2(d0.y, d1.y, dh[1][r / 2], dl[1][r / 2]);
                 }
                 // Kdec^T: row = key channel, 16 row indices along K = two 16-byte cells, of which this thread has one
 #pragma unroll
                 for (int x = 0; x < 2; ++x) {
                     unsigned char* to = smem + cKdT + ((upper ? DK : 0) + ch0 + x) * 16;
-                    *reinterpret_cast<uint4*>(to) = make_uint4(dh[x][0], dh[x][1], dh[x][2], dh[x][3]);
-                    *reinterpret_cast<uint4*>(to + 4096) = make_uint4(dl[x][0], dl[x][1], dl[x][2], dl[x][3]);
+                    *reinterpret_cast<uint4*>(to) = upper ? make_uint4(dh[x][0], dh[x][1], dh[x][2], dh[x][3]) : make_uint4(dh[x][3], dh[x][2], dh[x][1], dh[x][0]);
+                    *reinterpret_cast<uint4*>(to + 4096) = upper ? make_uint4(dl[x][0], dl[x][1], dl[x][2], dl[x][3]) : make_uint4(dl[x][3], dl[x][2], dl[x][1], dl[x][0]);
                 }
-                if (!upper) *reinterpret_cast<float2*>(&En[ch0]) = exp2f_(gl);
+                if (!upper) *reinterpret_cast<float2*>(&En[ch0]) = fac.all;
                 all_rows(kgp, upper, kg);
 #pragma unroll
                 for (int r = 0; r < WIN; ++r) vv[r] = r < nr ? bf16_bits_to_f32(reinterpret_cast<const uint16_t*>(smem + cRawV)[r * DV + t]) : 0.0f;
@@ -734,7 +793,8 @@ __global__ void __launch_bounds__(kVThreads, kCBlocks) commit_tc_kernel(const __
             // ---- B. L^T ---------------------------------------------------------------------------------------------------
             if (warp == 0) {
                 const uint32_t leader = tc::elect_one();
-                constexpr uint32_t id = tc::idesc_bf16(128, WIN, 0, 0, 0);
+                constexpr uint32_t id = tc::idesc_bf16(64, WIN, 0, 0, 0);
+#pragma unroll
                 for (int k0 = 0; k0 < DK; k0 += 16)
                     tc::mma_bf16_if(leader, tm, tc::desc_sw128_kmajor(smem + cKc, WIN, k0), tc::desc_sw128_kmajor(smem + cKgb, WIN, k0), id, k0 > 0);
                 tc::mma_commit_if(leader, bar);
@@ -747,15 +807,15 @@ __global__ void __launch_bounds__(kVThreads, kCBlocks) commit_tc_kernel(const __
             if (!ok) break;
             tc::fence_after_sync();
             if (warp == 0) {
-                uint32_t l16[16];
-                tc::tmem_ld16(tc::tmem_addr(tm, 0, 0), l16);
+                uint32_t l16[8];  // the fragment layout, as in the verify
+                tc::tmem_ld_frag(tm, l16);
                 tc::tmem_ld_wait();
-                if (lane < WIN) {
 #pragma unroll
-                    for (int i = 0; i < WIN; ++i) {
-                        const float l = i > lane ? -betas[i] * __uint_as_float(l16[i]) : 0.0f;
-                        Ln[i * LN + lane] = make_float2(l, l);
-                    }
+                for (int x = 0; x < 4; ++x) {
+                    const int j = (lane >> 2) + 8 * (x & 1), i = 8 * (x >> 1) + 2 * (lane & 3);
+                    const float l0 = i > j ? -betas[i] * __uint_as_float(l16[2 * x]) : 0.0f, l1 = i + 1 > j ? -betas[i + 1] * __uint_as_float(l16[2 * x + 1]) : 0.0f;
+                    Ln[i * LN + j] = make_float2(l0, l0);
+                    Ln[(i + 1) * LN + j] = make_float2(l1, l1);
                 }
             }
             tc::fence_before_sync();
@@ -827,11 +887,13 @@ __global__ void __launch_bounds__(kVThreads, kCBlocks) commit_tc_kernel(const __
             tc::fence_after_sync();
 
             // ---- G. S <- E S + update, rounded to bf16, back into the tile (thread = value row) ------------------------------
-#pragma unroll 1
+            uint32_t acc[2][32];  // a quarter of the row, and the next on its way
+            tc::tmem_ld32(tc::tmem_addr(tm, warp, 0), acc[0]);
+#pragma unroll
             for (int cg = 0; cg < DK / 32; ++cg) {
-                uint32_t a16[32];
-                tc::tmem_ld32(tc::tmem_addr(tm, warp, cg * 32), a16);
                 tc::tmem_ld_wait();
+                if (cg + 1 < DK / 32) tc::tmem_ld32(tc::tmem_addr(tm, warp, (cg + 1) * 32), acc[(cg + 1) & 1]);
+                const uint32_t* a16 = acc[cg & 1];
 #pragma unroll
                 for (int half = 0; half < 4; ++half) {
                     unsigned char* at = smem + state_piece(t, cg * 4 + half);
