@@ -221,7 +221,7 @@ __device__ __forceinline__ float2 lo_hi(uint32_t w) { return make_float2(__uint_
 __device__ __forceinline__ float2 add2(float2 a, float2 b) { return fma2(a, {1.0f, 1.0f}, b); }
 // 1 / (1 + e^-x)
 __device__ __forceinline__ float2 sigmoid2(float2 x) {
-    const float2 t = mul2(x, {-kLog2e, -kLog2e}), d = add2({ex2_approx(t.x), ex2_approx(t.y)}, {1.0f, 1.0f});
+    const float2 t = mul2(x, {-kLog2e, -kLog2e}), d = add2({ex2_ftz(t.x), ex2_ftz(t.y)}, {1.0f, 1.0f});
     return make_float2(rcp_approx(d.x), rcp_approx(d.y));
 }
 __device__ __forceinline__ uint32_t fp16x2(float2 x) {
