@@ -1400,14 +1400,18 @@ int core_entry(int32_t heads, int32_t batch, const int32_t* cu_rows, const glm53
     // The exact verify (saves requested, inputs used as given, no fused output norm) runs on the small-block kernel: two
     // units' serial rows at once wait less on their own latencies than the persistent kernel's one (48 slots x 16 rows x 34 layers, bf16,
     // 9.6 against 11.9 ms; 6 slots x 8 rows 841 against 990 us, f32 757 and 901; a single slot's windows are the exception, four rows
-    // 335 against 254).  Single-row decode stays on the persistent kernel, which keeps more bytes in flight (bf16, 16 slots 458
-    // against 635 us, 48 slots 1,208 and 1,704; f32 845 and 786, 2,335 and 2,117, not so).  GLM53F_KDA_DECODE=pipeline / small forces one or
-    // the other; the bits are the same either way.
+    // 335 against 254).  Decode stays on the persistent kernel, which keeps more bytes in flight (bf16, 16 slots 458 against 635 us, 48
+    // slots 1,208 and 1,704; f32 single rows 845 and 786, 2,335 and 2,117, but windows of two rows 880 and 924), except with more than
+    // one and at most two units an SM: some of its blocks have two then, one after the other, and the rest wait (single rows of 160,
+    // 192, 256 and 288 units, f32 287 -> 247 us for 34 launches, 300 -> 257, 318 -> 280, 324 -> 288, bf16 221 -> 197, 229 -> 205, 237 -> 215, 239 -> 220; windows
+    // of two to six rows 2 to 13 % less; at 320 units small blocks are the slower for bf16).  GLM53F_KDA_DECODE=pipeline / small forces one
+    // or the other; the bits are the same either way.
     static const int forced = [] {
         const char* e = getenv("GLM53F_KDA_DECODE");
         return e == nullptr ? 0 : (strcmp(e, "pipeline") == 0 ? 1 : (strcmp(e, "small") == 0 ? 2 : 0));
     }();
-    const bool small = forced == 2 || (forced == 0 && k_save != nullptr);
+    const long long sms = sm_count();
+    const bool small = forced == 2 || (forced == 0 && (k_save != nullptr || (x.units > sms && x.units <= 2 * sms)));
     if (small && flags == 0 && gate == nullptr && x.units * kSmallParts <= 0x7fffffffll)
         return state_bf16 != 0 ? launch_small<__nv_bfloat16>(x, (cudaStream_t)stream) : launch_small<float>(x, (cudaStream_t)stream);
     return launch_typed<kCore>(x, state_bf16 != 0, (cudaStream_t)stream);
