@@ -55,11 +55,9 @@ struct TcParams {
     int* status;
 };
 
-__device__ __forceinline__ void widen2(uint32_t w, float& lo, float& hi) {
-    lo = __uint_as_float(w << 16);
-    hi = __uint_as_float(w & 0xffff0000u);
-}
+__device__ __forceinline__ float2 widen2(uint32_t w) { return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)); }
 
+template <bool GATED>
 __global__ void __launch_bounds__(kThreadsTc, 1) prefill_tc_kernel(const __grid_constant__ TcParams p) {
     extern __shared__ __align__(1024) unsigned char smem[];
     uint64_t* bar_raw = reinterpret_cast<uint64_t*>(smem + oBars);
@@ -72,7 +70,6 @@ __global__ void __launch_bounds__(kThreadsTc, 1) prefill_tc_kernel(const __grid_
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int quad = warp & 3, cg = warp >> 2;   // TMEM lane quadrant, column group
     const int lane_row128 = quad * 32 + lane;     // row of an M = 128 accumulator this thread reaches
-    const int lane_row64 = quad * 16 + lane;      // row of an M = 64 accumulator (lanes 0..15 only)
     const int h = blockIdx.x, b = blockIdx.y, H = p.H;
     const long long row0 = p.cu[b];
     const int T = p.cu[b + 1] - p.cu[b];
@@ -91,6 +88,14 @@ __global__ void __launch_bounds__(kThreadsTc, 1) prefill_tc_kernel(const __grid_
     __syncthreads();
     tc::fence_after_sync();
     const uint32_t tm = *tmem_slot;
+    // M = 64 accumulators are read in the fragment layout, every lane at work: this thread has their rows frag_row and frag_row + 8, columns
+    // 8 g + frag_col and the next.
+    const int frag_row = quad * 16 + (lane >> 2), frag_col = 2 * (lane & 3);
+    auto frag32 = [&](uint32_t col, uint32_t (&f)[2][8]) {  // 32 columns
+        tc::tmem_ld_frag(tc::tmem_addr(tm, quad, (int)col), f[0]);
+        tc::tmem_ld_frag(tc::tmem_addr(tm, quad, (int)col + 16), f[1]);
+        tc::tmem_ld_wait();
+    };
     const WaitCtx ctx{ctl, ctl + 1, p.status};
     uint32_t raw_phase = 0, mma_phase = 0;
     bool alive = true;
@@ -135,7 +140,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1) prefill_tc_kernel(const __grid_
 
     // One round of MMAs: warp 0 issues (one lane, the warp converged: see tc::mma_bf16_if) and commits, everybody waits for the
     // tensor core.
-    auto mma_round = [&](auto&& issue) -> bool {
+    auto mma_issue = [&](auto&& issue) {
         if (warp == 0) {
             const uint32_t leader = tc::elect_one();
             issue(leader);
@@ -143,10 +148,16 @@ __global__ void __launch_bounds__(kThreadsTc, 1) prefill_tc_kernel(const __grid_
             if (leader) atomicAdd(const_cast<uint32_t*>(ctl), 1u);
             __syncwarp();
         }
+    };
+    auto mma_wait = [&]() -> bool {
         if (!mbar_wait(bar_mma, mma_phase, ctx, kStatusWaitPrefill)) return false;
         mma_phase ^= 1u;
         tc::fence_after_sync();
         return true;
+    };
+    auto mma_round = [&](auto&& issue) -> bool {
+        mma_issue(issue);
+        return mma_wait();
     };
     auto publish_operands = [&]() {  // generic-proxy writes -> tensor core, and TMEM accesses ordered across the block
         fence_proxy_async_smem();
@@ -169,6 +180,70 @@ __global__ void __launch_bounds__(kThreadsTc, 1) prefill_tc_kernel(const __grid_
         tc::tmem_st_wait();
     }
 
+    // A chunk's outputs: bf16(y), or the gated RMSNorm of bf16(y).  From the fragments four lanes trade, so that each has eight consecutive
+    // channels of its two rows.  They leave while the next chunk's first products run.
+    // (A chunk's end, with 32 gate values and norm weights a thread read one by one, half of the lanes idle and an IEEE division each: 4
+    // sequences of 8,192 rows in all, 64 heads, with the norm 1,335 -> 1,000 us, all fragment reads together; without it 824 -> 810.)
+    int out_n = 0;
+    long long out_row = 0;
+    auto outputs = [&] {
+        const int q = lane & 3, c0 = cg * 32 + q * 8;
+        const bool odd = q & 1, up = q & 2;
+        const long long at = ((out_row + frag_row) * H + h) * DV + c0, step = 8LL * H * DV;
+        uint4 gate4[2];
+        if constexpr (GATED)
+#pragma unroll
+            for (int x = 0; x < 2; ++x) gate4[x] = frag_row + 8 * x < out_n ? *reinterpret_cast<const uint4*>(p.gate + at + x * step) : make_uint4(0, 0, 0, 0);
+        uint32_t f[2][8], y[2][4];
+        frag32(cQS + cg * 32, f);
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+            uint32_t w[4], pr[2][2];
+#pragma unroll
+            for (int g = 0; g < 4; ++g) w[g] = tc::bf16x2(__uint_as_float(f[g >> 1][4 * (g & 1) + 2 * x]), __uint_as_float(f[g >> 1][4 * (g & 1) + 2 * x + 1]));
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const uint32_t r = __shfl_xor_sync(0xffffffffu, odd ? w[2 * i] : w[2 * i + 1], 1);
+                pr[i][0] = odd ? r : w[2 * i];
+                pr[i][1] = odd ? w[2 * i + 1] : r;
+            }
+            const uint32_t r0 = __shfl_xor_sync(0xffffffffu, up ? pr[0][0] : pr[1][0], 2), r1 = __shfl_xor_sync(0xffffffffu, up ? pr[0][1] : pr[1][1], 2);
+            y[x][0] = up ? r0 : pr[0][0]; y[x][1] = up ? r1 : pr[0][1];
+            y[x][2] = up ? pr[1][0] : r0; y[x][3] = up ? pr[1][1] : r1;
+        }
+        if constexpr (GATED) {
+            float* red = reinterpret_cast<float*>(smem + oRed);
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+                float2 s2 = {0.0f, 0.0f};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) s2 = fma2(widen2(y[x][j]), widen2(y[x][j]), s2);
+                float ss = s2.x + s2.y;
+                ss += __shfl_xor_sync(0xffffffffu, ss, 1);
+                ss += __shfl_xor_sync(0xffffffffu, ss, 2);
+                if (q == 0) red[cg * CH + frag_row + 8 * x] = ss;
+            }
+            compute_sync();
+            const uint4 w4 = *reinterpret_cast<const uint4*>(p.norm_w + c0);
+            const uint32_t ww[4] = {w4.x, w4.y, w4.z, w4.w};
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+                const int i = frag_row + 8 * x;
+                const float tot = (red[i] + red[CH + i]) + (red[2 * CH + i] + red[3 * CH + i]), rinv = 1.0f / sqrtf(tot / (float)DV + p.eps);
+                const uint32_t gw[4] = {gate4[x].x, gate4[x].y, gate4[x].z, gate4[x].w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float2 g = widen2(gw[j]), sig = {rcp_approx(1.0f + ex2_ftz(-kLog2e * g.x)), rcp_approx(1.0f + ex2_ftz(-kLog2e * g.y))};
+                    const float2 v = mul2(mul2(widen2(ww[j]), mul2(widen2(y[x][j]), {rinv, rinv})), sig);
+                    y[x][j] = tc::bf16x2(v.x, v.y);
+                }
+            }
+        }
+#pragma unroll
+        for (int x = 0; x < 2; ++x)
+            if (frag_row + 8 * x < out_n) *reinterpret_cast<uint4*>(p.out + at + x * step) = make_uint4(y[x][0], y[x][1], y[x][2], y[x][3]);
+    };
+
     for (int s = 0; s < T; s += CH) {
         const int n = min(CH, T - s);
         const long long gr0 = row0 + s;
@@ -188,7 +263,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1) prefill_tc_kernel(const __grid_
             float loc[16], G = 0.0f;
 #pragma unroll
             for (int r = 0; r < 16; ++r) {
-                G += *reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(col) + r * RS32);
+                G = fmaf(*reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(col) + r * RS32), kLog2e, G);  // in powers of two from here on
                 loc[r] = G;
             }
             totals[part * 128 + d] = G;
@@ -196,7 +271,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1) prefill_tc_kernel(const __grid_
             float amax = 0.0f;
 #pragma unroll
             for (int r = 0; r < 16; ++r) {
-                const float av = __expf(loc[r] - loc[8]);
+                const float av = ex2_ftz(max_nan(loc[r] - loc[8], -126.0f));  // never 0: its reciprocal is taken
                 amax = fmaxf(amax, av);
                 *reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(col) + r * RS32) = av;
             }
@@ -211,13 +286,13 @@ __global__ void __launch_bounds__(kThreadsTc, 1) prefill_tc_kernel(const __grid_
 #pragma unroll
             for (int q2 = 0; q2 < 4; ++q2) gm[q2] = start[q2] + tab[q2 * 128];
             compute_sync();  // the relative middles have been read: the tables may be written over them
-            tab[(tE0 + part) * 128] = __expf(gm[part]);
-            tab[(tEL + part) * 128] = __expf(start[4] - gm[part]);
+            tab[(tE0 + part) * 128] = ex2_approx(gm[part]);  // (denormals are wanted here: see kda_prefill_sp.cu)
+            tab[(tEL + part) * 128] = ex2_approx(start[4] - gm[part]);
 #pragma unroll
             for (int I = 1; I < 4; ++I)
-                if (I > part) tab[(tF + I * (I - 1) / 2 + part) * 128] = __expf(gm[I] - gm[part]);
-            if (part == 3) egl[d] = __expf(start[4]);
-            mild = start[4] > -60.0f;
+                if (I > part) tab[(tF + I * (I - 1) / 2 + part) * 128] = ex2_approx(gm[I] - gm[part]);
+            if (part == 3) egl[d] = ex2_approx(start[4]);
+            mild = start[4] > -60.0f * kLog2e;
         }
         // A chunk whose whole decay stays above e^-60 in every channel takes one reference row (the chunk's start): one
         // column-side tile, one product each for L^T and M^T, no second operand pass.  The block decides together (the
@@ -239,26 +314,18 @@ __global__ void __launch_bounds__(kThreadsTc, 1) prefill_tc_kernel(const __grid_
                 const float4 e1 = *reinterpret_cast<const float4*>(tabs + (tE0 + J) * 128 + c * 8 + 4);
                 const float4 l0 = *reinterpret_cast<const float4*>(egl + c * 8);
                 const float4 l1 = *reinterpret_cast<const float4*>(egl + c * 8 + 4);
-                const float E[8] = {a0.x * e0.x, a0.y * e0.y, a0.z * e0.z, a0.w * e0.w, a1.x * e1.x, a1.y * e1.y, a1.z * e1.z, a1.w * e1.w};
-                const float EL[8] = {l0.x, l0.y, l0.z, l0.w, l1.x, l1.y, l1.z, l1.w};
+                const float2 A[4] = {{a0.x, a0.y}, {a0.z, a0.w}, {a1.x, a1.y}, {a1.z, a1.w}}, E0[4] = {{e0.x, e0.y}, {e0.z, e0.w}, {e1.x, e1.y}, {e1.z, e1.w}};
+                const float2 EL[4] = {{l0.x, l0.y}, {l0.z, l0.w}, {l1.x, l1.y}, {l1.z, l1.w}};
                 const uint32_t kw[4] = {k8.x, k8.y, k8.z, k8.w}, qw[4] = {q8.x, q8.y, q8.z, q8.w};
                 uint32_t kg[4], qg[4], ki[4], dh[4], dl[4];
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    float kf[2], qf[2], vi[2], hi[2], lo[2];
-                    widen2(kw[j], kf[0], kf[1]);
-                    widen2(qw[j], qf[0], qf[1]);
-#pragma unroll
-                    for (int u = 0; u < 2; ++u) {
-                        const float einv = __fdividef(1.0f, E[2 * j + u]);
-                        vi[u] = kf[u] * einv;
-                        tc::split_bf16(kf[u] * (EL[2 * j + u] * einv), hi[u], lo[u]);
-                    }
-                    kg[j] = tc::bf16x2(kf[0] * E[2 * j], kf[1] * E[2 * j + 1]);
-                    qg[j] = tc::bf16x2(qf[0] * E[2 * j], qf[1] * E[2 * j + 1]);
-                    ki[j] = tc::bf16x2(vi[0], vi[1]);
-                    dh[j] = tc::bf16x2(hi[0], hi[1]);
-                    dl[j] = tc::bf16x2(lo[0], lo[1]);
+                    const float2 kf = widen2(kw[j]), e = mul2(A[j], E0[j]), einv = {rcp_approx(e.x), rcp_approx(e.y)};
+                    const float2 v_kg = mul2(kf, e), v_qg = mul2(widen2(qw[j]), e), v_ki = mul2(kf, einv), v_kd = mul2(kf, mul2(EL[j], einv));
+                    kg[j] = tc::bf16x2(v_kg.x, v_kg.y);
+                    qg[j] = tc::bf16x2(v_qg.x, v_qg.y);
+                    ki[j] = tc::bf16x2(v_ki.x, v_ki.y);
+                    tc::split_bf16x2(v_kd.x, v_kd.y, dh[j], dl[j]);
                 }
                 *reinterpret_cast<uint4*>(cell(smem + oKg, CH, c, r)) = make_uint4(kg[0], kg[1], kg[2], kg[3]);
                 *reinterpret_cast<uint4*>(cell(smem + oQg, CH, c, r)) = make_uint4(qg[0], qg[1], qg[2], qg[3]);
@@ -269,14 +336,14 @@ __global__ void __launch_bounds__(kThreadsTc, 1) prefill_tc_kernel(const __grid_
             }
             publish_operands();
             if (tid == 0 && s + CH < T) mbar_arrive(bar_free);  // the staging area is free for the next chunk's rows
-            if (!mma_round([&](uint32_t leader) {
+            mma_issue([&](uint32_t leader) {
                     constexpr uint32_t id = tc::idesc_bf16(64, 64, 0, 0, 0);
                     const unsigned char* kit = smem + oKc + kc_tile(3);
                     for (int k0 = 0; k0 < DK; k0 += 16)
                         tc::mma_bf16_if(leader, tm + cL, tc::desc_kmajor_bf16(kit, CH, 0, k0), tc::desc_kmajor_bf16(smem + oKg, CH, 0, k0), id, k0 > 0);
                     for (int k0 = 0; k0 < DK; k0 += 16)
                         tc::mma_bf16_if(leader, tm + cMm, tc::desc_kmajor_bf16(kit, CH, 0, k0), tc::desc_kmajor_bf16(smem + oQg, CH, 0, k0), id, k0 > 0);
-                })) { alive = false; break; }
+                });
         } else {
         // ---- 2. operand tiles: lane <-> row, one 16-byte cell (8 channels) at a time.  Row sides Kgb = K a -> oKg, Qgb = Q a ->
         // oQg; the column sides K exp(Gm_I - G) into the four tiles I >= J; Kdec = K exp(G_last - G) as bf16 hi + lo; V as it is.
@@ -293,27 +360,19 @@ __global__ void __launch_bounds__(kThreadsTc, 1) prefill_tc_kernel(const __grid_
                 const float4 a1 = *reinterpret_cast<const float4*>(smem + oRawG + r * RS32 + c * 32 + 16);
                 const float4 l0 = *reinterpret_cast<const float4*>(tabs + (tEL + J) * 128 + c * 8);
                 const float4 l1 = *reinterpret_cast<const float4*>(tabs + (tEL + J) * 128 + c * 8 + 4);
-                const float A[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-                const float EL[8] = {l0.x, l0.y, l0.z, l0.w, l1.x, l1.y, l1.z, l1.w};
+                const float2 A[4] = {{a0.x, a0.y}, {a0.z, a0.w}, {a1.x, a1.y}, {a1.z, a1.w}}, EL[4] = {{l0.x, l0.y}, {l0.z, l0.w}, {l1.x, l1.y}, {l1.z, l1.w}};
                 const uint32_t kw[4] = {k8.x, k8.y, k8.z, k8.w}, qw[4] = {q8.x, q8.y, q8.z, q8.w};
                 uint32_t kgb[4], qgb[4], kcd[4], dh[4], dl[4];
-                float kc[8];
+                float2 kc[4];
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    float kf[2], qf[2];
-                    widen2(kw[j], kf[0], kf[1]);
-                    widen2(qw[j], qf[0], qf[1]);
-                    float hi[2], lo[2];
-#pragma unroll
-                    for (int u = 0; u < 2; ++u) {
-                        kc[2 * j + u] = kf[u] * __fdividef(1.0f, A[2 * j + u]);
-                        tc::split_bf16(kc[2 * j + u] * EL[2 * j + u], hi[u], lo[u]);
-                    }
-                    kgb[j] = tc::bf16x2(kf[0] * A[2 * j], kf[1] * A[2 * j + 1]);
-                    qgb[j] = tc::bf16x2(qf[0] * A[2 * j], qf[1] * A[2 * j + 1]);
-                    kcd[j] = tc::bf16x2(kc[2 * j], kc[2 * j + 1]);
-                    dh[j] = tc::bf16x2(hi[0], hi[1]);
-                    dl[j] = tc::bf16x2(lo[0], lo[1]);
+                    const float2 kf = widen2(kw[j]), v_kgb = mul2(kf, A[j]), v_qgb = mul2(widen2(qw[j]), A[j]);
+                    kc[j] = mul2(kf, {rcp_approx(A[j].x), rcp_approx(A[j].y)});
+                    const float2 v_kd = mul2(kc[j], EL[j]);
+                    kgb[j] = tc::bf16x2(v_kgb.x, v_kgb.y);
+                    qgb[j] = tc::bf16x2(v_qgb.x, v_qgb.y);
+                    kcd[j] = tc::bf16x2(kc[j].x, kc[j].y);
+                    tc::split_bf16x2(v_kd.x, v_kd.y, dh[j], dl[j]);
                 }
                 *reinterpret_cast<uint4*>(cell(smem + oKg, CH, c, r)) = make_uint4(kgb[0], kgb[1], kgb[2], kgb[3]);
                 *reinterpret_cast<uint4*>(cell(smem + oQg, CH, c, r)) = make_uint4(qgb[0], qgb[1], qgb[2], qgb[3]);
@@ -324,16 +383,21 @@ __global__ void __launch_bounds__(kThreadsTc, 1) prefill_tc_kernel(const __grid_
                 for (int I = J + 1; I < 4; ++I) {  // the later row blocks see this row through exp(Gm_I - Gm_J) <= 1
                     const float* f = tabs + (tF + I * (I - 1) / 2 + J) * 128 + c * 8;
                     const float4 fa = *reinterpret_cast<const float4*>(f), fb = *reinterpret_cast<const float4*>(f + 4);
-                    *reinterpret_cast<uint4*>(cell(smem + oKc + kc_tile(I), 16 * (I + 1), c, r)) =
-                        make_uint4(tc::bf16x2(kc[0] * fa.x, kc[1] * fa.y), tc::bf16x2(kc[2] * fa.z, kc[3] * fa.w),
-                                   tc::bf16x2(kc[4] * fb.x, kc[5] * fb.y), tc::bf16x2(kc[6] * fb.z, kc[7] * fb.w));
+                    const float2 F[4] = {{fa.x, fa.y}, {fa.z, fa.w}, {fb.x, fb.y}, {fb.z, fb.w}};
+                    uint32_t kcf[4];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const float2 x = mul2(kc[j], F[j]);
+                        kcf[j] = tc::bf16x2(x.x, x.y);
+                    }
+                    *reinterpret_cast<uint4*>(cell(smem + oKc + kc_tile(I), 16 * (I + 1), c, r)) = make_uint4(kcf[0], kcf[1], kcf[2], kcf[3]);
                 }
             }
         }
         publish_operands();
 
         // ---- 3. L^T and M^T, one block column of 16 rows i at a time: [64 j x 16 i] = column side (tile I) x row side (block I)^T
-        if (!mma_round([&](uint32_t leader) {
+        mma_issue([&](uint32_t leader) {
                 constexpr uint32_t id = tc::idesc_bf16(64, 16, 0, 0, 0);
                 for (int I = 0; I < 4; ++I) {
                     const unsigned char* kct = smem + oKc + kc_tile(I);
@@ -343,10 +407,14 @@ __global__ void __launch_bounds__(kThreadsTc, 1) prefill_tc_kernel(const __grid_
                     for (int k0 = 0; k0 < DK; k0 += 16)
                         tc::mma_bf16_if(leader, tm + cMm + 16 * I, tc::desc_kmajor_bf16(kct, R, 0, k0), tc::desc_kmajor_bf16(smem + oQg, CH, 16 * I, k0), id, k0 > 0);
                 }
-            })) { alive = false; break; }
+            });
+        }
+        if (out_n > 0) outputs();
+        if (!mma_wait()) { alive = false; break; }
 
-        // ---- 3b. the tiles that take the decay from the chunk's start, over the row sides (the tensor core is done with
+        // ---- 3b. block-wise: the tiles that take the decay from the chunk's start, over the row sides (the tensor core is done with
         // them): Kg = K exp(G) for W, Qg = Q exp(G) for Q S.  Then the staging area is free.
+        if (!narrow) {
         {
             const int r = tid & 63, cgrp = tid >> 6, J = r >> 4;
             const float* tabs = reinterpret_cast<const float*>(smem + oTab);
@@ -359,16 +427,14 @@ __global__ void __launch_bounds__(kThreadsTc, 1) prefill_tc_kernel(const __grid_
                 const float4 a1 = *reinterpret_cast<const float4*>(smem + oRawG + r * RS32 + c * 32 + 16);
                 const float4 e0 = *reinterpret_cast<const float4*>(tabs + (tE0 + J) * 128 + c * 8);
                 const float4 e1 = *reinterpret_cast<const float4*>(tabs + (tE0 + J) * 128 + c * 8 + 4);
-                const float E[8] = {a0.x * e0.x, a0.y * e0.y, a0.z * e0.z, a0.w * e0.w, a1.x * e1.x, a1.y * e1.y, a1.z * e1.z, a1.w * e1.w};
+                const float2 E[4] = {mul2({a0.x, a0.y}, {e0.x, e0.y}), mul2({a0.z, a0.w}, {e0.z, e0.w}), mul2({a1.x, a1.y}, {e1.x, e1.y}), mul2({a1.z, a1.w}, {e1.z, e1.w})};
                 const uint32_t kw[4] = {k8.x, k8.y, k8.z, k8.w}, qw[4] = {q8.x, q8.y, q8.z, q8.w};
                 uint32_t kg[4], qg[4];
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    float kf[2], qf[2];
-                    widen2(kw[j], kf[0], kf[1]);
-                    widen2(qw[j], qf[0], qf[1]);
-                    kg[j] = tc::bf16x2(kf[0] * E[2 * j], kf[1] * E[2 * j + 1]);
-                    qg[j] = tc::bf16x2(qf[0] * E[2 * j], qf[1] * E[2 * j + 1]);
+                    const float2 v_kg = mul2(widen2(kw[j]), E[j]), v_qg = mul2(widen2(qw[j]), E[j]);
+                    kg[j] = tc::bf16x2(v_kg.x, v_kg.y);
+                    qg[j] = tc::bf16x2(v_qg.x, v_qg.y);
                 }
                 *reinterpret_cast<uint4*>(cell(smem + oKg, CH, c, r)) = make_uint4(kg[0], kg[1], kg[2], kg[3]);
                 *reinterpret_cast<uint4*>(cell(smem + oQg, CH, c, r)) = make_uint4(qg[0], qg[1], qg[2], qg[3]);
@@ -379,32 +445,26 @@ __global__ void __launch_bounds__(kThreadsTc, 1) prefill_tc_kernel(const __grid_
         if (tid == 0 && s + CH < T) mbar_arrive(bar_free);
         }
 
-        // ---- 4. from L^T and M^T (lane = column j, tensor-memory column = row i): L (FP32, strictly lower, times beta_i); M
-        // (lower with the diagonal) as bf16 cells of eight consecutive rows i, [8 cells][64 columns j].  Column groups 0, 1
-        // take the two halves (of i) of L, groups 2, 3 those of M; lanes 0..15 hold the columns.
+        // ---- 4. from L^T and M^T (accumulator row = column j, column = row i): L (FP32, strictly lower, times beta_i), transposed as it
+        // comes; M (lower with the diagonal) as bf16 cells of eight consecutive rows i, [8 cells][64 columns j], of which four lanes have
+        // a pair each.  Column groups 0, 1 take the two halves (of i) of L, groups 2, 3 those of M.
         {
-            uint32_t r[32];
-            const int half = cg & 1, j = lane_row64;
-            tc::tmem_ld32(tc::tmem_addr(tm, quad, (cg < 2 ? cL : cMm) + half * 32), r);
-            tc::tmem_ld_wait();
-            if (lane < 16) {
-                if (cg < 2) {  // L stays transposed: this thread's column j, 32 consecutive rows i
-                    float* Lt = reinterpret_cast<float*>(smem + oL) + j * LS + half * 32;
+            const int half = (cg & 1) * 32;
+            uint32_t f[2][8];
+            frag32((cg < 2 ? cL : cMm) + half, f);
 #pragma unroll
-                    for (int i4 = 0; i4 < 8; ++i4) {
-                        const float4 b4 = *reinterpret_cast<const float4*>(betas + half * 32 + i4 * 4);
-                        const int i = half * 32 + i4 * 4;
-                        *reinterpret_cast<float4*>(Lt + i4 * 4) = make_float4(i > j ? b4.x * __uint_as_float(r[i4 * 4]) : 0.0f, i + 1 > j ? b4.y * __uint_as_float(r[i4 * 4 + 1]) : 0.0f,
-                                                                              i + 2 > j ? b4.z * __uint_as_float(r[i4 * 4 + 2]) : 0.0f, i + 3 > j ? b4.w * __uint_as_float(r[i4 * 4 + 3]) : 0.0f);
+            for (int g = 0; g < 4; ++g)
+#pragma unroll
+                for (int x = 0; x < 2; ++x) {
+                    const int i = half + g * 8 + frag_col, j = frag_row + 8 * x;
+                    const float v0 = __uint_as_float(f[g >> 1][4 * (g & 1) + 2 * x]), v1 = __uint_as_float(f[g >> 1][4 * (g & 1) + 2 * x + 1]);
+                    if (cg < 2) {
+                        const float2 b2 = *reinterpret_cast<const float2*>(betas + i);
+                        *reinterpret_cast<float2*>(reinterpret_cast<float*>(smem + oL) + j * LS + i) = make_float2(i > j ? b2.x * v0 : 0.0f, i + 1 > j ? b2.y * v1 : 0.0f);
+                    } else {
+                        *reinterpret_cast<uint32_t*>(cell(smem + oMm, CH, half / 8 + g, j) + 2 * frag_col) = tc::bf16x2(i >= j ? v0 : 0.0f, i + 1 >= j ? v1 : 0.0f);
                     }
-                } else {
-#pragma unroll
-                    for (int i2 = 0; i2 < 32; ++i2)
-                        if (half * 32 + i2 < j) r[i2] = 0u;
-#pragma unroll
-                    for (int cc = 0; cc < 4; ++cc) *reinterpret_cast<uint4*>(cell(smem + oMm, CH, half * 4 + cc, j)) = pack8(r + cc * 8);
                 }
-            }
         }
         compute_sync();
 
@@ -425,11 +485,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1) prefill_tc_kernel(const __grid_
                 uint32_t wh[4], wl[4];
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    float h0, l0, h1, l1;
-                    tc::split_bf16(t8[2 * j], h0, l0);
-                    tc::split_bf16(t8[2 * j + 1], h1, l1);
-                    wh[j] = tc::bf16x2(h0, h1);
-                    wl[j] = tc::bf16x2(l0, l1);
+                    tc::split_bf16x2(t8[2 * j], t8[2 * j + 1], wh[j], wl[j]);
                 }
                 *reinterpret_cast<uint4*>(cell(smem + oTpHi, CH, c, i)) = make_uint4(wh[0], wh[1], wh[2], wh[3]);
                 *reinterpret_cast<uint4*>(cell(smem + oTpLo, CH, c, i)) = make_uint4(wl[0], wl[1], wl[2], wl[3]);
@@ -450,13 +506,14 @@ __global__ void __launch_bounds__(kThreadsTc, 1) prefill_tc_kernel(const __grid_
 
         // ---- 7. W to bf16 cells; 8. S to bf16 cells (over Kg | Kinv, both dead), the decayed S back to tensor memory ------------
         {
-            uint32_t r[32];
-            tc::tmem_ld32(tc::tmem_addr(tm, quad, cW + cg * 32), r);
-            tc::tmem_ld_wait();
-            if (lane < 16) {
+            uint32_t r[32], f[2][8];
+            frag32(cW + cg * 32, f);
 #pragma unroll
-                for (int cc = 0; cc < 4; ++cc) *reinterpret_cast<uint4*>(cell(smem + oW, CH, cg * 4 + cc, lane_row64)) = pack8(r + cc * 8);
-            }
+            for (int g = 0; g < 4; ++g)
+#pragma unroll
+                for (int x = 0; x < 2; ++x)
+                    *reinterpret_cast<uint32_t*>(cell(smem + oW, CH, cg * 4 + g, frag_row + 8 * x) + 2 * frag_col) =
+                        tc::bf16x2(__uint_as_float(f[g >> 1][4 * (g & 1) + 2 * x]), __uint_as_float(f[g >> 1][4 * (g & 1) + 2 * x + 1]));
             tc::tmem_ld32(tc::tmem_addr(tm, quad, cS + cg * 32), r);
             tc::tmem_ld_wait();
             if (p.state_bf16) {  // a bf16 state is rounded once per chunk
@@ -484,25 +541,17 @@ __global__ void __launch_bounds__(kThreadsTc, 1) prefill_tc_kernel(const __grid_
 
         // ---- 10. D as bf16 hi + lo cells (over T' | V, both dead) -------------------------------------------------------------------
         {
-            uint32_t r[32];
-            tc::tmem_ld32(tc::tmem_addr(tm, quad, cU + cg * 32), r);
-            tc::tmem_ld_wait();
-            if (lane < 16) {
+            uint32_t f[2][8];
+            frag32(cU + cg * 32, f);
 #pragma unroll
-                for (int cc = 0; cc < 4; ++cc) {
-                    uint32_t wh[4], wl[4];
+            for (int g = 0; g < 4; ++g)
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        float h0, l0, h1, l1;
-                        tc::split_bf16(__uint_as_float(r[cc * 8 + 2 * j]), h0, l0);
-                        tc::split_bf16(__uint_as_float(r[cc * 8 + 2 * j + 1]), h1, l1);
-                        wh[j] = tc::bf16x2(h0, h1);
-                        wl[j] = tc::bf16x2(l0, l1);
-                    }
-                    *reinterpret_cast<uint4*>(cell(smem + oDhi, CH, cg * 4 + cc, lane_row64)) = make_uint4(wh[0], wh[1], wh[2], wh[3]);
-                    *reinterpret_cast<uint4*>(cell(smem + oDlo, CH, cg * 4 + cc, lane_row64)) = make_uint4(wl[0], wl[1], wl[2], wl[3]);
+                for (int x = 0; x < 2; ++x) {
+                    uint32_t hi, lo;
+                    tc::split_bf16x2(__uint_as_float(f[g >> 1][4 * (g & 1) + 2 * x]), __uint_as_float(f[g >> 1][4 * (g & 1) + 2 * x + 1]), hi, lo);
+                    *reinterpret_cast<uint32_t*>(cell(smem + oDhi, CH, cg * 4 + g, frag_row + 8 * x) + 2 * frag_col) = hi;
+                    *reinterpret_cast<uint32_t*>(cell(smem + oDlo, CH, cg * 4 + g, frag_row + 8 * x) + 2 * frag_col) = lo;
                 }
-            }
         }
         publish_operands();
 
@@ -519,45 +568,10 @@ __global__ void __launch_bounds__(kThreadsTc, 1) prefill_tc_kernel(const __grid_
                     tc::mma_bf16_if(leader, tm + cS, tc::desc_mnmajor_bf16(smem + oKdLo, CH, 0, k0), tc::desc_mnmajor_bf16(smem + oDhi, CH, 0, k0), ids, true);
             })) { alive = false; break; }
 
-        // ---- 12. outputs: bf16(y), or the gated RMSNorm of bf16(y); a thread holds 32 columns of its row -------------------------------
-        {
-            uint32_t r[32];
-            tc::tmem_ld32(tc::tmem_addr(tm, quad, cQS + cg * 32), r);
-            tc::tmem_ld_wait();
-            const int i = lane_row64;
-            const bool live = lane < 16 && i < n;
-            const long long at = ((gr0 + i) * H + h) * DV + cg * 32;
-            float y[32];
-#pragma unroll
-            for (int j = 0; j < 32; ++j) y[j] = bf16_round(__uint_as_float(r[j]));
-            if (p.gate != nullptr) {
-                float* red = reinterpret_cast<float*>(smem + oRed);
-                float ss = 0.0f;
-#pragma unroll
-                for (int j = 0; j < 32; ++j) ss = fmaf(y[j], y[j], ss);
-                if (lane < 16) red[cg * CH + i] = ss;
-                compute_sync();
-                if (live) {
-                    const float tot = (red[i] + red[CH + i]) + (red[2 * CH + i] + red[3 * CH + i]);
-                    const float rinv = 1.0f / sqrtf(tot / (float)DV + p.eps);
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) {
-                        const float gt = bf16_bits_to_f32(p.gate[at + j]), w = bf16_bits_to_f32(p.norm_w[cg * 32 + j]);
-                        y[j] = w * (y[j] * rinv) * (1.0f / (1.0f + __expf(-gt)));
-                    }
-                }
-            }
-            if (live) {
-#pragma unroll
-                for (int c = 0; c < 4; ++c)
-                    *reinterpret_cast<uint4*>(p.out + at + c * 8) = make_uint4(tc::bf16x2(y[c * 8], y[c * 8 + 1]), tc::bf16x2(y[c * 8 + 2], y[c * 8 + 3]),
-                                                                            tc::bf16x2(y[c * 8 + 4], y[c * 8 + 5]), tc::bf16x2(y[c * 8 + 6], y[c * 8 + 7]));
-            }
-        }
-        tc::fence_before_sync();
-        compute_sync();
-        tc::fence_after_sync();
+        out_n = n;
+        out_row = gr0;
     }
+    if (alive && out_n > 0) outputs();
 
     // ---- the outgoing state -------------------------------------------------------------------------------------------------------
     if (alive) {
@@ -586,7 +600,8 @@ int core_prefill_tc_launch(int32_t heads, int32_t batch, const int32_t* cu_seqle
     int dev = 0;
     cudaGetDevice(&dev);
     if (configured_dev != dev) {
-        const cudaError_t e = cudaFuncSetAttribute(prefill_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemTc);
+        cudaError_t e = cudaFuncSetAttribute(prefill_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemTc);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(prefill_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemTc);
         if (e != cudaSuccess) return (int)e;
         configured_dev = dev;
     }
@@ -601,7 +616,7 @@ int core_prefill_tc_launch(int32_t heads, int32_t batch, const int32_t* cu_seqle
     p.out = out;
     p.status = status_word();
     if (p.status == nullptr) return (int)cudaErrorUnknown;
-    prefill_tc_kernel<<<dim3(heads, batch), kThreadsTc, kSmemTc, stream>>>(p);
+    (gate != nullptr ? prefill_tc_kernel<true> : prefill_tc_kernel<false>)<<<dim3(heads, batch), kThreadsTc, kSmemTc, stream>>>(p);
     return (int)cudaGetLastError();
 }
 
