@@ -25,14 +25,16 @@
 // RMSNorm into its outputs.
 //
 // One block of 128 threads per (request, head) unit, three blocks per SM, blocks walk the units persistently.  A unit's
-// rows and state arrive by asynchronous 16-byte copies issued one unit ahead (the state straight into the 128-byte
-// swizzle the tensor core reads), so one unit's arithmetic covers the next one's loads.  All waits are bounded.
+// rows arrive by asynchronous 16-byte copies, its state by two tensor copies straight into the 128-byte swizzle the tensor core
+// reads, all issued one unit ahead, so one unit's arithmetic covers the next one's loads.  All waits are bounded.
 //
 // A unit's serial stages bound it, at twelve warps an SM.  What they took and take, cycles of a unit of the core form (48 requests of 8 to
 // 16 rows): operand tiles 4,400 with two exponentials and a division an element and the saves between them, 1,800 as products of
 // multipliers; the saves 1,300, beside the first products; the next rows' copies 1,800 with a load of beta to wait for, 570 without;
 // products 870 + 880 as eight of N = 32 each instead of sixteen of N = 16; outputs 3,000 as two-byte stores, now sixteen bytes a unit
-// later.  Verify and commit of 34 layers together: 3,806 -> 3,183 us, 20 requests of 4 to 8 rows 1,625 -> 1,371.
+// later.  Verify and commit of 34 layers together: 3,806 -> 3,183 us, 20 requests of 4 to 8 rows 1,625 -> 1,371; with the state in boxes,
+// in both kernels and both ways, instead of 2,048 pieces that pass through the threads, 2,894 and 1,240 (the commit's way out alone was
+// 2,000 cycles of a unit's 14,000).
 
 #include <cuda_fp16.h>
 
@@ -40,6 +42,7 @@
 #include "glm53f_kda.h"
 #include "kda_internal.h"
 #include "tc.cuh"
+#include "tensor_map.cuh"
 
 namespace kda {
 namespace {
@@ -63,12 +66,39 @@ struct Raw {
 template <bool LAYER>
 struct Map {
     static constexpr int vOut = vRaw + Raw<LAYER>::kBytes;  // core form: a unit's outputs, bf16 [16][128], on their way out
-    static constexpr int vBeta = vOut + (LAYER ? 0 : WIN * DV * 2), vBar = vBeta + 64, vCtl = vBar + 16, kSmem = vCtl + 16;
+    static constexpr int vBeta = vOut + (LAYER ? 0 : WIN * DV * 2), vBar = vBeta + 64 /* products, state */, vCtl = vBar + 16, kSmem = vCtl + 16;
     static_assert(vBar % 8 == 0 && kSmem <= 75 * 1024, "three blocks per SM");
 };
 constexpr uint32_t kVCols = 32;  // tensor memory: [0, 16) L^T then (W S)^T, [16, 32) M^T then (Qg S)^T
 
+// A state buffer as rows of 128 elements in two halves, for copies of a unit's [128][128] that come in, and go out, in the tile's own
+// swizzle: two boxes instead of 2,048 pieces, and nothing of them passes through the threads.  For buffers on 16 bytes and units at a
+// multiple of a row; the others go piece by piece.
+bool state_map(CUtensorMap* tm, const void* base) {
+    EncodeTiled enc = encode_tiled();
+    if (enc == nullptr || (reinterpret_cast<uintptr_t>(base) & 15) != 0) return false;
+    const cuuint64_t dims[3] = {64u, 2u, 0x7fffffffu}, strides[2] = {128u, 256u};
+    const cuuint32_t box[3] = {64u, 1u, (cuuint32_t)DV}, step[3] = {1u, 1u, 1u};
+    return enc(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+__device__ __forceinline__ bool in_boxes(int mapped, long long s_elem) { return mapped && (s_elem & (DK - 1)) == 0 && s_elem >= 0 && s_elem <= (0x7fffffffll - DV) * DK; }
+__device__ __forceinline__ void load_boxes(unsigned char* tile, const CUtensorMap* tm, long long s_elem, uint64_t* bar) {
+    mbar_arrive_expect_tx(bar, DV * DK * 2);
+    for (int x = 0; x < 2; ++x) tensor_load_3d(tile + x * 16384, tm, 0, x, (int)(s_elem / DK), bar);
+}
+
+// After an abort a unit's boxes may still be on their way into this block's shared memory: a bounded time for them.
+__device__ __forceinline__ void abort_pause(volatile uint32_t* ctl) {
+    if (ctl[1] == 0u) return;
+    const uint64_t t0 = global_timer_ns();
+    while (global_timer_ns() - t0 < 2000000ull) {
+    }
+}
+
 struct VParams {
+    alignas(64) CUtensorMap tm_state;
+    int mapped;
     int H;
     long long units;
     const int32_t* cu;
@@ -274,9 +304,11 @@ __device__ __forceinline__ void fetch_rows(const VParams& p, unsigned char* smem
     cp_async_commit();
 }
 // The unit's state, 2,048 pieces of 16 bytes, into the swizzled tile.
-__device__ __forceinline__ void fetch_state(const VParams& p, unsigned char* smem, const Unit& un, int t) {
+__device__ __forceinline__ void fetch_state(const VParams& p, unsigned char* smem, const Unit& un, int t, uint64_t* bar_state) {
     const uint16_t* src = p.state + un.s_elem;
-    if ((reinterpret_cast<uintptr_t>(src) & 15) == 0) {
+    if (in_boxes(p.mapped, un.s_elem)) {
+        if (t == 0) load_boxes(smem + vS, &p.tm_state, un.s_elem, bar_state);
+    } else if ((reinterpret_cast<uintptr_t>(src) & 15) == 0) {
         unsigned char* to = smem + vS + state_piece(t >> 4, t & 15);  // eight rows a step: the swizzle stays
         src += t * 8;
 #pragma unroll
@@ -332,6 +364,7 @@ __global__ void __launch_bounds__(kVThreads, 3) verify_tc_kernel(const __grid_co
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     if (t == 0) {
         mbar_init(bar, 1);
+        mbar_init(bar + 1, 1);
         ctl[0] = 0u;
         ctl[1] = 0u;
         mbar_init_fence();
@@ -343,7 +376,7 @@ __global__ void __launch_bounds__(kVThreads, 3) verify_tc_kernel(const __grid_co
     const uint32_t tm = *tmem_slot;
     grid_ready();
     const WaitCtx ctx{ctl, ctl + 1, p.status};
-    uint32_t phase = 0;
+    uint32_t phase = 0, state_phase = 0;
     float2* Ln = reinterpret_cast<float2*>(smem + vL);
     float* Mf = reinterpret_cast<float*>(smem + vM);
     float* betas = reinterpret_cast<float*>(smem + MP::vBeta);
@@ -370,7 +403,7 @@ __global__ void __launch_bounds__(kVThreads, 3) verify_tc_kernel(const __grid_co
     bool more = units.take(p, nxt);
     if (more) {
         fetch_rows<LAYER>(p, smem, nxt, t);
-        fetch_state(p, smem, nxt, t);
+        fetch_state(p, smem, nxt, t, bar + 1);
     }
     while (more) {
         un = nxt;
@@ -493,9 +526,13 @@ __global__ void __launch_bounds__(kVThreads, 3) verify_tc_kernel(const __grid_co
 #pragma unroll
         for (int i = 0; i < WIN; ++i) *reinterpret_cast<uint16_t*>(smem + vRow + sw_elem(kRowR, i, c0 + upper)) = f32_to_bf16_bits(wu[i].x);
         cp_async_wait<1>();  // this unit's state has landed (the next unit's rows may still be on the way)
+        if (in_boxes(p.mapped, un.s_elem)) {
+            ok = mbar_wait(bar + 1, state_phase, ctx, kStatusWaitPrefill);
+            state_phase ^= 1u;
+        }
         fence_proxy_async_smem();
         tc::fence_before_sync();
-        __syncthreads();
+        if (!__syncthreads_and(ok)) break;
         tc::fence_after_sync();
 
         // ---- D. (W S)^T and (Qg S)^T: the state tile as it lies in memory is the M operand ---------------------------------------
@@ -514,7 +551,7 @@ __global__ void __launch_bounds__(kVThreads, 3) verify_tc_kernel(const __grid_co
         if (!__syncthreads_and(ok)) break;
         tc::fence_after_sync();
         // The state tile is consumed: the next unit's may come in.
-        if (more) fetch_state(p, smem, nxt, t);
+        if (more) fetch_state(p, smem, nxt, t, bar + 1);
         else cp_async_commit();
 
         // ---- E. D = U - W S,  O = Qg S + M D; thread = value channel = its tensor-memory lane -----------------------------------------
@@ -575,6 +612,7 @@ __global__ void __launch_bounds__(kVThreads, 3) verify_tc_kernel(const __grid_co
         }
     }
     cp_async_wait<0>();
+    abort_pause(ctl);
     tc::fence_before_sync();
     __syncthreads();
     if constexpr (!LAYER) {
@@ -600,7 +638,7 @@ __global__ void __launch_bounds__(kVThreads, 3) verify_tc_kernel(const __grid_co
 // The hi half of D^T shares its 4 KB with Kc and L: Kc is read by the L^T product only, L by the forward substitution only, and
 // D^T is written after the (W S)^T product, which comes after both.
 constexpr int cS = 0, cDT = 32768, cKc = cDT, cKgb = cDT + 8192, cKdT = cKgb + 4096, cE = cKdT + 8192, cBeta = cE + 512;
-constexpr int cBar = cBeta + 64, cCtl = cBar + 16, cRawK = cCtl + 16, cRawG = cRawK + WIN * DK * 4, cRawV = cRawG + WIN * DK * 4, kCSmem = cRawV + WIN * DV * 2;
+constexpr int cBar = cBeta + 64 /* products, state */, cCtl = cBar + 16, cRawK = cCtl + 16, cRawG = cRawK + WIN * DK * 4, cRawV = cRawG + WIN * DK * 4, kCSmem = cRawV + WIN * DV * 2;
 constexpr int cW = cKgb, cL = cKc;                    // W replaces Kgb, L replaces Kc once L^T is done
 constexpr uint32_t kCCols = 128;                      // tensor memory: L^T, then (W S)^T, then the 128 x 128 update
 constexpr int kCBlocks = 3;
@@ -608,6 +646,8 @@ static_assert(kCBlocks * (kCSmem + 1024) <= 228 * 1024 && kCBlocks * kCCols <= 5
 static_assert(cRawK % 16 == 0 && WIN * LN * 8 <= 4096, "");
 
 struct CParams {
+    alignas(64) CUtensorMap tm_in, tm_out;
+    int mapped;
     int H, layers, rows1;
     long long units;
     const int32_t* cu;
@@ -634,6 +674,7 @@ __global__ void __launch_bounds__(kVThreads, kCBlocks) commit_tc_kernel(const __
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     if (t == 0) {
         mbar_init(bar, 1);
+        mbar_init(bar + 1, 1);
         ctl[0] = 0u;
         ctl[1] = 0u;
         mbar_init_fence();
@@ -645,7 +686,7 @@ __global__ void __launch_bounds__(kVThreads, kCBlocks) commit_tc_kernel(const __
     const uint32_t tm = *tmem_slot;
     grid_ready();
     const WaitCtx ctx{ctl, ctl + 1, p.status};
-    uint32_t phase = 0;
+    uint32_t phase = 0, state_phase = 0;
     float2* Ln = reinterpret_cast<float2*>(smem + cL);
     float* En = reinterpret_cast<float*>(smem + cE);
     float* betas = reinterpret_cast<float*>(smem + cBeta);
@@ -715,16 +756,29 @@ __global__ void __launch_bounds__(kVThreads, kCBlocks) commit_tc_kernel(const __
         const long long b_base = (long long)ul * p.b_stride;
         __syncthreads();  // the previous unit's tile has been copied out
         // The unit's state into the swizzled tile.
-        const bool vec = ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0;
-        if (vec) {
+        const bool vec = ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0, boxes = in_boxes(p.mapped, s_elem);
+        if (t == 0) bulk_wait_read<0>();  // the unit before has left the tile
+        if (boxes) {
+            if (t == 0) load_boxes(smem + cS, &p.tm_in, s_elem, bar + 1);
+        } else if (vec) {
+            __syncthreads();
             unsigned char* to = smem + state_piece(t >> 4, t & 15);
 #pragma unroll
             for (int i = 0; i < 16; ++i) cp_async16(to + i * 1024, src + (t + i * kVThreads) * 8);
         } else {
+            __syncthreads();
             for (int e = t; e < DV * DK; e += kVThreads) *reinterpret_cast<uint16_t*>(smem + cS + sw_elem(DV, e >> 7, e & 127)) = src[e];
         }
         cp_async_commit();
         if (n == 0) fetch_next();
+        bool landed = !boxes;
+        auto state_lands = [&]() -> bool {
+            if (landed) return true;
+            landed = true;
+            const bool there = mbar_wait(bar + 1, state_phase, ctx, kStatusWaitPrefill);
+            state_phase ^= 1u;
+            return there;
+        };
 
         for (int c0 = 0; c0 < n && ok; c0 += WIN) {
             const int nr = min(WIN, n - c0);
@@ -828,9 +882,11 @@ __global__ void __launch_bounds__(kVThreads, kCBlocks) commit_tc_kernel(const __
 #pragma unroll
             for (int i = 0; i < WIN; ++i) *reinterpret_cast<uint16_t*>(smem + cW + sw_elem(WIN, i, ch0 + upper)) = f32_to_bf16_bits(wu[i].x);  // over Kgb, which is consumed
             cp_async_wait<1>();  // the state has landed (the next rows may still be on the way)
+            ok = state_lands();
             fence_proxy_async_smem();
             tc::fence_before_sync();
-            __syncthreads();
+            ok = __syncthreads_and(ok);
+            if (!ok) break;
             tc::fence_after_sync();
 
             // ---- D. (W S)^T = S W^T --------------------------------------------------------------------------------------------
@@ -918,10 +974,18 @@ __global__ void __launch_bounds__(kVThreads, kCBlocks) commit_tc_kernel(const __
             tc::fence_after_sync();
         }
         if (!ok) break;
-        if (n == 0) cp_async_wait<1>();  // a unit without rows: its state is only copied
-        __syncthreads();
+        if (n == 0) {  // a unit without rows: its state is only copied
+            cp_async_wait<1>();
+            ok = state_lands();
+            if (!__syncthreads_and(ok)) break;
+        }
         // ---- the tile back to global memory, coalesced ------------------------------------------------------------------------
-        if (vec) {
+        if (boxes) {  // (the last chunk's end has published the tile to these copies)
+            if (t == 0) {
+                for (int x = 0; x < 2; ++x) tensor_store_3d(&p.tm_out, 0, x, (int)(s_elem / DK), smem + cS + x * 16384);
+                bulk_commit();
+            }
+        } else if (vec) {
             const unsigned char* from = smem + state_piece(t >> 4, t & 15);
 #pragma unroll
             for (int i = 0; i < 16; ++i) *reinterpret_cast<uint4*>(dst + (t + i * kVThreads) * 8) = *reinterpret_cast<const uint4*>(from + i * 1024);
@@ -929,7 +993,9 @@ __global__ void __launch_bounds__(kVThreads, kCBlocks) commit_tc_kernel(const __
             for (int e = t; e < DV * DK; e += kVThreads) dst[e] = *reinterpret_cast<const uint16_t*>(smem + cS + sw_elem(DV, e >> 7, e & 127));
         }
     }
+    if (t == 0) bulk_wait_all<0>();
     cp_async_wait<0>();
+    abort_pause(ctl);
     tc::fence_before_sync();
     __syncthreads();
     if (warp == 0) tc::tmem_dealloc(tm, kCCols);
@@ -963,6 +1029,7 @@ int core_verify_tc_launch(int32_t heads, int32_t batch, const int32_t* cu_rows, 
     p.cu = cu_rows;
     p.q = q; p.k = k; p.v = v; p.g = g; p.beta = beta;
     p.state = reinterpret_cast<const uint16_t*>(state_in);
+    p.mapped = state_map(&p.tm_state, state_in);
     p.state_off = reinterpret_cast<const long long*>(state_off);
     p.out = out;
     p.out_stride = (long long)heads * DV;
@@ -981,6 +1048,7 @@ int layer_verify_tc_launch(int32_t heads, int32_t batch, const int32_t* cu_rows,
     p.units = (long long)heads * batch;
     p.cu = cu_rows;
     p.state = reinterpret_cast<const uint16_t*>(state_in);
+    p.mapped = state_map(&p.tm_state, state_in);
     p.state_off = reinterpret_cast<const long long*>(state_off);
     p.out = out;
     p.out_stride = out_stride;
@@ -1008,6 +1076,7 @@ int commit_tc_launch(int32_t heads, int32_t layers, int32_t batch, const int32_t
     p.cu = cu_rows; p.keep = keep;
     p.state_in = reinterpret_cast<const uint16_t*>(state_in);
     p.state_out = reinterpret_cast<uint16_t*>(state_out);
+    p.mapped = state_map(&p.tm_in, state_in) && state_map(&p.tm_out, state_out);
     p.state_stride = state_stride;
     p.state_off = reinterpret_cast<const long long*>(state_off);
     p.k_save = k_save; p.v_save = v_save; p.g_save = g_save; p.b_save = b_save;
