@@ -261,8 +261,9 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
                 amax = fmaxf(amax, av);
                 *reinterpret_cast<float*>(col + r * 128 + ((pc ^ (r & 7)) << 4)) = av;
             }
-            // Eight rows of decay must stay below e^85: per-row log decays below about -10.6 (or positive ones) do not.
-            if (!(amax < 1e37f)) atomicCAS(p.status, 0, kStatusPrefillRange);
+            // Eight rows of decay must stay below e^85: per-row log decays below about -10.6 (or positive ones) do not.  (Behind the
+            // middle the factors stop at 2^-126; a block's last row is the first to.)
+            if (!(amax < 1e37f) || run[15] - run[8] < -126.0f || run[31] - run[24] < -126.0f) atomicCAS(p.status, 0, kStatusPrefillRange);
             group_sync();
             const float base1 = tmp[d];
             const float gm0 = tmp[2 * 128 + d], gm1 = tmp[3 * 128 + d], gm2 = base1 + tmp[4 * 128 + d], gm3 = base1 + tmp[5 * 128 + d];

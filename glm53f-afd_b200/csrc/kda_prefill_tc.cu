@@ -276,7 +276,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1) prefill_tc_kernel(const __grid_
                 *reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(col) + r * RS32) = av;
             }
             // Eight rows of decay must stay below e^85: per-row log decays below about -10.6 (or positive ones) do not.
-            if (!(amax < 1e37f)) atomicCAS(p.status, 0, kStatusPrefillRange);
+            if (!(amax < 1e37f) || loc[15] - loc[8] < -126.0f) atomicCAS(p.status, 0, kStatusPrefillRange);
             compute_sync();
             float start[5];  // G before each block's first row, and after the last row
             start[0] = 0.0f;

@@ -176,6 +176,8 @@ struct Factors {
         a = {upper ? p.x : r.x, upper ? p.y : r.y};
         inva = {upper ? r.x : p.x, upper ? r.y : p.y};
     }
+    // Whether the last rows' factors have stopped there: more decay than the products can be split for.
+    __device__ __forceinline__ bool lost() const { return upper && (between[WIN / 2 - 1].x < 0x1p-126f || between[WIN / 2 - 1].y < 0x1p-126f); }
     __device__ __forceinline__ float2 from_start(int s) const {  // exp(G)
         const float2 x = mul2(beyond, between[s]);
         return {upper ? x.x : out[s].x, upper ? x.y : out[s].y};
@@ -463,7 +465,7 @@ __global__ void __launch_bounds__(kVThreads, 3) verify_tc_kernel(const __grid_co
             all_rows(kgp, upper, kg);
 #pragma unroll
             for (int r = 0; r < WIN; ++r) vv[r] = bf16_bits_to_f32(reinterpret_cast<const uint16_t*>(raw + R::V)[r * DK + t]);
-            if (!(amax < 1e37f)) atomicCAS(p.status, 0, kStatusPrefillRange);
+            if (!(amax < 1e37f) || fac.lost()) atomicCAS(p.status, 0, kStatusPrefillRange);
             if (t < WIN) {
                 const float bt = reinterpret_cast<const float*>(raw + R::B)[t];
                 betas[t] = bt;
@@ -832,7 +834,7 @@ __global__ void __launch_bounds__(kVThreads, kCBlocks) commit_tc_kernel(const __
                 all_rows(kgp, upper, kg);
 #pragma unroll
                 for (int r = 0; r < WIN; ++r) vv[r] = r < nr ? bf16_bits_to_f32(reinterpret_cast<const uint16_t*>(smem + cRawV)[r * DV + t]) : 0.0f;
-                if (!(amax < 1e37f)) atomicCAS(p.status, 0, kStatusPrefillRange);
+                if (!(amax < 1e37f) || fac.lost()) atomicCAS(p.status, 0, kStatusPrefillRange);
                 if (t < WIN) betas[t] = bt;
             }
             fence_proxy_async_smem();

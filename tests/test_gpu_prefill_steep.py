@@ -38,3 +38,26 @@ def test_steep_blocks(decay, workspace):
     # bf16 operands: the bound of the other chunked prefill tests, 1e-2 of the norm; a lost pair is 0.9 of its row
     assert (got - want).norm() <= 1e-2 * want.norm()
     assert (state.view(heads, DK, DK).double().cpu() - s).norm() <= 2e-3 * s.norm()
+
+
+@pytest.mark.parametrize("decay, status", [(-12.0, 0), (-13.0, 121)])
+@pytest.mark.parametrize("kind", ["single pass", "workspace", "verify"])
+def test_decay_behind_a_middle_row(kind, decay, status):
+    """Seven rows behind a block's middle row: e^-84 can be split into factors, e^-91 cannot and is reported."""
+    core = importlib.import_module("glm53f-afd_b200.core")
+    heads, rows, gen = 2, 16 if kind == "verify" else 70, torch.Generator(device="cuda").manual_seed(6)
+    n = rows * heads * DK
+    rn = lambda m, s=1.0: (torch.randn(m, device="cuda", generator=gen) * s)
+    q, k, v, beta = rn(n, 0.01).bfloat16(), rn(n, 0.08).bfloat16(), rn(n).bfloat16(), torch.sigmoid(rn(rows * heads))
+    g = torch.full((rows, heads * DK), -0.1, device="cuda")
+    g[9:16] = decay
+    cu, off, out = torch.tensor([0, rows], dtype=torch.int32, device="cuda"), torch.zeros(1, dtype=torch.int64, device="cuda"), torch.zeros(n, dtype=torch.bfloat16, device="cuda")
+    if kind == "verify":
+        core.decode_batch(heads, rows, cu, q, k, v, g.view(-1), beta, rn(heads * DK * DK, 0.05).bfloat16(), off, state_out=None, flags=core.TENSOR, out=out)
+    else:
+        ws = torch.empty(core.prefill_workspace_bytes(heads, 1, 2), dtype=torch.uint8, device="cuda") if kind == "workspace" else None
+        core.prefill_varlen(heads, rows, cu, rows, q, k, v, g.view(-1), beta, torch.zeros(heads * DK * DK, device="cuda"), off, out=out, workspace=ws)
+    torch.cuda.synchronize()
+    assert core.device_status() == status
+    assert core.device_status() == 0
+    assert bool(torch.isfinite(out).all())
