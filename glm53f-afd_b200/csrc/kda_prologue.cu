@@ -13,7 +13,7 @@
 // sinks): one warp per (request, head, row).  The work is bound by instruction issue (about 850 instructions per row and lane,
 // most of them IEEE divisions and exponentials), so a warp takes ONE row and reads its three predecessors again (the four warps of a block take four
 // consecutive rows; the predecessors come from L1/L2): every load of a warp is in flight at once and 79 registers
-// allow 24 resident warps per SM.  (A warp that walks 16 rows with the three earlier rows sliding in registers needs
+// allow 24 resident warps per SM (72 and 28 in the exact sink: 701 rows 400.8 -> 397.3 us; the verify sink gains nothing by it).  (A warp that walks 16 rows with the three earlier rows sliding in registers needs
 // 143 registers and was half as fast.)
 //
 // Three sinks:
@@ -111,7 +111,7 @@ __device__ __forceinline__ uint2 load4(const uint16_t* at) {
 __device__ __forceinline__ bool unaligned8(const void* at) { return (reinterpret_cast<uintptr_t>(at) & 7) != 0; }
 
 template <int SINK>
-__global__ void __launch_bounds__(128, 6) layer_prologue_kernel(const ProParams p) {
+__global__ void __launch_bounds__(128, SINK == kExact ? 7 : 6) layer_prologue_kernel(const ProParams p) {
     constexpr bool VERIFY = SINK == kVerify, EXACT = SINK == kExact;
     grid_ready();
     const int lane = threadIdx.x & 31, H = p.H;
@@ -215,7 +215,8 @@ __global__ void __launch_bounds__(128, 6) layer_prologue_kernel(const ProParams 
 // ---- the prefill sink ---------------------------------------------------------------------------------------------------
 // Bound by instruction issue before it is bound by memory (a row and head: 1 KiB in, 1.3 KiB out).  A warp takes four consecutive
 // rows: seven rows of inputs instead of sixteen, the weights once, and everything in pairs of channels (two-wide multiply-adds).
-// 1,280 rows x 64 heads: 79 us with a warp per row as in the kernel above, 52 so with four blocks an SM; five take another 4 us off a pass of the whole call.
+// 1,280 rows x 64 heads: 79 us with a warp per row as in the kernel above, 52 so with four blocks an SM; five take another 4 us off a pass of the whole call, and six, at 80 registers now that exponentials are single
+// instructions, 3 more (4 x 2,048 rows 941 -> 923 us, 3 x 700 246 -> 238); seven spill (244).
 constexpr int kRowsPer = 4;
 __device__ __forceinline__ float2 lo_hi(uint32_t w) { return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)); }
 __device__ __forceinline__ float2 add2(float2 a, float2 b) { return fma2(a, {1.0f, 1.0f}, b); }
@@ -231,7 +232,7 @@ __device__ __forceinline__ uint32_t fp16x2(float2 x) {
 
 // FIRST: the pass with the requests' first rows, which reach back into the conv windows.
 template <bool FIRST>
-__global__ void __launch_bounds__(128, 5) prefill_prologue_kernel(const ProParams p) {
+__global__ void __launch_bounds__(128, 6) prefill_prologue_kernel(const ProParams p) {
     const int lane = threadIdx.x & 31, H = p.H, groups = p.pass_rows / (4 * kRowsPer), c0 = lane * 4;
     // heads innermost: neighbouring blocks read neighbouring pieces of the same rows
     const int h = (int)(blockIdx.x % H), b = (int)(blockIdx.x / H / groups), j0 = (int)(blockIdx.x / H % groups) * 4 * kRowsPer + (threadIdx.x >> 5) * kRowsPer;
