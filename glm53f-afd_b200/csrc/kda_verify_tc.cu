@@ -141,7 +141,7 @@ __device__ __forceinline__ int sw_elem(int R, int r, int c) {
 }
 // The output gate: these outputs carry the rounding of bf16 operands already, so the hardware's approximate exponential
 // and division do (the file's other divisions and exponentials keep IEEE arithmetic for the replay saves).
-__device__ __forceinline__ float sigmoid_(float x) { return __fdividef(1.0f, 1.0f + __expf(-x)); }
+__device__ __forceinline__ float sigmoid_(float x) { return rcp_approx(1.0f + ex2_ftz(-kLog2e * x)); }
 
 // The operand tiles are made two channels and eight rows a thread, outwards from the chunk's middle: lanes 0-15 have rows 7, 6, .. 0, lanes
 // 16-31 rows 8, 9, .. 15.  Four-byte shared-memory accesses, packed conversions.  What a lane of the other half holds:
@@ -557,6 +557,12 @@ __global__ void __launch_bounds__(kVThreads, 3) verify_tc_kernel(const __grid_co
         else cp_async_commit();
 
         // ---- E. D = U - W S,  O = Qg S + M D; thread = value channel = its tensor-memory lane -----------------------------------------
+        uint2 gate[4] = {};  // layer form: the gate values of the four rows that this warp normalises, on their way meanwhile
+        if constexpr (LAYER) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (warp * 4 + k < n) gate[k] = *reinterpret_cast<const uint2*>(p.gate + (un.row0 + warp * 4 + k) * p.gate_stride + (long long)un.h * DV + lane * 4);
+        }
         {
             uint32_t ws[16], qs[16];
             tc::tmem_ld16(tc::tmem_addr(tm, warp, 0), ws);
@@ -586,28 +592,33 @@ __global__ void __launch_bounds__(kVThreads, 3) verify_tc_kernel(const __grid_co
         if constexpr (LAYER) {
             // The gated RMSNorm (reference kda.cu:188-201): a warp takes four rows, a lane four value channels.
             __syncthreads();
+            float y[4][4], ss[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {  // (rows past the window: sums of numbers that nobody takes)
+                const float4 y4 = *reinterpret_cast<const float4*>(smem + vStage + ((warp * 4 + k) * DV + lane * 4) * 4);
+                y[k][0] = y4.x; y[k][1] = y4.y; y[k][2] = y4.z; y[k][3] = y4.w;
+                ss[k] = 0.0f;
+#pragma unroll
+                for (int x = 0; x < 4; ++x) ss[k] = ss[k] + y[k][x] * y[k][x];
+            }
+#pragma unroll
+            for (int o = 16; o; o >>= 1)
+#pragma unroll
+                for (int k = 0; k < 4; ++k) ss[k] = ss[k] + __shfl_xor_sync(0xffffffffu, ss[k], o);
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 const int i = warp * 4 + k;
                 if (i >= n) break;
-                const float4 y4 = *reinterpret_cast<const float4*>(smem + vStage + (i * DV + lane * 4) * 4);
-                const float y[4] = {y4.x, y4.y, y4.z, y4.w};
-                float ss = 0.0f;
-#pragma unroll
-                for (int x = 0; x < 4; ++x) ss = ss + y[x] * y[x];
-#pragma unroll
-                for (int o = 16; o; o >>= 1) ss = ss + __shfl_xor_sync(0xffffffffu, ss, o);
-                const float rinv = rsqrtf(ss * (1.0f / (float)DV) + p.eps);
+                const float rinv = rsqrtf(ss[k] * (1.0f / (float)DV) + p.eps);
                 const long long gr = un.row0 + i;
-                const uint2 gw = *reinterpret_cast<const uint2*>(p.gate + gr * p.gate_stride + (long long)un.h * DV + lane * 4);
-                const float gt[4] = {__uint_as_float(gw.x << 16), __uint_as_float(gw.x & 0xffff0000u), __uint_as_float(gw.y << 16),
-                                     __uint_as_float(gw.y & 0xffff0000u)};
+                const float gt[4] = {__uint_as_float(gate[k].x << 16), __uint_as_float(gate[k].x & 0xffff0000u), __uint_as_float(gate[k].y << 16),
+                                     __uint_as_float(gate[k].y & 0xffff0000u)};
                 uint32_t o2[2];
 #pragma unroll
                 for (int x = 0; x < 2; ++x) {
-                    const float lo = (nw[2 * x] * (y[2 * x] * rinv)) * sigmoid_(gt[2 * x]);
-                    const float hi = (nw[2 * x + 1] * (y[2 * x + 1] * rinv)) * sigmoid_(gt[2 * x + 1]);
-                    o2[x] = (uint32_t)f32_to_bf16_bits(lo) | ((uint32_t)f32_to_bf16_bits(hi) << 16);
+                    const float lo = (nw[2 * x] * (y[k][2 * x] * rinv)) * sigmoid_(gt[2 * x]);
+                    const float hi = (nw[2 * x + 1] * (y[k][2 * x + 1] * rinv)) * sigmoid_(gt[2 * x + 1]);
+                    o2[x] = tc::bf16x2(lo, hi);
                 }
                 *reinterpret_cast<uint2*>(p.out + gr * p.out_stride + (long long)un.h * DV + lane * 4) = make_uint2(o2[0], o2[1]);
             }
