@@ -75,7 +75,8 @@ int core_prefill_tc_launch(int32_t heads, int32_t batch, const int32_t* cu_seqle
                            float eps, glm53f_bf16* out, cudaStream_t stream);
 
 // Draft verification as one 16-row chunk on the tensor cores (kda_verify_tc.cu): bf16 states, read only; outputs to the
-// rounding of bf16 operands, replay saves as the exact path writes them.  q, k, v, g must be 16-byte aligned.
+// rounding of bf16 operands, replay saves as the exact path writes them.  q, k, v, g must be 16-byte aligned; states, outputs
+// and saves may lie at any element.
 int core_verify_tc_launch(int32_t heads, int32_t batch, const int32_t* cu_rows, const glm53f_bf16* q, const glm53f_bf16* k,
                           const glm53f_bf16* v, const float* g, const float* beta, const void* state_in, const int64_t* state_off,
                           glm53f_bf16* out, float* k_save, glm53f_bf16* v_save, float* g_save, float* b_save, cudaStream_t stream);

@@ -390,14 +390,19 @@ __global__ void __launch_bounds__(kVThreads, 3) verify_tc_kernel(const __grid_co
 
     const bool vec_saves = ((reinterpret_cast<uintptr_t>(p.k_save) | reinterpret_cast<uintptr_t>(p.g_save) | reinterpret_cast<uintptr_t>(p.v_save)) & 15) == 0;
     // The core form's outputs leave sixteen bytes a thread (two bytes a thread, sixteen stores each, held up whatever came after them),
-    // behind the next unit's first barrier.
+    // behind the next unit's first barrier.  An output buffer off 16 bytes takes them two bytes a thread, a row at a time.
+    const bool vec_out = (reinterpret_cast<uintptr_t>(p.out) & 15) == 0;
     long long out_at = 0;
     int out_n = 0;
     auto out_rows = [&] {
+        if (vec_out) {
 #pragma unroll
-        for (int i = 0; i < WIN / 8; ++i) {
-            const int r = (t >> 4) + 8 * i, c = (t & 15) * 8;
-            if (r < out_n) *reinterpret_cast<uint4*>(p.out + out_at + (long long)r * p.H * DV + c) = *reinterpret_cast<const uint4*>(smem + MP::vOut + (r * DV + c) * 2);
+            for (int i = 0; i < WIN / 8; ++i) {
+                const int r = (t >> 4) + 8 * i, c = (t & 15) * 8;
+                if (r < out_n) *reinterpret_cast<uint4*>(p.out + out_at + (long long)r * p.H * DV + c) = *reinterpret_cast<const uint4*>(smem + MP::vOut + (r * DV + c) * 2);
+            }
+        } else {
+            for (int r = 0; r < out_n; ++r) p.out[out_at + (long long)r * p.H * DV + t] = reinterpret_cast<const uint16_t*>(smem + MP::vOut)[r * DV + t];
         }
     };
     Units units(p);
@@ -1031,8 +1036,8 @@ int launch_verify(const VParams& p, cudaStream_t stream) {
 
 }  // namespace
 
-// The chunked verify of the core entry point: bf16 states, no state written, no fused norm, 16-byte aligned rows (the
-// caller checks).
+// The chunked verify of the core entry point: bf16 states, no state written, no fused norm, q, k, v and g on 16 bytes (the
+// caller checks); states, outputs and saves at any element.
 int core_verify_tc_launch(int32_t heads, int32_t batch, const int32_t* cu_rows, const glm53f_bf16* q, const glm53f_bf16* k,
                           const glm53f_bf16* v, const float* g, const float* beta, const void* state_in, const int64_t* state_off,
                           glm53f_bf16* out, float* k_save, glm53f_bf16* v_save, float* g_save, float* b_save, cudaStream_t stream) {
