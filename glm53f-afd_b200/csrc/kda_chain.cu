@@ -1411,7 +1411,12 @@ int core_entry(int32_t heads, int32_t batch, const int32_t* cu_rows, const glm53
         return e == nullptr ? 0 : (strcmp(e, "pipeline") == 0 ? 1 : (strcmp(e, "small") == 0 ? 2 : 0));
     }();
     const long long sms = sm_count();
-    const bool small = forced == 2 || (forced == 0 && (k_save != nullptr || (x.units > sms && x.units <= 2 * sms)));
+    // A unit's two small blocks read all of a row's q and k each, and for the saves one of them all of v, and neither waits for the other before
+    // it stores its half of the outputs: outputs over these rows stay on the persistent kernel, where one block has the unit.  Outputs
+    // over other rows' inputs meet other units' on any kernel, except those of a single request over its earlier rows.
+    const bool over_inputs = out == q || out == k || (k_save != nullptr && out == v);
+    const bool two_units = x.units > sms && x.units <= 2 * sms && batch > 1;
+    const bool small = !over_inputs && (forced == 2 || (forced == 0 && (k_save != nullptr || two_units)));
     if (small && flags == 0 && gate == nullptr && x.units * kSmallParts <= 0x7fffffffll)
         return state_bf16 != 0 ? launch_small<__nv_bfloat16>(x, (cudaStream_t)stream) : launch_small<float>(x, (cudaStream_t)stream);
     return launch_typed<kCore>(x, state_bf16 != 0, (cudaStream_t)stream);
