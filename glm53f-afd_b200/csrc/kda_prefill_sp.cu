@@ -728,7 +728,8 @@ __device__ __forceinline__ int state_bar_count(int i) {
 }
 static_assert(kStateBars * 8 <= oChain - oBarsState && oChain % 16 == 0, "state role barriers");
 
-// Waits until a count in global memory has reached `want`; gives up when it has stood still for the waits' limit.
+// Waits until a count in global memory has reached `want`; gives up when it has stood still for the waits' limit.  As long as it rises, the
+// block's other warps, which wait for what follows, are told of progress, so that their limit is no shorter.
 __device__ __forceinline__ bool count_wait(const unsigned int* at, unsigned want, const WaitCtx& ctx, int code) {
     unsigned seen = 0;
     uint64_t t0 = global_timer_ns();
@@ -740,6 +741,7 @@ __device__ __forceinline__ bool count_wait(const unsigned int* at, unsigned want
         if (v != seen) {
             seen = v;
             t0 = now;
+            atomicAdd(const_cast<uint32_t*>(ctx.progress), 1u);
         } else if (now - t0 > ctx.limit_ns) {
             atomicCAS(ctx.status, 0, code);
             return false;
