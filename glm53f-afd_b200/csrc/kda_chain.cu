@@ -986,11 +986,15 @@ __global__ void __launch_bounds__(kThreadsOf<S, MODE, ONE_UNIT>, 1) recurrent_ke
 // warp, which never interact with the others -- loads that part of the state straight from global memory into registers, cooks
 // each row's inputs itself (128 threads, one channel each: widen q, k, v, exp of the log decay, beta; loaded a row ahead, into the other
 // of two buffers, so a row takes one barrier), steps through the request's rows and stores its rows of the state back.  No rings, no
-// bulk copies: four such blocks on an SM are two units' serial rows at once.  Used for the exact verify; single-row decode runs on the
-// persistent kernel above (core_entry).
+// bulk copies: four such blocks on an SM are two units' serial rows at once.  Used for the exact verify and, with more than one and at
+// most two units an SM, for decode of any number of rows, the row-by-row fallback of the core prefill among it (core_entry).
 constexpr int kSmallWarps = 4, kSmallThreads = kSmallWarps * 32, kR = 4, kSmallParts = DV / (4 * kR * kSmallWarps), kSmallPerSm = 4;
 
-template <typename S>
+// DECODE: calls without saves.  A unit's halves are neighbours, which read the same rows; in a verify so are a request's units, in a decode
+// those of different requests (a grid of heads by requests): neighbouring blocks share an SM when there are four for each, and one long
+// request among single rows had its blocks on a few (288 units, one of 18 requests with 40 rows, 34 launches: bf16 2,465 -> 1,485 us, f32
+// 2,244 -> 1,320).
+template <typename S, bool DECODE>
 __global__ void __launch_bounds__(kSmallThreads, kSmallPerSm) core_small_kernel(const __grid_constant__ Params p) {
     __shared__ __align__(16) float sq[2][DK], sk[2][DK], sg[2][DK], sv[2][DV];
     __shared__ float sbeta[2];
@@ -999,7 +1003,7 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallPerSm) core_small_kernel(
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     const long long unit = blockIdx.x / kSmallParts;
     const int part = blockIdx.x % kSmallParts, uw = part * kSmallWarps + warp;  // this warp's place among the unit's
-    const int b = (int)(unit / p.H), h = (int)(unit % p.H);
+    const int b = (int)(DECODE ? unit : unit / p.H), h = (int)(DECODE ? blockIdx.y : unit % p.H);
     const int r0 = p.cu_rows[b], rows = max(p.cu_rows[b + 1] - r0, 0);
     const bool writes = p.state_out != nullptr;
     if (rows == 0 && !copies_state(p)) return;
@@ -1034,7 +1038,7 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallPerSm) core_small_kernel(
         sg[buf][t] = gf;
         sv[buf][t] = bf16_bits_to_f32(next.v);
         if (t == 0) sbeta[buf] = next.beta;
-        if (p.k_save != nullptr && part == 0) {
+        if (!DECODE && part == 0) {
             p.k_save[at] = kf;
             p.g_save[at] = gf;
             p.v_save[at] = next.v;
@@ -1064,14 +1068,15 @@ int launch_small(const Params& p, cudaStream_t stream) {
     Params q = p;
     q.neg_zero2 = 0x8000000080000000ull;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(p.units * kSmallParts));
+    const bool decode = p.k_save == nullptr;
+    cfg.gridDim = decode ? dim3((unsigned)(p.units / p.H * kSmallParts), (unsigned)p.H) : dim3((unsigned)(p.units * kSmallParts));
     cfg.blockDim = dim3(kSmallThreads);
     cfg.dynamicSmemBytes = 0;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     cfg.attrs = attr;
     cfg.numAttrs = early_attribute(attr[0]);
-    return (int)cudaLaunchKernelEx(&cfg, core_small_kernel<S>, q);
+    return (int)cudaLaunchKernelEx(&cfg, decode ? core_small_kernel<S, true> : core_small_kernel<S, false>, q);
 }
 
 // ---- the replay on many small blocks ---------------------------------------------------------------------------
@@ -1403,8 +1408,10 @@ int core_entry(int32_t heads, int32_t batch, const int32_t* cu_rows, const glm53
     // 335 against 254).  Decode stays on the persistent kernel, which keeps more bytes in flight (bf16, 16 slots 458 against 635 us, 48
     // slots 1,208 and 1,704; f32 single rows 845 and 786, 2,335 and 2,117, but windows of two rows 880 and 924), except with more than
     // one and at most two units an SM: some of its blocks have two then, one after the other, and the rest wait (single rows of 160,
-    // 192, 256 and 288 units, f32 287 -> 247 us for 34 launches, 300 -> 257, 318 -> 280, 324 -> 288, bf16 221 -> 197, 229 -> 205, 237 -> 215, 239 -> 220; windows
-    // of two to six rows 2 to 13 % less; at 320 units small blocks are the slower for bf16).  GLM53F_KDA_DECODE=pipeline / small forces one
+    // 192, 256 and 288 units, f32 285 -> 244 us for 34 launches, 301 -> 256, 319 -> 280, 325 -> 292, bf16 221 -> 195, 230 -> 201, 238 -> 210, 240 -> 215; windows
+    // of two to six rows 3 to 15 % less, of 16, 64 and 1,000 rows 9 to 19 %, one request of 40 rows among single ones 1 to 10 %; rows
+    // of four and one in turn 160 units up to 10 % more, 288 7 to 17 % less, half of the requests empty 1 to 5 % more where states are
+    // written; single rows of 320 units 372 -> 311 and 275 -> 287).  GLM53F_KDA_DECODE=pipeline / small forces one
     // or the other; the bits are the same either way.
     static const int forced = [] {
         const char* e = getenv("GLM53F_KDA_DECODE");
