@@ -180,8 +180,9 @@ constexpr uint32_t gcL = 0, gcM = 64, gcW = 0, gcU = 64, kGroupCols = 128;
 // LAYER: the items' inputs are in their slots (kda_internal.h), which the results then replace.  G = 0 or 1, a runtime value: both groups run the same instructions (one copy of this code in the instruction cache).
 template <bool LAYER, bool FUSED>
 __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* smem, const uint32_t tm_block, const WaitCtx& ctx, const int G) {
-    // The layer form's items take the block-wise branch, whose instructions are the most: there the issue loops stay loops (4 x 2,048 rows
-    // 985 -> 955 us), which on the one-product branch of the core form costs more than it saves (8,192 rows 480 -> 494).
+    // The issue loops stay loops in the layer form's instance and are unrolled in the core form's, whichever branch an item takes: 4 x 2,048
+    // rows of the layer form 972 -> 944 us as loops; the core form's 8,192 rows in 8 sequences 462 both ways with mild gates, 548 and 555 with
+    // strong ones, 32,768 rows in one sequence 1,968 and 1,995, 2,138 and 2,207.
     constexpr int kIssue = LAYER ? 1 : 8;
     const int BAR = 2 + G;
     unsigned char* gs = smem + G * kGroupBytes;
