@@ -402,12 +402,12 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
                     for (int k0 = 0; k0 < DK; k0 += 16)
                         tc::mma_bf16_if(leader, tm + gcL, tc::desc_sw128_kmajor(gs + gKb, CH, k0), tc::desc_sw128_kmajor(gs + gK, CH, k0), id64, k0 > 0);
             } else {
-            constexpr uint32_t id = tc::idesc_bf16(64, 16, 0, 0, 0);
-            const int I = gw;
-            const unsigned char* kct = gs + gKc + kc_tile(I);
+                constexpr uint32_t id = tc::idesc_bf16(64, 16, 0, 0, 0);
+                const int I = gw;
+                const unsigned char* kct = gs + gKc + kc_tile(I);
 #pragma unroll kIssue
-            for (int k0 = 0; k0 < DK; k0 += 16)
-                tc::mma_bf16_if(leader, tm + gcL + 16 * I, tc::desc_sw128_kmajor(kct, 16 * (I + 1), k0), tc::desc_sw128_kmajor(gs + gKb + I * 2048, CH, k0), id, k0 > 0);
+                for (int k0 = 0; k0 < DK; k0 += 16)
+                    tc::mma_bf16_if(leader, tm + gcL + 16 * I, tc::desc_sw128_kmajor(kct, 16 * (I + 1), k0), tc::desc_sw128_kmajor(gs + gKb + I * 2048, CH, k0), id, k0 > 0);
             }
             tc::mma_commit_if(leader, bar_lm);
             if (leader) atomicAdd(const_cast<uint32_t*>(ctx.progress), 1u);
@@ -444,12 +444,12 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
                     for (int k0 = 0; k0 < DK; k0 += 16)
                         tc::mma_bf16_if(leader, tm + gcM, tc::desc_sw128_kmajor(gs + gKb, CH, k0), tc::desc_sw128_kmajor(gs + gQ, CH, k0), id64, k0 > 0);
             } else {
-            constexpr uint32_t id = tc::idesc_bf16(64, 16, 0, 0, 0);
-            const int I = gw - 4;
-            const unsigned char* kct = gs + gKc + kc_tile(I);
+                constexpr uint32_t id = tc::idesc_bf16(64, 16, 0, 0, 0);
+                const int I = gw - 4;
+                const unsigned char* kct = gs + gKc + kc_tile(I);
 #pragma unroll kIssue
-            for (int k0 = 0; k0 < DK; k0 += 16)
-                tc::mma_bf16_if(leader, tm + gcM + 16 * I, tc::desc_sw128_kmajor(kct, 16 * (I + 1), k0), tc::desc_sw128_kmajor(gs + gQ + I * 2048, CH, k0), id, k0 > 0);
+                for (int k0 = 0; k0 < DK; k0 += 16)
+                    tc::mma_bf16_if(leader, tm + gcM + 16 * I, tc::desc_sw128_kmajor(kct, 16 * (I + 1), k0), tc::desc_sw128_kmajor(gs + gQ + I * 2048, CH, k0), id, k0 > 0);
             }
             tc::mma_commit_if(leader, bar_lm);
             if (leader) atomicAdd(const_cast<uint32_t*>(ctx.progress), 1u);
@@ -905,37 +905,37 @@ __device__ void state_role(const SpParams& p, unsigned char* smem, const uint32_
         // chunk by the warp's own stores, so that no row beyond the sequence is touched.
         bool alive = wk.emit;
         for (int seq = 0, C = 0; alive; ++seq) {
-        const int count = chain_count(seq);
-        if (count < 0) break;
-        const int rows = recs[seq & 1].rows, h = recs[seq & 1].h;
-        const long long row = recs[seq & 1].row;
-        release(seq);
-        for (int c = 0; c < count; ++c, ++C) {
-            const int n = min(CH, rows - c * CH);
-            const long long gr0 = row + (long long)c * CH;
-            if (!wait(bOutFull + (C & 1), C >> 1)) { alive = false; break; }
-            const unsigned char* tile = smem + sOut + (C & 1) * kOutTile;
-            if (n == CH) {
-                if (lane == 0) {
-                    for (int x = 0; x < 2; ++x) {
-                        if (p.out != nullptr) tensor_store_3d(&p.tm_out, x * 64, h, (int)gr0, tile + x * kBox);
-                        for (int pe = 0; pe < p.ranks; ++pe) tensor_store_3d(&p.tm_full[pe], x * 64, p.head0 + h, (int)gr0, tile + x * kBox);
+            const int count = chain_count(seq);
+            if (count < 0) break;
+            const int rows = recs[seq & 1].rows, h = recs[seq & 1].h;
+            const long long row = recs[seq & 1].row;
+            release(seq);
+            for (int c = 0; c < count; ++c, ++C) {
+                const int n = min(CH, rows - c * CH);
+                const long long gr0 = row + (long long)c * CH;
+                if (!wait(bOutFull + (C & 1), C >> 1)) { alive = false; break; }
+                const unsigned char* tile = smem + sOut + (C & 1) * kOutTile;
+                if (n == CH) {
+                    if (lane == 0) {
+                        for (int x = 0; x < 2; ++x) {
+                            if (p.out != nullptr) tensor_store_3d(&p.tm_out, x * 64, h, (int)gr0, tile + x * kBox);
+                            for (int pe = 0; pe < p.ranks; ++pe) tensor_store_3d(&p.tm_full[pe], x * 64, p.head0 + h, (int)gr0, tile + x * kBox);
+                        }
+                        bulk_commit();
+                        bulk_wait_read<0>();  // the tile has been read: the compute warps may refill it
                     }
-                    bulk_commit();
-                    bulk_wait_read<0>();  // the tile has been read: the compute warps may refill it
+                } else {
+                    for (int e = lane; e < n * 16; e += 32) {
+                        const int r = e >> 4, piece = e & 15;
+                        const uint4 v4 = *reinterpret_cast<const uint4*>(tile + box_piece(r, piece));
+                        if (p.out != nullptr) *reinterpret_cast<uint4*>(p.out + ((gr0 + r) * p.H + h) * DV + piece * 8) = v4;
+                        const long long at_full = ((gr0 + r) * p.heads_total + p.head0 + h) * DV + piece * 8;
+                        for (int pe = 0; pe < p.ranks; ++pe) *reinterpret_cast<uint4*>(p.full[pe] + at_full) = v4;
+                    }
                 }
-            } else {
-                for (int e = lane; e < n * 16; e += 32) {
-                    const int r = e >> 4, piece = e & 15;
-                    const uint4 v4 = *reinterpret_cast<const uint4*>(tile + box_piece(r, piece));
-                    if (p.out != nullptr) *reinterpret_cast<uint4*>(p.out + ((gr0 + r) * p.H + h) * DV + piece * 8) = v4;
-                    const long long at_full = ((gr0 + r) * p.heads_total + p.head0 + h) * DV + piece * 8;
-                    for (int pe = 0; pe < p.ranks; ++pe) *reinterpret_cast<uint4*>(p.full[pe] + at_full) = v4;
-                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&bars[bOutEmpty + (C & 1)]);
             }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&bars[bOutEmpty + (C & 1)]);
-        }
         }
         if (lane == 0) bulk_wait_all<0>();
         tc::fence_before_sync();
@@ -1037,47 +1037,47 @@ __device__ void state_role(const SpParams& p, unsigned char* smem, const uint32_
         bool alive = true;
         int C = 0;
         for (int seq = 0; alive; ++seq) {
-        const int count = chain_count(seq);
-        if (!tc::warp_all(count >= 0)) break;
-        release(seq);
-        for (int c = 0; tc::warp_all(c < count); ++c, ++C) {
-            alive = false;
-            const int x = C & 1;
-            const uint32_t acc = tm + tO + (uint32_t)x * 64;
-            const unsigned char *qw = smem + sQW + x * kQW, *mm = smem + sMKd + x * kMKd, *kdhi = mm + kTile / 2, *kdlo = kdhi + kTile;
-            if (!ready(bFullQW + x, C >> 1) || !ready(bS16, C)) break;
-            tc::fence_after_sync();
-#pragma unroll
-            for (int k0 = 0; k0 < DK; k0 += 16)
-                tc::mma_bf16_ts_if(leader, tm + tWS, tm + tS16 + k0 / 2, tc::desc_mnmajor_bf16(qw + kTile, DK, 0, k0), idw, k0 > 0);
-            tc::mma_commit_if(leader, &bars[bWS]);
-            if (wk.emit) {
-                if (C >= 2 && !ready(bOFree + x, (C >> 1) - 1)) break;  // chunk C - 2's outputs have left this accumulator
+            const int count = chain_count(seq);
+            if (!tc::warp_all(count >= 0)) break;
+            release(seq);
+            for (int c = 0; tc::warp_all(c < count); ++c, ++C) {
+                alive = false;
+                const int x = C & 1;
+                const uint32_t acc = tm + tO + (uint32_t)x * 64;
+                const unsigned char *qw = smem + sQW + x * kQW, *mm = smem + sMKd + x * kMKd, *kdhi = mm + kTile / 2, *kdlo = kdhi + kTile;
+                if (!ready(bFullQW + x, C >> 1) || !ready(bS16, C)) break;
                 tc::fence_after_sync();
 #pragma unroll
                 for (int k0 = 0; k0 < DK; k0 += 16)
-                    tc::mma_bf16_ts_if(leader, acc, tm + tS16 + k0 / 2, tc::desc_kmajor_bf16(qw, CH, 0, k0), idq, k0 > 0);
+                    tc::mma_bf16_ts_if(leader, tm + tWS, tm + tS16 + k0 / 2, tc::desc_mnmajor_bf16(qw + kTile, DK, 0, k0), idw, k0 > 0);
+                tc::mma_commit_if(leader, &bars[bWS]);
+                if (wk.emit) {
+                    if (C >= 2 && !ready(bOFree + x, (C >> 1) - 1)) break;  // chunk C - 2's outputs have left this accumulator
+                    tc::fence_after_sync();
+#pragma unroll
+                    for (int k0 = 0; k0 < DK; k0 += 16)
+                        tc::mma_bf16_ts_if(leader, acc, tm + tS16 + k0 / 2, tc::desc_kmajor_bf16(qw, CH, 0, k0), idq, k0 > 0);
+                }
+                tc::mma_commit_if(leader, &bars[bEmptyQW + x]);
+                if (!ready(bFullMKd + x, C >> 1) || !ready(bSDec, C) || !ready(bD, C)) break;
+                tc::fence_after_sync();
+#pragma unroll
+                for (int k0 = 0; k0 < CH; k0 += 16) tc::mma_bf16_ts_if(leader, tm + tS, tm + tDhi + k0 / 2, tc::desc_mnmajor_bf16(kdhi, CH, 0, k0), ids, true);
+#pragma unroll
+                for (int k0 = 0; k0 < CH; k0 += 16) tc::mma_bf16_ts_if(leader, tm + tS, tm + tDlo + k0 / 2, tc::desc_mnmajor_bf16(kdhi, CH, 0, k0), ids, true);
+#pragma unroll
+                for (int k0 = 0; k0 < CH; k0 += 16) tc::mma_bf16_ts_if(leader, tm + tS, tm + tDhi + k0 / 2, tc::desc_mnmajor_bf16(kdlo, CH, 0, k0), ids, true);
+                tc::mma_commit_if(leader, &bars[bSNew]);
+                if (wk.emit) {
+#pragma unroll
+                    for (int k0 = 0; k0 < CH; k0 += 16) tc::mma_bf16_ts_if(leader, acc, tm + tDhi + k0 / 2, tc::desc_mnmajor_bf16(mm, CH, 0, k0), idw, true);
+                    tc::mma_commit_if(leader, &bars[bO + x]);
+                }
+                tc::mma_commit_if(leader, &bars[bEmptyMKd + x]);
+                if (leader) atomicAdd(const_cast<uint32_t*>(ctl), 1u);
+                __syncwarp();
+                alive = true;
             }
-            tc::mma_commit_if(leader, &bars[bEmptyQW + x]);
-            if (!ready(bFullMKd + x, C >> 1) || !ready(bSDec, C) || !ready(bD, C)) break;
-            tc::fence_after_sync();
-#pragma unroll
-            for (int k0 = 0; k0 < CH; k0 += 16) tc::mma_bf16_ts_if(leader, tm + tS, tm + tDhi + k0 / 2, tc::desc_mnmajor_bf16(kdhi, CH, 0, k0), ids, true);
-#pragma unroll
-            for (int k0 = 0; k0 < CH; k0 += 16) tc::mma_bf16_ts_if(leader, tm + tS, tm + tDlo + k0 / 2, tc::desc_mnmajor_bf16(kdhi, CH, 0, k0), ids, true);
-#pragma unroll
-            for (int k0 = 0; k0 < CH; k0 += 16) tc::mma_bf16_ts_if(leader, tm + tS, tm + tDhi + k0 / 2, tc::desc_mnmajor_bf16(kdlo, CH, 0, k0), ids, true);
-            tc::mma_commit_if(leader, &bars[bSNew]);
-            if (wk.emit) {
-#pragma unroll
-                for (int k0 = 0; k0 < CH; k0 += 16) tc::mma_bf16_ts_if(leader, acc, tm + tDhi + k0 / 2, tc::desc_mnmajor_bf16(mm, CH, 0, k0), idw, true);
-                tc::mma_commit_if(leader, &bars[bO + x]);
-            }
-            tc::mma_commit_if(leader, &bars[bEmptyMKd + x]);
-            if (leader) atomicAdd(const_cast<uint32_t*>(ctl), 1u);
-            __syncwarp();
-            alive = true;
-        }
         }
         // Nobody else waits for the last two chunks' buffers.
         for (int c = max(C - 2, 0); c < C; ++c)
@@ -1283,82 +1283,82 @@ __device__ void state_role(const SpParams& p, unsigned char* smem, const uint32_
         return emit_due();
     };
     for (int seq = 0;; ++seq) {
-    const int count = chain_count(seq);
-    if (MANY) {
-        if (!named_bar_all(4 + cg, 128, count != -2)) { alive = false; break; }
-    } else if (count == -2) { leave(); break; }
-    if (count < 0) break;
-    state_in(recs[seq & 1].start, recs[seq & 1].s_elem);
-    // A sequence of no rows has no D to wait for, and the output warp, which has to read its record too, may wait for these.
-    if (count == 0 && held >= 0) {
-        if (due >= 0 && !emit_last()) break;
-        release(held);
-        held = -1;
-    }
-    if (count > 0 && !begin_chunk(C)) { leave(); break; }
-    for (int c = 0; c < count; ++c, ++C) {
-        // ---- D^T = U^T - (W S)^T as bf16 hi + lo pairs of rows ------------------------------------------------------------
-        float uu[16];
-        if (votes && due >= 0 && !out_boxes()) fetch_gate(recs[due_seq & 1], due);
-        if (!wait(bFullU, C)) { leave(); break; }
-#pragma unroll
-        for (int x = 0; x < 4; ++x) {
-            const float4 u4 = *reinterpret_cast<const float4*>(smem + sU + u_cell(cg * 4 + x, v));
-            uu[4 * x] = wk.use_u ? u4.x : 0.0f; uu[4 * x + 1] = wk.use_u ? u4.y : 0.0f; uu[4 * x + 2] = wk.use_u ? u4.z : 0.0f; uu[4 * x + 3] = wk.use_u ? u4.w : 0.0f;
+        const int count = chain_count(seq);
+        if (MANY) {
+            if (!named_bar_all(4 + cg, 128, count != -2)) { alive = false; break; }
+        } else if (count == -2) { leave(); break; }
+        if (count < 0) break;
+        state_in(recs[seq & 1].start, recs[seq & 1].s_elem);
+        // A sequence of no rows has no D to wait for, and the output warp, which has to read its record too, may wait for these.
+        if (count == 0 && held >= 0) {
+            if (due >= 0 && !emit_last()) break;
+            release(held);
+            held = -1;
         }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&bars[bEmptyU]);  // U is consumed
-        if (!wait(bWS, C)) { leave(); break; }
-        tc::fence_after_sync();
-        {
-            uint32_t r[16], wh[8], wl[8];
-            tc::tmem_ld16(tc::tmem_addr(tm, quad, tWS + i0), r);
-            tc::tmem_ld_wait();
+        if (count > 0 && !begin_chunk(C)) { leave(); break; }
+        for (int c = 0; c < count; ++c, ++C) {
+            // ---- D^T = U^T - (W S)^T as bf16 hi + lo pairs of rows ------------------------------------------------------------
+            float uu[16];
+            if (votes && due >= 0 && !out_boxes()) fetch_gate(recs[due_seq & 1], due);
+            if (!wait(bFullU, C)) { leave(); break; }
 #pragma unroll
-            for (int x = 0; x < 8; ++x) tc::split_bf16x2(uu[2 * x] - __uint_as_float(r[2 * x]), uu[2 * x + 1] - __uint_as_float(r[2 * x + 1]), wh[x], wl[x]);
-            tc::tmem_st8(tc::tmem_addr(tm, quad, tDhi + i0 / 2), wh);
-            tc::tmem_st8(tc::tmem_addr(tm, quad, tDlo + i0 / 2), wl);
-            tc::tmem_st_wait();
-            arrive(bD);
-        }
-        // The outputs of the chunk before leave while the state's product runs.
-        if (due >= 0 && !emit_due()) break;
-        if (held >= 0) release(held);
-        held = -1;
-        if (wk.emit) due = c;
-        due_seq = seq;
-        if (!wait(bSNew, C)) { leave(); break; }
-        tc::fence_after_sync();
-        if (c + 1 < count && !begin_chunk(C + 1)) { leave(); break; }
-    }
-
-    // ---- the outgoing state ---------------------------------------------------------------------------------------------
-    if (!alive) break;
-    const long long s_out = recs[seq & 1].s_elem + b_at;
-    if (wk.fin != 2) {
-        const uint32_t from = tc::tmem_addr(tm, quad, tS + k_first);
-        uint16_t* to16 = reinterpret_cast<uint16_t*>(p.state_out) + s_out;
-        float* to32 = wk.fin == 1 ? wk.to + b_at : reinterpret_cast<float*>(p.state_out) + s_out;
-        const bool to_bf16 = wk.fin == 0 && p.state_bf16;
-        if (piece_aligned(to_bf16 ? (const void*)to16 : (const void*)to32)) {
-            if (to_bf16) state_from_tmem(from, to16 - lane * DK, lane);
-            else state_from_tmem(from, to32 - lane * DK, lane);
-        } else {
-#pragma unroll
-            for (int half = 0; half < 2; ++half) {
-                uint32_t r[16];
-                tc::tmem_ld16(from + half * 16, r);
+            for (int x = 0; x < 4; ++x) {
+                const float4 u4 = *reinterpret_cast<const float4*>(smem + sU + u_cell(cg * 4 + x, v));
+                uu[4 * x] = wk.use_u ? u4.x : 0.0f; uu[4 * x + 1] = wk.use_u ? u4.y : 0.0f; uu[4 * x + 2] = wk.use_u ? u4.z : 0.0f; uu[4 * x + 3] = wk.use_u ? u4.w : 0.0f;
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bars[bEmptyU]);  // U is consumed
+            if (!wait(bWS, C)) { leave(); break; }
+            tc::fence_after_sync();
+            {
+                uint32_t r[16], wh[8], wl[8];
+                tc::tmem_ld16(tc::tmem_addr(tm, quad, tWS + i0), r);
                 tc::tmem_ld_wait();
 #pragma unroll
-                for (int x = 0; x < 16; ++x) {
-                    if (to_bf16) to16[half * 16 + x] = f32_to_bf16_bits(__uint_as_float(r[x]));
-                    else to32[half * 16 + x] = __uint_as_float(r[x]);
+                for (int x = 0; x < 8; ++x) tc::split_bf16x2(uu[2 * x] - __uint_as_float(r[2 * x]), uu[2 * x + 1] - __uint_as_float(r[2 * x + 1]), wh[x], wl[x]);
+                tc::tmem_st8(tc::tmem_addr(tm, quad, tDhi + i0 / 2), wh);
+                tc::tmem_st8(tc::tmem_addr(tm, quad, tDlo + i0 / 2), wl);
+                tc::tmem_st_wait();
+                arrive(bD);
+            }
+            // The outputs of the chunk before leave while the state's product runs.
+            if (due >= 0 && !emit_due()) break;
+            if (held >= 0) release(held);
+            held = -1;
+            if (wk.emit) due = c;
+            due_seq = seq;
+            if (!wait(bSNew, C)) { leave(); break; }
+            tc::fence_after_sync();
+            if (c + 1 < count && !begin_chunk(C + 1)) { leave(); break; }
+        }
+
+        // ---- the outgoing state ---------------------------------------------------------------------------------------------
+        if (!alive) break;
+        const long long s_out = recs[seq & 1].s_elem + b_at;
+        if (wk.fin != 2) {
+            const uint32_t from = tc::tmem_addr(tm, quad, tS + k_first);
+            uint16_t* to16 = reinterpret_cast<uint16_t*>(p.state_out) + s_out;
+            float* to32 = wk.fin == 1 ? wk.to + b_at : reinterpret_cast<float*>(p.state_out) + s_out;
+            const bool to_bf16 = wk.fin == 0 && p.state_bf16;
+            if (piece_aligned(to_bf16 ? (const void*)to16 : (const void*)to32)) {
+                if (to_bf16) state_from_tmem(from, to16 - lane * DK, lane);
+                else state_from_tmem(from, to32 - lane * DK, lane);
+            } else {
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    uint32_t r[16];
+                    tc::tmem_ld16(from + half * 16, r);
+                    tc::tmem_ld_wait();
+#pragma unroll
+                    for (int x = 0; x < 16; ++x) {
+                        if (to_bf16) to16[half * 16 + x] = f32_to_bf16_bits(__uint_as_float(r[x]));
+                        else to32[half * 16 + x] = __uint_as_float(r[x]);
+                    }
                 }
             }
         }
-    }
-    if (count == 0) release(seq);
-    else held = seq;
+        if (count == 0) release(seq);
+        else held = seq;
     }
     if (alive && due >= 0) emit_last();
     tc::fence_before_sync();
