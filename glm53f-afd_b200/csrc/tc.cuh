@@ -178,13 +178,7 @@ __device__ __forceinline__ uint32_t bf16x2(float lo, float hi) {
     const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<const uint32_t*>(&v);
 }
-// x = hi + lo with hi = bf16(x), lo = bf16(x - hi): 16 bits of mantissa in two bf16 operands.
-__device__ __forceinline__ void split_bf16(float x, float& hi, float& lo) {
-    hi = bf16_round(x);
-    lo = x - hi;
-}
-
-// The same for a pair, packed: hi and lo halves of (x0, x1).
+// x = hi + lo with hi = bf16(x), lo = bf16(x - hi): 16 bits of mantissa in two bf16 operands.  For a pair, packed: hi and lo halves of (x0, x1).
 __device__ __forceinline__ void split_bf16x2(float x0, float x1, uint32_t& hi, uint32_t& lo) {
     hi = bf16x2(x0, x1);
     lo = bf16x2(x0 - __uint_as_float(hi << 16), x1 - __uint_as_float(hi & 0xffff0000u));
