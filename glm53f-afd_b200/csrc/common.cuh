@@ -24,7 +24,7 @@ enum : int {
     kStatusWaitYFull = 107,
     kStatusWaitYEmpty = 108,
     kStatusWaitPrefill = 120,
-    kStatusPrefillRange = 121,  // eight rows of decay beyond what the tensor-core kernels can factor (or a positive log decay)
+    kStatusPrefillRange = 121,  // eight rows up to, or seven behind, a middle row decay by more than the tensor-core kernels can factor (or grow)
     kStatusVerifyWindow = 122,  // the tensor-core verify met a window of more than 16 rows (it computed the first 16)
 };
 

@@ -46,7 +46,7 @@ __global__ void single_request_meta(unsigned int* meta, int32_t rows) { meta[thr
 // kNotEligible when the call does not meet the kernels' layout requirements (dense output rows, aligned rows, room for
 // one chunk a pass); the caller then runs the exact form.
 // 4 requests x 2,048 rows x 64 heads with 256-row workspaces: 1,800 us with one block doing all of a chain
-// (kda_prefill_tc.cu, passes of six chunks), 1,216 so.
+// (kda_prefill_tc.cu, passes of six chunks), 921 to 947 so.
 int chunked_layer_prefill(int32_t heads, int32_t batch, const int32_t* cu_rows, int32_t max_rows, const glm53f_bf16* p,
                           int64_t p_stride, int64_t b_off, const glm53f_bf16* a, int64_t a_stride, const glm53f_bf16* g,
                           int64_t g_stride, const glm53f_bf16* conv, const int64_t* conv_off, const glm53f_bf16* conv_w,

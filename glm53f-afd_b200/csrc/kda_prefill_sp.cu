@@ -706,7 +706,8 @@ __device__ void intra_role(const SpParams& p, unsigned char* smem, const uint32_
 // are A operands that never leave tensor memory; what comes from the workspace is the B side, so shared memory has room for
 // two chunks of it and a load has a whole chunk's time to arrive.
 // Measured per chunk at 64 chains: 5,800 cycles with products of 64 rows, S and D through shared memory and block barriers
-// around every step; 3,700 to 4,000 so; 3,500 with U asked into L2 a chunk ahead.  With the gated norm 5,400: 16,384 exponentials and
+// around every step; 3,700 to 4,000 so; 3,500 with U asked into L2 a chunk ahead (8 chains of 1,024 chunks: a whole call is 3,240 a chunk), 4,400
+// with a chain on every SM, when the workspace comes at 5.9 TB/s.  With the gated norm 5,400: 16,384 exponentials and
 // reciprocals a chunk are 1,000 cycles of the units that do them (before U and D instead of behind D they are as long, and cost registers).
 // =====================================================================================================================
 // Shared memory: two buffers of [Qg | W], two of [M | Kdec hi | Kdec lo] and exp(G_last), one of U, each with a full / empty pair.
@@ -1535,8 +1536,8 @@ static int fused_launch(SpParams& p, unsigned char* slots, unsigned int* tail, i
     p.sets = tail + kTailSets;
     p.ctr = pass & 1;
     p.group = (int)((chains + kTailGroups - 1) / kTailGroups);
-    // (The prologue in front is a plain launch: begun early too, its blocks crowd onto the SMs that come free first, 1,243 against
-    // 1,203 us for 4 requests x 2,048 rows.)
+    // (The prologue in front is a plain launch: begun early too, its blocks crowd onto the SMs that come free first, 952 against
+    // 921 us for 4 requests x 2,048 rows.)
     return launch_early(LAYER || p.gate != nullptr ? prefill_sp_kernel<LAYER, true, true> : prefill_sp_kernel<LAYER, true, LAYER>, (unsigned)(most < sms ? most : sms), kThreadsSp, kSmemSp, stream, p);
 }
 

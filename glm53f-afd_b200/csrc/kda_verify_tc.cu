@@ -32,9 +32,10 @@
 // 16 rows): operand tiles 4,400 with two exponentials and a division an element and the saves between them, 1,800 as products of
 // multipliers; the saves 1,300, beside the first products; the next rows' copies 1,800 with a load of beta to wait for, 570 without;
 // products 870 + 880 as eight of N = 32 each instead of sixteen of N = 16; outputs 3,000 as two-byte stores, now sixteen bytes a unit
-// later.  Verify and commit of 34 layers together: 3,806 -> 3,183 us, 20 requests of 4 to 8 rows 1,625 -> 1,371; with the state in boxes,
-// in both kernels and both ways, instead of 2,048 pieces that pass through the threads, 2,894 and 1,240 (the commit's way out alone was
-// 2,000 cycles of a unit's 14,000).
+// later.  Verify and commit of 34 layers together, the same buffers in every call: 3,806 -> 3,183 us, 20 requests of 4 to 8 rows 1,625 -> 1,371;
+// with the state in boxes, in both kernels and both ways, instead of 2,048 pieces that pass through the threads, 2,870 to 2,920 and 1,230 to 1,240
+// (the commit's way out alone was 2,000 cycles of a unit's 14,000).  With buffers that change from call to call 48 requests take
+// 3,065 to 3,120 us, before all of it 3,800.
 
 #include <cuda_fp16.h>
 
