@@ -183,7 +183,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1) prefill_tc_kernel(const __grid_
     // A chunk's outputs: bf16(y), or the gated RMSNorm of bf16(y).  From the fragments four lanes trade, so that each has eight consecutive
     // channels of its two rows.  They leave while the next chunk's first products run.
     // (A chunk's end, with 32 gate values and norm weights a thread read one by one, half of the lanes idle and an IEEE division each: 4
-    // sequences of 8,192 rows in all, 64 heads, with the norm 1,335 -> 1,000 us, all fragment reads together; without it 824 -> 810.)
+    // sequences of 8,192 rows in all, 64 heads, with the norm 1,335 -> 1,000 us, all fragment reads together; in 2 without it 824 -> 810.)
     // (The gate's reciprocal keeps its denormals, as a division does: a gate of -88 leaves outputs that bf16 holds.  Of 16.4 million outputs 166,
     // 236 and 423 are not the bf16 next to the 64-bit value, gates of deviation 1, 4 and 12; with an IEEE division 165, 228 and 427, and
     // 8,192 rows in 4 sequences take 1,016 us instead of 1,000, 1,000 in 8 166 instead of 152.)
