@@ -79,6 +79,19 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
     return ok != 0;
 }
 
+// Whether the phase has completed, without waiting for it.
+__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+
 // A wait that cannot spin forever.  It gives up when neither the barrier flips nor the block's progress
 // counter moves for kWaitLimitNs; the caller then records `code`, raises the block's abort flag and returns
 // from the kernel.  Every other wait of the block sees the abort flag and returns false at once.

@@ -10,14 +10,20 @@
 // tensor memory and only the short dependent part per chunk: S as bf16 operand, QS = Qg S and -W S, D = U - W S,
 // O = QS + M D, S <- E_last S + Kdec^T D.
 //
+// Where many chains are walked (WALK_U), T' as bf16 hi + lo goes into the workspace in U's place and the walk forms U itself, from V as the
+// caller has it: 16 KiB less to write and to read an item, a product and a result less in the intra role, but eight products more in
+// the walk, which only a walk that waits for memory does not notice.  The products and sums are the same, and so are the bits.  U in the items / in
+// the walk, us: 262,144 rows x 64 heads 15,316 / 14,020, 8,192 rows x 64 heads in 8 sequences 517 / 484, the layer form's 4 x 2,048 rows 922 / 883.
+//
 // The sequence is cut into segments sized by the workspace.  One kernel launch runs the state role for segment s-1
 // (blocks 0..chains-1) and the intra role for segment s (every block, the chain blocks after their state work; items
 // are handed out through a counter in the workspace), on two halves of the workspace that swap from launch to
 // launch; stream order between launches is the only synchronisation.  With more chains than SMs, and for the layer entry
 // points, one persistent launch a pass runs both roles over all the slots (fused_roles).
 //
-// Workspace slot of one (chain, chunk) item, bytes: Qg 0 | W 16,384 (cells of eight rows, [8][128 key channels]) | M 32,768 | Kdec hi 40,960 | Kdec lo 57,344 |
-// U 73,728 (FP32, cells of four rows, [2][16][64 value channels]) | E_last 106,496 (128 floats); 107,008 per slot = 1,672 per row and head, inside
+// Workspace slot of one (chain, chunk) item, bytes: U 0 (FP32, cells of four rows, [2][16][64 value channels]), or T' hi 0, lo 8,192 and V 16,384 (boxes as
+// they are staged: the layer prologue's, and of a sequence's partial chunk; any other V is read where the caller has it) | Qg 32,768 |
+// W 49,152 (cells of eight rows, [8][128 key channels]) | M 65,536 | Kdec hi 73,728 | Kdec lo 90,112 | E_last 106,496 (128 floats); 107,008 per slot = 1,672 per row and head, inside
 // the 2,176 the reference's prefill workspace formula provides (kernels/kda_prefill.cu:40-43, 695-698).  The last
 // 256 bytes of the workspace hold the counters (kda_internal.h).
 
@@ -39,11 +45,12 @@ namespace {
 using namespace pf;
 
 // U is kept in FP32 as 16-byte cells of four rows of a value channel, the channels in two halves, so that both its writer (a
-// thread holds a channel's rows) and its reader store and load consecutive cells and half of the channels is one piece.
+// thread holds a channel's rows) and its reader store and load consecutive cells.
 __device__ __forceinline__ int u_cell(int row4, int v) { return (((v >> 6) * 16 + row4) * 64 + (v & 63)) * 16; }
-constexpr int wQg = 0, wW = kTile, wMm = 2 * kTile, wKdHi = wMm + kTile / 2, wKdLo = wKdHi + kTile, wU = wKdLo + kTile;
-constexpr int kUBytes = CH * DV * 4, wEgl = wU + kUBytes, kSlotBytes = wEgl + 512;
-static_assert(kSlotBytes == kPrefillSlotBytes && wU == 73728, "workspace slot layout");
+// What the walk's loader brings in together lies together: U, or T' and V; Qg and W; M and Kdec.
+constexpr int wU = 0, wTp = 0, wV = kTile, wQg = 2 * kTile, wW = 3 * kTile, wMm = 4 * kTile, wKdHi = wMm + kTile / 2, wKdLo = wKdHi + kTile;
+constexpr int kUBytes = CH * DV * 4, wEgl = wKdLo + kTile, kSlotBytes = wEgl + 512;
+static_assert(kSlotBytes == kPrefillSlotBytes && wV == kSlotInV && wTp == kSlotInK && kSlotInK + kTile <= wV && wU + kUBytes == wQg, "a chunk's V stays where the layer prologue put it; T' goes over K");
 
 // Staging of a chunk's raw rows in the intra kernel: dense boxes of 64 rows x 128 bytes written by tiled tensor copies
 // with the 128-byte swizzle (16-byte piece p of row r sits at piece p ^ (r & 7)), so that threads walking down the
@@ -62,7 +69,7 @@ __device__ __forceinline__ float2 widen2(uint32_t w) {
 }
 
 struct SpParams {
-    alignas(64) CUtensorMap tm_q, tm_k, tm_v, tm_g;  // [rows][H][128] as (128, H, rows); boxes of 64 rows x 128 bytes, 128-byte swizzle
+    alignas(64) CUtensorMap tm_q, tm_k, tm_v, tm_g;  // [rows][H][128] as (128, H, rows); boxes of 64 rows (v: 32) x 128 bytes, 128-byte swizzle
     alignas(64) CUtensorMap tm_out;                  // the shard-local output, the same way
     alignas(64) CUtensorMap tm_gate;                 // the gate rows, the same way (gate_boxes != 0)
     alignas(64) CUtensorMap tm_full[8];              // every rank's full output buffer: (128, heads_total, rows)
@@ -147,7 +154,7 @@ static_assert(kSmemSp <= 232448, "shared memory budget");
 // products over key channels, MN-major for the products over rows), so k and q are turned into Kg and Qg in place and
 // v is used as it lands; the log decays become E in place; the inverse's FP32 scratch goes over E and Kinv once they
 // are dead; and everything the state role needs leaves for the workspace straight from registers (Qg, Kdec hi/lo,
-// E_last, M, W, U), in the un-swizzled cell layout the state role reads, so no result tile lives in shared memory.
+// E_last, M, W, U or T'), in the un-swizzled cell layout the state role reads, so no result tile lives in shared memory.
 // =====================================================================================================================
 constexpr int kGroupThreads = 256, kGroups = 2;
 // Decay range.  L and M hold exp(G_i - G_j) for every pair of rows j <= i of a chunk, and a tensor-core product can
@@ -164,7 +171,7 @@ constexpr int kKcBytes = 2 * 128 * (16 + 32 + 48 + 64);  // the four column-side
 __device__ __forceinline__ int kc_piece(int I, int r, int piece) {
     return kc_tile(I) + (piece >> 3) * (I + 1) * 2048 + r * 128 + (((piece & 7) ^ (r & 7)) << 4);
 }
-constexpr int gK = 0, gV = kTile, gQ = 2 * kTile, gKb = 3 * kTile, gKc = 4 * kTile;  // K/Kg | V | Q/Qgb | Kgb | the column-side tiles
+constexpr int gK = 0, gV = kTile, gQ = 2 * kTile, gKb = 3 * kTile, gKc = 4 * kTile;  // K/Kg | V (unless WALK_U) | Q/Qgb | Kgb | the column-side tiles
 // The log decays lie over the column-side tiles; the inverse's scratch and T' (hi | lo box, over L) over Q, Kgb and the 8 KiB before
 // the log decays, so that the next item's log decays can arrive as soon as L and M are formed.
 constexpr int gG = gKc + 8192, gT = gQ, gL = gT + CH * LS * 4, gTp = gL;
@@ -178,7 +185,7 @@ static_assert(kGroups * kGroupBytes <= oCtl, "two groups must fit below the bloc
 constexpr uint32_t gcL = 0, gcM = 64, gcW = 0, gcU = 64, kGroupCols = 128;
 
 // LAYER: the items' inputs are in their slots (kda_internal.h), which the results then replace.  G = 0 or 1, a runtime value: both groups run the same instructions (one copy of this code in the instruction cache).
-template <bool LAYER, bool FUSED>
+template <bool LAYER, bool FUSED, bool WALK_U>
 __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* smem, const uint32_t tm_block, const WaitCtx& ctx, const int G) {
     // The issue loops stay loops in the layer form's instance and are unrolled in the core form's, whichever branch an item takes: 4 x 2,048
     // rows of the layer form 972 -> 944 us as loops; the core form's 8,192 rows in 8 sequences 462 both ways with mild gates, 548 and 555 with
@@ -231,7 +238,7 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
 
     for (;;) {
         if (!mbar_wait(bar_g, raw_phase, ctx, kStatusWaitPrefill)) break;
-        const int item = *item_slot;
+        const int item = item_slot[0], live = item_slot[1];  // (the next item's from when L and M are formed)
         if (item < 0) break;
         const Item at_item = item_of<FUSED>(p, item);
         unsigned char* slot = slot_of(p.ws_intra, p.seg_chunks, at_item.chain, at_item.jj);
@@ -511,7 +518,12 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
                     tc::split_bf16x2(t4.z * b4.z, t4.w * b4.w, wh[2 * j2 + 1], wl[2 * j2 + 1]);
                 }
                 *reinterpret_cast<uint4*>(gs + gTp + box_piece(i, c)) = make_uint4(wh[0], wh[1], wh[2], wh[3]);
-                *reinterpret_cast<uint4*>(gs + gTp + kBox + box_piece(i, c)) = make_uint4(wl[0], wl[1], wl[2], wl[3]);
+                if constexpr (WALK_U) {
+                    *reinterpret_cast<uint4*>(cell(slot + wTp, CH, c, i)) = make_uint4(wh[0], wh[1], wh[2], wh[3]);
+                    *reinterpret_cast<uint4*>(cell(slot + wTp + kBox, CH, c, i)) = make_uint4(wl[0], wl[1], wl[2], wl[3]);
+                } else {
+                    *reinterpret_cast<uint4*>(gs + gTp + kBox + box_piece(i, c)) = make_uint4(wl[0], wl[1], wl[2], wl[3]);
+                }
             }
         }
         publish();
@@ -520,19 +532,35 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
         // products take the same instructions at half the rate) ------------------------------------------------------------
         mma_issue(bar_mma, [&](uint32_t leader) {
             constexpr uint32_t id = tc::idesc_bf16(128, 64, 1, 0, 0);
-            const unsigned char* tph = gs + gTp;
-            const unsigned char* tpl = gs + gTp + kBox;
 #pragma unroll kIssue
             for (int k0 = 0; k0 < CH; k0 += 16)
-                tc::mma_bf16_if(leader, tm + gcW, tc::desc_sw128_mnmajor(gs + gK, CH, k0), tc::desc_sw128_kmajor(tph, CH, k0), id, k0 > 0);
+                tc::mma_bf16_if(leader, tm + gcW, tc::desc_sw128_mnmajor(gs + gK, CH, k0), tc::desc_sw128_kmajor(gs + gTp, CH, k0), id, k0 > 0);
+            if constexpr (!WALK_U) {
 #pragma unroll kIssue
-            for (int k0 = 0; k0 < CH; k0 += 16)
-                tc::mma_bf16_if(leader, tm + gcU, tc::desc_sw128_mnmajor(gs + gV, CH, k0), tc::desc_sw128_kmajor(tph, CH, k0), id, k0 > 0);
+                for (int k0 = 0; k0 < CH; k0 += 16)
+                    tc::mma_bf16_if(leader, tm + gcU, tc::desc_sw128_mnmajor(gs + gV, CH, k0), tc::desc_sw128_kmajor(gs + gTp, CH, k0), id, k0 > 0);
 #pragma unroll kIssue
-            for (int k0 = 0; k0 < CH; k0 += 16)
-                tc::mma_bf16_if(leader, tm + gcU, tc::desc_sw128_mnmajor(gs + gV, CH, k0), tc::desc_sw128_kmajor(tpl, CH, k0), id, true);
+                for (int k0 = 0; k0 < CH; k0 += 16)
+                    tc::mma_bf16_if(leader, tm + gcU, tc::desc_sw128_mnmajor(gs + gV, CH, k0), tc::desc_sw128_kmajor(gs + gTp + kBox, CH, k0), id, true);
+            }
         });
         report();
+        // A walk that forms U reads V itself, a partial chunk's from the slot: zero past the sequence's end (the layer form's live rows lie there).
+        if (WALK_U && live < CH) {
+            const int h = at_item.chain % p.H;
+            const long long row0 = LAYER ? 0 : p.cu[at_item.chain / p.H] + (long long)(p.intra_chunk0 + at_item.jj) * CH;
+            uint4 v8[4];
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                const int r = t * 16 + (gt >> 4);
+                v8[t] = !LAYER && r < live ? *reinterpret_cast<const uint4*>(p.v + ((row0 + r) * p.H + h) * DK + (gt & 15) * 8) : make_uint4(0u, 0u, 0u, 0u);
+            }
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                const int r = t * 16 + (gt >> 4);
+                if (!LAYER || r >= live) *reinterpret_cast<uint4*>(slot + wV + box_piece(r, gt & 15)) = v8[t];
+            }
+        }
         if (!mma_wait(bar_mma, mma_phase)) break;
         // Nothing of this item is left in the group's shared memory: the loader may bring the next item in.
         if (gt == 0) mbar_arrive(bar_free);
@@ -545,11 +573,13 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
             tc::tmem_ld_wait();
 #pragma unroll
             for (int cc = 0; cc < 4; ++cc) *reinterpret_cast<uint4*>(cell(slot + wW, DK, cg * 4 + cc, ch)) = pack8(r + cc * 8);
-            tc::tmem_ld32(tc::tmem_addr(tm, quad, gcU + cg * 32), r);
-            tc::tmem_ld_wait();
+            if constexpr (!WALK_U) {
+                tc::tmem_ld32(tc::tmem_addr(tm, quad, gcU + cg * 32), r);
+                tc::tmem_ld_wait();
 #pragma unroll
-            for (int j2 = 0; j2 < 8; ++j2)
-                *reinterpret_cast<uint4*>(slot + wU + u_cell(cg * 8 + j2, ch)) = make_uint4(r[j2 * 4], r[j2 * 4 + 1], r[j2 * 4 + 2], r[j2 * 4 + 3]);
+                for (int j2 = 0; j2 < 8; ++j2)
+                    *reinterpret_cast<uint4*>(slot + wU + u_cell(cg * 8 + j2, ch)) = make_uint4(r[j2 * 4], r[j2 * 4 + 1], r[j2 * 4 + 2], r[j2 * 4 + 3]);
+            }
         }
         if (FUSED) fence_proxy_async_global();  // another block's bulk copies read the slot
         tc::fence_before_sync();
@@ -567,11 +597,11 @@ __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src,
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // The loader warp of group G: takes items off the counter and brings each one's rows into the group's staging.  A full
-// chunk arrives by ten tiled tensor copies issued by one lane; a sequence's last, partial chunk by the warp's own
+// chunk arrives by eight or ten tiled tensor copies issued by one lane; a sequence's last, partial chunk by the warp's own
 // 16-byte copies (rows past the sequence's end are not read, they become zero), so no copy ever reaches
-// past the rows the caller's metadata names.  They are asynchronous, all in flight at once: as loads and stores, a row's after
+// past the rows the caller's metadata names.    They are asynchronous, all in flight at once: as loads and stores, a row's after
 // the other's, they were 8 to 12 us of a launch (33 rows x 64 heads by the chunked layer prefill: 59 us, 64 rows 52).
-template <bool LAYER, bool FUSED>
+template <bool LAYER, bool FUSED, bool WALK_U>
 __device__ __forceinline__ void intra_loader(const SpParams& p, unsigned char* smem, const WaitCtx& ctx, const int G) {
     unsigned char* gs = smem + G * kGroupBytes;
     uint64_t* bar_raw = reinterpret_cast<uint64_t*>(gs + gBars);
@@ -611,12 +641,15 @@ __device__ __forceinline__ void intra_loader(const SpParams& p, unsigned char* s
             for (int x = 0; x < 4; ++x) tensor_prefetch_3d(&p.tm_g, x * 32, h, row);
             for (int x = 0; x < 2; ++x) tensor_prefetch_3d(&p.tm_k, x * 64, h, row);
             for (int x = 0; x < 2; ++x) tensor_prefetch_3d(&p.tm_q, x * 64, h, row);
-            for (int x = 0; x < 2; ++x) tensor_prefetch_3d(&p.tm_v, x * 64, h, row);
+            for (int x = 0; !WALK_U && x < 2; ++x) tensor_prefetch_3d(&p.tm_v, x * 64, h, row);
         }
         const int row = (int)gr0;
         // The log decays, as soon as the item before has formed its L and M; then the other rows, when it is through with its own.
         if (it > 0 && !mbar_wait(bar_gfree, free_phase, ctx, kStatusWaitPrefill)) break;
-        if (lane == 0) *item_slot = last ? -1 : (int)item;
+        if (lane == 0) {
+            item_slot[0] = last ? -1 : (int)item;
+            item_slot[1] = n;
+        }
         if (last) {  // tell the compute warps that there is nothing more
             if (lane == 0) mbar_arrive(bar_g);
             break;
@@ -648,13 +681,14 @@ __device__ __forceinline__ void intra_loader(const SpParams& p, unsigned char* s
         if (n == CH) {
             __syncwarp();
             if (lane == 0) {
-                mbar_arrive_expect_tx(bar_raw, 3u * kTile);
+                mbar_arrive_expect_tx(bar_raw, (WALK_U ? 2u : 3u) * kTile);
                 if constexpr (LAYER) {
-                    bulk_load(gs + gK, in + kSlotInK, 3 * kTile, bar_raw);
+                    bulk_load(gs + gK, in + kSlotInK, kTile, bar_raw);
+                    bulk_load(gs + gQ, in + kSlotInQ, kTile, bar_raw);
                 } else {
                     for (int x = 0; x < 2; ++x) tensor_load_3d(gs + gK + x * kBox, &p.tm_k, x * 64, h, row, bar_raw);
                     for (int x = 0; x < 2; ++x) tensor_load_3d(gs + gQ + x * kBox, &p.tm_q, x * 64, h, row, bar_raw);
-                    for (int x = 0; x < 2; ++x) tensor_load_3d(gs + gV + x * kBox, &p.tm_v, x * 64, h, row, bar_raw);
+                    for (int x = 0; !WALK_U && x < 2; ++x) tensor_load_3d(gs + gV + x * kBox, &p.tm_v, x * 64, h, row, bar_raw);
                 }
             }
         } else {
@@ -662,18 +696,18 @@ __device__ __forceinline__ void intra_loader(const SpParams& p, unsigned char* s
                 const int c = lane & 15, live = min(r, n - 1), from = box_piece(live, c), to = box_piece(r, c);
                 const long long at = ((gr0 + live) * H + h) * DK + c * 8;
                 cp_async16(gs + gK + to, LAYER ? (const void*)(in + kSlotInK + from) : (const void*)(p.k + at), r < n);
-                cp_async16(gs + gV + to, LAYER ? (const void*)(in + kSlotInV + from) : (const void*)(p.v + at), r < n);
                 cp_async16(gs + gQ + to, LAYER ? (const void*)(in + kSlotInQ + from) : (const void*)(p.q + at), r < n);
+                if (!WALK_U) cp_async16(gs + gV + to, p.v + at, r < n);
             }
             cp_async_wait_all();
-            fence_proxy_async_smem();  // V is read by the tensor core as it stands
+            if (!WALK_U) fence_proxy_async_smem();  // V is read by the tensor core as it stands
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_raw);
         }
     }
 }
 
-template <bool LAYER, bool FUSED>
+template <bool LAYER, bool FUSED, bool WALK_U>
 __device__ void intra_role(const SpParams& p, unsigned char* smem, const uint32_t tm) {
     volatile uint32_t* ctl = reinterpret_cast<volatile uint32_t*>(smem + oCtl);
     const WaitCtx ctx{ctl, ctl + 1, p.status};
@@ -686,8 +720,8 @@ __device__ void intra_role(const SpParams& p, unsigned char* smem, const uint32_
         mbar_init_fence();
     }
     __syncthreads();
-    if (warp == kLoaderWarp || warp == kOutWarp) intra_loader<LAYER, FUSED>(p, smem, ctx, warp == kLoaderWarp ? 0 : 1);
-    else if (warp != kMmaWarp) intra_group<LAYER, FUSED>(p, smem, tm, ctx, warp < kGroupThreads / 32 ? 0 : 1);
+    if (warp == kLoaderWarp || warp == kOutWarp) intra_loader<LAYER, FUSED, WALK_U>(p, smem, ctx, warp == kLoaderWarp ? 0 : 1);
+    else if (warp != kMmaWarp) intra_group<LAYER, FUSED, WALK_U>(p, smem, tm, ctx, warp < kGroupThreads / 32 ? 0 : 1);
     tc::fence_before_sync();
     __syncthreads();
 }
@@ -700,32 +734,33 @@ __device__ void intra_role(const SpParams& p, unsigned char* smem, const uint32_
 //   all 16 warps     S^T to bf16 pairs, in tensor memory; then, behind the first product, the decayed S^T back
 //   MMA warp         (W S)^T = S^T W^T, 128 value channels x 64 rows, which D waits for; then (Qg S)^T, which it does not
 //   all 16 warps     D^T = U^T - (W S)^T as bf16 hi + lo pairs, in tensor memory
-//   MMA warp         S^T += D^T Kdec (hi hi + lo hi + hi lo), which the next chunk waits for; then O^T = (Qg S)^T + D^T M^T
+//   MMA warp         S^T += D^T Kdec (hi hi + lo hi + hi lo), which the next chunk waits for; then O^T = (Qg S)^T + D^T M^T, and
+//                    (WALK_U) the next chunk's U^T = V^T T'^T (T' hi + lo)
 //   all 16 warps     the outputs of the chunk before, while the state's product runs
 // Transposed, every product uses the tensor core's full height, every lane holds results, and the operands that change (S, D)
 // are A operands that never leave tensor memory; what comes from the workspace is the B side, so shared memory has room for
 // two chunks of it and a load has a whole chunk's time to arrive.
 // Measured per chunk at 64 chains: 5,800 cycles with products of 64 rows, S and D through shared memory and block barriers
-// around every step; 3,700 to 4,000 so; 3,500 with U asked into L2 a chunk ahead (8 chains of 1,024 chunks: a whole call is 3,240 a chunk), 4,400
+// around every step; 3,700 to 4,000 so; 3,500 with the single buffer's piece asked into L2 a chunk ahead (8 chains of 1,024 chunks: a whole call is 3,240 a chunk), 4,400
 // with a chain on every SM, when the workspace comes at 5.9 TB/s.  With the gated norm 5,400: 16,384 exponentials and
 // reciprocals a chunk are 1,000 cycles of the units that do them (before U and D instead of behind D they are as long, and cost registers).
 // =====================================================================================================================
-// Shared memory: two buffers of [Qg | W], two of [M | Kdec hi | Kdec lo] and exp(G_last), one of U, each with a full / empty pair.
+// Shared memory: two buffers of [Qg | W] and exp(G_last), two of [M | Kdec hi | Kdec lo], one of U, or T' hi | T' lo | V, each with a full / empty pair.
 // Finished output rows (bf16) wait in one of two tiles for the output warp: two boxes of 64 rows x 128 bytes each (value
 // channels 0-63, 64-127) in the 128-byte swizzle of box_piece(), which is what the tiled tensor stores read.
 constexpr int kQW = 2 * kTile, kMKd = kTile / 2 + 2 * kTile, kOutTile = 2 * kBox;
 constexpr int sQW = 0, sMKd = sQW + 2 * kQW, sU = sMKd + 2 * kMKd, sOut = sU + kUBytes, sRed = sOut + 2 * kOutTile, sE = sRed + 2 * 4 * CH * 4;
-static_assert(sOut % 1024 == 0 && sE + 2 * 512 <= oBars, "state role shared memory");
-// Tensor memory columns: S^T; its bf16 pairs; (W S)^T; (Qg S)^T and O^T, two accumulators that alternate between chunks; D^T hi, lo.
-constexpr uint32_t tS = 0, tS16 = 128, tWS = 192, tO = 256, tDhi = 384, tDlo = 416;
+static_assert(sOut % 1024 == 0 && (sU + kTile) % 1024 == 0 && sE + 2 * 512 <= oBars, "state role shared memory");
+// Tensor memory columns: S^T; its bf16 pairs; (W S)^T; (Qg S)^T and O^T, two accumulators that alternate between chunks; D^T hi, lo; U^T.
+constexpr uint32_t tS = 0, tS16 = 128, tWS = 192, tO = 256, tDhi = 384, tDlo = 416, tU = 448;
 
 // The state role's barriers and their arrival counts.  Those of a buffer that alternates between chunks come in pairs, so that
 // no barrier can complete a phase while somebody still has to see the one before.
 enum : int { bFullQW = 0, bFullMKd = 2, bFullU = 4, bEmptyQW = 5, bEmptyMKd = 7, bEmptyU = 9, bWS = 10, bSNew = 11, bS16 = 12, bSDec = 13, bD = 14, bO = 15, bOFree = 17,
              bOutFull = 19, bOutEmpty = 21, bChainFull = 23, bChainEmpty = 25, bGate = 27, kStateBars = 29 };
-__device__ __forceinline__ int state_bar_count(int i) {
+__device__ __forceinline__ int state_bar_count(int i, bool walk_u) {
     // one arrival per compute warp, or one in all
-    const bool warps = i == bEmptyU || i == bS16 || i == bSDec || i == bD || i == bOFree || i == bOFree + 1 || i == bOutFull || i == bOutFull + 1;
+    const bool warps = (i == bEmptyU && !walk_u) || i == bS16 || i == bSDec || i == bD || i == bOFree || i == bOFree + 1 || i == bOutFull || i == bOutFull + 1;
     return warps ? kCompute / 32 : i == bChainEmpty || i == bChainEmpty + 1 ? kCompute / 32 + 2 : 1;  // a chain is read by the MMA and the output warp too
 }
 static_assert(kStateBars * 8 <= oChain - oBarsState && oChain % 16 == 0, "state role barriers");
@@ -753,7 +788,7 @@ __device__ __forceinline__ bool count_wait(const unsigned int* at, unsigned want
 }
 
 // What one walk of the state role covers: chunks [ja, jb) of its chain, where the state comes from and goes to, whether
-// U takes part (not in the walk that yields a segment's transition) and whether outputs are produced.
+// T'V takes part (not in the walk that yields a segment's transition) and whether outputs are produced.
 struct Walk {
     int ja, jb;
     int init;          // 0: the state buffer (state_in for the first chunk of a sequence, else state_out); 1: zero; 2: identity; 3: FP32 `from`
@@ -880,7 +915,7 @@ __device__ __forceinline__ void state_to_tmem(uint32_t at, const uint16_t* from,
 // chunks: counter, metadata, barriers and first loads one after another, the state a line per 16 bytes, the last chunk's gate.  Whole
 // calls, us: chunked layer prefill of 4 x 2,048 rows 1,136 -> 1,043, of 3 x 700 342 -> 301; core prefill of 8,192 rows in 8 sequences 525 -> 504, with
 // the norm in 3 sequences 663 -> 582; 8 chains of 1,024 chunks (one walk each) 1,968 -> 1,845.
-template <bool MANY, bool GATED>
+template <bool MANY, bool GATED, bool WALK_U>
 __device__ void state_role(const SpParams& p, unsigned char* smem, const uint32_t tm, const int chain, const Walk wk) {
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + oBarsState);
     volatile uint32_t* ctl = reinterpret_cast<volatile uint32_t*>(smem + oCtl);
@@ -1006,17 +1041,26 @@ __device__ void state_role(const SpParams& p, unsigned char* smem, const uint32_
                     const unsigned char* slot = slot_of(p.ws_state, p.seg_chunks, ch, j0 + c);
                     const int x = C & 1;
                     if (!(ok = wait(bEmptyQW + x, (C >> 1) ^ 1))) break;  // an empty barrier starts released
-                    mbar_arrive_expect_tx(&bars[bFullQW + x], kQW);
+                    mbar_arrive_expect_tx(&bars[bFullQW + x], kQW + 512);
+                    bulk_load(smem + sE + x * 512, slot + wEgl, 512, &bars[bFullQW + x]);
                     bulk_load(smem + sQW + x * kQW, slot + wQg, kQW, &bars[bFullQW + x]);
+                    // U, or what it is made from, has one buffer: asked for before the chunk's other one, and from L2.
+                    const bool walk_v = WALK_U && p.v != nullptr;  // else V lies in the slots
+                    if (!WALK_U || wk.use_u) {
+                        const bool whole = walk_v && at.rows - c * CH >= CH;
+                        if (!(ok = wait(bEmptyU, C ^ 1))) break;
+                        mbar_arrive_expect_tx(&bars[bFullU], kUBytes);
+                        bulk_load(smem + sU, slot + wU, whole ? kTile : kUBytes, &bars[bFullU]);
+                        for (int y = 0; whole && y < 2; ++y) tensor_load_3d(smem + sU + kTile + y * kBox, &p.tm_v, y * 64, at.h, (int)at.row + c * CH, &bars[bFullU]);
+                    }
                     if (!(ok = wait(bEmptyMKd + x, (C >> 1) ^ 1))) break;
-                    mbar_arrive_expect_tx(&bars[bFullMKd + x], kMKd + 512);
-                    bulk_load(smem + sE + x * 512, slot + wEgl, 512, &bars[bFullMKd + x]);
+                    mbar_arrive_expect_tx(&bars[bFullMKd + x], kMKd);
                     bulk_load(smem + sMKd + x * kMKd, slot + wMm, kMKd, &bars[bFullMKd + x]);
-                    if (!(ok = wait(bEmptyU, C ^ 1))) break;
-                    mbar_arrive_expect_tx(&bars[bFullU], kUBytes);
-                    bulk_load(smem + sU, slot + wU, kUBytes, &bars[bFullU]);
-                    // U has one buffer, so its load is on the walk: from L2.
-                    if (c + 1 < at.count) bulk_prefetch(slot + kSlotBytes + wU, kUBytes);
+                    if (wk.use_u && c + 1 < at.count) {
+                        const bool whole = walk_v && at.rows - (c + 1) * CH >= CH;
+                        bulk_prefetch(slot + kSlotBytes + wU, whole ? kTile : kUBytes);
+                        for (int y = 0; whole && y < 2; ++y) tensor_prefetch_3d(&p.tm_v, y * 64, at.h, (int)at.row + (c + 1) * CH);
+                    }
                     if (gate_due && !(ok = load_gate(C - 1))) break;
                     gate_due = GATED && wk.emit && p.gate_boxes != 0;
                     gate_row = at.rows - c * CH >= CH ? (int)(at.row + c * CH) : -1;
@@ -1035,7 +1079,18 @@ __device__ void state_role(const SpParams& p, unsigned char* smem, const uint32_
         const uint32_t leader = tc::elect_one();
         auto ready = [&](int i, int phase) { return tc::warp_all(wait(i, phase)); };
         constexpr uint32_t idw = tc::idesc_bf16(DV, CH, 0, 1, 0), idq = tc::idesc_bf16(DV, CH, 0, 0, 0), ids = tc::idesc_bf16(DV, DK, 0, 1, 0);
+        constexpr uint32_t idv = tc::idesc_bf16(DV, CH, 1, 0, 0);
         bool alive = true;
+        // U^T = V^T T'^T (T' hi, then lo).  Behind the wait for the D of the chunk before: the accumulator has been read.
+        const bool walk_u = WALK_U && wk.use_u;
+        bool have_u = false;  // the chunk to come's is on its way
+        auto issue_u = [&]() {
+            tc::fence_after_sync();
+#pragma unroll
+            for (int k0 = 0; k0 < 2 * CH; k0 += 16)
+                tc::mma_bf16_if(leader, tm + tU, tc::desc_sw128_mnmajor(smem + sU + kTile, CH, k0 & (CH - 1)), tc::desc_kmajor_bf16(smem + sU + (k0 < CH ? 0 : kBox), CH, 0, k0 & (CH - 1)), idv, k0 > 0);
+            tc::mma_commit_if(leader, &bars[bEmptyU]);
+        };
         int C = 0;
         for (int seq = 0; alive; ++seq) {
             const int count = chain_count(seq);
@@ -1043,6 +1098,10 @@ __device__ void state_role(const SpParams& p, unsigned char* smem, const uint32_
             release(seq);
             for (int c = 0; tc::warp_all(c < count); ++c, ++C) {
                 alive = false;
+                if (walk_u && !have_u) {
+                    if (!ready(bFullU, C)) break;
+                    issue_u();
+                }
                 const int x = C & 1;
                 const uint32_t acc = tm + tO + (uint32_t)x * 64;
                 const unsigned char *qw = smem + sQW + x * kQW, *mm = smem + sMKd + x * kMKd, *kdhi = mm + kTile / 2, *kdlo = kdhi + kTile;
@@ -1059,8 +1118,9 @@ __device__ void state_role(const SpParams& p, unsigned char* smem, const uint32_
                     for (int k0 = 0; k0 < DK; k0 += 16)
                         tc::mma_bf16_ts_if(leader, acc, tm + tS16 + k0 / 2, tc::desc_kmajor_bf16(qw, CH, 0, k0), idq, k0 > 0);
                 }
+                if (!ready(bSDec, C)) break;  // the warps have read exp(G_last) too
                 tc::mma_commit_if(leader, &bars[bEmptyQW + x]);
-                if (!ready(bFullMKd + x, C >> 1) || !ready(bSDec, C) || !ready(bD, C)) break;
+                if (!ready(bFullMKd + x, C >> 1) || !ready(bD, C)) break;
                 tc::fence_after_sync();
 #pragma unroll
                 for (int k0 = 0; k0 < CH; k0 += 16) tc::mma_bf16_ts_if(leader, tm + tS, tm + tDhi + k0 / 2, tc::desc_mnmajor_bf16(kdhi, CH, 0, k0), ids, true);
@@ -1075,6 +1135,8 @@ __device__ void state_role(const SpParams& p, unsigned char* smem, const uint32_
                     tc::mma_commit_if(leader, &bars[bO + x]);
                 }
                 tc::mma_commit_if(leader, &bars[bEmptyMKd + x]);
+                have_u = walk_u && tc::warp_all(c + 1 < count) && tc::warp_all(mbar_test(&bars[bFullU], (uint32_t)((C + 1) & 1)));
+                if (have_u) issue_u();
                 if (leader) atomicAdd(const_cast<uint32_t*>(ctl), 1u);
                 __syncwarp();
                 alive = true;
@@ -1114,7 +1176,7 @@ __device__ void state_role(const SpParams& p, unsigned char* smem, const uint32_
                 r[2 * x + 1] = pr[x] & 0xffff0000u;
             }
         }
-        if (!wait(bFullMKd + (c & 1), c >> 1)) return false;
+        if (!wait(bFullQW + (c & 1), c >> 1)) return false;
         const float4* el = reinterpret_cast<const float4*>(smem + sE + (c & 1) * 512 + k_first * 4);
 #pragma unroll
         for (int x = 0; x < 8; ++x) {
@@ -1299,24 +1361,31 @@ __device__ void state_role(const SpParams& p, unsigned char* smem, const uint32_
         if (count > 0 && !begin_chunk(C)) { leave(); break; }
         for (int c = 0; c < count; ++c, ++C) {
             // ---- D^T = U^T - (W S)^T as bf16 hi + lo pairs of rows ------------------------------------------------------------
-            float uu[16];
             if (votes && due >= 0 && !out_boxes()) fetch_gate(recs[due_seq & 1], due);
-            if (!wait(bFullU, C)) { leave(); break; }
+            uint32_t uu[16];
+            if constexpr (!WALK_U) {
+                if (!wait(bFullU, C)) { leave(); break; }
 #pragma unroll
-            for (int x = 0; x < 4; ++x) {
-                const float4 u4 = *reinterpret_cast<const float4*>(smem + sU + u_cell(cg * 4 + x, v));
-                uu[4 * x] = wk.use_u ? u4.x : 0.0f; uu[4 * x + 1] = wk.use_u ? u4.y : 0.0f; uu[4 * x + 2] = wk.use_u ? u4.z : 0.0f; uu[4 * x + 3] = wk.use_u ? u4.w : 0.0f;
+                for (int x = 0; x < 4; ++x) {
+                    const uint4 u4 = *reinterpret_cast<const uint4*>(smem + sU + u_cell(cg * 4 + x, v));
+                    uu[4 * x] = u4.x; uu[4 * x + 1] = u4.y; uu[4 * x + 2] = u4.z; uu[4 * x + 3] = u4.w;
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&bars[bEmptyU]);  // U is consumed
             }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&bars[bEmptyU]);  // U is consumed
-            if (!wait(bWS, C)) { leave(); break; }
+            if (!wait(bWS, C)) { leave(); break; }  // (U^T was issued before)
             tc::fence_after_sync();
             {
                 uint32_t r[16], wh[8], wl[8];
+                if constexpr (WALK_U) tc::tmem_ld16(tc::tmem_addr(tm, quad, tU + i0), uu);
                 tc::tmem_ld16(tc::tmem_addr(tm, quad, tWS + i0), r);
                 tc::tmem_ld_wait();
+                if (!wk.use_u)
 #pragma unroll
-                for (int x = 0; x < 8; ++x) tc::split_bf16x2(uu[2 * x] - __uint_as_float(r[2 * x]), uu[2 * x + 1] - __uint_as_float(r[2 * x + 1]), wh[x], wl[x]);
+                    for (int x = 0; x < 16; ++x) uu[x] = 0u;
+#pragma unroll
+                for (int x = 0; x < 8; ++x)
+                    tc::split_bf16x2(__uint_as_float(uu[2 * x]) - __uint_as_float(r[2 * x]), __uint_as_float(uu[2 * x + 1]) - __uint_as_float(r[2 * x + 1]), wh[x], wl[x]);
                 tc::tmem_st8(tc::tmem_addr(tm, quad, tDhi + i0 / 2), wh);
                 tc::tmem_st8(tc::tmem_addr(tm, quad, tDlo + i0 / 2), wl);
                 tc::tmem_st_wait();
@@ -1372,21 +1441,21 @@ template <bool LAYER, bool GATED>
 __device__ void fused_roles(const SpParams& p, unsigned char* smem, const uint32_t tm) {
     volatile uint32_t* ctl = reinterpret_cast<volatile uint32_t*>(smem + oCtl);
     const int tid = threadIdx.x;
-    intra_role<LAYER, true>(p, smem, tm);
+    intra_role<LAYER, true, true>(p, smem, tm);
     if (ctl[1] != 0u) return;
     if (tid < kGroupBars * kGroups) mbar_inval(reinterpret_cast<uint64_t*>(smem + tid / kGroupBars * kGroupBytes + gBars) + tid % kGroupBars);
     fence_proxy_async_smem();  // what the intra role left in shared memory is overwritten by bulk copies
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
-    state_role<true, GATED>(p, smem, tm, 0, Walk{p.state_chunk0, p.state_chunk0 + p.seg_chunks, 0, nullptr, 0, nullptr, true, true});
+    state_role<true, GATED, true>(p, smem, tm, 0, Walk{p.state_chunk0, p.state_chunk0 + p.seg_chunks, 0, nullptr, 0, nullptr, true, true});
 }
 
 // One launch: the state role of one segment on the chain blocks, then the intra role of the next segment on all blocks.
 // (An instance for each set of roles and for the norm: both roles are bound by their own instructions, and what an instance does not run costs
 // it registers and room in the instruction caches.  Against one for all of the core form: 2 sequences of 10,000 rows x 32 heads 980 -> 865 us,
 // 8 chains of 1,024 chunks 1,880 -> 1,680; 4 x 2,048 rows of the layer form 1,011 -> 985.)
-template <bool LAYER, bool FUSED, bool GATED>
+template <bool LAYER, bool FUSED, bool GATED, bool WALK_U>
 __global__ void __launch_bounds__(kThreadsSp, 1) prefill_sp_kernel(const __grid_constant__ SpParams p) {
     extern __shared__ __align__(1024) unsigned char smem[];
     volatile uint32_t* ctl = reinterpret_cast<volatile uint32_t*>(smem + oCtl);
@@ -1394,7 +1463,7 @@ __global__ void __launch_bounds__(kThreadsSp, 1) prefill_sp_kernel(const __grid_
     const int tid = threadIdx.x, warp = tid >> 5;
     if (tid == 0) {
         uint64_t* bs = reinterpret_cast<uint64_t*>(smem + oBarsState);
-        for (int i = 0; i < kStateBars; ++i) mbar_init(bs + i, state_bar_count(i));
+        for (int i = 0; i < kStateBars; ++i) mbar_init(bs + i, state_bar_count(i, WALK_U));
         ctl[0] = 0u;
         ctl[1] = 0u;
         mbar_init_fence();
@@ -1436,11 +1505,11 @@ __global__ void __launch_bounds__(kThreadsSp, 1) prefill_sp_kernel(const __grid_
                     wk.fin = last ? 0 : 2;
                 }
             }
-            state_role<false, GATED>(p, smem, tm, chain, wk);
+            state_role<false, GATED, WALK_U>(p, smem, tm, chain, wk);
             tc::fence_after_sync();
         }
     }
-    if (!FUSED && p.has_intra && ctl[1] == 0u) intra_role<LAYER, false>(p, smem, tm);
+    if (!FUSED && p.has_intra && ctl[1] == 0u) intra_role<LAYER, false, WALK_U>(p, smem, tm);
     if (ctl[1] != 0u) {  // after an abort copies into this block's shared memory may still be in flight: give them a bounded time
         const uint64_t t0 = global_timer_ns();
         while (global_timer_ns() - t0 < 2000000ull) {
@@ -1497,14 +1566,14 @@ __global__ void __launch_bounds__(128) scan_compose_kernel(const __grid_constant
 
 }  // namespace
 
-// A [rows][H][128] tensor of `elem`-byte elements, its rows row_bytes apart (0: dense), as (128, H, rows) with boxes of 64 rows of one
-// head, 128 bytes wide.
-static bool row_tensor_map(CUtensorMap* tm, const void* base, int elem, int H, long long rows, long long row_bytes = 0) {
+// A [rows][H][128] tensor of `elem`-byte elements, its rows row_bytes apart (0: dense), as (128, H, rows) with boxes of 64 (or
+// box_rows) rows of one head, 128 bytes wide.
+static bool row_tensor_map(CUtensorMap* tm, const void* base, int elem, int H, long long rows, long long row_bytes = 0, int box_rows = CH) {
     EncodeTiled enc = encode_tiled();
     if (enc == nullptr) return false;
     const cuuint64_t dims[3] = {(cuuint64_t)DK, (cuuint64_t)H, (cuuint64_t)rows};
     const cuuint64_t strides[2] = {(cuuint64_t)DK * elem, row_bytes != 0 ? (cuuint64_t)row_bytes : (cuuint64_t)H * DK * elem};
-    const cuuint32_t box[3] = {(cuuint32_t)(128 / elem), 1u, (cuuint32_t)CH};
+    const cuuint32_t box[3] = {(cuuint32_t)(128 / elem), 1u, (cuuint32_t)box_rows};
     const cuuint32_t estr[3] = {1u, 1u, 1u};
     return enc(tm, elem == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<void*>(base), dims, strides, box, estr,
                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -1538,7 +1607,7 @@ static int fused_launch(SpParams& p, unsigned char* slots, unsigned int* tail, i
     p.group = (int)((chains + kTailGroups - 1) / kTailGroups);
     // (The prologue in front is a plain launch: begun early too, its blocks crowd onto the SMs that come free first, 952 against
     // 921 us for 4 requests x 2,048 rows.)
-    return launch_early(LAYER || p.gate != nullptr ? prefill_sp_kernel<LAYER, true, true> : prefill_sp_kernel<LAYER, true, LAYER>, (unsigned)(most < sms ? most : sms), kThreadsSp, kSmemSp, stream, p);
+    return launch_early(LAYER || p.gate != nullptr ? prefill_sp_kernel<LAYER, true, true, true> : prefill_sp_kernel<LAYER, true, LAYER, true>, (unsigned)(most < sms ? most : sms), kThreadsSp, kSmemSp, stream, p);
 }
 
 // The launches over every segment of the longest sequence, in stream order.  A workspace of two or more chunks per
@@ -1585,7 +1654,8 @@ int core_prefill_sp_launch(int32_t heads, int32_t batch, const int32_t* cu_seqle
     cudaGetDevice(&dev);
     if (configured_dev != dev) {
         cudaError_t e = cudaSuccess;
-        for (auto kernel : {prefill_sp_kernel<false, false, false>, prefill_sp_kernel<false, false, true>, prefill_sp_kernel<false, true, false>, prefill_sp_kernel<false, true, true>})
+        for (auto kernel : {prefill_sp_kernel<false, false, false, false>, prefill_sp_kernel<false, false, true, false>, prefill_sp_kernel<false, false, false, true>,
+                            prefill_sp_kernel<false, false, true, true>, prefill_sp_kernel<false, true, false, true>, prefill_sp_kernel<false, true, true, true>})
             if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemSp);
         if (e != cudaSuccess) return (int)e;
         configured_dev = dev;
@@ -1633,7 +1703,12 @@ int core_prefill_sp_launch(int32_t heads, int32_t batch, const int32_t* cu_seqle
     gate_tensor_map(p, rows_cap);
     for (int r = 0; r < p.ranks; ++r)
         if (!row_tensor_map(&p.tm_full[r], p.full[r], 2, p.heads_total, rows_cap)) return (int)cudaErrorNotSupported;
-    const auto kernel = gate != nullptr ? prefill_sp_kernel<false, false, true> : prefill_sp_kernel<false, false, false>;
+    // U in the walk (WALK_U) from a chain on every fourth SM on: below that the walks wait for one another's products, not for memory, and SMs without a
+    // chain form U for nothing.  us, 30,000 rows, workspaces of 128 chunks, U in the items / in the walk: 16 heads 876 / 957, 32 heads 1,040 / 1,080 (with the
+    // norm 1,350 / 1,358), 48 heads 1,322 / 1,302 (1,541 / 1,521), 64 heads 1,753 / 1,603 (1,925 / 1,836); 64 heads x 1,000 rows 120 / 115.
+    const bool walk_u = chains * 4 > sm_count();
+    const auto kernel = gate != nullptr ? (walk_u ? prefill_sp_kernel<false, false, true, true> : prefill_sp_kernel<false, false, true, false>)
+                                        : (walk_u ? prefill_sp_kernel<false, false, false, true> : prefill_sp_kernel<false, false, false, false>);
     cudaError_t e = cudaMemsetAsync(p.counters, 0, kCounterBytes, stream);
     if (e != cudaSuccess) return (int)e;
     const long long sms = sm_count();
@@ -1807,7 +1882,7 @@ int layer_pass_launch(int32_t heads, int32_t batch, const int32_t* cu_rows, int3
     int dev = 0;
     cudaGetDevice(&dev);
     if (configured_dev != dev) {
-        const cudaError_t e = cudaFuncSetAttribute(prefill_sp_kernel<true, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemSp);
+        const cudaError_t e = cudaFuncSetAttribute(prefill_sp_kernel<true, true, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemSp);
         if (e != cudaSuccess) return (int)e;
         configured_dev = dev;
     }
