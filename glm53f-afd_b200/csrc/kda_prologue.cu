@@ -217,6 +217,8 @@ __global__ void __launch_bounds__(128, SINK == kExact ? 7 : 6) layer_prologue_ke
 // rows: seven rows of inputs instead of sixteen, the weights once, and everything in pairs of channels (two-wide multiply-adds).
 // 1,280 rows x 64 heads: 79 us with a warp per row as in the kernel above, 52 so with four blocks an SM; five take another 4 us off a pass of the whole call, and six, at 80 registers now that exponentials are single
 // instructions, 3 more (4 x 2,048 rows 941 -> 923 us, 3 x 700 246 -> 238); seven spill (244).
+// Sums of the norms by halves and a row's beta by one lane of every four, 4 x 2,048 rows 889.5 -> 880.0, passes of 1,024 785 -> 769.  (Eight rows a warp spill, 963
+// to 1,000; the parts' rows fetched one part ahead instead of all at once, 899.)
 constexpr int kRowsPer = 4;
 __device__ __forceinline__ float2 lo_hi(uint32_t w) { return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)); }
 __device__ __forceinline__ float2 add2(float2 a, float2 b) { return fma2(a, {1.0f, 1.0f}, b); }
@@ -228,6 +230,20 @@ __device__ __forceinline__ float2 sigmoid2(float2 x) {
 __device__ __forceinline__ uint32_t fp16x2(float2 x) {
     const __half2 h = __float22half2_rn(x);
     return *reinterpret_cast<const uint32_t*>(&h);
+}
+
+// The sums over the warp of a value a row: v[i] of every lane goes in, the sum of row lane / 8 comes out.  At each of the first two steps a lane gives half
+// of its rows away, so four sums take six shuffles and not twenty; the tree is the butterfly's.
+__device__ __forceinline__ float row_sums(float (&v)[kRowsPer], int lane) {
+#pragma unroll
+    for (int n = kRowsPer / 2, o = 16; n > 0; n >>= 1, o >>= 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int i = 0; i < n; ++i) v[i] = (up ? v[i + n] : v[i]) + __shfl_xor_sync(FULL, up ? v[i] : v[i + n], o);
+    }
+#pragma unroll
+    for (int o = 16 / kRowsPer; o; o >>= 1) v[0] += __shfl_xor_sync(FULL, v[0], o);
+    return v[0];
 }
 
 // FIRST: the pass with the requests' first rows, which reach back into the conv windows.
@@ -261,15 +277,14 @@ __global__ void __launch_bounds__(128, 6) prefill_prologue_kernel(const ProParam
         fetch(nullptr, vec);
     }
     uint2 a_bits[kRowsPer];
-    float bl[kRowsPer];
 #pragma unroll
     for (int i = 0; i < kRowsPer; ++i) {
         const long long gr = (long long)r0 + min(first + i, last);
         a_bits[i] = *reinterpret_cast<const uint2*>(p.A + gr * p.a_stride + (long long)h * DK + c0);
-        bl[i] = bf16_bits_to_f32(p.P[gr * p.p_stride + p.b_off + h]);
     }
     const float4 dtb = *reinterpret_cast<const float4*>(p.dt_bias + (long long)h * DK + c0);
     const float rate = expf(p.a_log[h]);
+    const float bl = bf16_bits_to_f32(p.P[((long long)r0 + min(first + (lane & (kRowsPer - 1)), last)) * p.p_stride + p.b_off + h]);  // of row lane % 4
     unsigned char* slot = p.slots + (((long long)b * H + h) * (p.pass_rows / 64) + (j0 >> 6)) * kPrefillSlotBytes;
     const int r = j0 & 63;
 
@@ -305,13 +320,10 @@ __global__ void __launch_bounds__(128, 6) prefill_prologue_kernel(const ProParam
             }
         }
         if (part < 2) {  // L2 norms of q and k (eps 1e-6 inside the root), q also times 128^-0.5
-#pragma unroll
-            for (int o = 16; o; o >>= 1)
-#pragma unroll
-                for (int i = 0; i < kRowsPer; ++i) ss[i] += __shfl_xor_sync(FULL, ss[i], o);
+            const float rinv = rsqrtf(row_sums(ss, lane) + 1e-6f) * (part == 0 ? 0.08838834764831845f : 1.0f);
 #pragma unroll
             for (int i = 0; i < kRowsPer; ++i) {
-                const float s = rsqrtf(ss[i] + 1e-6f) * (part == 0 ? 0.08838834764831845f : 1.0f);
+                const float s = __shfl_sync(FULL, rinv, i * (32 / kRowsPer));
                 y[i] = make_uint2(fp16x2(mul2(lo_hi(y[i].x), {s, s})), fp16x2(mul2(lo_hi(y[i].y), {s, s})));
             }
         }
@@ -326,8 +338,8 @@ __global__ void __launch_bounds__(128, 6) prefill_prologue_kernel(const ProParam
         const float2 s01 = sigmoid2(mul2(add2(lo_hi(a_bits[i].x), {dtb.x, dtb.y}), {rate, rate})), s23 = sigmoid2(mul2(add2(lo_hi(a_bits[i].y), {dtb.z, dtb.w}), {rate, rate}));
         const float2 g01 = mul2(s01, {p.lower, p.lower}), g23 = mul2(s23, {p.lower, p.lower});
         *reinterpret_cast<float4*>(slot + kSlotInG + prefill_box_piece(r + i, lane)) = make_float4(g01.x, g01.y, g23.x, g23.y);
-        if (lane == 0) reinterpret_cast<float*>(slot + kSlotInBeta)[r + i] = bf16_round(sigmoid2({bl[i], bl[i]}).x);
     }
+    if (lane < kRowsPer && j0 + lane < n) reinterpret_cast<float*>(slot + kSlotInBeta)[r + lane] = bf16_round(sigmoid2({bl, bl}).x);
 }
 
 template <int SINK>
