@@ -62,8 +62,8 @@ int conv_shift_launch(int32_t channels, int32_t layers, int32_t batch, const int
 // the 128-byte swizzle (the 16-byte piece p of row r at box p / 8, piece (p % 8) ^ (r % 8)), then beta.
 constexpr int kPrefillSlotBytes = 107008, kPrefillTailBytes = 256;
 // The workspace's last 256 bytes, as words: two item counters | a single request's metadata (an offset, cu_rows) | from word 8
-// on two sets, which consecutive launches use in turn: items and chains handed out, and finished items per group of chains.
-constexpr int kTailMeta = 2, kTailSets = 8, kTailSet = 28, kTailGroups = kTailSet - 2;
+// on two sets, which consecutive launches use in turn: items and chains handed out, blocks that have begun, and finished items per group of chains.
+constexpr int kTailMeta = 2, kTailSets = 8, kTailSet = 28, kTailBegun = 2, kTailDone = 3, kTailGroups = kTailSet - kTailDone;
 static_assert(kPrefillTailBytes == 4 * 64 && kTailSets + 2 * kTailSet == 64, "the workspace's tail");
 constexpr int kSlotInK = 0, kSlotInV = 16384, kSlotInQ = 32768, kSlotInG = 49152, kSlotInBeta = 81920;
 __host__ __device__ inline int prefill_box_piece(int r, int piece) { return (piece >> 3) * 8192 + r * 128 + (((piece & 7) ^ (r & 7)) << 4); }

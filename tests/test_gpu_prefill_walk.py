@@ -78,3 +78,33 @@ def test_gate_rows_of_the_layer_form(lens, gate_at, gap):
         assert all(torch.equal(x.view(torch.int16), y.view(torch.int16)) for x, y in zip(run(gate_at, gap), want))
     finally:
         K.set_prefill_form(K.Form.EXACT)
+
+
+@pytest.mark.parametrize("lens", [[320, 320, 320], [700, 260, 301], [256, 300, 64, 500, 257]])
+def test_blocks_that_leave_the_last_items_to_others(lens):
+    """Chains that do not divide evenly by the SMs, four chunks and more each: the bits of each sequence alone, in every one of many launches."""
+    core = importlib.import_module("glm53f-afd_b200.core")
+    gen = torch.Generator(device="cuda").manual_seed(sum(lens))
+    total, per = sum(lens), HEADS * DK * DK
+    n = total * HEADS
+    rn = lambda *s: torch.randn(*s, device="cuda", generator=gen)
+    unit = lambda s: torch.nn.functional.normalize(rn(n, DK), dim=1).mul(s).bfloat16().view(-1)
+    rows = (unit(DK ** -0.5), unit(1.0), rn(n * DK).bfloat16(), torch.nn.functional.logsigmoid(rn(n * DK) + 3), torch.sigmoid(rn(n)))
+
+    def run(first, ls, launches):
+        m, st = first * HEADS, torch.zeros(len(ls) * per, device="cuda")
+        cut = [t[m * w:(m + sum(ls) * HEADS) * w].clone() for t, w in zip(rows, (DK, DK, DK, DK, 1))]
+        cu, off = torch.tensor([0] + ls, device="cuda").cumsum(0).int(), torch.arange(len(ls), device="cuda") * per
+        ws = torch.zeros(core.prefill_workspace_bytes(HEADS, len(ls), (max(ls) + 63) // 64), dtype=torch.uint8, device="cuda")
+        outs = [torch.zeros(sum(ls) * HEADS * DK, dtype=torch.bfloat16, device="cuda") for _ in range(launches)]
+        for out in outs:
+            st.zero_()
+            core.prefill_varlen(HEADS, sum(ls), cu, max(ls), *cut, st, off, out=out, workspace=ws)
+        torch.cuda.synchronize()
+        assert core.device_status() == 0
+        return outs, st
+
+    alone = [run(sum(lens[:i]), [ls], 1) for i, ls in enumerate(lens)]
+    want, states = torch.cat([o[0] for o, _ in alone]).view(torch.int16), torch.cat([s for _, s in alone])
+    outs, st = run(0, lens, 10)
+    assert all(torch.equal(o.view(torch.int16), want) for o in outs) and torch.equal(st, states)
