@@ -14,6 +14,8 @@
 // caller has it: 16 KiB less to write and to read an item, a product and a result less in the intra role, but eight products more in
 // the walk, which only a walk that waits for memory does not notice.  The products and sums are the same, and so are the bits.  U in the items / in
 // the walk, us: 262,144 rows x 64 heads 15,316 / 14,020, 8,192 rows x 64 heads in 8 sequences 517 / 484, the layer form's 4 x 2,048 rows 922 / 883.
+// Of T', the quarter above the diagonal that is zero stays behind: another 2 to 4 % of the first two (65,536 rows 3,456 -> 3,383, 473 -> 454).  (M's
+// likewise, for two products more: nothing.)
 //
 // The sequence is cut into segments sized by the workspace.  One kernel launch runs the state role for segment s-1
 // (blocks 0..chains-1) and the intra role for segment s (every block, the chain blocks after their state work; items
@@ -21,8 +23,8 @@
 // launch; stream order between launches is the only synchronisation.  With more chains than SMs, and for the layer entry
 // points, one persistent launch a pass runs both roles over all the slots (fused_roles).
 //
-// Workspace slot of one (chain, chunk) item, bytes: U 0 (FP32, cells of four rows, [2][16][64 value channels]), or T' hi 0, lo 8,192 and V 16,384 (boxes as
-// they are staged: the layer prologue's, and of a sequence's partial chunk; any other V is read where the caller has it) | Qg 32,768 |
+// Workspace slot of one (chain, chunk) item, bytes: U 0 (FP32, cells of four rows, [2][16][64 value channels]), or T' 4,096 (its columns 0-31 hi, lo: cells [4][64 rows],
+// its columns 32-63 below the diagonal block's first row hi, lo: [4][32 rows]) and V 16,384 (boxes as they are staged: the layer prologue's, and of a sequence's partial chunk; any other V is read where the caller has it) | Qg 32,768 |
 // W 49,152 (cells of eight rows, [8][128 key channels]) | M 65,536 | Kdec hi 73,728 | Kdec lo 90,112 | E_last 106,496 (128 floats); 107,008 per slot = 1,672 per row and head, inside
 // the 2,176 the reference's prefill workspace formula provides (kernels/kda_prefill.cu:40-43, 695-698).  The last
 // 256 bytes of the workspace hold the counters (kda_internal.h).
@@ -48,9 +50,9 @@ using namespace pf;
 // thread holds a channel's rows) and its reader store and load consecutive cells.
 __device__ __forceinline__ int u_cell(int row4, int v) { return (((v >> 6) * 16 + row4) * 64 + (v & 63)) * 16; }
 // What the walk's loader brings in together lies together: U, or T' and V; Qg and W; M and Kdec.
-constexpr int wU = 0, wTp = 0, wV = kTile, wQg = 2 * kTile, wW = 3 * kTile, wMm = 4 * kTile, wKdHi = wMm + kTile / 2, wKdLo = wKdHi + kTile;
+constexpr int kTpBytes = 3 * kTile / 4, wU = 0, wTp = kTile - kTpBytes, wV = kTile, wQg = 2 * kTile, wW = 3 * kTile, wMm = 4 * kTile, wKdHi = wMm + kTile / 2, wKdLo = wKdHi + kTile;
 constexpr int kUBytes = CH * DV * 4, wEgl = wKdLo + kTile, kSlotBytes = wEgl + 512;
-static_assert(kSlotBytes == kPrefillSlotBytes && wV == kSlotInV && wTp == kSlotInK && kSlotInK + kTile <= wV && wU + kUBytes == wQg, "a chunk's V stays where the layer prologue put it; T' goes over K");
+static_assert(kSlotBytes == kPrefillSlotBytes && wV == kSlotInV && wTp >= kSlotInK && kSlotInK + kTile <= wV && wU + kUBytes == wQg, "a chunk's V stays where the layer prologue put it; T' goes over K");
 
 // Staging of a chunk's raw rows in the intra kernel: dense boxes of 64 rows x 128 bytes written by tiled tensor copies
 // with the 128-byte swizzle (16-byte piece p of row r sits at piece p ^ (r & 7)), so that threads walking down the
@@ -522,8 +524,13 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
                 }
                 *reinterpret_cast<uint4*>(gs + gTp + box_piece(i, c)) = make_uint4(wh[0], wh[1], wh[2], wh[3]);
                 if constexpr (WALK_U) {
-                    *reinterpret_cast<uint4*>(cell(slot + wTp, CH, c, i)) = make_uint4(wh[0], wh[1], wh[2], wh[3]);
-                    *reinterpret_cast<uint4*>(cell(slot + wTp + kBox, CH, c, i)) = make_uint4(wl[0], wl[1], wl[2], wl[3]);
+                    if (cc == 0) {
+                        *reinterpret_cast<uint4*>(cell(slot + wTp, CH, c, i)) = make_uint4(wh[0], wh[1], wh[2], wh[3]);
+                        *reinterpret_cast<uint4*>(cell(slot + wTp + kBox / 2, CH, c, i)) = make_uint4(wl[0], wl[1], wl[2], wl[3]);
+                    } else if (i >= CH / 2) {  // (above it there are only zeros)
+                        *reinterpret_cast<uint4*>(cell(slot + wTp + kBox, CH / 2, c - 4, i - CH / 2)) = make_uint4(wh[0], wh[1], wh[2], wh[3]);
+                        *reinterpret_cast<uint4*>(cell(slot + wTp + kBox + kBox / 4, CH / 2, c - 4, i - CH / 2)) = make_uint4(wl[0], wl[1], wl[2], wl[3]);
+                    }
                 } else {
                     *reinterpret_cast<uint4*>(gs + gTp + kBox + box_piece(i, c)) = make_uint4(wl[0], wl[1], wl[2], wl[3]);
                 }
@@ -1060,8 +1067,9 @@ __device__ void state_role(const SpParams& p, unsigned char* smem, const uint32_
                     if (!WALK_U || wk.use_u) {
                         const bool whole = walk_v && at.rows - c * CH >= CH;
                         if (!(ok = wait(bEmptyU, C ^ 1))) break;
-                        mbar_arrive_expect_tx(&bars[bFullU], kUBytes);
-                        bulk_load(smem + sU, slot + wU, whole ? kTile : kUBytes, &bars[bFullU]);
+                        constexpr int skip = WALK_U ? wTp : 0;
+                        mbar_arrive_expect_tx(&bars[bFullU], kUBytes - skip);
+                        bulk_load(smem + sU + skip, slot + wU + skip, (whole ? kTile : kUBytes) - skip, &bars[bFullU]);
                         for (int y = 0; whole && y < 2; ++y) tensor_load_3d(smem + sU + kTile + y * kBox, &p.tm_v, y * 64, at.h, (int)at.row + c * CH, &bars[bFullU]);
                     }
                     if (!(ok = wait(bEmptyMKd + x, (C >> 1) ^ 1))) break;
@@ -1069,7 +1077,7 @@ __device__ void state_role(const SpParams& p, unsigned char* smem, const uint32_
                     bulk_load(smem + sMKd + x * kMKd, slot + wMm, kMKd, &bars[bFullMKd + x]);
                     if (wk.use_u && c + 1 < at.count) {
                         const bool whole = walk_v && at.rows - (c + 1) * CH >= CH;
-                        bulk_prefetch(slot + kSlotBytes + wU, whole ? kTile : kUBytes);
+                        bulk_prefetch(slot + kSlotBytes + wU + (WALK_U ? wTp : 0), (whole ? kTile : kUBytes) - (WALK_U ? wTp : 0));
                         for (int y = 0; whole && y < 2; ++y) tensor_prefetch_3d(&p.tm_v, y * 64, at.h, (int)at.row + (c + 1) * CH);
                     }
                     if (gate_due && !(ok = load_gate(C - 1))) break;
@@ -1090,16 +1098,25 @@ __device__ void state_role(const SpParams& p, unsigned char* smem, const uint32_
         const uint32_t leader = tc::elect_one();
         auto ready = [&](int i, int phase) { return tc::warp_all(wait(i, phase)); };
         constexpr uint32_t idw = tc::idesc_bf16(DV, CH, 0, 1, 0), idq = tc::idesc_bf16(DV, CH, 0, 0, 0), ids = tc::idesc_bf16(DV, DK, 0, 1, 0);
-        constexpr uint32_t idv = tc::idesc_bf16(DV, CH, 1, 0, 0);
+        constexpr uint32_t idv = tc::idesc_bf16(DV, CH, 1, 0, 0), idv2 = tc::idesc_bf16(DV, CH / 2, 1, 0, 0);
         bool alive = true;
-        // U^T = V^T T'^T (T' hi, then lo).  Behind the wait for the D of the chunk before: the accumulator has been read.
+        // U^T = V^T T'^T (T' hi, then lo; the rows of V behind the 31st are of the rows of U behind it only).  Behind the wait for the D of the chunk before:
+        // the accumulator has been read.
         const bool walk_u = WALK_U && wk.use_u;
         bool have_u = false;  // the chunk to come's is on its way
         auto issue_u = [&]() {
             tc::fence_after_sync();
+            const unsigned char* tp = smem + sU + wTp;
 #pragma unroll
-            for (int k0 = 0; k0 < 2 * CH; k0 += 16)
-                tc::mma_bf16_if(leader, tm + tU, tc::desc_sw128_mnmajor(smem + sU + kTile, CH, k0 & (CH - 1)), tc::desc_kmajor_bf16(smem + sU + (k0 < CH ? 0 : kBox), CH, 0, k0 & (CH - 1)), idv, k0 > 0);
+            for (int lo = 0; lo < 2; ++lo) {
+#pragma unroll
+                for (int k0 = 0; k0 < CH / 2; k0 += 16)
+                    tc::mma_bf16_if(leader, tm + tU, tc::desc_sw128_mnmajor(smem + sU + kTile, CH, k0), tc::desc_kmajor_bf16(tp + lo * (kBox / 2), CH, 0, k0), idv, lo + k0 > 0);
+#pragma unroll
+                for (int k0 = 0; k0 < CH / 2; k0 += 16)
+                    tc::mma_bf16_if(leader, tm + tU + CH / 2, tc::desc_sw128_mnmajor(smem + sU + kTile, CH, CH / 2 + k0),
+                                    tc::desc_kmajor_bf16(tp + kBox + lo * (kBox / 4), CH / 2, 0, k0), idv2, true);
+            }
             tc::mma_commit_if(leader, &bars[bEmptyU]);
         };
         int C = 0;
