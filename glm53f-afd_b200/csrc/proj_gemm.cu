@@ -27,6 +27,9 @@
 // split over the blocks of a thread-block cluster, each with its own accumulator, and the blocks add the partial tiles,
 // each for some of the rows, in rank order through distributed shared memory (no scratch in global memory, the same bits every run).
 //
+// Two GEMMs that do not depend on one another share a launch without clusters where that is the shorter way (share_launch): a tile list for both, and a
+// split k is summed part after part by the tile's one block, the sums in tensor memory behind the two accumulators.  The same bits.
+//
 // Every wait is bounded (codes 130-135 in the device status word); TMEM is freed on every path; every block of a
 // cluster reaches the closing cluster barrier on every path.
 
@@ -48,31 +51,35 @@ constexpr int kBK = 64;             // k per stage: one 128-byte swizzle row of 
 constexpr int kGemmThreads = 192;   // producer, MMA, 4 epilogue warps
 constexpr int kEpiThreads = 128;
 constexpr int kABytes = kBM * 128;  // a stage's weight tile
+constexpr int kBlocksPerSm = 2;     // of any tile
 
 enum : int { kStatusGemmEmpty = 130, kStatusGemmFull = 131, kStatusGemmAccFull = 132, kStatusGemmAccEmpty = 133, kStatusGemmRedFull = 134, kStatusGemmRedEmpty = 135 };
 
-template <int NR, bool SPLIT>
+template <int NR, bool SPLIT, bool TWO = false>
 struct Cfg {
     static constexpr int kBBytes = NR * 128;
     static constexpr int kStageBytes = kABytes + kBBytes;
     static constexpr int kStages = SPLIT ? (NR == 16 ? 5 : NR == 32 ? 4 : 3) : (NR == 16 ? 6 : NR == 32 ? 5 : 4);
-    static constexpr int kTmemCols = 2 * NR < 32 ? 32 : 2 * NR;
+    static constexpr int kTmemCols = TWO ? 4 * NR : 2 * NR < 32 ? 32 : 2 * NR;  // two accumulators, and the sums of a split k
     static constexpr int kRedBytes = SPLIT ? kBM * NR * 4 : 0;  // this block's partial tile, f32 [NR][128]
     static constexpr int oRed = kStages * kStageBytes;
     static constexpr int oBars = oRed + kRedBytes;  // full[S], empty[S], acc_full[2], acc_empty[2], red_full, red_empty
     static constexpr int oCtl = oBars + (2 * kStages + 6) * 8;
     static constexpr int kBytes = oCtl + 16 + 1024;      // + slack to align the stages to 1024 bytes
-    static constexpr int kBlocksPerSm = 2;
 };
 
-struct GemmParams {
+struct GemmProblem {
     CUtensorMap tm_w, tm_x;
     void* out;
     long long ldo, o_gstride;
     int rows, n, kblocks, out_f32;
+    int segments;              // without a cluster: k runs in so many equal parts, each a sum of its own
     int n_tiles, r_tiles;
     int w_swapped, x_swapped;  // the map's coordinates are (k, group, row) instead of (k, row, group)
-    long long tiles;
+};
+struct GemmParams {
+    GemmProblem problem[2];    // the second: none, or (without clusters) another GEMM's tiles behind the first's
+    long long tiles0, tiles;
     int overlap;  // 0: alone; 1: the first of two independent launches; 2: the second (see glm53f_kda_proj_bf16_many)
     int* status;
 };
@@ -110,11 +117,26 @@ __device__ __forceinline__ float peer_load(uint32_t remote_addr) {
     return v;
 }
 
-// KS = blocks per cluster = K splits of a tile (1: no cluster).
-template <int NR, int KS>
-__global__ void __launch_bounds__(kGemmThreads, Cfg<NR, (KS > 1)>::kBlocksPerSm) proj_gemm_kernel(const __grid_constant__ GemmParams p) {
+// Tile t of the launch: its problem and its place there, the row tile fastest.
+struct GemmTile {
+    const GemmProblem& q;
+    int rt, nt, g;
+};
+template <bool TWO>
+__device__ __forceinline__ GemmTile gemm_tile(const GemmParams& p, long long t) {
+    const bool second = TWO && t >= p.tiles0;
+    const GemmProblem& q = p.problem[second ? 1 : 0];
+    const long long i = second ? t - p.tiles0 : t, u = i / q.r_tiles;
+    return {q, (int)(i % q.r_tiles), (int)(u % q.n_tiles), (int)(u / q.n_tiles)};
+}
+
+// KS = blocks per cluster = K splits of a tile (1: no cluster).  TWO: two problems, KS = 1 (an instance to itself: reading the parameters by a tile's problem
+// and the sums of a split k cost a launch of one 1 to 3 us).
+template <int NR, int KS, bool TWO>
+__global__ void __launch_bounds__(kGemmThreads, kBlocksPerSm) proj_gemm_kernel(const __grid_constant__ GemmParams p) {
     constexpr bool SPLIT = KS > 1;
-    using C = Cfg<NR, SPLIT>;
+    static_assert(!SPLIT || !TWO, "");
+    using C = Cfg<NR, SPLIT, TWO>;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + C::oBars);
@@ -126,7 +148,6 @@ __global__ void __launch_bounds__(kGemmThreads, Cfg<NR, (KS > 1)>::kBlocksPerSm)
     constexpr uint32_t ks = KS;
     const uint32_t kr = SPLIT ? cluster_rank() : 0u;
     const long long tile0 = blockIdx.x / ks, tile_step = gridDim.x / ks;
-    const int kb_n = p.kblocks / (int)ks, kb0 = (int)kr * kb_n;
     volatile uint32_t* ctl = reinterpret_cast<volatile uint32_t*>(smem + C::oCtl);
     uint32_t* tmem_slot = const_cast<uint32_t*>(ctl) + 2;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -147,8 +168,9 @@ __global__ void __launch_bounds__(kGemmThreads, Cfg<NR, (KS > 1)>::kBlocksPerSm)
     }
     if (warp == 1) tc::tmem_alloc(tmem_slot, C::kTmemCols);
     if (tid == 0) {
-        prefetch_tensormap(&p.tm_w);
-        prefetch_tensormap(&p.tm_x);
+        const GemmProblem& q = gemm_tile<TWO>(p, tile0).q;
+        prefetch_tensormap(&q.tm_w);
+        prefetch_tensormap(&q.tm_x);
     }
     tc::fence_before_sync();
     __syncthreads();
@@ -171,17 +193,16 @@ __global__ void __launch_bounds__(kGemmThreads, Cfg<NR, (KS > 1)>::kBlocksPerSm)
             int s = 0;
             uint32_t ph = 0;
             for (long long t = tile0; t < p.tiles; t += tile_step) {
-                const int rt = (int)(t % p.r_tiles);
-                const long long u = t / p.r_tiles;
-                const int nt = (int)(u % p.n_tiles), g = (int)(u / p.n_tiles);
+                const GemmTile x = gemm_tile<TWO>(p, t);
+                const int kb_n = x.q.kblocks / (int)ks, kb0 = (int)kr * kb_n;
+                const void *mw = &x.q.tm_w, *mx = &x.q.tm_x;
+                const bool ws = x.q.w_swapped != 0, xs = x.q.x_swapped != 0;
                 for (int kb = kb0; kb < kb0 + kb_n; ++kb) {
                     if (!mbar_wait(&empty[s], ph ^ 1u, ctx, kStatusGemmEmpty)) goto done;
                     unsigned char* st = smem + s * C::kStageBytes;
                     mbar_arrive_expect_tx(&full[s], C::kStageBytes);
-                    if (p.w_swapped) tensor_load_3d(st, &p.tm_w, kb * kBK, g, nt * kBM, &full[s]);
-                    else tensor_load_3d(st, &p.tm_w, kb * kBK, nt * kBM, g, &full[s]);
-                    if (p.x_swapped) tensor_load_3d(st + kABytes, &p.tm_x, kb * kBK, g, rt * NR, &full[s]);
-                    else tensor_load_3d(st + kABytes, &p.tm_x, kb * kBK, rt * NR, g, &full[s]);
+                    tensor_load_3d(st, mw, kb * kBK, ws ? x.g : x.nt * kBM, ws ? x.nt * kBM : x.g, &full[s]);
+                    tensor_load_3d(st + kABytes, mx, kb * kBK, xs ? x.g : x.rt * NR, xs ? x.rt * NR : x.g, &full[s]);
                     if (++s == C::kStages) {
                         s = 0;
                         ph ^= 1u;
@@ -196,61 +217,98 @@ __global__ void __launch_bounds__(kGemmThreads, Cfg<NR, (KS > 1)>::kBlocksPerSm)
         int s = 0, buf = 0;
         uint32_t ph = 0, acc_ph[2] = {0, 0};
         for (long long t = tile0; t < p.tiles; t += tile_step) {
-            if (!tc::warp_all(mbar_wait(&acc_empty[buf], acc_ph[buf] ^ 1u, ctx, kStatusGemmAccEmpty))) goto done;
-            tc::fence_after_sync();
-            const uint32_t d = tm + (uint32_t)(buf * NR);
-            for (int kb = 0; kb < kb_n; ++kb) {
-                if (!tc::warp_all(mbar_wait(&full[s], ph, ctx, kStatusGemmFull))) goto done;
+            const GemmProblem& q = gemm_tile<TWO>(p, t).q;
+            const int segments = TWO ? q.segments : 1, kb_n = q.kblocks / (SPLIT ? (int)ks : segments);
+            for (int seg = 0; seg < segments; ++seg) {
+                if (!tc::warp_all(mbar_wait(&acc_empty[buf], acc_ph[buf] ^ 1u, ctx, kStatusGemmAccEmpty))) goto done;
                 tc::fence_after_sync();
-                const unsigned char* st = smem + s * C::kStageBytes;
+                const uint32_t d = tm + (uint32_t)(buf * NR);
+                for (int kb = 0; kb < kb_n; ++kb) {
+                    if (!tc::warp_all(mbar_wait(&full[s], ph, ctx, kStatusGemmFull))) goto done;
+                    tc::fence_after_sync();
+                    const unsigned char* st = smem + s * C::kStageBytes;
 #pragma unroll
-                for (int i = 0; i < kBK / 16; ++i)
-                    tc::mma_bf16_if(leader, d, tc::desc_sw128_kmajor(st, kBM, 16 * i), tc::desc_sw128_kmajor(st + kABytes, NR, 16 * i), idesc, kb > 0 || i > 0);
-                tc::mma_commit_if(leader, &empty[s]);
-                if (++s == C::kStages) {
-                    s = 0;
-                    ph ^= 1u;
+                    for (int i = 0; i < kBK / 16; ++i)
+                        tc::mma_bf16_if(leader, d, tc::desc_sw128_kmajor(st, kBM, 16 * i), tc::desc_sw128_kmajor(st + kABytes, NR, 16 * i), idesc, kb > 0 || i > 0);
+                    tc::mma_commit_if(leader, &empty[s]);
+                    if (++s == C::kStages) {
+                        s = 0;
+                        ph ^= 1u;
+                    }
                 }
+                tc::mma_commit_if(leader, &acc_full[buf]);
+                acc_ph[buf] ^= 1u;
+                buf ^= 1;
+                if (leader) ctl[0] = ctl[0] + 1u;
             }
-            tc::mma_commit_if(leader, &acc_full[buf]);
-            acc_ph[buf] ^= 1u;
-            buf ^= 1;
-            if (leader) ctl[0] = ctl[0] + 1u;
         }
     } else {
         const int q = warp & 3;  // the TMEM lane quarter this warp may read
         int buf = 0;
         uint32_t acc_ph[2] = {0, 0}, red_ph = 0;
         for (long long t = tile0; t < p.tiles; t += tile_step) {
-            const int rt = (int)(t % p.r_tiles);
-            const long long u = t / p.r_tiles;
-            const int nt = (int)(u % p.n_tiles), g = (int)(u / p.n_tiles);
+            const GemmTile tile = gemm_tile<TWO>(p, t);
+            const GemmProblem& x = tile.q;
             if (!mbar_wait(&acc_full[buf], acc_ph[buf], ctx, kStatusGemmAccFull)) goto done;
             acc_ph[buf] ^= 1u;
             tc::fence_after_sync();
-            const int fl = q * 32 + lane, f = nt * kBM + fl;
-            const bool f_ok = f < p.n;
-            const long long row0 = (long long)rt * NR;
-            unsigned char* base = reinterpret_cast<unsigned char*>(p.out) + ((long long)g * p.o_gstride + f) * (p.out_f32 ? 4 : 2);
+            const int fl = q * 32 + lane, f = tile.nt * kBM + fl;
+            const bool f_ok = f < x.n;
+            const long long row0 = (long long)tile.rt * NR;
+            const long long ldo = x.ldo;
+            const int rows = x.rows, out_f32 = x.out_f32;
+            unsigned char* base = reinterpret_cast<unsigned char*>(x.out) + ((long long)tile.g * x.o_gstride + f) * (out_f32 ? 4 : 2);
             auto store = [&](int c, float v) {
                 const long long row = row0 + c;
-                if (f_ok && row < p.rows) {
-                    if (p.out_f32) *reinterpret_cast<float*>(base + row * p.ldo * 4) = v;
-                    else *reinterpret_cast<uint16_t*>(base + row * p.ldo * 2) = f32_to_bf16_bits(v);
+                if (f_ok && row < rows) {
+                    if (out_f32) *reinterpret_cast<float*>(base + row * ldo * 4) = v;
+                    else *reinterpret_cast<uint16_t*>(base + row * ldo * 2) = f32_to_bf16_bits(v);
                 }
             };
-            if constexpr (!SPLIT) {
-#pragma unroll 1
-                for (int c0 = 0; c0 < NR; c0 += 16) {
-                    uint32_t r[16];
-                    tc::tmem_ld16(tc::tmem_addr(tm, q, buf * NR + c0), r);
-                    tc::tmem_ld_wait();
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) store(c0 + j, __uint_as_float(r[j]));
-                }
+            auto release = [&] {
                 tc::fence_before_sync();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&acc_empty[buf]);
+            };
+            if constexpr (!SPLIT) {
+                if (!TWO || x.segments == 1) {
+#pragma unroll 1
+                    for (int c0 = 0; c0 < NR; c0 += 16) {
+                        uint32_t r[16];
+                        tc::tmem_ld16(tc::tmem_addr(tm, q, buf * NR + c0), r);
+                        tc::tmem_ld_wait();
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) store(c0 + j, __uint_as_float(r[j]));
+                    }
+                    release();
+                } else {  // the parts of k, added in their order, the sums in tensor memory behind the accumulators
+                    for (int seg = 0; seg < x.segments; ++seg) {
+                        if (seg > 0) {
+                            buf ^= 1;
+                            if (!mbar_wait(&acc_full[buf], acc_ph[buf], ctx, kStatusGemmAccFull)) goto done;
+                            acc_ph[buf] ^= 1u;
+                            tc::fence_after_sync();
+                        }
+#pragma unroll 1
+                        for (int c0 = 0; c0 < NR; c0 += 16) {
+                            uint32_t r[16], sum[16];
+                            tc::tmem_ld16(tc::tmem_addr(tm, q, buf * NR + c0), r);
+                            if (seg > 0) tc::tmem_ld16(tc::tmem_addr(tm, q, 2 * NR + c0), sum);
+                            tc::tmem_ld_wait();
+                            if (seg > 0)
+#pragma unroll
+                                for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(__uint_as_float(sum[j]) + __uint_as_float(r[j]));
+                            if (seg + 1 < x.segments) {
+                                tc::tmem_st16(tc::tmem_addr(tm, q, 2 * NR + c0), r);
+                            } else {
+#pragma unroll
+                                for (int j = 0; j < 16; ++j) store(c0 + j, __uint_as_float(r[j]));
+                            }
+                        }
+                        tc::tmem_st_wait();
+                        release();
+                    }
+                }
             } else {
                 // The tile's K splits live in the blocks of this cluster.  Every block parks its partial tile in its own shared
                 // memory and then finishes NR / KS of the tile's rows: it adds the blocks' partials in rank order (a fixed order:
@@ -354,14 +412,14 @@ int pick_ksplit(long long tiles, int kblocks, long long resident) {
     return 1;
 }
 
-template <int NR, int KS>
+template <int NR, int KS, bool TWO = false>
 int launch_one(GemmParams& p, long long clusters, cudaStream_t stream) {
-    using C = Cfg<NR, (KS > 1)>;
+    using C = Cfg<NR, (KS > 1), TWO>;
     static int configured_dev = -1;
     int dev = 0;
     cudaGetDevice(&dev);
     if (configured_dev != dev) {
-        const cudaError_t e = cudaFuncSetAttribute(proj_gemm_kernel<NR, KS>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kBytes);
+        const cudaError_t e = cudaFuncSetAttribute(proj_gemm_kernel<NR, KS, TWO>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kBytes);
         if (e != cudaSuccess) return (int)e;
         configured_dev = dev;
     }
@@ -383,23 +441,47 @@ int launch_one(GemmParams& p, long long clusters, cudaStream_t stream) {
     }
     cfg.attrs = attr;
     cfg.numAttrs = na;
-    return (int)cudaLaunchKernelEx(&cfg, proj_gemm_kernel<NR, KS>, p);
+    return (int)cudaLaunchKernelEx(&cfg, proj_gemm_kernel<NR, KS, TWO>, p);
 }
 
-template <int NR>
-int launch_gemm(GemmParams& p, const void* x, long long ldx, long long x_gstride, int groups, int k, cudaStream_t stream) {
-    if (!matrix_map(&p.tm_x, &p.x_swapped, x, k, p.rows, groups, ldx, x_gstride, NR)) return (int)cudaErrorNotSupported;
-    p.r_tiles = (p.rows + NR - 1) / NR;
-    p.tiles = (long long)groups * p.n_tiles * p.r_tiles;
-    const long long cap = (long long)sm_count() * Cfg<NR, false>::kBlocksPerSm;
+// The GEMM `j` as a launch's problem with tiles of nr rows; its tiles, 0 where it has no such form.
+long long few_rows_problem(GemmProblem& q, const glm53f_proj_job& j, int nr) {
+    q.out = j.out;
+    q.ldo = j.ldo;
+    q.o_gstride = j.groups > 1 ? j.o_gstride : 0;
+    q.rows = j.rows;
+    q.n = j.n;
+    q.kblocks = j.k / kBK;
+    q.out_f32 = j.out_f32 != 0;
     // The split is chosen for ONE row tile, whatever the launch's row count: a row's bits then depend on (groups, n, k) only.
-    const int ks = pick_ksplit((long long)groups * p.n_tiles, p.kblocks, sm_count());  // clusters were measured at one block per SM
+    q.n_tiles = (j.n + kBM - 1) / kBM;
+    q.r_tiles = (j.rows + nr - 1) / nr;
+    q.segments = pick_ksplit((long long)j.groups * q.n_tiles, q.kblocks, sm_count());  // clusters were measured at one block per SM
+    if (!matrix_map(&q.tm_w, &q.w_swapped, j.w, j.k, j.n, j.groups, j.ldw, j.w_gstride, kBM) ||
+        !matrix_map(&q.tm_x, &q.x_swapped, j.x, j.k, j.rows, j.groups, j.ldx, j.x_gstride, nr))
+        return 0;
+    return (long long)j.groups * q.n_tiles * q.r_tiles;
+}
+
+// One GEMM, or (b) two that share a launch without clusters.
+template <int NR>
+int launch_gemm(GemmParams& p, const glm53f_proj_job& a, const glm53f_proj_job* b, cudaStream_t stream) {
+    p.tiles = p.tiles0 = few_rows_problem(p.problem[0], a, NR);
+    if (p.tiles0 == 0) return (int)cudaErrorNotSupported;
+    const long long cap = (long long)sm_count() * kBlocksPerSm;
+    if (b != nullptr) {
+        const long long more = few_rows_problem(p.problem[1], *b, NR);
+        if (more == 0) return (int)cudaErrorNotSupported;
+        p.tiles += more;
+        return launch_one<NR, 1, true>(p, p.tiles < cap ? p.tiles : cap, stream);
+    }
+    const int ks = p.problem[0].segments;
     const long long fit = cap / ks;
     const long long clusters = p.tiles < fit ? p.tiles : fit;
     if (ks == 8) return launch_one<NR, 8>(p, clusters, stream);
     if (ks == 4) return launch_one<NR, 4>(p, clusters, stream);
     if (ks == 2) return launch_one<NR, 2>(p, clusters, stream);
-    return launch_one<NR, 1>(p, p.tiles < cap ? p.tiles : cap, stream);
+    return launch_one<NR, 1>(p, clusters, stream);
 }
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
@@ -469,22 +551,22 @@ int check_job(const glm53f_proj_job& j) {
     return 0;
 }
 
-int few_rows(const glm53f_proj_job& j, int overlap, int* status, cudaStream_t stream) {
+int few_rows(const glm53f_proj_job& a, const glm53f_proj_job* b, int overlap, int* status, cudaStream_t stream) {
     GemmParams p{};
-    p.out = j.out;
-    p.ldo = j.ldo;
-    p.o_gstride = j.groups > 1 ? j.o_gstride : 0;
-    p.rows = j.rows;
-    p.n = j.n;
-    p.kblocks = j.k / kBK;
-    p.out_f32 = j.out_f32 != 0;
-    p.n_tiles = (j.n + kBM - 1) / kBM;
     p.overlap = overlap;
     p.status = status;
-    if (!matrix_map(&p.tm_w, &p.w_swapped, j.w, j.k, j.n, j.groups, j.ldw, j.w_gstride, kBM)) return (int)cudaErrorNotSupported;
-    if (j.rows <= 16) return launch_gemm<16>(p, j.x, j.ldx, j.x_gstride, j.groups, j.k, stream);
-    if (j.rows <= 32) return launch_gemm<32>(p, j.x, j.ldx, j.x_gstride, j.groups, j.k, stream);
-    return launch_gemm<64>(p, j.x, j.ldx, j.x_gstride, j.groups, j.k, stream);
+    const int rows = b != nullptr && b->rows > a.rows ? b->rows : a.rows;
+    if (rows <= 16) return launch_gemm<16>(p, a, b, stream);
+    if (rows <= 32) return launch_gemm<32>(p, a, b, stream);
+    return launch_gemm<64>(p, a, b, stream);
+}
+
+// Whether two GEMMs of few rows are one launch, the parts of a split k one after another in one block each: where one of them has tiles enough by itself
+// and the other one's are no longer than its.  (As two launches side by side, the second not waiting for the first, the 4096 -> 256 factor cost nearly all of
+// its own time beside the fused projection: both and the second factor 45.5 us at 16 rows, 41.2 so; 58.5 and 46.6 at 64.)
+bool share_launch(const glm53f_proj_job& a, const glm53f_proj_job& b) {
+    const int ka = k_segments(a), kb = k_segments(b);
+    return (ka == 1 && b.k <= a.k) || (kb == 1 && a.k <= b.k);
 }
 
 }  // namespace
@@ -503,8 +585,10 @@ extern "C" int32_t glm53f_kda_proj_bf16_many(const glm53f_proj_job* jobs, int32_
         const bool two = i + 1 < count && jobs[i + 1].rows > 0 && (jobs[i + 1].rows <= kFewRows) == (j.rows <= kFewRows);
         int rc = 0;
         if (j.rows <= kFewRows || (!two && j.rows <= kFewRowsSplit && k_segments(j) > 1)) {
-            rc = few_rows(j, two ? 1 : 0, status, stream);
-            if (rc == 0 && two) rc = few_rows(jobs[++i], 2, status, stream);
+            const bool share = two && share_launch(j, jobs[i + 1]);
+            rc = few_rows(j, share ? &jobs[i + 1] : nullptr, two && !share ? 1 : 0, status, stream);
+            if (rc == 0 && two && !share) rc = few_rows(jobs[i + 1], nullptr, 2, status, stream);
+            i += two ? 1 : 0;
         } else {
             PairProblem q[kPairProblems];
             if (!pair_problem(q[0], j) || (two && !pair_problem(q[1], jobs[i + 1]))) return (int)cudaErrorNotSupported;

@@ -42,3 +42,29 @@ def test_many_equals_one_by_one(rows):
     bad = (ffi.ProjJob * 2)(jobs[0][0], jobs[1][0])
     bad[1].k = 100
     assert lib.glm53f_kda_proj_bf16_many(bad, 2, stream) == 1  # checked before anything is launched
+
+
+@pytest.mark.parametrize("rows", [1, 16, 17, 32, 33, 64])
+@pytest.mark.parametrize("shapes", [[(1, 256, 1024), (1, 1112, 1024)], [(1, 9608, 512), (1, 264, 512)], [(2, 4808, 128), (1, 9600, 256)], [(1, 256, 4096), (1, 9600, 4096)]])
+def test_few_rows_share_a_launch(rows, shapes):
+    """Two GEMMs of few rows whose tiles share a launch, and one that has to stay apart (both split): with a split k (its parts summed by one block then),
+    without, ragged features and rows; the bits of each alone."""
+    ffi = importlib.import_module("glm53f-afd_b200.ffi")
+    lib, g = ffi.load(), torch.Generator(device="cuda").manual_seed(rows)
+    mk = lambda *s: (torch.randn(*s, device="cuda", generator=g) * 0.1).bfloat16()
+    jobs, outs, keep = [], [], []
+    for f32, (groups, n, k) in enumerate(shapes):
+        x, w = mk(rows, groups * k), mk(groups, n, k)
+        ldo, kind = groups * n + 8, torch.float32 if f32 else torch.bfloat16
+        pair = [torch.full((rows * ldo + 64,), 3.0, dtype=kind, device="cuda") for _ in range(2)]
+        keep.append((x, w))
+        outs.append(pair)
+        jobs.append([ffi.ProjJob(x.data_ptr(), groups * k, k, w.data_ptr(), k, n * k, groups, rows, n, k, o.data_ptr(), f32, ldo, n) for o in pair])
+    stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    assert lib.glm53f_kda_proj_bf16_many((ffi.ProjJob * 2)(*[j[0] for j in jobs]), 2, stream) == 0
+    for j in jobs:
+        assert lib.glm53f_kda_proj_bf16(*(getattr(j[1], f) for f, _ in ffi.ProjJob._fields_), stream) == 0
+    torch.cuda.synchronize()
+    assert importlib.import_module("glm53f-afd_b200.core").device_status() == 0
+    for a, b in outs:
+        assert torch.equal(a, b)
