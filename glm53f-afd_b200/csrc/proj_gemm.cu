@@ -7,7 +7,7 @@
 // low-rank gate pair 4096 -> 256 -> 2 x 8192; 3772-3790: o_proj 8192 -> 4096).
 //
 // Shape of the kernel.  The weight is the M operand: a tile is 128 output features x NR activation rows, NR in
-// {16, 32, 64} chosen from the row count (more rows: proj_gemm_pair.cu), so a decode step's 16 rows waste nothing and the weight -- which
+// {16, 32, 64, 96} chosen from the row count (more rows: proj_gemm_pair.cu), so a decode step's 16 rows waste nothing and the weight -- which
 // dominates the traffic at few rows (202 MB for the fused projection) -- streams through once.  Both operands are
 // K-major in global memory ([o][k] and [r][k]), so tiled tensor copies in the 128-byte swizzle feed tcgen05.mma
 // in place: a stage is 64 k of the weight tile (16 KiB) and of the row tile (NR x 128 bytes).  Roles per block:
@@ -59,8 +59,12 @@ template <int NR, bool SPLIT, bool TWO = false>
 struct Cfg {
     static constexpr int kBBytes = NR * 128;
     static constexpr int kStageBytes = kABytes + kBBytes;
-    static constexpr int kStages = SPLIT ? (NR == 16 ? 5 : NR == 32 ? 4 : 3) : (NR == 16 ? 6 : NR == 32 ? 5 : 4);
-    static constexpr int kTmemCols = TWO ? 4 * NR : 2 * NR < 32 ? 32 : 2 * NR;  // two accumulators, and the sums of a split k
+    static constexpr int kStages = SPLIT ? (NR == 16 ? 5 : NR == 32 ? 4 : 3) : (NR == 16 ? 6 : NR == 32 ? 5 : NR <= 64 ? 4 : 3);
+    // Tensor memory columns: two accumulators kAcc apart and (TWO) the sums of a split k.  With tiles of more than 64 rows there are no columns left for those where
+    // two blocks share an SM: the parts then come one after the other in one accumulator, the sums lie in the other.
+    static constexpr int kAcc = NR <= 64 ? NR : 128;
+    static constexpr bool kApart = NR <= 64;
+    static constexpr int kTmemCols = TWO && kApart ? 4 * kAcc : 2 * kAcc;
     static constexpr int kRedBytes = SPLIT ? kBM * NR * 4 : 0;  // this block's partial tile, f32 [NR][128]
     static constexpr int oRed = kStages * kStageBytes;
     static constexpr int oBars = oRed + kRedBytes;  // full[S], empty[S], acc_full[2], acc_empty[2], red_full, red_empty
@@ -222,7 +226,7 @@ __global__ void __launch_bounds__(kGemmThreads, kBlocksPerSm) proj_gemm_kernel(c
             for (int seg = 0; seg < segments; ++seg) {
                 if (!tc::warp_all(mbar_wait(&acc_empty[buf], acc_ph[buf] ^ 1u, ctx, kStatusGemmAccEmpty))) goto done;
                 tc::fence_after_sync();
-                const uint32_t d = tm + (uint32_t)(buf * NR);
+                const uint32_t d = tm + (uint32_t)(buf * C::kAcc);
                 for (int kb = 0; kb < kb_n; ++kb) {
                     if (!tc::warp_all(mbar_wait(&full[s], ph, ctx, kStatusGemmFull))) goto done;
                     tc::fence_after_sync();
@@ -238,7 +242,7 @@ __global__ void __launch_bounds__(kGemmThreads, kBlocksPerSm) proj_gemm_kernel(c
                 }
                 tc::mma_commit_if(leader, &acc_full[buf]);
                 acc_ph[buf] ^= 1u;
-                buf ^= 1;
+                if (C::kApart || segments == 1) buf ^= 1;
                 if (leader) ctl[0] = ctl[0] + 1u;
             }
         }
@@ -275,31 +279,32 @@ __global__ void __launch_bounds__(kGemmThreads, kBlocksPerSm) proj_gemm_kernel(c
 #pragma unroll 1
                     for (int c0 = 0; c0 < NR; c0 += 16) {
                         uint32_t r[16];
-                        tc::tmem_ld16(tc::tmem_addr(tm, q, buf * NR + c0), r);
+                        tc::tmem_ld16(tc::tmem_addr(tm, q, buf * C::kAcc + c0), r);
                         tc::tmem_ld_wait();
 #pragma unroll
                         for (int j = 0; j < 16; ++j) store(c0 + j, __uint_as_float(r[j]));
                     }
                     release();
-                } else {  // the parts of k, added in their order, the sums in tensor memory behind the accumulators
+                } else {  // the parts of k, added in their order
                     for (int seg = 0; seg < x.segments; ++seg) {
                         if (seg > 0) {
-                            buf ^= 1;
+                            if (C::kApart) buf ^= 1;
                             if (!mbar_wait(&acc_full[buf], acc_ph[buf], ctx, kStatusGemmAccFull)) goto done;
                             acc_ph[buf] ^= 1u;
                             tc::fence_after_sync();
                         }
+                        const int sums = C::kApart ? 2 * C::kAcc : (buf ^ 1) * C::kAcc;
 #pragma unroll 1
                         for (int c0 = 0; c0 < NR; c0 += 16) {
                             uint32_t r[16], sum[16];
-                            tc::tmem_ld16(tc::tmem_addr(tm, q, buf * NR + c0), r);
-                            if (seg > 0) tc::tmem_ld16(tc::tmem_addr(tm, q, 2 * NR + c0), sum);
+                            tc::tmem_ld16(tc::tmem_addr(tm, q, buf * C::kAcc + c0), r);
+                            if (seg > 0) tc::tmem_ld16(tc::tmem_addr(tm, q, sums + c0), sum);
                             tc::tmem_ld_wait();
                             if (seg > 0)
 #pragma unroll
                                 for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(__uint_as_float(sum[j]) + __uint_as_float(r[j]));
                             if (seg + 1 < x.segments) {
-                                tc::tmem_st16(tc::tmem_addr(tm, q, 2 * NR + c0), r);
+                                tc::tmem_st16(tc::tmem_addr(tm, q, sums + c0), r);
                             } else {
 #pragma unroll
                                 for (int j = 0; j < 16; ++j) store(c0 + j, __uint_as_float(r[j]));
@@ -308,6 +313,7 @@ __global__ void __launch_bounds__(kGemmThreads, kBlocksPerSm) proj_gemm_kernel(c
                         tc::tmem_st_wait();
                         release();
                     }
+                    if (!C::kApart) buf ^= 1;  // (back at the end: the next tile takes the same accumulator)
                 }
             } else {
                 // The tile's K splits live in the blocks of this cluster.  Every block parks its partial tile in its own shared
@@ -325,7 +331,7 @@ __global__ void __launch_bounds__(kGemmThreads, kBlocksPerSm) proj_gemm_kernel(c
 #pragma unroll 1
                 for (int c0 = 0; c0 < NR; c0 += 16) {
                     uint32_t r[16];
-                    tc::tmem_ld16(tc::tmem_addr(tm, q, buf * NR + c0), r);
+                    tc::tmem_ld16(tc::tmem_addr(tm, q, buf * C::kAcc + c0), r);
                     tc::tmem_ld_wait();
 #pragma unroll
                     for (int j = 0; j < 16; ++j) red[(c0 + j) * kBM] = __uint_as_float(r[j]);
@@ -377,7 +383,8 @@ done:
     }
 }
 
-constexpr int kFewRows = 64;        // launches of up to this many rows run here, larger ones on SM pairs
+constexpr int kFewRows = 96;        // launches of up to this many rows run here, larger ones on SM pairs (a layer's four at 80 rows 75.4 us, on pairs 77.9; at 128 with tiles
+                                    // of 128 rows, which leave the sums of a split k no columns of their own, 80.0 and 79.5)
 // ... and a K-split shape by itself up to here: its splits run side by side on a cluster, on a pair one after another (o_proj at
 // 128 rows: 36 us on pairs, 24 so)
 constexpr int kFewRowsSplit = 128;
@@ -478,9 +485,11 @@ int launch_gemm(GemmParams& p, const glm53f_proj_job& a, const glm53f_proj_job* 
     const int ks = p.problem[0].segments;
     const long long fit = cap / ks;
     const long long clusters = p.tiles < fit ? p.tiles : fit;
-    if (ks == 8) return launch_one<NR, 8>(p, clusters, stream);
-    if (ks == 4) return launch_one<NR, 4>(p, clusters, stream);
-    if (ks == 2) return launch_one<NR, 2>(p, clusters, stream);
+    if constexpr (NR <= 64) {
+        if (ks == 8) return launch_one<NR, 8>(p, clusters, stream);
+        if (ks == 4) return launch_one<NR, 4>(p, clusters, stream);
+        if (ks == 2) return launch_one<NR, 2>(p, clusters, stream);
+    }
     return launch_one<NR, 1>(p, clusters, stream);
 }
 
@@ -558,7 +567,8 @@ int few_rows(const glm53f_proj_job& a, const glm53f_proj_job* b, int overlap, in
     const int rows = b != nullptr && b->rows > a.rows ? b->rows : a.rows;
     if (rows <= 16) return launch_gemm<16>(p, a, b, stream);
     if (rows <= 32) return launch_gemm<32>(p, a, b, stream);
-    return launch_gemm<64>(p, a, b, stream);
+    if (rows <= 64 || (b == nullptr && k_segments(a) > 1)) return launch_gemm<64>(p, a, b, stream);
+    return launch_gemm<96>(p, a, b, stream);
 }
 
 // Whether two GEMMs of few rows are one launch, the parts of a split k one after another in one block each: where one of them has tiles enough by itself

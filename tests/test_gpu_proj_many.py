@@ -44,7 +44,7 @@ def test_many_equals_one_by_one(rows):
     assert lib.glm53f_kda_proj_bf16_many(bad, 2, stream) == 1  # checked before anything is launched
 
 
-@pytest.mark.parametrize("rows", [1, 16, 17, 32, 33, 64])
+@pytest.mark.parametrize("rows", [1, 16, 17, 32, 33, 64, 65, 96])
 @pytest.mark.parametrize("shapes", [[(1, 256, 1024), (1, 1112, 1024)], [(1, 9608, 512), (1, 264, 512)], [(2, 4808, 128), (1, 9600, 256)], [(1, 256, 4096), (1, 9600, 4096)]])
 def test_few_rows_share_a_launch(rows, shapes):
     """Two GEMMs of few rows whose tiles share a launch, and one that has to stay apart (both split): with a split k (its parts summed by one block then),
