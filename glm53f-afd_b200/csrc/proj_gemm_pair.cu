@@ -12,7 +12,7 @@
 //   MMA (warp 1 of the leader)      one thread issues the pair's MMAs (M = 256, N = NR, K = 16) and commits each stage
 //                                   to both blocks' `empty` barriers, each finished accumulator to both `acc_full` barriers;
 //   epilogue (warps 2-9, both)      each block drains its own 128 features x NR rows from its tensor memory, through
-//                                   shared memory (a thread holds ONE feature of sixteen rows; rows of 64 features leave as
+//                                   shared memory (transposing matrix stores; rows of 64 features leave as
 //                                   tiled tensor stores), and arrives on the leader's `acc_empty`.
 // The epilogue's way out was what bounded wide launches: with two-byte stores straight from the registers a 256 x 256 tile
 // took 17 us to leave, as long as a k of 4,096 takes to compute, and the k = 128 gate factor (67 MB of results at 2,048 rows)
@@ -234,7 +234,27 @@ __global__ void __launch_bounds__(kPairThreads, 1) proj_gemm_pair_kernel(const _
         const bool issuer = (q & 1) == 0 && lane == 0;      // issues the boxes' tensor stores
         int buf = 0, out_buf = 0;
         uint32_t acc_ph[2] = {0, 0};
-        // The tile's rows c0 .. c0 + 31 (those below row_tile) out: lane = feature, v[j] = row c0 + j.
+        // Sixteen rows of the accumulator from c0 on.  For tensor stores in the fragment layout, from which transposing matrix stores put rows of eight
+        // features into the boxes: v[8 h + 4 g + 2 p + e] = feature 16 h + 8 p + lane / 4 of the warp, row c0 + 8 g + 2 (lane % 4) + e.  (With lane = feature, 32
+        // two-byte stores where four are enough now: the k = 128 gate factor at 512 rows
+        // 13.8 -> 12.5 us, at 1,024 24.5 -> 21.3.)  Else lane = feature, v[j] = row c0 + j.
+        auto load = [&](const PairTile& x, int c0, float* v) {
+            uint32_t r[16];
+            if (x.q.tensor_out) {
+                uint32_t a[8], b[8];
+                tc::tmem_ld_frag(tc::tmem_addr(tm, q, buf * kPN + c0), a);
+                tc::tmem_ld_frag(tc::tmem_addr(tm, q, buf * kPN + c0) + (16u << 16), b);
+                tc::tmem_ld_wait();
+#pragma unroll
+                for (int j = 0; j < 8; ++j) r[j] = a[j], r[8 + j] = b[j];
+            } else {
+                tc::tmem_ld16(tc::tmem_addr(tm, q, buf * kPN + c0), r);
+                tc::tmem_ld_wait();
+            }
+#pragma unroll
+            for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
+        };
+        // The tile's rows c0 .. c0 + 31 (those below row_tile) out, as load() gave them.
         auto emit = [&](const PairTile& x, int c0, const float (&v)[kChunk]) {
             const long long row0 = (long long)x.rt * x.q.row_tile + c0;
             const int f0 = x.nt * 2 * kPM + (int)rank * kPM + side * 64;
@@ -244,12 +264,16 @@ __global__ void __launch_bounds__(kPairThreads, 1) proj_gemm_pair_kernel(const _
                 out_buf ^= 1;
                 if (issuer) bulk_wait_read<1>();  // this buffer's last stores have been read
                 named_bar_sync(bar, 64);
+                // A lane names row lane % 8 of matrix lane / 8: features 8 ((lane / 8) % 2), rows 8 (lane / 16) of the sixteen by sixteen.
+                const int row = (lane >> 4) * 8 + (lane & 7), piece = (q & 1) * 4 + ((lane >> 3) & 1);
 #pragma unroll
-                for (int j = 0; j < kChunk; j += 2) {
-                    const uint32_t two = tc::bf16x2(v[j], v[j + 1]);
-                    *reinterpret_cast<uint16_t*>(box + j * 128 + (((fl >> 3) ^ (j & 7)) << 4) + (fl & 7) * 2) = (uint16_t)two;
-                    *reinterpret_cast<uint16_t*>(box + (j + 1) * 128 + (((fl >> 3) ^ ((j + 1) & 7)) << 4) + (fl & 7) * 2) = (uint16_t)(two >> 16);
-                }
+                for (int c = 0; c < 2; ++c)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const float* w = v + 16 * c + 8 * h;
+                        tc::stmatrix_t4(box + (16 * c + row) * 128 + (((piece + 2 * h) ^ (row & 7)) << 4), tc::bf16x2(w[0], w[1]), tc::bf16x2(w[2], w[3]), tc::bf16x2(w[4], w[5]),
+                                        tc::bf16x2(w[6], w[7]));
+                    }
                 fence_proxy_async_smem();
                 named_bar_sync(bar, 64);
                 if (issuer) {
@@ -298,12 +322,9 @@ __global__ void __launch_bounds__(kPairThreads, 1) proj_gemm_pair_kernel(const _
             if (x.q.segments == 1) {
                 if (!arrived()) goto done;
                 for (int c0 = set * kChunk; c0 < x.q.row_tile; c0 += 2 * kChunk) {
-                    uint32_t r[kChunk];
-                    tc::tmem_ld32(tc::tmem_addr(tm, q, buf * kPN + c0), r);
-                    tc::tmem_ld_wait();
                     float v[kChunk];
-#pragma unroll
-                    for (int j = 0; j < kChunk; ++j) v[j] = __uint_as_float(r[j]);
+                    load(x, c0, v);
+                    load(x, c0 + 16, v + 16);
                     emit(x, c0, v);
                 }
                 release();
@@ -317,11 +338,10 @@ __global__ void __launch_bounds__(kPairThreads, 1) proj_gemm_pair_kernel(const _
                         if (c0 >= x.q.row_tile) break;
 #pragma unroll
                         for (int j0 = 0; j0 < kChunk; j0 += 16) {
-                            uint32_t r[16];
-                            tc::tmem_ld16(tc::tmem_addr(tm, q, buf * kPN + c0 + j0), r);
-                            tc::tmem_ld_wait();
+                            float r[16];
+                            load(x, c0 + j0, r);
 #pragma unroll
-                            for (int j = 0; j < 16; ++j) sum[c][j0 + j] = seg == 0 ? __uint_as_float(r[j]) : sum[c][j0 + j] + __uint_as_float(r[j]);
+                            for (int j = 0; j < 16; ++j) sum[c][j0 + j] = seg == 0 ? r[j] : sum[c][j0 + j] + r[j];
                         }
                     }
                     release();
