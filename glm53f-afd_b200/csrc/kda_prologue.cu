@@ -13,7 +13,8 @@
 // sinks): one warp per (request, head, row).  The work is bound by instruction issue (about 850 instructions per row and lane,
 // most of them IEEE divisions and exponentials), so a warp takes ONE row and reads its three predecessors again (the four warps of a block take four
 // consecutive rows; the predecessors come from L1/L2): every load of a warp is in flight at once and 79 registers
-// allow 24 resident warps per SM (72 and 28 in the exact sink: 701 rows 400.8 -> 397.3 us; the verify sink gains nothing by it).  (A warp that walks 16 rows with the three earlier rows sliding in registers needs
+// allow 24 resident warps per SM (72 and 28 in the exact sink: 701 rows 400.8 -> 397.3 us; the verify sink gains nothing by it).  (The convolution two channels at a time
+// and the two norms from one sum, its root and its division: chunked layer verify of 6 slots x 4 to 8 rows 738 -> 724 us, 9 x 3 to 6 975 -> 953, 12 slots 1,218 and 1,223; 701 rows exact 398 -> 395.)  (A warp that walks 16 rows with the three earlier rows sliding in registers needs
 // 143 registers and was half as fast.)
 //
 // Three sinks:
@@ -77,16 +78,7 @@ __device__ __forceinline__ float silu_(float x) {
     if constexpr (FAST) return __fdividef(x, 1.0f + __expf(-x));
     else return x / (1.0f + expf(-x));
 }
-template <bool FAST>
-__device__ __forceinline__ float inv_norm_(float ss) {
-    if constexpr (FAST) return rsqrtf(ss + 1e-6f);
-    else return 1.0f / sqrtf(ss + 1e-6f);
-}
-__device__ __forceinline__ float butterfly(float x) {
-#pragma unroll
-    for (int o = 16; o; o >>= 1) x = x + __shfl_xor_sync(FULL, x, o);
-    return x;
-}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) { return fma2(a, {1.0f, 1.0f}, b); }
 __device__ __forceinline__ void unpack4(uint2 w, float (&x)[4]) {
     x[0] = __uint_as_float(w.x << 16);
     x[1] = __uint_as_float(w.x & 0xffff0000u);
@@ -160,14 +152,17 @@ __global__ void __launch_bounds__(128, SINK == kExact ? 7 : 6) layer_prologue_ke
         for (int d = 0; d < TAPS; ++d) unpack4(x[d][part], xv[d]);
         const uint32_t ww[8] = {wq[part][0].x, wq[part][0].y, wq[part][0].z, wq[part][0].w, wq[part][1].x, wq[part][1].y, wq[part][1].z, wq[part][1].w};
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            float acc = 0.0f;
-            acc = acc + __uint_as_float(ww[2 * c] << 16) * xv[0][c];
-            acc = acc + __uint_as_float(ww[2 * c] & 0xffff0000u) * xv[1][c];
-            acc = acc + __uint_as_float(ww[2 * c + 1] << 16) * xv[2][c];
-            acc = acc + __uint_as_float(ww[2 * c + 1] & 0xffff0000u) * xv[3][c];
+        for (int c = 0; c < 4; c += 2) {  // two channels at a time, every product and sum rounded by itself
+            float2 acc = {0.0f, 0.0f};
+#pragma unroll
+            for (int d = 0; d < TAPS; ++d) {
+                const uint32_t w0 = ww[2 * c + d / 2], w1 = ww[2 * c + 2 + d / 2];
+                acc = add2(acc, mul2(d & 1 ? float2{__uint_as_float(w0 & 0xffff0000u), __uint_as_float(w1 & 0xffff0000u)} : float2{__uint_as_float(w0 << 16), __uint_as_float(w1 << 16)},
+                                     {xv[d][c], xv[d][c + 1]}));
+            }
             // q reaches only the outputs, which carry bf16-operand rounding in both chunked forms: the fast form there
-            act[part][c] = bf16_round(part == 0 ? silu_<!EXACT>(acc) : silu_<false>(acc));
+            act[part][c] = bf16_round(part == 0 ? silu_<!EXACT>(acc.x) : silu_<false>(acc.x));
+            act[part][c + 1] = bf16_round(part == 0 ? silu_<!EXACT>(acc.y) : silu_<false>(acc.y));
         }
     }
     // L2 norms of q and k (eps 1e-6 inside the root), q also times 128^-0.5.
@@ -179,9 +174,12 @@ __global__ void __launch_bounds__(128, SINK == kExact ? 7 : 6) layer_prologue_ke
             sq = sq + act[0][c] * act[0][c];
             sk = sk + act[1][c] * act[1][c];
         }
-        sq = butterfly(sq);
-        sk = butterfly(sk);
-        const float iq = inv_norm_<!EXACT>(sq), ik = inv_norm_<false>(sk);
+        // Half of the lanes go on with q's sum, half with k's, and so does all that follows from it; the butterfly's pairs.
+        const bool up = lane >= 16;
+        float ss = (up ? sk : sq) + __shfl_xor_sync(FULL, up ? sq : sk, 16);
+#pragma unroll
+        for (int o = 8; o; o >>= 1) ss = ss + __shfl_xor_sync(FULL, ss, o);
+        const float inv = 1.0f / sqrtf(ss + 1e-6f), iq = __shfl_sync(FULL, inv, 0), ik = __shfl_sync(FULL, inv, 16);
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
             qn[c] = (act[0][c] * iq) * (1.0f / sqrtf((float)DK));
@@ -221,7 +219,6 @@ __global__ void __launch_bounds__(128, SINK == kExact ? 7 : 6) layer_prologue_ke
 // to 1,000; the parts' rows fetched one part ahead instead of all at once, 899.)
 constexpr int kRowsPer = 4;
 __device__ __forceinline__ float2 lo_hi(uint32_t w) { return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)); }
-__device__ __forceinline__ float2 add2(float2 a, float2 b) { return fma2(a, {1.0f, 1.0f}, b); }
 // 1 / (1 + e^-x)
 __device__ __forceinline__ float2 sigmoid2(float2 x) {
     const float2 t = mul2(x, {-kLog2e, -kLog2e}), d = add2({ex2_ftz(t.x), ex2_ftz(t.y)}, {1.0f, 1.0f});
