@@ -128,6 +128,10 @@ __device__ __forceinline__ unsigned char* slot_of(unsigned char* ws, int seg_chu
     return ws + ((size_t)chain * seg_chunks + jj) * kSlotBytes;
 }
 
+// Chain number n of a fused launch, in the order in which items and walks are handed out.  The layer form's goes backwards through the batch: its prologue has
+// written the last requests' rows last, and those are still in L2.
+__device__ __forceinline__ int chain_at(const SpParams& p, int n) { return p.v == nullptr ? p.batch * p.H - 1 - n : n; }
+
 struct Item {
     int chain, jj, group;
 };
@@ -137,7 +141,7 @@ __device__ __forceinline__ Item item_of(const SpParams& p, int item) {
     const int chains = p.batch * p.H;
     if (!FUSED) return {item % chains, item / chains, 0};
     const int per = p.group * p.seg_chunks, g = item / per, rem = item - g * per, n = min(p.group, chains - g * p.group);
-    return {g * p.group + rem % n, rem / n, g};
+    return {chain_at(p, g * p.group + rem % n), rem / n, g};
 }
 
 // The state role's barriers sit behind every tile (set up once at kernel entry, never repurposed).  The intra role's
@@ -1030,7 +1034,8 @@ __device__ void state_role(const SpParams& p, unsigned char* smem, const uint32_
                     publish(seq, Chain{-1, 0, 0, 0, 0, 0});
                     break;
                 }
-                const Chain at = chain_of(p, wk, ch);
+                const int real = MANY ? chain_at(p, ch) : ch;
+                const Chain at = chain_of(p, wk, real);
                 if constexpr (MANY) {
                     if (nothing_to_do(p, at)) {
                         next = take();
@@ -1056,7 +1061,7 @@ __device__ void state_role(const SpParams& p, unsigned char* smem, const uint32_
                 const int j0 = (wk.ja - p.state_chunk0);
                 bool ok = true;
                 for (int c = 0; ok && c < at.count; ++c, ++C) {
-                    const unsigned char* slot = slot_of(p.ws_state, p.seg_chunks, ch, j0 + c);
+                    const unsigned char* slot = slot_of(p.ws_state, p.seg_chunks, real, j0 + c);
                     const int x = C & 1;
                     if (!(ok = wait(bEmptyQW + x, (C >> 1) ^ 1))) break;  // an empty barrier starts released
                     mbar_arrive_expect_tx(&bars[bFullQW + x], kQW + 512);
