@@ -827,7 +827,7 @@ def run_prefill(torch, dist, pkg, core, rank, world, tokens, passes, ws_chunks, 
                                 "flop_per_token": PREFILL_FLOP_PER_TOKEN},
                      "algorithmic_bytes_per_token": PREFILL_BYTES_PER_TOKEN,
                      "traffic_bytes_per_token": NCU_PREFILL_DRAM_BYTES_PER_TOKEN if ws_chunks > 0 else None,
-                     "kernel": "prefill_sp_kernel (state role + intra role)" if ws_chunks > 0 else "prefill_tc_kernel",
+                     "kernel": "prefill_sp_kernel (state role + intra role)" if ws_chunks > 0 else "prefill_one_kernel",
                      "workspace_bytes": 0 if ws is None else ws.numel()},
         "gpu_launches": passes * kernels_per_pass,
         "collective": None if world == 1 else {

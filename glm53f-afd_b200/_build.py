@@ -20,7 +20,6 @@ SOURCES = {
     "kda_prefill.cu": IEEE,
     "kda_verify_tc.cu": IEEE,  # the chunked verify: its replay saves must carry the exact path's bits (the same expf)
     "kda_prologue.cu": IEEE,  # the layer prologue in front of the chunked prefill: the chain's prologue arithmetic
-    "kda_prefill_tc.cu": [],
     "kda_prefill_sp.cu": [],  # tensor-core prefill: agrees with the chain to rounding, so default FP flags
     "proj_gemm.cu": [],      # the projections: tcgen05 GEMM
     "proj_gemm_pair.cu": [], # the same on SM pairs (cta_group::2) for many rows

@@ -68,8 +68,8 @@ static_assert(kPrefillTailBytes == 4 * 64 && kTailSets + 2 * kTailSet == 64, "th
 constexpr int kSlotInK = 0, kSlotInV = 16384, kSlotInQ = 32768, kSlotInG = 49152, kSlotInBeta = 81920;
 __host__ __device__ inline int prefill_box_piece(int r, int piece) { return (piece >> 3) * 8192 + r * 128 + (((piece & 7) ^ (r & 7)) << 4); }
 
-// The chunk-64 tensor-core prefill (kda_prefill_tc.cu).  q, k, v, g, out (and norm_w) must be 16-byte aligned.
-int core_prefill_tc_launch(int32_t heads, int32_t batch, const int32_t* cu_seqlens, const glm53f_bf16* q, const glm53f_bf16* k,
+// The chunk-64 tensor-core prefill without a workspace (kda_prefill_sp.cu).  q, k, v, g, out, gate and norm_w must be 16-byte aligned, heads * batch below 2^31.
+int core_prefill_one_launch(int32_t heads, int32_t batch, const int32_t* cu_seqlens, const glm53f_bf16* q, const glm53f_bf16* k,
                            const glm53f_bf16* v, const float* g, const float* beta, const void* state_in, void* state_out,
                            const int64_t* state_off, bool bf16_state, const glm53f_bf16* gate, const glm53f_bf16* norm_w,
                            float eps, glm53f_bf16* out, cudaStream_t stream);

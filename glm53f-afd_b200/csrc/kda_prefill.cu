@@ -46,7 +46,7 @@ __global__ void single_request_meta(unsigned int* meta, int32_t rows) { meta[thr
 // kNotEligible when the call does not meet the kernels' layout requirements (dense output rows, aligned rows, room for
 // one chunk a pass); the caller then runs the exact form.
 // 4 requests x 2,048 rows x 64 heads with 256-row workspaces: 1,800 us with one block doing all of a chain
-// (kda_prefill_tc.cu, passes of six chunks), 921 to 947 so.
+// (in passes of six chunks), 921 to 947 so.
 int chunked_layer_prefill(int32_t heads, int32_t batch, const int32_t* cu_rows, int32_t max_rows, const glm53f_bf16* p,
                           int64_t p_stride, int64_t b_off, const glm53f_bf16* a, int64_t a_stride, const glm53f_bf16* g,
                           int64_t g_stride, const glm53f_bf16* conv, const int64_t* conv_off, const glm53f_bf16* conv_w,
@@ -255,9 +255,9 @@ extern "C" int glm53f_kda_core_prefill_varlen(int32_t heads, int32_t batch, cons
         const char* e = getenv("GLM53F_KDA_PREFILL");
         return e != nullptr && strcmp(e, "chain") == 0;
     }();
-    if (!force_chain && flags == 0 && aligned(q) && aligned(k) && aligned(v) && aligned(g) && aligned(out) &&
+    if (!force_chain && flags == 0 && (int64_t)heads * batch <= INT32_MAX && aligned(q) && aligned(k) && aligned(v) && aligned(g) && aligned(out) &&
         (!gate || (aligned(gate) && aligned(norm_w))))
-        return core_prefill_tc_launch(heads, batch, cu_seqlens, q, k, v, g, beta, state_in, state_out, state_off, state_bf16 != 0,
+        return core_prefill_one_launch(heads, batch, cu_seqlens, q, k, v, g, beta, state_in, state_out, state_off, state_bf16 != 0,
                                       gate, norm_w, eps, out, (cudaStream_t)stream);
     return core_chain_launch(heads, batch, cu_seqlens, q, k, v, g, beta, state_in, state_out, state_off, state_bf16 != 0, flags,
                              gate, norm_w, eps, out, (cudaStream_t)stream);

@@ -1,8 +1,26 @@
-// Chunk-64 tensor-core prefill in two passes over a caller-provided workspace: the core entry points that take one, and the
-// chunked form of the layer prefill.
+// Chunk-64 KDA prefill on the 5th-generation tensor cores (tcgen05 + TMEM): in two roles over a caller-provided workspace (the core entry points
+// that take one, and the chunked form of the layer prefill), or one block a chain without one (prefill_one_kernel).
 //
-// The arithmetic is that of kda_prefill_tc.cu (same operand tiles, same products, same precision mix).  What
-// changes is where it runs.  Everything of a chunk that does not need the recurrent state -- the decay scan, the
+// The head's 128 x 128 state stays in tensor memory (FP32) from a walk's first chunk to its last.  Per chunk (the algebra of the reference's CPU
+// definition crates/glm53f-kda/src/chunked.rs:67-198, which itself restates chunk_kimi_delta_attention):
+//
+//   G_i   = g_0 + ... + g_i per key channel (FP32 scan), E = exp(G), E_last = exp(G_63)
+//   Kg = k*E, Qg = q*E, Kinv = k/E, Kdec = k * E_last/E                       (operand tiles, written by hand)
+//   L = Kg Kinv^T, M = Qg Kinv^T      64x64x128 MMAs; L strictly lower * beta_i, M lower incl. diagonal
+//   T  = (I + L)^-1                   16 x 16 diagonal blocks by substitution, then the lower-left block of every
+//                                     2sz x 2sz diagonal block is -T22 (L21 T11), sz = 16, 32;  T' = T diag(beta)
+//   W  = T' Kg,  U = T' V             T' as bf16 hi + lo for U
+//   D  = U - W S,  QS = Qg S          MMAs on a bf16 copy of S
+//   O  = QS + M D
+//   S <- E_last * S + Kdec^T D        Kdec and D as bf16 hi + lo (three products)
+//
+// Operand precision follows a CPU study of this exact scheme on the benchmark's input distribution: bf16
+// operands are enough for every product that only reaches the output (M, QS, M D) and for L, W and W S, but not
+// for U and Kdec^T D, which carry the state: those use two-term bf16 splits (16 mantissa bits).  With that mix
+// the final state is within 5e-4 rel-L2 of the FP32 recurrence (limit 1e-3) and the bf16 outputs within 4e-3
+// (limit 5e-3).
+//
+// Where it runs with a workspace.  Everything of a chunk that does not need the recurrent state -- the decay scan, the
 // operand tiles, L, M, the triangular inverse, W = T'Kg and U = T'V, about two thirds of a chunk's time -- is
 // independent from chunk to chunk, so the *intra role* spreads those (chain, chunk) items over every SM and leaves
 // per item, in the workspace, exactly what the state recurrence consumes: Qg, W, M, Kdec hi/lo (bf16 cell tiles),
@@ -147,7 +165,8 @@ __device__ __forceinline__ Item item_of(const SpParams& p, int item) {
 // The state role's barriers sit behind every tile (set up once at kernel entry, never repurposed).  The intra role's
 // live inside its two groups' areas, which the state role -- it runs first in a block -- uses as tile space, so they are
 // set up when the intra role starts.
-constexpr int oBarsState = kSmemTc, oChain = oBarsState + 240, kSmemSp = oChain + 64;
+constexpr int oCtl = 14 * kTile;  // the block's control words
+constexpr int oBarsState = oCtl + 32, oChain = oBarsState + 240, kSmemSp = oChain + 64;
 // 16 compute warps, the loader warp, and (state role only) a warp that moves finished output rows to global memory and one that
 // issues the tensor-core products.
 constexpr int kThreadsSp = kCompute + 96, kLoaderWarp = kCompute / 32, kOutWarp = kCompute / 32 + 1, kMmaWarp = kCompute / 32 + 2;
@@ -193,8 +212,14 @@ static_assert(gG + 4 * kBox <= gTab && gG % 1024 == 0 && 32 * PS * 4 <= kTabs * 
 static_assert(kGroups * kGroupBytes <= oCtl, "two groups must fit below the block's control words");
 constexpr uint32_t gcL = 0, gcM = 64, gcW = 0, gcU = 64, kGroupCols = 128;
 
+// prefill_one_kernel: one group's area, the slot (its U's place takes the outputs when U is consumed), sums of the norm, barriers.
+enum : int { o1Full = 0, o1Free, o1WS, o1S16, o1SDec, o1D, o1SNew, o1O, o1OFree, o1OutFull, o1OutEmpty, o1Gate, kOneBars };
+constexpr int oSlotOne = kGroupBytes, oRedOne = oSlotOne + kSlotBytes, oBarsOne = oRedOne + 4 * CH * 4, oCtlOne = oBarsOne + (kOneBars + 1) / 2 * 16, kSmemOne = oCtlOne + 16;
+static_assert(oSlotOne % 1024 == 0 && wU == 0 && kSmemOne <= 232448, "shared memory of the single-pass kernel");
+
 // LAYER: the items' inputs are in their slots (kda_internal.h), which the results then replace.  G = 0 or 1, a runtime value: both groups run the same instructions (one copy of this code in the instruction cache).
-template <bool LAYER, bool FUSED, bool WALK_U>
+// ONE: the items are the chunks of the block's own chain, one after another, and the "slot" lies in the block's shared memory (prefill_one_kernel).
+template <bool LAYER, bool FUSED, bool WALK_U, bool ONE = false>
 __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* smem, const uint32_t tm_block, const WaitCtx& ctx, const int G) {
     // The issue loops stay loops in the layer form's instance and are unrolled in the core form's, whichever branch an item takes: 4 x 2,048
     // rows of the layer form 972 -> 944 us as loops; the core form's 8,192 rows in 8 sequences 462 both ways with mild gates, 548 and 555 with
@@ -249,8 +274,9 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
         if (!mbar_wait(bar_g, raw_phase, ctx, kStatusWaitPrefill)) break;
         const int item = item_slot[0], live = item_slot[1];  // (the next item's from when L and M are formed)
         if (item < 0) break;
-        const Item at_item = item_of<FUSED>(p, item);
-        unsigned char* slot = slot_of(p.ws_intra, p.seg_chunks, at_item.chain, at_item.jj);
+        const Item at_item = ONE ? Item{(int)blockIdx.x, item, 0} : item_of<FUSED>(p, item);
+        unsigned char* slot = ONE ? smem + oSlotOne : slot_of(p.ws_intra, p.seg_chunks, at_item.chain, at_item.jj);
+        uint64_t* one = reinterpret_cast<uint64_t*>(smem + oBarsOne);
 
         bool mild;
         // ---- 1. per key channel: the cumulative log decay; a = exp(G - Gm), every row relative to the middle row of its block of
@@ -296,7 +322,7 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
                 tab[(tF + 1) * 128] = ex2_approx(gm2 - gm0); tab[(tF + 2) * 128] = ex2_approx(gm2 - gm1);
                 tab[(tF + 3) * 128] = ex2_approx(gm3 - gm0); tab[(tF + 4) * 128] = ex2_approx(gm3 - gm1); tab[(tF + 5) * 128] = ex2_approx(gm3 - gm2);
                 const float egl = ex2_approx(gl);
-                reinterpret_cast<float*>(slot + wEgl)[d] = egl;
+                if (!ONE) reinterpret_cast<float*>(slot + wEgl)[d] = egl;
                 reinterpret_cast<float*>(gs + gGl)[d] = egl;
             }
             mild = gl > -60.0f * kLog2e;
@@ -308,6 +334,7 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
         const bool narrow = named_bar_all(BAR, kGroupThreads, mild);
 
         // ---- 2., 3. operand tiles -------------------------------------------------------------------------------------------------
+        if (ONE && !mbar_wait(one + o1Free, (uint32_t)(item + 1) & 1u, ctx, kStatusWaitPrefill)) break;  // the walk is through with the chunk before
         const float* tabs = reinterpret_cast<const float*>(gs + gTab);
         float a[32];
         // The block-wise form's share of a thread: a row of blocks J and 3 - J, sixteen channels each, so that every warp makes as many
@@ -575,6 +602,7 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
                 if (!LAYER || r >= live) *reinterpret_cast<uint4*>(slot + wV + box_piece(r, gt & 15)) = v8[t];
             }
         }
+        const float egl_here = ONE && gt < DK ? reinterpret_cast<const float*>(gs + gGl)[gt] : 0.0f;
         if (!mma_wait(bar_mma, mma_phase)) break;
         // Nothing of this item is left in the group's shared memory: the loader may bring the next item in.
         if (gt == 0) mbar_arrive(bar_free);
@@ -590,15 +618,21 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
             if constexpr (!WALK_U) {
                 tc::tmem_ld32(tc::tmem_addr(tm, quad, gcU + cg * 32), r);
                 tc::tmem_ld_wait();
+                if (ONE && !mbar_wait(one + o1OutEmpty, (uint32_t)(item + 1) & 1u, ctx, kStatusWaitPrefill)) break;  // its outputs have left U's place
 #pragma unroll
                 for (int j2 = 0; j2 < 8; ++j2)
                     *reinterpret_cast<uint4*>(slot + wU + u_cell(cg * 8 + j2, ch)) = make_uint4(r[j2 * 4], r[j2 * 4 + 1], r[j2 * 4 + 2], r[j2 * 4 + 3]);
             }
         }
+        if (ONE) {
+            if (gt < DK) reinterpret_cast<float*>(slot + wEgl)[gt] = egl_here;
+            fence_proxy_async_smem();
+        }
         if (FUSED) fence_proxy_async_global();  // another block's bulk copies read the slot
         tc::fence_before_sync();
         group_sync();
         tc::fence_after_sync();
+        if (ONE && gt == 0) mbar_arrive(one + o1Full);
         unreported = at_item.group;
     }
     report();
@@ -615,7 +649,7 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // 16-byte copies (rows past the sequence's end are not read, they become zero), so no copy ever reaches
 // past the rows the caller's metadata names.    They are asynchronous, all in flight at once: as loads and stores, a row's after
 // the other's, they were 8 to 12 us of a launch (33 rows x 64 heads by the chunked layer prefill: 59 us, 64 rows 52).
-template <bool LAYER, bool FUSED, bool WALK_U>
+template <bool LAYER, bool FUSED, bool WALK_U, bool ONE = false>
 __device__ __forceinline__ void intra_loader(const SpParams& p, unsigned char* smem, const WaitCtx& ctx, const int G) {
     unsigned char* gs = smem + G * kGroupBytes;
     uint64_t* bar_raw = reinterpret_cast<uint64_t*>(gs + gBars);
@@ -627,8 +661,8 @@ __device__ __forceinline__ void intra_loader(const SpParams& p, unsigned char* s
     const long long items = (long long)chains * p.seg_chunks;  // item = jj * chains + chain: chunk-major
     uint32_t free_phase = 0;
     for (int it = 0;;) {
-        long long item = 0;
-        if (lane == 0) {
+        long long item = ONE ? it : 0;
+        if (!ONE && lane == 0) {
             unsigned int* taken = FUSED ? p.sets + p.ctr * kTailSet : p.counters + p.ctr;
             // (Only when every block has begun: those that stay run then, and a chain whose items they have may be waited for.)
             if (FUSED && (int)blockIdx.x < p.early_blocks && *reinterpret_cast<volatile unsigned int*>(taken) >= p.early_from &&
@@ -638,16 +672,18 @@ __device__ __forceinline__ void intra_loader(const SpParams& p, unsigned char* s
                 item = atomicAdd(taken, 1u);
         }
         item = __shfl_sync(0xffffffffu, item, 0);
-        const bool last = item >= items;
+        bool last = !ONE && item >= items;
         int h = 0, n = 0;
         long long gr0 = 0;
         const unsigned char* in = nullptr;
         if (!last) {
-            const Item at = item_of<FUSED>(p, (int)item);
+            const Item at = ONE ? Item{(int)blockIdx.x, (int)item, 0} : item_of<FUSED>(p, (int)item);
             const int j = p.intra_chunk0 + at.jj, b = at.chain / H;
             h = at.chain % H;
             const int r0 = p.cu[b], T = p.cu[b + 1] - r0;
-            if ((long long)j * CH >= T) {  // the sequence has no such chunk
+            if (ONE && (long long)j * CH >= T) {
+                last = true;
+            } else if ((long long)j * CH >= T) {  // the sequence has no such chunk
                 if (FUSED && lane == 0) atomicAdd(p.sets + p.ctr * kTailSet + kTailDone + at.group, 1u);
                 continue;
             }
@@ -658,7 +694,7 @@ __device__ __forceinline__ void intra_loader(const SpParams& p, unsigned char* s
         float b0 = 0.0f, b1 = 0.0f;
         if (lane < n) b0 = LAYER ? reinterpret_cast<const float*>(in + kSlotInBeta)[lane] : p.beta[(gr0 + lane) * H + h];
         if (lane + 32 < n) b1 = LAYER ? reinterpret_cast<const float*>(in + kSlotInBeta)[lane + 32] : p.beta[(gr0 + lane + 32) * H + h];
-        if (!LAYER && !last && n == CH && lane == 0) {  // on their way into L2 while the group is still busy with the item before
+        if (!LAYER && !last && n == CH && lane == 0 && !(ONE && it == 0)) {  // on their way into L2 while the group is still busy with the item before
             const int row = (int)gr0;
             for (int x = 0; x < 4; ++x) tensor_prefetch_3d(&p.tm_g, x * 32, h, row);
             for (int x = 0; x < 2; ++x) tensor_prefetch_3d(&p.tm_k, x * 64, h, row);
@@ -772,7 +808,7 @@ __device__ void intra_role(const SpParams& p, unsigned char* smem, const uint32_
 // channels 0-63, 64-127) in the 128-byte swizzle of box_piece(), which is what the tiled tensor stores read.
 constexpr int kQW = 2 * kTile, kMKd = kTile / 2 + 2 * kTile, kOutTile = 2 * kBox;
 constexpr int sQW = 0, sMKd = sQW + 2 * kQW, sU = sMKd + 2 * kMKd, sOut = sU + kUBytes, sRed = sOut + 2 * kOutTile, sE = sRed + 2 * 4 * CH * 4;
-static_assert(sOut % 1024 == 0 && (sU + kTile) % 1024 == 0 && sE + 2 * 512 <= oBars, "state role shared memory");
+static_assert(sOut % 1024 == 0 && (sU + kTile) % 1024 == 0 && sE + 2 * 512 <= oCtl, "state role shared memory");
 // Tensor memory columns: S^T; its bf16 pairs; (W S)^T; (Qg S)^T and O^T, two accumulators that alternate between chunks; D^T hi, lo; U^T.
 constexpr uint32_t tS = 0, tS16 = 128, tWS = 192, tO = 256, tDhi = 384, tDlo = 416, tU = 448;
 
@@ -928,6 +964,49 @@ __device__ __forceinline__ void state_to_tmem(uint32_t at, const uint16_t* from,
         tc::tmem_st_frag(at + ((uint32_t)x << 20), f[0]);
         tc::tmem_st_frag(at + ((uint32_t)x << 20) + 16, f[1]);
     }
+}
+
+// The gated RMSNorm of sixteen output rows from i0 on by four warps, which have 32 channels each and meet at barrier `bar`; red: their sums, [4][64].  y2[g][q]:
+// rows fi + 8 g and the next (fi = i0 + 2 (lane % 4)) of channel fv + 8 q as bf16, gt the gate's values alike, which `fetch` may bring behind the barrier.
+// False on all four when one of them comes without `ok`.  FULL: the sigmoid also where it is too faint for rcp_approx().
+template <bool FULL, typename Fetch>
+__device__ __forceinline__ bool gated_rows(float* red, float eps, int quad, int lane, int i0, const float (&nw)[4], uint32_t (&gt)[2][4], uint32_t (&y2)[2][4], int bar, bool ok, Fetch&& fetch) {
+    float sq[4];  // [2 g + e]
+#pragma unroll
+    for (int g = 0; g < 2; ++g) {
+        float2 s2 = {0.0f, 0.0f};
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const float2 y = {__uint_as_float(y2[g][q] << 16), __uint_as_float(y2[g][q] & 0xffff0000u)};
+            s2 = fma2(y, y, s2);
+        }
+        sq[2 * g] = s2.x;
+        sq[2 * g + 1] = s2.y;
+    }
+    // The sum over the eight lanes of a row; at the first two steps a lane gives away the rows that it does not go on with.
+    const bool up4 = lane & 4, up8 = lane & 8;
+    const float a0 = (up4 ? sq[2] : sq[0]) + __shfl_xor_sync(0xffffffffu, up4 ? sq[0] : sq[2], 4);
+    const float a1 = (up4 ? sq[3] : sq[1]) + __shfl_xor_sync(0xffffffffu, up4 ? sq[1] : sq[3], 4);
+    float a = (up8 ? a1 : a0) + __shfl_xor_sync(0xffffffffu, up8 ? a0 : a1, 8);
+    a += __shfl_xor_sync(0xffffffffu, a, 16);
+    if (lane < 16) red[quad * CH + i0 + 2 * (lane & 3) + 8 * (up4 ? 1 : 0) + (up8 ? 1 : 0)] = a;
+    ok = named_bar_all(bar, 128, ok);
+    if (ok) fetch();
+    // A row's factor is formed by one lane of each of the first two quarters (a square root and a division, both IEEE).
+    const float* at = red + i0 + (lane & 15);
+    const float rinv = 1.0f / sqrtf((((at[0] + at[CH]) + at[2 * CH]) + at[3 * CH]) / (float)DV + eps);
+    auto rcp = [](float x) { return FULL ? rcp_full(x) : rcp_approx(x); };
+#pragma unroll
+    for (int g = 0; g < 2; ++g) {
+        const float2 rv = {__shfl_sync(0xffffffffu, rinv, 2 * (lane & 3) + 8 * g), __shfl_sync(0xffffffffu, rinv, 2 * (lane & 3) + 8 * g + 1)};
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const float2 sig = {rcp(1.0f + ex2_ftz(-kLog2e * __uint_as_float(gt[g][q] << 16))), rcp(1.0f + ex2_ftz(-kLog2e * __uint_as_float(gt[g][q] & 0xffff0000u)))};
+            const float2 y = mul2(mul2({nw[q], nw[q]}, mul2({__uint_as_float(y2[g][q] << 16), __uint_as_float(y2[g][q] & 0xffff0000u)}, rv)), sig);
+            y2[g][q] = tc::bf16x2(y.x, y.y);
+        }
+    }
+    return ok;
 }
 
 // Walks `chain`, or (MANY) the chains of a fused launch that this block's loader warp takes off the counter, until there are none.
@@ -1310,47 +1389,13 @@ __device__ void state_role(const SpParams& p, unsigned char* smem, const uint32_
         }
         unsigned char* dst = smem + sOut + (c & 1) * kOutTile;
         if (votes) {
-            float sq[4];  // [2 g + e]
-#pragma unroll
-            for (int g = 0; g < 2; ++g) {
-                float2 s2 = {0.0f, 0.0f};
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const float2 y = {__uint_as_float(y2[g][q] << 16), __uint_as_float(y2[g][q] & 0xffff0000u)};
-                    s2 = fma2(y, y, s2);
-                }
-                sq[2 * g] = s2.x;
-                sq[2 * g + 1] = s2.y;
-            }
-            // The sum over the eight lanes of a row; at the first two steps a lane gives away the rows that it does not go on with.
-            const bool up4 = lane & 4, up8 = lane & 8;
-            const float a0 = (up4 ? sq[2] : sq[0]) + __shfl_xor_sync(0xffffffffu, up4 ? sq[0] : sq[2], 4);
-            const float a1 = (up4 ? sq[3] : sq[1]) + __shfl_xor_sync(0xffffffffu, up4 ? sq[1] : sq[3], 4);
-            float a = (up8 ? a1 : a0) + __shfl_xor_sync(0xffffffffu, up8 ? a0 : a1, 8);
-            a += __shfl_xor_sync(0xffffffffu, a, 16);
-            if (lane < 16) reinterpret_cast<float*>(smem + sRed)[((c & 1) * 4 + quad) * CH + fi + 8 * (up4 ? 1 : 0) + (up8 ? 1 : 0)] = a;
             if (boxes) ok = ok && wait(bGate + (c & 1), c >> 1);
-            ok = named_bar_all(4 + cg, 128, ok);
-            if (boxes && ok) {
-                tc::ldmatrix_t4(dst + box_piece(tile_row, tile_piece), gt[0][0], gt[0][1], gt[1][0], gt[1][1]);
-                tc::ldmatrix_t4(dst + box_piece(tile_row, tile_piece + 2), gt[0][2], gt[0][3], gt[1][2], gt[1][3]);
-            }
-            // A row's factor is formed by one lane of each of the first two quarters (a square root and a division, both IEEE).
-            float rinv;
-            {
-                const float* at = reinterpret_cast<const float*>(smem + sRed) + (c & 1) * 4 * CH + i0 + (lane & 15);
-                rinv = 1.0f / sqrtf((((at[0] + at[CH]) + at[2 * CH]) + at[3 * CH]) / (float)DV + p.eps);
-            }
-#pragma unroll
-            for (int g = 0; g < 2; ++g) {
-                const float2 rv = {__shfl_sync(0xffffffffu, rinv, 2 * (lane & 3) + 8 * g), __shfl_sync(0xffffffffu, rinv, 2 * (lane & 3) + 8 * g + 1)};
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const float2 sig = {rcp_approx(1.0f + ex2_ftz(-kLog2e * __uint_as_float(gt[g][q] << 16))), rcp_approx(1.0f + ex2_ftz(-kLog2e * __uint_as_float(gt[g][q] & 0xffff0000u)))};
-                    const float2 y = mul2(mul2({nw[q], nw[q]}, mul2({__uint_as_float(y2[g][q] << 16), __uint_as_float(y2[g][q] & 0xffff0000u)}, rv)), sig);
-                    y2[g][q] = tc::bf16x2(y.x, y.y);
+            ok = gated_rows<false>(reinterpret_cast<float*>(smem + sRed) + (c & 1) * 4 * CH, p.eps, quad, lane, i0, nw, gt, y2, 4 + cg, ok, [&] {
+                if (boxes) {
+                    tc::ldmatrix_t4(dst + box_piece(tile_row, tile_piece), gt[0][0], gt[0][1], gt[1][0], gt[1][1]);
+                    tc::ldmatrix_t4(dst + box_piece(tile_row, tile_piece + 2), gt[0][2], gt[0][3], gt[1][2], gt[1][3]);
                 }
-            }
+            });
         }
         if (!ok) return false;  // else the output warp takes it from there
         tc::stmatrix_t4(dst + box_piece(tile_row, tile_piece), y2[0][0], y2[0][1], y2[1][0], y2[1][1]);
@@ -1560,6 +1605,314 @@ __global__ void __launch_bounds__(kThreadsSp, 1) prefill_sp_kernel(const __grid_
     if (warp == 0) tc::tmem_dealloc(tm, kTmemCols);
 }
 
+// =====================================================================================================================
+// The prefill without a workspace: a block has a chain, one group of eight warps forms its chunks' items (intra_group) and eight warps walk them, the
+// slot between them in shared memory.  The walk of a chunk runs beside the next one's item; the slot is one, and is free when the walk's last product of
+// the chunk has read it, by which time the group has come to its operand tiles.  HBM sees the algorithm's bytes.
+// Bound by a chunk's item, a chain of group-wide steps (scan 2,000 cycles, tiles 2,700, L and M 1,200, inverse 4,000, T' 800, products 1,000, results 1,200):
+// 12,800 cycles a chunk.  One kernel of sixteen warps that did all of a chunk's steps one after the other took 22,900.  us, that / this: 64 rows x 64 heads
+// 21.6 / 14.7, 1,000 rows 199 / 116, 8,192 rows in one sequence 1,558 / 861, in eight 774 / 444 (with the norm 788 / 517); 16,384 rows x 8 heads 3,052 / 1,682.
+// =====================================================================================================================
+constexpr int kOneThreads = 2 * kGroupThreads + 96, kOneLoader = 16, kOneOut = 17, kOneMma = 18;
+constexpr uint32_t t1S = 128, t1S16 = 256, t1WS = 320, t1O = 384, t1Dhi = 448, t1Dlo = 480;  // behind the group's columns
+
+template <bool GATED>
+__device__ __forceinline__ void walk_one(const SpParams& p, unsigned char* smem, const uint32_t tm, const WaitCtx& ctx, const Chain& at) {
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + oBarsOne);
+    const unsigned char* slot = smem + oSlotOne;
+    unsigned char* tile = smem + oSlotOne + wU;  // the outputs of a chunk, boxes of 64 rows x 128 bytes
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, quad = warp & 3, half = (warp >> 2) & 1;
+    auto wait = [&](int i, int phase) { return mbar_wait(&bars[i], (uint32_t)(phase & 1), ctx, kStatusWaitPrefill); };
+    const int count = at.count;
+    if (warp == kOneOut) {
+        for (int c = 0; c < count; ++c) {
+            const int n = min(CH, at.rows - c * CH);
+            const long long gr0 = at.row + (long long)c * CH;
+            if (GATED && n == CH) {  // the gate's values into the tile that the outputs will take, as soon as U has left it
+                if (lane == 0)
+                    for (int x = 0; x < 2; ++x) tensor_prefetch_3d(&p.tm_gate, x * 64, at.h, (int)gr0);
+                if (!wait(o1D, c)) break;
+                if (lane == 0) {
+                    mbar_arrive_expect_tx(&bars[o1Gate], kTile);
+                    for (int x = 0; x < 2; ++x) tensor_load_3d(tile + x * kBox, &p.tm_gate, x * 64, at.h, (int)gr0, &bars[o1Gate]);
+                }
+            }
+            if (!wait(o1OutFull, c)) break;
+            if (n == CH) {
+                if (lane == 0) {
+                    for (int x = 0; x < 2; ++x) tensor_store_3d(&p.tm_out, x * 64, at.h, (int)gr0, tile + x * kBox);
+                    bulk_commit();
+                    bulk_wait_read<0>();
+                }
+            } else {
+                for (int e = lane; e < n * 16; e += 32)
+                    *reinterpret_cast<uint4*>(p.out + ((gr0 + (e >> 4)) * p.H + at.h) * DV + (e & 15) * 8) = *reinterpret_cast<const uint4*>(tile + box_piece(e >> 4, e & 15));
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bars[o1OutEmpty]);
+        }
+        if (lane == 0) bulk_wait_all<0>();
+        return;
+    }
+    if (warp == kOneMma) {
+        const uint32_t leader = tc::elect_one();
+        auto ready = [&](int i, int phase) { return tc::warp_all(wait(i, phase)); };
+        constexpr uint32_t idw = tc::idesc_bf16(DV, CH, 0, 1, 0), idq = tc::idesc_bf16(DV, CH, 0, 0, 0), ids = tc::idesc_bf16(DV, DK, 0, 1, 0);
+        const unsigned char *mm = slot + wMm, *kdhi = slot + wKdHi, *kdlo = slot + wKdLo;
+        for (int c = 0; tc::warp_all(c < count); ++c) {
+            if (!ready(o1Full, c) || !ready(o1S16, c)) break;
+            tc::fence_after_sync();
+#pragma unroll
+            for (int k0 = 0; k0 < DK; k0 += 16)
+                tc::mma_bf16_ts_if(leader, tm + t1WS, tm + t1S16 + k0 / 2, tc::desc_mnmajor_bf16(slot + wW, DK, 0, k0), idw, k0 > 0);
+            tc::mma_commit_if(leader, &bars[o1WS]);
+            if (c > 0 && !ready(o1OFree, c - 1)) break;
+            tc::fence_after_sync();
+#pragma unroll
+            for (int k0 = 0; k0 < DK; k0 += 16)
+                tc::mma_bf16_ts_if(leader, tm + t1O, tm + t1S16 + k0 / 2, tc::desc_kmajor_bf16(slot + wQg, CH, 0, k0), idq, k0 > 0);
+            if (!ready(o1SDec, c) || !ready(o1D, c)) break;
+            tc::fence_after_sync();
+#pragma unroll
+            for (int k0 = 0; k0 < CH; k0 += 16) tc::mma_bf16_ts_if(leader, tm + t1S, tm + t1Dhi + k0 / 2, tc::desc_mnmajor_bf16(kdhi, CH, 0, k0), ids, true);
+#pragma unroll
+            for (int k0 = 0; k0 < CH; k0 += 16) tc::mma_bf16_ts_if(leader, tm + t1S, tm + t1Dlo + k0 / 2, tc::desc_mnmajor_bf16(kdhi, CH, 0, k0), ids, true);
+#pragma unroll
+            for (int k0 = 0; k0 < CH; k0 += 16) tc::mma_bf16_ts_if(leader, tm + t1S, tm + t1Dhi + k0 / 2, tc::desc_mnmajor_bf16(kdlo, CH, 0, k0), ids, true);
+            tc::mma_commit_if(leader, &bars[o1SNew]);
+#pragma unroll
+            for (int k0 = 0; k0 < CH; k0 += 16) tc::mma_bf16_ts_if(leader, tm + t1O, tm + t1Dhi + k0 / 2, tc::desc_mnmajor_bf16(mm, CH, 0, k0), idw, true);
+            tc::mma_commit_if(leader, &bars[o1O]);
+            tc::mma_commit_if(leader, &bars[o1Free]);
+            if (leader) atomicAdd(const_cast<uint32_t*>(ctx.progress), 1u);
+            __syncwarp();
+        }
+        return;
+    }
+    // Eight warps: a thread has a value channel (tensor-memory lane) and two pieces of 32 key channels or 16 rows.
+    auto arrive = [&](int i) {
+        tc::fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars[i]);
+    };
+    const int v = quad * 32 + lane, piece0 = half * 2;
+    const bool same = p.state_in == p.state_out;
+    auto aligned = [](const void* a) { return (reinterpret_cast<uintptr_t>(a) & 15) == 0; };  // for all lanes or none
+    // S^T as bf16 pairs for chunk c's products.
+    auto operand = [&]() {
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+            uint32_t r[32], pr[16];
+            tc::tmem_ld32(tc::tmem_addr(tm, quad, t1S + (piece0 + s) * 32), r);
+            tc::tmem_ld_wait();
+#pragma unroll
+            for (int x = 0; x < 16; ++x) pr[x] = tc::bf16x2(__uint_as_float(r[2 * x]), __uint_as_float(r[2 * x + 1]));
+            tc::tmem_st16(tc::tmem_addr(tm, quad, t1S16 + (piece0 + s) * 16), pr);
+        }
+        tc::tmem_st_wait();
+        arrive(o1S16);
+    };
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {  // the incoming state
+        const int k_first = (piece0 + s) * 32;
+        const uint32_t to = tc::tmem_addr(tm, quad, t1S + k_first);
+        const long long from = at.s_elem + v * DK + k_first;
+        const uint16_t* a16 = reinterpret_cast<const uint16_t*>(p.state_in) + from;
+        const float* a32 = reinterpret_cast<const float*>(p.state_in) + from;
+        if (p.state_bf16 ? aligned(a16) : aligned(a32)) {
+            if (p.state_bf16) state_to_tmem(to, a16 - lane * DK, lane);
+            else state_to_tmem(to, a32 - lane * DK, lane);
+        } else {
+            uint32_t r[32];
+#pragma unroll
+            for (int x = 0; x < 32; ++x) r[x] = p.state_bf16 ? (uint32_t)a16[x] << 16 : __float_as_uint(a32[x]);
+            tc::tmem_st32(to, r);
+        }
+    }
+    tc::tmem_st_wait();
+    __syncwarp();
+    const int fv = quad * 32 + (lane >> 2), tile_piece = quad * 4 + ((lane >> 3) & 1);
+    float nw[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    if (GATED)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) nw[q] = bf16_bits_to_f32(p.norm_w[fv + 8 * q]);
+    bool alive = true;
+    auto leave = [&] {  // the four warps that share output rows vote at a barrier when the norm is fused
+        if (GATED) named_bar_all(4 + half, 128, false);
+        alive = false;
+    };
+    if (count > 0) operand();
+    for (int c = 0; c < count; ++c) {
+        if (!wait(o1Full, c)) { leave(); break; }
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {  // the decayed S^T
+            const int k_first = (piece0 + s) * 32;
+            uint32_t r[32];
+            tc::tmem_ld32(tc::tmem_addr(tm, quad, t1S + k_first), r);
+            tc::tmem_ld_wait();
+            const float4* el = reinterpret_cast<const float4*>(slot + wEgl + k_first * 4);
+#pragma unroll
+            for (int x = 0; x < 8; ++x) {
+                const float4 e = el[x];
+                const float ee[4] = {e.x, e.y, e.z, e.w};
+#pragma unroll
+                for (int y = 0; y < 4; y += 2) {
+                    float s0 = __uint_as_float(r[4 * x + y]), s1 = __uint_as_float(r[4 * x + y + 1]);
+                    if (p.state_bf16) {  // a bf16 state is rounded once per chunk
+                        const uint32_t two = tc::bf16x2(s0, s1);
+                        s0 = __uint_as_float(two << 16);
+                        s1 = __uint_as_float(two & 0xffff0000u);
+                    }
+                    r[4 * x + y] = __float_as_uint(s0 * ee[y]);
+                    r[4 * x + y + 1] = __float_as_uint(s1 * ee[y + 1]);
+                }
+            }
+            tc::tmem_st32(tc::tmem_addr(tm, quad, t1S + k_first), r);
+        }
+        tc::tmem_st_wait();
+        arrive(o1SDec);
+        uint32_t gt[2][2][4];
+        const int n = at.rows - c * CH;
+        const bool boxes = n >= CH;  // else the threads read the gate's values that they want
+        if (GATED && !boxes) {
+#pragma unroll
+            for (int s = 0; s < 2; ++s) {
+                const int fi = (piece0 + s) * 16 + 2 * (lane & 3);
+                const uint16_t* g = p.gate + (at.row + c * CH + fi) * p.gate_stride + at.h * DV + fv;
+#pragma unroll
+                for (int y = 0; y < 2; ++y)
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const uint32_t lo = fi + 8 * y < n ? g[8 * y * p.gate_stride + 8 * q] : 0u, hi = fi + 8 * y + 1 < n ? g[(8 * y + 1) * p.gate_stride + 8 * q] : 0u;
+                        gt[s][y][q] = lo | hi << 16;
+                    }
+            }
+        }
+        if (!wait(o1WS, c)) { leave(); break; }
+        tc::fence_after_sync();
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {  // D^T = U^T - (W S)^T as bf16 hi + lo pairs of rows
+            const int cg = piece0 + s;
+            uint32_t r[16], wh[8], wl[8];
+            tc::tmem_ld16(tc::tmem_addr(tm, quad, t1WS + cg * 16), r);
+            float uu[16];
+#pragma unroll
+            for (int x = 0; x < 4; ++x) {
+                const float4 u4 = *reinterpret_cast<const float4*>(slot + wU + u_cell(cg * 4 + x, v));
+                uu[4 * x] = u4.x; uu[4 * x + 1] = u4.y; uu[4 * x + 2] = u4.z; uu[4 * x + 3] = u4.w;
+            }
+            tc::tmem_ld_wait();
+#pragma unroll
+            for (int x = 0; x < 8; ++x) tc::split_bf16x2(uu[2 * x] - __uint_as_float(r[2 * x]), uu[2 * x + 1] - __uint_as_float(r[2 * x + 1]), wh[x], wl[x]);
+            tc::tmem_st8(tc::tmem_addr(tm, quad, t1Dhi + cg * 8), wh);
+            tc::tmem_st8(tc::tmem_addr(tm, quad, t1Dlo + cg * 8), wl);
+        }
+        tc::tmem_st_wait();
+        arrive(o1D);
+        if (!wait(o1SNew, c)) { leave(); break; }
+        tc::fence_after_sync();
+        if (c + 1 < count) operand();
+        // ---- the chunk's outputs: bf16(y), or the gated RMSNorm of bf16(y); U has been consumed by all --------------------------------
+        if (!wait(o1O, c)) { leave(); break; }
+        tc::fence_after_sync();
+        uint32_t y2[2][2][4];
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+            uint32_t ra[8], rb[8];
+            const uint32_t from = tc::tmem_addr(tm, quad, t1O + (piece0 + s) * 16);
+            tc::tmem_ld_frag(from, ra);
+            tc::tmem_ld_frag(from + (16u << 16), rb);
+            tc::tmem_ld_wait();
+#pragma unroll
+            for (int g = 0; g < 2; ++g) {
+                y2[s][g][0] = tc::bf16x2(__uint_as_float(ra[4 * g]), __uint_as_float(ra[4 * g + 1]));
+                y2[s][g][1] = tc::bf16x2(__uint_as_float(ra[4 * g + 2]), __uint_as_float(ra[4 * g + 3]));
+                y2[s][g][2] = tc::bf16x2(__uint_as_float(rb[4 * g]), __uint_as_float(rb[4 * g + 1]));
+                y2[s][g][3] = tc::bf16x2(__uint_as_float(rb[4 * g + 2]), __uint_as_float(rb[4 * g + 3]));
+            }
+        }
+        arrive(o1OFree);
+        const bool ok = !GATED || !boxes || wait(o1Gate, c);
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+            const int i0 = (piece0 + s) * 16, tile_row = i0 + (lane >> 4) * 8 + (lane & 7);
+            if (GATED && !gated_rows<true>(reinterpret_cast<float*>(smem + oRedOne), p.eps, quad, lane, i0, nw, gt[s], y2[s], 4 + half, ok, [&] {
+                    if (boxes) {
+                        tc::ldmatrix_t4(tile + box_piece(tile_row, tile_piece), gt[s][0][0], gt[s][0][1], gt[s][1][0], gt[s][1][1]);
+                        tc::ldmatrix_t4(tile + box_piece(tile_row, tile_piece + 2), gt[s][0][2], gt[s][0][3], gt[s][1][2], gt[s][1][3]);
+                    }
+                })) {
+                alive = false;
+                break;
+            }
+            tc::stmatrix_t4(tile + box_piece(tile_row, tile_piece), y2[s][0][0], y2[s][0][1], y2[s][1][0], y2[s][1][1]);
+            tc::stmatrix_t4(tile + box_piece(tile_row, tile_piece + 2), y2[s][0][2], y2[s][0][3], y2[s][1][2], y2[s][1][3]);
+        }
+        if (!alive) break;
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars[o1OutFull]);
+    }
+    if (!alive || (count == 0 && (same || !at.start))) return;
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {  // the outgoing state
+        const int k_first = (piece0 + s) * 32;
+        const uint32_t from = tc::tmem_addr(tm, quad, t1S + k_first);
+        const long long to = at.s_elem + v * DK + k_first;
+        uint16_t* to16 = reinterpret_cast<uint16_t*>(p.state_out) + to;
+        float* to32 = reinterpret_cast<float*>(p.state_out) + to;
+        if (p.state_bf16 ? aligned(to16) : aligned(to32)) {
+            if (p.state_bf16) state_from_tmem(from, to16 - lane * DK, lane);
+            else state_from_tmem(from, to32 - lane * DK, lane);
+        } else {
+            uint32_t r[32];
+            tc::tmem_ld32(from, r);
+            tc::tmem_ld_wait();
+#pragma unroll
+            for (int x = 0; x < 32; ++x) {
+                if (p.state_bf16) to16[x] = f32_to_bf16_bits(__uint_as_float(r[x]));
+                else to32[x] = __uint_as_float(r[x]);
+            }
+        }
+    }
+}
+
+template <bool GATED>
+__global__ void __launch_bounds__(kOneThreads, 1) prefill_one_kernel(const __grid_constant__ SpParams p) {
+    extern __shared__ __align__(1024) unsigned char smem[];
+    volatile uint32_t* ctl = reinterpret_cast<volatile uint32_t*>(smem + oCtlOne);
+    uint32_t* tmem_slot = const_cast<uint32_t*>(ctl) + 2;
+    const int tid = threadIdx.x, warp = tid >> 5;
+    if (tid == 0) {
+        uint64_t* b = reinterpret_cast<uint64_t*>(smem + gBars);
+        for (int i = 0; i < kGroupBars; ++i) mbar_init(b + i, i == 2 ? 8 : 1);  // as in intra_role()
+        uint64_t* one = reinterpret_cast<uint64_t*>(smem + oBarsOne);
+        for (int i = 0; i < kOneBars; ++i) mbar_init(one + i, i == o1S16 || i == o1SDec || i == o1D || i == o1OFree || i == o1OutFull ? 8 : 1);
+        ctl[0] = 0u;
+        ctl[1] = 0u;
+        mbar_init_fence();
+    }
+    if (warp == 0) tc::tmem_alloc(tmem_slot, kTmemCols);
+    tc::fence_before_sync();
+    __syncthreads();
+    tc::fence_after_sync();
+    const uint32_t tm = *tmem_slot;
+    grid_ready();
+    const WaitCtx ctx{ctl, ctl + 1, p.status};
+    const Chain at = chain_of(p, Walk{0, 0x7fffffff, 0, nullptr, 0, nullptr, true, true}, (int)blockIdx.x);
+    if (warp < kGroupThreads / 32) intra_group<false, false, false, true>(p, smem, tm, ctx, 0);
+    else if (warp == kOneLoader) intra_loader<false, false, false, true>(p, smem, ctx, 0);
+    else walk_one<GATED>(p, smem, tm, ctx, at);
+    if (ctl[1] != 0u) {  // after an abort copies into this block's shared memory may still be in flight: give them a bounded time
+        const uint64_t t0 = global_timer_ns();
+        while (global_timer_ns() - t0 < 2000000ull) {
+        }
+    }
+    tc::fence_before_sync();
+    __syncthreads();
+    if (warp == 0) tc::tmem_dealloc(tm, kTmemCols);
+}
+
 // Between the two scan passes: the state before every segment, S_start[s + 1] = A_s S_start[s] + B_s in FP32, from the
 // caller's state.  A state's value columns never mix, so a block owns two of them (held in shared memory across the
 // segments) and a thread one key channel: acc[v] += A_s[k][k'] S[k'][v] with A_s read along k (coalesced; A_s lies in
@@ -1715,6 +2068,12 @@ int core_prefill_sp_launch(int32_t heads, int32_t batch, const int32_t* cu_seqle
     long long seg = overlap ? whole / 2 : whole;
     const long long need = ((long long)max_len + CH - 1) / CH;
     if (seg > need) seg = need > 0 ? need : 1;
+    // One block a chain, without the workspace, where every chain has an SM and few chunks: up to three, and up to six where the chains take most of the SMs
+    // (with fewer the roles form a chain's items side by side, 16 to 7 % sooner from six chunks on).  (Lengths are not known here: one long sequence among
+    // short ones may then be on its own.)  us, over a workspace / so: 64 chains x 64 rows 25.6 / 14.7, 128 rows 28.8 / 20.4, 192 rows 30.8 / 27.4, 256 rows
+    // 32.1 / 34.5; 128 chains x 192 rows 49.8 / 35.8, 384 rows 80.2 / 56.2, 1,000 rows 129 / 118.  With more chains than SMs the last of them fill no wave.
+    if (scatter == nullptr && out != nullptr && chains <= sm_count() && max_len <= (chains * 4 > 3 * sm_count() ? 6 : 3) * CH)
+        return core_prefill_one_launch(heads, batch, cu_seqlens, q, k, v, g, beta, state_in, state_out, state_off, bf16_state, gate, norm_w, eps, out, stream);
     SpParams p{};
     p.H = heads; p.batch = batch; p.cu = cu_seqlens;
     p.q = q; p.k = k; p.v = v; p.g = g; p.beta = beta;
@@ -1984,6 +2343,36 @@ int core_prefill_static_launch(int32_t heads, int32_t batch, const int32_t* cu_s
     }
     return core_prefill_sp_launch(heads, batch, cu_seqlens, max_len, q, k, v, g, beta, state_in, state_out, state_off, bf16_state,
                                   gate, norm_w, eps, out, scratch_of[dev], kStaticScratchBytes, stream);
+}
+
+int core_prefill_one_launch(int32_t heads, int32_t batch, const int32_t* cu_seqlens, const glm53f_bf16* q, const glm53f_bf16* k,
+                            const glm53f_bf16* v, const float* g, const float* beta, const void* state_in, void* state_out,
+                            const int64_t* state_off, bool bf16_state, const glm53f_bf16* gate, const glm53f_bf16* norm_w,
+                            float eps, glm53f_bf16* out, cudaStream_t stream) {
+    static int configured_dev = -1;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (configured_dev != dev) {
+        cudaError_t e = cudaFuncSetAttribute(prefill_one_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemOne);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(prefill_one_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemOne);
+        if (e != cudaSuccess) return (int)e;
+        configured_dev = dev;
+    }
+    SpParams p{};
+    p.H = heads; p.batch = batch; p.cu = cu_seqlens;
+    p.q = q; p.k = k; p.v = v; p.g = g; p.beta = beta;
+    p.state_in = state_in; p.state_out = state_out;
+    p.state_off = reinterpret_cast<const long long*>(state_off);
+    p.state_bf16 = bf16_state ? 1 : 0;
+    p.gate = gate; p.gate_stride = (long long)heads * DV; p.norm_w = norm_w; p.eps = eps; p.out = out;
+    p.status = status_word();
+    if (p.status == nullptr) return (int)cudaErrorUnknown;
+    constexpr long long rows_cap = 0x7fffffffll;  // only whole chunks go by the maps, and max_len is not asked for here
+    if (!row_tensor_map(&p.tm_q, q, 2, heads, rows_cap) || !row_tensor_map(&p.tm_k, k, 2, heads, rows_cap) ||
+        !row_tensor_map(&p.tm_v, v, 2, heads, rows_cap) || !row_tensor_map(&p.tm_g, g, 4, heads, rows_cap) || !row_tensor_map(&p.tm_out, out, 2, heads, rows_cap) ||
+        (gate != nullptr && !row_tensor_map(&p.tm_gate, gate, 2, heads, rows_cap)))
+        return (int)cudaErrorNotSupported;
+    return launch_early(gate != nullptr ? prefill_one_kernel<true> : prefill_one_kernel<false>, (unsigned)(heads * batch), kOneThreads, kSmemOne, stream, p);
 }
 
 }  // namespace kda

@@ -1,5 +1,4 @@
-// Pieces shared by the chunk-64 tensor-core prefill kernels: the chunk geometry, the shared-memory map of the
-// state-independent ("intra") phase, the cell helpers and the FP32 triangular inverse.
+// Pieces of the chunk-64 tensor-core prefill kernels: the chunk geometry, the cell helpers and the FP32 triangular inverse.
 #pragma once
 
 #include "common.cuh"
@@ -10,42 +9,14 @@ namespace pf {
 
 constexpr int CH = 64;            // rows per chunk
 constexpr int kCompute = 512;     // 16 compute warps: warp w reaches TMEM lanes 32*(w%4).., and takes columns 32*(w/4)..
-constexpr int kThreadsTc = kCompute + 32;  // + one loader warp that streams the next chunk's rows in
-constexpr int RS16 = 272;         // staging row stride, bf16 tensors (256 + 16: rows 4 banks apart)
-constexpr int RS32 = 528;         // staging row stride, f32 tensor
-// Shared memory map (bytes).  Tiles are 64-row (R = 64) cell arrays unless noted; buffers whose lifetimes do not
-// overlap inside a chunk share space, so that the staging area is free again as soon as the operands are built and
-// the next chunk's rows can stream in behind the current chunk's arithmetic.
 constexpr int kTile = CH * 16 * 16;  // 16 KiB: 64 rows x 128 bf16
-constexpr int oRawQ = 0, oRawK = oRawQ + CH * RS16, oRawV = oRawK + CH * RS16, oRawG = oRawV + CH * RS16;
-constexpr int oKg = oRawG + CH * RS32;   // Kg                       (steps 2-6)   } later S16 [128 rows] (steps 8-9)
-constexpr int oKinv = oKg + kTile;        // Kinv (2-3)                             }
-constexpr int oTp = oKinv + kTile;        // T' hi | T' lo (5c-6), later D hi (steps 10-11)
-constexpr int oW = oTp + kTile;           // W                        (steps 7-9)
-constexpr int oV = oW + kTile;            // V                        (steps 2-6), later D lo
-constexpr int oQg = oV + kTile;           // Qg                       (steps 2-9)
-constexpr int oKdHi = oQg + kTile, oKdLo = oKdHi + kTile;  // Kdec hi, lo (steps 2-11)
-constexpr int oMm = oKdLo + kTile;        // M, 64 x 64 bf16          (steps 4-11)
-constexpr int oS16 = oKg, oDhi = oTp, oDlo = oV, oTpHi = oTp, oTpLo = oTp + kTile / 2;
-// The column sides of L and M, one tile per row block I (rows 0 .. 16 I + 15, 256 bytes a row), over Kinv | T' | W
-// (steps 2-3); the per-block decay factor tables (14 x 128 floats: E0[4], EL[4], F[6]) over M (steps 1-3).
-constexpr int oKc = oKinv, oTab = oMm, kTabs = 14, tE0 = 0, tEL = 4, tF = 8;
+// The column sides of L and M, one tile per row block I (rows 0 .. 16 I + 15, 256 bytes a row); the per-block decay factor tables (14 x 128
+// floats: E0[4], EL[4], F[6]).
+constexpr int kTabs = 14, tE0 = 0, tEL = 4, tF = 8;
 __device__ __forceinline__ int kc_tile(int I) { return 2048 * I * (I + 1); }
-static_assert(2 * 128 * (16 + 32 + 48 + 64) <= 3 * kTile && kTabs * 512 <= kTile / 2, "column-side tiles and tables");
-// FP32 scratch of the inversion (steps 4-5) over Kinv | T' | W, all dead then: T, P, L.  Rows are padded to 68
-// floats so that one lane per row spreads over the banks while float4 loads stay aligned.
+// FP32 scratch of the inversion: rows padded to 68 floats so that one lane per row spreads over the banks while float4 loads stay aligned.
 constexpr int LS = 68;
-constexpr int oT = oKinv, oP = oT + CH * LS * 4, oL = oKinv + 24576;
-static_assert(oP + 32 * 40 * 4 <= oL && oL + CH * LS * 4 <= oKinv + 3 * kTile, "inversion scratch");
-constexpr int oBeta = oMm + kTile / 2, oEGL = oBeta + 2 * CH * 4, oScan = oEGL + 128 * 4, oRed = oScan + 4 * 128 * 4;
-constexpr int oBars = oRed + 4 * CH * 4, oCtl = oBars + 32;
-constexpr int kSmemTc = oCtl + 32;
-static_assert(kSmemTc <= 232448, "shared memory budget");
-// Tensor memory columns.
-constexpr uint32_t cS = 0, cL = 128, cMm = 192, cW = 256, cQS = 256, cU = 384, kTmemCols = 512;
-
-
-__device__ __forceinline__ void compute_sync() { named_bar_sync(1, kCompute); }
+constexpr uint32_t kTmemCols = 512;
 
 __device__ __forceinline__ unsigned char* cell(unsigned char* tile, int R, int c, int r) { return tile + ((size_t)c * R + r) * 16; }
 
@@ -103,8 +74,8 @@ __device__ __forceinline__ float4 tile_row(const float2 (&c)[4][2], int kp) {
 constexpr int PS = 36;  // row stride of the merges' intermediate product
 
 // NT threads (numbered tid = 0 .. NT-1, at least eight warps) take part and meet at named barrier `bar`; ends with a barrier.
-template <int NT = kCompute>
-__device__ __forceinline__ void invert(const float* Lm, float* Tm, float* Pm, int tid, int bar = 1) {
+template <int NT>
+__device__ __forceinline__ void invert(const float* Lm, float* Tm, float* Pm, int tid, int bar) {
     const int warp = tid >> 5, lane = tid & 31;
     if (tid < 64) {  // a diagonal block's columns, one thread each, by substitution: a settled row at once goes into all later ones
         const int o = (tid >> 4) * 16, j = tid & 15;
