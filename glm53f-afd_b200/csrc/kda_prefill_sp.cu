@@ -2245,6 +2245,19 @@ int core_prefill_sp_launch(int32_t heads, int32_t batch, const int32_t* cu_seqle
         }
         return 0;
     }
+    // A workspace that holds everything is not reason enough for one segment, whose items and walks would run one after the other: from 64 chunks on two, from
+    // 128 on three, where there are items enough to wait for and SMs without a chain to form the next ones.  us, one / two / three segments: 64 heads, 2,048 rows 139 / 148 / 160,
+    // 4,096 rows 249 / 247 / 254, 8,192 rows 468 / 453 / 453 (with the norm 574 / 533 / 530); 32 heads, 8,192 rows 350 / 326 / 322, 12,288 rows 511 / 468 / 458;
+    // 20 heads, 8,192 rows 296 / 284 / 278; 16 heads, bf16 states, 4,096 rows 156 / 151; but 72 chains of as many 275 / 277, 96 with the norm 371 / 381 / 398,
+    // 8 heads, bf16 states, 8,192 rows with the norm 358 / - / 362, 4 heads, 4,096 rows 121 / 127.
+    if (scatter == nullptr && chains >= 16 && chains * 9 <= 4 * sms && need >= 64) {
+        const long long parts = need >= 128 ? 3 : 2, most = (need + parts - 1) / parts;
+        if (seg > most) {
+            seg = most;
+            p.seg_chunks = (int)seg;
+            half[1] = base + chains * seg * kSlotBytes;  // (a workspace of one chunk a chain has no halves, and its segments are below `most`)
+        }
+    }
     const long long segs = need > 0 ? (need + seg - 1) / seg : 0;
     int launch_no = 0;
     auto launch = [&](long long intra_seg, long long state_seg) -> int {
