@@ -44,8 +44,8 @@ TOKEN_OUT_BYTES = HEADS * DK * 2
 # of an 8-layer step (256 MiB of distinct states, caches left as they are between launches, so that one launch's
 # writes are evicted during the next ones as in the timed run); summarised under profiles/.
 NCU_DRAM_BYTES_PER_LAUNCH = 34_876_112 + 32_331_792
-# The same for the prefill kernel: 601 MB per captured launch of 2,048 (chain, chunk) items = 32 chunks of all 64 heads.
-NCU_PREFILL_DRAM_BYTES_PER_TOKEN = (393_953_280 + 207_395_072) // (32 * 64)
+# The same for the prefill kernel: 1,479 MB per captured launch of 5,504 (chain, chunk) items = 86 chunks of all 64 heads.
+NCU_PREFILL_DRAM_BYTES_PER_TOKEN = (955_447_808 + 523_866_368) // (86 * 64)
 
 
 def peaks():
