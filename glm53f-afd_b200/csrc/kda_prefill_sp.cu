@@ -104,6 +104,7 @@ struct SpParams {
     int state_bf16;
     const uint16_t* gate;
     long long gate_stride;  // elements between consecutive gate rows
+    int longest_first;      // prefill_one_kernel: blocks take the longest sequences' chains first
     int gate_boxes;         // full chunks' gate values come by tiled tensor copies (base and stride on 16 bytes)
     const uint16_t* norm_w;
     float eps;
@@ -274,7 +275,7 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
         if (!mbar_wait(bar_g, raw_phase, ctx, kStatusWaitPrefill)) break;
         const int item = item_slot[0], live = item_slot[1];  // (the next item's from when L and M are formed)
         if (item < 0) break;
-        const Item at_item = ONE ? Item{(int)blockIdx.x, item, 0} : item_of<FUSED>(p, item);
+        const Item at_item = ONE ? Item{0, item, 0} : item_of<FUSED>(p, item);
         unsigned char* slot = ONE ? smem + oSlotOne : slot_of(p.ws_intra, p.seg_chunks, at_item.chain, at_item.jj);
         uint64_t* one = reinterpret_cast<uint64_t*>(smem + oBarsOne);
 
@@ -650,7 +651,7 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // past the rows the caller's metadata names.    They are asynchronous, all in flight at once: as loads and stores, a row's after
 // the other's, they were 8 to 12 us of a launch (33 rows x 64 heads by the chunked layer prefill: 59 us, 64 rows 52).
 template <bool LAYER, bool FUSED, bool WALK_U, bool ONE = false>
-__device__ __forceinline__ void intra_loader(const SpParams& p, unsigned char* smem, const WaitCtx& ctx, const int G) {
+__device__ __forceinline__ void intra_loader(const SpParams& p, unsigned char* smem, const WaitCtx& ctx, const int G, const int one_chain = 0) {
     unsigned char* gs = smem + G * kGroupBytes;
     uint64_t* bar_raw = reinterpret_cast<uint64_t*>(gs + gBars);
     uint64_t *bar_free = bar_raw + 3, *bar_g = bar_raw + 4, *bar_gfree = bar_raw + 5;
@@ -677,7 +678,7 @@ __device__ __forceinline__ void intra_loader(const SpParams& p, unsigned char* s
         long long gr0 = 0;
         const unsigned char* in = nullptr;
         if (!last) {
-            const Item at = ONE ? Item{(int)blockIdx.x, (int)item, 0} : item_of<FUSED>(p, (int)item);
+            const Item at = ONE ? Item{one_chain, (int)item, 0} : item_of<FUSED>(p, (int)item);
             const int j = p.intra_chunk0 + at.jj, b = at.chain / H;
             h = at.chain % H;
             const int r0 = p.cu[b], T = p.cu[b + 1] - r0;
@@ -1877,6 +1878,21 @@ __device__ __forceinline__ void walk_one(const SpParams& p, unsigned char* smem,
     }
 }
 
+// The sequence that comes n-th when the longest come first (by each warp; up to kOrderSeqs of them).  Blocks of more chains than SMs are handed out in order, and a
+// long chain begun when the others end runs alone.  us, as they come / so: 16,384 rows x 32 heads in 8 sequences 621 / 446, 50,000 rows in 7 1,698 / 1,317; 64 heads,
+// 8,192 rows in 3 619 / 515, in 16 465 / 451, 12,000 in 6 678 / 643; where neither order fills the last round, 8,192 rows in 8 443 / 457, 3,000 in 3 245 / 249.  (The
+// fused launches' blocks take items as they go: there 1 to 2 % slower.)
+constexpr int kOrderSeqs = 32;
+__device__ __forceinline__ int nth_longest(const SpParams& p, int n) {
+    const int lane = threadIdx.x & 31, chunks = lane < p.batch ? (p.cu[lane + 1] - p.cu[lane] + CH - 1) / CH : -1;
+    int rank = 0;
+    for (int i = 0; i < p.batch; ++i) {
+        const int other = __shfl_sync(0xffffffffu, chunks, i);
+        rank += other > chunks || (other == chunks && i < lane) ? 1 : 0;
+    }
+    return __ffs(__ballot_sync(0xffffffffu, lane < p.batch && rank == n)) - 1;
+}
+
 template <bool GATED>
 __global__ void __launch_bounds__(kOneThreads, 1) prefill_one_kernel(const __grid_constant__ SpParams p) {
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -1899,9 +1915,11 @@ __global__ void __launch_bounds__(kOneThreads, 1) prefill_one_kernel(const __gri
     const uint32_t tm = *tmem_slot;
     grid_ready();
     const WaitCtx ctx{ctl, ctl + 1, p.status};
-    const Chain at = chain_of(p, Walk{0, 0x7fffffff, 0, nullptr, 0, nullptr, true, true}, (int)blockIdx.x);
+    int chain = blockIdx.x;
+    if (p.longest_first) chain = nth_longest(p, chain / p.H) * p.H + chain % p.H;
+    const Chain at = chain_of(p, Walk{0, 0x7fffffff, 0, nullptr, 0, nullptr, true, true}, chain);
     if (warp < kGroupThreads / 32) intra_group<false, false, false, true>(p, smem, tm, ctx, 0);
-    else if (warp == kOneLoader) intra_loader<false, false, false, true>(p, smem, ctx, 0);
+    else if (warp == kOneLoader) intra_loader<false, false, false, true>(p, smem, ctx, 0, chain);
     else walk_one<GATED>(p, smem, tm, ctx, at);
     if (ctl[1] != 0u) {  // after an abort copies into this block's shared memory may still be in flight: give them a bounded time
         const uint64_t t0 = global_timer_ns();
@@ -2380,6 +2398,7 @@ int core_prefill_one_launch(int32_t heads, int32_t batch, const int32_t* cu_seql
     p.gate = gate; p.gate_stride = (long long)heads * DV; p.norm_w = norm_w; p.eps = eps; p.out = out;
     p.status = status_word();
     if (p.status == nullptr) return (int)cudaErrorUnknown;
+    p.longest_first = batch > 1 && batch <= kOrderSeqs && (long long)heads * batch > sm_count() ? 1 : 0;
     constexpr long long rows_cap = 0x7fffffffll;  // only whole chunks go by the maps, and max_len is not asked for here
     if (!row_tensor_map(&p.tm_q, q, 2, heads, rows_cap) || !row_tensor_map(&p.tm_k, k, 2, heads, rows_cap) ||
         !row_tensor_map(&p.tm_v, v, 2, heads, rows_cap) || !row_tensor_map(&p.tm_g, g, 4, heads, rows_cap) || !row_tensor_map(&p.tm_out, out, 2, heads, rows_cap) ||
