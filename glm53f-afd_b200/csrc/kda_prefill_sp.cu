@@ -2086,11 +2086,13 @@ int core_prefill_sp_launch(int32_t heads, int32_t batch, const int32_t* cu_seqle
     long long seg = overlap ? whole / 2 : whole;
     const long long need = ((long long)max_len + CH - 1) / CH;
     if (seg > need) seg = need > 0 ? need : 1;
-    // One block a chain, without the workspace, where every chain has an SM and few chunks: up to three, and up to six where the chains take most of the SMs
-    // (with fewer the roles form a chain's items side by side, 16 to 7 % sooner from six chunks on).  (Lengths are not known here: one long sequence among
-    // short ones may then be on its own.)  us, over a workspace / so: 64 chains x 64 rows 25.6 / 14.7, 128 rows 28.8 / 20.4, 192 rows 30.8 / 27.4, 256 rows
-    // 32.1 / 34.5; 128 chains x 192 rows 49.8 / 35.8, 384 rows 80.2 / 56.2, 1,000 rows 129 / 118.  With more chains than SMs the last of them fill no wave.
-    if (scatter == nullptr && out != nullptr && chains <= sm_count() && max_len <= (chains * 4 > 3 * sm_count() ? 6 : 3) * CH)
+    // One block a chain, without the workspace, where the chains have few chunks: up to three where every chain has an SM, or where a second round of them takes
+    // more than half of the SMs; up to six where the chains are more than three quarters of one round.  (With fewer chains the roles form a chain's items side by
+    // side, 7 to 16 % sooner from six chunks on.  Lengths are not known here: one long sequence among short ones may then be on its own.)  us, over a workspace / so:
+    // 64 chains x 64 rows 25.6 / 14.7, 128 rows 28.8 / 20.4, 192 rows 30.8 / 27.4, 256 rows 32.1 / 34.5; 128 chains x 192 rows 49.8 / 35.8, 384 rows 80.2 / 56.2;
+    // 256 chains x 64 rows 43.0 / 35.3, x 128 rows (the longest 192) 55.5 / 48.5; but 192 chains x 128 rows 47.2 / 47.1, 160 x 192 52.9 / 54.0, 320 x 128 65.2 / 66.4.
+    const long long at_once = sm_count(), chunks_alone = chains > 2 * at_once ? 0 : chains > at_once ? (chains * 2 > 3 * at_once ? 3 : 0) : chains * 4 > 3 * at_once ? 6 : 3;
+    if (scatter == nullptr && out != nullptr && max_len <= chunks_alone * CH)
         return core_prefill_one_launch(heads, batch, cu_seqlens, q, k, v, g, beta, state_in, state_out, state_off, bf16_state, gate, norm_w, eps, out, stream);
     SpParams p{};
     p.H = heads; p.batch = batch; p.cu = cu_seqlens;
