@@ -66,3 +66,27 @@ def test_layer(rows):
         K.set_prefill_form(form)
     for a, b in zip(*got):
         assert torch.isfinite(a).all() and torch.equal(a, b)
+
+
+def test_scan_over_segments(monkeypatch):
+    core = importlib.import_module("glm53f-afd_b200.core")
+    heads, lens, gen = 40, [300, 130], torch.Generator(device="cuda").manual_seed(5)
+    n, per = sum(lens) * heads, heads * DK * DK
+    rn = lambda *s: torch.randn(*s, device="cuda", generator=gen)
+    unit = lambda s: torch.nn.functional.normalize(rn(n, DK), dim=1).mul(s).bfloat16().view(-1)
+    q, k, v = unit(DK ** -0.5), unit(1.0), rn(n * DK).bfloat16()
+    g, beta, start = torch.nn.functional.logsigmoid(rn(n * DK) + 3), torch.sigmoid(rn(n)), rn(2 * per) * 0.05
+    cu, off = torch.tensor([0] + lens, device="cuda").cumsum(0).int(), torch.arange(2, device="cuda") * per
+
+    def run(segments):
+        monkeypatch.setenv("GLM53F_KDA_PREFILL_SEGMENTS", str(segments))
+        out, st = torch.zeros(n * DK, dtype=torch.bfloat16, device="cuda"), start.clone()
+        ws = torch.full((core.prefill_workspace_bytes(heads, 2, 20),), 0xff, dtype=torch.uint8, device="cuda")
+        core.prefill_varlen(heads, sum(lens), cu, max(lens), q, k, v, g, beta, st, off, out=out, workspace=ws)
+        torch.cuda.synchronize()
+        assert core.device_status() == 0
+        return out.double(), st.double()
+
+    (out, st), (out_1, st_1) = run(2), run(1)  # the bounds of the other scans: an ulp of bf16 of the largest output, the states' error of the chunked form
+    assert float((out - out_1).abs().max() / out_1.abs().max()) <= 1 / 128
+    assert 0 < float((st - st_1).norm() / st_1.norm()) <= 3e-4
