@@ -237,7 +237,9 @@ __global__ void __launch_bounds__(kPairThreads, 1) proj_gemm_pair_kernel(const _
         // Sixteen rows of the accumulator from c0 on.  For tensor stores in the fragment layout, from which transposing matrix stores put rows of eight
         // features into the boxes: v[8 h + 4 g + 2 p + e] = feature 16 h + 8 p + lane / 4 of the warp, row c0 + 8 g + 2 (lane % 4) + e.  (With lane = feature, 32
         // two-byte stores where four are enough now: the k = 128 gate factor at 512 rows
-        // 13.8 -> 12.5 us, at 1,024 24.5 -> 21.3.)  Else lane = feature, v[j] = row c0 + j.
+        // 13.8 -> 12.5 us, at 1,024 24.5 -> 21.3.)  Else lane = feature, v[j] = row c0 + j; and so in the instance that keeps the sums of more than 128 rows,
+        // whose registers are full (o_proj at 513, 660 and 768 rows 40.6, 43.4 and 44.6 us, from fragments 45.9, 48.8 to 52.4 and 51.0 to 56.9).
+        constexpr bool kFragments = SPLIT_ROWS <= 128;
         auto load = [&](const PairTile& x, int c0, float* v) {
             uint32_t r[16];
             if (x.q.tensor_out) {
@@ -264,16 +266,25 @@ __global__ void __launch_bounds__(kPairThreads, 1) proj_gemm_pair_kernel(const _
                 out_buf ^= 1;
                 if (issuer) bulk_wait_read<1>();  // this buffer's last stores have been read
                 named_bar_sync(bar, 64);
-                // A lane names row lane % 8 of matrix lane / 8: features 8 ((lane / 8) % 2), rows 8 (lane / 16) of the sixteen by sixteen.
-                const int row = (lane >> 4) * 8 + (lane & 7), piece = (q & 1) * 4 + ((lane >> 3) & 1);
+                if constexpr (kFragments) {
+                    // A lane names row lane % 8 of matrix lane / 8: features 8 ((lane / 8) % 2), rows 8 (lane / 16) of the sixteen by sixteen.
+                    const int row = (lane >> 4) * 8 + (lane & 7), piece = (q & 1) * 4 + ((lane >> 3) & 1);
 #pragma unroll
-                for (int c = 0; c < 2; ++c)
+                    for (int c = 0; c < 2; ++c)
 #pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const float* w = v + 16 * c + 8 * h;
-                        tc::stmatrix_t4(box + (16 * c + row) * 128 + (((piece + 2 * h) ^ (row & 7)) << 4), tc::bf16x2(w[0], w[1]), tc::bf16x2(w[2], w[3]), tc::bf16x2(w[4], w[5]),
-                                        tc::bf16x2(w[6], w[7]));
+                        for (int h = 0; h < 2; ++h) {
+                            const float* w = v + 16 * c + 8 * h;
+                            tc::stmatrix_t4(box + (16 * c + row) * 128 + (((piece + 2 * h) ^ (row & 7)) << 4), tc::bf16x2(w[0], w[1]), tc::bf16x2(w[2], w[3]),
+                                            tc::bf16x2(w[4], w[5]), tc::bf16x2(w[6], w[7]));
+                        }
+                } else {
+#pragma unroll
+                    for (int j = 0; j < kChunk; j += 2) {
+                        const uint32_t two = tc::bf16x2(v[j], v[j + 1]);
+                        *reinterpret_cast<uint16_t*>(box + j * 128 + (((fl >> 3) ^ (j & 7)) << 4) + (fl & 7) * 2) = (uint16_t)two;
+                        *reinterpret_cast<uint16_t*>(box + (j + 1) * 128 + (((fl >> 3) ^ ((j + 1) & 7)) << 4) + (fl & 7) * 2) = (uint16_t)(two >> 16);
                     }
+                }
                 fence_proxy_async_smem();
                 named_bar_sync(bar, 64);
                 if (issuer) {
@@ -323,8 +334,16 @@ __global__ void __launch_bounds__(kPairThreads, 1) proj_gemm_pair_kernel(const _
                 if (!arrived()) goto done;
                 for (int c0 = set * kChunk; c0 < x.q.row_tile; c0 += 2 * kChunk) {
                     float v[kChunk];
-                    load(x, c0, v);
-                    load(x, c0 + 16, v + 16);
+                    if constexpr (kFragments) {
+                        load(x, c0, v);
+                        load(x, c0 + 16, v + 16);
+                    } else {
+                        uint32_t r[kChunk];
+                        tc::tmem_ld32(tc::tmem_addr(tm, q, buf * kPN + c0), r);
+                        tc::tmem_ld_wait();
+#pragma unroll
+                        for (int j = 0; j < kChunk; ++j) v[j] = __uint_as_float(r[j]);
+                    }
                     emit(x, c0, v);
                 }
                 release();
@@ -338,10 +357,18 @@ __global__ void __launch_bounds__(kPairThreads, 1) proj_gemm_pair_kernel(const _
                         if (c0 >= x.q.row_tile) break;
 #pragma unroll
                         for (int j0 = 0; j0 < kChunk; j0 += 16) {
-                            float r[16];
-                            load(x, c0 + j0, r);
+                            if constexpr (kFragments) {
+                                float r[16];
+                                load(x, c0 + j0, r);
 #pragma unroll
-                            for (int j = 0; j < 16; ++j) sum[c][j0 + j] = seg == 0 ? r[j] : sum[c][j0 + j] + r[j];
+                                for (int j = 0; j < 16; ++j) sum[c][j0 + j] = seg == 0 ? r[j] : sum[c][j0 + j] + r[j];
+                            } else {
+                                uint32_t r[16];
+                                tc::tmem_ld16(tc::tmem_addr(tm, q, buf * kPN + c0 + j0), r);
+                                tc::tmem_ld_wait();
+#pragma unroll
+                                for (int j = 0; j < 16; ++j) sum[c][j0 + j] = seg == 0 ? __uint_as_float(r[j]) : sum[c][j0 + j] + __uint_as_float(r[j]);
+                            }
                         }
                     }
                     release();
