@@ -223,11 +223,6 @@ __device__ __forceinline__ float rcp_approx(float x) {
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
-__device__ __forceinline__ float rcp_full(float x) {  // the same with denormal results
-    float r;
-    asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
-}
 __device__ __forceinline__ float ex2_approx(float x) {
     float r;
     asm("ex2.approx.f32 %0, %1;" : "=f"(r) : "f"(x));

@@ -988,8 +988,9 @@ __device__ __forceinline__ void state_to_tmem(uint32_t at, const uint16_t* from,
 
 // The gated RMSNorm of sixteen output rows from i0 on by four warps, which have 32 channels each and meet at barrier `bar`; red: their sums, [4][64].  y2[g][q]:
 // rows fi + 8 g and the next (fi = i0 + 2 (lane % 4)) of channel fv + 8 q as bf16, gt the gate's values alike, which `fetch` may bring behind the barrier.
-// False on all four when one of them comes without `ok`.  FULL: the sigmoid also where it is too faint for rcp_approx().
-template <bool FULL, typename Fetch>
+// False on all four when one of them comes without `ok`.  The sigmoid is formed sixteenfold and a row's factor a sixteenth: below -87.3 the gate's sigmoid is not
+// a normal number, which the reciprocal would flush, but leaves outputs that bf16 holds.
+template <typename Fetch>
 __device__ __forceinline__ bool gated_rows(float* red, float eps, int quad, int lane, int i0, const float (&nw)[4], uint32_t (&gt)[2][4], uint32_t (&y2)[2][4], int bar, bool ok, Fetch&& fetch) {
     float sq[4];  // [2 g + e]
 #pragma unroll
@@ -1014,14 +1015,14 @@ __device__ __forceinline__ bool gated_rows(float* red, float eps, int quad, int 
     if (ok) fetch();
     // A row's factor is formed by one lane of each of the first two quarters (a square root and a division, both IEEE).
     const float* at = red + i0 + (lane & 15);
-    const float rinv = 1.0f / sqrtf((((at[0] + at[CH]) + at[2 * CH]) + at[3 * CH]) / (float)DV + eps);
-    auto rcp = [](float x) { return FULL ? rcp_full(x) : rcp_approx(x); };
+    const float rinv = 0.0625f * (1.0f / sqrtf((((at[0] + at[CH]) + at[2 * CH]) + at[3 * CH]) / (float)DV + eps));
+    auto sigmoid16 = [](float x) { return rcp_approx(fmaf(ex2_ftz(-kLog2e * x), 0.0625f, 0.0625f)); };
 #pragma unroll
     for (int g = 0; g < 2; ++g) {
         const float2 rv = {__shfl_sync(0xffffffffu, rinv, 2 * (lane & 3) + 8 * g), __shfl_sync(0xffffffffu, rinv, 2 * (lane & 3) + 8 * g + 1)};
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-            const float2 sig = {rcp(1.0f + ex2_ftz(-kLog2e * __uint_as_float(gt[g][q] << 16))), rcp(1.0f + ex2_ftz(-kLog2e * __uint_as_float(gt[g][q] & 0xffff0000u)))};
+            const float2 sig = {sigmoid16(__uint_as_float(gt[g][q] << 16)), sigmoid16(__uint_as_float(gt[g][q] & 0xffff0000u))};
             const float2 y = mul2(mul2({nw[q], nw[q]}, mul2({__uint_as_float(y2[g][q] << 16), __uint_as_float(y2[g][q] & 0xffff0000u)}, rv)), sig);
             y2[g][q] = tc::bf16x2(y.x, y.y);
         }
@@ -1410,7 +1411,7 @@ __device__ void state_role(const SpParams& p, unsigned char* smem, const uint32_
         unsigned char* dst = smem + sOut + (c & 1) * kOutTile;
         if (votes) {
             if (boxes) ok = ok && wait(bGate + (c & 1), c >> 1);
-            ok = gated_rows<false>(reinterpret_cast<float*>(smem + sRed) + (c & 1) * 4 * CH, p.eps, quad, lane, i0, nw, gt, y2, 4 + cg, ok, [&] {
+            ok = gated_rows(reinterpret_cast<float*>(smem + sRed) + (c & 1) * 4 * CH, p.eps, quad, lane, i0, nw, gt, y2, 4 + cg, ok, [&] {
                 if (boxes) {
                     tc::ldmatrix_t4(dst + box_piece(tile_row, tile_piece), gt[0][0], gt[0][1], gt[1][0], gt[1][1]);
                     tc::ldmatrix_t4(dst + box_piece(tile_row, tile_piece + 2), gt[0][2], gt[0][3], gt[1][2], gt[1][3]);
@@ -1856,7 +1857,7 @@ __device__ __forceinline__ void walk_one(const SpParams& p, unsigned char* smem,
 #pragma unroll
         for (int s = 0; s < 2; ++s) {
             const int i0 = (piece0 + s) * 16, tile_row = i0 + (lane >> 4) * 8 + (lane & 7);
-            if (GATED && !gated_rows<true>(reinterpret_cast<float*>(smem + oRedOne), p.eps, quad, lane, i0, nw, gt[s], y2[s], 4 + half, ok, [&] {
+            if (GATED && !gated_rows(reinterpret_cast<float*>(smem + oRedOne), p.eps, quad, lane, i0, nw, gt[s], y2[s], 4 + half, ok, [&] {
                     if (boxes) {
                         tc::ldmatrix_t4(tile + box_piece(tile_row, tile_piece), gt[s][0][0], gt[s][0][1], gt[s][1][0], gt[s][1][1]);
                         tc::ldmatrix_t4(tile + box_piece(tile_row, tile_piece + 2), gt[s][0][2], gt[s][0][3], gt[s][1][2], gt[s][1][3]);
