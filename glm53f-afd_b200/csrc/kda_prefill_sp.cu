@@ -1708,6 +1708,7 @@ __device__ __forceinline__ void walk_one(const SpParams& p, unsigned char* smem,
             if (leader) atomicAdd(const_cast<uint32_t*>(ctx.progress), 1u);
             __syncwarp();
         }
+        if (tc::warp_all(count > 0)) ready(o1Free, count - 1);  // nobody else waits for the last chunk's
         return;
     }
     // Eight warps: a thread has a value channel (tensor-memory lane) and two pieces of 32 key channels or 16 rows.
