@@ -2107,12 +2107,17 @@ int core_prefill_sp_launch(int32_t heads, int32_t batch, const int32_t* cu_seqle
     long long seg = overlap ? whole / 2 : whole;
     const long long need = ((long long)max_len + CH - 1) / CH;
     if (seg > need) seg = need > 0 ? need : 1;
-    // One block a chain, without the workspace, where the chains have few chunks: up to three where every chain has an SM, or where a second round of them takes
-    // more than half of the SMs; up to six where the chains are more than three quarters of one round.  (With fewer chains the roles form a chain's items side by
-    // side, 7 to 16 % sooner from six chunks on.  Lengths are not known here: one long sequence among short ones may then be on its own.)  us, over a workspace / so:
-    // 64 chains x 64 rows 25.6 / 14.7, 128 rows 28.8 / 20.4, 192 rows 30.8 / 27.4, 256 rows 32.1 / 34.5; 128 chains x 192 rows 49.8 / 35.8, 384 rows 80.2 / 56.2;
-    // 256 chains x 64 rows 43.0 / 35.3, x 128 rows (the longest 192) 55.5 / 48.5; but 192 chains x 128 rows 47.2 / 47.1, 160 x 192 52.9 / 54.0, 320 x 128 65.2 / 66.4.
-    const long long at_once = sm_count(), chunks_alone = chains > 2 * at_once ? 0 : chains > at_once ? (chains * 2 > 3 * at_once ? 3 : 0) : chains * 4 > 3 * at_once ? 6 : 3;
+    // One block a chain, without the workspace, where the chains have few chunks.  The lengths are not known here, and a long sequence among short ones has only its
+    // own chains' blocks at work where the two roles would spread its items, so the line is where that call, too, is no slower.  us, over a workspace of 32
+    // chunks / so, inputs not in L2:
+    //  - every chain has an SM: up to three chunks (1 chain x 192 rows 42 / 38, with the norm 52 / 44; 64 chains + 64 of one row 47 / 38; 128 alike 61 / 40);
+    //  - of more than three quarters of the SMs: four (4 chains x 256 rows + 136 of one row 45 / 42), and where one sequence's chains are more than a quarter of the
+    //    SMs, five and six (39 heads, 3 sequences, one of 320 rows 50 / 50, of 384 61 / 58; 48 heads 61 / 52 and 64 / 59; 112 chains x 384 rows 78 / 60; but 4 heads, one
+    //    of 35 sequences of 320 rows 46 / 48, 14 heads, one of 8 of 384 rows 45 / 53);
+    //  - in a second round of more than half of the SMs: two, without the norm (256 chains x 64 rows 45 / 42, x 128 rows 60 / 58, one sequence of four that long
+    //    52 / 46, 8 heads and one of 30 45 / 45; x 192 rows 69 / 73; with the norm x 128 rows 65 / 66, 192 rows 77 / 85); 192 chains x 128 rows 47 / 47, 320 65 / 66.
+    const long long at_once = sm_count(), nearly_all = heads * 4ll > at_once ? 6 : 4;
+    const long long chunks_alone = chains <= at_once ? (chains * 4 > 3 * at_once ? nearly_all : 3) : chains <= 2 * at_once && chains * 2 > 3 * at_once && gate == nullptr ? 2 : 0;
     if (scatter == nullptr && out != nullptr && max_len <= chunks_alone * CH)
         return core_prefill_one_launch(heads, batch, cu_seqlens, q, k, v, g, beta, state_in, state_out, state_off, bf16_state, gate, norm_w, eps, out, stream);
     SpParams p{};
