@@ -719,6 +719,32 @@ def cpu_prefill_toks(seconds: float):
     return n * t / dt, cores, f"{n} x {t} tokens x {HEADS} heads, chunk-64 form, in {dt:.1f} s"
 
 
+def prefill_launches(chains, need, ws_chunks, sms, ranks=1):
+    """Kernels of one core prefill call: a sequence of `need` chunks (more than six), `chains` heads on `sms` SMs, FP32 states, over a workspace of `ws_chunks`
+    chunks a chain (0: none), its rows stored into `ranks` full buffers: the segments that core_prefill_sp_launch cuts the call into."""
+    up = lambda a, b: -(-a // b)
+    if ws_chunks == 0:
+        return 1
+    slot, scan_state = 107008, 128 * 128 * 4
+    if chains <= 16:  # the scan over segments, where the workspace holds every chunk and the segments' states
+        k = min(sms // (2 * chains) + 1, sms // chains, 16, need // 32)
+        if ranks > 1 and k >= 2:
+            blocks, ks = 8, min(k, max(48 // chains, 2))
+            while blocks > 1 and need // (blocks * ks) < 32:
+                blocks -= 1
+            per = up(need, blocks)
+            if blocks > 1 and blocks * (per * slot + (3 * ks + 1) * scan_state) <= ws_chunks * slot:
+                return 4 * up(need, per)  # items, two walks of every segment, composition, walk with the outputs
+        if k >= 2 and need * slot + (3 * k - 2) * scan_state <= ws_chunks * slot:
+            return 4
+    if chains > sms:  # one launch a pass
+        return up(need, ws_chunks)
+    seg = min(max(ws_chunks // 2, 1), need)
+    if ranks == 1 and chains >= 16 and chains * 9 <= 4 * sms and need >= 64:  # two or three parts also where the workspace holds all
+        seg = min(seg, up(need, 3 if need >= 128 else 2))
+    return up(need, seg) + 1 if ws_chunks >= 2 else 2 * need
+
+
 def run_prefill(torch, dist, pkg, core, rank, world, tokens, passes, ws_chunks, check_heads=0):
     """Config 3: chunked prefill of one long sequence, heads sharded over the ranks, outputs all-gathered."""
     import ctypes as C
@@ -810,12 +836,8 @@ def run_prefill(torch, dist, pkg, core, rank, world, tokens, passes, ws_chunks, 
     gbs = tokens * PREFILL_BYTES_PER_TOKEN * (hl / HEADS) / (ms_compute * 1e-3) / 1e9      # per GPU
     tflops = tokens * PREFILL_FLOP_PER_TOKEN * (hl / HEADS) / (ms_compute * 1e-3) / 1e12  # per GPU
     chunks = (tokens + 63) // 64
-    if world > 1 and ws_chunks > chunks:  # the scan over segments: intra role, two passes of walks, the composition
-        kernels_per_pass = 4
-    elif ws_chunks >= 2:  # workspace halves: one launch per segment of ws_chunks // 2 chunks, plus the last state role
-        kernels_per_pass = (chunks + ws_chunks // 2 - 1) // (ws_chunks // 2) + 1
-    else:                 # one chunk per launch pair, or the single-pass kernel
-        kernels_per_pass = 2 * chunks if ws_chunks == 1 else 1
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    kernels_per_pass = prefill_launches(hl, chunks, ws_chunks, sms, world)
     res = {
         "workload": f"config 3: one sequence of {tokens} tokens, H=64 ({hl} heads per GPU), d=128, chunk 64, FP32 state",
         "value": tokens / (ms_total * 1e-3), "unit": "tokens/s per layer", "ms_per_layer": ms_total,
@@ -826,7 +848,7 @@ def run_prefill(torch, dist, pkg, core, rank, world, tokens, passes, ws_chunks, 
                      "tensor": {"achieved": tflops, "peak": tf, "unit": "TFLOP/s", "frac": tflops / tf, "peak_source": tf_kind,
                                 "flop_per_token": PREFILL_FLOP_PER_TOKEN},
                      "algorithmic_bytes_per_token": PREFILL_BYTES_PER_TOKEN,
-                     "traffic_bytes_per_token": NCU_PREFILL_DRAM_BYTES_PER_TOKEN if ws_chunks > 0 else None,
+                     "traffic_bytes_per_token": NCU_PREFILL_DRAM_BYTES_PER_TOKEN if ws_chunks > 1 and hl == HEADS else None,  # measured at 64 heads, the walk beside the items
                      "kernel": "prefill_sp_kernel (state role + intra role)" if ws_chunks > 0 else "prefill_one_kernel",
                      "workspace_bytes": 0 if ws is None else ws.numel()},
         "gpu_launches": passes * kernels_per_pass,
