@@ -89,7 +89,7 @@ __device__ __forceinline__ float2 widen2(uint32_t w) {
 }
 
 struct SpParams {
-    alignas(64) CUtensorMap tm_q, tm_k, tm_v, tm_g;  // [rows][H][128] as (128, H, rows); boxes of 64 rows (v: 32) x 128 bytes, 128-byte swizzle
+    alignas(64) CUtensorMap tm_q, tm_k, tm_v, tm_g;  // [rows][H][128] as (128, H, rows); boxes of 64 rows x 128 bytes, 128-byte swizzle
     alignas(64) CUtensorMap tm_out;                  // the shard-local output, the same way
     alignas(64) CUtensorMap tm_gate;                 // the gate rows, the same way (gate_boxes != 0)
     alignas(64) CUtensorMap tm_full[8];              // every rank's full output buffer: (128, heads_total, rows)
@@ -667,7 +667,7 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // The loader warp of group G: takes items off the counter and brings each one's rows into the group's staging.  A full
 // chunk arrives by eight or ten tiled tensor copies issued by one lane; a sequence's last, partial chunk by the warp's own
 // 16-byte copies (rows past the sequence's end are not read, they become zero), so no copy ever reaches
-// past the rows the caller's metadata names.    They are asynchronous, all in flight at once: as loads and stores, a row's after
+// past the rows the caller's metadata names.  They are asynchronous, all in flight at once: as loads and stores, a row's after
 // the other's, they were 8 to 12 us of a launch (33 rows x 64 heads by the chunked layer prefill: 59 us, 64 rows 52).
 template <bool LAYER, bool FUSED, bool WALK_U, bool ONE = false>
 __device__ __forceinline__ void intra_loader(const SpParams& p, unsigned char* smem, const WaitCtx& ctx, const int G, const int one_chain = 0) {
@@ -1998,14 +1998,14 @@ __global__ void __launch_bounds__(128) scan_compose_kernel(const __grid_constant
 
 }  // namespace
 
-// A [rows][H][128] tensor of `elem`-byte elements, its rows row_bytes apart (0: dense), as (128, H, rows) with boxes of 64 (or
-// box_rows) rows of one head, 128 bytes wide.
-static bool row_tensor_map(CUtensorMap* tm, const void* base, int elem, int H, long long rows, long long row_bytes = 0, int box_rows = CH) {
+// A [rows][H][128] tensor of `elem`-byte elements, its rows row_bytes apart (0: dense), as (128, H, rows) with boxes of 64 rows of one
+// head, 128 bytes wide.
+static bool row_tensor_map(CUtensorMap* tm, const void* base, int elem, int H, long long rows, long long row_bytes = 0) {
     EncodeTiled enc = encode_tiled();
     if (enc == nullptr) return false;
     const cuuint64_t dims[3] = {(cuuint64_t)DK, (cuuint64_t)H, (cuuint64_t)rows};
     const cuuint64_t strides[2] = {(cuuint64_t)DK * elem, row_bytes != 0 ? (cuuint64_t)row_bytes : (cuuint64_t)H * DK * elem};
-    const cuuint32_t box[3] = {(cuuint32_t)(128 / elem), 1u, (cuuint32_t)box_rows};
+    const cuuint32_t box[3] = {(cuuint32_t)(128 / elem), 1u, (cuuint32_t)CH};
     const cuuint32_t estr[3] = {1u, 1u, 1u};
     return enc(tm, elem == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<void*>(base), dims, strides, box, estr,
                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,

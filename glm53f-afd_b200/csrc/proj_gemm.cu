@@ -410,8 +410,8 @@ bool matrix_map(CUtensorMap* tm, int* swapped, const void* base, long long k, lo
 
 // K splits for a launch of few tiles (little n, deep k: o_proj at decode): the largest of 8, 4, 2 that divides the
 // k blocks into runs of at least four and still leaves every block of a one-row-tile launch resident at once.  It is
-// a function of (n, k, groups) alone in all launches of up to 512 rows (beyond 64 rows the same parts of k are summed in the
-// same order on SM pairs), so a row's bits do not depend on `rows` there.  Measured for
+// a function of (n, k, groups) alone in all launches of up to 512 rows (beyond 96 rows, 128 for a split k by itself, the same parts of k are summed
+// in the same order on SM pairs), so a row's bits do not depend on `rows` there.  Measured for
 // o_proj at 16 rows (32 tiles): no split 40.7 us, 2 splits 27.1, 4 splits 20.9, 8 splits (two waves of clusters) 24.7.
 int pick_ksplit(long long tiles, int kblocks, long long resident) {
     for (int s = 8; s >= 2; s >>= 1)
