@@ -327,18 +327,20 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
             const float first2 = all[0] + all[1], first3 = first2 + all[2], gl = first3 + all[3];
             // (Denormals are wanted here: sixteen rows at the gate's bound decay by e^-93, and their factor meets others of e^+40 and e^+46.)
             float* tab = reinterpret_cast<float*>(gs + gTab) + d;
+            auto own = [&](int b, float before, float after) {
+                const float e0 = ex2_approx(before), el = ex2_approx(after);
+                tab[(tE0 + b) * 128] = e0;
+                tab[(tEL + b) * 128] = el;
+                reinterpret_cast<float*>(gs + gE0L)[b * 128 + d] = e0 * el;
+            };
             if (part == 0) {
                 const float last2 = all[2] + all[3];
-                const float e0[4] = {ex2_approx(to[0]), ex2_approx(all[0] + to[1]), ex2_approx(first2 + to[2]), ex2_approx(first3 + to[3])};
-                const float el[4] = {ex2_approx(behind[0] + (all[1] + last2)), ex2_approx(behind[1] + last2), ex2_approx(behind[2] + all[3]), ex2_approx(behind[3])};
-#pragma unroll
-                for (int b = 0; b < 4; ++b) {
-                    tab[(tE0 + b) * 128] = e0[b];
-                    tab[(tEL + b) * 128] = el[b];
-                    reinterpret_cast<float*>(gs + gE0L)[b * 128 + d] = e0[b] * el[b];
-                }
-            } else {
+                own(0, to[0], behind[0] + (all[1] + last2));
+                own(1, all[0] + to[1], behind[1] + last2);
+                own(2, first2 + to[2], behind[2] + all[3]);
                 tab[(tF + 0) * 128] = ex2_approx(behind[0] + to[1]);
+            } else {
+                own(3, first3 + to[3], behind[3]);
                 tab[(tF + 1) * 128] = ex2_approx((behind[0] + all[1]) + to[2]); tab[(tF + 2) * 128] = ex2_approx(behind[1] + to[2]);
                 tab[(tF + 3) * 128] = ex2_approx((behind[0] + (all[1] + all[2])) + to[3]); tab[(tF + 4) * 128] = ex2_approx((behind[1] + all[2]) + to[3]); tab[(tF + 5) * 128] = ex2_approx(behind[2] + to[3]);
                 const float egl = ex2_approx(gl);
