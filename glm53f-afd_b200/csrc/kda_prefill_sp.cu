@@ -186,6 +186,14 @@ static_assert(kSmemSp <= 232448, "shared memory budget");
 // E_last, M, W, U or T'), in the un-swizzled cell layout the state role reads, so no result tile lives in shared memory.
 // =====================================================================================================================
 constexpr int kGroupThreads = 256, kGroups = 2;
+// Strong decays (core forms).  A thread sums its channel's decays over 32 rows, and what lies between two rows is a difference.  Of strong decays the rounding of long sums
+// would pass through the exponential into the states.  So a thread whose first nine rows decay by more than e^-8.5 (as in a chunk of e^-60, from where on chunks take
+// block-wise references) begins its sums anew at a block's first row and behind its middle row, and block-wise chunks form their tables once more, from the sums of
+// just the decays between two rows.  The states' distance from 64 bits, decays of e^-4 and e^-5.8 a row that vary by a fifth: 4.5e-6 and 3.4e-6; from differences
+// 1.1e-5 and 1.7e-5, of sums over sixteen rows 1.0e-5 and 1.5e-5; at e^-0.9 and milder the operands' rounding is all there is to see, either way.
+// us, before / so: 8,192 rows in 8 sequences 467 / 467, strong 496 / 498; 65,536 rows x 64 heads 3,532 / 3,544; 16,384 rows x 8 heads without a workspace 1,686 / 1,691.
+// The choice by a branch, or before the factors are formed, cost all chunks 1 to 3 %.
+constexpr float kStrong = -8.5f * kLog2e;
 // Decay range.  L and M hold exp(G_i - G_j) for every pair of rows j <= i of a chunk, and a tensor-core product can
 // only form it as (row factor) x (column factor).  With the model's gate bound (log decay down to -5.8 per row, -371
 // per chunk) neither exp(G) nor exp(-G) is representable, so the pair is split at a reference row r between j and i:
@@ -206,11 +214,10 @@ constexpr int gK = 0, gV = kTile, gQ = 2 * kTile, gKb = 3 * kTile, gKc = 4 * kTi
 constexpr int gG = gKc + 8192, gT = gQ, gL = gT + CH * LS * 4, gTp = gL;
 static_assert(gTp % 1024 == 0 && gKc % 1024 == 0, "swizzled tiles are 1024-byte aligned");
 // Per-block decay factors, 128 channels each: E0[J] = exp(Gm_J), EL[J] = exp(G_last - Gm_J), F[I(I-1)/2 + J] =
-// exp(Gm_I - Gm_J) for I > J.  E0[J] EL[J], for chunks of one reference row, lies over the column-side tiles, which those do not have.
-constexpr int gE0L = gKc;
-constexpr int gTab = gKc + kKcBytes, gP = gTab, gBeta = gTab + kTabs * 512, gBars = gBeta + CH * 4, kGroupBars = 6, gItem = gBars + kGroupBars * 8, gGl = gItem + 16;  // gGl: exp(G_last) [128] (ONE)
+// exp(Gm_I - Gm_J) for I > J.
+constexpr int gTab = gKc + kKcBytes, gP = gTab, gBeta = gTab + kTabs * 512, gBars = gBeta + CH * 4, kGroupBars = 6, gItem = gBars + kGroupBars * 8, gGl = gItem + 16;  // gGl: exp(G_last) [128]
 constexpr int kGroupBytes = 114688;
-static_assert(gG + 4 * kBox <= gTab && gG % 1024 == 0 && 32 * PS * 4 <= kTabs * 512 && gL + CH * LS * 4 <= gG && gE0L + 4 * 512 <= gG && gGl + 512 <= kGroupBytes && kGroupBytes % 1024 == 0, "group map");
+static_assert(gG + 4 * kBox <= gTab && gG % 1024 == 0 && 32 * PS * 4 <= kTabs * 512 && gL + CH * LS * 4 <= gG && gGl + 512 <= kGroupBytes && kGroupBytes % 1024 == 0, "group map");
 static_assert(kGroups * kGroupBytes <= oCtl, "two groups must fit below the block's control words");
 constexpr uint32_t gcL = 0, gcM = 64, gcW = 0, gcU = 64, kGroupCols = 128;
 
@@ -284,68 +291,58 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
         // ---- 1. per key channel: the cumulative log decay; a = exp(G - Gm), every row relative to the middle row of its block of
         // 16, left in the staging boxes in place of g; then the per-block factor tables.  Thread (part, d): rows 32 part ..
         // 32 part + 31 of channel d, i.e. row blocks 2 part and 2 part + 1 (a needs nothing from the other half).
-        // A block's sums begin anew at its first row and behind its middle row, and a table entry is the exponential of the sum of just the decays between its
-        // two rows: no difference of long sums, whose rounding the exponential would pass on.  The states' distance from 64 bits, decays of e^-4 and e^-5.8 a
-        // row that vary by a fifth: 4.5e-6 and 3.4e-6; with sums over 32 rows and their differences 1.1e-5 and 1.7e-5, over sixteen 1.0e-5 and 1.5e-5; at e^-2 and
-        // milder the operands' rounding is all there is to see, either way.
         {
             const int part = gt >> 7, d = gt & 127;
             // Row r of this thread's channel: box d / 32, piece (d % 32) / 4 swizzled by r & 7, float d % 4.
             unsigned char* col = gs + gG + (d >> 5) * kBox + part * 32 * 128 + (d & 3) * 4;
             const int pc = (d >> 2) & 7;
-            float* tmp = reinterpret_cast<float*>(gs + gKb) + d;  // to the middles [4][128], behind them [4][128]: the Kgb tile is not in use yet
+            float* tmp = reinterpret_cast<float*>(gs + gKb);  // totals [2][128], middles [4][128]; for strong decays, from a half's first middle to its second and on to its end [2][2][128]: the Kgb tile is not in use yet
             float run[32], acc = 0.0f;
+            bool strong = false;
 #pragma unroll
             for (int r = 0; r < 32; ++r) {
-                if ((r & 15) == 0 || (r & 15) == 9) acc = 0.0f;
+                if (!LAYER && r == 9) strong = acc < kStrong;
+                if ((r & 15) == 9 || r == 16) acc = strong ? 0.0f : acc;
                 acc = fmaf(*reinterpret_cast<const float*>(col + r * 128 + ((pc ^ (r & 7)) << 4)), kLog2e, acc);  // in powers of two from here on
                 run[r] = acc;
             }
-#pragma unroll
-            for (int b = 0; b < 2; ++b) {
-                tmp[(2 * part + b) * 128] = run[16 * b + 8];
-                tmp[(4 + 2 * part + b) * 128] = run[16 * b + 15];
+            const float mid0 = strong ? 0.0f : run[8], mid1 = strong ? 0.0f : run[24];
+            const float upto = (run[8] + run[15]) + run[24], to_mid1 = strong ? upto : run[24];
+            acc = strong ? upto + run[31] : acc;
+            if (!LAYER) {
+                tmp[(6 + 2 * part) * 128 + d] = run[15] + run[24];
+                tmp[(7 + 2 * part) * 128 + d] = run[31];
             }
+            tmp[part * 128 + d] = acc;
+            tmp[(2 + 2 * part) * 128 + d] = run[8];
+            tmp[(3 + 2 * part) * 128 + d] = to_mid1;
             float amax = 0.0f;
 #pragma unroll
             for (int r = 0; r < 32; ++r) {
-                const float av = ex2_ftz(max_nan((r & 15) <= 8 ? run[r] - run[(r & 16) | 8] : run[r], -126.0f));  // never 0: its reciprocal is taken
+                const float av = ex2_ftz(max_nan(run[r] - ((r & 15) <= 8 ? run[(r & 16) | 8] : r < 16 ? mid0 : mid1), -126.0f));  // never 0: its reciprocal is taken
                 amax = fmaxf(amax, av);
                 *reinterpret_cast<float*>(col + r * 128 + ((pc ^ (r & 7)) << 4)) = av;
             }
             // Eight rows of decay must stay below e^85: per-row log decays below about -10.6 (or positive ones) do not.  (Behind the
             // middle the factors stop at 2^-126; a block's last row is the first to.)
-            if (!(amax < 1e37f) || run[15] < -126.0f || run[31] < -126.0f) atomicCAS(p.status, 0, kStatusPrefillRange);
+            if (!(amax < 1e37f) || run[15] - mid0 < -126.0f || run[31] - mid1 < -126.0f) atomicCAS(p.status, 0, kStatusPrefillRange);
             group_sync();
-            float to[4], behind[4], all[4];
-#pragma unroll
-            for (int b = 0; b < 4; ++b) {
-                to[b] = tmp[b * 128];
-                behind[b] = tmp[(4 + b) * 128];
-                all[b] = to[b] + behind[b];
-            }
-            const float first2 = all[0] + all[1], first3 = first2 + all[2], gl = first3 + all[3];
+            const float base1 = tmp[d];
+            const float gm0 = tmp[2 * 128 + d], gm1 = tmp[3 * 128 + d], gm2 = base1 + tmp[4 * 128 + d], gm3 = base1 + tmp[5 * 128 + d];
+            const float gl = base1 + tmp[128 + d];
             // (Denormals are wanted here: sixteen rows at the gate's bound decay by e^-93, and their factor meets others of e^+40 and e^+46.)
             float* tab = reinterpret_cast<float*>(gs + gTab) + d;
-            auto own = [&](int b, float before, float after) {
-                const float e0 = ex2_approx(before), el = ex2_approx(after);
-                tab[(tE0 + b) * 128] = e0;
-                tab[(tEL + b) * 128] = el;
-                reinterpret_cast<float*>(gs + gE0L)[b * 128 + d] = e0 * el;
-            };
             if (part == 0) {
-                const float last2 = all[2] + all[3];
-                own(0, to[0], behind[0] + (all[1] + last2));
-                own(1, all[0] + to[1], behind[1] + last2);
-                own(2, first2 + to[2], behind[2] + all[3]);
-                tab[(tF + 0) * 128] = ex2_approx(behind[0] + to[1]);
+                tab[(tE0 + 0) * 128] = ex2_approx(gm0); tab[(tE0 + 1) * 128] = ex2_approx(gm1); tab[(tE0 + 2) * 128] = ex2_approx(gm2); tab[(tE0 + 3) * 128] = ex2_approx(gm3);
+                tab[(tEL + 0) * 128] = ex2_approx(gl - gm0); tab[(tEL + 1) * 128] = ex2_approx(gl - gm1);
+                tab[(tEL + 2) * 128] = ex2_approx(gl - gm2); tab[(tEL + 3) * 128] = ex2_approx(gl - gm3);
             } else {
-                own(3, first3 + to[3], behind[3]);
-                tab[(tF + 1) * 128] = ex2_approx((behind[0] + all[1]) + to[2]); tab[(tF + 2) * 128] = ex2_approx(behind[1] + to[2]);
-                tab[(tF + 3) * 128] = ex2_approx((behind[0] + (all[1] + all[2])) + to[3]); tab[(tF + 4) * 128] = ex2_approx((behind[1] + all[2]) + to[3]); tab[(tF + 5) * 128] = ex2_approx(behind[2] + to[3]);
+                tab[(tF + 0) * 128] = ex2_approx(gm1 - gm0);
+                tab[(tF + 1) * 128] = ex2_approx(gm2 - gm0); tab[(tF + 2) * 128] = ex2_approx(gm2 - gm1);
+                tab[(tF + 3) * 128] = ex2_approx(gm3 - gm0); tab[(tF + 4) * 128] = ex2_approx(gm3 - gm1); tab[(tF + 5) * 128] = ex2_approx(gm3 - gm2);
                 const float egl = ex2_approx(gl);
                 if (!ONE) reinterpret_cast<float*>(slot + wEgl)[d] = egl;
-                else reinterpret_cast<float*>(gs + gGl)[d] = egl;
+                reinterpret_cast<float*>(gs + gGl)[d] = egl;
             }
             mild = gl > -60.0f * kLog2e;
         }
@@ -366,8 +363,8 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
         auto piece = [&](int t) { return (gw >> 1) * 4 + (lane >> 4) * 2 + (t & 1); };
         if (narrow) {
             // One reference (the chunk's start): Kg = K exp(G) (over K) is the row side of L and the operand of W, Kinv = K exp(-G)
-            // (in Kgb's place) the one column-side tile, Kdec = Kinv exp(Gm) exp(G_last - Gm), the two as one factor, which meets the reciprocal of
-            // the same exp(Gm), as bf16 hi + lo out to the workspace, Qg = Q exp(G) (over Q and out) the row side of M.  All from one read of a, in a loop that stays a loop: the group's instructions are more than
+            // (in Kgb's place) the one column-side tile, Kdec = Kinv exp(G_last) as bf16 hi + lo out to the workspace, Qg = Q exp(G) (over Q and
+            // out) the row side of M.  All from one read of a, in a loop that stays a loop: the group's instructions are more than
             // the cache next to the warps holds.
             if (!mbar_wait(bar_raw, raw_phase, ctx, kStatusWaitPrefill)) break;
             raw_phase ^= 1u;
@@ -377,7 +374,7 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
                 const uint4 k8 = *reinterpret_cast<const uint4*>(gs + gK + box_piece(r, c)), q8 = *reinterpret_cast<const uint4*>(gs + gQ + box_piece(r, c));
                 const float4 aa = *reinterpret_cast<const float4*>(gs + gG + box_piece(r, 2 * c)), ab = *reinterpret_cast<const float4*>(gs + gG + box_piece(r, 2 * c + 1));
                 const float4 e0a = *reinterpret_cast<const float4*>(tabs + (tE0 + J) * 128 + c * 8), e0b = *reinterpret_cast<const float4*>(tabs + (tE0 + J) * 128 + c * 8 + 4);
-                const float4 gla = *reinterpret_cast<const float4*>(gs + gE0L + J * 512 + c * 32), glb = *reinterpret_cast<const float4*>(gs + gE0L + J * 512 + c * 32 + 16);
+                const float4 gla = *reinterpret_cast<const float4*>(gs + gGl + c * 32), glb = *reinterpret_cast<const float4*>(gs + gGl + c * 32 + 16);
                 const float2 A[4] = {{aa.x, aa.y}, {aa.z, aa.w}, {ab.x, ab.y}, {ab.z, ab.w}};
                 const float2 E0[4] = {{e0a.x, e0a.y}, {e0a.z, e0a.w}, {e0b.x, e0b.y}, {e0b.z, e0b.w}};
                 const float2 GL[4] = {{gla.x, gla.y}, {gla.z, gla.w}, {glb.x, glb.y}, {glb.z, glb.w}};
@@ -400,6 +397,22 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
                 *reinterpret_cast<uint4*>(cell(slot + wQg, CH, c, r)) = make_uint4(qg[0], qg[1], qg[2], qg[3]);
             }
         } else {
+            if constexpr (!LAYER) {  // the factors between two rows once more (kStrong)
+                const int part = gt >> 7, d = gt & 127;
+                const float* tmp = reinterpret_cast<const float*>(gs + gKb) + d;
+                float* tab = reinterpret_cast<float*>(gs + gTab) + d;
+                const float end0 = tmp[0], end1 = tmp[128], m0 = tmp[2 * 128], m1 = tmp[3 * 128], m2 = tmp[4 * 128], m3 = tmp[5 * 128];
+                const bool s0 = m0 < kStrong, s1 = m2 < kStrong;
+                const float b01 = s0 ? tmp[6 * 128] : m1 - m0, b23 = s1 ? tmp[8 * 128] : m3 - m2;
+                const float r1 = s0 ? tmp[7 * 128] : end0 - m1, r3 = s1 ? tmp[9 * 128] : end1 - m3, r0 = b01 + r1, r2 = b23 + r3;
+                if (part == 0) {
+                    tab[(tEL + 0) * 128] = ex2_approx(r0 + end1); tab[(tEL + 1) * 128] = ex2_approx(r1 + end1); tab[(tEL + 2) * 128] = ex2_approx(r2); tab[(tEL + 3) * 128] = ex2_approx(r3);
+                } else {
+                    tab[(tF + 0) * 128] = ex2_approx(b01);
+                    tab[(tF + 1) * 128] = ex2_approx(r0 + m2); tab[(tF + 2) * 128] = ex2_approx(r1 + m2);
+                    tab[(tF + 3) * 128] = ex2_approx(r0 + m3); tab[(tF + 4) * 128] = ex2_approx(r1 + m3); tab[(tF + 5) * 128] = ex2_approx(b23);
+                }
+            }
             // a into registers: the column-side tiles go over it.  Then the tiles made from k: row side Kgb = K a; Kg = K exp(G)
             // (over K) for W; Kdec = K exp(G_last - G) as bf16 hi + lo out to the workspace; column sides K exp(Gm_I - G) into the
             // tiles I >= J.
