@@ -191,8 +191,8 @@ constexpr int kGroupThreads = 256, kGroups = 2;
 // block-wise references) begins its sums anew at a block's first row and behind its middle row, and block-wise chunks form their tables once more, from the sums of
 // just the decays between two rows.  The states' distance from 64 bits, decays of e^-4 and e^-5.8 a row that vary by a fifth: 4.5e-6 and 3.4e-6; from differences
 // 1.1e-5 and 1.7e-5, of sums over sixteen rows 1.0e-5 and 1.5e-5; at e^-0.9 and milder the operands' rounding is all there is to see, either way.
-// us, before / so: 8,192 rows in 8 sequences 467 / 467, strong 496 / 498; 65,536 rows x 64 heads 3,532 / 3,544; 16,384 rows x 8 heads without a workspace 1,686 / 1,691.
-// The choice by a branch, or before the factors are formed, cost all chunks 1 to 3 %.
+// us, before / so: 8,192 rows in 8 sequences 463 / 463, 65,536 rows x 64 heads 3,555 / 3,559, 1,000 without a workspace 122.0 / 122.4; strong decays, 16,384 x 64 940 / 956, 1,000
+// without 141.2 / 141.9.  The choice by a branch, or before the factors are formed, cost all chunks 1 to 3 %.
 constexpr float kStrong = -8.5f * kLog2e;
 // Decay range.  L and M hold exp(G_i - G_j) for every pair of rows j <= i of a chunk, and a tensor-core product can
 // only form it as (row factor) x (column factor).  With the model's gate bound (log decay down to -5.8 per row, -371
@@ -398,7 +398,9 @@ __device__ __forceinline__ void intra_group(const SpParams& p, unsigned char* sm
             }
         } else {
             if constexpr (!LAYER) {  // the factors between two rows once more (kStrong)
-                const int part = gt >> 7, d = gt & 127;
+                int thread = threadIdx.x - G * kGroupThreads;
+                asm volatile("" : "+r"(thread));  // formed anew: kept from the sums on it costs registers all the way (with the norm, 1,000 rows 131.7 -> 136.1 us)
+                const int part = thread >> 7, d = thread & 127;
                 const float* tmp = reinterpret_cast<const float*>(gs + gKb) + d;
                 float* tab = reinterpret_cast<float*>(gs + gTab) + d;
                 const float end0 = tmp[0], end1 = tmp[128], m0 = tmp[2 * 128], m1 = tmp[3 * 128], m2 = tmp[4 * 128], m3 = tmp[5 * 128];
